@@ -623,16 +623,21 @@ attn_fwd_v2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             }
             packed[i / 2] = pack_bf16(e0, e1);
           }
+          // P has one set of columns: P(j-1)·V(j-1) must have read it before block j's probabilities overwrite it.  S(j)
+          // says nothing about that (Q·K(j) is issued ahead of P(j-1)·V(j-1)).  The MMA was issued a whole pass 1 and half
+          // a pass 2 ago, so the wait is short; without it single warps' 32 rows came out wrong when two CTAs shared an SM.
+          if (c == 0 && j > 0) {
+            mbar_wait(o_full, (j - 1) & 1);
+            tc_fence_after_sync();
+          }
           tmem_st_32x32b_x16(p_addr + c * 16, packed);
         }
         rowsum = rs0 + rs1;
       };
       if (need_mask) pass2(std::true_type{}); else pass2(std::false_type{});
       l_run = l_run * alpha + rowsum;
-      // ---- O *= alpha (rare): wait until P·V of block j-1 has retired, then rescale this half's O columns
+      // ---- O *= alpha (rare): P·V of block j-1 has retired (waited for above), rescale this half's O columns
       if (bump_any) {
-        mbar_wait(o_full, (j - 1) & 1);
-        tc_fence_after_sync();
 #pragma unroll
         for (int c = 0; c < D / 64; ++c) {
           uint32_t t[32];
