@@ -38,12 +38,16 @@ struct Vec8<float> {
   }
 };
 
-// H = VPL * 256 elements per row (each lane owns VPL vectors of 8, interleaved for coalescing)
-template <typename T, typename W, int VPL, bool RMS>
+// H = VPL * 256 elements per row (each lane owns VPL vectors of 8, interleaved for coalescing); with TAIL any H % 8 == 0
+// in (256 (VPL - 1), 256 VPL): the lanes behind the row's end hold zeros.  h = 384 and 192 (the shipped GPT / T5 recipes)
+// took the one-element-per-lane kernel below before: forward 3.4 -> 2.7 us on [200, 384], backward 27 -> 6.6 us on [2048, 384].
+// Whole multiples of 256 keep a compile-time width (the backward of [8192, 1024] is 8 % slower with a run-time one).
+template <typename T, typename W, int VPL, bool RMS, bool TAIL>
 __global__ void __launch_bounds__(NORM_WARPS * 32)
 norm_fwd_kernel(const T* __restrict__ x, const W* __restrict__ gamma, const W* __restrict__ beta, T* __restrict__ y,
-                float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, float eps) {
-  constexpr int H = VPL * 256;
+                float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, float eps, int h_tail) {
+  const int H = TAIL ? h_tail : VPL * 256;
+  const float inv_h = 1.0f / static_cast<float>(H);
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   for (int row = blockIdx.x * NORM_WARPS + warp; row < rows; row += gridDim.x * NORM_WARPS) {
     const T* xr = x + static_cast<size_t>(row) * H;
@@ -51,21 +55,28 @@ norm_fwd_kernel(const T* __restrict__ x, const W* __restrict__ gamma, const W* _
     float s = 0.f;
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
+      if (TAIL && (i * 32 + lane) * 8 >= H) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[i][j] = 0.f;
+        continue;
+      }
       Vec8<T>::load(xr + (i * 32 + lane) * 8, v[i]);
 #pragma unroll
       for (int j = 0; j < 8; ++j) s += v[i][j];
     }
     float mean = 0.f;
-    if (!RMS) mean = warp_sum(s) * (1.0f / H);
+    if (!RMS) mean = warp_sum(s) * inv_h;
     float sq = 0.f;
 #pragma unroll
-    for (int i = 0; i < VPL; ++i)
+    for (int i = 0; i < VPL; ++i) {
+      if (TAIL && (i * 32 + lane) * 8 >= H) continue;
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const float d = v[i][j] - mean;
         sq += d * d;
       }
-    const float rstd = rsqrtf(warp_sum(sq) * (1.0f / H) + eps);
+    }
+    const float rstd = rsqrtf(warp_sum(sq) * inv_h + eps);
     if (lane == 0) {
       if (mean_out) mean_out[row] = mean;
       rstd_out[row] = rstd;
@@ -73,6 +84,7 @@ norm_fwd_kernel(const T* __restrict__ x, const W* __restrict__ gamma, const W* _
     T* yr = y + static_cast<size_t>(row) * H;
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
+      if (TAIL && (i * 32 + lane) * 8 >= H) continue;
       float g[8], b[8], o[8];
       Vec8<W>::load(gamma + (i * 32 + lane) * 8, g);
       if (beta != nullptr) Vec8<W>::load(beta + (i * 32 + lane) * 8, b);
@@ -169,13 +181,15 @@ norm_bwd_kernel(const T* __restrict__ gy, const T* __restrict__ x, const W* __re
 // ALU is free here), and blocks are 4 warps at <= 168 registers → 12 warps per SM with 12 loads each in flight.
 constexpr int NORM_BWD_WARPS = 4;
 
-template <typename W, int VPL, bool RMS>
+template <typename W, int VPL, bool RMS, bool TAIL>
 __global__ void __launch_bounds__(NORM_BWD_WARPS * 32, 3)
 norm_bwd_bf16_kernel(const __nv_bfloat16* __restrict__ gy, const __nv_bfloat16* __restrict__ x, const W* __restrict__ gamma,
                      const float* __restrict__ mean_in, const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ gx,
                      float* __restrict__ part_dgamma, float* __restrict__ part_dbeta, int rows,
-                     const __nv_bfloat16* __restrict__ gadd, float* __restrict__ acc_dgamma, float* __restrict__ acc_dbeta) {
-  constexpr int H = VPL * 256;
+                     const __nv_bfloat16* __restrict__ gadd, float* __restrict__ acc_dgamma, float* __restrict__ acc_dbeta,
+                     int h_tail) {
+  const int H = TAIL ? h_tail : VPL * 256;       // TAIL: lanes behind the row's end neither load nor store
+  const float inv_h = 1.0f / static_cast<float>(H);
   __shared__ float red[NORM_BWD_WARPS][32 * 8 + 8];
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   float dg[VPL][8], db[VPL][8];
@@ -194,18 +208,21 @@ norm_bwd_bf16_kernel(const __nv_bfloat16* __restrict__ gy, const __nv_bfloat16* 
     uint4 xq[VPL], gq[VPL], aq[VPL];
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
-      xq[i] = *reinterpret_cast<const uint4*>(x + base + (i * 32 + lane) * 8);
-      gq[i] = *reinterpret_cast<const uint4*>(gy + base + (i * 32 + lane) * 8);
+      const bool ok = !TAIL || (i * 32 + lane) * 8 < H;
+      xq[i] = ok ? *reinterpret_cast<const uint4*>(x + base + (i * 32 + lane) * 8) : make_uint4(0, 0, 0, 0);
+      gq[i] = ok ? *reinterpret_cast<const uint4*>(gy + base + (i * 32 + lane) * 8) : make_uint4(0, 0, 0, 0);
     }
     if (gadd != nullptr) {
 #pragma unroll
-      for (int i = 0; i < VPL; ++i) aq[i] = *reinterpret_cast<const uint4*>(gadd + base + (i * 32 + lane) * 8);
+      for (int i = 0; i < VPL; ++i)
+        aq[i] = (!TAIL || (i * 32 + lane) * 8 < H) ? *reinterpret_cast<const uint4*>(gadd + base + (i * 32 + lane) * 8) : make_uint4(0, 0, 0, 0);
     }
     const float mean = RMS ? 0.f : mean_in[row];
     const float rstd = rstd_in[row];
     float s1 = 0.f, s2 = 0.f;
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
+      if (TAIL && (i * 32 + lane) * 8 >= H) continue;
       float xv[8], gv[8], gm[8];
       unpack8(xq[i], xv);
       unpack8(gq[i], gv);
@@ -220,10 +237,11 @@ norm_bwd_bf16_kernel(const __nv_bfloat16* __restrict__ gy, const __nv_bfloat16* 
         db[i][j] += gv[j];
       }
     }
-    s1 = RMS ? 0.f : warp_sum(s1) * (1.0f / H);
-    s2 = warp_sum(s2) * (1.0f / H);
+    s1 = RMS ? 0.f : warp_sum(s1) * inv_h;
+    s2 = warp_sum(s2) * inv_h;
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
+      if (TAIL && (i * 32 + lane) * 8 >= H) continue;
       float xv[8], gv[8], gm[8], o[8];
       unpack8(xq[i], xv);
       unpack8(gq[i], gv);
@@ -251,6 +269,7 @@ norm_bwd_bf16_kernel(const __nv_bfloat16* __restrict__ gy, const __nv_bfloat16* 
       __syncthreads();
       for (int c = threadIdx.x; c < 256; c += NORM_BWD_WARPS * 32) {
         float acc = 0.f;
+        if (TAIL && i * 256 + c >= H) continue;
 #pragma unroll
         for (int w = 0; w < NORM_BWD_WARPS; ++w) acc += red[w][c];
         if (acc_dgamma != nullptr) {
@@ -261,6 +280,181 @@ norm_bwd_bf16_kernel(const __nv_bfloat16* __restrict__ gy, const __nv_bfloat16* 
           float* dst = (which == 0 ? part_dgamma : part_dbeta) + static_cast<size_t>(blockIdx.x) * H + i * 256 + c;
           *dst = acc;
         }
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
+// Wide bf16 rows (1024 < H <= 8192, H % 8 == 0): one 256-thread block per row, V = ceil(H / 2048) 16-byte vectors per
+// thread.  Bandwidth-bound.  With a warp per row a lane of a 4096-wide row held 16 vectors, i.e. 2 x 128 fp32 column sums
+// next to x̂ and g·γ: it spilled, and [2048, 4096] took 298 us backward (13.6 us forward) where the 50 MB (34 MB) it moves
+// take 8 us (5 us).  Spread over a block the column sums are 16 V registers, every row's loads are issued at once and the two
+// row sums cost one barrier: 20.6 us backward, 7.6 us forward.  Few rows (a decoding step) gain as well: a row is no longer one
+// warp's serial walk (4 rows of 4096: 9.9 -> 2.8 us).
+// ---------------------------------------------------------------------------------------------------------------------
+constexpr int NORM_WIDE_THREADS = 256;
+
+// sums of two values over the block; `buf` alternates so that one barrier per call is enough
+LB_DEVICE float2 norm_block_sum2(float a, float b, float2 (*red)[NORM_WIDE_THREADS / 32], int& buf) {
+  a = warp_sum(a);
+  b = warp_sum(b);
+  if (threadIdx.x % 32 == 0) red[buf][threadIdx.x / 32] = make_float2(a, b);
+  __syncthreads();
+  float2 t = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int w = 0; w < NORM_WIDE_THREADS / 32; ++w) {
+    const float2 r = red[buf][w];
+    t.x += r.x;
+    t.y += r.y;
+  }
+  buf ^= 1;
+  return t;
+}
+LB_DEVICE void norm_unpack8(const uint4& q, float (&v)[8]) {
+  const float2 a = unpack_bf16(q.x), b = unpack_bf16(q.y), c = unpack_bf16(q.z), d = unpack_bf16(q.w);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = c.x; v[5] = c.y; v[6] = d.x; v[7] = d.y;
+}
+
+template <typename W, int V, bool RMS>
+__global__ void __launch_bounds__(NORM_WIDE_THREADS)
+norm_fwd_wide_kernel(const __nv_bfloat16* __restrict__ x, const W* __restrict__ gamma, const W* __restrict__ beta,
+                     __nv_bfloat16* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int H,
+                     float eps) {
+  __shared__ float2 red[2][NORM_WIDE_THREADS / 32];
+  int buf = 0;
+  const float inv_h = 1.0f / static_cast<float>(H);
+  for (int row = blockIdx.x; row < rows; row += gridDim.x) {
+    const size_t base = static_cast<size_t>(row) * H;
+    uint4 q[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      const int c = (i * NORM_WIDE_THREADS + threadIdx.x) * 8;
+      q[i] = c < H ? *reinterpret_cast<const uint4*>(x + base + c) : make_uint4(0, 0, 0, 0);
+    }
+    float mean = 0.f;
+    if (!RMS) {
+      float s = 0.f;
+#pragma unroll
+      for (int i = 0; i < V; ++i) {
+        float v[8];
+        norm_unpack8(q[i], v);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s += v[j];
+      }
+      mean = norm_block_sum2(s, 0.f, red, buf).x * inv_h;
+    }
+    float sq = 0.f;
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      if ((i * NORM_WIDE_THREADS + static_cast<int>(threadIdx.x)) * 8 >= H) continue;
+      float v[8];
+      norm_unpack8(q[i], v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sq += (v[j] - mean) * (v[j] - mean);
+    }
+    const float rstd = rsqrtf(norm_block_sum2(sq, 0.f, red, buf).x * inv_h + eps);
+    if (threadIdx.x == 0) {
+      if (mean_out) mean_out[row] = mean;
+      rstd_out[row] = rstd;
+    }
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      const int c = (i * NORM_WIDE_THREADS + threadIdx.x) * 8;
+      if (c >= H) continue;
+      float v[8], g[8], b[8], o[8];
+      norm_unpack8(q[i], v);
+      Vec8<W>::load(gamma + c, g);
+      if (beta != nullptr) Vec8<W>::load(beta + c, b);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        o[j] = (v[j] - mean) * rstd * g[j];
+        if (beta != nullptr) o[j] += b[j];
+      }
+      Vec8<__nv_bfloat16>::store(y + base + c, o);
+    }
+  }
+}
+
+// Column sums: added straight into the fp32 gradients (`acc_*`: 16-byte aligned, one vector reduction per 4 columns and
+// block), or left as one row of partials per block for colreduce_kernel.
+template <typename W, int V, bool RMS>
+__global__ void __launch_bounds__(NORM_WIDE_THREADS, V <= 2 ? 3 : 1)
+norm_bwd_wide_kernel(const __nv_bfloat16* __restrict__ gy, const __nv_bfloat16* __restrict__ x, const W* __restrict__ gamma,
+                     const float* __restrict__ mean_in, const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ gx,
+                     float* __restrict__ part_dgamma, float* __restrict__ part_dbeta, int rows, int H,
+                     const __nv_bfloat16* __restrict__ gadd, float* __restrict__ acc_dgamma, float* __restrict__ acc_dbeta) {
+  __shared__ float2 red[2][NORM_WIDE_THREADS / 32];
+  int buf = 0;
+  const float inv_h = 1.0f / static_cast<float>(H);
+  float dg[V][8], db[V][8];
+#pragma unroll
+  for (int i = 0; i < V; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) dg[i][j] = db[i][j] = 0.f;
+  for (int row = blockIdx.x; row < rows; row += gridDim.x) {
+    const size_t base = static_cast<size_t>(row) * H;
+    uint4 xq[V], gq[V], aq[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      const int c = (i * NORM_WIDE_THREADS + threadIdx.x) * 8;
+      const bool ok = c < H;
+      xq[i] = ok ? *reinterpret_cast<const uint4*>(x + base + c) : make_uint4(0, 0, 0, 0);
+      gq[i] = ok ? *reinterpret_cast<const uint4*>(gy + base + c) : make_uint4(0, 0, 0, 0);
+      aq[i] = (ok && gadd != nullptr) ? *reinterpret_cast<const uint4*>(gadd + base + c) : make_uint4(0, 0, 0, 0);
+    }
+    const float mean = RMS ? 0.f : mean_in[row];
+    const float rstd = rstd_in[row];
+    float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      const int c = (i * NORM_WIDE_THREADS + threadIdx.x) * 8;
+      if (c >= H) continue;
+      float xv[8], gv[8], gm[8];
+      norm_unpack8(xq[i], xv);
+      norm_unpack8(gq[i], gv);
+      Vec8<W>::load(gamma + c, gm);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float xh = (xv[j] - mean) * rstd, gw = gv[j] * gm[j];
+        s1 += gw;
+        s2 += gw * xh;
+        dg[i][j] += gv[j] * xh;
+        db[i][j] += gv[j];
+      }
+    }
+    const float2 t = norm_block_sum2(s1, s2, red, buf);
+    s1 = RMS ? 0.f : t.x * inv_h;
+    s2 = t.y * inv_h;
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      const int c = (i * NORM_WIDE_THREADS + threadIdx.x) * 8;
+      if (c >= H) continue;
+      float xv[8], gv[8], gm[8], av[8], o[8];
+      norm_unpack8(xq[i], xv);
+      norm_unpack8(gq[i], gv);
+      norm_unpack8(aq[i], av);
+      Vec8<W>::load(gamma + c, gm);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] = rstd * (gv[j] * gm[j] - s1 - (xv[j] - mean) * rstd * s2) + av[j];
+      Vec8<__nv_bfloat16>::store(gx + base + c, o);
+    }
+  }
+  const bool direct = acc_dgamma != nullptr;
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    const int c = (i * NORM_WIDE_THREADS + threadIdx.x) * 8;
+    if (c >= H) continue;
+#pragma unroll
+    for (int which = 0; which < 2; ++which) {
+      if (which == 1 && part_dbeta == nullptr) continue;
+      const float(&v)[8] = which == 0 ? dg[i] : db[i];
+      if (direct) {
+        float* dst = (which == 0 ? acc_dgamma : acc_dbeta) + c;
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"l"(dst), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"l"(dst + 4), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
+      } else {
+        Vec8<float>::store((which == 0 ? part_dgamma : part_dbeta) + static_cast<size_t>(blockIdx.x) * H + c, v);
       }
     }
   }
@@ -370,31 +564,34 @@ int norm_sms() {
   }
   return sms;
 }
-int norm_grid(int rows) {
-  const int need = (rows + lb::NORM_WARPS - 1) / lb::NORM_WARPS;
-  const int cap = norm_sms() * 2;
+int norm_grid_of(int rows, int rows_per_block, int blocks_per_sm) {
+  const int need = (rows + rows_per_block - 1) / rows_per_block;
+  const int cap = norm_sms() * blocks_per_sm;
   return need < cap ? need : cap;
 }
+int norm_grid(int rows) { return norm_grid_of(rows, lb::NORM_WARPS, 2); }
 // forward: 64 registers → four 8-warp blocks per SM
-int norm_fwd_grid(int rows) {
-  const int need = (rows + lb::NORM_WARPS - 1) / lb::NORM_WARPS;
-  const int cap = norm_sms() * 4;
-  return need < cap ? need : cap;
-}
+int norm_fwd_grid(int rows) { return norm_grid_of(rows, lb::NORM_WARPS, 4); }
 // bf16 backward: three 4-warp blocks per SM (one wave; every block leaves one row of column partials)
-int norm_bwd_bf16_grid(int rows) {
-  const int need = (rows + lb::NORM_BWD_WARPS - 1) / lb::NORM_BWD_WARPS;
-  const int cap = norm_sms() * 3;
-  return need < cap ? need : cap;
-}
+int norm_bwd_bf16_grid(int rows) { return norm_grid_of(rows, lb::NORM_BWD_WARPS, 3); }
+// wide rows: blocks loop over rows; the backward keeps to one wave because every block adds its column sums at the end
+int norm_fwd_wide_grid(int rows) { return norm_grid_of(rows, 1, 6); }
+int norm_bwd_wide_grid(int rows, int H) { return norm_grid_of(rows, 1, H <= 4096 ? 3 : 1); }
 
-template <typename T, typename W, bool RMS>
-bool fwd_dispatch(int vpl, const T* x, const W* g, const W* b, T* y, float* mean, float* rstd, int rows, float eps,
-                  cudaStream_t s) {
+bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+// bf16 rows of whole 16-byte vectors: the warp kernel up to 1024 columns (four vectors per lane: beyond that its column sums
+// spill), the block kernel up to 8192
+constexpr int NORM_WARP_MAX_H = 1024, NORM_WIDE_MAX_H = 8192;
+bool norm_vec_bf16(int H, int dtype) { return dtype == 0 && H % 8 == 0 && H <= NORM_WIDE_MAX_H; }
+
+// fp32 activations: H = 256 VPL
+template <bool RMS>
+bool fwd_dispatch_f32(int vpl, const float* x, const float* g, const float* b, float* y, float* mean, float* rstd, int rows,
+                      float eps, cudaStream_t s) {
   const int grid = norm_fwd_grid(rows);
-#define LB_CASE(V)                                                                                             \
-  case V:                                                                                                      \
-    lb::norm_fwd_kernel<T, W, V, RMS><<<grid, lb::NORM_WARPS * 32, 0, s>>>(x, g, b, y, mean, rstd, rows, eps); \
+#define LB_CASE(V)                                                                                                            \
+  case V:                                                                                                                     \
+    lb::norm_fwd_kernel<float, float, V, RMS, false><<<grid, lb::NORM_WARPS * 32, 0, s>>>(x, g, b, y, mean, rstd, rows, eps, 0); \
     return true;
   switch (vpl) {
     LB_CASE(1) LB_CASE(2) LB_CASE(3) LB_CASE(4) LB_CASE(5) LB_CASE(6) LB_CASE(8) LB_CASE(10) LB_CASE(12) LB_CASE(16)
@@ -406,35 +603,63 @@ bool fwd_dispatch(int vpl, const T* x, const W* g, const W* b, T* y, float* mean
 }
 
 template <typename W, bool RMS>
-bool bwd_dispatch_bf16(int vpl, const __nv_bfloat16* gy, const __nv_bfloat16* x, const W* g, const float* mean,
-                       const float* rstd, __nv_bfloat16* gx, float* pdg, float* pdb, int rows, int grid, cudaStream_t s,
-                       const __nv_bfloat16* gadd, float* acc_dg, float* acc_db) {
-#define LB_CASE(V)                                                                                                        \
-  case V:                                                                                                                 \
-    lb::norm_bwd_bf16_kernel<W, V, RMS><<<grid, lb::NORM_BWD_WARPS * 32, 0, s>>>(gy, x, g, mean, rstd, gx, pdg, pdb, rows, gadd, \
-                                                                                 acc_dg, acc_db);                         \
-    return true;
-  switch (vpl) {
-    LB_CASE(1) LB_CASE(2) LB_CASE(3) LB_CASE(4)
-    default:
-      return false;
+void fwd_dispatch_bf16(int H, const __nv_bfloat16* x, const W* g, const W* b, __nv_bfloat16* y, float* mean, float* rstd, int rows,
+                       float eps, cudaStream_t s) {
+  if (H <= NORM_WARP_MAX_H) {
+    const int grid = norm_fwd_grid(rows);
+#define LB_CASE(V)                                                                                                                  \
+  case V:                                                                                                                           \
+    if (H % 256 == 0)                                                                                                               \
+      lb::norm_fwd_kernel<__nv_bfloat16, W, V, RMS, false><<<grid, lb::NORM_WARPS * 32, 0, s>>>(x, g, b, y, mean, rstd, rows, eps, H); \
+    else                                                                                                                            \
+      lb::norm_fwd_kernel<__nv_bfloat16, W, V, RMS, true><<<grid, lb::NORM_WARPS * 32, 0, s>>>(x, g, b, y, mean, rstd, rows, eps, H);  \
+    break;
+    switch ((H + 255) / 256) { LB_CASE(1) LB_CASE(2) LB_CASE(3) LB_CASE(4) }
+#undef LB_CASE
+    return;
   }
+  const int grid = norm_fwd_wide_grid(rows);
+#define LB_CASE(V)                                                                                                             \
+  case V:                                                                                                                      \
+    lb::norm_fwd_wide_kernel<W, V, RMS><<<grid, lb::NORM_WIDE_THREADS, 0, s>>>(x, g, b, y, mean, rstd, rows, H, eps);          \
+    break;
+  switch ((H + 2047) / 2048) { LB_CASE(1) LB_CASE(2) LB_CASE(3) LB_CASE(4) }
 #undef LB_CASE
 }
-// H <= 1024 with bf16 activations takes the bandwidth-oriented kernel (wider rows would spill at 168 registers)
-bool norm_bwd_uses_bf16_kernel(int H, int dtype) { return dtype == 0 && H % 256 == 0 && H / 256 <= 4; }
 
-template <typename T, typename W, bool RMS>
-bool bwd_dispatch(int vpl, const T* gy, const T* x, const W* g, const float* mean, const float* rstd, T* gx, float* pdg,
-                  float* pdb, int rows, int grid, cudaStream_t s, const T* gadd, float* acc_dg = nullptr,
-                  float* acc_db = nullptr) {
-  if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-    if (norm_bwd_uses_bf16_kernel(vpl * 256, 0))
-      return bwd_dispatch_bf16<W, RMS>(vpl, gy, x, g, mean, rstd, gx, pdg, pdb, rows, grid, s, gadd, acc_dg, acc_db);
+template <typename W, bool RMS>
+void bwd_dispatch_bf16(int H, const __nv_bfloat16* gy, const __nv_bfloat16* x, const W* g, const float* mean, const float* rstd,
+                       __nv_bfloat16* gx, float* pdg, float* pdb, int rows, int grid, cudaStream_t s, const __nv_bfloat16* gadd,
+                       float* acc_dg, float* acc_db) {
+  if (H <= NORM_WARP_MAX_H) {
+#define LB_CASE(V)                                                                                                                 \
+  case V:                                                                                                                          \
+    if (H % 256 == 0)                                                                                                             \
+      lb::norm_bwd_bf16_kernel<W, V, RMS, false><<<grid, lb::NORM_BWD_WARPS * 32, 0, s>>>(gy, x, g, mean, rstd, gx, pdg, pdb, rows, \
+                                                                                          gadd, acc_dg, acc_db, H);               \
+    else                                                                                                                          \
+      lb::norm_bwd_bf16_kernel<W, V, RMS, true><<<grid, lb::NORM_BWD_WARPS * 32, 0, s>>>(gy, x, g, mean, rstd, gx, pdg, pdb, rows,  \
+                                                                                         gadd, acc_dg, acc_db, H);                \
+    break;
+    switch ((H + 255) / 256) { LB_CASE(1) LB_CASE(2) LB_CASE(3) LB_CASE(4) }
+#undef LB_CASE
+    return;
   }
-#define LB_CASE(V)                                                                                                   \
-  case V:                                                                                                            \
-    lb::norm_bwd_kernel<T, W, V, RMS><<<grid, lb::NORM_WARPS * 32, 0, s>>>(gy, x, g, mean, rstd, gx, pdg, pdb, rows, gadd); \
+#define LB_CASE(V)                                                                                                              \
+  case V:                                                                                                                       \
+    lb::norm_bwd_wide_kernel<W, V, RMS><<<grid, lb::NORM_WIDE_THREADS, 0, s>>>(gy, x, g, mean, rstd, gx, pdg, pdb, rows, H,     \
+                                                                               gadd, acc_dg, acc_db);                           \
+    break;
+  switch ((H + 2047) / 2048) { LB_CASE(1) LB_CASE(2) LB_CASE(3) LB_CASE(4) }
+#undef LB_CASE
+}
+
+template <bool RMS>
+bool bwd_dispatch_f32(int vpl, const float* gy, const float* x, const float* g, const float* mean, const float* rstd, float* gx,
+                      float* pdg, float* pdb, int rows, int grid, cudaStream_t s, const float* gadd) {
+#define LB_CASE(V)                                                                                                           \
+  case V:                                                                                                                    \
+    lb::norm_bwd_kernel<float, float, V, RMS><<<grid, lb::NORM_WARPS * 32, 0, s>>>(gy, x, g, mean, rstd, gx, pdg, pdb, rows, gadd); \
     return true;
   switch (vpl) {
     LB_CASE(1) LB_CASE(2) LB_CASE(3) LB_CASE(4) LB_CASE(5) LB_CASE(6) LB_CASE(8) LB_CASE(10) LB_CASE(12) LB_CASE(16)
@@ -443,48 +668,67 @@ bool bwd_dispatch(int vpl, const T* gy, const T* x, const W* g, const float* mea
   }
 #undef LB_CASE
 }
+
+template <typename W>
+void norm_fwd_bf16(const void* x, const void* gamma, const void* beta, void* y, float* mean, float* rstd, int rows, int H, float eps,
+                   int rms, cudaStream_t s) {
+  using T = __nv_bfloat16;
+  if (norm_vec_bf16(H, 0) && aligned16(x) && aligned16(y) && aligned16(gamma) && aligned16(beta)) {
+    if (rms) fwd_dispatch_bf16<W, true>(H, (const T*)x, (const W*)gamma, (const W*)beta, (T*)y, mean, rstd, rows, eps, s);
+    else fwd_dispatch_bf16<W, false>(H, (const T*)x, (const W*)gamma, (const W*)beta, (T*)y, mean, rstd, rows, eps, s);
+    return;
+  }
+  const int wpb = 8, grid = (rows + wpb - 1) / wpb;
+  if (rms) lb::norm_fwd_generic<T, W, true><<<grid, wpb * 32, 0, s>>>((const T*)x, (const W*)gamma, (const W*)beta, (T*)y, mean, rstd, rows, H, eps);
+  else lb::norm_fwd_generic<T, W, false><<<grid, wpb * 32, 0, s>>>((const T*)x, (const W*)gamma, (const W*)beta, (T*)y, mean, rstd, rows, H, eps);
+}
+template <typename T, typename W>
+void norm_bwd_any(const void* gy, const void* x, const void* gamma, const float* mean, const float* rstd, void* gx, float* dgamma,
+                  float* dbeta, int rows, int H, int rms, int accumulate, cudaStream_t s) {
+  if (!accumulate) {
+    cudaMemsetAsync(dgamma, 0, sizeof(float) * H, s);
+    if (dbeta != nullptr) cudaMemsetAsync(dbeta, 0, sizeof(float) * H, s);
+  }
+  const int wpb = 8, grid = (rows + wpb - 1) / wpb;
+  if (rms) lb::norm_bwd_generic<T, W, true><<<grid, wpb * 32, 0, s>>>((const T*)gy, (const T*)x, (const W*)gamma, mean, rstd, (T*)gx, dgamma, dbeta, rows, H);
+  else lb::norm_bwd_generic<T, W, false><<<grid, wpb * 32, 0, s>>>((const T*)gy, (const T*)x, (const W*)gamma, mean, rstd, (T*)gx, dgamma, dbeta, rows, H);
+}
 }  // namespace
 
 // dtype codes: 0 = bf16 activations, 1 = fp32 activations; wdtype: 0 = bf16 params, 1 = fp32 params
 extern "C" int lb_norm_fwd(const void* x, const void* gamma, const void* beta, void* y, float* mean, float* rstd,
                            int rows, int H, float eps, int rms, int dtype, int wdtype, cudaStream_t s) {
   if (rows == 0) return 0;
-  const bool fast = (H % 256 == 0);
-  bool done = false;
-#define LB_GO(T, W)                                                                                                   \
-  {                                                                                                                   \
-    if (fast) {                                                                                                       \
-      done = rms ? fwd_dispatch<T, W, true>(H / 256, (const T*)x, (const W*)gamma, (const W*)beta, (T*)y, mean, rstd, \
-                                            rows, eps, s)                                                             \
-                 : fwd_dispatch<T, W, false>(H / 256, (const T*)x, (const W*)gamma, (const W*)beta, (T*)y, mean,      \
-                                             rstd, rows, eps, s);                                                     \
-    }                                                                                                                 \
-    if (!done) {                                                                                                      \
-      const int wpb = 8;                                                                                              \
-      const int grid = (rows + wpb - 1) / wpb;                                                                        \
-      if (rms)                                                                                                        \
-        lb::norm_fwd_generic<T, W, true><<<grid, wpb * 32, 0, s>>>((const T*)x, (const W*)gamma, (const W*)beta,      \
-                                                                   (T*)y, mean, rstd, rows, H, eps);                  \
-      else                                                                                                            \
-        lb::norm_fwd_generic<T, W, false><<<grid, wpb * 32, 0, s>>>((const T*)x, (const W*)gamma, (const W*)beta,     \
-                                                                    (T*)y, mean, rstd, rows, H, eps);                 \
-    }                                                                                                                 \
+  if (dtype == 0 && wdtype == 0) {
+    norm_fwd_bf16<__nv_bfloat16>(x, gamma, beta, y, mean, rstd, rows, H, eps, rms, s);
+  } else if (dtype == 0 && wdtype == 1) {
+    norm_fwd_bf16<float>(x, gamma, beta, y, mean, rstd, rows, H, eps, rms, s);
+  } else if (dtype == 1 && wdtype == 1) {
+    const float *xf = (const float*)x, *gf = (const float*)gamma, *bf = (const float*)beta;
+    bool done = false;
+    if (H % 256 == 0)
+      done = rms ? fwd_dispatch_f32<true>(H / 256, xf, gf, bf, (float*)y, mean, rstd, rows, eps, s)
+                 : fwd_dispatch_f32<false>(H / 256, xf, gf, bf, (float*)y, mean, rstd, rows, eps, s);
+    if (!done) {
+      const int wpb = 8, grid = (rows + wpb - 1) / wpb;
+      if (rms) lb::norm_fwd_generic<float, float, true><<<grid, wpb * 32, 0, s>>>(xf, gf, bf, (float*)y, mean, rstd, rows, H, eps);
+      else lb::norm_fwd_generic<float, float, false><<<grid, wpb * 32, 0, s>>>(xf, gf, bf, (float*)y, mean, rstd, rows, H, eps);
+    }
+  } else {
+    return -1;
   }
-  if (dtype == 0 && wdtype == 0) LB_GO(__nv_bfloat16, __nv_bfloat16)
-  else if (dtype == 0 && wdtype == 1) LB_GO(__nv_bfloat16, float)
-  else if (dtype == 1 && wdtype == 1) LB_GO(float, float)
-  else return -1;
-#undef LB_GO
   return (int)cudaGetLastError();
 }
 
 // workspace: float[2 * grid_cap * H] where grid_cap = lb_norm_bwd_workspace_rows(); dgamma/dbeta fp32 [H]
-extern "C" int lb_norm_bwd_workspace_rows(int rows) {
-  const int a = norm_grid(rows), b = norm_bwd_bf16_grid(rows);
-  return a > b ? a : b;
+extern "C" int lb_norm_bwd_workspace_rows(int rows, int H) {
+  const int a = norm_grid(rows), b = norm_bwd_bf16_grid(rows), c = norm_bwd_wide_grid(rows, H);
+  return a > b ? (a > c ? a : c) : (b > c ? b : c);
 }
-// the fused "+ residual gradient" is implemented by the register-cached kernel only (H = 256 * {1..6, 8, 10, 12, 16})
-extern "C" int lb_norm_bwd_supports_gadd(int H) {
+// the fused "+ residual gradient" is implemented by the register-cached kernels only: bf16 rows of whole aligned vectors, fp32
+// rows of H = 256 * {1..6, 8, 10, 12, 16}
+extern "C" int lb_norm_bwd_supports_gadd(int H, int dtype, const void* gy, const void* x, const void* gamma, const void* gadd) {
+  if (dtype == 0) return norm_vec_bf16(H, dtype) && aligned16(gy) && aligned16(x) && aligned16(gamma) && aligned16(gadd);
   if (H % 256 != 0) return 0;
   const int v = H / 256;
   return (v >= 1 && v <= 6) || v == 8 || v == 10 || v == 12 || v == 16;
@@ -494,48 +738,41 @@ extern "C" int lb_norm_bwd(const void* gy, const void* x, const void* gamma, con
                            void* gx, float* dgamma, float* dbeta, float* workspace, int rows, int H, int rms, int dtype,
                            int wdtype, int accumulate, const void* gadd, cudaStream_t s) {
   if (rows == 0) return 0;
-  const bool fast = (H % 256 == 0) && (H / 256 <= 16);
-  if (gadd != nullptr && !lb_norm_bwd_supports_gadd(H)) return -3;  // caller adds the residual gradient itself
-  const int grid = norm_bwd_uses_bf16_kernel(H, dtype) ? norm_bwd_bf16_grid(rows) : norm_grid(rows);
-  bool done = false;
-  float* pdg = workspace;
-  float* pdb = dbeta != nullptr ? workspace + static_cast<size_t>(grid) * H : nullptr;
-  // accumulate mode + bandwidth-oriented bf16 kernel: the blocks add their column partials straight into dgamma / dbeta
-  const bool direct = accumulate && norm_bwd_uses_bf16_kernel(H, dtype);
-  float* direct_dg = direct ? dgamma : nullptr;
-  float* direct_db = (direct && dbeta != nullptr) ? dbeta : nullptr;
-  if (direct && dbeta == nullptr) pdb = nullptr;
-#define LB_GO(T, W)                                                                                                  \
-  {                                                                                                                  \
-    if (fast) {                                                                                                      \
-      done = rms ? bwd_dispatch<T, W, true>(H / 256, (const T*)gy, (const T*)x, (const W*)gamma, mean, rstd, (T*)gx, \
-                                            pdg, pdb, rows, grid, s, (const T*)gadd, direct_dg, direct_db)           \
-                 : bwd_dispatch<T, W, false>(H / 256, (const T*)gy, (const T*)x, (const W*)gamma, mean, rstd,        \
-                                             (T*)gx, pdg, pdb, rows, grid, s, (const T*)gadd, direct_dg, direct_db); \
-      if (done && direct_dg == nullptr) {                                                                            \
-        lb::colreduce_kernel<<<dim3((H + 31) / 32, dbeta != nullptr ? 2 : 1), 256, 0, s>>>(pdg, dgamma, pdb, dbeta, grid, \
-                                                                                           H, accumulate);           \
-      }                                                                                                              \
-    }                                                                                                                \
-    if (!done) {                                                                                                     \
-      if (!accumulate) {                                                                                             \
-        cudaMemsetAsync(dgamma, 0, sizeof(float) * H, s);                                                            \
-        if (dbeta != nullptr) cudaMemsetAsync(dbeta, 0, sizeof(float) * H, s);                                       \
-      }                                                                                                              \
-      const int wpb = 8;                                                                                             \
-      const int g2 = (rows + wpb - 1) / wpb;                                                                         \
-      if (rms)                                                                                                       \
-        lb::norm_bwd_generic<T, W, true><<<g2, wpb * 32, 0, s>>>((const T*)gy, (const T*)x, (const W*)gamma, mean,   \
-                                                                 rstd, (T*)gx, dgamma, dbeta, rows, H);              \
-      else                                                                                                           \
-        lb::norm_bwd_generic<T, W, false><<<g2, wpb * 32, 0, s>>>((const T*)gy, (const T*)x, (const W*)gamma, mean,  \
-                                                                  rstd, (T*)gx, dgamma, dbeta, rows, H);             \
-    }                                                                                                                \
-  }
-  if (dtype == 0 && wdtype == 0) LB_GO(__nv_bfloat16, __nv_bfloat16)
-  else if (dtype == 0 && wdtype == 1) LB_GO(__nv_bfloat16, float)
-  else if (dtype == 1 && wdtype == 1) LB_GO(float, float)
-  else return -1;
+  if (gadd != nullptr && !lb_norm_bwd_supports_gadd(H, dtype, gy, x, gamma, gadd)) return -3;  // caller adds the residual gradient itself
+  using B = __nv_bfloat16;
+  if (dtype == 0 && (wdtype == 0 || wdtype == 1)) {
+    if (!norm_vec_bf16(H, dtype) || !aligned16(gy) || !aligned16(x) || !aligned16(gamma) || !aligned16(gx)) {
+      if (wdtype == 0) norm_bwd_any<B, B>(gy, x, gamma, mean, rstd, gx, dgamma, dbeta, rows, H, rms, accumulate, s);
+      else norm_bwd_any<B, float>(gy, x, gamma, mean, rstd, gx, dgamma, dbeta, rows, H, rms, accumulate, s);
+      return (int)cudaGetLastError();
+    }
+    const int grid = H <= NORM_WARP_MAX_H ? norm_bwd_bf16_grid(rows) : norm_bwd_wide_grid(rows, H);
+    float* pdg = workspace;
+    float* pdb = dbeta != nullptr ? workspace + static_cast<size_t>(grid) * H : nullptr;
+    // accumulate mode: the blocks add their column sums straight into dgamma / dbeta (vector reductions in the wide kernel)
+    const bool direct = accumulate && (H <= NORM_WARP_MAX_H || (aligned16(dgamma) && aligned16(dbeta)));
+    float* adg = direct ? dgamma : nullptr;
+    float* adb = direct ? dbeta : nullptr;
+#define LB_GO(W, R) bwd_dispatch_bf16<W, R>(H, (const B*)gy, (const B*)x, (const W*)gamma, mean, rstd, (B*)gx, pdg, pdb, rows, grid, s, (const B*)gadd, adg, adb)
+    if (wdtype == 0) { if (rms) LB_GO(B, true); else LB_GO(B, false); }
+    else { if (rms) LB_GO(float, true); else LB_GO(float, false); }
 #undef LB_GO
+    if (!direct)
+      lb::colreduce_kernel<<<dim3((H + 31) / 32, dbeta != nullptr ? 2 : 1), 256, 0, s>>>(pdg, dgamma, pdb, dbeta, grid, H, accumulate);
+  } else if (dtype == 1 && wdtype == 1) {
+    const int grid = norm_grid(rows);
+    float* pdg = workspace;
+    float* pdb = dbeta != nullptr ? workspace + static_cast<size_t>(grid) * H : nullptr;
+    bool done = false;
+    if (H % 256 == 0 && H / 256 <= 16)
+      done = rms ? bwd_dispatch_f32<true>(H / 256, (const float*)gy, (const float*)x, (const float*)gamma, mean, rstd, (float*)gx, pdg, pdb, rows, grid, s, (const float*)gadd)
+                 : bwd_dispatch_f32<false>(H / 256, (const float*)gy, (const float*)x, (const float*)gamma, mean, rstd, (float*)gx, pdg, pdb, rows, grid, s, (const float*)gadd);
+    if (done)
+      lb::colreduce_kernel<<<dim3((H + 31) / 32, dbeta != nullptr ? 2 : 1), 256, 0, s>>>(pdg, dgamma, pdb, dbeta, grid, H, accumulate);
+    else
+      norm_bwd_any<float, float>(gy, x, gamma, mean, rstd, gx, dgamma, dbeta, rows, H, rms, accumulate, s);
+  } else {
+    return -1;
+  }
   return (int)cudaGetLastError();
 }

@@ -39,3 +39,30 @@ def test_attention_rows_do_not_depend_on_timing(dim, causal):
     assert float(row.max()) < 4 * 2.0 ** -8
     for _ in range(5):
         assert torch.equal(OF.attention_qkvpacked(qkv, causal=causal, scale=dim ** -0.5), first)
+
+
+@pytest.mark.parametrize("rms", [False, True])
+@pytest.mark.parametrize("rows,h", [(1, 8), (3, 192), (257, 384), (2048, 768), (130, 1000), (515, 1024), (4, 1032), (300, 1280), (37, 2048),
+                                    (450, 4096), (33, 6152), (5, 8192), (3, 8200), (9, 99)])
+def test_norm_kernels_at_their_edges(rows, h, rms):
+    """Rows of a warp (up to 1024 columns), of a block (up to 8192) and of the generic kernel, forward, backward, with the gradient of a
+    residual path, into new tensors and into fp32 gradients."""
+    x, gy, skip = _rand((rows, h), 1), _rand((rows, h), 2), _rand((rows, h), 3)
+    w, b = _rand((h,), 4), None if rms else _rand((h,), 5)
+    x64, w64 = x.double().requires_grad_(True), w.double().requires_grad_(True)
+    b64 = None if rms else b.double().requires_grad_(True)
+    d = x64 if rms else x64 - x64.mean(-1, keepdim=True)
+    y64 = d * torch.rsqrt(d.square().mean(-1, keepdim=True) + 1e-5) * w64
+    y64 = y64 if rms else y64 + b64
+    y64.backward(gy.double())
+    ext = OF.load_ext()
+    y, mean, rstd = ext.norm_fwd(x, w, b, 1e-5, rms)
+    close = lambda got, want, tol: float((got.double() - want).norm() / want.norm().clamp_min(1e-30)) < tol
+    assert close(y, y64, 2.0 ** -8)                              # one rounding to bf16
+    for acc in (False, True):
+        gw = torch.ones(h, device="cuda") if acc else None
+        gb = torch.ones(h, device="cuda") if acc and not rms else None
+        gx, dw, db = ext.norm_bwd(gy, x, w, mean, rstd, rms, not rms, gw, gb, skip)
+        dw, db = (gw - 1, None if rms else gb - 1) if acc else (dw, db)
+        assert close(gx, x64.grad + skip.double(), 2.0 ** -7)    # bf16, and once more where the residual gradient is added outside
+        assert close(dw, w64.grad, 1e-5) and (rms or close(db, b64.grad, 1e-5))
