@@ -66,3 +66,20 @@ def test_norm_kernels_at_their_edges(rows, h, rms):
         dw, db = (gw - 1, None if rms else gb - 1) if acc else (dw, db)
         assert close(gx, x64.grad + skip.double(), 2.0 ** -7)    # bf16, and once more where the residual gradient is added outside
         assert close(dw, w64.grad, 1e-5) and (rms or close(db, b64.grad, 1e-5))
+
+
+@pytest.mark.parametrize("b,s,a,d,off", [(1, 1, 1, 16, 0), (2, 37, 3, 128, 5), (1, 2100, 4, 64, 0), (3, 9, 5, 48, 1), (2, 7, 2, 24, 3), (1, 5, 32, 256, 0)])
+def test_rotary_on_the_packed_projection(b, s, a, d, off):
+    qkv, g = _rand((b, s, a, 3 * d), 1), _rand((b, s, a, 3 * d), 2)
+    ang = torch.outer(torch.arange(s + off, device="cuda").float(), 1.0 / 10000 ** (torch.arange(0, d, 2, device="cuda") / d))
+    cos, sin = torch.cat([ang, ang], -1).cos().contiguous(), torch.cat([ang, ang], -1).sin().contiguous()
+    x = qkv.clone().requires_grad_(True)
+    y = OF.apply_rotary_qkv(x, cos, sin, off)
+    x64 = qkv.double().requires_grad_(True)
+    c, n = cos[off:off + s, None].double(), sin[off:off + s, None].double()
+    q, k, v = x64.split(d, -1)
+    y64 = torch.cat([q * c + OF.rotate_half(q) * n, k * c + OF.rotate_half(k) * n, v], -1)
+    y.backward(g.clone())
+    y64.backward(g.double())
+    assert float((y.double() - y64).norm() / y64.norm()) < 2.0 ** -8
+    assert float((x.grad.double() - x64.grad).norm() / x64.grad.norm()) < 2.0 ** -8
