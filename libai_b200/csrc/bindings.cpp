@@ -5,6 +5,7 @@
 #include <ATen/cuda/CUDAGeneratorImpl.h>
 #include <cstring>
 #include <mutex>
+#include <mutex>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/library.h>
 #include <torch/torch.h>
@@ -91,6 +92,15 @@ int lb_attn_bwd(const void* dout, const void* q, const void* k, const void* v, c
                 const long* q_strides, const long* k_strides, const long* v_strides, const long* do_strides, int causal,
                 float scale, const int* kv_lens, const void* bias, const long* bias_strides, const float* alibi_slopes,
                 float* dbias, float p_drop, const long long* rng_state, cudaStream_t s);
+int lb_attn_mask_pack(const void* mask, int elem, unsigned long long and_mask, int Bm, int Am, int Sq, int Sk, const long* strides, int causal,
+                      int off, uint32_t* words, float* fill, cudaStream_t s);
+int lb_attn_split_fwd(const void* q, const void* k, const void* v, void* o, void* o_lo, float* lse, int B, int A, int Sq, int Sk, int d,
+                      const long* qs, const long* ks, const long* vs, int causal, float scale, const uint32_t* mask, const float* fill, long mask_b,
+                      long mask_a, int* err, cudaStream_t s);
+int lb_attn_split_bwd(const void* dout, const void* q, const void* k, const void* v, const void* o, const void* o_lo, const float* lse, void* dq,
+                      void* dk, void* dv, float* delta, float* dq_acc, int B, int A, int Sq, int Sk, int d, const long* qs, const long* ks,
+                      const long* vs, const long* dos, const long* dqs, const long* dks, const long* dvs, int causal, float scale,
+                      const uint32_t* mask, const float* fill, long mask_b, long mask_a, int* err, cudaStream_t s);
 int lb_bias_dropout_residual(const void* x, const void* bias, const void* res, void* y, long rows, int N, float p,
                              const LbRngArgs* rng, const long long* rng_in, long long* rng_out, cudaStream_t s);
 }
@@ -178,11 +188,20 @@ void gemm_grouped(const Tensor& a, const Tensor& w, const std::vector<int64_t>& 
 
 // a mapped host word that a kernel sets when one of its bounded waits ran out; `what` has its own, checked before every launch
 struct WaitWord {
+  std::mutex lock;
   int* host = nullptr;
   int* device(const char* what) {
+    std::lock_guard<std::mutex> guard(lock);
     if (host == nullptr) {
-      TORCH_CHECK(cudaHostAlloc(reinterpret_cast<void**>(&host), sizeof(int), cudaHostAllocMapped) == cudaSuccess, what, ": mapped host word");
-      *host = 0;
+      // (the first call may come while this thread captures a graph: the allocation is no part of it)
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      int* word = nullptr;
+      const cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&word), sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable);
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      TORCH_CHECK(e == cudaSuccess, what, ": mapped host word");
+      *word = 0;
+      host = word;
     }
     TORCH_CHECK(*static_cast<volatile int*>(host) == 0, what, ": a wait ran out in an earlier launch; its result is invalid");
     int* dev = nullptr;
@@ -789,6 +808,110 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> attn_bwd(const Tensor& dout, const Te
   return std::make_tuple(dq, dk, dv, dqkv);
 }
 
+// ---- attention with 32-bit probabilities (csrc/attention_split_sm100.cu) ---------------------------------------
+// mask [B|1, A|1, Sq, Sk] (any strides, expanded) of any integer, boolean or floating type -> (words int32 [Bm, Am, Sq, 4 ceil(Sk/128)],
+// fill fp32 [Bm, Am, Sq])
+std::tuple<Tensor, Tensor> attn_mask_pack(const Tensor& mask, bool causal) {
+  TORCH_CHECK(mask.is_cuda() && mask.dim() == 4, "attn_mask_pack: [B|1, A|1, Sq, Sk]");
+  c10::cuda::CUDAGuard guard(mask.device());
+  const int64_t elem = mask.element_size();
+  TORCH_CHECK(!mask.is_complex() && (elem == 1 || elem == 2 || elem == 4 || elem == 8), "attn_mask_pack: mask type");
+  unsigned long long keep = ~0ull;
+  if (mask.is_floating_point()) keep = (1ull << (8 * elem - 1)) - 1;       // a negative zero is zero
+  const int Bm = (int)mask.size(0), Am = (int)mask.size(1), Sq = (int)mask.size(2), Sk = (int)mask.size(3);
+  long st[4] = {mask.stride(0), mask.stride(1), mask.stride(2), mask.stride(3)};
+  Tensor words = at::empty({Bm, Am, Sq, (Sk + 127) / 128 * 4}, mask.options().dtype(at::kInt));
+  Tensor fill = at::empty({Bm, Am, Sq}, mask.options().dtype(at::kFloat));
+  check(lb_attn_mask_pack(mask.data_ptr(), (int)elem, keep, Bm, Am, Sq, Sk, st, causal ? 1 : 0, Sk - Sq,
+                          reinterpret_cast<uint32_t*>(words.data_ptr<int>()), fill.data_ptr<float>(), cur_stream()),
+        "attn_mask_pack");
+  return std::make_tuple(words, fill);
+}
+
+struct SplitMask {
+  const uint32_t* words = nullptr;
+  const float* fill = nullptr;
+  long b = 0, a = 0;
+};
+SplitMask split_mask(const c10::optional<Tensor>& words, const c10::optional<Tensor>& fill, int B, int A, int Sq, int Sk) {
+  SplitMask m;
+  if (!(words.has_value() && words->defined())) return m;
+  TORCH_CHECK(fill.has_value() && fill->defined() && words->is_cuda() && words->scalar_type() == at::kInt && words->is_contiguous() &&
+                  fill->scalar_type() == at::kFloat && fill->is_contiguous() && words->dim() == 4 && words->size(2) == Sq &&
+                  words->size(3) == (Sk + 127) / 128 * 4 && (words->size(0) == 1 || words->size(0) == B) &&
+                  (words->size(1) == 1 || words->size(1) == A) && fill->numel() == words->size(0) * words->size(1) * Sq,
+              "split attention: a mask from attn_mask_pack for these sizes");
+  m.words = reinterpret_cast<const uint32_t*>(words->data_ptr<int>());
+  m.fill = fill->data_ptr<float>();
+  m.a = words->size(1) == 1 ? 0 : Sq;
+  m.b = words->size(0) == 1 ? 0 : words->size(1) * Sq;
+  return m;
+}
+void split_strides(const Tensor& t, long (&st)[3]) {
+  TORCH_CHECK(t.is_cuda() && t.dim() == 4 && t.scalar_type() == at::kBFloat16 && t.stride(3) == 1, "split attention: bf16 [B, A, S, d] views with contiguous d");
+  // the stride of a dimension of one element is free: give the tensor map a legal one
+  int64_t full = t.size(3);
+  for (int i = 2; i >= 0; --i) {
+    st[i] = t.size(i) == 1 ? (long)((full + 7) / 8 * 8) : (long)t.stride(i);
+    full = std::max<int64_t>(full, st[i] * t.size(i));
+  }
+}
+WaitWord& split_word() {
+  static WaitWord word;
+  return word;
+}
+
+// (o [B, A, Sq, d] as a view of [B, Sq, A, d], o_lo (what its rounding left over, only with `train`), lse)
+std::tuple<Tensor, Tensor, Tensor> attn_split_fwd(const Tensor& q, const Tensor& k, const Tensor& v, bool causal, double scale,
+                                                  const c10::optional<Tensor>& words, const c10::optional<Tensor>& fill, bool train) {
+  c10::cuda::CUDAGuard guard(q.device());
+  long qs[3], ks[3], vs[3];
+  split_strides(q, qs);
+  split_strides(k, ks);
+  split_strides(v, vs);
+  const int B = (int)q.size(0), A = (int)q.size(1), Sq = (int)q.size(2), Sk = (int)k.size(2), d = (int)q.size(3);
+  TORCH_CHECK(k.sizes() == v.sizes() && k.size(0) == B && k.size(1) == A && k.size(3) == d, "split attention: shapes");
+  const SplitMask m = split_mask(words, fill, B, A, Sq, Sk);
+  Tensor o = at::empty({B, Sq, A, d}, q.options());
+  Tensor lo = train ? at::empty({B, Sq, A, d}, q.options()) : at::empty({0}, q.options());
+  Tensor lse = at::empty({B, A, Sq}, q.options().dtype(at::kFloat));
+  check(lb_attn_split_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), train ? lo.data_ptr() : nullptr, lse.data_ptr<float>(), B, A, Sq,
+                          Sk, d, qs, ks, vs, causal ? 1 : 0, (float)scale, m.words, m.fill, m.b, m.a, split_word().device("attn_split"), cur_stream()),
+        "attn_split_fwd");
+  return std::make_tuple(o.permute({0, 2, 1, 3}), lo, lse);
+}
+
+// gradients into the given [B, A, S, d] views (slices of packed projections' gradients)
+void attn_split_bwd(const Tensor& dout, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& o_lo, const Tensor& lse,
+                    Tensor dq, Tensor dk, Tensor dv, bool causal, double scale, const c10::optional<Tensor>& words,
+                    const c10::optional<Tensor>& fill) {
+  c10::cuda::CUDAGuard guard(q.device());
+  const int B = (int)q.size(0), A = (int)q.size(1), Sq = (int)q.size(2), Sk = (int)k.size(2), d = (int)q.size(3);
+  Tensor g = dout;
+  if (g.stride(3) != 1 || g.stride(0) % 8 || g.stride(1) % 8 || g.stride(2) % 8 || (reinterpret_cast<uintptr_t>(g.data_ptr()) & 15) ||
+      g.stride(0) <= 0 || g.stride(1) <= 0 || g.stride(2) <= 0)
+    g = g.contiguous();
+  if (reinterpret_cast<uintptr_t>(g.data_ptr()) & 15) g = g.clone();
+  TORCH_CHECK(g.sizes() == q.sizes() && dq.sizes() == q.sizes() && dk.sizes() == k.sizes() && dv.sizes() == k.sizes() && k.sizes() == v.sizes() &&
+                  o.is_contiguous() && o_lo.is_contiguous() && o.numel() == q.numel() && o_lo.numel() == q.numel(),
+              "split attention: shapes");
+  long qs[3], ks[3], vs[3], gs[3], dqs[3], dks[3], dvs[3];
+  split_strides(q, qs);
+  split_strides(k, ks);
+  split_strides(v, vs);
+  split_strides(g, gs);
+  split_strides(dq, dqs);
+  split_strides(dk, dks);
+  split_strides(dv, dvs);
+  const SplitMask m = split_mask(words, fill, B, A, Sq, Sk);
+  auto f32 = q.options().dtype(at::kFloat);
+  Tensor delta = at::empty({B, A, Sq}, f32), acc = at::empty({B, A, Sq, d}, f32);      // cleared by the delta kernel
+  check(lb_attn_split_bwd(g.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), o_lo.data_ptr(), lse.data_ptr<float>(), dq.data_ptr(),
+                          dk.data_ptr(), dv.data_ptr(), delta.data_ptr<float>(), acc.data_ptr<float>(), B, A, Sq, Sk, d, qs, ks, vs, gs, dqs, dks,
+                          dvs, causal ? 1 : 0, (float)scale, m.words, m.fill, m.b, m.a, split_word().device("attn_split"), cur_stream()),
+        "attn_split_bwd");
+}
+
 // ---- fused collectives ---------------------------------------------------------------------------------------
 std::vector<long> to_longs(at::IntArrayRef v) { return std::vector<long>(v.begin(), v.end()); }
 
@@ -938,6 +1061,9 @@ TORCH_LIBRARY(libai_b200, m) {
   m.def("ce_bwd(Tensor(a!) logits, Tensor labels, Tensor lse, Tensor gloss, int vocab_start) -> Tensor(a!)", &ce_bwd);
   m.def("fused_adamw(Tensor(a!) master, Tensor grad, Tensor(b!) m, Tensor(c!) v, Tensor? lp_out, Tensor scale, float lr, float b1, float b2, float eps, float wd, float bc1, float bc2, bool decoupled) -> ()", &fused_adamw);
   m.def("sqnorm(Tensor x) -> Tensor", &sqnorm);
+  m.def("attn_mask_pack(Tensor mask, bool causal) -> (Tensor, Tensor)", &attn_mask_pack);
+  m.def("attn_split_fwd(Tensor q, Tensor k, Tensor v, bool causal, float scale, Tensor? words, Tensor? fill, bool train) -> (Tensor, Tensor, Tensor)", &attn_split_fwd);
+  m.def("attn_split_bwd(Tensor dout, Tensor q, Tensor k, Tensor v, Tensor o, Tensor o_lo, Tensor lse, Tensor(a!) dq, Tensor(b!) dk, Tensor(c!) dv, bool causal, float scale, Tensor? words, Tensor? fill) -> ()", &attn_split_bwd);
   m.def("attn_fwd(Tensor q, Tensor k, Tensor v, bool causal, float scale, Tensor? kv_lens, Tensor? bias=None, Tensor? alibi_slopes=None, float p_drop=0.0, int salt=0) -> (Tensor, Tensor, Tensor)", &attn_fwd);
   m.def("attn_bwd(Tensor dout, Tensor q, Tensor k, Tensor v, Tensor o, Tensor lse, bool causal, float scale, Tensor? kv_lens, Tensor? bias=None, Tensor? alibi_slopes=None, Tensor(a!)? dbias=None, float p_drop=0.0, Tensor? rng_state=None) -> (Tensor, Tensor, Tensor, Tensor)", &attn_bwd);
   m.def("bias_dropout_residual(Tensor x, Tensor? bias, Tensor? res, float p, int salt, Tensor? rng_state=None) -> (Tensor, Tensor)", &bias_dropout_residual);

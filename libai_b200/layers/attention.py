@@ -8,9 +8,9 @@ multiplying it back (``apply_query_key_layer_scaling``, :87-91, numerically the 
 exact arithmetic) — masked positions filled with −10000 (:223-245), row-parallel output
 projection, bias+dropout fused with the residual add.
 
-The softmax(QKᵀ)V core runs in the sm_100a flash-attention kernel (no ``[b,a,s,s]`` tensor, no
-materialised masks) whenever the mask is purely causal or absent; padding-mask / bias / dropout
-variants fall back to the reference math in :func:`libai_b200.ops.functional.attention_ref`.
+The softmax(QKᵀ)V core runs in the sm_100a flash-attention kernels (no ``[b,a,s,s]`` tensor): causal, full and
+right-padded self-attention with head dims 64 / 128, and — without dropout — any head dim up to 64 that is a multiple
+of 8, dense masks and cross attention.  The rest falls back to :func:`libai_b200.ops.functional.attention_ref`.
 """
 from __future__ import annotations
 
@@ -145,43 +145,44 @@ class MultiheadAttention(nn.Module):
         else:
             bsz, tgt_len = hidden_states.shape[:2]
 
+        packed = past_key_value is None and not use_cache
         if self.is_cross_attention:
-            query = self.query(hidden_states).view(bsz, -1, a, d).permute(0, 2, 1, 3)
+            query = self.query(hidden_states).view(bsz, -1, a, d)
             if past_key_value is not None:
                 key, value = past_key_value
             elif encoder_states is not None:
-                kv = self.key_value(encoder_states).view(bsz, -1, a, 2 * d).permute(0, 2, 1, 3)
+                kv = self.key_value(encoder_states).view(bsz, -1, a, 2 * d)
+                if packed:
+                    dense = attention_mask.dense() if isinstance(attention_mask, KeyPaddingMask) else attention_mask
+                    context = OF.attention_packed("q_kv", (query, kv), causal=False, scale=self.softmax_scale, mask=dense,
+                                                  dropout_p=self.attention_dropout_prob, training=self.training)
+                    if context is not None:
+                        return self._project(context.reshape(bsz, -1, a * d), hidden_states, residual, sp)
+                kv = kv.permute(0, 2, 1, 3)
                 key, value = kv[..., :d], kv[..., d:]
             else:
                 raise ValueError("past_key_value and encoder_states cannot be None at the same time.")
+            query = query.permute(0, 2, 1, 3)
         else:
             qkv_packed = self.query_key_value(hidden_states).view(bsz, -1, a, 3 * d)
             kv_lens = None
             if isinstance(attention_mask, KeyPaddingMask) and attention_mask.is_prefix():
                 kv_lens = attention_mask.lengths
-            if (
-                past_key_value is None and not use_cache
-                and (attention_mask is None or kv_lens is not None)
-                and OF.attention_qkvpacked_supported(qkv_packed, None, self.attention_dropout_prob, self.training)
-            ):
-                # fast path: flash attention directly on the packed projection
-                context = OF.attention_qkvpacked(
-                    qkv_packed, causal=self.attn_mask_type == AttnMaskType.causal, scale=self.softmax_scale,
-                    kv_lens=kv_lens, dropout_p=self.attention_dropout_prob, training=self.training,
-                ).reshape(bsz, -1, a * d)
-                if sp and hidden_states.dim() == 2:
-                    context = context.reshape(-1, a * d)
-                topo = dutil.get_dist_util()
-                if (residual is not None and topo.tensor_parallel_size == 1 and context.dtype == torch.bfloat16
-                        and (self.output_dropout_prob == 0.0 or not self.training)):
-                    # bias + residual in the epilogue of the output projection
-                    return OF.linear_bias_residual(context, self.dense.weight, self.dense.bias, residual)
-                if residual is not None and (self.output_dropout_prob == 0.0 or not self.training):
-                    fused = self.dense.fused_bias_residual(context, residual)   # GEMM→RS + bias + residual, one kernel
-                    if fused is not None:
-                        return fused
-                output, bias = self.dense(context)
-                return OF.bias_dropout_add(output, bias, residual, self.output_dropout_prob, self.training)
+            if packed:
+                # flash attention directly on the packed projection
+                if ((attention_mask is None or kv_lens is not None)
+                        and OF.attention_qkvpacked_supported(qkv_packed, None, self.attention_dropout_prob, self.training)):
+                    context = OF.attention_qkvpacked(
+                        qkv_packed, causal=self.attn_mask_type == AttnMaskType.causal, scale=self.softmax_scale,
+                        kv_lens=kv_lens, dropout_p=self.attention_dropout_prob, training=self.training,
+                    )
+                else:
+                    dense = attention_mask.dense() if isinstance(attention_mask, KeyPaddingMask) else attention_mask
+                    context = OF.attention_packed("qkv", (qkv_packed,), causal=self.attn_mask_type == AttnMaskType.causal and dense is None,
+                                                  scale=self.softmax_scale, mask=dense, dropout_p=self.attention_dropout_prob,
+                                                  training=self.training)
+                if context is not None:
+                    return self._project(context.reshape(bsz, -1, a * d), hidden_states, residual, sp)
             qkv = qkv_packed.permute(0, 2, 1, 3)
             query, key, value = qkv[..., :d], qkv[..., d : 2 * d], qkv[..., 2 * d :]
             if past_key_value is not None:
@@ -206,14 +207,23 @@ class MultiheadAttention(nn.Module):
             dropout_p=self.attention_dropout_prob,
             training=self.training,
         )  # [b, a, s, d]
-        context = context.transpose(1, 2).reshape(bsz, -1, a * d)
-        if sp and hidden_states.dim() == 2:
-            context = context.reshape(-1, a * d)
-        output, bias = self.dense(context)
-        output = OF.bias_dropout_add(output, bias, residual, self.output_dropout_prob, self.training)
+        output = self._project(context.transpose(1, 2).reshape(bsz, -1, a * d), hidden_states, residual, sp)
         if use_cache:
             return output, past_key_value
         return output
+
+    def _project(self, context, hidden_states, residual, sp):
+        """Output projection with bias, dropout and residual; without dropout bias and residual ride in the GEMM's epilogue."""
+        if sp and hidden_states.dim() == 2:
+            context = context.reshape(-1, context.shape[-1])
+        if residual is not None and (self.output_dropout_prob == 0.0 or not self.training):
+            if dutil.get_dist_util().tensor_parallel_size == 1 and context.dtype == torch.bfloat16:
+                return OF.linear_bias_residual(context, self.dense.weight, self.dense.bias, residual)
+            fused = self.dense.fused_bias_residual(context, residual)   # GEMM→RS + bias + residual, one kernel
+            if fused is not None:
+                return fused
+        output, bias = self.dense(context)
+        return OF.bias_dropout_add(output, bias, residual, self.output_dropout_prob, self.training)
 
     def extra_repr(self) -> str:
         return "hidden_size={}, num_heads={}, is_cross_attention={}".format(

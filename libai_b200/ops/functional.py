@@ -614,6 +614,92 @@ class _FlashAttnPackedFn(torch.autograd.Function):
         return dqkv.view(qkv.shape), None, None, None, None, None
 
 
+# ---- attention with 32-bit probabilities (csrc/attention_split_sm100.cu) ----------------------------------------------
+def _plain_call() -> bool:
+    """False where an operator is transformed (vmap, jvp, …), differentiated forward or traced: those see PyTorch operators."""
+    return not (torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0 or torch.jit.is_tracing())
+
+
+def _rows_of_vectors(t) -> bool:
+    """A view whose rows TMA can read: contiguous last dimension, every other stride and the base on 16 bytes."""
+    return t.data_ptr() % 16 == 0 and t.stride(-1) == 1 and all(n == 1 or (st > 0 and st % 8 == 0) for n, st in zip(t.shape[:-1], t.stride()))
+
+
+def _split_views(layout: str, ts):
+    """``[b, a, s, d]`` views of q, k, v; ``qkv``: packed ``[b, s, a, 3d]``, ``q_kv``: ``[b, s, a, d]`` and ``[b, sk, a, 2d]``."""
+    if layout == "qkv":
+        return ts[0].permute(0, 2, 1, 3).chunk(3, -1)
+    if layout == "q_kv":
+        return (ts[0].permute(0, 2, 1, 3), *ts[1].permute(0, 2, 1, 3).chunk(2, -1))
+    return ts
+
+
+def _split_supported(q, k, v, scale, causal, mask) -> bool:
+    """Sizes and types of the kernels with 32-bit probabilities, from ``[b, a, s, d]`` views.  Other head dims stay with the flash
+    kernels (64 / 128 without a mask: bf16 probabilities, as ever) or with the unfused form."""
+    if not (use_native(q) and q.dtype == k.dtype == v.dtype == torch.bfloat16 and q.dim() == k.dim() == 4 and k.shape == v.shape
+            and q.shape[:2] == k.shape[:2] and q.shape[-1] == k.shape[-1] and q.shape[-1] % 8 == 0 and 8 <= q.shape[-1] <= 64
+            and min(q.shape) > 0 and k.shape[2] > 0 and max(q.shape[:2]) <= 65535 and scale > 0 and (not causal or k.shape[2] >= q.shape[2])):
+        return False
+    if mask is not None:
+        full = (q.shape[0], q.shape[1], q.shape[2], k.shape[2])
+        if mask.device != q.device or mask.is_complex() or mask.dim() > 4 or any(m not in (1, n) for m, n in zip(reversed(mask.shape), reversed(full))):
+            return False
+    return _plain_call()
+
+
+class _SplitAttnFn(torch.autograd.Function):
+    """Attention whose probabilities reach the tensor core as two bf16 parts (``layout``: see :func:`_split_views`)."""
+
+    @staticmethod
+    def forward(ctx, layout, causal, scale, mask, *ts):
+        ext = load_ext()
+        q, k, v = _split_views(layout, ts)
+        words = fill = None
+        if mask is not None:
+            m = mask[(None,) * (4 - mask.dim())]
+            words, fill = ext.attn_mask_pack(m.expand(m.shape[0], m.shape[1], q.shape[2], k.shape[2]), causal)
+            count_launch()
+        train = any(ctx.needs_input_grad[4:])
+        o, o_lo, lse = ext.attn_split_fwd(q, k, v, causal and mask is None, scale, words, fill, train)
+        count_launch()
+        out = o if layout == "q_k_v" else o.permute(0, 2, 1, 3)
+        if train:
+            ctx.save_for_backward(out, o_lo, lse, words, fill, *ts)
+            ctx.layout, ctx.causal, ctx.scale, ctx.mask = layout, causal, scale, mask
+        return out
+
+    @staticmethod
+    def backward(ctx, go):
+        o, o_lo, lse, words, fill, *ts = ctx.saved_tensors
+        q, k, v = _split_views(ctx.layout, ts)
+        if torch.is_grad_enabled():            # a graph of the gradients is wanted: differentiate the unfused form
+            out = attention_ref(q, k, v, causal=ctx.causal, scale=ctx.scale, mask=ctx.mask)
+            out = out if ctx.layout == "q_k_v" else out.permute(0, 2, 1, 3)
+            need = [t for t, n in zip(ts, ctx.needs_input_grad[4:]) if n]
+            grads = iter(torch.autograd.grad(out, need, go, create_graph=True))
+            return (None,) * 4 + tuple(next(grads) if n else None for n in ctx.needs_input_grad[4:])
+        if ctx.layout == "q_k_v":              # gradients backed by [b, s, a, d], as the projections around an attention read them
+            gs = [torch.empty(t.shape[0], t.shape[2], t.shape[1], t.shape[3], dtype=t.dtype, device=t.device).permute(0, 2, 1, 3) for t in ts]
+            o = o.permute(0, 2, 1, 3)
+        else:
+            gs = [torch.empty(t.shape, dtype=t.dtype, device=t.device) for t in ts]
+            go = go.permute(0, 2, 1, 3)
+        load_ext().attn_split_bwd(go, q, k, v, o, o_lo, lse, *_split_views(ctx.layout, gs), ctx.causal and words is None, ctx.scale, words, fill)
+        count_launch(3)
+        return (None,) * 4 + tuple(gs)
+
+
+def attention_packed(layout: str, ts, *, causal: bool, scale: float, mask=None, dropout_p: float = 0.0, training: bool = False):
+    """Attention straight from packed projections, ``qkv`` ``([b, s, a, 3d],)`` or ``q_kv`` ``([b, s, a, d], [b, sk, a, 2d])``, with an
+    optional dense 0/1 mask, → ``[b, s, a, d]``; ``None`` where the kernels do not apply (the caller slices and takes :func:`attention`)."""
+    if (dropout_p > 0.0 and training) or not all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in ts):
+        return None
+    if not _split_supported(*_split_views(layout, ts), scale, causal, mask):
+        return None
+    return _SplitAttnFn.apply(layout, causal, float(scale), mask, *ts)
+
+
 def attention_qkvpacked_supported(qkv, mask, dropout_p, training) -> bool:
     return (
         use_native(qkv)
@@ -637,8 +723,9 @@ def attention(q, k, v, *, causal: bool = False, scale: Optional[float] = None, m
               dropout_p: float = 0.0, training: bool = False, alibi_slopes=None, kv_lens=None):
     """Softmax attention on ``[b, a, s, d]``.  The native flash kernels handle causal / full / key-padding
     (``kv_lens``) masking, an additive score bias (dense ``[b|1, a|1, s, s]`` — T5 relative positions — or
-    ``alibi_slopes`` ``[a]``) and dropout on the probabilities; arbitrary dense 0/1 masks and cross attention with
-    different query / key lengths use the reference math."""
+    ``alibi_slopes`` ``[a]``) and dropout on the probabilities.  Dense 0/1 masks, query and key lengths of their own and the
+    head dims below 64 run in the kernels with 32-bit probabilities; what is left (dropout or bias beside those, head dims
+    above 64 beside those) uses the unfused form."""
     if scale is None:
         scale = 1.0 / math.sqrt(q.shape[-1])
     if (
@@ -653,6 +740,11 @@ def attention(q, k, v, *, causal: bool = False, scale: Optional[float] = None, m
         # strided [b, a, s, d] views of the packed QKV projection are consumed directly (TMA strides)
         return _FlashAttnFn.apply(q, k, v, causal, float(scale), bias, alibi_slopes,
                                   float(dropout_p) if training else 0.0, kv_lens)
+    if (bias is None and alibi_slopes is None and kv_lens is None and not (dropout_p > 0.0 and training)
+            and _split_supported(q, k, v, scale, causal, mask)):
+        ts = [t if _rows_of_vectors(t) else t.contiguous() for t in (q, k, v)]
+        if all(_rows_of_vectors(t) for t in ts):
+            return _SplitAttnFn.apply("q_k_v", causal, float(scale), mask, *ts)
     if alibi_slopes is not None:
         sq, sk = q.shape[-2], k.shape[-2]
         rel = torch.arange(sk, device=q.device)[None, :] - torch.arange(sk - sq, sk, device=q.device)[:, None]

@@ -83,3 +83,78 @@ def test_rotary_on_the_packed_projection(b, s, a, d, off):
     y64.backward(g.double())
     assert float((y.double() - y64).norm() / y64.norm()) < 2.0 ** -8
     assert float((x.grad.double() - x64.grad).norm() / x64.grad.norm()) < 2.0 ** -8
+
+
+def _split_mask(kind, b, a, sq, sk):
+    g = torch.Generator(device="cuda").manual_seed(11)
+    on = torch.rand(b, 1, sq, sk, device="cuda", generator=g) < 0.6
+    on[:, :, sq // 2] = False                                       # a query that sees no key: uniform over all of them
+    if kind == "bool":
+        return on
+    if kind == "keys_int64":
+        return on[:, :, :1].long() * 3
+    if kind == "float_2d":
+        return torch.where(on[0, 0], 0.5, -0.0)                     # a negative zero masks
+    if kind == "heads_strided":
+        heads = torch.rand(sk, a, sq, device="cuda", generator=g) < 0.5
+        return heads.to(torch.int8).permute(1, 2, 0)[None]
+    return None
+
+
+@pytest.mark.parametrize("mask", ["none", "causal", "bool", "keys_int64", "float_2d", "heads_strided"])
+@pytest.mark.parametrize("b,sq,sk,a,d", [(1, 1, 1, 1, 8), (2, 128, 136, 3, 64), (2, 129, 257, 2, 48), (1, 300, 300, 2, 24), (3, 17, 512, 2, 32),
+                                         (2, 200, 130, 1, 40), (1, 127, 385, 2, 56), (1, 1, 700, 5, 16)])
+def test_attention_with_32_bit_probabilities(b, sq, sk, a, d, mask):
+    """Head dims up to 64, lengths around the 128-wide tiles, masks of every type and broadcast; forward and backward are as close to
+    64-bit arithmetic as the unfused fp32 form that these calls took before."""
+    causal = mask == "causal"
+    if causal and sk < sq:
+        pytest.skip("more queries than keys under a causal mask: unfused form")
+    m = _split_mask(mask, b, a, sq, sk)
+    q, k, v, go = _rand((b, a, sq, d), 1), _rand((b, sk, a, d), 2).permute(0, 2, 1, 3), _rand((b, a, sk, d), 3), _rand((b, a, sq, d), 4)
+    keep = torch.ones(sq, sk, dtype=torch.bool, device="cuda").tril(sk - sq) if causal else None if m is None else m.bool()
+    got = []
+    for fn in (lambda *t: OF.attention(*t, causal=causal, scale=0.3, mask=m),
+               lambda *t: OF.attention_ref(*t, causal=causal, scale=0.3, mask=m),
+               lambda *t: _attend64(*t, 0.3, keep)):
+        ts = [t.detach().clone().requires_grad_(True) for t in (q, k, v)]
+        before = OF.ops.launch_count()
+        y = fn(*ts)
+        if not got:
+            assert OF.ops.launch_count() > before and OF._split_supported(q, k, v, 0.3, causal, m)
+        y.backward(go.to(y.dtype))
+        got.append([y] + [t.grad for t in ts])
+        if len(got) == 2:
+            q, k, v, go = (t.double() for t in (q, k, v, go))
+    for new, old, want in zip(*got):
+        err = [float((t.double() - want).norm()) for t in (new, old)]
+        # both round once to bf16: the errors differ by chance only, and by the fp32 sums' order where the results cancel to nothing
+        assert err[0] <= 1.3 * err[1] + 1e-5 * float(want.norm()) + 1e-6 * math.sqrt(want.numel()), err
+
+
+@pytest.mark.parametrize("layout", ["qkv", "q_kv"])
+def test_attention_from_packed_projections(layout):
+    b, s, sk, a, d = 2, 150, 150 if layout == "qkv" else 333, 3, 48
+    keep = torch.rand(b, 1, s, sk, device="cuda") < 0.7
+    ts = [_rand((b, s, a, 3 * d), 1)] if layout == "qkv" else [_rand((b, s, a, d), 1), _rand((b, sk, a, 2 * d), 2)]
+    go, out = _rand((b, s, a, d), 3), []
+    for packed in (True, False):
+        xs = [t.clone().requires_grad_(True) for t in ts]
+        if packed:
+            y = OF.attention_packed(layout, tuple(xs), causal=False, scale=d ** -0.5, mask=keep)
+        else:
+            y = _attend64(*OF._split_views(layout, xs), d ** -0.5, keep).permute(0, 2, 1, 3)
+        y.backward(go.to(y.dtype))
+        out.append([y] + [x.grad for x in xs])
+    for got, want in zip(*out):
+        assert float((got.double() - want.double()).norm() / want.double().norm()) < 2.0 ** -7
+
+
+def test_attention_gradients_can_be_differentiated_again():
+    q, k, v = (_rand((1, 2, 20, 24), i).requires_grad_(True) for i in range(3))
+    (g,) = torch.autograd.grad(OF.attention(q, k, v, scale=0.2).float().square().sum(), q, create_graph=True)
+    (h,) = torch.autograd.grad(g.float().square().sum(), k)
+    ref = [t.detach().double().requires_grad_(True) for t in (q, k, v)]
+    (g64,) = torch.autograd.grad(_attend64(*ref, 0.2).square().sum(), ref[0], create_graph=True)
+    (h64,) = torch.autograd.grad(g64.square().sum(), ref[1])
+    assert float((h.double() - h64).norm() / h64.norm()) < 0.05      # three bf16 roundings in a chain of products
