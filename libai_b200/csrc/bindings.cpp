@@ -101,6 +101,9 @@ int lb_attn_split_bwd(const void* dout, const void* q, const void* k, const void
                       void* dk, void* dv, float* delta, float* dq_acc, int B, int A, int Sq, int Sk, int d, const long* qs, const long* ks,
                       const long* vs, const long* dos, const long* dqs, const long* dks, const long* dvs, int causal, float scale,
                       const uint32_t* mask, const float* fill, long mask_b, long mask_a, int* err, cudaStream_t s);
+int lb_attn_decode(const void* q, const void* k_new, const void* v_new, const void* k_past, const void* v_past, void* k_out, void* v_out, void* o,
+                   int B, int A, int past, int d, const long* q_st, const long* kn_st, const long* vn_st, const long* kp_st, const long* vp_st,
+                   float scale, const uint32_t* mask, const float* fill, long mask_b, long mask_a, cudaStream_t s);
 int lb_bias_dropout_residual(const void* x, const void* bias, const void* res, void* y, long rows, int N, float p,
                              const LbRngArgs* rng, const long long* rng_in, long long* rng_out, cudaStream_t s);
 }
@@ -912,6 +915,26 @@ void attn_split_bwd(const Tensor& dout, const Tensor& q, const Tensor& k, const 
         "attn_split_bwd");
 }
 
+// One token per sequence against a key / value cache (csrc/attention_decode.cu): q, k_new, v_new [B, A, 1, d] views, k_past, v_past
+// [B, A, past, d] views -> (context [B, 1, A, d], the caches grown by the token [B, A, past + 1, d])
+std::tuple<Tensor, Tensor, Tensor> attn_decode(const Tensor& q, const Tensor& k_new, const Tensor& v_new, const Tensor& k_past, const Tensor& v_past,
+                                               double scale, const c10::optional<Tensor>& words, const c10::optional<Tensor>& fill) {
+  c10::cuda::CUDAGuard guard(q.device());
+  long st[5][3];
+  int i = 0;
+  for (const Tensor* t : {&q, &k_new, &v_new, &k_past, &v_past}) split_strides(*t, st[i++]);
+  const int B = (int)q.size(0), A = (int)q.size(1), d = (int)q.size(3), past = (int)k_past.size(2);
+  TORCH_CHECK(q.size(2) == 1 && k_new.sizes() == q.sizes() && v_new.sizes() == q.sizes() && k_past.sizes() == v_past.sizes() && k_past.size(0) == B &&
+                  k_past.size(1) == A && k_past.size(3) == d, "attn_decode: shapes");
+  const SplitMask m = split_mask(words, fill, B, A, 1, past + 1);
+  Tensor o = at::empty({B, 1, A, d}, q.options());
+  Tensor k = at::empty({B, A, past + 1, d}, q.options()), v = at::empty({B, A, past + 1, d}, q.options());
+  check(lb_attn_decode(q.data_ptr(), k_new.data_ptr(), v_new.data_ptr(), k_past.data_ptr(), v_past.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(),
+                       B, A, past, d, st[0], st[1], st[2], st[3], st[4], (float)scale, m.words, m.fill, m.b, m.a, cur_stream()),
+        "attn_decode");
+  return std::make_tuple(o, k, v);
+}
+
 // ---- fused collectives ---------------------------------------------------------------------------------------
 std::vector<long> to_longs(at::IntArrayRef v) { return std::vector<long>(v.begin(), v.end()); }
 
@@ -1064,6 +1087,7 @@ TORCH_LIBRARY(libai_b200, m) {
   m.def("attn_mask_pack(Tensor mask, bool causal) -> (Tensor, Tensor)", &attn_mask_pack);
   m.def("attn_split_fwd(Tensor q, Tensor k, Tensor v, bool causal, float scale, Tensor? words, Tensor? fill, bool train) -> (Tensor, Tensor, Tensor)", &attn_split_fwd);
   m.def("attn_split_bwd(Tensor dout, Tensor q, Tensor k, Tensor v, Tensor o, Tensor o_lo, Tensor lse, Tensor(a!) dq, Tensor(b!) dk, Tensor(c!) dv, bool causal, float scale, Tensor? words, Tensor? fill) -> ()", &attn_split_bwd);
+  m.def("attn_decode(Tensor q, Tensor k_new, Tensor v_new, Tensor k_past, Tensor v_past, float scale, Tensor? words, Tensor? fill) -> (Tensor, Tensor, Tensor)", &attn_decode);
   m.def("attn_fwd(Tensor q, Tensor k, Tensor v, bool causal, float scale, Tensor? kv_lens, Tensor? bias=None, Tensor? alibi_slopes=None, float p_drop=0.0, int salt=0) -> (Tensor, Tensor, Tensor)", &attn_fwd);
   m.def("attn_bwd(Tensor dout, Tensor q, Tensor k, Tensor v, Tensor o, Tensor lse, bool causal, float scale, Tensor? kv_lens, Tensor? bias=None, Tensor? alibi_slopes=None, Tensor(a!)? dbias=None, float p_drop=0.0, Tensor? rng_state=None) -> (Tensor, Tensor, Tensor, Tensor)", &attn_bwd);
   m.def("bias_dropout_residual(Tensor x, Tensor? bias, Tensor? res, float p, int salt, Tensor? rng_state=None) -> (Tensor, Tensor)", &bias_dropout_residual);

@@ -187,6 +187,14 @@ class MultiheadAttention(nn.Module):
             query, key, value = qkv[..., :d], qkv[..., d : 2 * d], qkv[..., 2 * d :]
             if past_key_value is not None:
                 past_key, past_value = past_key_value
+                grown = OF.attention_cached(
+                    query, key, value, past_key, past_value, scale=self.softmax_scale,
+                    mask=attention_mask.dense() if isinstance(attention_mask, KeyPaddingMask) else attention_mask,
+                    dropout_p=self.attention_dropout_prob, training=self.training,
+                )
+                if grown is not None:
+                    output = self._project(grown[0].reshape(bsz, -1, a * d), hidden_states, residual, sp)
+                    return (output, tuple(grown[1:])) if use_cache else output
                 key = torch.cat((past_key.type_as(key), key), dim=2)
                 value = torch.cat((past_value.type_as(value), value), dim=2)
         if use_cache:

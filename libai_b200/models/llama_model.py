@@ -142,17 +142,23 @@ class LlamaAttention(nn.Module):
         else:
             q4 = qkv.permute(0, 2, 1, 3)
             query, key, value = q4[..., :d], q4[..., d : 2 * d], q4[..., 2 * d :]
+            grown = None
             if past_key_value is not None:
-                key = torch.cat((past_key_value[0].type_as(key), key), dim=2)
-                value = torch.cat((past_key_value[1].type_as(value), value), dim=2)
-            if use_cache:
-                past_key_value = (key, value)
-            causal = attention_mask is None and key.shape[2] == query.shape[2]
-            mask = attention_mask
-            if mask is None and not causal:  # decoding with a cache: every cached key is visible
-                mask = None
-            context = OF.attention(query, key, value, causal=causal, scale=self.norm_factor, mask=mask)
-            context = context.transpose(1, 2).reshape(bsz, -1, a * d)
+                grown = OF.attention_cached(query, key, value, *past_key_value, scale=self.norm_factor, mask=attention_mask)
+            if grown is not None:      # one new token: attention and the grown caches in one kernel
+                context, past_key_value = grown[0].reshape(bsz, -1, a * d), tuple(grown[1:])
+            else:
+                if past_key_value is not None:
+                    key = torch.cat((past_key_value[0].type_as(key), key), dim=2)
+                    value = torch.cat((past_key_value[1].type_as(value), value), dim=2)
+                if use_cache:
+                    past_key_value = (key, value)
+                causal = attention_mask is None and key.shape[2] == query.shape[2]
+                mask = attention_mask
+                if mask is None and not causal:  # decoding with a cache: every cached key is visible
+                    mask = None
+                context = OF.attention(query, key, value, causal=causal, scale=self.norm_factor, mask=mask)
+                context = context.transpose(1, 2).reshape(bsz, -1, a * d)
         if sp:
             context = context.reshape(-1, a * d)
         output = self.o_proj(context)

@@ -634,6 +634,18 @@ def _split_views(layout: str, ts):
     return ts
 
 
+def _mask_supported(mask, q, sk: int) -> bool:
+    full = (q.shape[0], q.shape[1], q.shape[2], sk)
+    return (mask.device == q.device and not mask.is_complex() and mask.dim() <= 4
+            and all(m in (1, n) for m, n in zip(reversed(mask.shape), reversed(full))))
+
+
+def _pack_mask(ext, mask, q, sk: int, causal: bool):
+    m = mask[(None,) * (4 - mask.dim())]
+    count_launch()
+    return ext.attn_mask_pack(m.expand(m.shape[0], m.shape[1], q.shape[2], sk), causal)
+
+
 def _split_supported(q, k, v, scale, causal, mask) -> bool:
     """Sizes and types of the kernels with 32-bit probabilities, from ``[b, a, s, d]`` views.  Other head dims stay with the flash
     kernels (64 / 128 without a mask: bf16 probabilities, as ever) or with the unfused form."""
@@ -641,10 +653,8 @@ def _split_supported(q, k, v, scale, causal, mask) -> bool:
             and q.shape[:2] == k.shape[:2] and q.shape[-1] == k.shape[-1] and q.shape[-1] % 8 == 0 and 8 <= q.shape[-1] <= 64
             and min(q.shape) > 0 and k.shape[2] > 0 and max(q.shape[:2]) <= 65535 and scale > 0 and (not causal or k.shape[2] >= q.shape[2])):
         return False
-    if mask is not None:
-        full = (q.shape[0], q.shape[1], q.shape[2], k.shape[2])
-        if mask.device != q.device or mask.is_complex() or mask.dim() > 4 or any(m not in (1, n) for m, n in zip(reversed(mask.shape), reversed(full))):
-            return False
+    if mask is not None and not _mask_supported(mask, q, k.shape[2]):
+        return False
     return _plain_call()
 
 
@@ -655,11 +665,7 @@ class _SplitAttnFn(torch.autograd.Function):
     def forward(ctx, layout, causal, scale, mask, *ts):
         ext = load_ext()
         q, k, v = _split_views(layout, ts)
-        words = fill = None
-        if mask is not None:
-            m = mask[(None,) * (4 - mask.dim())]
-            words, fill = ext.attn_mask_pack(m.expand(m.shape[0], m.shape[1], q.shape[2], k.shape[2]), causal)
-            count_launch()
+        words, fill = (None, None) if mask is None else _pack_mask(ext, mask, q, k.shape[2], causal)
         train = any(ctx.needs_input_grad[4:])
         o, o_lo, lse = ext.attn_split_fwd(q, k, v, causal and mask is None, scale, words, fill, train)
         count_launch()
@@ -698,6 +704,24 @@ def attention_packed(layout: str, ts, *, causal: bool, scale: float, mask=None, 
     if not _split_supported(*_split_views(layout, ts), scale, causal, mask):
         return None
     return _SplitAttnFn.apply(layout, causal, float(scale), mask, *ts)
+
+
+def attention_cached(q, k_new, v_new, past_key, past_value, *, scale: float, mask=None, dropout_p: float = 0.0, training: bool = False):
+    """One new token per sequence: ``q``, ``k_new``, ``v_new`` ``[b, a, 1, d]``, the caches ``[b, a, past, d]`` → (context
+    ``[b, 1, a, d]``, the caches with the token appended) in one kernel; ``None`` where it does not apply (gradients, several new
+    tokens, other types): the caller concatenates and takes :func:`attention`."""
+    ts = (q, k_new, v_new, past_key, past_value)
+    if (not use_native(q) or q.dim() != 4 or q.shape[2] != 1 or (dropout_p > 0.0 and training) or scale <= 0
+            or any(t.dtype != torch.bfloat16 for t in ts) or k_new.shape != q.shape or v_new.shape != q.shape
+            or past_key.dim() != 4 or past_key.shape != past_value.shape or past_key.shape[:2] != q.shape[:2] or past_key.shape[3] != q.shape[3]
+            or past_key.shape[2] == 0 or min(q.shape) == 0 or max(q.shape[:2]) > 65535 or q.shape[3] % 8 or q.shape[3] > 256
+            or not all(_rows_of_vectors(t) for t in ts) or (torch.is_grad_enabled() and any(t.requires_grad for t in ts))
+            or (mask is not None and not _mask_supported(mask, q, past_key.shape[2] + 1)) or not _plain_call()):
+        return None
+    ext = load_ext()
+    words, fill = (None, None) if mask is None else _pack_mask(ext, mask, q, past_key.shape[2] + 1, False)
+    count_launch()
+    return ext.attn_decode(q, k_new, v_new, past_key, past_value, float(scale), words, fill)
 
 
 def attention_qkvpacked_supported(qkv, mask, dropout_p, training) -> bool:

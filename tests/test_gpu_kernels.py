@@ -158,3 +158,24 @@ def test_attention_gradients_can_be_differentiated_again():
     (g64,) = torch.autograd.grad(_attend64(*ref, 0.2).square().sum(), ref[0], create_graph=True)
     (h64,) = torch.autograd.grad(g64.square().sum(), ref[1])
     assert float((h.double() - h64).norm() / h64.norm()) < 0.05      # three bf16 roundings in a chain of products
+
+
+@pytest.mark.parametrize("mask", [None, "bool", "int64"])
+@pytest.mark.parametrize("b,a,past,d", [(1, 1, 1, 8), (8, 16, 511, 64), (2, 3, 63, 24), (3, 2, 1000, 128), (1, 4, 64, 48), (2, 1, 300, 256), (5, 7, 129, 16)])
+def test_attention_against_a_cache(b, a, past, d, mask):
+    """One new token: context and grown caches, caches as strided views, with and without masked keys, every split over a cluster."""
+    qkv = _rand((b, 1, a, 3 * d), 1)
+    q, k, v = qkv.permute(0, 2, 1, 3).chunk(3, -1)
+    kp, vp = _rand((b, past, a, d), 2).permute(0, 2, 1, 3), _rand((b, a, past, d), 3)
+    m = None
+    if mask is not None:
+        m = torch.rand(b, 1, 1, past + 1, device="cuda") < 0.6
+        m[0] = False                                                # no visible key at all: uniform
+        m = m if mask == "bool" else m.long() * 2
+    got = OF.attention_cached(q, k, v, kp, vp, scale=d ** -0.5, mask=m)
+    key, value = torch.cat([kp, k], 2), torch.cat([vp, v], 2)
+    assert torch.equal(got[1], key) and torch.equal(got[2], value)
+    want = _attend64(q, key, value, d ** -0.5, None if m is None else m.bool()).permute(0, 2, 1, 3)
+    old = OF.attention_ref(q, key, value, causal=False, scale=d ** -0.5, mask=m).permute(0, 2, 1, 3)
+    err = [float((t.double() - want).norm()) for t in (got[0], old)]
+    assert err[0] <= 1.3 * err[1] + 1e-5 * float(want.norm()), err   # both: fp32 throughout, one rounding to bf16
