@@ -984,6 +984,10 @@ static int gemm_allow_2cta() {
   return v;
 }
 
+extern "C" int lb_gemm_small_rule(int M, int N, int K, int* nt, int* ranks);
+extern "C" int lb_gemm_small(const void* x, const void* w, void* out, int M, int N, int K, int ldx, int ldw, int ldo, const void* bias, int act,
+                             void* pre_out, const void* residual, int nt, int ranks, cudaStream_t s);
+
 static int gemm_impl(const void* a, const void* b, void* out, int M, int N, int K, int lda, int ldb, int ldo, int layout,
                      int epi, const void* bias, int act, void* pre_out, const void* pre_in, int force_bn,
                      int force_splits, const lb::CommParams& cp_in, cudaStream_t stream, const float* deq_a = nullptr,
@@ -992,6 +996,14 @@ static int gemm_impl(const void* a, const void* b, void* out, int M, int N, int 
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (tile_group && (layout != 0 || epi == 2 || cp_in.mode != lb::COMM_NONE || deq_a || groups < 1)) return -8;
   if ((lda % 8) || (ldb % 8) || (N % 8) || (ldo % 4)) return -1;
+  if (layout == 0 && epi == 0 && cp.mode == lb::COMM_NONE && deq_a == nullptr && !tile_group && colsum == nullptr && force_bn == 0 &&
+      force_splits == 0 && (pre_in == nullptr || act == lb::ACT_RESADD)) {
+    int nt = 0, ranks = 0;      // few rows: w is streamed by clusters of CTAs (gemm_small_sm100.cu)
+    if (lb_gemm_small_rule(M, N, K, &nt, &ranks)) {
+      const int rc = lb_gemm_small(a, b, out, M, N, K, lda, ldb, ldo, bias, act, pre_out, pre_in, nt, ranks, stream);
+      if (rc != -1) return rc;
+    }
+  }
   const bool a_mn = (layout == 2);
   const bool b_mn = (layout != 0);
   const int sms = num_sms();

@@ -179,3 +179,19 @@ def test_attention_against_a_cache(b, a, past, d, mask):
     old = OF.attention_ref(q, key, value, causal=False, scale=d ** -0.5, mask=m).permute(0, 2, 1, 3)
     err = [float((t.double() - want).norm()) for t in (got[0], old)]
     assert err[0] <= 1.3 * err[1] + 1e-5 * float(want.norm()), err   # both: fp32 throughout, one rounding to bf16
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 8, 8), (1, 1024, 1024), (5, 1160, 72), (16, 128, 640), (17, 384, 1536), (33, 4096, 200), (64, 136, 4096), (64, 3072, 1024)])
+def test_linear_of_few_rows(m, n, k):
+    """Edges of the row, column and K tiles, every cluster size, bias, activation, pre-activation copy and residual; the sums of a
+    cluster meet in a fixed order."""
+    x, w, b, r = _rand((m, k), 1), _rand((n, k), 2, k ** -0.5), _rand((n,), 3), _rand((m, n), 4)
+    ext = OF.load_ext()
+    z = x.double() @ w.double().t() + b.double()
+    near = lambda got, want: float((got.double() - want).norm() / want.norm()) < 2.0 ** -8       # one rounding of an fp32 sum
+    for act, fn in ((OF.ACT_NONE, lambda t: t), (OF.ACT_GELU, torch.nn.functional.gelu), (OF.ACT_SILU, torch.nn.functional.silu)):
+        y, pre = ext.linear_fwd(x, w, b, act, act != OF.ACT_NONE)
+        assert near(y, fn(z)) and (act == OF.ACT_NONE or near(pre, z))
+        assert torch.equal(ext.linear_fwd(x, w, b, act, False)[0], y)
+    assert near(ext.linear_bias_residual(x, w, b, r), z + r.double())
+    assert near(ext.linear_fwd(x, w, None, OF.ACT_NONE, False)[0], z - b.double())
