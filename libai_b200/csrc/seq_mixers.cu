@@ -318,6 +318,231 @@ delta_scan_kernel(const T* __restrict__ qkv, long ldq, int voff, const float* __
   }
 }
 
+// ------------------------------------------------------------------------------------------------------------------
+// The same scan for one decay per head, two tokens at a time.  With k0, k1, q0, q1 the unit keys and queries of two consecutive
+// tokens, all four products with the state are taken on the state before them, and two inner products (k1·k0, q1·k0) carry the
+// first token's write over to the second:
+//   u0 = b0 (v0 - g0 k0ᵀS);                          o0 = g0 q0ᵀS + (q0·k0) u0
+//   u1 = b1 (v1 - g1 (g0 k1ᵀS + (k1·k0) u0));        o1 = g1 (g0 q1ᵀS + (q1·k0) u0) + (q1·k1) u1
+//   S <- g0 g1 S + g1 k0 u0ᵀ + k1 u1ᵀ
+// Everything stays fp32.  The scan is a serial chain over the tokens, bounded by the latency of one link and by the issue of its
+// multiply-adds, so: one reduction and one scaling of the state per two tokens instead of per token; packed pairs of fp32
+// (fma.rn.f32x2); four lanes per column with CPT columns each, so that a staged vector is read once for CPT columns (with eight
+// lanes and one column per lane the 16-byte shared-memory reads took most of a token's 1370 cycles); the next tokens arrive by
+// cp.async meanwhile.  [2560 tokens of 4 sequences up to 1024, 16 heads, 128 x 128]: 755 -> 330 us (one column per lane:
+// 434 us).
+// Lane r of a column holds rows 16 d + 4 r + 0..3: the four lanes read 64 contiguous bytes.
+// ------------------------------------------------------------------------------------------------------------------
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+  unsigned long long d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
+  return d;
+}
+__device__ __forceinline__ void unpack2(unsigned long long a, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a)); }
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, int bytes) {        // the rest of the 16 is zero
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src), "r"(bytes));
+}
+__device__ __forceinline__ void cp_async4(void* dst, const void* src, int bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src), "r"(bytes));
+}
+
+constexpr int PAIR_THREADS = 128;
+// floats of shared memory: two buffers of k, q, v for CT tokens, and of their scalars (beta, g, q·k, then k1·k0 and q1·k0 per pair)
+constexpr int pair_buffer_floats(int rows, int cols) { return CT * rows * 2 + CT * cols; }
+constexpr int pair_smem_floats(int rows, int cols) { return 2 * (pair_buffer_floats(rows, cols) + 4 * CT); }
+
+// D <= 16 D4 rows (D % 4 == 0), 32 CPT columns per block; v's rows in whole aligned 16-byte vectors
+template <typename T, int D4, int CPT>
+__global__ void __launch_bounds__(PAIR_THREADS)
+delta_scan_pair_kernel(const T* __restrict__ qkv, long ldq, int voff, const float* __restrict__ qn, const float* __restrict__ kn,
+                       const float* __restrict__ kqs, const float* __restrict__ gs, const float* __restrict__ betas,
+                       float* __restrict__ S, const int* __restrict__ seq_off, const int* __restrict__ slots,
+                       const int* __restrict__ past, float* __restrict__ out, int H, int KH, int D, int V) {
+  constexpr int DP = 16 * D4, VB = 32 * CPT, BUF = pair_buffer_floats(DP, VB), VE = 16 / sizeof(T);
+  extern __shared__ __align__(16) float sm[];
+  float* scal = sm + 2 * BUF;
+  const int tid = threadIdx.x, r = tid & 3, cg = tid >> 2, bit0 = r & 1;
+  const int b = blockIdx.x / H, h = blockIdx.x % H, kh = h / (H / KH), j0 = blockIdx.y * VB;
+  const int n = seq_off[b + 1] - seq_off[b];
+  const long tok0 = seq_off[b];
+  float* Sg = S + ((long)slots[b] * H + h) * (long)D * V;
+  const int jc = j0 + cg * CPT;
+  unsigned long long s[CPT][2 * D4];
+#pragma unroll
+  for (int d = 0; d < D4; ++d) {
+#pragma unroll
+    for (int c = 0; c < CPT; ++c) {
+      float x[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int i = d * 16 + r * 4 + e;
+        x[e] = (past[b] > 0 && jc + c < V && i < D) ? Sg[(long)i * V + jc + c] : 0.f;
+      }
+      s[c][2 * d] = pack2(x[0], x[1]);
+      s[c][2 * d + 1] = pack2(x[2], x[3]);
+    }
+  }
+  auto stage = [&](int c0, int buf) {
+    const int ct = min(CT, n - c0);
+    float* sk = sm + buf * BUF;
+    float* sq = sk + CT * DP;
+    T* sv = reinterpret_cast<T*>(sq + CT * DP);
+    float* sc = scal + buf * 4 * CT;
+    for (int e = tid; e < CT * DP / 4; e += PAIR_THREADS) {
+      const int t = e / (DP / 4), i = (e % (DP / 4)) * 4;
+      const bool in = t < ct && i < D;
+      const long at = in ? ((tok0 + c0 + t) * KH + kh) * (long)D + i : 0;
+      cp_async16(sk + t * DP + i, kn + at, in ? 16 : 0);
+      cp_async16(sq + t * DP + i, qn + at, in ? 16 : 0);
+    }
+    for (int e = tid; e < CT * VB / VE; e += PAIR_THREADS) {
+      const int t = e / (VB / VE), c = (e % (VB / VE)) * VE;
+      const bool in = t < ct && j0 + c < V;
+      cp_async16(sv + t * VB + c, in ? qkv + (tok0 + c0 + t) * ldq + voff + (long)h * V + j0 + c : qkv, in ? 16 : 0);
+    }
+    if (tid < CT) {
+      const bool in = tid < ct;
+      const long row = in ? tok0 + c0 + tid : tok0;
+      cp_async4(sc + tid, betas + row * H + h, in ? 4 : 0);
+      cp_async4(sc + CT + tid, gs + row * H + h, in ? 4 : 0);
+      cp_async4(sc + 2 * CT + tid, kqs + row * KH + kh, in ? 4 : 0);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  stage(0, 0);
+  for (int c0 = 0, buf = 0; c0 < n; c0 += CT, buf ^= 1) {
+    const int ct = min(CT, n - c0);
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();                              // the tokens are here, and nobody reads the other buffer any more
+    if (c0 + CT < n) stage(c0 + CT, buf ^ 1);
+    const float* sk = sm + buf * BUF;
+    const float* sq = sk + CT * DP;
+    const T* sv = reinterpret_cast<const T*>(sq + CT * DP);
+    float* sc = scal + buf * 4 * CT;
+    for (int p = tid >> 5; p < CT / 2; p += PAIR_THREADS / 32) {     // inner products between the tokens of a pair, one pair per warp
+      const int lane = tid & 31;
+      float kk = 0.f, qk = 0.f;
+      for (int i = lane * 4; i < DP; i += 128) {
+        const float4 k0 = *reinterpret_cast<const float4*>(sk + 2 * p * DP + i), k1 = *reinterpret_cast<const float4*>(sk + (2 * p + 1) * DP + i),
+                     q1 = *reinterpret_cast<const float4*>(sq + (2 * p + 1) * DP + i);
+        kk += (k1.x * k0.x + k1.y * k0.y) + (k1.z * k0.z + k1.w * k0.w);
+        qk += (q1.x * k0.x + q1.y * k0.y) + (q1.z * k0.z + q1.w * k0.w);
+      }
+      kk = warp_sum(kk);
+      qk = warp_sum(qk);
+      if (lane == 0) { sc[3 * CT + 2 * p] = kk; sc[3 * CT + 2 * p + 1] = qk; }
+    }
+    __syncthreads();
+    for (int t = 0; t < ct; t += 2) {
+      const ulonglong2* k0p = reinterpret_cast<const ulonglong2*>(sk + t * DP) + r;
+      const ulonglong2* k1p = reinterpret_cast<const ulonglong2*>(sk + (t + 1) * DP) + r;
+      const ulonglong2* q0p = reinterpret_cast<const ulonglong2*>(sq + t * DP) + r;
+      const ulonglong2* q1p = reinterpret_cast<const ulonglong2*>(sq + (t + 1) * DP) + r;
+      unsigned long long acc[CPT][4];
+#pragma unroll
+      for (int c = 0; c < CPT; ++c)
+#pragma unroll
+        for (int m = 0; m < 4; ++m) acc[c][m] = 0ull;
+      ulonglong2 K0[D4], K1[D4];
+#pragma unroll
+      for (int d = 0; d < D4; ++d) {
+        K0[d] = k0p[d * 4];
+        K1[d] = k1p[d * 4];
+        const ulonglong2 Q0 = q0p[d * 4], Q1 = q1p[d * 4];
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) {
+          acc[c][0] = fma2(K0[d].x, s[c][2 * d], acc[c][0]);
+          acc[c][1] = fma2(Q0.x, s[c][2 * d], acc[c][1]);
+          acc[c][2] = fma2(K1[d].x, s[c][2 * d], acc[c][2]);
+          acc[c][3] = fma2(Q1.x, s[c][2 * d], acc[c][3]);
+          acc[c][0] = fma2(K0[d].y, s[c][2 * d + 1], acc[c][0]);
+          acc[c][1] = fma2(Q0.y, s[c][2 * d + 1], acc[c][1]);
+          acc[c][2] = fma2(K1[d].y, s[c][2 * d + 1], acc[c][2]);
+          acc[c][3] = fma2(Q1.y, s[c][2 * d + 1], acc[c][3]);
+        }
+      }
+      // sums over the four lanes; with two columns the even lanes end up with the first, the odd ones with the second
+      float w[4];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        float x, y, a0, a1 = 0.f;
+        unpack2(acc[0][m], x, y);
+        a0 = x + y;
+        if constexpr (CPT == 2) {
+          unpack2(acc[CPT - 1][m], x, y);
+          a1 = x + y;
+          const float keep = bit0 ? a1 : a0, send = bit0 ? a0 : a1;
+          w[m] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
+        } else {
+          w[m] = a0 + __shfl_xor_sync(0xffffffffu, a0, 1);
+        }
+      }
+#pragma unroll
+      for (int m = 0; m < 4; ++m) w[m] += __shfl_xor_sync(0xffffffffu, w[m], 2);
+      const bool two = t + 1 < ct;                // the last token of an odd count: k1 = q1 = 0, b1 = 0, its decay is left out
+      const float b0 = sc[t], b1 = sc[t + 1], g0 = sc[CT + t], g1 = two ? sc[CT + t + 1] : 1.f, kq0 = sc[2 * CT + t], kq1 = sc[2 * CT + t + 1];
+      const float kk = sc[3 * CT + t], qk = sc[3 * CT + t + 1];
+      const int vc = cg * CPT + (CPT == 2 ? bit0 : 0);
+      const float u0 = b0 * (ldf(sv + t * VB + vc) - g0 * w[0]);
+      const float o0 = g0 * w[1] + kq0 * u0;
+      const float u1 = b1 * (ldf(sv + (t + 1) * VB + vc) - g1 * (g0 * w[2] + kk * u0));
+      const float o1 = g1 * (g0 * w[3] + qk * u0) + kq1 * u1;
+      const float gg = g0 * g1, w0 = g1 * u0;
+      const unsigned long long G = pack2(gg, gg);
+      float U0[CPT], U1[CPT];
+      if constexpr (CPT == 2) {
+        const float x0 = __shfl_xor_sync(0xffffffffu, w0, 1), x1 = __shfl_xor_sync(0xffffffffu, u1, 1);
+        U0[0] = bit0 ? x0 : w0;
+        U1[0] = bit0 ? x1 : u1;
+        U0[CPT - 1] = bit0 ? w0 : x0;
+        U1[CPT - 1] = bit0 ? u1 : x1;
+      } else {
+        U0[0] = w0;
+        U1[0] = u1;
+      }
+#pragma unroll
+      for (int c = 0; c < CPT; ++c) {
+        const unsigned long long p0 = pack2(U0[c], U0[c]), p1 = pack2(U1[c], U1[c]);
+#pragma unroll
+        for (int d = 0; d < D4; ++d) {
+          s[c][2 * d] = fma2(K1[d].x, p1, fma2(K0[d].x, p0, mul2(s[c][2 * d], G)));
+          s[c][2 * d + 1] = fma2(K1[d].y, p1, fma2(K0[d].y, p0, mul2(s[c][2 * d + 1], G)));
+        }
+      }
+      if (r < CPT && j0 + vc < V) {
+        float* o = out + (tok0 + c0 + t) * (long)(H * V) + (long)h * V + j0 + vc;
+        o[0] = o0;
+        if (two) o[(long)H * V] = o1;
+      }
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < CPT; ++c) {
+    if (jc + c >= V) continue;
+#pragma unroll
+    for (int d = 0; d < D4; ++d) {
+      float x[4];
+      unpack2(s[c][2 * d], x[0], x[1]);
+      unpack2(s[c][2 * d + 1], x[2], x[3]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int i = d * 16 + r * 4 + e;
+        if (i < D) Sg[(long)i * V + jc + c] = x[e];
+      }
+    }
+  }
+}
+
 // y[tok, h, :] = o / rms(o over V) * w * act(gate[tok, h, :]);  act 0: silu, 1: sigmoid.  One warp per (token, head).
 template <typename T>
 __global__ void gated_rmsnorm_kernel(const float* __restrict__ o, const T* __restrict__ gate, long ldg, const T* __restrict__ w,
@@ -800,6 +1025,26 @@ int lbs_delta_scan(const void* qkv, long ldq, int koff, int voff, const void* a,
   DISPATCH(dtype, delta_prep_kernel<T><<<cdiv(tokens * KH * 32, 256), 256, 0, s>>>((const T*)qkv, ldq, koff, (const T*)a, lda, (const T*)bl,
                                                                                   ldb, (const T*)A_log, (const T*)dt_bias, qn, kn, kq, g,
                                                                                   beta, tokens, H, KH, D, chan));
+  // one decay per head: two tokens at a time where rows and columns come in whole 16-byte vectors (the general kernel takes the rest:
+  // decays per channel, more than 128 rows, odd sizes)
+  const int vec = dtype == 0 ? 4 : 8;
+  if (!chan && D <= 128 && D % 4 == 0 && V % vec == 0 && ldq % vec == 0 && voff % vec == 0 && (reinterpret_cast<uintptr_t>(qkv) & 15) == 0 &&
+      (reinterpret_cast<uintptr_t>(work) & 15) == 0 && (tokens * KH * D) % 4 == 0) {
+    const int cpt = (long)B * H * ((V + 63) / 64) >= 100 ? 2 : 1;    // two columns per lane once the blocks fill two thirds of the SMs
+    const dim3 pgrid((unsigned)(B * H), (unsigned)((V + 32 * cpt - 1) / (32 * cpt)));
+#define DSP(TT, D4, CPT)                                                                                                                \
+  delta_scan_pair_kernel<TT, D4, CPT><<<pgrid, PAIR_THREADS, pair_smem_floats(16 * D4, 32 * CPT) * sizeof(float), s>>>(                 \
+      (const TT*)qkv, ldq, voff, qn, kn, kq, g, beta, S, seq_off, slots, past, out, H, KH, D, V)
+#define DSP4(TT)                                          \
+  {                                                       \
+    if (D <= 64) { if (cpt == 2) DSP(TT, 4, 2); else DSP(TT, 4, 1); } \
+    else { if (cpt == 2) DSP(TT, 8, 2); else DSP(TT, 8, 1); }         \
+  }
+    if (dtype == 0) DSP4(float) else DSP4(bf16)
+#undef DSP4
+#undef DSP
+    return ok();
+  }
   const int dpt = D <= 32 ? 8 : (D <= 128 ? 16 : 32);  // rows per lane: 4 lanes per column up to D = 64, 8 lanes up to 256
   int R = 1;
   while (R * dpt < D) R <<= 1;                   // a power of two <= 8

@@ -195,3 +195,39 @@ def test_linear_of_few_rows(m, n, k):
         assert torch.equal(ext.linear_fwd(x, w, b, act, False)[0], y)
     assert near(ext.linear_bias_residual(x, w, b, r), z + r.double())
     assert near(ext.linear_fwd(x, w, None, OF.ACT_NONE, False)[0], z - b.double())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, BF16])
+@pytest.mark.parametrize("lens,heads,kv,d,v", [([1], 1, 1, 4, 8), ([2, 1, 17], 4, 2, 64, 64), ([16, 33], 2, 1, 128, 72), ([5, 31, 48, 7], 32, 16, 100, 128),
+                                               ([40], 3, 3, 12, 136), ([9, 20], 2, 2, 60, 24)])
+def test_delta_scan_two_tokens_at_a_time(lens, heads, kv, d, v, dtype):
+    """Odd and even numbers of tokens, rows and columns that do not fill a block, shared key heads, states that go on; every output and
+    the final state against the recurrence in 64 bits."""
+    from libai_b200.inference.ragged import RaggedBatch
+    from libai_b200.ops import seq_functional as SF
+
+    tokens, kd = sum(lens), kv * d
+    past = [3 * (i % 2) for i in range(len(lens))]
+    rb = RaggedBatch(lens, list(range(len(lens))), past, "cuda")
+    qkv, a, b = _rand((tokens, 2 * kd + heads * v), 1, 1.0, dtype), _rand((tokens, heads), 2, 1.0, dtype), _rand((tokens, heads), 3, 1.0, dtype)
+    rate, bias = _rand((heads,), 4, 0.5, dtype), _rand((heads,), 5, 0.5, dtype)
+    state = _rand((len(lens), heads, d, v), 6, 1.0, torch.float32)
+    S = state.clone()
+    out = SF.delta_scan(qkv, kd, 2 * kd, a, b, rate, bias, S, rb, kv, False)
+    x, unit = qkv.double(), lambda t: t / torch.sqrt(t.square().sum(-1, keepdim=True) + 1e-6)
+    q = unit(x[:, :kd].view(tokens, kv, d)).repeat_interleave(heads // kv, 1) / math.sqrt(d)
+    k = unit(x[:, kd:2 * kd].view(tokens, kv, d)).repeat_interleave(heads // kv, 1)
+    val, beta = x[:, 2 * kd:].view(tokens, heads, v), torch.sigmoid(b.double())
+    g = torch.exp(-torch.exp(rate.double()) * torch.nn.functional.softplus(a.double() + bias.double(), threshold=200.0))
+    at = 0
+    for i, n in enumerate(lens):
+        s = state[i].double() if past[i] else torch.zeros_like(state[i]).double()
+        for t in range(at, at + n):
+            s = s * g[t, :, None, None]
+            u = beta[t, :, None] * (val[t] - torch.einsum("hdv,hd->hv", s, k[t]))
+            s = s + k[t, :, :, None] * u[:, None]
+            want = torch.einsum("hdv,hd->hv", s, q[t]).reshape(-1)
+            # fp32 sums of d products per token, the state's own error carried along
+            assert float((out[t].double() - want).norm()) < 2e-6 * float(want.norm()) + 2e-6 * float(s.norm()) / math.sqrt(d)
+        assert float((S[i].double() - s).norm() / s.norm()) < 2e-6
+        at += n
