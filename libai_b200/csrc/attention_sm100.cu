@@ -356,6 +356,7 @@ struct AttnCfg2 {
   // S fp32 [0,128) | O fp32 [128,128+D) | P bf16 (64 columns) behind O: P no longer aliases S, so the two softmax
   // halves never race on it and Q·Kᵀ of the next block may be issued right behind P·V of the current one
   static constexpr uint32_t S_COL = 0, O_COL = 128, P_COL = 128 + D;
+  static constexpr int P_BUFS = (D == 64) ? 1 : 2;    // D = 128 has the columns for a second P: no wait for the previous block's P·V
   static constexpr int MIN_CTAS = (D == 64) ? 2 : 1;
 };
 
@@ -378,8 +379,8 @@ attn_fwd_v2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   uint64_t* v_empty = bars + 7;
   uint64_t* s_full = bars + 9;
   uint64_t* p_full = bars + 10;
-  uint64_t* o_full = bars + 11;
-  uint64_t* s_free = bars + 12;      // the softmax warps hold S(j) in registers: Q·Kᵀ(j+1) may overwrite the columns
+  uint64_t* o_full = bars + 11;      // 2: P·V of even and of odd blocks
+  uint64_t* s_free = bars + 13;      // the softmax warps hold S(j) in registers: Q·Kᵀ(j+1) may overwrite the columns
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 14);
 
   const int warp_idx = threadIdx.x / 32, lane = threadIdx.x % 32;
@@ -404,7 +405,8 @@ attn_fwd_v2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     }
     mbar_init(s_full, 1);
     mbar_init(p_full, 8);        // one arrival per softmax warp
-    mbar_init(o_full, 1);
+    mbar_init(&o_full[0], 1);
+    mbar_init(&o_full[1], 1);
     mbar_init(s_free, 8);
     fence_barrier_init();
     fence_proxy_async();
@@ -474,11 +476,11 @@ attn_fwd_v2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
 #pragma unroll
         for (int kk = 0; kk < ATT_BN / 16; ++kk) {
           // A = P from tensor memory: 16 bf16 per row = 8 columns per k-step
-          umma_f16_ts(tmem_base + Cfg::O_COL, tmem_base + Cfg::P_COL + kk * 8,
+          umma_f16_ts(tmem_base + Cfg::O_COL, tmem_base + Cfg::P_COL + (j % Cfg::P_BUFS) * 64 + kk * 8,
                       make_smem_desc_sw128(v_addr + kk * (16 * 128), ATT_BN * 128, 1024), idesc_pv,
                       (j > 0 || kk > 0) ? 1u : 0u);
         }
-        umma_commit(o_full);
+        umma_commit(&o_full[j & 1]);
         umma_commit(&v_empty[b]);
       }
       __syncwarp();
@@ -577,6 +579,15 @@ attn_fwd_v2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       }
       const bool bump_any = __any_sync(0xffffffffu, bump && j > 0);
       const float m_use = (m_run == -INFINITY) ? 0.f : m_run;
+      // P·V of the block that used these P columns last must have read them before they are overwritten.  With two sets (D = 128) S(j)
+      // says so: its commit follows P(j-2)·V(j-2) in the MMA warp's order.  With one set (D = 64) it does not (Q·K(j) is issued ahead of
+      // P(j-1)·V(j-1)): without a wait single warps' 32 rows came out wrong when two CTAs shared an SM.  It comes as late as can be,
+      // behind the first exponentials.
+      auto wait_p_free = [&]() {
+        if (j == 0) return;
+        mbar_wait(&o_full[(j - 1) & 1], ((j - 1) >> 1) & 1);
+        tc_fence_after_sync();
+      };
       // ---- pass 2: P = exp2(s * scale - m) as bf16 into the P columns
       float rowsum = 0.f;
       auto pass2 = [&](auto mask_tag) {
@@ -623,21 +634,17 @@ attn_fwd_v2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             }
             packed[i / 2] = pack_bf16(e0, e1);
           }
-          // P has one set of columns: P(j-1)·V(j-1) must have read it before block j's probabilities overwrite it.  S(j)
-          // says nothing about that (Q·K(j) is issued ahead of P(j-1)·V(j-1)).  The MMA was issued a whole pass 1 and half
-          // a pass 2 ago, so the wait is short; without it single warps' 32 rows came out wrong when two CTAs shared an SM.
-          if (c == 0 && j > 0) {
-            mbar_wait(o_full, (j - 1) & 1);
-            tc_fence_after_sync();
-          }
-          tmem_st_32x32b_x16(p_addr + c * 16, packed);
+          if (Cfg::P_BUFS == 1 && c == 0) wait_p_free();
+          tmem_st_32x32b_x16(p_addr + (j % Cfg::P_BUFS) * 64 + c * 16, packed);
         }
         rowsum = rs0 + rs1;
       };
       if (need_mask) pass2(std::true_type{}); else pass2(std::false_type{});
       l_run = l_run * alpha + rowsum;
-      // ---- O *= alpha (rare): P·V of block j-1 has retired (waited for above), rescale this half's O columns
+      // ---- O *= alpha (rare): wait until P·V of block j-1 has retired, then rescale this half's O columns
       if (bump_any) {
+        mbar_wait(&o_full[(j - 1) & 1], ((j - 1) >> 1) & 1);
+        tc_fence_after_sync();
 #pragma unroll
         for (int c = 0; c < D / 64; ++c) {
           uint32_t t[32];
@@ -658,7 +665,7 @@ attn_fwd_v2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     xch[half * 128 + r] = l_run;
     pair_sync(quad);
     l_run += xch[(half ^ 1) * 128 + r];
-    mbar_wait(o_full, (nkv - 1) & 1);
+    mbar_wait(&o_full[(nkv - 1) & 1], ((nkv - 1) >> 1) & 1);
     tc_fence_after_sync();
     const float inv = l_run > 0.f ? (DROP ? p.inv_keep : 1.0f) / l_run : 0.f;
     __nv_bfloat16* orow = p.o + ((static_cast<size_t>(batch) * p.S + q_idx) * p.A + head) * D + half * (D / 2);
@@ -1755,11 +1762,25 @@ cudaError_t launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUten
       return drop ? launch_bwd_pipe_t<lb::BIAS_ALIBI, true>(tq, tk, tv, tdo, tdq, p, s) : launch_bwd_pipe_t<lb::BIAS_ALIBI, false>(tq, tk, tv, tdo, tdq, p, s);
     }
   }
-  if (bias == lb::BIAS_NONE) return drop ? launch_bwd_t<D, lb::BIAS_NONE, true>(tq, tk, tv, tdo, tdq, p, s) : launch_bwd_t<D, lb::BIAS_NONE, false>(tq, tk, tv, tdo, tdq, p, s);
+  if constexpr (D == 128) {
+    if (bias == lb::BIAS_NONE && !drop) return cudaErrorInvalidValue;     // attention_bwd128_sm100.cu
+    if (bias == lb::BIAS_NONE) return launch_bwd_t<D, lb::BIAS_NONE, true>(tq, tk, tv, tdo, tdq, p, s);
+  } else {
+    if (bias == lb::BIAS_NONE) return drop ? launch_bwd_t<D, lb::BIAS_NONE, true>(tq, tk, tv, tdo, tdq, p, s) : launch_bwd_t<D, lb::BIAS_NONE, false>(tq, tk, tv, tdo, tdq, p, s);
+  }
   if (bias == lb::BIAS_DENSE) return drop ? launch_bwd_t<D, lb::BIAS_DENSE, true>(tq, tk, tv, tdo, tdq, p, s) : launch_bwd_t<D, lb::BIAS_DENSE, false>(tq, tk, tv, tdo, tdq, p, s);
   return drop ? launch_bwd_t<D, lb::BIAS_ALIBI, true>(tq, tk, tv, tdo, tdq, p, s) : launch_bwd_t<D, lb::BIAS_ALIBI, false>(tq, tk, tv, tdo, tdq, p, s);
 }
 }  // namespace
+
+// dq ([B, A, S, D] view, bf16) = acc (fp32 [B, A, S, D])
+extern "C" int lb_attn_dq_convert(const float* acc, void* dq, int B, int A, int S, int D, const long* st, cudaStream_t s) {
+  const long nvec = (long)B * A * S * D / 8;
+  int blocks = (int)((nvec + 511) / 512);
+  if (blocks > 148 * 8) blocks = 148 * 8;
+  lb::attn_dq_convert_kernel<<<blocks, 256, 0, s>>>(acc, (__nv_bfloat16*)dq, B, A, S, D, st[0], st[1], st[2]);
+  return (int)cudaGetLastError();
+}
 
 extern "C" int lb_attn_bwd(const void* dout, const void* q, const void* k, const void* v, const void* o,
                            const float* lse, void* dq, void* dk, void* dv, float* delta, float* dq_accum, int B, int A,
@@ -1844,10 +1865,5 @@ extern "C" int lb_attn_bwd(const void* dout, const void* q, const void* k, const
   cudaError_t e = (D == 64) ? launch_bwd<64>(tq, tk, tv, tdo, tdq, p, s) : launch_bwd<128>(tq, tk, tv, tdo, tdq, p, s);
   if (e != cudaSuccess) return (int)e;
   if (skip_helpers) return 0;
-  const long nvec = rows * D / 8;
-  int blocks = (int)((nvec + 511) / 512);
-  if (blocks > 148 * 8) blocks = 148 * 8;
-  lb::attn_dq_convert_kernel<<<blocks, 256, 0, s>>>(dq_accum, (__nv_bfloat16*)dq, B, A, S, D, p.g_strides[0],
-                                                    p.g_strides[1], p.g_strides[2]);
-  return (int)cudaGetLastError();
+  return lb_attn_dq_convert(dq_accum, dq, B, A, S, D, p.g_strides, s);
 }

@@ -92,6 +92,9 @@ int lb_attn_bwd(const void* dout, const void* q, const void* k, const void* v, c
                 const long* q_strides, const long* k_strides, const long* v_strides, const long* do_strides, int causal,
                 float scale, const int* kv_lens, const void* bias, const long* bias_strides, const float* alibi_slopes,
                 float* dbias, float p_drop, const long long* rng_state, cudaStream_t s);
+int lb_attn_bwd128(const void* dout, const void* q, const void* k, const void* v, const void* o, const float* lse, void* dq, void* dk, void* dv,
+                   float* stats, float* dq_acc, int B, int A, int S, const long* qs, const long* ks, const long* vs, const long* dos,
+                   const long* g_strides, int causal, float scale, const int* kv_lens, int* err, cudaStream_t s);
 int lb_attn_mask_pack(const void* mask, int elem, unsigned long long and_mask, int Bm, int Am, int Sq, int Sk, const long* strides, int causal,
                       int off, uint32_t* words, float* fill, cudaStream_t s);
 int lb_attn_split_fwd(const void* q, const void* k, const void* v, void* o, void* o_lo, float* lse, int B, int A, int Sq, int Sk, int d,
@@ -800,6 +803,16 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> attn_bwd(const Tensor& dout, const Te
     dbp = dbias->data_ptr<float>();
   }
   const bool has_rng = p_drop > 0.0 && rng_state.has_value() && rng_state->defined() && rng_state->numel() == 2;
+  if (D == 128 && !has_rng && bd.ptr == nullptr && !(alibi_slopes.has_value() && alibi_slopes->defined())) {
+    static WaitWord word;
+    Tensor stats = at::empty({(int64_t)B * A * ((S + 63) / 64) * 128}, q.options().dtype(at::kFloat));
+    const long gs[3] = {(long)dq.stride(0), (long)dq.stride(1), (long)dq.stride(2)};
+    check(lb_attn_bwd128(dout_c.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr<float>(), dq.data_ptr(), dk.data_ptr(),
+                         dv.data_ptr(), stats.data_ptr<float>(), dq_acc.data_ptr<float>(), B, A, S, qs, ks, vs, ds, gs, causal ? 1 : 0, (float)scale,
+                         (kv_lens.has_value() && kv_lens->defined()) ? kv_lens->data_ptr<int>() : nullptr, word.device("attn_bwd128"), cur_stream()),
+          "attn_bwd128");
+    return std::make_tuple(dq, dk, dv, dqkv);
+  }
   check(lb_attn_bwd(dout_c.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr<float>(),
                     dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), delta.data_ptr<float>(), dq_acc.data_ptr<float>(), B, A,
                     S, D, qs, ks, vs, ds, causal ? 1 : 0, (float)scale,

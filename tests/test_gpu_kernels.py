@@ -231,3 +231,24 @@ def test_delta_scan_two_tokens_at_a_time(lens, heads, kv, d, v, dtype):
             assert float((out[t].double() - want).norm()) < 2e-6 * float(want.norm()) + 2e-6 * float(s.norm()) / math.sqrt(d)
         assert float((S[i].double() - s).norm() / s.norm()) < 2e-6
         at += n
+
+
+@pytest.mark.parametrize("lens", [False, True])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("b,s,a", [(1, 1, 1), (2, 63, 2), (1, 64, 3), (2, 65, 1), (1, 127, 2), (3, 128, 1), (1, 130, 2), (2, 333, 4), (1, 1024, 16)])
+def test_attention_backward_head_dim_128(b, s, a, causal, lens):
+    """Lengths around the 64-query and 128-key tiles, causal, full and right-padded."""
+    qkv, go = _rand((b, s, a, 384), 1).requires_grad_(True), _rand((b, s, a, 128), 2)
+    n = torch.tensor([max(1, s - 37 * i) for i in range(b)], dtype=torch.int32, device="cuda") if lens else None
+    y = OF.attention_qkvpacked(qkv, causal=causal, scale=0.09, kv_lens=n)
+    y.backward(go)
+    x = qkv.detach().double().requires_grad_(True)
+    keep = torch.ones(b, 1, s, s, dtype=torch.bool, device="cuda")
+    keep = keep.tril() if causal else keep
+    if lens:
+        keep = keep & (torch.arange(s, device="cuda")[None, None, None] < n[:, None, None, None])
+    # a causal query always sees key 0, which every sequence has
+    _attend64(*(t.permute(0, 2, 1, 3) for t in x.split(128, -1)), 0.09, keep).permute(0, 2, 1, 3).backward(go.double())
+    for got, want in zip(qkv.grad.split(128, -1), x.grad.split(128, -1)):
+        # probabilities and their gradients pass through bf16, then the result does; where everything cancels (one key) the bf16 result's own scale
+        assert float((got.double() - want).norm()) < 2.0 ** -7 * float(want.norm()) + 2.0 ** -9 * float(go.norm()) * (s == 1)
