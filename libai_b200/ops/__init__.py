@@ -26,13 +26,19 @@ _SO_PATH = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__
 _LAUNCH_COUNT = 0
 
 
+# the process environment as ``os.environ`` keeps it (encoded): asked once per operator call, where ``os.environ.get`` costs 1 us
+_ENV = getattr(os.environ, "_data", os.environ)
+_IMPL_KEY = "LIBAI_B200_IMPL" if _ENV is os.environ else os.environ.encodekey("LIBAI_B200_IMPL")
+
+
 def so_path() -> str:
     return _SO_PATH
 
 
 def impl() -> str:
     """'native' (default) or 'ref' (``LIBAI_B200_IMPL=ref`` forces the PyTorch path on GPU)."""
-    return os.environ.get("LIBAI_B200_IMPL", "native")
+    v = _ENV.get(_IMPL_KEY)
+    return "native" if v is None else os.fsdecode(v)
 
 
 class _FastOps:

@@ -21,6 +21,28 @@ import torch.nn.functional as F
 from . import count_launch, load_ext, use_native
 from .. import ops
 
+def _plain_call() -> bool:
+    """False where an operator is transformed (vmap, jvp, …), differentiated forward or traced: those see PyTorch operators."""
+    return not (torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0 or torch.jit.is_tracing())
+
+
+class _NoGradContext:
+    """Stands in for the context of an autograd function whose backward will never run: keeps nothing."""
+
+    needs_input_grad = (False,) * 32
+
+    def save_for_backward(self, *tensors):
+        pass
+
+
+def _call(fn, *args):
+    """``fn.apply(*args)``; where no graph is recorded the forward alone (an ``apply`` costs ~10 us of host time, more than most
+    kernels of a generation step take)."""
+    if torch.is_grad_enabled() or not _plain_call():
+        return fn.apply(*args)
+    return fn.forward(_NoGradContext(), *args)
+
+
 # --------------------------------------------------------------------------------------
 # activations (reference math)
 # --------------------------------------------------------------------------------------
@@ -135,7 +157,7 @@ class _LinearFn(torch.autograd.Function):
         x2 = x.reshape(-1, x.shape[-1])
         if not x2.is_contiguous():
             x2 = x2.contiguous()
-        need_pre = act not in (None, "none") and (x.requires_grad or w.requires_grad)
+        need_pre = act not in (None, "none") and any(ctx.needs_input_grad[:2])
         y, pre = _linear_fwd_any(ext, x2, w, bias, _ACT_IDS[act], need_pre)
         ctx.act = act
         ctx.has_bias = bias is not None
@@ -176,7 +198,7 @@ class _LinearFn(torch.autograd.Function):
 def linear(x, w, bias=None, act: Optional[str] = None):
     """``act(x @ w.T + bias)``; ``w`` is ``[out, in]``."""
     if use_native(x, w) and _gemm_ok(x, w):
-        return _LinearFn.apply(x, w, bias, act)
+        return _call(_LinearFn, x, w, bias, act)
     y = F.linear(x, w.to(x.dtype) if w.dtype != x.dtype else w, None if bias is None else bias.to(x.dtype))
     return _act_ref(y, act)
 
@@ -193,7 +215,7 @@ class _MLPFn(torch.autograd.Function):
         x2 = x.reshape(-1, x.shape[-1])
         if not x2.is_contiguous():
             x2 = x2.contiguous()
-        h, pre = _linear_fwd_any(ext, x2, w1, b1, _ACT_IDS[act], True)
+        h, pre = _linear_fwd_any(ext, x2, w1, b1, _ACT_IDS[act], any(ctx.needs_input_grad))
         # with a residual, the second bias and the block's residual add ride in the epilogue of the second GEMM
         res2 = residual.reshape(-1, w2.shape[0]).contiguous() if residual is not None else None
         y, _ = _linear_fwd_any(ext, h, w2, b2, 0, False, res2)
@@ -255,8 +277,8 @@ def mlp(x, w1, b1, w2, act: str = "gelu", b2=None, residual=None):
     (without it the second bias is left to the fused bias+dropout+residual op)."""
     if use_native(x, w1) and _gemm_ok(x, w1) and _gemm_ok(x.new_empty(1, w1.shape[0]), w2):
         if residual is not None:
-            return _MLPFn.apply(x, w1, b1, w2, act, b2, residual)
-        return _MLPFn.apply(x, w1, b1, w2, act)
+            return _call(_MLPFn, x, w1, b1, w2, act, b2, residual)
+        return _call(_MLPFn, x, w1, b1, w2, act)
     y = linear(linear(x, w1, b1, act), w2, b2)
     return y if residual is None else y + residual
 
@@ -303,7 +325,7 @@ class _LinearResidualFn(torch.autograd.Function):
 def linear_bias_residual(x, w, bias, residual):
     """``x @ wᵀ + bias + residual`` (output projection of a block, dropout-free)."""
     if use_native(x, w) and _gemm_ok(x, w) and residual is not None and residual.dtype == torch.bfloat16:
-        return _LinearResidualFn.apply(x, w, bias, residual)
+        return _call(_LinearResidualFn, x, w, bias, residual)
     y = linear(x, w, bias)
     return y if residual is None else y + residual
 
@@ -362,13 +384,13 @@ class _LayerNormFn(torch.autograd.Function):
 def layer_norm_with_skip(x, weight, bias, eps: float = 1e-5):
     """``(layer_norm(x), x)`` where the second output carries the skip connection (see ``_LayerNormFn``)."""
     if use_native(x) and x.dtype in (torch.bfloat16, torch.float32) and weight is not None and x.requires_grad:
-        return _LayerNormFn.apply(x, weight, bias, eps, False, True)
+        return _call(_LayerNormFn, x, weight, bias, eps, False, True)
     return layer_norm(x, weight, bias, eps), x
 
 
 def layer_norm(x, weight, bias, eps: float = 1e-5):
     if use_native(x) and x.dtype in (torch.bfloat16, torch.float32) and weight is not None:
-        return _LayerNormFn.apply(x, weight, bias, eps, False)
+        return _call(_LayerNormFn, x, weight, bias, eps, False)
     w = None if weight is None else weight.float()
     b = None if bias is None else bias.float()
     return F.layer_norm(x.float(), (x.shape[-1],), w, b, eps).to(x.dtype)
@@ -376,7 +398,7 @@ def layer_norm(x, weight, bias, eps: float = 1e-5):
 
 def rms_norm(x, weight, eps: float = 1e-6):
     if use_native(x) and x.dtype in (torch.bfloat16, torch.float32):
-        return _LayerNormFn.apply(x, weight, None, eps, True)
+        return _call(_LayerNormFn, x, weight, None, eps, True)
     xf = x.float()
     y = xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + eps)
     return (y * weight.float()).to(x.dtype)
@@ -413,7 +435,7 @@ class _BiasActFn(torch.autograd.Function):
 def bias_act(x, bias, act: str = "gelu"):
     """``act(x + bias)`` (replaces ``fused_bias_add_gelu``)."""
     if use_native(x) and x.dtype == torch.bfloat16:
-        return _BiasActFn.apply(x, bias, act)
+        return _call(_BiasActFn, x, bias, act)
     y = x if bias is None else x + bias.to(x.dtype)
     return _act_ref(y, act)
 
@@ -474,10 +496,10 @@ def bias_dropout_add(x, bias, residual, p: float, training: bool, sharded=None):
     sharded over the tensor-parallel group (default: yes iff sequence parallelism is on), see :func:`tp_rng_salt`."""
     if use_native(x) and x.dtype == torch.bfloat16 and x.shape[-1] % 8 == 0:
         if p == 0.0 or not training:
-            return _BiasAddFn.apply(x, bias, residual)
+            return _call(_BiasAddFn, x, bias, residual)
         if sharded is None:
             sharded = _activations_token_sharded()
-        return _BiasDropoutAddFn.apply(x, bias, residual, float(p), tp_rng_salt(sharded))
+        return _call(_BiasDropoutAddFn, x, bias, residual, float(p), tp_rng_salt(sharded))
     y = x if bias is None else x + bias.to(x.dtype)
     y = F.dropout(y, p=p, training=training)
     return y if residual is None else residual + y
@@ -488,7 +510,7 @@ def dropout(x, p: float, training: bool, sharded: bool = False):
     if p == 0.0 or not training:
         return x
     if use_native(x) and x.dtype == torch.bfloat16 and x.shape[-1] % 8 == 0:
-        return _BiasDropoutAddFn.apply(x, None, None, float(p), tp_rng_salt(sharded))
+        return _call(_BiasDropoutAddFn, x, None, None, float(p), tp_rng_salt(sharded))
     return F.dropout(x, p=p, training=training)
 
 
@@ -615,11 +637,6 @@ class _FlashAttnPackedFn(torch.autograd.Function):
 
 
 # ---- attention with 32-bit probabilities (csrc/attention_split_sm100.cu) ----------------------------------------------
-def _plain_call() -> bool:
-    """False where an operator is transformed (vmap, jvp, …), differentiated forward or traced: those see PyTorch operators."""
-    return not (torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0 or torch.jit.is_tracing())
-
-
 def _rows_of_vectors(t) -> bool:
     """A view whose rows TMA can read: contiguous last dimension, every other stride and the base on 16 bytes."""
     return t.data_ptr() % 16 == 0 and t.stride(-1) == 1 and all(n == 1 or (st > 0 and st % 8 == 0) for n, st in zip(t.shape[:-1], t.stride()))
@@ -634,10 +651,10 @@ def _split_views(layout: str, ts):
     return ts
 
 
-def _mask_supported(mask, q, sk: int) -> bool:
-    full = (q.shape[0], q.shape[1], q.shape[2], sk)
-    return (mask.device == q.device and not mask.is_complex() and mask.dim() <= 4
-            and all(m in (1, n) for m, n in zip(reversed(mask.shape), reversed(full))))
+def _mask_supported(mask, q_sizes, device, sk: int) -> bool:
+    """``q_sizes``: ``(b, a, sq)``."""
+    return (mask.device == device and not mask.is_complex() and mask.dim() <= 4
+            and all(m in (1, n) for m, n in zip(reversed(mask.shape), (sk, q_sizes[2], q_sizes[1], q_sizes[0]))))
 
 
 def _pack_mask(ext, mask, q, sk: int, causal: bool):
@@ -646,16 +663,17 @@ def _pack_mask(ext, mask, q, sk: int, causal: bool):
     return ext.attn_mask_pack(m.expand(m.shape[0], m.shape[1], q.shape[2], sk), causal)
 
 
+def _split_sizes_ok(b, a, sq, sk, d, scale, causal) -> bool:
+    return (d % 8 == 0 and 8 <= d <= 64 and min(b, a, sq, sk) > 0 and max(a, b) <= 65535 and scale > 0 and (not causal or sk >= sq))
+
+
 def _split_supported(q, k, v, scale, causal, mask) -> bool:
     """Sizes and types of the kernels with 32-bit probabilities, from ``[b, a, s, d]`` views.  Other head dims stay with the flash
     kernels (64 / 128 without a mask: bf16 probabilities, as ever) or with the unfused form."""
-    if not (use_native(q) and q.dtype == k.dtype == v.dtype == torch.bfloat16 and q.dim() == k.dim() == 4 and k.shape == v.shape
-            and q.shape[:2] == k.shape[:2] and q.shape[-1] == k.shape[-1] and q.shape[-1] % 8 == 0 and 8 <= q.shape[-1] <= 64
-            and min(q.shape) > 0 and k.shape[2] > 0 and max(q.shape[:2]) <= 65535 and scale > 0 and (not causal or k.shape[2] >= q.shape[2])):
-        return False
-    if mask is not None and not _mask_supported(mask, q, k.shape[2]):
-        return False
-    return _plain_call()
+    return (use_native(q) and q.dtype == k.dtype == v.dtype == torch.bfloat16 and q.dim() == k.dim() == 4 and k.shape == v.shape
+            and q.shape[:2] == k.shape[:2] and q.shape[-1] == k.shape[-1]
+            and _split_sizes_ok(*q.shape[:3], k.shape[2], q.shape[3], scale, causal)
+            and (mask is None or _mask_supported(mask, q.shape[:3], q.device, k.shape[2])) and _plain_call())
 
 
 class _SplitAttnFn(torch.autograd.Function):
@@ -699,11 +717,15 @@ class _SplitAttnFn(torch.autograd.Function):
 def attention_packed(layout: str, ts, *, causal: bool, scale: float, mask=None, dropout_p: float = 0.0, training: bool = False):
     """Attention straight from packed projections, ``qkv`` ``([b, s, a, 3d],)`` or ``q_kv`` ``([b, s, a, d], [b, sk, a, 2d])``, with an
     optional dense 0/1 mask, → ``[b, s, a, d]``; ``None`` where the kernels do not apply (the caller slices and takes :func:`attention`)."""
-    if (dropout_p > 0.0 and training) or not all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in ts):
+    x, y = ts[0], ts[-1]
+    b, sq, a, d = x.shape
+    d = d // 3 if layout == "qkv" else d
+    if ((dropout_p > 0.0 and training) or not use_native(x) or not _split_sizes_ok(b, a, sq, y.shape[1], d, scale, causal)
+            or any(t.dtype != torch.bfloat16 or not t.is_contiguous() or t.data_ptr() % 16 for t in ts)
+            or (layout == "q_kv" and y.shape != (b, y.shape[1], a, 2 * d)) or (layout == "qkv" and x.shape[3] != 3 * d)
+            or (mask is not None and not _mask_supported(mask, (b, a, sq), x.device, y.shape[1])) or not _plain_call()):
         return None
-    if not _split_supported(*_split_views(layout, ts), scale, causal, mask):
-        return None
-    return _SplitAttnFn.apply(layout, causal, float(scale), mask, *ts)
+    return _call(_SplitAttnFn, layout, causal, float(scale), mask, *ts)
 
 
 def attention_cached(q, k_new, v_new, past_key, past_value, *, scale: float, mask=None, dropout_p: float = 0.0, training: bool = False):
@@ -716,7 +738,7 @@ def attention_cached(q, k_new, v_new, past_key, past_value, *, scale: float, mas
             or past_key.dim() != 4 or past_key.shape != past_value.shape or past_key.shape[:2] != q.shape[:2] or past_key.shape[3] != q.shape[3]
             or past_key.shape[2] == 0 or min(q.shape) == 0 or max(q.shape[:2]) > 65535 or q.shape[3] % 8 or q.shape[3] > 256
             or not all(_rows_of_vectors(t) for t in ts) or (torch.is_grad_enabled() and any(t.requires_grad for t in ts))
-            or (mask is not None and not _mask_supported(mask, q, past_key.shape[2] + 1)) or not _plain_call()):
+            or (mask is not None and not _mask_supported(mask, q.shape[:3], q.device, past_key.shape[2] + 1)) or not _plain_call()):
         return None
     ext = load_ext()
     words, fill = (None, None) if mask is None else _pack_mask(ext, mask, q, past_key.shape[2] + 1, False)
@@ -740,7 +762,7 @@ def attention_qkvpacked(qkv, *, causal: bool, scale: float, kv_lens=None, dropou
     of a right-padded batch (keys beyond it are masked inside the kernel); ``dropout_p`` > 0 in training drops
     attention probabilities inside the kernel (Philox, TP-rank salted)."""
     p = float(dropout_p) if training else 0.0
-    return _FlashAttnPackedFn.apply(qkv, causal, float(scale), kv_lens, p, alibi_slopes)
+    return _call(_FlashAttnPackedFn, qkv, causal, float(scale), kv_lens, p, alibi_slopes)
 
 
 def attention(q, k, v, *, causal: bool = False, scale: Optional[float] = None, mask=None, bias=None,
@@ -762,13 +784,13 @@ def attention(q, k, v, *, causal: bool = False, scale: Optional[float] = None, m
         and (bias is None or (bias.shape[-1] == k.shape[-2] and bias.shape[-2] == q.shape[-2]))
     ):
         # strided [b, a, s, d] views of the packed QKV projection are consumed directly (TMA strides)
-        return _FlashAttnFn.apply(q, k, v, causal, float(scale), bias, alibi_slopes,
+        return _call(_FlashAttnFn, q, k, v, causal, float(scale), bias, alibi_slopes,
                                   float(dropout_p) if training else 0.0, kv_lens)
     if (bias is None and alibi_slopes is None and kv_lens is None and not (dropout_p > 0.0 and training)
             and _split_supported(q, k, v, scale, causal, mask)):
         ts = [t if _rows_of_vectors(t) else t.contiguous() for t in (q, k, v)]
         if all(_rows_of_vectors(t) for t in ts):
-            return _SplitAttnFn.apply("q_k_v", causal, float(scale), mask, *ts)
+            return _call(_SplitAttnFn, "q_k_v", causal, float(scale), mask, *ts)
     if alibi_slopes is not None:
         sq, sk = q.shape[-2], k.shape[-2]
         rel = torch.arange(sk, device=q.device)[None, :] - torch.arange(sk - sq, sk, device=q.device)[:, None]
@@ -839,7 +861,7 @@ class _VocabParallelCE(torch.autograd.Function):
 def vocab_parallel_cross_entropy(logits, labels, vocab_start: int = 0, group=None):
     """logits ``[..., V/t]``, labels ``[...]`` (global ids) → per-token loss ``[...]`` (fp32)."""
     shp = labels.shape
-    out = _VocabParallelCE.apply(logits.reshape(-1, logits.shape[-1]), labels.reshape(-1), vocab_start, group)
+    out = _call(_VocabParallelCE, logits.reshape(-1, logits.shape[-1]), labels.reshape(-1), vocab_start, group)
     return out.view(shp)
 
 
@@ -883,7 +905,7 @@ def embedding(ids, table, vocab_start: int = 0):
     rows = table.shape[0]
     if (use_native(table) and table.dtype == torch.bfloat16 and table.dim() == 2 and table.shape[1] % 8 == 0
             and table.is_contiguous() and ids.dtype == torch.long):
-        return _EmbeddingFn.apply(ids, table, int(vocab_start))
+        return _call(_EmbeddingFn, ids, table, int(vocab_start))
     local = ids - vocab_start
     inside = (local >= 0) & (local < rows)
     out = F.embedding(local.clamp(0, rows - 1), table)
@@ -918,7 +940,7 @@ def apply_rotary(x, cos, sin):
     """x ``[b, a, s, d]``; cos/sin ``[s, d]`` (HF "rotate_half" convention; reference
     projects/Llama/llama.py:31-43)."""
     if use_native(x) and x.dtype == torch.bfloat16 and cos.dtype == torch.float32:
-        return _RopeFn.apply(x, cos, sin)
+        return _call(_RopeFn, x, cos, sin)
     c = cos[None, None].to(x.dtype)
     s = sin[None, None].to(x.dtype)
     return x * c + rotate_half(x) * s
@@ -950,7 +972,7 @@ def apply_rotary_qkv(qkv, cos, sin, pos_offset: int = 0):
     """qkv ``[b, s, a, 3d]`` (per-head ``[q|k|v]``); cos/sin fp32 ``[max_pos, d]``; token ``i`` of the
     sequence uses position ``i + pos_offset``."""
     if use_native(qkv) and qkv.dtype == torch.bfloat16 and cos.dtype == torch.float32 and qkv.is_contiguous():
-        return _RopeQKVFn.apply(qkv, cos, sin, int(pos_offset))
+        return _call(_RopeQKVFn, qkv, cos, sin, int(pos_offset))
     d = qkv.shape[-1] // 3
     s_len = qkv.shape[1]
     c = cos[pos_offset : pos_offset + s_len, None, :].to(qkv.dtype)
@@ -976,7 +998,7 @@ def fused_scale_mask_softmax(scores, mask=None, scale: float = 1.0, causal: bool
 def swiglu(gate, up):
     """``silu(gate) * up`` (reference projects/Llama/llama.py:111-113)."""
     if use_native(gate) and gate.dtype == torch.bfloat16:
-        return _SwigluFn.apply(gate, up)
+        return _call(_SwigluFn, gate, up)
     return F.silu(gate) * up
 
 

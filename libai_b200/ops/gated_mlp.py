@@ -19,6 +19,7 @@ from typing import Optional, Tuple
 import torch
 
 from libai_b200.ops import count_launch, load_ext
+from libai_b200.ops.functional import _call
 
 _ENABLED = os.environ.get("LIBAI_B200_FUSED_GATE_UP", "1") == "1"
 
@@ -159,7 +160,7 @@ class TPGatedMLPFused(torch.autograd.Function):
 
 
 def gated_mlp(x, wg, wu, wd):
-    return GatedMLPFn.apply(x, wg, wu, wd)
+    return _call(GatedMLPFn, x, wg, wu, wd)
 
 
 def tp_gated_mlp(x_shard, wg, wu, wd, residual, group):
