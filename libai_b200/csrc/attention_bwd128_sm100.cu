@@ -11,16 +11,18 @@
 //                                one tile that also goes through shared memory; drained one tile late into the fp32 accumulator by TMA reductions
 // TMEM: 2 x (Sᵀ 64 + dPᵀ 64) + dV 128 + dK 128 = 512 columns.  Shared memory: K, V 64 KB, three stages of Q, dO 96 KB and their
 // row statistics, two dSᵀ tiles 32 KB, dQ staging 32 KB.
-// Eight softmax warps: a thread owns one key and 32 queries of a tile; the row statistics (log-sum-exp, δ) arrive per tile with Q and
-// dO.  Four more warps drain dQ (with the softmax warps draining it, a tile's chain was 4060 cycles long, tensor pipe 36 %; the reductions
-// themselves cost nothing: the same time without them).  [1, 8192, 16, 128] causal 1317 -> 956 us, [1, 2048, 32, 128] 224 -> 172 us.
-// What is left is the tensor pipe's turnaround: five short groups of products per tile, 1.8 of 3.4 thousand cycles in issue.
+// Two groups of eight softmax warps, one per buffer: a thread owns one key and 32 queries of every other tile; the row statistics
+// (log-sum-exp, δ) arrive per tile with Q and dO.  Four more warps drain dQ.  One thread issues every product.
+// What bounds it is shared memory: per tile the products read 176 KB of operands, and loads, dSᵀ and the dQ boxes move 112 KB, 2300
+// cycles at 128 bytes of the 2600 that a tile takes.  [1, 8192, 16, 128] causal 1317 -> 743 us, [1, 2048, 32, 128] 224 -> 145 us.  On the way:
+// one warp waiting per product group and Sᵀ, dPᵀ behind the whole group before 950; one group of softmax warps 768; dQ added by the drain
+// warps themselves (32-bit reductions from registers, no boxes) 890; without the reductions altogether the time is the same.
 // Every wait on an mbarrier is bounded (attention_tc.cuh).
 #include "attention_tc.cuh"
 
 namespace lb {
 
-constexpr int B128_THREADS = 448;                    // TMA warp, MMA warp, 8 softmax warps, 4 warps that drain dQ
+constexpr int B128_THREADS = 704;                    // TMA warp, MMA warp, 2 x 8 softmax warps, 4 warps that drain dQ
 constexpr int B128_KV = 128 * 128 * 2, B128_Q = 64 * 128 * 2, B128_DS = 128 * 64 * 2, B128_BOX = 32 * 128, B128_STAT = 2 * 64 * 4;
 constexpr int B128_ST = 3;                            // Q / dO stages: with two a tile's loads waited for the products of the tile before last
 constexpr int B128_SMEM = 2 * B128_KV + 2 * B128_ST * B128_Q + 2 * B128_DS + 8 * B128_BOX + B128_ST * B128_STAT + 1024 + 256;
@@ -58,8 +60,10 @@ attn_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   uint64_t* pds_full = bars + 9;     // 2
   uint64_t* dq_full = bars + 11;     // 2
   uint64_t* dq_empty = bars + 13;    // 2
-  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 15);
-  volatile int* stop = reinterpret_cast<volatile int*>(bars + 16);
+  uint64_t* dp_full = bars + 15;     // 2
+  uint64_t* dv_done = bars + 17;     // 2
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 19);
+  volatile int* stop = reinterpret_cast<volatile int*>(bars + 20);
 
   const int warp_idx = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int head = blockIdx.y, batch = blockIdx.z, k0 = blockIdx.x * 128;
@@ -85,6 +89,8 @@ attn_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       mbar_init(&pds_full[i], 8);
       mbar_init(&dq_full[i], 1);
       mbar_init(&dq_empty[i], 4);
+      mbar_init(&dp_full[i], 1);
+      mbar_init(&dv_done[i], 1);
     }
     *stop = 0;
     fence_barrier_init();
@@ -96,6 +102,8 @@ attn_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
 
+  // phases are taken in order, so one that is there needs no look at *stop (30 cycles, up to six times per tile)
+  auto ready = [&](uint64_t* bar, uint32_t parity) { return mbar_try_wait(bar, parity) || tc_wait(bar, parity, stop); };
   if (warp_idx == 0) {
     if (elect_one()) {
       mbar_arrive_expect_tx(kv_full, 2 * B128_KV);
@@ -121,56 +129,56 @@ attn_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     constexpr uint32_t idesc_s = make_idesc_bf16(128, 64, false, false);    // K·Qᵀ, V·dOᵀ
     constexpr uint32_t idesc_t = make_idesc_bf16(128, 128, false, true);    // Pᵀ·dO, dSᵀ·Q (A from TMEM)
     constexpr uint32_t idesc_q = make_idesc_bf16(128, 64, true, true);      // Kᵀ·dSᵀ
-    const uint32_t k_addr = smem_u32(sK), v_addr = smem_u32(sV);
-    bool ok = __all_sync(0xffffffffu, tc_wait(kv_full, 0, stop));
+    const uint64_t dk_s = make_smem_desc_sw128(smem_u32(sK), 0, 1024), dv_s = make_smem_desc_sw128(smem_u32(sV), 0, 1024);
+    const uint64_t dk_t = make_smem_desc_sw128(smem_u32(sK), 128 * 128, 1024);
+    // A tile's scores overwrite the buffer of the tile before last.  Sᵀ waits for its dQᵀ to be drained and its dV product to have read
+    // Pᵀ, under its dK product; dPᵀ waits for that one, under Sᵀ: the tensor pipe stays fed over both waits.
     auto issue_s = [&](int it) {
       const int b = it & 1, st = it % B128_ST;
-      ok = __all_sync(0xffffffffu, ok && tc_wait(&q_full[st], (it / B128_ST) & 1, stop));
-      if (it >= 2) {      // the buffer's last tile: dQ has been drained, and the products have read P and dS
-        ok = __all_sync(0xffffffffu, ok && tc_wait(&dq_empty[b], ((it - 2) >> 1) & 1, stop));
-        ok = __all_sync(0xffffffffu, ok && tc_wait(&q_empty[(it - 2) % B128_ST], ((it - 2) / B128_ST) & 1, stop));
-      }
+      if (!ready(&q_full[st], (it / B128_ST) & 1)) return false;
+      if (it >= 2 && !(ready(&dq_empty[b], ((it - 2) >> 1) & 1) && ready(&dv_done[b], ((it - 2) >> 1) & 1))) return false;
       tc_fence_after_sync();
-      if (ok && elect_one()) {
-        const uint32_t q_addr = smem_u32(sQ + st * B128_Q), do_addr = smem_u32(sDO + st * B128_Q);
+      const uint64_t q_s = make_smem_desc_sw128(smem_u32(sQ + st * B128_Q), 0, 1024), do_s = make_smem_desc_sw128(smem_u32(sDO + st * B128_Q), 0, 1024);
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          umma_f16_ss(tmem_base + b * 128, make_smem_desc_sw128(k_addr + (kk / 4) * (128 * 128) + (kk % 4) * 32, 0, 1024),
-                      make_smem_desc_sw128(q_addr + (kk / 4) * (64 * 128) + (kk % 4) * 32, 0, 1024), idesc_s, kk > 0 ? 1u : 0u);
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          umma_f16_ss(tmem_base + b * 128 + 64, make_smem_desc_sw128(v_addr + (kk / 4) * (128 * 128) + (kk % 4) * 32, 0, 1024),
-                      make_smem_desc_sw128(do_addr + (kk / 4) * (64 * 128) + (kk % 4) * 32, 0, 1024), idesc_s, kk > 0 ? 1u : 0u);
-        umma_commit(&s_full[b]);
+      for (int kk = 0; kk < 8; ++kk)
+        umma_f16_ss(tmem_base + b * 128, dk_s + (((kk / 4) * (128 * 128) + (kk % 4) * 32) >> 4), q_s + (((kk / 4) * (64 * 128) + (kk % 4) * 32) >> 4),
+                    idesc_s, kk > 0 ? 1u : 0u);
+      umma_commit(&s_full[b]);
+      if (it >= 2) {
+        if (!ready(&q_empty[(it - 2) % B128_ST], ((it - 2) / B128_ST) & 1)) return false;
+        tc_fence_after_sync();
       }
-      __syncwarp();
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk)
+        umma_f16_ss(tmem_base + b * 128 + 64, dv_s + (((kk / 4) * (128 * 128) + (kk % 4) * 32) >> 4), do_s + (((kk / 4) * (64 * 128) + (kk % 4) * 32) >> 4),
+                    idesc_s, kk > 0 ? 1u : 0u);
+      umma_commit(&dp_full[b]);
+      return true;
     };
-    issue_s(0);
-    for (int it = 0; it < iters; ++it) {
-      const int b = it & 1, st = it % B128_ST;
-      if (it + 1 < iters) issue_s(it + 1);
-      ok = __all_sync(0xffffffffu, ok && tc_wait(&pds_full[b], (it >> 1) & 1, stop));
-      tc_fence_after_sync();
-      if (ok && elect_one()) {
-        const uint32_t q_addr = smem_u32(sQ + st * B128_Q), do_addr = smem_u32(sDO + st * B128_Q), ds_addr = smem_u32(sDS + b * B128_DS);
+    if (elect_one() && ready(kv_full, 0) && issue_s(0)) {
+      for (int it = 0; it < iters; ++it) {
+        const int b = it & 1, st = it % B128_ST;
+        if (it + 1 < iters && !issue_s(it + 1)) break;
+        if (!ready(&pds_full[b], (it >> 1) & 1)) break;
+        tc_fence_after_sync();
+        const uint64_t q_t = make_smem_desc_sw128(smem_u32(sQ + st * B128_Q), 64 * 128, 1024), do_t = make_smem_desc_sw128(smem_u32(sDO + st * B128_Q), 64 * 128, 1024);
+        const uint64_t ds_t = make_smem_desc_sw128(smem_u32(sDS + b * B128_DS), 128 * 128, 1024);
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)      // dQᵀ first: its drain is what the next but one tile waits for
-          umma_f16_ss(tmem_base + b * 128 + 32, make_smem_desc_sw128(k_addr + kk * 2048, 128 * 128, 1024),
-                      make_smem_desc_sw128(ds_addr + kk * 2048, 128 * 128, 1024), idesc_q, kk > 0 ? 1u : 0u);
+        for (int kk = 0; kk < 8; ++kk)      // dQᵀ first: its drain takes longest
+          umma_f16_ss(tmem_base + b * 128 + 32, dk_t + ((kk * 2048) >> 4), ds_t + ((kk * 2048) >> 4), idesc_q, kk > 0 ? 1u : 0u);
         umma_commit(&dq_full[b]);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
-          umma_f16_ts(tmem_base + DV_COL, tmem_base + b * 128 + kk * 8, make_smem_desc_sw128(do_addr + kk * 2048, 64 * 128, 1024), idesc_t,
-                      (it > 0 || kk > 0) ? 1u : 0u);
+          umma_f16_ts(tmem_base + DV_COL, tmem_base + b * 128 + kk * 8, do_t + ((kk * 2048) >> 4), idesc_t, (it > 0 || kk > 0) ? 1u : 0u);
+        umma_commit(&dv_done[b]);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
-          umma_f16_ts(tmem_base + DK_COL, tmem_base + b * 128 + 96 + kk * 8, make_smem_desc_sw128(q_addr + kk * 2048, 64 * 128, 1024), idesc_t,
-                      (it > 0 || kk > 0) ? 1u : 0u);
+          umma_f16_ts(tmem_base + DK_COL, tmem_base + b * 128 + 96 + kk * 8, q_t + ((kk * 2048) >> 4), idesc_t, (it > 0 || kk > 0) ? 1u : 0u);
         umma_commit(&q_empty[st]);          // Q, dO, Pᵀ, dSᵀ of this tile have been read
       }
-      __syncwarp();
     }
-  } else if (warp_idx >= 10) {
+    __syncwarp();
+  } else if (warp_idx >= 18) {
     // dQᵀ of every tile: thread = one of the 128 columns of dQ, 2 x 32 queries -> [32 queries x 32 floats] boxes (128-byte rows, swizzled) -> reduction
     const int quad = warp_idx % 4;
     const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
@@ -211,81 +219,104 @@ attn_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     if (lane == 0) tma_store_wait<0>();
     __syncwarp();
   } else {
-    const int quad = warp_idx % 4, half = (warp_idx - 2) / 4;        // TMEM lanes of this warp; its 32 of the tile's 64 queries
+    // TMEM lanes of this warp; its 32 of the tile's 64 queries; the buffer whose tiles it takes
+    const int quad = warp_idx % 4, half = (warp_idx - 2) / 4 % 2, b = (warp_idx - 2) / 8;
     const int r = quad * 32 + lane, k_idx = k0 + r;
     const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
-    for (int it = 0; it < iters; ++it) {
-      const int b = it & 1, st = it % B128_ST, q0 = (i_begin + it) * 64;
+    for (int it = b; it < iters; it += 2) {
+      const int st = it % B128_ST, q0 = (i_begin + it) * 64;
       const bool edge = (p.causal && q0 < k0 + 127) || q0 + 64 > p.S || k0 + 128 > kv_len;
       // queries [q_lo, q_hi) of this half see key k_idx
       const int q_lo = (k_idx < kv_len ? (p.causal ? k_idx : 0) : p.S) - q0 - half * 32, q_hi = p.S - q0 - half * 32;
-      tc_wait(&q_full[st], (it / B128_ST) & 1, stop);  // the tile's statistics
-      tc_wait(&s_full[b], (it >> 1) & 1, stop);
+      ready(&q_full[st], (it / B128_ST) & 1);          // the tile's statistics
+      ready(&s_full[b], (it >> 1) & 1);
       __syncwarp();
-      tc_fence_after_sync();
-      uint32_t ts[32], td[32];
-      tmem_ld_32x32b_x32(tmem_base + lane_off + b * 128 + half * 32, ts);
-      tmem_ld_32x32b_x32(tmem_base + lane_off + b * 128 + 64 + half * 32, td);
-      tmem_ld_wait();
-      tc_fence_before_sync();
-      tc_pair_sync(quad);                              // both halves hold their columns: Pᵀ and dSᵀ may overwrite them
       tc_fence_after_sync();
       const float4* lse4 = reinterpret_cast<const float4*>(sStat + st * 128 + half * 32);
       const float4* del4 = reinterpret_cast<const float4*>(sStat + st * 128 + 64 + half * 32);
-      uint32_t pp[16], dd[16];
-      auto softmax = [&](auto edge_tag) {
+      uint32_t pk[16];
+      uint32_t pv[32];
+      tmem_ld_32x32b_x32(tmem_base + lane_off + b * 128 + half * 32, pv);
+      tmem_ld_wait();
+      auto exps = [&](auto edge_tag) {
         constexpr bool EDGE = decltype(edge_tag)::value;
 #pragma unroll
         for (int v = 0; v < 8; ++v) {
-          const float4 l4 = lse4[v], d4 = del4[v];
-          const float ls[4] = {l4.x, l4.y, l4.z, l4.w}, de[4] = {d4.x, d4.y, d4.z, d4.w};
-          float pv[4], dv[4];
+          const float4 l4 = lse4[v];
+          const float ls[4] = {l4.x, l4.y, l4.z, l4.w};
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const int i = 4 * v + e;
-            pv[e] = fast_exp2(fmaf(__uint_as_float(ts[i]), p.scale_log2, -ls[e]));
-            if constexpr (EDGE) pv[e] = (i >= q_lo && i < q_hi) ? pv[e] : 0.f;
-            dv[e] = pv[e] * fmaf(__uint_as_float(td[i]), p.scale, -de[e]);
-            if constexpr (EDGE) dv[e] = (i >= q_lo && i < q_hi) ? dv[e] : 0.f;
+            float x = fast_exp2(fmaf(__uint_as_float(pv[i]), p.scale_log2, -ls[e]));
+            if constexpr (EDGE) x = (i >= q_lo && i < q_hi) ? x : 0.f;
+            pv[i] = __float_as_uint(x);
           }
-          pp[2 * v] = pack_bf16(pv[0], pv[1]);
-          pp[2 * v + 1] = pack_bf16(pv[2], pv[3]);
-          dd[2 * v] = pack_bf16(dv[0], dv[1]);
-          dd[2 * v + 1] = pack_bf16(dv[2], dv[3]);
+          pk[2 * v] = pack_bf16(__uint_as_float(pv[4 * v]), __uint_as_float(pv[4 * v + 1]));
+          pk[2 * v + 1] = pack_bf16(__uint_as_float(pv[4 * v + 2]), __uint_as_float(pv[4 * v + 3]));
         }
       };
-      if (edge) softmax(std::true_type{}); else softmax(std::false_type{});
-      tmem_st_32x32b_x16(tmem_base + lane_off + b * 128 + half * 16, pp);
-      tmem_st_32x32b_x16(tmem_base + lane_off + b * 128 + 96 + half * 16, dd);
+      if (edge) exps(std::true_type{}); else exps(std::false_type{});
+      tc_fence_before_sync();
+      tc_pair_sync(b * 4 + quad);                      // Pᵀ of both halves overwrites the first half's scores
+      tc_fence_after_sync();
+      tmem_st_32x32b_x16(tmem_base + lane_off + b * 128 + half * 16, pk);
+      ready(&dp_full[b], (it >> 1) & 1);
+      __syncwarp();
+      tc_fence_after_sync();
+      auto grads = [&](auto edge_tag) {
+        constexpr bool EDGE = decltype(edge_tag)::value;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t td[16];
+          tmem_ld_32x32b_x16(tmem_base + lane_off + b * 128 + 64 + half * 32 + c * 16, td);
+          tmem_ld_wait();
+#pragma unroll
+          for (int v = 4 * c; v < 4 * c + 4; ++v) {
+            const float4 d4 = del4[v];
+            const float de[4] = {d4.x, d4.y, d4.z, d4.w};
+            float dv[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const int i = 4 * v + e;
+              dv[e] = __uint_as_float(pv[i]) * fmaf(__uint_as_float(td[i - 16 * c]), p.scale, -de[e]);
+              if constexpr (EDGE) dv[e] = (i >= q_lo && i < q_hi) ? dv[e] : 0.f;
+            }
+            pk[2 * v] = pack_bf16(dv[0], dv[1]);
+            pk[2 * v + 1] = pack_bf16(dv[2], dv[3]);
+          }
+        }
+      };
+      if (edge) grads(std::true_type{}); else grads(std::false_type{});
+      tc_fence_before_sync();
+      tc_pair_sync(b * 4 + quad);                      // dSᵀ of both halves overwrites the second half's dPᵀ
+      tc_fence_after_sync();
+      tmem_st_32x32b_x16(tmem_base + lane_off + b * 128 + 96 + half * 16, pk);
       uint8_t* drow = sDS + b * B128_DS + r * 128;
 #pragma unroll
       for (int v = 0; v < 4; ++v)
-        *reinterpret_cast<uint4*>(drow + (((half * 4 + v) ^ (r & 7)) << 4)) = make_uint4(dd[4 * v], dd[4 * v + 1], dd[4 * v + 2], dd[4 * v + 3]);
+        *reinterpret_cast<uint4*>(drow + (((half * 4 + v) ^ (r & 7)) << 4)) = make_uint4(pk[4 * v], pk[4 * v + 1], pk[4 * v + 2], pk[4 * v + 3]);
       tmem_st_wait();
       tc_fence_before_sync();
       fence_proxy_async();
       __syncwarp();
       if (lane == 0) mbar_arrive(&pds_full[b]);
     }
-    // ---- dV / dK: thread = key row, this half's 64 columns
+    // ---- dV (first group) / dK (second): thread = key row, this half's 64 columns
     tc_wait(&q_empty[(iters - 1) % B128_ST], ((iters - 1) / B128_ST) & 1, stop);
     __syncwarp();
     tc_fence_after_sync();
+    __nv_bfloat16* row = (b == 0 ? p.dv : p.dk) + batch * p.g_strides[0] + head * p.g_strides[1] + static_cast<long>(k_idx) * p.g_strides[2] + half * 64;
 #pragma unroll
-    for (int which = 0; which < 2; ++which) {
-      __nv_bfloat16* row = (which == 0 ? p.dv : p.dk) + batch * p.g_strides[0] + head * p.g_strides[1] + static_cast<long>(k_idx) * p.g_strides[2] + half * 64;
+    for (int c = 0; c < 2; ++c) {
+      uint32_t t[32];
+      tmem_ld_32x32b_x32(tmem_base + lane_off + (b == 0 ? DV_COL : DK_COL) + half * 64 + c * 32, t);
+      tmem_ld_wait();
+      if (k_idx < p.S) {
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uint32_t t[32];
-        tmem_ld_32x32b_x32(tmem_base + lane_off + (which == 0 ? DV_COL : DK_COL) + half * 64 + c * 32, t);
-        tmem_ld_wait();
-        if (k_idx < p.S) {
-#pragma unroll
-          for (int i = 0; i < 32; i += 8)
-            *reinterpret_cast<uint4*>(row + c * 32 + i) = make_uint4(
-                pack_bf16(__uint_as_float(t[i]), __uint_as_float(t[i + 1])), pack_bf16(__uint_as_float(t[i + 2]), __uint_as_float(t[i + 3])),
-                pack_bf16(__uint_as_float(t[i + 4]), __uint_as_float(t[i + 5])), pack_bf16(__uint_as_float(t[i + 6]), __uint_as_float(t[i + 7])));
-        }
+        for (int i = 0; i < 32; i += 8)
+          *reinterpret_cast<uint4*>(row + c * 32 + i) = make_uint4(
+              pack_bf16(__uint_as_float(t[i]), __uint_as_float(t[i + 1])), pack_bf16(__uint_as_float(t[i + 2]), __uint_as_float(t[i + 3])),
+              pack_bf16(__uint_as_float(t[i + 4]), __uint_as_float(t[i + 5])), pack_bf16(__uint_as_float(t[i + 6]), __uint_as_float(t[i + 7])));
       }
     }
   }

@@ -17,11 +17,8 @@ LB_DEVICE bool tc_wait(uint64_t* bar, uint32_t parity, volatile int* stop) {
   *stop = 1;
   return false;
 }
-LB_DEVICE void tc_pair_sync(int quad) {       // the two warps that own the same TMEM lane quadrant
-  if (quad == 0) asm volatile("bar.sync 1, 64;\n" ::: "memory");
-  else if (quad == 1) asm volatile("bar.sync 2, 64;\n" ::: "memory");
-  else if (quad == 2) asm volatile("bar.sync 3, 64;\n" ::: "memory");
-  else asm volatile("bar.sync 4, 64;\n" ::: "memory");
+LB_DEVICE void tc_pair_sync(int quad) {       // the two warps that own the same TMEM lane quadrant (of group quad / 4, where there are several)
+  asm volatile("bar.sync %0, 64;\n" ::"r"(quad + 1) : "memory");
 }
 
 }  // namespace lb
