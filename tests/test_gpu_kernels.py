@@ -252,3 +252,18 @@ def test_attention_backward_head_dim_128(b, s, a, causal, lens):
     for got, want in zip(qkv.grad.split(128, -1), x.grad.split(128, -1)):
         # probabilities and their gradients pass through bf16, then the result does; where everything cancels (one key) the bf16 result's own scale
         assert float((got.double() - want).norm()) < 2.0 ** -7 * float(want.norm()) + 2.0 ** -9 * float(go.norm()) * (s == 1)
+
+
+@pytest.mark.parametrize("M", [40, 129, 1100, 2500])
+@pytest.mark.parametrize("layout", [0, 1])
+def test_gemm_tile_order_in_bands(M, layout):
+    """B beyond 24 MB: bands of row blocks, a last band of one block, ragged edges.  Whole numbers below 256: exact in bf16."""
+    N, K = (24600, 520) if layout == 0 else (264, 49160)
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x = torch.randint(-1, 2, (M, K), generator=g, device="cuda").to(BF16)
+    w = torch.randint(-1, 2, (N, K) if layout == 0 else (K, N), generator=g, device="cuda").to(BF16)
+    if layout == 1:
+        x[:, 512:-8] = 0        # sums stay below 256
+    want = x.float() @ (w.float().t() if layout == 0 else w.float())
+    assert want.abs().max() < 256
+    assert torch.equal(OF.load_ext().gemm(x, w, layout, None, None, False, BF16).float(), want)
