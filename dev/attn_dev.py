@@ -81,7 +81,7 @@ def main():
     od, lsed, std = ext.attn_fwd(q, k, v, True, 0.125, None, None, None, 0.1, 0)
     out["speed"]["fwd_ms_dropout0.1"] = timeit(lambda: ext.attn_fwd(q, k, v, True, 0.125, None, None, None, 0.1, 0))
     out["speed"]["bwd_ms_dropout0.1"] = timeit(lambda: ext.attn_bwd(go, q, k, v, od, lsed, True, 0.125, None, None, None, None, 0.1, std))
-    # Llama-like shape (head dim 128: the sequential backward kernel)
+    # Llama-like shape (head dim 128)
     q, k, v = inputs(2, 8, 2048, 128)
     go = torch.randn(2, 2048, 8, 128, device="cuda").bfloat16().permute(0, 2, 1, 3)
     sc = 1.0 / math.sqrt(128)
