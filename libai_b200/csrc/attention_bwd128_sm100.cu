@@ -318,6 +318,7 @@ attn_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
               pack_bf16(__uint_as_float(t[i]), __uint_as_float(t[i + 1])), pack_bf16(__uint_as_float(t[i + 2]), __uint_as_float(t[i + 3])),
               pack_bf16(__uint_as_float(t[i + 4]), __uint_as_float(t[i + 5])), pack_bf16(__uint_as_float(t[i + 6]), __uint_as_float(t[i + 7])));
       }
+      __syncwarp();                                    // whole warps read tensor memory
     }
   }
   tc_fence_before_sync();

@@ -142,6 +142,7 @@ attn_decode_kernel(const DecodeParams p) {
     c_acc[c] = O;
     if (c == 0) { c_ml[0] = M; c_ml[1] = L; }
   }
+  __syncwarp();                                                   // up to 16 columns are merged by a part of warp 0: the barriers take whole warps
   if (nsplit > 1) {
     cluster_sync_all();
     if (split == 0) {
@@ -163,6 +164,7 @@ attn_decode_kernel(const DecodeParams p) {
         if (c < p.d) p.o[(static_cast<size_t>(batch) * p.A + head) * p.d + c] = __float2bfloat16(O / L);
       }
     }
+    __syncwarp();
     cluster_sync_all();                                           // nobody leaves while its shared memory is read
   } else {
     __syncthreads();

@@ -173,6 +173,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       *reinterpret_cast<uint2*>(p.out + o) = make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
     }
   }
+  __syncwarp();                                    // lanes behind column N left the loop early; the cluster's barrier takes whole warps
   if constexpr (RANKS > 1) cluster_sync_all();     // nobody leaves while its partial sums are read
   tc_fence_before_sync();
   __syncthreads();

@@ -1,10 +1,12 @@
 """GPU tier: single kernels of the training path at the sizes where a tile, a remainder or a wait can go wrong, against plain PyTorch."""
+import ctypes
 import math
 
 import pytest
 import torch
 
 from libai_b200.ops import functional as OF
+from libai_b200.ops import so_path
 
 pytestmark = pytest.mark.gpu
 BF16 = torch.bfloat16
@@ -161,7 +163,8 @@ def test_attention_gradients_can_be_differentiated_again():
 
 
 @pytest.mark.parametrize("mask", [None, "bool", "int64"])
-@pytest.mark.parametrize("b,a,past,d", [(1, 1, 1, 8), (8, 16, 511, 64), (2, 3, 63, 24), (3, 2, 1000, 128), (1, 4, 64, 48), (2, 1, 300, 256), (5, 7, 129, 16)])
+@pytest.mark.parametrize("b,a,past,d", [(1, 1, 1, 8), (8, 16, 511, 64), (2, 3, 63, 24), (3, 2, 1000, 128), (1, 4, 64, 48), (2, 1, 300, 256), (5, 7, 129, 16),
+                                        (1, 2, 600, 8), (2, 1, 1030, 16)])
 def test_attention_against_a_cache(b, a, past, d, mask):
     """One new token: context and grown caches, caches as strided views, with and without masked keys, every split over a cluster."""
     qkv = _rand((b, 1, a, 3 * d), 1)
@@ -195,6 +198,32 @@ def test_linear_of_few_rows(m, n, k):
         assert torch.equal(ext.linear_fwd(x, w, b, act, False)[0], y)
     assert near(ext.linear_bias_residual(x, w, b, r), z + r.double())
     assert near(ext.linear_fwd(x, w, None, OF.ACT_NONE, False)[0], z - b.double())
+
+
+@pytest.mark.parametrize("ranks", [1, 2, 4, 8])
+@pytest.mark.parametrize("nt", [16, 32, 64, 128])
+@pytest.mark.parametrize("n,k", [(300, 200), (136, 1032), (1032, 520)])
+def test_linear_of_few_rows_every_tile_and_cluster(nt, ranks, n, k):
+    """Every instantiation, whatever the rule picks: two row tiles with the last one ragged, column tiles that end inside a warp's
+    four columns per lane, clusters some of whose CTAs have no k-block; the same bits in a second run."""
+    m = nt + nt // 2 + 1
+    x, w, b, r = _rand((m, k), 1), _rand((n, k), 2, k ** -0.5), _rand((n,), 3), _rand((m, n), 4)
+    lib = ctypes.CDLL(so_path())
+    ptr = lambda t: ctypes.c_void_p(0 if t is None else t.data_ptr())
+
+    def call(act, pre, residual):
+        y = torch.full((m, n), float("nan"), device="cuda", dtype=BF16)
+        rc = lib.lb_gemm_small(ptr(x), ptr(w), ptr(y), m, n, k, k, k, n, ptr(b), act, ptr(pre), ptr(residual), nt, ranks,
+                               ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+        assert rc == 0
+        return y
+
+    z = x.double() @ w.double().t() + b.double()
+    near = lambda got, want: float((got.double() - want).norm() / want.norm()) < 2.0 ** -8       # one rounding of an fp32 sum
+    pre = torch.empty(m, n, device="cuda", dtype=BF16)
+    y = call(OF.ACT_GELU, pre, None)
+    assert near(pre, z) and near(y, torch.nn.functional.gelu(z)) and torch.equal(y, call(OF.ACT_GELU, pre, None))
+    assert near(call(OF.ACT_NONE, None, r), z + r.double())
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, BF16])
