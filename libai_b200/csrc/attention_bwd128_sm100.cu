@@ -228,8 +228,10 @@ attn_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       const bool edge = (p.causal && q0 < k0 + 127) || q0 + 64 > p.S || k0 + 128 > kv_len;
       // queries [q_lo, q_hi) of this half see key k_idx
       const int q_lo = (k_idx < kv_len ? (p.causal ? k_idx : 0) : p.S) - q0 - half * 32, q_hi = p.S - q0 - half * 32;
-      ready(&q_full[st], (it / B128_ST) & 1);          // the tile's statistics
+      // The tile's statistics: this group sees a stage's phases two apart (tiles it, it + 6), whose parity is the same, so q_full alone
+      // may answer for the phase before last.  Behind s_full it cannot: Sᵀ was issued after q_full's phase had come.
       ready(&s_full[b], (it >> 1) & 1);
+      ready(&q_full[st], (it / B128_ST) & 1);
       __syncwarp();
       tc_fence_after_sync();
       const float4* lse4 = reinterpret_cast<const float4*>(sStat + st * 128 + half * 32);

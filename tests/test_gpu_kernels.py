@@ -283,6 +283,17 @@ def test_attention_backward_head_dim_128(b, s, a, causal, lens):
         assert float((got.double() - want).norm()) < 2.0 ** -7 * float(want.norm()) + 2.0 ** -9 * float(go.norm()) * (s == 1)
 
 
+@pytest.mark.parametrize("causal", [False, True])
+def test_attention_backward_head_dim_128_repeats(causal):
+    """dK and dV are sums in a fixed order inside one CTA: the same bits every time (a tile must not be taken with the row statistics
+    of an earlier one: 18 query tiles go through three stages and two groups of warps)."""
+    qkv, go = _rand((4, 1100, 16, 384), 1).requires_grad_(True), _rand((4, 1100, 16, 128), 2)
+    y = OF.attention_qkvpacked(qkv, causal=causal, scale=128 ** -0.5)
+    first = torch.autograd.grad(y, qkv, go, retain_graph=True)[0][..., 128:]
+    for _ in range(4):
+        assert torch.equal(torch.autograd.grad(y, qkv, go, retain_graph=True)[0][..., 128:], first)
+
+
 @pytest.mark.parametrize("M", [40, 129, 1100, 2500])
 @pytest.mark.parametrize("layout", [0, 1])
 def test_gemm_tile_order_in_bands(M, layout):
