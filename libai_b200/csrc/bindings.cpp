@@ -849,10 +849,10 @@ struct SplitMask {
   const float* fill = nullptr;
   long b = 0, a = 0;
 };
-SplitMask split_mask(const c10::optional<Tensor>& words, const c10::optional<Tensor>& fill, int B, int A, int Sq, int Sk) {
+SplitMask split_mask(const c10::optional<Tensor>& words, const c10::optional<Tensor>& fill, c10::Device device, int B, int A, int Sq, int Sk) {
   SplitMask m;
   if (!(words.has_value() && words->defined())) return m;
-  TORCH_CHECK(fill.has_value() && fill->defined() && words->is_cuda() && words->scalar_type() == at::kInt && words->is_contiguous() &&
+  TORCH_CHECK(fill.has_value() && fill->defined() && words->device() == device && fill->device() == device && words->scalar_type() == at::kInt && words->is_contiguous() &&
                   fill->scalar_type() == at::kFloat && fill->is_contiguous() && words->dim() == 4 && words->size(2) == Sq &&
                   words->size(3) == (Sk + 127) / 128 * 4 && (words->size(0) == 1 || words->size(0) == B) &&
                   (words->size(1) == 1 || words->size(1) == A) && fill->numel() == words->size(0) * words->size(1) * Sq,
@@ -863,8 +863,9 @@ SplitMask split_mask(const c10::optional<Tensor>& words, const c10::optional<Ten
   m.b = words->size(0) == 1 ? 0 : words->size(1) * Sq;
   return m;
 }
-void split_strides(const Tensor& t, long (&st)[3]) {
-  TORCH_CHECK(t.is_cuda() && t.dim() == 4 && t.scalar_type() == at::kBFloat16 && t.stride(3) == 1, "split attention: bf16 [B, A, S, d] views with contiguous d");
+void split_strides(const Tensor& t, c10::Device device, long (&st)[3]) {
+  TORCH_CHECK(t.is_cuda() && t.device() == device, "split attention: every tensor on the device of the queries");
+  TORCH_CHECK(t.dim() == 4 && t.scalar_type() == at::kBFloat16 && t.stride(3) == 1, "split attention: bf16 [B, A, S, d] views with contiguous d");
   // the stride of a dimension of one element is free: give the tensor map a legal one
   int64_t full = t.size(3);
   for (int i = 2; i >= 0; --i) {
@@ -882,12 +883,12 @@ std::tuple<Tensor, Tensor, Tensor> attn_split_fwd(const Tensor& q, const Tensor&
                                                   const c10::optional<Tensor>& words, const c10::optional<Tensor>& fill, bool train) {
   c10::cuda::CUDAGuard guard(q.device());
   long qs[3], ks[3], vs[3];
-  split_strides(q, qs);
-  split_strides(k, ks);
-  split_strides(v, vs);
+  split_strides(q, q.device(), qs);
+  split_strides(k, q.device(), ks);
+  split_strides(v, q.device(), vs);
   const int B = (int)q.size(0), A = (int)q.size(1), Sq = (int)q.size(2), Sk = (int)k.size(2), d = (int)q.size(3);
   TORCH_CHECK(k.sizes() == v.sizes() && k.size(0) == B && k.size(1) == A && k.size(3) == d, "split attention: shapes");
-  const SplitMask m = split_mask(words, fill, B, A, Sq, Sk);
+  const SplitMask m = split_mask(words, fill, q.device(), B, A, Sq, Sk);
   Tensor o = at::empty({B, Sq, A, d}, q.options());
   Tensor lo = train ? at::empty({B, Sq, A, d}, q.options()) : at::empty({0}, q.options());
   Tensor lse = at::empty({B, A, Sq}, q.options().dtype(at::kFloat));
@@ -912,14 +913,15 @@ void attn_split_bwd(const Tensor& dout, const Tensor& q, const Tensor& k, const 
                   o.is_contiguous() && o_lo.is_contiguous() && o.numel() == q.numel() && o_lo.numel() == q.numel(),
               "split attention: shapes");
   long qs[3], ks[3], vs[3], gs[3], dqs[3], dks[3], dvs[3];
-  split_strides(q, qs);
-  split_strides(k, ks);
-  split_strides(v, vs);
-  split_strides(g, gs);
-  split_strides(dq, dqs);
-  split_strides(dk, dks);
-  split_strides(dv, dvs);
-  const SplitMask m = split_mask(words, fill, B, A, Sq, Sk);
+  split_strides(q, q.device(), qs);
+  split_strides(k, q.device(), ks);
+  split_strides(v, q.device(), vs);
+  split_strides(g, q.device(), gs);
+  split_strides(dq, q.device(), dqs);
+  split_strides(dk, q.device(), dks);
+  split_strides(dv, q.device(), dvs);
+  TORCH_CHECK(o.device() == q.device() && o_lo.device() == q.device() && lse.device() == q.device(), "split attention: saved tensors on the device of the queries");
+  const SplitMask m = split_mask(words, fill, q.device(), B, A, Sq, Sk);
   auto f32 = q.options().dtype(at::kFloat);
   Tensor delta = at::empty({B, A, Sq}, f32), acc = at::empty({B, A, Sq, d}, f32);      // cleared by the delta kernel
   check(lb_attn_split_bwd(g.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), o_lo.data_ptr(), lse.data_ptr<float>(), dq.data_ptr(),
@@ -935,11 +937,11 @@ std::tuple<Tensor, Tensor, Tensor> attn_decode(const Tensor& q, const Tensor& k_
   c10::cuda::CUDAGuard guard(q.device());
   long st[5][3];
   int i = 0;
-  for (const Tensor* t : {&q, &k_new, &v_new, &k_past, &v_past}) split_strides(*t, st[i++]);
+  for (const Tensor* t : {&q, &k_new, &v_new, &k_past, &v_past}) split_strides(*t, q.device(), st[i++]);
   const int B = (int)q.size(0), A = (int)q.size(1), d = (int)q.size(3), past = (int)k_past.size(2);
   TORCH_CHECK(q.size(2) == 1 && k_new.sizes() == q.sizes() && v_new.sizes() == q.sizes() && k_past.sizes() == v_past.sizes() && k_past.size(0) == B &&
                   k_past.size(1) == A && k_past.size(3) == d, "attn_decode: shapes");
-  const SplitMask m = split_mask(words, fill, B, A, 1, past + 1);
+  const SplitMask m = split_mask(words, fill, q.device(), B, A, 1, past + 1);
   Tensor o = at::empty({B, 1, A, d}, q.options());
   Tensor k = at::empty({B, A, past + 1, d}, q.options()), v = at::empty({B, A, past + 1, d}, q.options());
   check(lb_attn_decode(q.data_ptr(), k_new.data_ptr(), v_new.data_ptr(), k_past.data_ptr(), v_past.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(),

@@ -1,4 +1,5 @@
 """Reference (CPU) paths of the fused functional ops agree with their unfused compositions."""
+import pytest
 import torch
 
 from libai_b200.ops import functional as OF
@@ -24,3 +25,29 @@ def test_layer_norm_with_skip_reference_path():
     assert torch.allclose(ln, torch.nn.functional.layer_norm(x, (10,), g, b, 1e-5), atol=1e-5)
     (ln.sum() + (skip * 2).sum()).backward()
     assert x.grad is not None and torch.isfinite(x.grad).all()
+
+
+@pytest.mark.parametrize("moved", range(5))
+def test_attention_kernels_are_not_given_tensors_of_another_device(moved, monkeypatch):
+    """A cache, or keys and values, held on another device than the queries: the kernels are not taken (no launch here: the support
+    checks are asked, the extension is a stand-in that records a call)."""
+
+    class Reached(Exception):
+        pass
+
+    class Ext:
+        def __getattr__(self, name):
+            raise Reached(name)
+
+    monkeypatch.setattr(OF, "use_native", lambda *t: True)
+    monkeypatch.setattr(OF, "load_ext", lambda *a, **k: Ext())
+    at = lambda i, *shape: torch.zeros(*shape, dtype=torch.bfloat16, device="meta" if i == moved else "cpu")
+    new, past = (2, 3, 1, 32), (2, 3, 7, 32)
+    with pytest.raises(Reached):
+        OF.attention_cached(*(at(-1, *s) for s in (new, new, new, past, past)), scale=0.1)
+    assert OF.attention_cached(*(at(i, *s) for i, s in enumerate((new, new, new, past, past))), scale=0.1) is None
+    if moved < 3:
+        assert OF._split_supported(*(at(-1, *past) for _ in range(3)), 0.1, False, None)
+        assert not OF._split_supported(*(at(i, *past) for i in range(3)), 0.1, False, None)
+    if moved < 2:
+        assert OF.attention_packed("q_kv", (at(0, 2, 7, 3, 32), at(1, 2, 9, 3, 64)), causal=False, scale=0.1) is None
