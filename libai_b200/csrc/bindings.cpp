@@ -25,7 +25,7 @@ int lb_gemm_fp8(const void* xq, const void* wq, void* out, int M, int N, int K, 
                 const void* residual, const float* deq_x, const float* deq_w, cudaStream_t s);
 int lb_quant_e4m3(const void* x, void* q, void* amax_scratch, float* deq, long n, cudaStream_t s);
 int lb_norm_bwd_workspace_rows(int rows, int H);
-int lb_norm_bwd_supports_gadd(int H, int dtype, const void* gy, const void* x, const void* gamma, const void* gadd);
+int lb_norm_bwd_supports_gadd(int H, int dtype, const void* gy, const void* x, const void* gamma, const void* gx, const void* gadd);
 int lb_norm_bwd(const void* gy, const void* x, const void* gamma, const float* mean, const float* rstd, void* gx,
                 float* dgamma, float* dbeta, float* workspace, int rows, int H, int rms, int dtype, int wdtype,
                 int accumulate, const void* gadd, cudaStream_t s);
@@ -515,7 +515,7 @@ std::tuple<Tensor, Tensor, Tensor> norm_bwd(const Tensor& gy, const Tensor& x, c
   // optional gradient of the skip connection around this norm: added to gx inside the kernel when supported
   const bool has_add = gadd.has_value() && gadd->defined();
   const bool fuse_add = has_add && gadd->is_contiguous() && gadd->scalar_type() == x.scalar_type() &&
-                        lb_norm_bwd_supports_gadd(H, dtype_code(x), gy.data_ptr(), x.data_ptr(), gamma.data_ptr(), gadd->data_ptr());
+                        lb_norm_bwd_supports_gadd(H, dtype_code(x), gy.data_ptr(), x.data_ptr(), gamma.data_ptr(), gx.data_ptr(), gadd->data_ptr());
   check(lb_norm_bwd(gy.data_ptr(), x.data_ptr(), gamma.data_ptr(), rms ? nullptr : mean.data_ptr<float>(),
                     rstd.data_ptr<float>(), gx.data_ptr(), dgamma.data_ptr<float>(),
                     has_bias ? dbeta.data_ptr<float>() : nullptr, ws.data_ptr<float>(), rows, H, rms ? 1 : 0,

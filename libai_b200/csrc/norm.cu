@@ -727,8 +727,8 @@ extern "C" int lb_norm_bwd_workspace_rows(int rows, int H) {
 }
 // the fused "+ residual gradient" is implemented by the register-cached kernels only: bf16 rows of whole aligned vectors, fp32
 // rows of H = 256 * {1..6, 8, 10, 12, 16}
-extern "C" int lb_norm_bwd_supports_gadd(int H, int dtype, const void* gy, const void* x, const void* gamma, const void* gadd) {
-  if (dtype == 0) return norm_vec_bf16(H, dtype) && aligned16(gy) && aligned16(x) && aligned16(gamma) && aligned16(gadd);
+extern "C" int lb_norm_bwd_supports_gadd(int H, int dtype, const void* gy, const void* x, const void* gamma, const void* gx, const void* gadd) {
+  if (dtype == 0) return norm_vec_bf16(H, dtype) && aligned16(gy) && aligned16(x) && aligned16(gamma) && aligned16(gx) && aligned16(gadd);
   if (H % 256 != 0) return 0;
   const int v = H / 256;
   return (v >= 1 && v <= 6) || v == 8 || v == 10 || v == 12 || v == 16;
@@ -738,7 +738,7 @@ extern "C" int lb_norm_bwd(const void* gy, const void* x, const void* gamma, con
                            void* gx, float* dgamma, float* dbeta, float* workspace, int rows, int H, int rms, int dtype,
                            int wdtype, int accumulate, const void* gadd, cudaStream_t s) {
   if (rows == 0) return 0;
-  if (gadd != nullptr && !lb_norm_bwd_supports_gadd(H, dtype, gy, x, gamma, gadd)) return -3;  // caller adds the residual gradient itself
+  if (gadd != nullptr && !lb_norm_bwd_supports_gadd(H, dtype, gy, x, gamma, gx, gadd)) return -3;  // caller adds the residual gradient itself
   using B = __nv_bfloat16;
   if (dtype == 0 && (wdtype == 0 || wdtype == 1)) {
     if (!norm_vec_bf16(H, dtype) || !aligned16(gy) || !aligned16(x) || !aligned16(gamma) || !aligned16(gx)) {

@@ -1,8 +1,12 @@
 """Reference (CPU) paths of the fused functional ops agree with their unfused compositions."""
+import ctypes
+import os
+
 import pytest
 import torch
 
 from libai_b200.ops import functional as OF
+from libai_b200.ops import so_path
 
 
 def test_linear_bias_residual_and_mlp_residual_reference_paths():
@@ -51,3 +55,17 @@ def test_attention_kernels_are_not_given_tensors_of_another_device(moved, monkey
         assert not OF._split_supported(*(at(i, *past) for i in range(3)), 0.1, False, None)
     if moved < 2:
         assert OF.attention_packed("q_kv", (at(0, 2, 7, 3, 32), at(1, 2, 9, 3, 64)), causal=False, scale=0.1) is None
+
+
+@pytest.mark.skipif(torch.cuda.is_available() or not os.path.exists(so_path()), reason="host side of the C entry only: no launch may follow")
+def test_norm_backward_never_drops_the_residual_gradient():
+    """A gradient of the residual path is added by the kernel or refused (-3), whichever of the tensors is not on 16 bytes; the pointers
+    are only looked at."""
+    lib = ctypes.CDLL(so_path())
+    p = lambda at: ctypes.c_void_p(at)
+    for odd in range(5):
+        gy, x, gamma, gx, gadd = (p(0x10000 * (i + 1) + (8 if i == odd else 0)) for i in range(5))
+        assert lib.lb_norm_bwd(gy, x, gamma, p(0), p(0x90000), gx, p(0xa0000), p(0), p(0xb0000), 4, 512, 1, 0, 0, 0, gadd, p(0)) == -3
+        assert lib.lb_norm_bwd_supports_gadd(512, 0, gy, x, gamma, gx, gadd) == 0
+    aligned = [p(0x10000 * (i + 1)) for i in range(5)]
+    assert lib.lb_norm_bwd_supports_gadd(512, 0, *aligned) == 1
