@@ -376,14 +376,14 @@ norm_fwd_wide_kernel(const __nv_bfloat16* __restrict__ x, const W* __restrict__ 
   }
 }
 
-// Column sums: added straight into the fp32 gradients (`acc_*`: 16-byte aligned, one vector reduction per 4 columns and
-// block), or left as one row of partials per block for colreduce_kernel.
+// Column sums: one row of partials per block, which colreduce_kernel adds up in a fixed order (vector reductions from every block straight
+// into the fp32 gradients saved that launch, but their order, and with it the last bits of a weight gradient, changed from run to run).
 template <typename W, int V, bool RMS>
 __global__ void __launch_bounds__(NORM_WIDE_THREADS, V <= 2 ? 3 : 1)
 norm_bwd_wide_kernel(const __nv_bfloat16* __restrict__ gy, const __nv_bfloat16* __restrict__ x, const W* __restrict__ gamma,
                      const float* __restrict__ mean_in, const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ gx,
                      float* __restrict__ part_dgamma, float* __restrict__ part_dbeta, int rows, int H,
-                     const __nv_bfloat16* __restrict__ gadd, float* __restrict__ acc_dgamma, float* __restrict__ acc_dbeta) {
+                     const __nv_bfloat16* __restrict__ gadd) {
   __shared__ float2 red[2][NORM_WIDE_THREADS / 32];
   int buf = 0;
   const float inv_h = 1.0f / static_cast<float>(H);
@@ -440,7 +440,6 @@ norm_bwd_wide_kernel(const __nv_bfloat16* __restrict__ gy, const __nv_bfloat16* 
       Vec8<__nv_bfloat16>::store(gx + base + c, o);
     }
   }
-  const bool direct = acc_dgamma != nullptr;
 #pragma unroll
   for (int i = 0; i < V; ++i) {
     const int c = (i * NORM_WIDE_THREADS + threadIdx.x) * 8;
@@ -449,13 +448,7 @@ norm_bwd_wide_kernel(const __nv_bfloat16* __restrict__ gy, const __nv_bfloat16* 
     for (int which = 0; which < 2; ++which) {
       if (which == 1 && part_dbeta == nullptr) continue;
       const float(&v)[8] = which == 0 ? dg[i] : db[i];
-      if (direct) {
-        float* dst = (which == 0 ? acc_dgamma : acc_dbeta) + c;
-        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"l"(dst), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
-        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"l"(dst + 4), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
-      } else {
-        Vec8<float>::store((which == 0 ? part_dgamma : part_dbeta) + static_cast<size_t>(blockIdx.x) * H + c, v);
-      }
+      Vec8<float>::store((which == 0 ? part_dgamma : part_dbeta) + static_cast<size_t>(blockIdx.x) * H + c, v);
     }
   }
 }
@@ -574,7 +567,7 @@ int norm_grid(int rows) { return norm_grid_of(rows, lb::NORM_WARPS, 2); }
 int norm_fwd_grid(int rows) { return norm_grid_of(rows, lb::NORM_WARPS, 4); }
 // bf16 backward: three 4-warp blocks per SM (one wave; every block leaves one row of column partials)
 int norm_bwd_bf16_grid(int rows) { return norm_grid_of(rows, lb::NORM_BWD_WARPS, 3); }
-// wide rows: blocks loop over rows; the backward keeps to one wave because every block adds its column sums at the end
+// wide rows: blocks loop over rows; the backward keeps to one wave because every block leaves a row of column sums at the end
 int norm_fwd_wide_grid(int rows) { return norm_grid_of(rows, 1, 6); }
 int norm_bwd_wide_grid(int rows, int H) { return norm_grid_of(rows, 1, H <= 4096 ? 3 : 1); }
 
@@ -647,8 +640,7 @@ void bwd_dispatch_bf16(int H, const __nv_bfloat16* gy, const __nv_bfloat16* x, c
   }
 #define LB_CASE(V)                                                                                                              \
   case V:                                                                                                                       \
-    lb::norm_bwd_wide_kernel<W, V, RMS><<<grid, lb::NORM_WIDE_THREADS, 0, s>>>(gy, x, g, mean, rstd, gx, pdg, pdb, rows, H,     \
-                                                                               gadd, acc_dg, acc_db);                           \
+    lb::norm_bwd_wide_kernel<W, V, RMS><<<grid, lb::NORM_WIDE_THREADS, 0, s>>>(gy, x, g, mean, rstd, gx, pdg, pdb, rows, H, gadd); \
     break;
   switch ((H + 2047) / 2048) { LB_CASE(1) LB_CASE(2) LB_CASE(3) LB_CASE(4) }
 #undef LB_CASE
@@ -749,8 +741,8 @@ extern "C" int lb_norm_bwd(const void* gy, const void* x, const void* gamma, con
     const int grid = H <= NORM_WARP_MAX_H ? norm_bwd_bf16_grid(rows) : norm_bwd_wide_grid(rows, H);
     float* pdg = workspace;
     float* pdb = dbeta != nullptr ? workspace + static_cast<size_t>(grid) * H : nullptr;
-    // accumulate mode: the blocks add their column sums straight into dgamma / dbeta (vector reductions in the wide kernel)
-    const bool direct = accumulate && (H <= NORM_WARP_MAX_H || (aligned16(dgamma) && aligned16(dbeta)));
+    // accumulate mode: the warp kernel's blocks add their column sums straight into dgamma / dbeta
+    const bool direct = accumulate && H <= NORM_WARP_MAX_H;
     float* adg = direct ? dgamma : nullptr;
     float* adb = direct ? dbeta : nullptr;
 #define LB_GO(W, R) bwd_dispatch_bf16<W, R>(H, (const B*)gy, (const B*)x, (const W*)gamma, mean, rstd, (B*)gx, pdg, pdb, rows, grid, s, (const B*)gadd, adg, adb)

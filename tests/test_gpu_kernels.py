@@ -70,6 +70,21 @@ def test_norm_kernels_at_their_edges(rows, h, rms):
         assert close(dw, w64.grad, 1e-5) and (rms or close(db, b64.grad, 1e-5))
 
 
+@pytest.mark.parametrize("rms", [False, True])
+@pytest.mark.parametrize("rows,h", [(2048, 4096), (300, 1280), (700, 8192)])
+def test_norm_weight_gradients_of_wide_rows_repeat(rows, h, rms):
+    """Added to fp32 gradients by many blocks: the same bits every time."""
+    x, gy, w = _rand((rows, h), 1), _rand((rows, h), 2), _rand((h,), 4)
+    ext = OF.load_ext()
+    _, mean, rstd = ext.norm_fwd(x, w, None if rms else w, 1e-5, rms)
+    runs = []
+    for _ in range(6):
+        gw, gb = torch.ones(h, device="cuda"), None if rms else torch.ones(h, device="cuda")
+        ext.norm_bwd(gy, x, w, mean, rstd, rms, not rms, gw, gb, None)
+        runs.append(gw if rms else torch.cat([gw, gb]))
+    assert all(torch.equal(r, runs[0]) for r in runs)
+
+
 @pytest.mark.parametrize("b,s,a,d,off", [(1, 1, 1, 16, 0), (2, 37, 3, 128, 5), (1, 2100, 4, 64, 0), (3, 9, 5, 48, 1), (2, 7, 2, 24, 3), (1, 5, 32, 256, 0)])
 def test_rotary_on_the_packed_projection(b, s, a, d, off):
     qkv, g = _rand((b, s, a, 3 * d), 1), _rand((b, s, a, 3 * d), 2)
