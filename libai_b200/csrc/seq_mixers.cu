@@ -489,13 +489,13 @@ delta_scan_pair_kernel(const T* __restrict__ qkv, long ldq, int voff, const floa
       }
 #pragma unroll
       for (int m = 0; m < 4; ++m) w[m] += __shfl_xor_sync(0xffffffffu, w[m], 2);
-      const bool two = t + 1 < ct;                // the last token of an odd count: k1 = q1 = 0, b1 = 0, its decay is left out
+      const bool two = t + 1 < ct;                // the last token of an odd count: k1 = q1 = 0, u1 = 0 (even behind a u0 that is not finite), no decay
       const float b0 = sc[t], b1 = sc[t + 1], g0 = sc[CT + t], g1 = two ? sc[CT + t + 1] : 1.f, kq0 = sc[2 * CT + t], kq1 = sc[2 * CT + t + 1];
       const float kk = sc[3 * CT + t], qk = sc[3 * CT + t + 1];
       const int vc = cg * CPT + (CPT == 2 ? bit0 : 0);
       const float u0 = b0 * (ldf(sv + t * VB + vc) - g0 * w[0]);
       const float o0 = g0 * w[1] + kq0 * u0;
-      const float u1 = b1 * (ldf(sv + (t + 1) * VB + vc) - g1 * (g0 * w[2] + kk * u0));
+      const float u1 = two ? b1 * (ldf(sv + (t + 1) * VB + vc) - g1 * (g0 * w[2] + kk * u0)) : 0.f;
       const float o1 = g1 * (g0 * w[3] + qk * u0) + kq1 * u1;
       const float gg = g0 * g1, w0 = g1 * u0;
       const unsigned long long G = pack2(gg, gg);

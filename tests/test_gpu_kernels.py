@@ -277,6 +277,36 @@ def test_delta_scan_two_tokens_at_a_time(lens, heads, kv, d, v, dtype):
         at += n
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, BF16])
+@pytest.mark.parametrize("n", [1, 17])
+def test_delta_scan_value_that_is_not_finite(n, dtype):
+    """An infinite value in the last of an odd number of tokens: its own column of the state becomes infinite with the sign of the key
+    (no pair partner that is not there may turn it into a NaN), the other columns stay what they are without it."""
+    from libai_b200.generation.ragged import RaggedBatch
+    from libai_b200.ops import seq_functional as SF
+
+    kv, heads, d, v = 1, 2, 64, 64
+    qkv, a, b = _rand((n, 2 * d + heads * v), 1, 1.0, dtype), _rand((n, heads), 2, 1.0, dtype), _rand((n, heads), 3, 1.0, dtype)
+    rate, bias = _rand((heads,), 4, 0.5, dtype), _rand((heads,), 5, 0.5, dtype)
+    rb = RaggedBatch([n], [0], [0], "cuda")
+
+    def run(x):
+        S = torch.zeros(1, heads, d, v, device="cuda")
+        return SF.delta_scan(x, d, 2 * d, a, b, rate, bias, S, rb, kv, False), S[0]
+
+    base = run(qkv)
+    x = qkv.clone()
+    x[-1, 2 * d + v + 5] = float("inf")                       # head 1, column 5
+    out, S = run(x)
+    key = x[-1, d:2 * d].float()
+    assert torch.equal(S[1, :, 5], torch.where(key > 0, 1.0, -1.0) * float("inf"))
+    assert not torch.isfinite(out[-1, v + 5]) and not torch.isnan(out[-1, v + 5])
+    keep = torch.ones(heads, v, dtype=torch.bool, device="cuda")
+    keep[1, 5] = False
+    assert torch.equal(S.transpose(1, 2)[keep], base[1].transpose(1, 2)[keep])
+    assert torch.equal(out[-1].view(heads, v)[keep], base[0][-1].view(heads, v)[keep]) and torch.equal(out[:-1], base[0][:-1])
+
+
 @pytest.mark.parametrize("lens", [False, True])
 @pytest.mark.parametrize("causal", [False, True])
 @pytest.mark.parametrize("b,s,a", [(1, 1, 1), (2, 63, 2), (1, 64, 3), (2, 65, 1), (1, 127, 2), (3, 128, 1), (1, 130, 2), (2, 333, 4), (1, 1024, 16)])
