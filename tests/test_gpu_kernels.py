@@ -282,7 +282,7 @@ def test_delta_scan_two_tokens_at_a_time(lens, heads, kv, d, v, dtype):
 def test_delta_scan_value_that_is_not_finite(n, dtype):
     """An infinite value in the last of an odd number of tokens: its own column of the state becomes infinite with the sign of the key
     (no pair partner that is not there may turn it into a NaN), the other columns stay what they are without it."""
-    from libai_b200.generation.ragged import RaggedBatch
+    from libai_b200.inference.ragged import RaggedBatch
     from libai_b200.ops import seq_functional as SF
 
     kv, heads, d, v = 1, 2, 64, 64
