@@ -27,8 +27,9 @@ _LAUNCH_COUNT = 0
 
 
 # the process environment as ``os.environ`` keeps it (encoded): asked once per operator call, where ``os.environ.get`` costs 1 us
-_ENV = getattr(os.environ, "_data", os.environ)
-_IMPL_KEY = "LIBAI_B200_IMPL" if _ENV is os.environ else os.environ.encodekey("LIBAI_B200_IMPL")
+_ENVIRON = os.environ
+_ENV = getattr(_ENVIRON, "_data", None)
+_IMPL_KEY = None if _ENV is None else _ENVIRON.encodekey("LIBAI_B200_IMPL")
 
 
 def so_path() -> str:
@@ -37,6 +38,8 @@ def so_path() -> str:
 
 def impl() -> str:
     """'native' (default) or 'ref' (``LIBAI_B200_IMPL=ref`` forces the PyTorch path on GPU)."""
+    if _ENV is None or os.environ is not _ENVIRON:       # a mapping that was put in its place
+        return os.environ.get("LIBAI_B200_IMPL", "native")
     v = _ENV.get(_IMPL_KEY)
     return "native" if v is None else os.fsdecode(v)
 

@@ -5,6 +5,7 @@ import os
 import pytest
 import torch
 
+from libai_b200 import ops
 from libai_b200.ops import functional as OF
 from libai_b200.ops import so_path
 
@@ -69,3 +70,14 @@ def test_norm_backward_never_drops_the_residual_gradient():
         assert lib.lb_norm_bwd_supports_gadd(512, 0, gy, x, gamma, gx, gadd) == 0
     aligned = [p(0x10000 * (i + 1)) for i in range(5)]
     assert lib.lb_norm_bwd_supports_gadd(512, 0, *aligned) == 1
+
+
+def test_implementation_switch_follows_the_environment(monkeypatch):
+    monkeypatch.delenv("LIBAI_B200_IMPL", raising=False)
+    assert ops.impl() == "native"
+    monkeypatch.setenv("LIBAI_B200_IMPL", "ref")
+    assert ops.impl() == "ref"
+    monkeypatch.setattr(os, "environ", {"LIBAI_B200_IMPL": "other"})       # the whole mapping replaced
+    assert ops.impl() == "other"
+    monkeypatch.setattr(os, "environ", {})
+    assert ops.impl() == "native"
