@@ -4,9 +4,11 @@ import math
 
 import pytest
 import torch
+from torch._subclasses.fake_tensor import FakeTensorMode
 
 from libai_b200.ops import functional as OF
 from libai_b200.ops import so_path
+from libai_b200.ops.gated_mlp import gated_mlp
 
 pytestmark = pytest.mark.gpu
 BF16 = torch.bfloat16
@@ -352,3 +354,69 @@ def test_gemm_tile_order_in_bands(M, layout):
     want = x.float() @ (w.float().t() if layout == 0 else w.float())
     assert want.abs().max() < 256
     assert torch.equal(OF.load_ext().gemm(x, w, layout, None, None, False, BF16).float(), want)
+
+
+_W = lambda *s, i=1: _rand(s, i, s[-1] ** -0.5)
+_ROT = lambda s, d: (torch.linspace(0, 3, s * d, device="cuda").view(s, d).cos().contiguous(), torch.linspace(0, 3, s * d, device="cuda").view(s, d).sin().contiguous())
+_GRAPHLESS = {
+    "linear": lambda x: OF.linear(x, _W(72, 64), _rand((72,), 2), "gelu"),
+    "mlp": lambda x: OF.mlp(x, _W(128, 64), _rand((128,), 2), _W(64, 128, i=3), "gelu", _rand((64,), 4), x),
+    "mlp_without_residual": lambda x: OF.mlp(x, _W(128, 64), _rand((128,), 2), _W(64, 128, i=3)),
+    "linear_bias_residual": lambda x: OF.linear_bias_residual(x, _W(64, 64), _rand((64,), 2), x),
+    "layer_norm": lambda x: OF.layer_norm(x, _rand((64,), 2), _rand((64,), 3)),
+    "layer_norm_with_skip": lambda x: OF.layer_norm_with_skip(x, _rand((64,), 2), _rand((64,), 3)),
+    "rms_norm": lambda x: OF.rms_norm(x, _rand((64,), 2)),
+    "bias_act": lambda x: OF.bias_act(x, _rand((64,), 2)),
+    "bias_add": lambda x: OF.bias_dropout_add(x, _rand((64,), 2), _rand((3, 40, 64), 3), 0.0, False),
+    "gated_mlp": lambda x: gated_mlp(x, _W(128, 64), _W(128, 64, i=2), _W(64, 128, i=3)),
+    "swiglu": lambda x: OF.swiglu(x, _rand((3, 40, 64), 2)),
+    "attention_64": lambda x: OF.attention(*(_rand((3, 4, 40, 64), i) + x.mean() for i in range(3)), causal=True),
+    "attention_48": lambda x: OF.attention(*(_rand((3, 4, 40, 48), i) + x.mean() for i in range(3)), causal=True),
+    "attention_packed": lambda x: OF.attention_packed("qkv", (_rand((3, 40, 4, 96), 1) + x.mean(),), causal=False, scale=0.2),
+    "attention_qkvpacked": lambda x: OF.attention_qkvpacked(_rand((3, 40, 4, 192), 1) + x.mean(), causal=True, scale=0.2),
+    "rotary": lambda x: OF.apply_rotary(x.view(3, 40, 1, 64).permute(0, 2, 1, 3).contiguous(), *_ROT(40, 64)),
+    "rotary_qkv": lambda x: OF.apply_rotary_qkv(_rand((3, 40, 4, 96), 1) + x.mean(), *_ROT(64, 32)),
+    "cross_entropy": lambda x: OF.vocab_parallel_cross_entropy(x.clone(), torch.arange(120, device="cuda").view(3, 40) % 64),
+    "embedding": lambda x: OF.embedding(torch.arange(30, device="cuda") % 40, x[0]),
+}
+
+
+@pytest.mark.parametrize("name", sorted(_GRAPHLESS))
+def test_calls_without_a_graph_equal_those_with_one(name):
+    """Without gradients the forwards run past the autograd functions: the same bits, nothing kept, nothing that asks for a gradient."""
+    x = _rand((3, 40, 64), 9)
+    one = lambda y: y[0] if isinstance(y, tuple) else y
+    with_graph = one(_GRAPHLESS[name](x.clone().requires_grad_(True)))
+    assert with_graph.requires_grad
+    for mode in (torch.no_grad, torch.inference_mode):
+        with mode():
+            got = one(_GRAPHLESS[name](x.clone().requires_grad_(True)))
+            assert not got.requires_grad and got.grad_fn is None and got.shape == with_graph.shape and torch.equal(got, with_graph.detach())
+
+
+@pytest.mark.parametrize("grad", [False, True])
+@pytest.mark.parametrize("d", [24, 48])
+def test_attention_transformed_differentiated_forward_and_traced(d, grad):
+    """vmap, both forward modes, tracing and tensors without memory see the unfused operators, in gradient mode and out of it."""
+    scale = d ** -0.5
+    q, k, v, t = (_rand((2, 3, 20, d), i) for i in range(4))
+    f = lambda x: OF.attention(x, k, v, causal=True, scale=scale)
+    ref = lambda x: OF.attention_ref(x, k, v, causal=True, scale=scale)
+    near = lambda a, b: float((a.double() - b.double()).norm() / b.double().norm()) < 2.0 ** -7
+    with torch.set_grad_enabled(grad):
+        assert near(torch.func.vmap(f)(torch.stack([q, t])), torch.stack([ref(q), ref(t)]))
+        packed = lambda x: OF.attention_packed("qkv", (x,), causal=False, scale=scale) is None
+        told = []
+        torch.func.vmap(lambda x: (told.append(packed(x)), x)[1])(_rand((2, 1, 20, 3, 3 * d), 5))
+        assert told == [True]
+        want = torch.func.jvp(ref, (q,), (t,))
+        assert all(near(a, b) for a, b in zip(torch.func.jvp(f, (q,), (t,)), want))
+        with torch.autograd.forward_ad.dual_level():
+            out = torch.autograd.forward_ad.unpack_dual(f(torch.autograd.forward_ad.make_dual(q, t)))
+            assert near(out.primal, want[0]) and near(out.tangent, want[1])
+        traced = torch.jit.trace(f, (q,), check_trace=False)
+        assert near(traced(t), ref(t))
+        with FakeTensorMode():
+            x = torch.empty(2, 3, 20, d, dtype=BF16, device="cuda")
+            assert OF.attention(x, x, x, causal=True).shape == x.shape
+            assert OF.attention_cached(x[:, :, :1], x[:, :, :1], x[:, :, :1], x, x, scale=scale) is None
