@@ -709,7 +709,7 @@ class _SplitAttnFn(torch.autograd.Function):
             return (None,) * 4 + tuple(next(grads) if n else None for n in ctx.needs_input_grad[4:])
         if ctx.layout == "q_k_v":              # gradients backed by [b, s, a, d], as the projections around an attention read them
             gs = [torch.empty(t.shape[0], t.shape[2], t.shape[1], t.shape[3], dtype=t.dtype, device=t.device).permute(0, 2, 1, 3) for t in ts]
-            o = o.permute(0, 2, 1, 3)
+            o = o.permute(0, 2, 1, 3).contiguous()        # (a hook on saved tensors may have packed it in another order)
         else:
             gs = [torch.empty(t.shape, dtype=t.dtype, device=t.device) for t in ts]
             go = go.permute(0, 2, 1, 3)

@@ -420,3 +420,15 @@ def test_attention_transformed_differentiated_forward_and_traced(d, grad):
             x = torch.empty(2, 3, 20, d, dtype=BF16, device="cuda")
             assert OF.attention(x, x, x, causal=True).shape == x.shape
             assert OF.attention_cached(x[:, :, :1], x[:, :, :1], x[:, :, :1], x, x, scale=scale) is None
+
+
+@pytest.mark.parametrize("d", [48, 64, 128])
+@pytest.mark.parametrize("pin", [False, True])
+def test_attention_backward_from_tensors_saved_on_the_host(d, pin):
+    """Saved-tensor hooks may give tensors back with other strides."""
+    q, k, v = (_rand((2, 3, 40, d), i).requires_grad_(True) for i in range(3))
+    go = _rand((2, 3, 40, d), 4)
+    want = torch.autograd.grad(OF.attention(q, k, v, causal=True), (q, k, v), go)
+    with torch.autograd.graph.save_on_cpu(pin_memory=pin):
+        out = OF.attention(q, k, v, causal=True)
+    assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(out, (q, k, v), go), want))
