@@ -3,26 +3,29 @@
 // and backward.
 //
 // These calls used to run as unfused fp32 matrix products over [b, a, sq, sk] tensors (head dims 24, 32 and 48 of the shipped GPT,
-// BERT and T5 recipes, every dense mask).  They held probabilities and their gradients in 32 bits, and so does this: P and dS go
-// to the tensor core as the sum of two bf16 numbers (hi = bf16(x), lo = bf16(x - hi), together 16 bits of mantissa), two MMAs in
-// place of one, accumulated in fp32; the row sums of dO ∘ O use O in the same two parts.  Errors against 64 bits are those of the
-// unfused form (both end in the rounding of the bf16 results).
+// BERT and T5 recipes where they run without dropout on the probabilities, every dense mask).  They held probabilities and their
+// gradients in 32 bits, and so does this: P and dS go to the tensor core as the sum of three bf16 numbers, which holds all 24 bits of
+// an fp32 significand, three MMAs in place of one, accumulated in fp32; the row sums of dO ∘ O use O in fp32.  Two parts (16 bits) are
+// not enough: where keys and values share a large common part, dP - δ and Σ dS·K cancel, and dQ of [4, 16, 512, 48] with a
+// common part of 20 standard deviations was 1.5e-2 off where the unfused form is 1.7e-3 off (the rounding of its bf16 result);
+// now 1.8e-3.  Without a common part all outputs are as far off as the unfused form's to three digits.
+// An infinity or NaN comes out as an infinity or NaN, an infinity mostly as a NaN (0 times it in the smaller parts).
 //
 // Head dims below 64: the tensor maps have the true inner extent, TMA fills columns [d, 64) of the tiles with zeros, which add
 // nothing to Q·Kᵀ / dO·Vᵀ; the surplus columns of the other products are not stored.  Masks arrive packed, one bit per (query,
 // key), with one fill value per row: -10000 (log2 domain), or 0 for a row without any visible key, whose probabilities are uniform
 // whatever the constant (0 keeps its log-sum-exp small and exact).
 //
-// Bounded by the softmax threads (two passes over S, two roundings per probability), not by the tensor core or memory: key tiles of
-// 128, two forward CTAs per SM.  Measured: [16, 512] BERT block with 16 heads of 48 and a padding mask, attention kernels 294 us (181
-// backward, 85 forward, 28 around them) where the unfused form took 2470 us; cross attention of 128 on 512 tokens, 12 heads of 32,
-// 16 sequences, with self attention 125 us against 780 us.
+// Bounded by the softmax threads (two passes over S, three roundings per probability), not by the tensor core or memory: key tiles of
+// 128, two forward CTAs per SM.  Measured: [16, 512] BERT block with 16 heads of 48 and a padding mask, forward and backward, 3100 us
+// with the unfused form, 877 us with two parts, 916 us with three.
 // Every wait on an mbarrier is bounded (attention_tc.cuh).
 #include "attention_tc.cuh"
 
 namespace lb {
 
-constexpr int SPL_THREADS = 320;                 // TMA warp, MMA warp, 8 softmax warps
+constexpr int SPL_THREADS = 320;                 // backward: TMA warp, MMA warp, 8 softmax warps
+constexpr int SPL_FWD_THREADS = 256;             // forward: 8 softmax warps, one thread of which issues loads and MMAs: two CTAs of more warps get 96 registers, and spill
 constexpr int SPL_TILE = 128 * 64 * 2;           // one [128, 64] bf16 tile, 128-byte rows, swizzled
 constexpr float SPL_LOG2E = 1.4426950408889634f;
 
@@ -34,7 +37,8 @@ struct SplitParams {
   const float* fill;            // [Bm, Am, Sq] score of the masked keys of a row, log2 domain
   long mask_b, mask_a;          // rows between batches / heads (0: shared)
   int pitch;                    // words per row, a multiple of 4
-  __nv_bfloat16 *o, *o_lo;      // [B, Sq, A, d]; o_lo (optional): what the rounding of o left over
+  __nv_bfloat16* o;             // [B, Sq, A, d]
+  float* o32;                   // optional: the same before its rounding, for the backward
   float* lse;                   // [B, A, Sq] natural log
   // backward
   const float* delta;           // [B, A, Sq]
@@ -43,10 +47,15 @@ struct SplitParams {
   int* err;
 };
 
-LB_DEVICE uint32_t split_hi(float x0, float x1) { return pack_bf16(x0, x1); }
-LB_DEVICE uint32_t split_lo(float x0, float x1, uint32_t hi) {
-  const float2 h = unpack_bf16(hi);
-  return pack_bf16(x0 - h.x, x1 - h.y);
+// two fp32 numbers as three bf16 parts each, h + m + l = x to the last bit (8 + 8 + 8 bits of significand; normal range)
+LB_DEVICE void split3(float x0, float x1, uint32_t& h, uint32_t& m, uint32_t& l) {
+  h = pack_bf16(x0, x1);
+  const float2 a = unpack_bf16(h);
+  x0 -= a.x;
+  x1 -= a.y;
+  m = pack_bf16(x0, x1);
+  const float2 b = unpack_bf16(m);
+  l = pack_bf16(x0 - b.x, x1 - b.y);
 }
 
 // ------------------------------------------------------------------------------------------------------------ mask -> bits
@@ -78,13 +87,15 @@ attn_mask_pack_kernel(const U* __restrict__ mask, unsigned long long and_mask, i
 }
 
 // ------------------------------------------------------------------------------------------------------------------ forward
-// One CTA per (128 queries, head, batch).  S in TMEM columns [0, 128), O in [128, 192), P hi in [192, 256); P lo of a half's 64 keys
-// overwrites the first 32 of that half's S columns once its threads have read them, so the whole fits 256 columns and two CTAs
-// share an SM.  The MMA warp issues S(j+1) after P(j)·V(j) has completed (it overwrites P lo); the other CTA fills the gap.
+// One CTA per (128 queries, head, batch).  S in TMEM columns [0, 128), O in [128, 192), P's first part in [192, 256); the second and third
+// parts of 16 keys (8 columns each) overwrite the 16 S columns of those keys once their thread has read them, so the whole fits 256 columns
+// and two CTAs share an SM.  The MMA warp issues S(j+1) after P(j)·V(j) has completed (it overwrites them); the other CTA fills the gap.
+// O is added up over the key blocks in registers: the tensor core rounds every addition into its accumulator towards zero, and 24 of them
+// per key block leave O, with it δ, some 1e-6 short (dQ of the example above: 8.5e-3 off).
 constexpr int SPL_FWD_SMEM = 5 * SPL_TILE + 2 * 2 * 128 * 4 + 1024 + 256;
 
 template <bool MASKED>
-__global__ void __launch_bounds__(SPL_THREADS, 2)
+__global__ void __launch_bounds__(SPL_FWD_THREADS, 2)
 attn_split_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                       const __grid_constant__ CUtensorMap tmap_v, SplitParams p) {
   constexpr uint32_t S_COL = 0, O_COL = 128, P_COL = 192;
@@ -96,15 +107,13 @@ attn_split_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   float* sXchg = reinterpret_cast<float*>(sV + 2 * SPL_TILE);      // [parity][half][row]
   uint64_t* bars = reinterpret_cast<uint64_t*>(sXchg + 2 * 2 * 128);
   uint64_t* q_full = bars;
-  uint64_t* k_full = bars + 1;
-  uint64_t* k_empty = bars + 3;
-  uint64_t* v_full = bars + 5;
-  uint64_t* v_empty = bars + 7;
-  uint64_t* s_full = bars + 9;
-  uint64_t* p_full = bars + 10;
-  uint64_t* o_full = bars + 11;
-  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 12);
-  volatile int* stop = reinterpret_cast<volatile int*>(bars + 13);
+  uint64_t* k_full = bars + 1;       // 2
+  uint64_t* v_full = bars + 3;       // 2
+  uint64_t* s_full = bars + 5;
+  uint64_t* p_full = bars + 6;
+  uint64_t* o_full = bars + 7;
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 8);
+  volatile int* stop = reinterpret_cast<volatile int*>(bars + 9);
 
   const int warp_idx = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int q_blk = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x);   // late query blocks have the most keys
@@ -117,7 +126,7 @@ attn_split_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     tma_prefetch_desc(&tmap_k);
     tma_prefetch_desc(&tmap_v);
     mbar_init(q_full, 1);
-    for (int i = 0; i < 2; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&k_full[i], 1); mbar_init(&v_full[i], 1); }
     mbar_init(s_full, 1);
     mbar_init(p_full, 8);
     mbar_init(o_full, 1);
@@ -125,68 +134,61 @@ attn_split_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     fence_barrier_init();
     fence_proxy_async();
   }
-  if (warp_idx == 1) tmem_alloc<256>(tmem_ptr_smem);
+  if (warp_idx == 0) tmem_alloc<256>(tmem_ptr_smem);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
 
+  // The block's chain is serial whoever issues it (the other CTA of the SM fills its gaps), so a thread of the softmax warps does.  K(j+1) and
+  // V(j+1) go where K(j-1) and V(j-1) were, and o_full(j-1) has said that nothing reads those any more.
+  const int ksteps = (p.d + 15) / 16;                                // the columns behind d are zeros
+  auto load = [&](int j) {
+    const int b = j & 1;
+    mbar_arrive_expect_tx(&k_full[b], SPL_TILE);
+    tma_load_4d(sK + b * SPL_TILE, &tmap_k, &k_full[b], 0, j * 128, head, batch);
+    mbar_arrive_expect_tx(&v_full[b], SPL_TILE);
+    tma_load_4d(sV + b * SPL_TILE, &tmap_v, &v_full[b], 0, j * 128, head, batch);
+  };
+  auto scores = [&](int j) {                                         // S(j)
+    constexpr uint32_t idesc = make_idesc_bf16(128, 128, false, false);
+    const int b = j & 1;
+    if (!tc_wait(&k_full[b], (j >> 1) & 1, stop)) return;
+    tc_fence_after_sync();
+    const uint32_t q_addr = smem_u32(sQ), k_addr = smem_u32(sK + b * SPL_TILE);
+    for (int kk = 0; kk < ksteps; ++kk)
+      umma_f16_ss(tmem_base + S_COL, make_smem_desc_sw128(q_addr + kk * 32, 0, 1024), make_smem_desc_sw128(k_addr + kk * 32, 0, 1024), idesc,
+                  kk > 0 ? 1u : 0u);
+    umma_commit(s_full);
+    if (j + 1 < nkv) load(j + 1);
+  };
+  auto values = [&](int j) {                                         // P(j)·V(j)
+    constexpr uint32_t idesc = make_idesc_bf16(128, 64, false, true);
+    const int b = j & 1;
+    if (!tc_wait(p_full, j & 1, stop) || !tc_wait(&v_full[b], (j >> 1) & 1, stop)) return;
+    tc_fence_after_sync();
+    const uint32_t v_addr = smem_u32(sV + b * SPL_TILE);
+    const uint64_t dv = make_smem_desc_sw128(v_addr, 128 * 128, 1024);
+#pragma unroll 1
+    for (int part = 2; part >= 0; --part) {                          // smallest first: the accumulator's roundings stay small until the last eight steps
+      const uint32_t at = tmem_base + (part == 0 ? P_COL : S_COL + (part - 1) * 8), step = part == 0 ? 8 : 16;
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk)
+        umma_f16_ts(tmem_base + O_COL, at + kk * step, dv + kk * ((16 * 128) >> 4), idesc, (part < 2 || kk > 0) ? 1u : 0u);
+    }
+    umma_commit(o_full);
+  };
   if (warp_idx == 0) {
     if (elect_one()) {
       mbar_arrive_expect_tx(q_full, SPL_TILE);
       tma_load_4d(sQ, &tmap_q, q_full, 0, q0, head, batch);
-      for (int j = 0; j < nkv; ++j) {
-        const int b = j & 1;
-        const uint32_t par = ((j >> 1) & 1) ^ 1;
-        if (tc_wait(&k_empty[b], par, stop)) {
-          mbar_arrive_expect_tx(&k_full[b], SPL_TILE);
-          tma_load_4d(sK + b * SPL_TILE, &tmap_k, &k_full[b], 0, j * 128, head, batch);
-        }
-        if (tc_wait(&v_empty[b], par, stop)) {
-          mbar_arrive_expect_tx(&v_full[b], SPL_TILE);
-          tma_load_4d(sV + b * SPL_TILE, &tmap_v, &v_full[b], 0, j * 128, head, batch);
-        }
-      }
+      load(0);
+      if (tc_wait(q_full, 0, stop)) scores(0);
     }
     __syncwarp();
-  } else if (warp_idx == 1) {
-    constexpr uint32_t idesc_qk = make_idesc_bf16(128, 128, false, false);
-    constexpr uint32_t idesc_pv = make_idesc_bf16(128, 64, false, true);
-    const int ksteps = (p.d + 15) / 16;                              // the columns behind d are zeros
-    const uint32_t q_addr = smem_u32(sQ);
-    bool ok = __all_sync(0xffffffffu, tc_wait(q_full, 0, stop));
-    for (int j = 0; j < nkv; ++j) {
-      const int b = j & 1;
-      ok = __all_sync(0xffffffffu, ok && tc_wait(&k_full[b], (j >> 1) & 1, stop));
-      if (j > 0) ok = __all_sync(0xffffffffu, ok && tc_wait(o_full, (j - 1) & 1, stop));
-      tc_fence_after_sync();
-      if (ok && elect_one()) {
-        const uint32_t k_addr = smem_u32(sK + b * SPL_TILE);
-        for (int kk = 0; kk < ksteps; ++kk)
-          umma_f16_ss(tmem_base + S_COL, make_smem_desc_sw128(q_addr + kk * 32, 0, 1024), make_smem_desc_sw128(k_addr + kk * 32, 0, 1024),
-                      idesc_qk, kk > 0 ? 1u : 0u);
-        umma_commit(s_full);
-        umma_commit(&k_empty[b]);
-      }
-      __syncwarp();
-      ok = __all_sync(0xffffffffu, ok && tc_wait(p_full, j & 1, stop));
-      ok = __all_sync(0xffffffffu, ok && tc_wait(&v_full[b], (j >> 1) & 1, stop));
-      tc_fence_after_sync();
-      if (ok && elect_one()) {
-        const uint32_t v_addr = smem_u32(sV + b * SPL_TILE);
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          const uint64_t bv = make_smem_desc_sw128(v_addr + kk * (16 * 128), 128 * 128, 1024);
-          umma_f16_ts(tmem_base + O_COL, tmem_base + P_COL + kk * 8, bv, idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
-          umma_f16_ts(tmem_base + O_COL, tmem_base + S_COL + (kk / 4) * 64 + (kk % 4) * 8, bv, idesc_pv, 1u);
-        }
-        umma_commit(o_full);
-        umma_commit(&v_empty[b]);
-      }
-      __syncwarp();
-    }
-  } else {
-    const int quad = warp_idx % 4, half = (warp_idx - 2) / 4;        // this warp's 64 of the 128 key columns
+  }
+  {
+    const int quad = warp_idx % 4, half = warp_idx / 4;              // this warp's 64 of the 128 key columns
     const int r = quad * 32 + lane, q_idx = q0 + r;
     const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
     const uint32_t s_addr = tmem_base + lane_off + S_COL + half * 64;
@@ -200,7 +202,9 @@ attn_split_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       mrow = p.mask + row * p.pitch + half * 2;
       fill = p.fill[row];
     }
-    float m_run = -INFINITY, l_run = 0.f;
+    float m_run = -INFINITY, l_run = 0.f, acc[32];                   // acc: this half's 32 columns of the output row
+#pragma unroll
+    for (int i = 0; i < 32; ++i) acc[i] = 0.f;
     for (int j = 0; j < nkv; ++j) {
       [[maybe_unused]] uint2 bits = make_uint2(0, 0);
       if constexpr (MASKED) bits = *reinterpret_cast<const uint2*>(mrow + j * 4);
@@ -213,16 +217,16 @@ attn_split_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       auto pass1 = [&](auto edge_tag) {
         constexpr bool EDGE = decltype(edge_tag)::value;
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          uint32_t t[32];
-          tmem_ld_32x32b_x32(s_addr + c * 32, t);
+        for (int c = 0; c < 4; ++c) {
+          uint32_t t[16];
+          tmem_ld_32x32b_x16(s_addr + c * 16, t);
           tmem_ld_wait();
-          [[maybe_unused]] const uint32_t word = c == 0 ? bits.x : bits.y;
+          [[maybe_unused]] const uint32_t word = (c < 2 ? bits.x : bits.y) >> ((c & 1) * 16);
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
+          for (int i = 0; i < 16; ++i) {
             float x = __uint_as_float(t[i]) * p.scale_log2;
             if constexpr (MASKED) x = (word >> i) & 1u ? x : fill;
-            if constexpr (EDGE) x = k0 + c * 32 + i < key_lim ? x : -INFINITY;
+            if constexpr (EDGE) x = k0 + c * 16 + i < key_lim ? x : -INFINITY;
             mx = fmaxf(mx, x);
           }
         }
@@ -236,20 +240,19 @@ attn_split_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       const bool bump = (m_cand - m_run > 8.0f) || (m_run == -INFINITY && m_cand != -INFINITY);   // lazy rescale
       float alpha = 1.0f;
       if (bump) { alpha = fast_exp2(m_run - m_cand); m_run = m_cand; }                            // 0 on the first tile
-      const bool bump_any = __any_sync(0xffffffffu, bump && j > 0);
       const float m_use = m_run == -INFINITY ? 0.f : m_run;
       float rowsum = 0.f;
       auto pass2 = [&](auto edge_tag) {
         constexpr bool EDGE = decltype(edge_tag)::value;
         float rs0 = 0.f, rs1 = 0.f;
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          uint32_t t[32], hi[16], lo[16];
-          tmem_ld_32x32b_x32(s_addr + c * 32, t);
+        for (int c = 0; c < 4; ++c) {          // 16 keys at a time: 32 would spill
+          uint32_t t[16], part[3][8];
+          tmem_ld_32x32b_x16(s_addr + c * 16, t);
           tmem_ld_wait();
-          [[maybe_unused]] const uint32_t word = c == 0 ? bits.x : bits.y;
+          [[maybe_unused]] const uint32_t word = (c < 2 ? bits.x : bits.y) >> ((c & 1) * 16);
 #pragma unroll
-          for (int i = 0; i < 32; i += 2) {
+          for (int i = 0; i < 16; i += 2) {
             float x0 = __uint_as_float(t[i]) * p.scale_log2, x1 = __uint_as_float(t[i + 1]) * p.scale_log2;
             if constexpr (MASKED) {
               x0 = (word >> i) & 1u ? x0 : fill;
@@ -258,60 +261,65 @@ attn_split_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
             x0 = fast_exp2(x0 - m_use);
             x1 = fast_exp2(x1 - m_use);
             if constexpr (EDGE) {
-              x0 = k0 + c * 32 + i < key_lim ? x0 : 0.f;
-              x1 = k0 + c * 32 + i + 1 < key_lim ? x1 : 0.f;
+              x0 = k0 + c * 16 + i < key_lim ? x0 : 0.f;
+              x1 = k0 + c * 16 + i + 1 < key_lim ? x1 : 0.f;
             }
             rs0 += x0;
             rs1 += x1;
-            hi[i / 2] = split_hi(x0, x1);
-            lo[i / 2] = split_lo(x0, x1, hi[i / 2]);
+            split3(x0, x1, part[0][i / 2], part[1][i / 2], part[2][i / 2]);
           }
-          // (S(j) follows the completion of P(j-1)·V(j-1): both sets of columns are free; lo covers S columns read above)
-          tmem_st_32x32b_x16(p_addr + c * 16, hi);
-          tmem_st_32x32b_x16(s_addr + c * 16, lo);
+          // (S(j) follows the completion of P(j-1)·V(j-1): all columns are free; the last two parts cover S columns read above)
+          tmem_st_32x32b_x8(p_addr + c * 8, part[0]);
+          tmem_st_32x32b_x8(s_addr + c * 16, part[1]);
+          tmem_st_32x32b_x8(s_addr + c * 16 + 8, part[2]);
         }
         rowsum = rs0 + rs1;
       };
       if (edge) pass2(std::true_type{}); else pass2(std::false_type{});
       l_run = l_run * alpha + rowsum;
-      if (bump_any) {
-        uint32_t t[32];
-        tmem_ld_32x32b_x32(o_addr, t);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 32; ++i) t[i] = __float_as_uint(__uint_as_float(t[i]) * alpha);
-        tmem_st_32x32b_x32(o_addr, t);
-      }
       tmem_st_wait();
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full);
+      if (warp_idx == 0) {
+        if (elect_one()) values(j);
+        __syncwarp();
+      }
+      // ---- O = O · alpha + P(j)·V(j), while S(j+1) is computed
+      tc_wait(o_full, j & 1, stop);
+      __syncwarp();
+      tc_fence_after_sync();
+      if (warp_idx == 0 && j + 1 < nkv) {
+        if (elect_one()) scores(j + 1);
+        __syncwarp();
+      }
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t t[16];
+        tmem_ld_32x32b_x16(o_addr + c * 16, t);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[c * 16 + i] = fmaf(acc[c * 16 + i], alpha, __uint_as_float(t[i]));
+      }
     }
     float* xch = sXchg + (nkv & 1) * 256;
     xch[half * 128 + r] = l_run;
     tc_pair_sync(quad);
     l_run += xch[(half ^ 1) * 128 + r];
-    tc_wait(o_full, (nkv - 1) & 1, stop);
-    __syncwarp();
-    tc_fence_after_sync();
     const float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
-    uint32_t t[32];
-    tmem_ld_32x32b_x32(o_addr, t);
-    tmem_ld_wait();
     if (q_idx < p.Sq) {
       const size_t at = ((static_cast<size_t>(batch) * p.Sq + q_idx) * p.A + head) * p.d + half * 32;
 #pragma unroll
       for (int i = 0; i < 32; i += 8) {
         if (half * 32 + i >= p.d) break;                             // d is a multiple of 8
-        uint32_t hi[4], lo[4];
+        float x[8];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float x0 = __uint_as_float(t[i + 2 * e]) * inv, x1 = __uint_as_float(t[i + 2 * e + 1]) * inv;
-          hi[e] = split_hi(x0, x1);
-          lo[e] = split_lo(x0, x1, hi[e]);
+        for (int e = 0; e < 8; ++e) x[e] = acc[i + e] * inv;
+        *reinterpret_cast<uint4*>(p.o + at + i) = make_uint4(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]), pack_bf16(x[4], x[5]), pack_bf16(x[6], x[7]));
+        if (p.o32 != nullptr) {
+          *reinterpret_cast<float4*>(p.o32 + at + i) = make_float4(x[0], x[1], x[2], x[3]);
+          *reinterpret_cast<float4*>(p.o32 + at + i + 4) = make_float4(x[4], x[5], x[6], x[7]);
         }
-        *reinterpret_cast<uint4*>(p.o + at + i) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-        if (p.o_lo != nullptr) *reinterpret_cast<uint4*>(p.o_lo + at + i) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
       }
       if (half == 0)
         p.lse[(static_cast<size_t>(batch) * p.A + head) * p.Sq + q_idx] =
@@ -325,20 +333,24 @@ attn_split_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     if (threadIdx.x == 0) { *const_cast<volatile int*>(p.err) = 1; __threadfence_system(); }
     __syncthreads();
   }
-  if (warp_idx == 1) {
+  if (warp_idx == 0) {
     tc_fence_after_sync();
     tmem_dealloc<256>(tmem_base);
   }
 }
 
 // ----------------------------------------------------------------------------------------------------------------- backward
-// One CTA per (128 keys, head, batch), looping over the query blocks that see them:
-//   S = Q·Kᵀ, dP = dO·Vᵀ;  P = exp(S - lse), dS = P ∘ (dP - δ) · scale, both to shared memory in two bf16 parts;
-//   dV += Pᵀ·dO, dK += dSᵀ·Q, dQ_i = dS·K (added to the fp32 accumulator by TMA reductions).
-// Shared memory: K, V, Q, dO 64 KB, the four P / dS tiles 128 KB, dQ staging 32 KB.
+// One CTA per (128 keys, head, batch), looping over the query blocks that see them, with the keys on the M side:
+//   Sᵀ = K·Qᵀ, dPᵀ = V·dOᵀ;  P = exp(S - lse), dS = P ∘ (dP - δ) · scale, in three bf16 parts each;
+//   dV += Pᵀ·dO with Pᵀ from TMEM, dK += dSᵀ·Q and dQ_i = dS·K (added to the fp32 accumulator by TMA reductions) with dSᵀ from shared memory.
+// Six tiles of parts do not fit shared memory beside the operands, so Pᵀ stays in TMEM, which wants it as [keys, queries]: the first part in
+// columns of its own, the second and third of 16 queries over the 16 Sᵀ columns that their thread has read.
+// Shared memory: K, V, Q, dO 64 KB, three dSᵀ tiles 96 KB, dQ staging 32 KB, two stages of what a query's thread row needs: log-sum-exp, δ, the
+// probability of a masked key and the mask bits, one word per (32 keys, query).
 constexpr int SPL_PS = 128 * 128 * 2;
 constexpr int SPL_DQ_BOX = 32 * 128;
-constexpr int SPL_BWD_SMEM = 4 * SPL_TILE + 4 * SPL_PS + 8 * SPL_DQ_BOX + 1024 + 256;
+constexpr int SPL_STAT = (3 + 4) * 128;                              // 32-bit words per stage
+constexpr int SPL_BWD_SMEM = 4 * SPL_TILE + 3 * SPL_PS + 8 * SPL_DQ_BOX + 2 * SPL_STAT * 4 + 1024 + 256;
 static_assert(SPL_BWD_SMEM <= 232448, "split attention backward: shared memory");
 
 template <bool MASKED>
@@ -346,20 +358,20 @@ __global__ void __launch_bounds__(SPL_THREADS, 1)
 attn_split_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                       const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
                       const __grid_constant__ CUtensorMap tmap_dq, SplitParams p) {
-  constexpr uint32_t S_COL = 0, DP_COL = 128, DV_COL = 256, DK_COL = 320, DQ_COL = 384;
+  constexpr uint32_t S_COL = 0, DP_COL = 128, DV_COL = 256, DK_COL = 320, DQ_COL = 384, P_COL = 448;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sK = smem;
   uint8_t* sV = sK + SPL_TILE;
   uint8_t* sQ = sV + SPL_TILE;
   uint8_t* sDO = sQ + SPL_TILE;
-  uint8_t* sP = sDO + SPL_TILE;                 // hi, lo
-  uint8_t* sDS = sP + 2 * SPL_PS;               // hi, lo
-  uint8_t* sDQ = sDS + 2 * SPL_PS;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sDQ + 8 * SPL_DQ_BOX);
+  uint8_t* sDS = sDO + SPL_TILE;                // three parts: two chunks of 64 queries, 128 key rows x 128 bytes each
+  uint8_t* sDQ = sDS + 3 * SPL_PS;
+  uint32_t* sStat = reinterpret_cast<uint32_t*>(sDQ + 8 * SPL_DQ_BOX);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + 2 * SPL_STAT);
   uint64_t* kv_full = bars;
   uint64_t* qdo_full = bars + 1;
-  uint64_t* qdo_empty = bars + 2;               // also: P / dS tiles and dQ columns may be written again (with dq_empty)
+  uint64_t* qdo_empty = bars + 2;               // also: the parts of P and dS may be written again (and, with dq_empty, the dQ columns)
   uint64_t* sdp_full = bars + 3;
   uint64_t* pds_full = bars + 4;
   uint64_t* dq_full = bars + 5;
@@ -404,11 +416,10 @@ attn_split_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     }
     __syncwarp();
   } else if (warp_idx == 1) {
-    constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);   // Q·Kᵀ, dO·Vᵀ
-    constexpr uint32_t idesc_t = make_idesc_bf16(128, 64, true, true);      // Pᵀ·dO, dSᵀ·Q
-    constexpr uint32_t idesc_q = make_idesc_bf16(128, 64, false, true);     // dS·K
-    const uint32_t k_addr = smem_u32(sK), v_addr = smem_u32(sV), q_addr = smem_u32(sQ), do_addr = smem_u32(sDO);
-    const uint32_t p_addr = smem_u32(sP), ds_addr = smem_u32(sDS);
+    constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);   // K·Qᵀ, V·dOᵀ
+    constexpr uint32_t idesc_t = make_idesc_bf16(128, 64, false, true);     // Pᵀ·dO, dSᵀ·Q
+    constexpr uint32_t idesc_q = make_idesc_bf16(128, 64, true, true);      // dS·K
+    const uint32_t k_addr = smem_u32(sK), v_addr = smem_u32(sV), q_addr = smem_u32(sQ), do_addr = smem_u32(sDO), ds_addr = smem_u32(sDS);
     const int ksteps = (p.d + 15) / 16;
     bool ok = __all_sync(0xffffffffu, tc_wait(kv_full, 0, stop));
     for (int it = 0; it < iters; ++it) {
@@ -416,10 +427,10 @@ attn_split_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       tc_fence_after_sync();
       if (ok && elect_one()) {
         for (int kk = 0; kk < ksteps; ++kk)
-          umma_f16_ss(tmem_base + S_COL, make_smem_desc_sw128(q_addr + kk * 32, 0, 1024), make_smem_desc_sw128(k_addr + kk * 32, 0, 1024), idesc_s,
+          umma_f16_ss(tmem_base + S_COL, make_smem_desc_sw128(k_addr + kk * 32, 0, 1024), make_smem_desc_sw128(q_addr + kk * 32, 0, 1024), idesc_s,
                       kk > 0 ? 1u : 0u);
         for (int kk = 0; kk < ksteps; ++kk)
-          umma_f16_ss(tmem_base + DP_COL, make_smem_desc_sw128(do_addr + kk * 32, 0, 1024), make_smem_desc_sw128(v_addr + kk * 32, 0, 1024), idesc_s,
+          umma_f16_ss(tmem_base + DP_COL, make_smem_desc_sw128(v_addr + kk * 32, 0, 1024), make_smem_desc_sw128(do_addr + kk * 32, 0, 1024), idesc_s,
                       kk > 0 ? 1u : 0u);
         umma_commit(sdp_full);
       }
@@ -429,88 +440,135 @@ attn_split_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       tc_fence_after_sync();
       if (ok && elect_one()) {
 #pragma unroll
-        for (int part = 0; part < 2; ++part) {       // dQ first: its drain is the only consumer that is waited for
+        for (int part = 0; part < 3; ++part) {       // dQ first: its drain is the only consumer that is waited for
 #pragma unroll
-          for (int kk = 0; kk < 8; ++kk)
-            umma_f16_ss(tmem_base + DQ_COL, make_smem_desc_sw128(ds_addr + part * SPL_PS + (kk / 4) * (128 * 128) + (kk % 4) * 32, 0, 1024),
+          for (int kk = 0; kk < 8; ++kk)             // 16 keys per step
+            umma_f16_ss(tmem_base + DQ_COL, make_smem_desc_sw128(ds_addr + part * SPL_PS + kk * 2048, 128 * 128, 1024),
                         make_smem_desc_sw128(k_addr + kk * 2048, 128 * 128, 1024), idesc_q, (part > 0 || kk > 0) ? 1u : 0u);
         }
         umma_commit(dq_full);
 #pragma unroll
-        for (int part = 0; part < 2; ++part) {
+        for (int kk = 0; kk < 8; ++kk) {             // 16 queries per step
+          const uint64_t bo = make_smem_desc_sw128(do_addr + kk * 2048, 128 * 128, 1024), bq = make_smem_desc_sw128(q_addr + kk * 2048, 128 * 128, 1024);
+          umma_f16_ts(tmem_base + DV_COL, tmem_base + P_COL + kk * 8, bo, idesc_t, (it > 0 || kk > 0) ? 1u : 0u);
+          umma_f16_ts(tmem_base + DV_COL, tmem_base + S_COL + kk * 16, bo, idesc_t, 1u);
+          umma_f16_ts(tmem_base + DV_COL, tmem_base + S_COL + kk * 16 + 8, bo, idesc_t, 1u);
 #pragma unroll
-          for (int kk = 0; kk < 8; ++kk)
-            umma_f16_ss(tmem_base + DV_COL, make_smem_desc_sw128(p_addr + part * SPL_PS + kk * 2048, 128 * 128, 1024),
-                        make_smem_desc_sw128(do_addr + kk * 2048, 128 * 128, 1024), idesc_t, (it > 0 || part > 0 || kk > 0) ? 1u : 0u);
-#pragma unroll
-          for (int kk = 0; kk < 8; ++kk)
-            umma_f16_ss(tmem_base + DK_COL, make_smem_desc_sw128(ds_addr + part * SPL_PS + kk * 2048, 128 * 128, 1024),
-                        make_smem_desc_sw128(q_addr + kk * 2048, 128 * 128, 1024), idesc_t, (it > 0 || part > 0 || kk > 0) ? 1u : 0u);
+          for (int part = 0; part < 3; ++part)
+            umma_f16_ss(tmem_base + DK_COL, make_smem_desc_sw128(ds_addr + part * SPL_PS + (kk / 4) * (128 * 128) + (kk % 4) * 32, 0, 1024), bq, idesc_t,
+                        (it > 0 || kk > 0 || part > 0) ? 1u : 0u);
         }
         umma_commit(qdo_empty);
       }
       __syncwarp();
     }
   } else {
-    const int quad = warp_idx % 4, half = (warp_idx - 2) / 4;        // this warp's 64 of the 128 key columns
-    const int r = quad * 32 + lane;
+    const int quad = warp_idx % 4, half = (warp_idx - 2) / 4;        // this warp's 32 of the 128 keys, its 64 of a tile's 128 queries
+    const int r = quad * 32 + lane, k_idx = k0 + r;
     const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
     const size_t bh = static_cast<size_t>(batch) * p.A + head;
-    for (int it = 0; it < iters; ++it) {
-      const int q_blk = i_begin + it, q_idx = q_blk * 128 + r;
-      const bool q_ok = q_idx < p.Sq;
-      const float lse2 = q_ok ? p.lse[bh * p.Sq + q_idx] * SPL_LOG2E : 0.f;
-      const float delta_s = q_ok ? p.delta[bh * p.Sq + q_idx] * p.scale : 0.f;
-      [[maybe_unused]] uint2 bits = make_uint2(0, 0);
-      [[maybe_unused]] float fill = 0.f;
-      if constexpr (MASKED) {
-        const long row = batch * p.mask_b + head * p.mask_a + min(q_idx, p.Sq - 1);
-        bits = *reinterpret_cast<const uint2*>(p.mask + row * p.pitch + (k0 / 32) + half * 2);
-        fill = p.fill[row];
+    // what a tile's queries bring along: 128 threads fetch a query's numbers, the other 128 its mask words, one tile ahead
+    const int tid = static_cast<int>(threadIdx.x) - 64, fq = tid & 127;
+    float f_lse = 0.f, f_delta = 0.f;
+    [[maybe_unused]] float f_fill = 0.f;
+    [[maybe_unused]] uint4 f_bits = make_uint4(0, 0, 0, 0);
+    auto fetch = [&](int it) {
+      const int q = min((i_begin + it) * 128 + fq, p.Sq - 1);        // (queries behind Sq are masked below)
+      [[maybe_unused]] const long row = MASKED ? batch * p.mask_b + head * p.mask_a + q : 0;
+      if (tid < 128) {
+        f_lse = p.lse[bh * p.Sq + q];
+        f_delta = p.delta[bh * p.Sq + q];
+        if constexpr (MASKED) f_fill = p.fill[row];
+      } else if constexpr (MASKED) {
+        f_bits = *reinterpret_cast<const uint4*>(p.mask + row * p.pitch + k0 / 32);
       }
-      const int key_lim = !q_ok ? 0 : (p.causal ? min(p.Sk, q_idx + p.off + 1) : p.Sk);
-      tc_wait(sdp_full, it & 1, stop);        // S(it) was issued after the products of block it-1 had read the P / dS tiles (one Q stage)
+    };
+    fetch(0);
+    for (int it = 0; it < iters; ++it) {
+      const int q_blk = i_begin + it;
+      uint32_t* st = sStat + (it & 1) * SPL_STAT;                    // (whoever still reads the tile before last has not passed the barrier below)
+      if (tid < 128) {
+        const float lse2 = f_lse * SPL_LOG2E;
+        st[fq] = __float_as_uint(lse2);
+        st[128 + fq] = __float_as_uint(f_delta * p.scale);
+        if constexpr (MASKED) st[256 + fq] = __float_as_uint(fast_exp2(f_fill - lse2));
+      } else if constexpr (MASKED) {
+        st[384 + fq] = f_bits.x;
+        st[512 + fq] = f_bits.y;
+        st[640 + fq] = f_bits.z;
+        st[768 + fq] = f_bits.w;
+      }
+      __syncwarp();
+      asm volatile("bar.sync 1, 256;\n" ::: "memory");              // the eight warps of this branch
+      if (it + 1 < iters) fetch(it + 1);
+      // queries [q_lo, q_hi) of this half see key k_idx (the mask apart)
+      const int q_first = q_blk * 128 + half * 64;
+      const int q_lo = k_idx >= p.Sk ? 128 : (p.causal ? k_idx - p.off - q_first : 0), q_hi = p.Sq - q_first;
+      const bool edge = k0 + 128 > p.Sk || q_blk * 128 + 128 > p.Sq || (p.causal && k0 + 127 - p.off > q_blk * 128);
+      tc_wait(sdp_full, it & 1, stop);        // S(it) was issued after the products of block it-1 had read the parts of P and dS (one Q stage)
       __syncwarp();
       tc_fence_after_sync();
+      auto tile = [&](auto edge_tag) {
+        constexpr bool EDGE = decltype(edge_tag)::value;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {            // 16 keys at a time: four packed tiles of 32 would spill
-        uint32_t ts[16], td[16];
-        tmem_ld_32x32b_x16(tmem_base + lane_off + S_COL + half * 64 + c * 16, ts);
-        tmem_ld_32x32b_x16(tmem_base + lane_off + DP_COL + half * 64 + c * 16, td);
-        tmem_ld_wait();
-        [[maybe_unused]] const uint32_t word = (c < 2 ? bits.x : bits.y) >> ((c & 1) * 16);
-        uint32_t ph[8], pl[8], dh[8], dl[8];
+        for (int c = 0; c < 4; ++c) {          // 16 queries at a time
+          const int kk = half * 4 + c;
+          uint32_t ts[16], td[16];
+          tmem_ld_32x32b_x16(tmem_base + lane_off + S_COL + kk * 16, ts);
+          tmem_ld_32x32b_x16(tmem_base + lane_off + DP_COL + kk * 16, td);
+          tmem_ld_wait();
+          uint32_t pp[3][8], dd[3][8];
 #pragma unroll
-        for (int i = 0; i < 16; i += 2) {
-          float pv[2], dv[2];
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            float x = __uint_as_float(ts[i + e]) * p.scale_log2;
-            bool on = true;
+          for (int v = 0; v < 4; ++v) {
+            const int at = kk * 16 + v * 4;
+            const float4 l4 = *reinterpret_cast<const float4*>(st + at), d4 = *reinterpret_cast<const float4*>(st + 128 + at);
+            float4 m4 = make_float4(0.f, 0.f, 0.f, 0.f);
+            uint4 w4 = make_uint4(0, 0, 0, 0);
             if constexpr (MASKED) {
-              on = (word >> (i + e)) & 1u;
-              x = on ? x : fill;
+              m4 = *reinterpret_cast<const float4*>(st + 256 + at);
+              w4 = *reinterpret_cast<const uint4*>(st + 384 + quad * 128 + at);
             }
-            const bool in = k0 + half * 64 + c * 16 + i + e < key_lim;
-            pv[e] = in ? fast_exp2(x - lse2) : 0.f;
-            dv[e] = on ? pv[e] * fmaf(__uint_as_float(td[i + e]), p.scale, -delta_s) : 0.f;    // a masked score is a constant
-          }
-          ph[i / 2] = split_hi(pv[0], pv[1]);
-          pl[i / 2] = split_lo(pv[0], pv[1], ph[i / 2]);
-          dh[i / 2] = split_hi(dv[0], dv[1]);
-          dl[i / 2] = split_lo(dv[0], dv[1], dh[i / 2]);
-        }
-        uint8_t* prow = sP + half * (128 * 128) + r * 128;
-        uint8_t* drow = sDS + half * (128 * 128) + r * 128;
+            const float ls[4] = {l4.x, l4.y, l4.z, l4.w}, de[4] = {d4.x, d4.y, d4.z, d4.w};
+            [[maybe_unused]] const float pm[4] = {m4.x, m4.y, m4.z, m4.w};
+            [[maybe_unused]] const uint32_t wd[4] = {w4.x, w4.y, w4.z, w4.w};
+            float pv[4], dv[4];
 #pragma unroll
-        for (int v = 0; v < 2; ++v) {
-          const int phys = ((c * 2 + v) ^ (r & 7)) * 16;
-          *reinterpret_cast<uint4*>(prow + phys) = make_uint4(ph[4 * v], ph[4 * v + 1], ph[4 * v + 2], ph[4 * v + 3]);
-          *reinterpret_cast<uint4*>(prow + SPL_PS + phys) = make_uint4(pl[4 * v], pl[4 * v + 1], pl[4 * v + 2], pl[4 * v + 3]);
-          *reinterpret_cast<uint4*>(drow + phys) = make_uint4(dh[4 * v], dh[4 * v + 1], dh[4 * v + 2], dh[4 * v + 3]);
-          *reinterpret_cast<uint4*>(drow + SPL_PS + phys) = make_uint4(dl[4 * v], dl[4 * v + 1], dl[4 * v + 2], dl[4 * v + 3]);
+            for (int e = 0; e < 4; ++e) {
+              const int i = 4 * v + e;
+              pv[e] = fast_exp2(fmaf(__uint_as_float(ts[i]), p.scale_log2, -ls[e]));
+              dv[e] = pv[e] * fmaf(__uint_as_float(td[i]), p.scale, -de[e]);
+              if constexpr (MASKED) {
+                const bool on = (wd[e] >> lane) & 1u;
+                pv[e] = on ? pv[e] : pm[e];
+                dv[e] = on ? dv[e] : 0.f;                            // a masked score is a constant
+              }
+              if constexpr (EDGE) {
+                const bool in = c * 16 + i >= q_lo && c * 16 + i < q_hi;
+                pv[e] = in ? pv[e] : 0.f;
+                dv[e] = in ? dv[e] : 0.f;
+              }
+            }
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              split3(pv[2 * e], pv[2 * e + 1], pp[0][2 * v + e], pp[1][2 * v + e], pp[2][2 * v + e]);
+              split3(dv[2 * e], dv[2 * e + 1], dd[0][2 * v + e], dd[1][2 * v + e], dd[2][2 * v + e]);
+            }
+          }
+          tmem_st_32x32b_x8(tmem_base + lane_off + P_COL + kk * 8, pp[0]);
+          tmem_st_32x32b_x8(tmem_base + lane_off + S_COL + kk * 16, pp[1]);
+          tmem_st_32x32b_x8(tmem_base + lane_off + S_COL + kk * 16 + 8, pp[2]);
+          uint8_t* drow = sDS + half * (128 * 128) + r * 128;
+#pragma unroll
+          for (int v = 0; v < 2; ++v) {
+            const int phys = ((c * 2 + v) ^ (r & 7)) * 16;
+#pragma unroll
+            for (int part = 0; part < 3; ++part)
+              *reinterpret_cast<uint4*>(drow + part * SPL_PS + phys) = make_uint4(dd[part][4 * v], dd[part][4 * v + 1], dd[part][4 * v + 2], dd[part][4 * v + 3]);
+          }
         }
-      }
+      };
+      if (edge) tile(std::true_type{}); else tile(std::false_type{});
+      tmem_st_wait();
       tc_fence_before_sync();
       fence_proxy_async();
       __syncwarp();
@@ -553,7 +611,6 @@ attn_split_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     tc_wait(qdo_empty, (iters - 1) & 1, stop);
     __syncwarp();
     tc_fence_after_sync();
-    const int k_idx = k0 + r;
 #pragma unroll
     for (int which = 0; which < 2; ++which) {
       uint32_t t[32];
@@ -586,11 +643,10 @@ attn_split_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   }
 }
 
-// delta[b, a, s] = Σ_d dO · (O + O_lo); 8 lanes per row, rows in memory order of the [b, s, a, d] tensors; clears the dQ accumulator
+// delta[b, a, s] = Σ_d dO · O, O as the forward left it in fp32; 8 lanes per row, rows in memory order of the [b, s, a, d] tensors; clears the dQ accumulator
 __global__ void __launch_bounds__(256)
-attn_split_delta_kernel(const __nv_bfloat16* __restrict__ dout, long sb, long sa, long ss, const __nv_bfloat16* __restrict__ o,
-                        const __nv_bfloat16* __restrict__ o_lo, float* __restrict__ delta, int B, int A, int S, int d,
-                        float4* __restrict__ zero_fill, long zero_n4) {
+attn_split_delta_kernel(const __nv_bfloat16* __restrict__ dout, long sb, long sa, long ss, const float* __restrict__ o32,
+                        float* __restrict__ delta, int B, int A, int S, int d, float4* __restrict__ zero_fill, long zero_n4) {
   const long total = static_cast<long>(B) * A * S;
   const long gid = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x, threads = static_cast<long>(gridDim.x) * blockDim.x;
   for (long z = gid; z < zero_n4; z += threads) zero_fill[z] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -603,13 +659,9 @@ attn_split_delta_kernel(const __nv_bfloat16* __restrict__ dout, long sb, long sa
     const long b = r / (static_cast<long>(A) * S);
     if (r < total && sub * 8 < d) {
       const uint4 x = *reinterpret_cast<const uint4*>(dout + b * sb + a * sa + s * ss + sub * 8);
-      const uint4 y = *reinterpret_cast<const uint4*>(o + r * d + sub * 8), z = *reinterpret_cast<const uint4*>(o_lo + r * d + sub * 8);
-      const uint32_t *xw = &x.x, *yw = &y.x, *zw = &z.x;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 u = unpack_bf16(xw[e]), v = unpack_bf16(yw[e]), w = unpack_bf16(zw[e]);
-        acc += u.x * (v.x + w.x) + u.y * (v.y + w.y);
-      }
+      const float4 y = *reinterpret_cast<const float4*>(o32 + r * d + sub * 8), z = *reinterpret_cast<const float4*>(o32 + r * d + sub * 8 + 4);
+      const float2 u0 = unpack_bf16(x.x), u1 = unpack_bf16(x.y), u2 = unpack_bf16(x.z), u3 = unpack_bf16(x.w);
+      acc = ((u0.x * y.x + u0.y * y.y) + (u1.x * y.z + u1.y * y.w)) + ((u2.x * z.x + u2.y * z.y) + (u3.x * z.z + u3.y * z.w));
     }
 #pragma unroll
     for (int m = 4; m >= 1; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
@@ -686,7 +738,7 @@ extern "C" int lb_attn_mask_pack(const void* mask, int elem, unsigned long long 
   return (int)cudaGetLastError();
 }
 
-extern "C" int lb_attn_split_fwd(const void* q, const void* k, const void* v, void* o, void* o_lo, float* lse, int B, int A, int Sq, int Sk, int d,
+extern "C" int lb_attn_split_fwd(const void* q, const void* k, const void* v, void* o, float* o32, float* lse, int B, int A, int Sq, int Sk, int d,
                                  const long* qs, const long* ks, const long* vs, int causal, float scale, const uint32_t* mask,
                                  const float* fill, long mask_b, long mask_a, int* err, cudaStream_t s) {
   if (!split_sizes_ok(B, A, Sq, Sk, d, causal, scale)) return -1;
@@ -694,19 +746,19 @@ extern "C" int lb_attn_split_fwd(const void* q, const void* k, const void* v, vo
   CUtensorMap tq, tk, tv;
   if (!split_tmap(&tq, q, B, A, Sq, d, qs) || !split_tmap(&tk, k, B, A, Sk, d, ks) || !split_tmap(&tv, v, B, A, Sk, d, vs)) return -2;
   lb::SplitParams p = split_params(B, A, Sq, Sk, d, causal, scale, mask, fill, mask_b, mask_a, err);
-  p.o = (__nv_bfloat16*)o; p.o_lo = (__nv_bfloat16*)o_lo; p.lse = lse;
+  p.o = (__nv_bfloat16*)o; p.o32 = o32; p.lse = lse;
   static bool c0 = false, c1 = false;
   const dim3 grid((Sq + 127) / 128, A, B);
   cudaError_t e = mask ? split_configure(lb::attn_split_fwd_kernel<true>, lb::SPL_FWD_SMEM, c1) : split_configure(lb::attn_split_fwd_kernel<false>, lb::SPL_FWD_SMEM, c0);
   if (e != cudaSuccess) return (int)e;
-  if (mask) lb::attn_split_fwd_kernel<true><<<grid, lb::SPL_THREADS, lb::SPL_FWD_SMEM, s>>>(tq, tk, tv, p);
-  else lb::attn_split_fwd_kernel<false><<<grid, lb::SPL_THREADS, lb::SPL_FWD_SMEM, s>>>(tq, tk, tv, p);
+  if (mask) lb::attn_split_fwd_kernel<true><<<grid, lb::SPL_FWD_THREADS, lb::SPL_FWD_SMEM, s>>>(tq, tk, tv, p);
+  else lb::attn_split_fwd_kernel<false><<<grid, lb::SPL_FWD_THREADS, lb::SPL_FWD_SMEM, s>>>(tq, tk, tv, p);
   return (int)cudaGetLastError();
 }
 
 // dq / dk / dv: [B, A, S, d] views; delta fp32 [B, A, Sq] and dq_acc fp32 [B, A, Sq, d] are scratch
-extern "C" int lb_attn_split_bwd(const void* dout, const void* q, const void* k, const void* v, const void* o, const void* o_lo, const float* lse,
-                                 void* dq, void* dk, void* dv, float* delta, float* dq_acc, int B, int A, int Sq, int Sk, int d, const long* qs,
+extern "C" int lb_attn_split_bwd(const void* dout, const void* q, const void* k, const void* v, const float* o32, const float* lse, void* dq,
+                                 void* dk, void* dv, float* delta, float* dq_acc, int B, int A, int Sq, int Sk, int d, const long* qs,
                                  const long* ks, const long* vs, const long* dos, const long* dqs, const long* dks, const long* dvs, int causal,
                                  float scale, const uint32_t* mask, const float* fill, long mask_b, long mask_a, int* err, cudaStream_t s) {
   if (!split_sizes_ok(B, A, Sq, Sk, d, causal, scale)) return -1;
@@ -726,8 +778,8 @@ extern "C" int lb_attn_split_bwd(const void* dout, const void* q, const void* k,
   const long rows = (long)B * A * Sq;
   long blocks = (rows * 8 + 255) / 256;
   if (blocks > 148L * 16) blocks = 148L * 16;
-  lb::attn_split_delta_kernel<<<(unsigned)blocks, 256, 0, s>>>((const __nv_bfloat16*)dout, dos[0], dos[1], dos[2], (const __nv_bfloat16*)o,
-                                                               (const __nv_bfloat16*)o_lo, delta, B, A, Sq, d, (float4*)dq_acc, rows * d / 4);
+  lb::attn_split_delta_kernel<<<(unsigned)blocks, 256, 0, s>>>((const __nv_bfloat16*)dout, dos[0], dos[1], dos[2], o32, delta, B, A, Sq, d,
+                                                               (float4*)dq_acc, rows * d / 4);
   lb::SplitParams p = split_params(B, A, Sq, Sk, d, causal, scale, mask, fill, mask_b, mask_a, err);
   p.lse = const_cast<float*>(lse);
   p.delta = delta;

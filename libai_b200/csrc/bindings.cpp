@@ -97,10 +97,10 @@ int lb_attn_bwd128(const void* dout, const void* q, const void* k, const void* v
                    const long* g_strides, int causal, float scale, const int* kv_lens, int* err, cudaStream_t s);
 int lb_attn_mask_pack(const void* mask, int elem, unsigned long long and_mask, int Bm, int Am, int Sq, int Sk, const long* strides, int causal,
                       int off, uint32_t* words, float* fill, cudaStream_t s);
-int lb_attn_split_fwd(const void* q, const void* k, const void* v, void* o, void* o_lo, float* lse, int B, int A, int Sq, int Sk, int d,
+int lb_attn_split_fwd(const void* q, const void* k, const void* v, void* o, float* o32, float* lse, int B, int A, int Sq, int Sk, int d,
                       const long* qs, const long* ks, const long* vs, int causal, float scale, const uint32_t* mask, const float* fill, long mask_b,
                       long mask_a, int* err, cudaStream_t s);
-int lb_attn_split_bwd(const void* dout, const void* q, const void* k, const void* v, const void* o, const void* o_lo, const float* lse, void* dq,
+int lb_attn_split_bwd(const void* dout, const void* q, const void* k, const void* v, const float* o32, const float* lse, void* dq,
                       void* dk, void* dv, float* delta, float* dq_acc, int B, int A, int Sq, int Sk, int d, const long* qs, const long* ks,
                       const long* vs, const long* dos, const long* dqs, const long* dks, const long* dvs, int causal, float scale,
                       const uint32_t* mask, const float* fill, long mask_b, long mask_a, int* err, cudaStream_t s);
@@ -878,7 +878,7 @@ WaitWord& split_word() {
   return word;
 }
 
-// (o [B, A, Sq, d] as a view of [B, Sq, A, d], o_lo (what its rounding left over, only with `train`), lse)
+// (o [B, A, Sq, d] as a view of [B, Sq, A, d], with `train` the same in fp32 as [B, Sq, A, d], lse)
 std::tuple<Tensor, Tensor, Tensor> attn_split_fwd(const Tensor& q, const Tensor& k, const Tensor& v, bool causal, double scale,
                                                   const c10::optional<Tensor>& words, const c10::optional<Tensor>& fill, bool train) {
   c10::cuda::CUDAGuard guard(q.device());
@@ -890,16 +890,17 @@ std::tuple<Tensor, Tensor, Tensor> attn_split_fwd(const Tensor& q, const Tensor&
   TORCH_CHECK(k.sizes() == v.sizes() && k.size(0) == B && k.size(1) == A && k.size(3) == d, "split attention: shapes");
   const SplitMask m = split_mask(words, fill, q.device(), B, A, Sq, Sk);
   Tensor o = at::empty({B, Sq, A, d}, q.options());
-  Tensor lo = train ? at::empty({B, Sq, A, d}, q.options()) : at::empty({0}, q.options());
-  Tensor lse = at::empty({B, A, Sq}, q.options().dtype(at::kFloat));
-  check(lb_attn_split_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), train ? lo.data_ptr() : nullptr, lse.data_ptr<float>(), B, A, Sq,
+  auto f32 = q.options().dtype(at::kFloat);
+  Tensor o32 = train ? at::empty({B, Sq, A, d}, f32) : at::empty({0}, f32);
+  Tensor lse = at::empty({B, A, Sq}, f32);
+  check(lb_attn_split_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), train ? o32.data_ptr<float>() : nullptr, lse.data_ptr<float>(), B, A, Sq,
                           Sk, d, qs, ks, vs, causal ? 1 : 0, (float)scale, m.words, m.fill, m.b, m.a, split_word().device("attn_split"), cur_stream()),
         "attn_split_fwd");
-  return std::make_tuple(o.permute({0, 2, 1, 3}), lo, lse);
+  return std::make_tuple(o.permute({0, 2, 1, 3}), o32, lse);
 }
 
 // gradients into the given [B, A, S, d] views (slices of packed projections' gradients)
-void attn_split_bwd(const Tensor& dout, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& o_lo, const Tensor& lse,
+void attn_split_bwd(const Tensor& dout, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o32, const Tensor& lse,
                     Tensor dq, Tensor dk, Tensor dv, bool causal, double scale, const c10::optional<Tensor>& words,
                     const c10::optional<Tensor>& fill) {
   c10::cuda::CUDAGuard guard(q.device());
@@ -910,7 +911,7 @@ void attn_split_bwd(const Tensor& dout, const Tensor& q, const Tensor& k, const 
     g = g.contiguous();
   if (reinterpret_cast<uintptr_t>(g.data_ptr()) & 15) g = g.clone();
   TORCH_CHECK(g.sizes() == q.sizes() && dq.sizes() == q.sizes() && dk.sizes() == k.sizes() && dv.sizes() == k.sizes() && k.sizes() == v.sizes() &&
-                  o.is_contiguous() && o_lo.is_contiguous() && o.numel() == q.numel() && o_lo.numel() == q.numel(),
+                  o32.is_contiguous() && o32.scalar_type() == at::kFloat && o32.numel() == q.numel(),
               "split attention: shapes");
   long qs[3], ks[3], vs[3], gs[3], dqs[3], dks[3], dvs[3];
   split_strides(q, q.device(), qs);
@@ -920,11 +921,11 @@ void attn_split_bwd(const Tensor& dout, const Tensor& q, const Tensor& k, const 
   split_strides(dq, q.device(), dqs);
   split_strides(dk, q.device(), dks);
   split_strides(dv, q.device(), dvs);
-  TORCH_CHECK(o.device() == q.device() && o_lo.device() == q.device() && lse.device() == q.device(), "split attention: saved tensors on the device of the queries");
+  TORCH_CHECK(o32.device() == q.device() && lse.device() == q.device(), "split attention: saved tensors on the device of the queries");
   const SplitMask m = split_mask(words, fill, q.device(), B, A, Sq, Sk);
   auto f32 = q.options().dtype(at::kFloat);
   Tensor delta = at::empty({B, A, Sq}, f32), acc = at::empty({B, A, Sq, d}, f32);      // cleared by the delta kernel
-  check(lb_attn_split_bwd(g.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), o_lo.data_ptr(), lse.data_ptr<float>(), dq.data_ptr(),
+  check(lb_attn_split_bwd(g.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), o32.data_ptr<float>(), lse.data_ptr<float>(), dq.data_ptr(),
                           dk.data_ptr(), dv.data_ptr(), delta.data_ptr<float>(), acc.data_ptr<float>(), B, A, Sq, Sk, d, qs, ks, vs, gs, dqs, dks,
                           dvs, causal ? 1 : 0, (float)scale, m.words, m.fill, m.b, m.a, split_word().device("attn_split"), cur_stream()),
         "attn_split_bwd");
@@ -1101,7 +1102,7 @@ TORCH_LIBRARY(libai_b200, m) {
   m.def("sqnorm(Tensor x) -> Tensor", &sqnorm);
   m.def("attn_mask_pack(Tensor mask, bool causal) -> (Tensor, Tensor)", &attn_mask_pack);
   m.def("attn_split_fwd(Tensor q, Tensor k, Tensor v, bool causal, float scale, Tensor? words, Tensor? fill, bool train) -> (Tensor, Tensor, Tensor)", &attn_split_fwd);
-  m.def("attn_split_bwd(Tensor dout, Tensor q, Tensor k, Tensor v, Tensor o, Tensor o_lo, Tensor lse, Tensor(a!) dq, Tensor(b!) dk, Tensor(c!) dv, bool causal, float scale, Tensor? words, Tensor? fill) -> ()", &attn_split_bwd);
+  m.def("attn_split_bwd(Tensor dout, Tensor q, Tensor k, Tensor v, Tensor o32, Tensor lse, Tensor(a!) dq, Tensor(b!) dk, Tensor(c!) dv, bool causal, float scale, Tensor? words, Tensor? fill) -> ()", &attn_split_bwd);
   m.def("attn_decode(Tensor q, Tensor k_new, Tensor v_new, Tensor k_past, Tensor v_past, float scale, Tensor? words, Tensor? fill) -> (Tensor, Tensor, Tensor)", &attn_decode);
   m.def("attn_fwd(Tensor q, Tensor k, Tensor v, bool causal, float scale, Tensor? kv_lens, Tensor? bias=None, Tensor? alibi_slopes=None, float p_drop=0.0, int salt=0) -> (Tensor, Tensor, Tensor)", &attn_fwd);
   m.def("attn_bwd(Tensor dout, Tensor q, Tensor k, Tensor v, Tensor o, Tensor lse, bool causal, float scale, Tensor? kv_lens, Tensor? bias=None, Tensor? alibi_slopes=None, Tensor(a!)? dbias=None, float p_drop=0.0, Tensor? rng_state=None) -> (Tensor, Tensor, Tensor, Tensor)", &attn_bwd);

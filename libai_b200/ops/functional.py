@@ -689,17 +689,17 @@ class _SplitAttnFn(torch.autograd.Function):
         q, k, v = _split_views(layout, ts)
         words, fill = (None, None) if mask is None else _pack_mask(ext, mask, q, k.shape[2], causal)
         train = any(ctx.needs_input_grad[4:])
-        o, o_lo, lse = ext.attn_split_fwd(q, k, v, causal and mask is None, scale, words, fill, train)
+        o, o32, lse = ext.attn_split_fwd(q, k, v, causal and mask is None, scale, words, fill, train)
         count_launch()
         out = o if layout == "q_k_v" else o.permute(0, 2, 1, 3)
         if train:
-            ctx.save_for_backward(out, o_lo, lse, words, fill, *ts)
+            ctx.save_for_backward(o32, lse, words, fill, *ts)
             ctx.layout, ctx.causal, ctx.scale, ctx.mask = layout, causal, scale, mask
         return out
 
     @staticmethod
     def backward(ctx, go):
-        o, o_lo, lse, words, fill, *ts = ctx.saved_tensors
+        o32, lse, words, fill, *ts = ctx.saved_tensors
         q, k, v = _split_views(ctx.layout, ts)
         if torch.is_grad_enabled():            # a graph of the gradients is wanted: differentiate the unfused form
             out = attention_ref(q, k, v, causal=ctx.causal, scale=ctx.scale, mask=ctx.mask)
@@ -709,11 +709,10 @@ class _SplitAttnFn(torch.autograd.Function):
             return (None,) * 4 + tuple(next(grads) if n else None for n in ctx.needs_input_grad[4:])
         if ctx.layout == "q_k_v":              # gradients backed by [b, s, a, d], as the projections around an attention read them
             gs = [torch.empty(t.shape[0], t.shape[2], t.shape[1], t.shape[3], dtype=t.dtype, device=t.device).permute(0, 2, 1, 3) for t in ts]
-            o = o.permute(0, 2, 1, 3).contiguous()        # (a hook on saved tensors may have packed it in another order)
         else:
             gs = [torch.empty(t.shape, dtype=t.dtype, device=t.device) for t in ts]
             go = go.permute(0, 2, 1, 3)
-        load_ext().attn_split_bwd(go, q, k, v, o, o_lo, lse, *_split_views(ctx.layout, gs), ctx.causal and words is None, ctx.scale, words, fill)
+        load_ext().attn_split_bwd(go, q, k, v, o32, lse, *_split_views(ctx.layout, gs), ctx.causal and words is None, ctx.scale, words, fill)
         count_launch(3)
         return (None,) * 4 + tuple(gs)
 

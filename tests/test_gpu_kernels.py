@@ -151,6 +151,27 @@ def test_attention_with_32_bit_probabilities(b, sq, sk, a, d, mask):
         assert err[0] <= 1.3 * err[1] + 1e-5 * float(want.norm()) + 1e-6 * math.sqrt(want.numel()), err
 
 
+@pytest.mark.parametrize("mask", ["none", "causal", "bool"])
+@pytest.mark.parametrize("b,sq,sk,a,d,common", [(2, 512, 512, 4, 48, 20.0), (1, 700, 700, 4, 24, 20.0), (1, 128, 1100, 2, 64, 6.0)])
+def test_attention_of_keys_and_values_with_a_common_part(b, sq, sk, a, d, common, mask):
+    """Biases of the projections give all keys and all values of a head a common part, which dP - delta and the sum of dS·K cancel:
+    probabilities and their gradients need their 24 bits there.  No output further from 64 bits than the unfused fp32 form's; what
+    the order of fp32 sums leaves (2^-24 of dP, some hundred times the result of the cancellation) may add a tenth."""
+    causal = mask == "causal"
+    m = _split_mask(mask, b, a, sq, sk)
+    keep = torch.ones(sq, sk, dtype=torch.bool, device="cuda").tril(sk - sq) if causal else None if m is None else m.bool()
+    q, go = _rand((b, a, sq, d), 1), _rand((b, a, sq, d), 4)
+    k, v = ((_rand((b, a, sk, d), i).float() + common * _rand((1, a, 1, d), i + 4).float()).to(BF16) for i in (2, 3))
+    got = []
+    for fn, to in ((OF.attention, BF16), (OF.attention_ref, BF16), (None, torch.float64)):
+        ts = [t.to(to).requires_grad_(True) for t in (q, k, v)]
+        y = _attend64(*ts, d ** -0.5, keep) if fn is None else fn(*ts, causal=causal, scale=d ** -0.5, mask=m)
+        got.append([y, *torch.autograd.grad(y, ts, go.to(to))])
+    for new, old, want in zip(*got):
+        err = [float((t.double() - want).norm()) for t in (new, old)]
+        assert err[0] <= 1.1 * err[1], err
+
+
 @pytest.mark.parametrize("layout", ["qkv", "q_kv"])
 def test_attention_from_packed_projections(layout):
     b, s, sk, a, d = 2, 150, 150 if layout == "qkv" else 333, 3, 48
@@ -368,7 +389,7 @@ _GRAPHLESS = {
     "rms_norm": lambda x: OF.rms_norm(x, _rand((64,), 2)),
     "bias_act": lambda x: OF.bias_act(x, _rand((64,), 2)),
     "bias_add": lambda x: OF.bias_dropout_add(x, _rand((64,), 2), _rand((3, 40, 64), 3), 0.0, False),
-    "gated_mlp": lambda x: gated_mlp(x, _W(128, 64), _W(128, 64, i=2), _W(64, 128, i=3)),
+    "gated_mlp": lambda x: gated_mlp(x, *_W(256, 64).split(128), _W(64, 128, i=3)),
     "swiglu": lambda x: OF.swiglu(x, _rand((3, 40, 64), 2)),
     "attention_64": lambda x: OF.attention(*(_rand((3, 4, 40, 64), i) + x.mean() for i in range(3)), causal=True),
     "attention_48": lambda x: OF.attention(*(_rand((3, 4, 40, 48), i) + x.mean() for i in range(3)), causal=True),
