@@ -342,7 +342,9 @@ attn_split_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 // ----------------------------------------------------------------------------------------------------------------- backward
 // One CTA per (128 keys, head, batch), looping over the query blocks that see them, with the keys on the M side:
 //   Sᵀ = K·Qᵀ, dPᵀ = V·dOᵀ;  P = exp(S - lse), dS = P ∘ (dP - δ) · scale, in three bf16 parts each;
-//   dV += Pᵀ·dO with Pᵀ from TMEM, dK += dSᵀ·Q and dQ_i = dS·K (added to the fp32 accumulator by TMA reductions) with dSᵀ from shared memory.
+//   dV += Pᵀ·dO with Pᵀ from TMEM, dK += dSᵀ·Q and dQ_i = dS·K with dSᵀ from shared memory.
+// dQ_i goes out in fp32, one layer per key block (attn_split_dq_kernel adds the layers up in order): the unfused product had a fixed order,
+// and additions into one accumulator by several CTAs have none.
 // Six tiles of parts do not fit shared memory beside the operands, so Pᵀ stays in TMEM, which wants it as [keys, queries]: the first part in
 // columns of its own, the second and third of 16 queries over the 16 Sᵀ columns that their thread has read.
 // Shared memory: K, V, Q, dO 64 KB, three dSᵀ tiles 96 KB, dQ staging 32 KB, two stages of what a query's thread row needs: log-sum-exp, δ, the
@@ -594,12 +596,10 @@ attn_split_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(dq_empty);
-        if (dq_ok && half * 32 < p.d && q_blk * 128 + quad * 32 < p.Sq) {   // boxes start inside the accumulator; its edge clips them
-          asm volatile(
-              "cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2, %3}], [%4];\n" ::"l"(
-                  reinterpret_cast<uint64_t>(&tmap_dq)),
-              "r"(half * 32), "r"(q_blk * 128 + quad * 32), "r"(static_cast<int>(bh)), "r"(smem_u32(box))
-              : "memory");
+        if (dq_ok && half * 32 < p.d && q_blk * 128 + quad * 32 < p.Sq) {   // boxes start inside the layer; its edge clips them
+          asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3}], [%4];\n" ::"l"(reinterpret_cast<uint64_t>(&tmap_dq)),
+                       "r"(half * 32), "r"(q_blk * 128 + quad * 32), "r"(static_cast<int>(blockIdx.x * gridDim.z * gridDim.y + bh)), "r"(smem_u32(box))
+                       : "memory");
         }
         tma_store_commit();
       }
@@ -643,13 +643,12 @@ attn_split_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   }
 }
 
-// delta[b, a, s] = Σ_d dO · O, O as the forward left it in fp32; 8 lanes per row, rows in memory order of the [b, s, a, d] tensors; clears the dQ accumulator
+// delta[b, a, s] = Σ_d dO · O, O as the forward left it in fp32; 8 lanes per row, rows in memory order of the [b, s, a, d] tensors
 __global__ void __launch_bounds__(256)
 attn_split_delta_kernel(const __nv_bfloat16* __restrict__ dout, long sb, long sa, long ss, const float* __restrict__ o32,
-                        float* __restrict__ delta, int B, int A, int S, int d, float4* __restrict__ zero_fill, long zero_n4) {
+                        float* __restrict__ delta, int B, int A, int S, int d) {
   const long total = static_cast<long>(B) * A * S;
   const long gid = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x, threads = static_cast<long>(gridDim.x) * blockDim.x;
-  for (long z = gid; z < zero_n4; z += threads) zero_fill[z] = make_float4(0.f, 0.f, 0.f, 0.f);
   const int sub = threadIdx.x % 8;
   const long warp_first = (gid - threadIdx.x % 32) / 8;
   for (long base = 0; warp_first + base < total; base += threads / 8) {
@@ -669,15 +668,25 @@ attn_split_delta_kernel(const __nv_bfloat16* __restrict__ dout, long sb, long sa
   }
 }
 
-// dq (bf16 view) = accumulator (fp32 [B, A, S, d]), 8 values per thread
+// dq (bf16 view) = the sum of its layers (fp32 [key blocks, B, A, S, d]) in the order of the key blocks, 8 values per thread.  Under the causal
+// mask (off >= 0) a block of 128 queries has the layers of the key blocks that it sees.
 __global__ void __launch_bounds__(256)
-attn_split_dq_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, int B, int A, int S, int d, long sb, long sa, long ss) {
+attn_split_dq_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, int B, int A, int S, int d, long sb, long sa, long ss,
+                     int key_blocks, int causal, int off) {
   const long nvec = static_cast<long>(B) * A * S * d / 8;
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < nvec; i += static_cast<long>(gridDim.x) * blockDim.x) {
-    const float4 lo = reinterpret_cast<const float4*>(acc)[2 * i], hi = reinterpret_cast<const float4*>(acc)[2 * i + 1];
     const long row = i * 8 / d;
     const int c = static_cast<int>(i * 8 % d), s = static_cast<int>(row % S), a = static_cast<int>((row / S) % A);
     const long b = row / (static_cast<long>(S) * A);
+    const int layers = causal ? min(key_blocks, (s / 128 * 128 + 127 + off) / 128 + 1) : key_blocks;
+    const float4* src = reinterpret_cast<const float4*>(acc) + 2 * i;
+    float4 lo = src[0], hi = src[1];
+#pragma unroll 4
+    for (int k = 1; k < layers; ++k) {
+      const float4 x = src[2 * nvec * k], y = src[2 * nvec * k + 1];
+      lo.x += x.x; lo.y += x.y; lo.z += x.z; lo.w += x.w;
+      hi.x += y.x; hi.y += y.y; hi.z += y.z; hi.w += y.w;
+    }
     *reinterpret_cast<uint4*>(dq + b * sb + a * sa + s * ss + c) =
         make_uint4(pack_bf16(lo.x, lo.y), pack_bf16(lo.z, lo.w), pack_bf16(hi.x, hi.y), pack_bf16(hi.z, hi.w));
   }
@@ -756,7 +765,7 @@ extern "C" int lb_attn_split_fwd(const void* q, const void* k, const void* v, vo
   return (int)cudaGetLastError();
 }
 
-// dq / dk / dv: [B, A, S, d] views; delta fp32 [B, A, Sq] and dq_acc fp32 [B, A, Sq, d] are scratch
+// dq / dk / dv: [B, A, S, d] views; delta fp32 [B, A, Sq] and dq_acc fp32 [ceil(Sk / 128), B, A, Sq, d] are scratch
 extern "C" int lb_attn_split_bwd(const void* dout, const void* q, const void* k, const void* v, const float* o32, const float* lse, void* dq,
                                  void* dk, void* dv, float* delta, float* dq_acc, int B, int A, int Sq, int Sk, int d, const long* qs,
                                  const long* ks, const long* vs, const long* dos, const long* dqs, const long* dks, const long* dvs, int causal,
@@ -765,12 +774,14 @@ extern "C" int lb_attn_split_bwd(const void* dout, const void* q, const void* k,
   if (!split_view_ok(q, qs) || !split_view_ok(k, ks) || !split_view_ok(v, vs) || !split_view_ok(dout, dos) || !split_view_ok(dq, dqs) ||
       !split_view_ok(dk, dks) || !split_view_ok(dv, dvs))
     return -3;
+  const int key_blocks = (Sk + 127) / 128;
+  if ((long)B * A * key_blocks > 0x7fffffffL) return -1;
   CUtensorMap tq, tk, tv, tdo, tdq;
   if (!split_tmap(&tq, q, B, A, Sq, d, qs) || !split_tmap(&tk, k, B, A, Sk, d, ks) || !split_tmap(&tv, v, B, A, Sk, d, vs) ||
       !split_tmap(&tdo, dout, B, A, Sq, d, dos))
     return -2;
   {
-    uint64_t dims[3] = {(uint64_t)d, (uint64_t)Sq, (uint64_t)B * A};
+    uint64_t dims[3] = {(uint64_t)d, (uint64_t)Sq, (uint64_t)B * A * key_blocks};
     uint64_t strides[3] = {4, (uint64_t)d * 4, (uint64_t)Sq * d * 4};
     uint32_t box[3] = {32, 32, 1};
     if (!lb_host::make_tmap_typed(&tdq, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, dq_acc, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B)) return -2;
@@ -778,15 +789,14 @@ extern "C" int lb_attn_split_bwd(const void* dout, const void* q, const void* k,
   const long rows = (long)B * A * Sq;
   long blocks = (rows * 8 + 255) / 256;
   if (blocks > 148L * 16) blocks = 148L * 16;
-  lb::attn_split_delta_kernel<<<(unsigned)blocks, 256, 0, s>>>((const __nv_bfloat16*)dout, dos[0], dos[1], dos[2], o32, delta, B, A, Sq, d,
-                                                               (float4*)dq_acc, rows * d / 4);
+  lb::attn_split_delta_kernel<<<(unsigned)blocks, 256, 0, s>>>((const __nv_bfloat16*)dout, dos[0], dos[1], dos[2], o32, delta, B, A, Sq, d);
   lb::SplitParams p = split_params(B, A, Sq, Sk, d, causal, scale, mask, fill, mask_b, mask_a, err);
   p.lse = const_cast<float*>(lse);
   p.delta = delta;
   p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv;
   for (int i = 0; i < 3; ++i) { p.dk_strides[i] = dks[i]; p.dv_strides[i] = dvs[i]; }
   static bool c0 = false, c1 = false;
-  const dim3 grid((Sk + 127) / 128, A, B);
+  const dim3 grid(key_blocks, A, B);
   cudaError_t e = mask ? split_configure(lb::attn_split_bwd_kernel<true>, lb::SPL_BWD_SMEM, c1) : split_configure(lb::attn_split_bwd_kernel<false>, lb::SPL_BWD_SMEM, c0);
   if (e != cudaSuccess) return (int)e;
   if (mask) lb::attn_split_bwd_kernel<true><<<grid, lb::SPL_THREADS, lb::SPL_BWD_SMEM, s>>>(tq, tk, tv, tdo, tdq, p);
@@ -795,6 +805,7 @@ extern "C" int lb_attn_split_bwd(const void* dout, const void* q, const void* k,
   if (e != cudaSuccess) return (int)e;
   blocks = (rows * d / 8 + 255) / 256;
   if (blocks > 148L * 8) blocks = 148L * 8;
-  lb::attn_split_dq_kernel<<<(unsigned)blocks, 256, 0, s>>>(dq_acc, (__nv_bfloat16*)dq, B, A, Sq, d, dqs[0], dqs[1], dqs[2]);
+  lb::attn_split_dq_kernel<<<(unsigned)blocks, 256, 0, s>>>(dq_acc, (__nv_bfloat16*)dq, B, A, Sq, d, dqs[0], dqs[1], dqs[2], key_blocks,
+                                                              causal, Sk - Sq);
   return (int)cudaGetLastError();
 }

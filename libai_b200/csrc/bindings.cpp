@@ -924,7 +924,7 @@ void attn_split_bwd(const Tensor& dout, const Tensor& q, const Tensor& k, const 
   TORCH_CHECK(o32.device() == q.device() && lse.device() == q.device(), "split attention: saved tensors on the device of the queries");
   const SplitMask m = split_mask(words, fill, q.device(), B, A, Sq, Sk);
   auto f32 = q.options().dtype(at::kFloat);
-  Tensor delta = at::empty({B, A, Sq}, f32), acc = at::empty({B, A, Sq, d}, f32);      // cleared by the delta kernel
+  Tensor delta = at::empty({B, A, Sq}, f32), acc = at::empty({(Sk + 127) / 128, B, A, Sq, d}, f32);      // dQ by key block, added up in order
   check(lb_attn_split_bwd(g.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), o32.data_ptr<float>(), lse.data_ptr<float>(), dq.data_ptr(),
                           dk.data_ptr(), dv.data_ptr(), delta.data_ptr<float>(), acc.data_ptr<float>(), B, A, Sq, Sk, d, qs, ks, vs, gs, dqs, dks,
                           dvs, causal ? 1 : 0, (float)scale, m.words, m.fill, m.b, m.a, split_word().device("attn_split"), cur_stream()),

@@ -172,6 +172,20 @@ def test_attention_of_keys_and_values_with_a_common_part(b, sq, sk, a, d, common
         assert err[0] <= 1.1 * err[1], err
 
 
+@pytest.mark.parametrize("mask", ["none", "causal", "bool"])
+@pytest.mark.parametrize("b,sq,sk,a,d", [(8, 512, 512, 8, 48), (4, 200, 1100, 4, 32), (2, 700, 700, 4, 64)])
+def test_attention_gradients_of_many_key_blocks_repeat(b, sq, sk, a, d, mask):
+    """Every query's gradient is added up over the key blocks in their order: the same bits every time."""
+    causal = mask == "causal"
+    m = torch.ones(1, 1, 1, sk, dtype=torch.bool, device="cuda") if d == 64 and mask == "none" else _split_mask(mask, b, a, sq, sk)
+    q, k, v = (_rand((b, a, s, d), i).requires_grad_(True) for i, s in ((1, sq), (2, sk), (3, sk)))
+    m = torch.ones(sq, sk, dtype=torch.bool, device="cuda").tril(sk - sq) if d == 64 and causal else m      # head dim 64 takes these kernels with a mask
+    out, go = OF.attention(q, k, v, causal=causal and d != 64, scale=d ** -0.5, mask=m), _rand((b, a, sq, d), 4)
+    first = torch.autograd.grad(out, (q, k, v), go, retain_graph=True)
+    for _ in range(5):
+        assert all(torch.equal(x, y) for x, y in zip(torch.autograd.grad(out, (q, k, v), go, retain_graph=True), first))
+
+
 @pytest.mark.parametrize("layout", ["qkv", "q_kv"])
 def test_attention_from_packed_projections(layout):
     b, s, sk, a, d = 2, 150, 150 if layout == "qkv" else 333, 3, 48
