@@ -1131,10 +1131,12 @@ static int gemm_impl(const void* a, const void* b, void* out, int M, int N, int 
   // not stay in L2 beside the output is read from HBM again for (nearly) every row block (LM head [8192, 1024] x [50304, 1024]: 32 x
   // 103 MB).  In bands of G row blocks they hold G of A and C / G of B, the least bytes at equal sides: G = sqrt(C * columns / rows of a
   // tile).  Measured, row by row -> bands: LM head 693 -> 585 us, its input gradient 641 -> 575; [2048, 4096] x [12288, 4096] 163 -> 143.
-  // Up to a B of 8 MB both orders take the same time (0.4 us more where a launch has two tiles per CTA); the fp32 accumulate epilogue
-  // writes long rows faster than bands ([2048, 4096]ᵀ x [2048, 11008] 152 against 158 us) and keeps the old order.
+  // The line lies at a B of 48 MB: from 8 to 32 MB the orders are within 1 % of each other for 2048 rows and bands 1 to 3 % behind for 8192
+  // ([8192, 1024] x [12288, 1024], 24 MB: 150 against 155 us; x [16384, 1024] 215 against 218); at 48 MB 81 against 78 us (2048 rows) and
+  // equal (8192); at 64 MB 109 against 100 and 430 against 396 us.  The fp32 accumulate epilogue writes long rows faster than bands
+  // ([2048, 4096]ᵀ x [2048, 11008] 152 against 158 us) and keeps the old order.
   p.group_m = 1;
-  if (cp.mode == lb::COMM_NONE && !tile_group && epi == 0 && (long)N * K * 2 >= (24L << 20)) {
+  if (cp.mode == lb::COMM_NONE && !tile_group && epi == 0 && (long)N * K * 2 >= (48L << 20)) {
     const double in_flight = two_cta ? sms / 2 : sms, side = two_cta ? 1.0 : (double)bn / lb::BLOCK_M;
     p.group_m = (int)(std::sqrt(in_flight * side) + 0.5);
   }

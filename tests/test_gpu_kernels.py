@@ -378,9 +378,11 @@ def test_attention_backward_head_dim_128_repeats(causal):
 
 @pytest.mark.parametrize("M", [40, 129, 1100, 2500])
 @pytest.mark.parametrize("layout", [0, 1])
-def test_gemm_tile_order_in_bands(M, layout):
-    """B beyond 24 MB: bands of row blocks, a last band of one block, ragged edges.  Whole numbers below 256: exact in bf16."""
-    N, K = (24600, 520) if layout == 0 else (264, 49160)
+@pytest.mark.parametrize("wide", [False, True])
+def test_gemm_tile_order_in_bands(M, layout, wide):
+    """B of 25 MB (row by row) and beyond 48 MB: bands of row blocks, a last band of one block, ragged edges.  Whole numbers below 256:
+    exact in bf16."""
+    N, K = (49176 if wide else 24600, 520) if layout == 0 else (264, 98312 if wide else 49160)
     g = torch.Generator(device="cuda").manual_seed(M)
     x = torch.randint(-1, 2, (M, K), generator=g, device="cuda").to(BF16)
     w = torch.randint(-1, 2, (N, K) if layout == 0 else (K, N), generator=g, device="cuda").to(BF16)
