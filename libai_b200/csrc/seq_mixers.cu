@@ -443,7 +443,7 @@ delta_scan_pair_kernel(const T* __restrict__ qkv, long ldq, int voff, const floa
       if (lane == 0) { sc[3 * CT + 2 * p] = kk; sc[3 * CT + 2 * p + 1] = qk; }
     }
     __syncthreads();
-    for (int t = 0; t < ct; t += 2) {
+    auto pair = [&](int t, auto two_tag) {
       const ulonglong2* k0p = reinterpret_cast<const ulonglong2*>(sk + t * DP) + r;
       const ulonglong2* k1p = reinterpret_cast<const ulonglong2*>(sk + (t + 1) * DP) + r;
       const ulonglong2* q0p = reinterpret_cast<const ulonglong2*>(sq + t * DP) + r;
@@ -489,13 +489,13 @@ delta_scan_pair_kernel(const T* __restrict__ qkv, long ldq, int voff, const floa
       }
 #pragma unroll
       for (int m = 0; m < 4; ++m) w[m] += __shfl_xor_sync(0xffffffffu, w[m], 2);
-      const bool two = t + 1 < ct;                // the last token of an odd count: k1 = q1 = 0, u1 = 0 (even behind a u0 that is not finite), no decay
+      constexpr bool two = decltype(two_tag)::value;   // the last of an odd number of tokens: no second decay, no second write (0 times what is not finite)
       const float b0 = sc[t], b1 = sc[t + 1], g0 = sc[CT + t], g1 = two ? sc[CT + t + 1] : 1.f, kq0 = sc[2 * CT + t], kq1 = sc[2 * CT + t + 1];
       const float kk = sc[3 * CT + t], qk = sc[3 * CT + t + 1];
       const int vc = cg * CPT + (CPT == 2 ? bit0 : 0);
       const float u0 = b0 * (ldf(sv + t * VB + vc) - g0 * w[0]);
       const float o0 = g0 * w[1] + kq0 * u0;
-      const float u1 = two ? b1 * (ldf(sv + (t + 1) * VB + vc) - g1 * (g0 * w[2] + kk * u0)) : 0.f;
+      const float u1 = b1 * (ldf(sv + (t + 1) * VB + vc) - g1 * (g0 * w[2] + kk * u0));
       const float o1 = g1 * (g0 * w[3] + qk * u0) + kq1 * u1;
       const float gg = g0 * g1, w0 = g1 * u0;
       const unsigned long long G = pack2(gg, gg);
@@ -512,11 +512,16 @@ delta_scan_pair_kernel(const T* __restrict__ qkv, long ldq, int voff, const floa
       }
 #pragma unroll
       for (int c = 0; c < CPT; ++c) {
-        const unsigned long long p0 = pack2(U0[c], U0[c]), p1 = pack2(U1[c], U1[c]);
+        const unsigned long long p0 = pack2(U0[c], U0[c]);
+        [[maybe_unused]] const unsigned long long p1 = pack2(U1[c], U1[c]);
 #pragma unroll
         for (int d = 0; d < D4; ++d) {
-          s[c][2 * d] = fma2(K1[d].x, p1, fma2(K0[d].x, p0, mul2(s[c][2 * d], G)));
-          s[c][2 * d + 1] = fma2(K1[d].y, p1, fma2(K0[d].y, p0, mul2(s[c][2 * d + 1], G)));
+          s[c][2 * d] = fma2(K0[d].x, p0, mul2(s[c][2 * d], G));
+          s[c][2 * d + 1] = fma2(K0[d].y, p0, mul2(s[c][2 * d + 1], G));
+          if constexpr (two) {
+            s[c][2 * d] = fma2(K1[d].x, p1, s[c][2 * d]);
+            s[c][2 * d + 1] = fma2(K1[d].y, p1, s[c][2 * d + 1]);
+          }
         }
       }
       if (r < CPT && j0 + vc < V) {
@@ -524,7 +529,10 @@ delta_scan_pair_kernel(const T* __restrict__ qkv, long ldq, int voff, const floa
         o[0] = o0;
         if (two) o[(long)H * V] = o1;
       }
-    }
+    };
+    int t = 0;
+    for (; t + 1 < ct; t += 2) pair(t, std::true_type{});
+    if (t < ct) pair(t, std::false_type{});
   }
 #pragma unroll
   for (int c = 0; c < CPT; ++c) {
