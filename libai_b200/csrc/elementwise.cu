@@ -227,7 +227,9 @@ __global__ void rope_kernel(const __nv_bfloat16* __restrict__ x, const float* __
 
 // The same on 16-byte vectors: a block owns one token, a thread one vector of the first half of a head (and its partner in the
 // second half), so the token's cos / sin sit in registers while the heads go by.  Bandwidth-bound (read and write the packed
-// projection once, 101 MB for [2048, 32, 3 x 128]): 84.6 us with one element pair per thread, 15.6 us with this kernel.
+// projection once, 101 MB for [2048, 32, 3 x 128]): 84.6 us with one element pair per thread, 15.6 us with this kernel.  Few tokens
+// (a generation step) are split over the heads as well, a pass per block: [1, 64, 3 x 128] 2.2 us with one pair per thread, 4.0 us by one
+// block of this kernel, 2.1 us by six.
 // Needs D % 16 == 0, 16-byte aligned tensors and D / 16 <= 32; other shapes keep the scalar kernel below.
 __global__ void __launch_bounds__(256)
 rope_qkv_vec_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ cosv, const float* __restrict__ sinv,
@@ -254,7 +256,7 @@ rope_qkv_vec_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict
     }
     const size_t base = static_cast<size_t>(tok) * A * 3 * D;
     const int parts = copy_v ? 3 : 2;
-    for (int r = lane_row; r < A * parts; r += rows_per_pass) {
+    for (int r = blockIdx.y * rows_per_pass + lane_row; r < A * parts; r += rows_per_pass * gridDim.y) {
       const int head = r / parts, part = r % parts;
       const size_t at = base + static_cast<size_t>(head) * 3 * D + static_cast<size_t>(part) * D + c;
       uint4 q1 = *reinterpret_cast<const uint4*>(x + at), q2 = *reinterpret_cast<const uint4*>(x + at + half);
@@ -682,8 +684,10 @@ extern "C" int lb_rope_qkv(const void* x, const float* cosv, const float* sinv, 
                         reinterpret_cast<uintptr_t>(sinv);
   if (D % 16 == 0 && D <= 512 && (any & 15) == 0) {
     const long tokens = heads / A;
-    const int grid = (int)(tokens < 148L * 8 ? tokens : 148L * 8);    // eight blocks of 256 threads per SM
-    lb::rope_qkv_vec_kernel<<<grid, 256, 0, s>>>((const bf16*)x, cosv, sinv, (bf16*)y, (int)tokens, S, A, D, pos_offset, backward, copy_v);
+    const int gx = (int)(tokens < 148L * 8 ? tokens : 148L * 8);      // eight blocks of 256 threads per SM
+    const int rows_per_pass = 256 / (D / 16), passes = (A * (copy_v ? 3 : 2) + rows_per_pass - 1) / rows_per_pass;
+    const int room = 148 * 8 / gx, gy = passes < room ? passes : room;
+    lb::rope_qkv_vec_kernel<<<dim3((unsigned)gx, (unsigned)gy), 256, 0, s>>>((const bf16*)x, cosv, sinv, (bf16*)y, (int)tokens, S, A, D, pos_offset, backward, copy_v);
     return (int)cudaGetLastError();
   }
   lb::rope_qkv_kernel<<<ew_grid((size_t)heads * (copy_v ? 3 : 2) * D / 2, 256), 256, 0, s>>>(

@@ -87,7 +87,8 @@ def test_norm_weight_gradients_of_wide_rows_repeat(rows, h, rms):
     assert all(torch.equal(r, runs[0]) for r in runs)
 
 
-@pytest.mark.parametrize("b,s,a,d,off", [(1, 1, 1, 16, 0), (2, 37, 3, 128, 5), (1, 2100, 4, 64, 0), (3, 9, 5, 48, 1), (2, 7, 2, 24, 3), (1, 5, 32, 256, 0)])
+@pytest.mark.parametrize("b,s,a,d,off", [(1, 1, 1, 16, 0), (2, 37, 3, 128, 5), (1, 2100, 4, 64, 0), (3, 9, 5, 48, 1), (2, 7, 2, 24, 3), (1, 5, 32, 256, 0),
+                                         (1, 1, 64, 128, 9), (4, 1, 37, 128, 0), (1, 700, 12, 64, 0)])
 def test_rotary_on_the_packed_projection(b, s, a, d, off):
     qkv, g = _rand((b, s, a, 3 * d), 1), _rand((b, s, a, 3 * d), 2)
     ang = torch.outer(torch.arange(s + off, device="cuda").float(), 1.0 / 10000 ** (torch.arange(0, d, 2, device="cuda") / d))
