@@ -50,7 +50,7 @@ attn_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   uint8_t* sQ = sV + B128_KV;                          // B128_ST stages of two chunks, 64 rows x 128 bytes each
   uint8_t* sDO = sQ + B128_ST * B128_Q;
   uint8_t* sDS = sDO + B128_ST * B128_Q;                     // 2 x dSᵀ: 128 key rows x 128 bytes
-  uint8_t* sDQ = sDS + 2 * B128_DS;                    // one [32 queries x 32 floats] box per softmax warp
+  uint8_t* sDQ = sDS + 2 * B128_DS;                    // two [32 queries x 32 floats] boxes per warp that drains dQ
   float* sStat = reinterpret_cast<float*>(sDQ + 8 * B128_BOX);
   uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + B128_ST * 128);
   uint64_t* kv_full = bars;          // 1

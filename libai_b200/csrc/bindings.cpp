@@ -5,7 +5,6 @@
 #include <ATen/cuda/CUDAGeneratorImpl.h>
 #include <cstring>
 #include <mutex>
-#include <mutex>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/library.h>
 #include <torch/torch.h>
@@ -783,7 +782,6 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> attn_bwd(const Tensor& dout, const Te
   Tensor dq = dqkv.select(3, 0).permute({0, 2, 1, 3});
   Tensor dk = dqkv.select(3, 1).permute({0, 2, 1, 3});
   Tensor dv = dqkv.select(3, 2).permute({0, 2, 1, 3});
-  Tensor delta = at::empty({B, A, S}, q.options().dtype(at::kFloat));
   Tensor dq_acc = at::empty({B, A, S, D}, q.options().dtype(at::kFloat));   // cleared by the delta kernel
   TORCH_CHECK(o.stride(3) == 1, "attn_bwd: o must have contiguous D");
   Tensor dout_c = dout;
@@ -813,6 +811,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> attn_bwd(const Tensor& dout, const Te
           "attn_bwd128");
     return std::make_tuple(dq, dk, dv, dqkv);
   }
+  Tensor delta = at::empty({B, A, S}, q.options().dtype(at::kFloat));
   check(lb_attn_bwd(dout_c.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr<float>(),
                     dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), delta.data_ptr<float>(), dq_acc.data_ptr<float>(), B, A,
                     S, D, qs, ks, vs, ds, causal ? 1 : 0, (float)scale,

@@ -25,7 +25,8 @@ struct GsCfg {
   static constexpr uint32_t TMEM = NT < 32 ? 32 : NT;
   static_assert(PART_BYTES <= 2 * STAGE, "partial sums fit the pipeline");
 };
-constexpr int GS_MAX_STAGES = 12, GS_TAIL = 1024 + 256;   // alignment, barriers
+constexpr int GS_SMEM = 104000;                   // of pipeline: two CTAs per SM (one with twice the stages leaves no room for clusters of 8 in some GPCs)
+constexpr int GS_MAX_STAGES = GS_SMEM / GsCfg<16>::STAGE, GS_TAIL = 1024 + 256;   // alignment, barriers
 
 struct GemmSmallParams {
   int M, N, K, kb_total, kb_per_cta, stages;
@@ -191,14 +192,13 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 template <int NT, int RANKS>
 cudaError_t launch_gemm_small_r(const CUtensorMap& tw, const CUtensorMap& tx, GemmSmallParams p, cudaStream_t s) {
   auto kern = gemm_small_kernel<NT, RANKS>;
-  const int fit = 104000 / GsCfg<NT>::STAGE;       // two CTAs per SM (one with twice the stages leaves no room for clusters of 8 in some GPCs)
+  const int fit = GS_SMEM / GsCfg<NT>::STAGE;
   p.stages = p.kb_per_cta < 2 ? 2 : p.kb_per_cta;
   if (p.stages > fit) p.stages = fit;
-  if (p.stages > GS_MAX_STAGES) p.stages = GS_MAX_STAGES;
   const int smem = p.stages * GsCfg<NT>::STAGE + GS_TAIL;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 104000 + GS_TAIL);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GS_SMEM + GS_TAIL);
     if (e != cudaSuccess) return e;
     configured = true;
   }

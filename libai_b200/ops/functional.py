@@ -787,8 +787,7 @@ def attention(q, k, v, *, causal: bool = False, scale: Optional[float] = None, m
         and (bias is None or (bias.shape[-1] == k.shape[-2] and bias.shape[-2] == q.shape[-2]))
     ):
         # strided [b, a, s, d] views of the packed QKV projection are consumed directly (TMA strides)
-        return _call(_FlashAttnFn, q, k, v, causal, float(scale), bias, alibi_slopes,
-                                  float(dropout_p) if training else 0.0, kv_lens)
+        return _call(_FlashAttnFn, q, k, v, causal, float(scale), bias, alibi_slopes, float(dropout_p) if training else 0.0, kv_lens)
     if (bias is None and alibi_slopes is None and kv_lens is None and not (dropout_p > 0.0 and training)
             and _split_supported(q, k, v, scale, causal, mask)):
         ts = [t if _rows_of_vectors(t) else t.contiguous() for t in (q, k, v)]
