@@ -251,31 +251,37 @@ int* small_wait_word() {
 }  // namespace
 
 // Whether this kernel is the better one, with `nt` rows of x per tile and `ranks` CTAs per tile.
-//   this kernel:     3.4 us + 0.03 us per row of the tile + the largest of: 0.28 us per k-block of a CTA (latency of the pipeline), all
-//                    operand tiles at 14 TB/s (shared-memory fill of the chip), w at 6 TB/s
-//   gemm_sm100.cu:   4.7 us + the larger of: waves x k-blocks x 0.235 us (64-wide tiles; 0.29 us 128-wide, 0.5 us 256 x 256 on
-//                    CTA pairs), w at 6 TB/s
-// Fitted over M = 4 .. 2048 and w from [1152, 384] to [50304, 1024], within 15 %.  Up to 32 rows this kernel was the better one
-// everywhere (nearest: [32, 1024] x [50304, 1024] 24.8 against 25.3 us); above that it is taken where the estimate is 12 % ahead:
-// few tiles and a long K ([128, 4096] x [1024, 4096] 9.3 against 19.9 us), not many tiles ([64, 1024] x [50304, 1024] 27.3 against 23.4 us).
+//   this kernel:     3.4 us + 0.03 us per row of the tile + the merge of a cluster (0.1 us of 2, 0.2 us of 4 CTAs, 8 ns per row of the tile
+//                    of 8) + the larger of: the k-blocks of a CTA (0.28 us each with 16 rows, 0.34 with 32 and 64, 0.38 with 128; up to 1.8
+//                    times that where two CTAs share an SM), w at 6 TB/s
+//   gemm_sm100.cu:   4.5 us + the larger of: waves x k-blocks x 0.235 us (64-wide tiles; 0.29 us 128-wide, 0.31 us 192-wide, 0.36 us 256 x 256
+//                    on CTA pairs), w at 6 TB/s
+// Fitted over 350 products, M = 1 .. 2048 and w from [384, 384] to [50304, 1024] and [4096, 11008] (7 % and 3 % rms).  Up to 32 rows this
+// kernel was the better one everywhere (nearest: [32, 1024] x [50304, 1024] 24.8 against 25.3 us); above that it is taken where the estimate
+// is 8 % and 0.5 us ahead: few tiles and a long K ([128, 4096] x [1024, 4096] 9.3 against 19.9 us, [200, 11008] x [4096, 11008] 28.6 against
+// 46.6), not many tiles ([64, 1024] x [50304, 1024] 27.3 against 23.4 us, [2048, 5120] x [1280, 5120] 39.6 against 29.3) and not a short K
+// ([256, 384] x [1536, 384] 6.2 against 5.8).  Clusters of 4 and 8 are kept to 264 CTAs: the SMs of a GPC do not divide by them, and 72
+// clusters of 4 with two CTAs per SM ran in two waves ([96, 1024] x [3072, 1024] 10.2 against 8.2 us).
 extern "C" int lb_gemm_small_rule(int M, int N, int K, int* nt, int* ranks) {
   if (M > 2048) return 0;
   const int kb = (K + 63) / 64, tiles_n = (N + 127) / 128;
   const double w_us = (double)N * K * 2 / 6e6;
+  const double block_us[4] = {0.28, 0.34, 0.34, 0.38};
   double best = 1e30;
-  for (int t = 16; t <= 128; t *= 2) {
+  for (int i = 0; i < 4; ++i) {
+    const int t = 16 << i;
     if (t < 128 && M > 8 * t) continue;                       // tiles of few rows would read w over and over
     if (t > 16 && M <= t / 2) break;
     const long tiles = (long)tiles_n * ((M + t - 1) / t);
-    for (int r = 1; r <= 8; r *= 2) {
-      if (r > 1 && (tiles * r > 296 || kb < r)) break;
+    for (int lg = 0; lg < 4; ++lg) {
+      const int r = 1 << lg;
+      if (r > 1 && (tiles * r > (r > 2 ? 264 : 296) || kb < r)) break;
       const int per = (kb + r - 1) / r;
-      const long waves = (tiles * r + 295) / 296;
-      const double fill = (double)tiles * r * per * (16384 + t * 128) / 14e6;
-      double us = waves * per * 0.28;
-      if (fill > us) us = fill;
+      const long ctas = tiles * r, waves = (ctas + 295) / 296;
+      const double load = (ctas < 296 ? ctas : 296) / 148.0;
+      double us = waves * per * block_us[i] * (load > 1 ? 1 + 0.8 * (load - 1) : 1);
       if (w_us > us) us = w_us;
-      us += 3.4 + 0.03 * t + 1.5 * (waves - 1);
+      us += 3.4 + 0.03 * t + (r < 8 ? 0.1 * lg : 0.008 * t) + 1.5 * (waves - 1);
       if (us < best - 1e-9) {
         best = us;
         *nt = t;
@@ -285,16 +291,17 @@ extern "C" int lb_gemm_small_rule(int M, int N, int K, int* nt, int* ranks) {
   }
   if (M <= 32) return 1;
   double old_us = 1e30;
-  const int bns[3] = {64, 128, 256};
-  const double slope[3] = {0.235, 0.29, 0.5};
-  for (int i = 0; i < 3; ++i) {
-    const long tiles = i == 2 ? (long)((M + 255) / 256) * ((N + 255) / 256) : (long)((M + 127) / 128) * ((N + bns[i] - 1) / bns[i]);
-    const long slots = i == 2 ? 74 : 148;
+  const int bns[4] = {64, 128, 192, 256};
+  const double slope[4] = {0.235, 0.29, 0.31, 0.36};
+  for (int i = 0; i < 4; ++i) {
+    const long tiles = i == 3 ? (long)((M + 255) / 256) * ((N + 255) / 256) : (long)((M + 127) / 128) * ((N + bns[i] - 1) / bns[i]);
+    const long slots = i == 3 ? 74 : 148;
     const double us = (double)((tiles + slots - 1) / slots) * kb * slope[i];
     if (us < old_us) old_us = us;
   }
   if (w_us > old_us) old_us = w_us;
-  return best * 1.12 < old_us + 4.7;
+  old_us += 4.5;
+  return best * 1.08 < old_us && best + 0.5 < old_us;
 }
 
 // Returns 0, a cudaError_t, or a negative code for unsupported arguments (-20: an earlier launch's wait ran out).
