@@ -567,15 +567,33 @@ int norm_grid(int rows) { return norm_grid_of(rows, lb::NORM_WARPS, 2); }
 int norm_fwd_grid(int rows) { return norm_grid_of(rows, lb::NORM_WARPS, 4); }
 // bf16 backward: three 4-warp blocks per SM (one wave; every block leaves one row of column partials)
 int norm_bwd_bf16_grid(int rows) { return norm_grid_of(rows, lb::NORM_BWD_WARPS, 3); }
-// wide rows: blocks loop over rows; the backward keeps to one wave because every block leaves a row of column sums at the end
+// wide rows: blocks loop over rows; the backward keeps to one wave, and to as few blocks as do it in the same number of rounds, because
+// every block leaves a row of column sums at the end
 int norm_fwd_wide_grid(int rows) { return norm_grid_of(rows, 1, 6); }
-int norm_bwd_wide_grid(int rows, int H) { return norm_grid_of(rows, 1, H <= 4096 ? 3 : 1); }
+int norm_bwd_wide_grid(int rows, int H) {
+  const int cap = norm_sms() * (H <= 4096 ? 3 : 1);
+  if (rows <= cap) return rows;
+  const int rounds = cap > 0 ? (rows + cap - 1) / cap : rows;
+  return (rows + rounds - 1) / rounds;
+}
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
-// bf16 rows of whole 16-byte vectors: the warp kernel up to 1024 columns (four vectors per lane: beyond that its column sums
-// spill), the block kernel up to 8192
+// bf16 rows of whole 16-byte vectors: the warp kernels up to 1024 columns (four vectors per lane: beyond that their column sums
+// spill), the block kernels up to 8192, but for the rules below
 constexpr int NORM_WARP_MAX_H = 1024, NORM_WIDE_MAX_H = 8192;
 bool norm_vec_bf16(int H, int dtype) { return dtype == 0 && H % 8 == 0 && H <= NORM_WIDE_MAX_H; }
+// Between 1024 and 2560 columns a warp still holds a row, and with enough rows to fill the chip with warps it is ahead of a block per row, whose
+// row sums cost barriers.  Forward, warp / block: layer norm [1024, 1280] 3.2 / 3.5, [8192, 1280] 10 / 17, [1024, 2048] 4.1 / 3.7, [1536, 2048]
+// 4.4 / 4.7, [8192, 2560] 19 / 31 us, [8192, 3072] equal; RMS norm [1024, 1280] 2.9 / 2.8, [1536, 1280] 2.8 / 3.1, [1536, 2048] 3.9 / 3.5, [8192, 2048]
+// 14 / 16 us.  Backward (column sums beside the row: up to 1536): [256, 1280] 6.1 / 5.6, [512, 1280] 6.2 / 8.5, [8192, 1280] 23 / 32, [512, 1536]
+// 6.8 / 9.1 us; [8192, 2048] 45 / 38, but [1024, 2048] 10.4 / 11.3 (one round of one block of warps per SM).  (2560 = 10 vectors per lane; 7 and
+// 9 are not compiled.)
+bool norm_fwd_by_warp(int rows, int H, bool rms) {
+  return H % 256 == 0 && H <= 2560 && H != 1792 && H != 2304 && rows >= (H <= 1536 ? 1024 : 1536) + (rms ? 512 : 0);
+}
+bool norm_bwd_by_warp(int rows, int H) {
+  return ((H == 1280 || H == 1536) && rows > 296) || (H == 2048 && rows > 888 && rows <= 148 * lb::NORM_WARPS);
+}
 
 // fp32 activations: H = 256 VPL
 template <bool RMS>
@@ -611,6 +629,16 @@ void fwd_dispatch_bf16(int H, const __nv_bfloat16* x, const W* g, const W* b, __
 #undef LB_CASE
     return;
   }
+  if (norm_fwd_by_warp(rows, H, RMS)) {
+    const int grid = norm_fwd_grid(rows);
+#define LB_CASE(V)                                                                                                                  \
+  case V:                                                                                                                           \
+    lb::norm_fwd_kernel<__nv_bfloat16, W, V, RMS, false><<<grid, lb::NORM_WARPS * 32, 0, s>>>(x, g, b, y, mean, rstd, rows, eps, H); \
+    break;
+    switch (H / 256) { LB_CASE(5) LB_CASE(6) LB_CASE(8) LB_CASE(10) }
+#undef LB_CASE
+    return;
+  }
   const int grid = norm_fwd_wide_grid(rows);
 #define LB_CASE(V)                                                                                                             \
   case V:                                                                                                                      \
@@ -635,6 +663,15 @@ void bwd_dispatch_bf16(int H, const __nv_bfloat16* gy, const __nv_bfloat16* x, c
                                                                                          gadd, acc_dg, acc_db, H);                \
     break;
     switch ((H + 255) / 256) { LB_CASE(1) LB_CASE(2) LB_CASE(3) LB_CASE(4) }
+#undef LB_CASE
+    return;
+  }
+  if (norm_bwd_by_warp(rows, H)) {
+#define LB_CASE(V)                                                                                                                            \
+  case V:                                                                                                                                     \
+    lb::norm_bwd_kernel<__nv_bfloat16, W, V, RMS><<<grid, lb::NORM_WARPS * 32, 0, s>>>(gy, x, g, mean, rstd, gx, pdg, pdb, rows, gadd);        \
+    break;
+    switch (H / 256) { LB_CASE(5) LB_CASE(6) LB_CASE(8) }
 #undef LB_CASE
     return;
   }
@@ -738,7 +775,7 @@ extern "C" int lb_norm_bwd(const void* gy, const void* x, const void* gamma, con
       else norm_bwd_any<B, float>(gy, x, gamma, mean, rstd, gx, dgamma, dbeta, rows, H, rms, accumulate, s);
       return (int)cudaGetLastError();
     }
-    const int grid = H <= NORM_WARP_MAX_H ? norm_bwd_bf16_grid(rows) : norm_bwd_wide_grid(rows, H);
+    const int grid = H <= NORM_WARP_MAX_H ? norm_bwd_bf16_grid(rows) : norm_bwd_by_warp(rows, H) ? norm_grid(rows) : norm_bwd_wide_grid(rows, H);
     float* pdg = workspace;
     float* pdb = dbeta != nullptr ? workspace + static_cast<size_t>(grid) * H : nullptr;
     // accumulate mode: the warp kernel's blocks add their column sums straight into dgamma / dbeta

@@ -47,7 +47,8 @@ def test_attention_rows_do_not_depend_on_timing(dim, causal):
 
 @pytest.mark.parametrize("rms", [False, True])
 @pytest.mark.parametrize("rows,h", [(1, 8), (3, 192), (257, 384), (2048, 768), (130, 1000), (515, 1024), (4, 1032), (300, 1280), (37, 2048),
-                                    (450, 4096), (33, 6152), (5, 8192), (3, 8200), (9, 99)])
+                                    (450, 4096), (33, 6152), (5, 8192), (3, 8200), (9, 99),
+                                    (296, 1280), (297, 1280), (1536, 1280), (600, 1536), (1535, 2048), (2048, 2048), (2100, 2560), (2048, 1792), (2048, 2304), (1024, 2048), (888, 2048)])
 def test_norm_kernels_at_their_edges(rows, h, rms):
     """Rows of a warp (up to 1024 columns), of a block (up to 8192) and of the generic kernel, forward, backward, with the gradient of a
     residual path, into new tensors and into fp32 gradients."""
