@@ -22,6 +22,8 @@
 // Every wait on an mbarrier is bounded (attention_tc.cuh).
 #include "attention_tc.cuh"
 
+#include <atomic>
+
 namespace lb {
 
 constexpr int SPL_THREADS = 320;                 // backward: TMA warp, MMA warp, 8 softmax warps
@@ -706,11 +708,16 @@ bool split_tmap(CUtensorMap* m, const void* ptr, int B, int A, int S, int d, con
 bool split_view_ok(const void* ptr, const long* st) {
   return (reinterpret_cast<uintptr_t>(ptr) & 15) == 0 && st[0] > 0 && st[1] > 0 && st[2] > 0 && ((st[0] | st[1] | st[2]) % 8) == 0;
 }
+// a function's limit on dynamic shared memory is per device: these calls ran on any device of a process before, and do
 template <typename K>
-cudaError_t split_configure(K kern, int smem, bool& done) {
-  if (done) return cudaSuccess;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  done = e == cudaSuccess;
+cudaError_t split_configure(K kern, int smem, std::atomic<unsigned long long>& done) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+  if (done.load(std::memory_order_relaxed) & bit) return cudaSuccess;
+  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_relaxed);
   return e;
 }
 lb::SplitParams split_params(int B, int A, int Sq, int Sk, int d, int causal, float scale, const uint32_t* mask, const float* fill, long mask_b,
@@ -756,7 +763,7 @@ extern "C" int lb_attn_split_fwd(const void* q, const void* k, const void* v, vo
   if (!split_tmap(&tq, q, B, A, Sq, d, qs) || !split_tmap(&tk, k, B, A, Sk, d, ks) || !split_tmap(&tv, v, B, A, Sk, d, vs)) return -2;
   lb::SplitParams p = split_params(B, A, Sq, Sk, d, causal, scale, mask, fill, mask_b, mask_a, err);
   p.o = (__nv_bfloat16*)o; p.o32 = o32; p.lse = lse;
-  static bool c0 = false, c1 = false;
+  static std::atomic<unsigned long long> c0{0}, c1{0};
   const dim3 grid((Sq + 127) / 128, A, B);
   cudaError_t e = mask ? split_configure(lb::attn_split_fwd_kernel<true>, lb::SPL_FWD_SMEM, c1) : split_configure(lb::attn_split_fwd_kernel<false>, lb::SPL_FWD_SMEM, c0);
   if (e != cudaSuccess) return (int)e;
@@ -795,7 +802,7 @@ extern "C" int lb_attn_split_bwd(const void* dout, const void* q, const void* k,
   p.delta = delta;
   p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv;
   for (int i = 0; i < 3; ++i) { p.dk_strides[i] = dks[i]; p.dv_strides[i] = dvs[i]; }
-  static bool c0 = false, c1 = false;
+  static std::atomic<unsigned long long> c0{0}, c1{0};
   const dim3 grid(key_blocks, A, B);
   cudaError_t e = mask ? split_configure(lb::attn_split_bwd_kernel<true>, lb::SPL_BWD_SMEM, c1) : split_configure(lb::attn_split_bwd_kernel<false>, lb::SPL_BWD_SMEM, c0);
   if (e != cudaSuccess) return (int)e;
