@@ -737,7 +737,8 @@ def attention_cached(q, k_new, v_new, past_key, past_value, *, scale: float, mas
     tokens, other types, caches held on another device): the caller concatenates and takes :func:`attention`."""
     ts = (q, k_new, v_new, past_key, past_value)
     if (not use_native(q) or not _plain_call(q) or q.dim() != 4 or q.shape[2] != 1 or (dropout_p > 0.0 and training) or scale <= 0
-            or any(t.dtype != torch.bfloat16 or t.device != q.device for t in ts) or k_new.shape != q.shape or v_new.shape != q.shape
+            or not torch.bfloat16 == q.dtype == k_new.dtype == v_new.dtype == past_key.dtype == past_value.dtype
+            or not q.device == k_new.device == v_new.device == past_key.device == past_value.device or k_new.shape != q.shape or v_new.shape != q.shape
             or past_key.dim() != 4 or past_key.shape != past_value.shape or past_key.shape[:2] != q.shape[:2] or past_key.shape[3] != q.shape[3]
             or past_key.shape[2] == 0 or min(q.shape) == 0 or max(q.shape[:2]) > 65535 or q.shape[3] % 8 or q.shape[3] > 256
             or not all(_rows_of_vectors(t) for t in ts) or (torch.is_grad_enabled() and any(t.requires_grad for t in ts))
