@@ -731,10 +731,20 @@ def attention_packed(layout: str, ts, *, causal: bool, scale: float, mask=None, 
     return _call(_SplitAttnFn, layout, causal, float(scale), mask, *ts)
 
 
+def _cache_too_long_for_one_cluster(heads: int, keys: int, d: int) -> bool:
+    """A head's keys are read by at most eight CTAs, in steps of 1.05 us (128 threads, ``lanes`` per key, four keys each); copies and products
+    over the whole chip take 28 us and 1.2e-5 us per number of the caches.  So up to three heads in all with a very long past stay with
+    those: 1 head x 100000 x 128 496 against 154 us, 2 x 32768 x 64 68 against 88, 4 x 4096 x 128 21 against 39, 8 x 32768 x 128 198 against 335."""
+    if heads > 3:
+        return False
+    lanes = 1 << (d // 8 - 1).bit_length()
+    return 5.0 + 1.05 * keys / (8 * 512 / lanes) > 28.0 + 1.2e-5 * heads * keys * d
+
+
 def attention_cached(q, k_new, v_new, past_key, past_value, *, scale: float, mask=None, dropout_p: float = 0.0, training: bool = False):
     """One new token per sequence: ``q``, ``k_new``, ``v_new`` ``[b, a, 1, d]``, the caches ``[b, a, past, d]`` → (context
     ``[b, 1, a, d]``, the caches with the token appended) in one kernel; ``None`` where it does not apply (gradients, several new
-    tokens, other types, caches held on another device): the caller concatenates and takes :func:`attention`."""
+    tokens, other types, caches held on another device, a very long past of up to three heads): the caller concatenates and takes :func:`attention`."""
     ts = (q, k_new, v_new, past_key, past_value)
     if (not use_native(q) or not _plain_call(q) or q.dim() != 4 or q.shape[2] != 1 or (dropout_p > 0.0 and training) or scale <= 0
             or not torch.bfloat16 == q.dtype == k_new.dtype == v_new.dtype == past_key.dtype == past_value.dtype
@@ -742,7 +752,8 @@ def attention_cached(q, k_new, v_new, past_key, past_value, *, scale: float, mas
             or past_key.dim() != 4 or past_key.shape != past_value.shape or past_key.shape[:2] != q.shape[:2] or past_key.shape[3] != q.shape[3]
             or past_key.shape[2] == 0 or min(q.shape) == 0 or max(q.shape[:2]) > 65535 or q.shape[3] % 8 or q.shape[3] > 256
             or not all(_rows_of_vectors(t) for t in ts) or (torch.is_grad_enabled() and any(t.requires_grad for t in ts))
-            or (mask is not None and not _mask_supported(mask, q.shape[:3], q.device, past_key.shape[2] + 1))):
+            or (mask is not None and not _mask_supported(mask, q.shape[:3], q.device, past_key.shape[2] + 1))
+            or _cache_too_long_for_one_cluster(q.shape[0] * q.shape[1], past_key.shape[2], past_key.shape[3])):
         return None
     ext = load_ext()
     words, fill = (None, None) if mask is None else _pack_mask(ext, mask, q, past_key.shape[2] + 1, False)

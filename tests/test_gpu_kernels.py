@@ -238,6 +238,18 @@ def test_attention_against_a_cache(b, a, past, d, mask):
     assert err[0] <= 1.3 * err[1] + 1e-5 * float(want.norm()), err   # both: fp32 throughout, one rounding to bf16
 
 
+def test_cache_of_few_heads_and_a_very_long_past():
+    """On both sides of the line between the one-kernel step and the concatenation."""
+    for heads, past, d, one_kernel in ((1, 2000, 64, True), (1, 8900, 128, True), (1, 9100, 128, False), (2, 30000, 64, True), (2, 30000, 128, False), (3, 1000, 256, True), (4, 60000, 128, True)):
+        q, k, v = (_rand((1, heads, 1, d), i) for i in range(3))
+        kp, vp = _rand((1, heads, past, d), 4), _rand((1, heads, past, d), 5)
+        got = OF.attention_cached(q, k, v, kp, vp, scale=d ** -0.5)
+        assert (got is not None) == one_kernel
+        if one_kernel:
+            want = _attend64(q, torch.cat([kp, k], 2), torch.cat([vp, v], 2), d ** -0.5).permute(0, 2, 1, 3)
+            assert float((got[0].double() - want).norm() / want.norm()) < 2.0 ** -8
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 8, 8), (1, 1024, 1024), (5, 1160, 72), (16, 128, 640), (17, 384, 1536), (33, 4096, 200), (64, 136, 4096), (64, 3072, 1024)])
 def test_linear_of_few_rows(m, n, k):
     """Edges of the row, column and K tiles, every cluster size, bias, activation, pre-activation copy and residual; the sums of a
