@@ -672,6 +672,7 @@ attn_fwd_v2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
 #pragma unroll
     for (int c = 0; c < D / 64; ++c) {
       uint32_t t[32];
+      __syncwarp();                                    // whole warps read tensor memory: the stores below are per lane
       tmem_ld_32x32b_x32(o_addr + c * 32, t);
       tmem_ld_wait();
       if (q_idx < p.S) {
@@ -1164,6 +1165,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 #pragma unroll
       for (int c = half * (D / 64); c < (half + 1) * (D / 64); ++c) {
         uint32_t t[32];
+        __syncwarp();                                  // whole warps read tensor memory: the stores below are per lane
         tmem_ld_32x32b_x32(tmem_base + lane_off + Cfg::DQ_COL + c * 32, t);
         tmem_ld_wait();
         if (q_ok) {
@@ -1194,6 +1196,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 #pragma unroll
       for (int c = half * (D / 64); c < (half + 1) * (D / 64); ++c) {
         uint32_t t[32];
+        __syncwarp();                                  // whole warps read tensor memory: the stores below are per lane
         tmem_ld_32x32b_x32(tmem_base + lane_off + col + c * 32, t);
         tmem_ld_wait();
         if (k_idx < p.S) {

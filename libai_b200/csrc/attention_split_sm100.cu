@@ -92,7 +92,7 @@ attn_mask_pack_kernel(const U* __restrict__ mask, unsigned long long and_mask, i
 // ------------------------------------------------------------------------------------------------------------------ forward
 // One CTA per (128 queries, head, batch).  S in TMEM columns [0, 128), O in [128, 192), P's first part in [192, 256); the second and third
 // parts of 16 keys (8 columns each) overwrite the 16 S columns of those keys once their thread has read them, so the whole fits 256 columns
-// and two CTAs share an SM.  The MMA warp issues S(j+1) after P(j)·V(j) has completed (it overwrites them); the other CTA fills the gap.
+// and two CTAs share an SM.  S(j+1) is issued after P(j)·V(j) has completed (it overwrites them); the other CTA fills the gap.
 // O is added up over the key blocks in registers: the tensor core rounds every addition into its accumulator towards zero, and 24 of them
 // per key block leave O, with it δ, some 1e-6 short (dQ of the example above: 8.5e-3 off).
 constexpr int SPL_FWD_SMEM = 5 * SPL_TILE + 2 * 2 * 128 * 4 + 1024 + 256;

@@ -280,6 +280,7 @@ latent_prompt_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
 #pragma unroll
     for (int c = 0; c < V / 64; ++c) {
       uint32_t t[32];
+      __syncwarp();                                    // whole warps read tensor memory: the stores below are per lane
       tmem_ld_32x32b_x32(o_addr + c * 32, t);
       tmem_ld_wait();
       if (r < nq) {
