@@ -23,11 +23,10 @@ from . import count_launch, load_ext, use_native
 from .. import ops
 
 
-def _plain_call(t=None) -> bool:
-    """False where an operator is transformed (vmap, jvp, …), differentiated forward or traced, or where ``t`` has a shape and no memory:
-    those see PyTorch operators.  Asked before anything looks at an address."""
-    return not (torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0 or torch.jit.is_tracing()
-                or isinstance(t, FakeTensor))
+def _plain_call() -> bool:
+    """False where an operator is transformed (vmap, jvp, …), differentiated forward or traced: those see PyTorch operators.  Asked (like the
+    type of a tensor without memory, ``FakeTensor``) before anything looks at an address."""
+    return not (torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0 or torch.jit.is_tracing())
 
 
 class _NoGradContext:
@@ -677,7 +676,7 @@ def _split_supported(q, k, v, scale, causal, mask) -> bool:
     return (use_native(q) and q.dtype == k.dtype == v.dtype == torch.bfloat16 and q.device == k.device == v.device
             and q.dim() == k.dim() == 4 and k.shape == v.shape and q.shape[:2] == k.shape[:2] and q.shape[-1] == k.shape[-1]
             and _split_sizes_ok(*q.shape[:3], k.shape[2], q.shape[3], scale, causal)
-            and (mask is None or _mask_supported(mask, q.shape[:3], q.device, k.shape[2])) and _plain_call(q))
+            and (mask is None or _mask_supported(mask, q.shape[:3], q.device, k.shape[2])) and type(q) is not FakeTensor and _plain_call())
 
 
 class _SplitAttnFn(torch.autograd.Function):
@@ -723,7 +722,7 @@ def attention_packed(layout: str, ts, *, causal: bool, scale: float, mask=None, 
     x, y = ts[0], ts[-1]
     b, sq, a, d = x.shape
     d = d // 3 if layout == "qkv" else d
-    if ((dropout_p > 0.0 and training) or not use_native(x) or not _plain_call(x) or not _split_sizes_ok(b, a, sq, y.shape[1], d, scale, causal)
+    if ((dropout_p > 0.0 and training) or not use_native(x) or type(x) is FakeTensor or not _plain_call() or not _split_sizes_ok(b, a, sq, y.shape[1], d, scale, causal)
             or any(t.dtype != torch.bfloat16 or t.device != x.device or not t.is_contiguous() or t.data_ptr() % 16 for t in ts)
             or (layout == "q_kv" and y.shape != (b, y.shape[1], a, 2 * d)) or (layout == "qkv" and x.shape[3] != 3 * d)
             or (mask is not None and not _mask_supported(mask, (b, a, sq), x.device, y.shape[1]))):
@@ -746,7 +745,7 @@ def attention_cached(q, k_new, v_new, past_key, past_value, *, scale: float, mas
     ``[b, 1, a, d]``, the caches with the token appended) in one kernel; ``None`` where it does not apply (gradients, several new
     tokens, other types, caches held on another device, a very long past of up to three heads): the caller concatenates and takes :func:`attention`."""
     ts = (q, k_new, v_new, past_key, past_value)
-    if (not use_native(q) or not _plain_call(q) or q.dim() != 4 or q.shape[2] != 1 or (dropout_p > 0.0 and training) or scale <= 0
+    if (not use_native(q) or type(q) is FakeTensor or not _plain_call() or q.dim() != 4 or q.shape[2] != 1 or (dropout_p > 0.0 and training) or scale <= 0
             or not torch.bfloat16 == q.dtype == k_new.dtype == v_new.dtype == past_key.dtype == past_value.dtype
             or not q.device == k_new.device == v_new.device == past_key.device == past_value.device or k_new.shape != q.shape or v_new.shape != q.shape
             or past_key.dim() != 4 or past_key.shape != past_value.shape or past_key.shape[:2] != q.shape[:2] or past_key.shape[3] != q.shape[3]
