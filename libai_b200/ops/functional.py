@@ -744,18 +744,20 @@ def attention_cached(q, k_new, v_new, past_key, past_value, *, scale: float, mas
     """One new token per sequence: ``q``, ``k_new``, ``v_new`` ``[b, a, 1, d]``, the caches ``[b, a, past, d]`` → (context
     ``[b, 1, a, d]``, the caches with the token appended) in one kernel; ``None`` where it does not apply (gradients, several new
     tokens, other types, caches held on another device, a very long past of up to three heads): the caller concatenates and takes :func:`attention`."""
-    ts = (q, k_new, v_new, past_key, past_value)
-    if (not use_native(q) or type(q) is FakeTensor or not _plain_call() or q.dim() != 4 or q.shape[2] != 1 or (dropout_p > 0.0 and training) or scale <= 0
+    if not use_native(q) or type(q) is FakeTensor or not _plain_call() or q.dim() != 4 or past_key.dim() != 4:
+        return None
+    ts, qs, ps = (q, k_new, v_new, past_key, past_value), q.shape, past_key.shape
+    b, a, new, d = qs
+    if (new != 1 or (dropout_p > 0.0 and training) or scale <= 0
             or not torch.bfloat16 == q.dtype == k_new.dtype == v_new.dtype == past_key.dtype == past_value.dtype
-            or not q.device == k_new.device == v_new.device == past_key.device == past_value.device or k_new.shape != q.shape or v_new.shape != q.shape
-            or past_key.dim() != 4 or past_key.shape != past_value.shape or past_key.shape[:2] != q.shape[:2] or past_key.shape[3] != q.shape[3]
-            or past_key.shape[2] == 0 or min(q.shape) == 0 or max(q.shape[:2]) > 65535 or q.shape[3] % 8 or q.shape[3] > 256
+            or not q.device == k_new.device == v_new.device == past_key.device == past_value.device or not qs == k_new.shape == v_new.shape
+            or ps != past_value.shape or ps[:2] != qs[:2] or ps[3] != d or ps[2] == 0 or min(b, a, d) == 0 or max(b, a) > 65535 or d % 8 or d > 256
             or not all(_rows_of_vectors(t) for t in ts) or (torch.is_grad_enabled() and any(t.requires_grad for t in ts))
-            or (mask is not None and not _mask_supported(mask, q.shape[:3], q.device, past_key.shape[2] + 1))
-            or _cache_too_long_for_one_cluster(q.shape[0] * q.shape[1], past_key.shape[2], past_key.shape[3])):
+            or (mask is not None and not _mask_supported(mask, qs[:3], q.device, ps[2] + 1))
+            or (b * a < 4 and _cache_too_long_for_one_cluster(b * a, ps[2], d))):
         return None
     ext = load_ext()
-    words, fill = (None, None) if mask is None else _pack_mask(ext, mask, q, past_key.shape[2] + 1, False)
+    words, fill = (None, None) if mask is None else _pack_mask(ext, mask, q, ps[2] + 1, False)
     count_launch()
     return ext.attn_decode(q, k_new, v_new, past_key, past_value, float(scale), words, fill)
 
