@@ -5,14 +5,7 @@
 // Q/K/V are read straight out of the packed QKV projection through strided 4-D TMA tensor maps
 // ([B, A, S, D] views), O is written in [B, S, A, D] so the output projection consumes it as-is.
 //
-// Forward, one CTA per (batch, head, 128-query block), 192 threads:
-//   warp 0        TMA producer : Q once, then K/V tiles of 128 keys (double buffered)
-//   warp 1        MMA issuer   : S_j = Q·K_jᵀ (TMEM, double buffered)  and  O_j = P_j·V_j (TMEM)
-//   warps 2..5    softmax      : thread r owns query row r: tcgen05.ld S → online softmax (exp2) →
-//                                P (bf16) to swizzled smem as the A operand of the PV MMA; running
-//                                output kept in registers: O ← (O + O_{j-1}) · α_j
-// The QKᵀ MMA of block j+1 is issued before the softmax of block j, so tensor-core work hides behind
-// the (MUFU-bound) softmax.
+// Forward without bias or dropout: attention_fwd_sm100.cu, but for the few sizes that its rule leaves here.
 #include "common.cuh"
 
 #include <type_traits>
@@ -24,21 +17,8 @@ namespace lb {
 
 constexpr int ATT_BM = 128;   // queries per CTA
 constexpr int ATT_BN = 128;   // keys per tile
-constexpr int ATT_THREADS = 192;
 constexpr int ATT_BWD_THREADS = 320;
 constexpr int ATT_FWD2_THREADS = 320; // forward v2: 8 softmax warps (row pairs exchange their block max through smem)  // TMA + MMA + 8 compute warps (two per TMEM lane quadrant: each takes half of the columns)
-
-template <int D>
-struct AttnCfg {
-  static constexpr int QK_CHUNKS = D / 64;                 // 64-element (128B) K-chunks of Q and K tiles
-  static constexpr int TILE_BYTES = ATT_BN * D * 2;        // one Q / K / V tile
-  static constexpr int P_BYTES = ATT_BM * ATT_BN * 2;      // 32 KB
-  static constexpr int P_STAGES = (D == 64) ? 2 : 1;
-  static constexpr int SMEM_BYTES = TILE_BYTES /*Q*/ + 4 * TILE_BYTES /*K,V x2*/ + P_STAGES * P_BYTES + 1024 + 256;
-  // TMEM columns: S0 [0,128) S1 [128,256) O [256, 256+D)
-  static constexpr uint32_t TMEM_COLS = 512;
-  static constexpr uint32_t O_COL = 256;
-};
 
 struct AttnFwdParams {
   __nv_bfloat16* o;   // [B, S, A, D]
@@ -72,259 +52,7 @@ LB_DEVICE uint32_t rnd_byte(const uint4& r, int i) {   // i in [0, 16)
   return (w >> ((i & 3) * 8)) & 0xFFu;
 }
 
-template <int D>
-__global__ void __launch_bounds__(ATT_THREADS, 1)
-attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                const __grid_constant__ CUtensorMap tmap_v, AttnFwdParams p) {
-  using Cfg = AttnCfg<D>;
-  constexpr int PST = Cfg::P_STAGES;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sQ = smem;
-  uint8_t* sK = sQ + Cfg::TILE_BYTES;            // 2 stages
-  uint8_t* sV = sK + 2 * Cfg::TILE_BYTES;        // 2 stages
-  uint8_t* sP = sV + 2 * Cfg::TILE_BYTES;        // PST stages
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sP + PST * Cfg::P_BYTES);
-  uint64_t* q_full = bars;            // 1
-  uint64_t* k_full = bars + 1;        // 2
-  uint64_t* k_empty = bars + 3;       // 2
-  uint64_t* v_full = bars + 5;        // 2
-  uint64_t* v_empty = bars + 7;       // 2
-  uint64_t* s_full = bars + 9;        // 2
-  uint64_t* s_empty = bars + 11;      // 2
-  uint64_t* p_full = bars + 13;       // 2
-  uint64_t* p_empty = bars + 15;      // 2
-  uint64_t* o_full = bars + 17;       // 1
-  uint64_t* o_empty = bars + 18;      // 1
-  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 20);
-
-  const int warp_idx = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int q_blk = blockIdx.x;
-  const int head = blockIdx.y, batch = blockIdx.z;
-  const int q0 = q_blk * ATT_BM;
-  const int kv_len = p.kv_lens != nullptr ? max(1, min(p.S, p.kv_lens[batch])) : p.S;
-  int nkv = (kv_len + ATT_BN - 1) / ATT_BN;
-  if (p.causal) nkv = min(nkv, q_blk + 1);
-
-  if (threadIdx.x == 0) {
-    tma_prefetch_desc(&tmap_q);
-    tma_prefetch_desc(&tmap_k);
-    tma_prefetch_desc(&tmap_v);
-    mbar_init(q_full, 1);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&k_full[i], 1);
-      mbar_init(&k_empty[i], 1);
-      mbar_init(&v_full[i], 1);
-      mbar_init(&v_empty[i], 1);
-      mbar_init(&s_full[i], 1);
-      mbar_init(&s_empty[i], 128);
-      mbar_init(&p_full[i], 128);
-      mbar_init(&p_empty[i], 1);
-    }
-    mbar_init(o_full, 1);
-    mbar_init(o_empty, 128);
-    fence_barrier_init();
-    fence_proxy_async();
-  }
-  if (warp_idx == 1) tmem_alloc<Cfg::TMEM_COLS>(tmem_ptr_smem);
-  tc_fence_before_sync();
-  __syncthreads();
-  tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_ptr_smem;
-
-  if (warp_idx == 0) {
-    // ================= TMA producer =================
-    if (elect_one()) {
-      mbar_arrive_expect_tx(q_full, Cfg::TILE_BYTES);
-#pragma unroll
-      for (int c = 0; c < Cfg::QK_CHUNKS; ++c)
-        tma_load_4d(sQ + c * (ATT_BM * 128), &tmap_q, q_full, c * 64, q0, head, batch);
-      for (int j = 0; j < nkv; ++j) {
-        const int b = j & 1;
-        const uint32_t par = ((j >> 1) & 1) ^ 1;
-        mbar_wait(&k_empty[b], par);
-        mbar_arrive_expect_tx(&k_full[b], Cfg::TILE_BYTES);
-#pragma unroll
-        for (int c = 0; c < Cfg::QK_CHUNKS; ++c)
-          tma_load_4d(sK + b * Cfg::TILE_BYTES + c * (ATT_BN * 128), &tmap_k, &k_full[b], c * 64, j * ATT_BN, head, batch);
-        mbar_wait(&v_empty[b], par);
-        mbar_arrive_expect_tx(&v_full[b], Cfg::TILE_BYTES);
-#pragma unroll
-        for (int c = 0; c < Cfg::QK_CHUNKS; ++c)
-          tma_load_4d(sV + b * Cfg::TILE_BYTES + c * (ATT_BN * 128), &tmap_v, &v_full[b], c * 64, j * ATT_BN, head, batch);
-      }
-    }
-  } else if (warp_idx == 1) {
-    // ================= MMA issuer =================
-    constexpr uint32_t idesc_qk = make_idesc_bf16(ATT_BM, ATT_BN, false, false);
-    constexpr uint32_t idesc_pv = make_idesc_bf16(ATT_BM, D, false, true);
-    const uint32_t q_addr = smem_u32(sQ);
-    auto issue_s = [&](int j) {
-      const int b = j & 1;
-      mbar_wait(&k_full[b], (j >> 1) & 1);
-      mbar_wait(&s_empty[b], ((j >> 1) & 1) ^ 1);
-      tc_fence_after_sync();
-      if (elect_one()) {
-        const uint32_t k_addr = smem_u32(sK + b * Cfg::TILE_BYTES);
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off = (kk / 4) * (ATT_BM * 128) + (kk % 4) * 32;
-          umma_f16_ss(tmem_base + b * ATT_BN, make_smem_desc_sw128(q_addr + off, 0, 1024),
-                      make_smem_desc_sw128(k_addr + off, 0, 1024), idesc_qk, kk > 0 ? 1u : 0u);
-        }
-        umma_commit(&s_full[b]);
-        umma_commit(&k_empty[b]);
-      }
-      __syncwarp();
-    };
-    mbar_wait(q_full, 0);
-    issue_s(0);
-    for (int j = 0; j < nkv; ++j) {
-      if (j + 1 < nkv) issue_s(j + 1);
-      const int b = j & 1, pb = j % PST;
-      mbar_wait(&p_full[pb], (j / PST) & 1);
-      mbar_wait(&v_full[b], (j >> 1) & 1);
-      mbar_wait(o_empty, (j & 1) ^ 1);
-      tc_fence_after_sync();
-      if (elect_one()) {
-        const uint32_t p_addr = smem_u32(sP + pb * Cfg::P_BYTES);
-        const uint32_t v_addr = smem_u32(sV + b * Cfg::TILE_BYTES);
-#pragma unroll
-        for (int kk = 0; kk < ATT_BN / 16; ++kk) {
-          const uint64_t da = make_smem_desc_sw128(p_addr + (kk / 4) * (ATT_BM * 128) + (kk % 4) * 32, 0, 1024);
-          const uint64_t db = make_smem_desc_sw128(v_addr + kk * (16 * 128), ATT_BN * 128, 1024);
-          umma_f16_ss(tmem_base + Cfg::O_COL, da, db, idesc_pv, kk > 0 ? 1u : 0u);
-        }
-        umma_commit(o_full);
-        umma_commit(&v_empty[b]);
-        umma_commit(&p_empty[pb]);
-      }
-      __syncwarp();
-    }
-  } else {
-    // ================= softmax / output (128 threads, thread <-> query row) =================
-    const int quad = warp_idx % 4;
-    const int r = quad * 32 + lane;          // row inside the tile
-    const int q_idx = q0 + r;
-    const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
-    float o_run[D];
-#pragma unroll
-    for (int i = 0; i < D; ++i) o_run[i] = 0.f;
-    float m_run = -INFINITY, l_run = 0.f;
-
-    auto add_o_block = [&](int jprev) {
-      mbar_wait(o_full, jprev & 1);
-      tc_fence_after_sync();
-#pragma unroll
-      for (int c = 0; c < D / 32; ++c) {
-        uint32_t t[32];
-        tmem_ld_32x32b_x32(tmem_base + lane_off + Cfg::O_COL + c * 32, t);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 32; ++i) o_run[c * 32 + i] += __uint_as_float(t[i]);
-      }
-      tc_fence_before_sync();
-      mbar_arrive(o_empty);
-    };
-
-    for (int j = 0; j < nkv; ++j) {
-      const int b = j & 1, pb = j % PST;
-      mbar_wait(&s_full[b], (j >> 1) & 1);
-      tc_fence_after_sync();
-      const uint32_t s_addr = tmem_base + lane_off + b * ATT_BN;
-      const int k0 = j * ATT_BN;
-      const bool need_mask = (p.causal && j == q_blk) || (k0 + ATT_BN > kv_len);
-      // ---- pass 1: row max
-      float mx = -INFINITY;
-#pragma unroll
-      for (int c = 0; c < ATT_BN / 32; ++c) {
-        uint32_t t[32];
-        tmem_ld_32x32b_x32(s_addr + c * 32, t);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          float x = __uint_as_float(t[i]);
-          if (need_mask) {
-            const int kidx = k0 + c * 32 + i;
-            if (kidx >= kv_len || (p.causal && kidx > q_idx)) x = -INFINITY;
-          }
-          mx = fmaxf(mx, x);
-        }
-      }
-      const float m_new = fmaxf(m_run, mx * p.scale_log2);
-      const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
-      const float alpha = fast_exp2(m_run - m_use);   // m_run = -inf -> 0
-      // ---- wait for the P buffer to be free, then pass 2: p = exp2(s*scale - m), write bf16 to swizzled smem
-      mbar_wait(&p_empty[pb], ((j / PST) & 1) ^ 1);
-      uint8_t* prow = sP + pb * Cfg::P_BYTES + r * 128;
-      float rowsum = 0.f;
-#pragma unroll
-      for (int c = 0; c < ATT_BN / 32; ++c) {
-        uint32_t t[32];
-        tmem_ld_32x32b_x32(s_addr + c * 32, t);
-        tmem_ld_wait();
-        uint32_t packed[16];
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          float x0 = __uint_as_float(t[i]), x1 = __uint_as_float(t[i + 1]);
-          float e0 = fast_exp2(x0 * p.scale_log2 - m_use), e1 = fast_exp2(x1 * p.scale_log2 - m_use);
-          if (need_mask) {
-            const int kidx = k0 + c * 32 + i;
-            if (kidx >= kv_len || (p.causal && kidx > q_idx)) e0 = 0.f;
-            if (kidx + 1 >= kv_len || (p.causal && kidx + 1 > q_idx)) e1 = 0.f;
-          }
-          rowsum += e0 + e1;
-          packed[i / 2] = pack_bf16(e0, e1);
-        }
-        // 32 keys = 64 bytes = four 16-byte chunks; key chunk (c / 2) selects the 64-key half of the tile
-        uint8_t* half_base = prow + (c / 2) * (ATT_BM * 128);
-#pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) {
-          const int chunk16 = (c % 2) * 4 + q4;               // 16B chunk index inside the 128B row
-          const int phys = chunk16 ^ (r & 7);                 // 128B swizzle
-          *reinterpret_cast<uint4*>(half_base + phys * 16) =
-              make_uint4(packed[q4 * 4], packed[q4 * 4 + 1], packed[q4 * 4 + 2], packed[q4 * 4 + 3]);
-        }
-      }
-      tc_fence_before_sync();
-      mbar_arrive(&s_empty[b]);      // S buffer b may be overwritten by QKᵀ of block j+2
-      fence_proxy_async();           // generic-proxy smem writes -> visible to the tensor core (async proxy)
-      mbar_arrive(&p_full[pb]);
-      l_run = l_run * alpha + rowsum;
-      // ---- fold the previous block's P·V into the running output, then rescale to the new max
-      if (j > 0) add_o_block(j - 1);
-      if (alpha != 1.0f) {
-#pragma unroll
-        for (int i = 0; i < D; ++i) o_run[i] *= alpha;
-      }
-      m_run = m_new;
-    }
-    add_o_block(nkv - 1);
-    if (q_idx < p.S) {
-      const float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
-      __nv_bfloat16* orow = p.o + ((static_cast<size_t>(batch) * p.S + q_idx) * p.A + head) * D;
-#pragma unroll
-      for (int i = 0; i < D; i += 8) {
-        *reinterpret_cast<uint4*>(orow + i) =
-            make_uint4(pack_bf16(o_run[i] * inv, o_run[i + 1] * inv), pack_bf16(o_run[i + 2] * inv, o_run[i + 3] * inv),
-                       pack_bf16(o_run[i + 4] * inv, o_run[i + 5] * inv), pack_bf16(o_run[i + 6] * inv, o_run[i + 7] * inv));
-      }
-      // natural-log LSE of the scaled scores
-      p.lse[(static_cast<size_t>(batch) * p.A + head) * p.S + q_idx] =
-          (m_run == -INFINITY) ? -INFINITY : (m_run + log2f(l_run)) * 0.6931471805599453f;
-    }
-  }
-
-  tc_fence_before_sync();
-  __syncthreads();
-  if (warp_idx == 1) {
-    tc_fence_after_sync();
-    tmem_dealloc<Cfg::TMEM_COLS>(tmem_base);
-  }
-}
-
 }  // namespace lb
-
 
 // =================================================================================================
 // Forward v2: P and O stay in tensor memory.
@@ -736,32 +464,6 @@ cudaError_t launch_fwd_v2(const CUtensorMap& tq, const CUtensorMap& tk, const CU
   return drop ? launch_fwd_v2_t<D, lb::BIAS_ALIBI, true>(tq, tk, tv, p, s) : launch_fwd_v2_t<D, lb::BIAS_ALIBI, false>(tq, tk, tv, p, s);
 }
 
-int attn_fwd_version() {
-  static int v = -1;
-  if (v < 0) {
-    const char* e = getenv("LIBAI_B200_ATTN_FWD");
-    v = (e != nullptr && e[0] == '1') ? 1 : 2;
-  }
-  return v;
-}
-
-template <int D>
-cudaError_t launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const lb::AttnFwdParams& p,
-                       cudaStream_t s) {
-  if (attn_fwd_version() == 2 || p.bias != nullptr || p.alibi_slopes != nullptr || p.drop_thresh > 0)
-    return launch_fwd_v2<D>(tq, tk, tv, p, s);   // (bias / dropout exist in the v2 kernel only)
-  using Cfg = lb::AttnCfg<D>;
-  auto kern = lb::attn_fwd_kernel<D>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
-  dim3 grid((p.S + lb::ATT_BM - 1) / lb::ATT_BM, p.A, p.B);
-  kern<<<grid, lb::ATT_THREADS, Cfg::SMEM_BYTES, s>>>(tq, tk, tv, p);
-  return cudaGetLastError();
-}
 }  // namespace
 
 // p_drop in [0, 1): attention dropout probability (quantised to 1/256 like the byte-threshold test of the kernel);
@@ -800,7 +502,7 @@ extern "C" int lb_attn_fwd(const void* q, const void* k, const void* v, void* o,
   memset(&p.rng, 0, sizeof(p.rng));
   if (rng != nullptr) p.rng = *rng;
   p.rng_out = rng_out;
-  cudaError_t e = (D == 64) ? launch_fwd<64>(tq, tk, tv, p, s) : launch_fwd<128>(tq, tk, tv, p, s);
+  cudaError_t e = (D == 64) ? launch_fwd_v2<64>(tq, tk, tv, p, s) : launch_fwd_v2<128>(tq, tk, tv, p, s);
   return (int)e;
 }
 

@@ -86,6 +86,9 @@ int lb_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse
                 const long* q_strides, const long* k_strides, const long* v_strides, int causal, float scale,
                 const int* kv_lens, const void* bias, const long* bias_strides, const float* alibi_slopes, float p_drop,
                 const LbRngArgs* rng, long long* rng_out, cudaStream_t s);
+int lb_attn_fwd_pair_rule(int B, int A, int S, int D);
+int lb_attn_fwd_pair(const void* q, const void* k, const void* v, void* o, float* lse, int B, int A, int S, int D, const long* qs, const long* ks,
+                     const long* vs, int causal, float scale, const int* kv_lens, int* err, cudaStream_t s);
 int lb_attn_bwd(const void* dout, const void* q, const void* k, const void* v, const void* o, const float* lse,
                 void* dq, void* dk, void* dv, float* delta, float* dq_accum, int B, int A, int S, int D,
                 const long* q_strides, const long* k_strides, const long* v_strides, const long* do_strides, int causal,
@@ -761,6 +764,13 @@ std::tuple<Tensor, Tensor, Tensor> attn_fwd(const Tensor& q, const Tensor& k, co
     a = next_rng(salt);
   } else {
     rng_state = at::empty({0}, q.options().dtype(at::kLong));
+  }
+  if (!drop && bd.ptr == nullptr && slopes == nullptr && (D == 64 || D == 128) && lb_attn_fwd_pair_rule(B, A, S, D)) {
+    static WaitWord word;
+    check(lb_attn_fwd_pair(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr<float>(), B, A, S, D, qs, ks, vs, causal ? 1 : 0,
+                           (float)scale, kvl, word.device("attn_fwd"), cur_stream()),
+          "attn_fwd");
+    return std::make_tuple(o.permute({0, 2, 1, 3}), lse, rng_state);
   }
   check(lb_attn_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr<float>(), B, A, S, D, qs, ks,
                     vs, causal ? 1 : 0, (float)scale, kvl, bd.ptr, bd.strides, slopes, (float)p_drop, drop ? &a : nullptr,

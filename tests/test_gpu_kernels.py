@@ -7,7 +7,7 @@ import torch
 from torch._subclasses.fake_tensor import FakeTensorMode
 
 from libai_b200.ops import functional as OF
-from libai_b200.ops import so_path
+from libai_b200.ops import load_ext, so_path
 from libai_b200.ops.gated_mlp import gated_mlp
 
 pytestmark = pytest.mark.gpu
@@ -43,6 +43,39 @@ def test_attention_rows_do_not_depend_on_timing(dim, causal):
     assert float(row.max()) < 4 * 2.0 ** -8
     for _ in range(5):
         assert torch.equal(OF.attention_qkvpacked(qkv, causal=causal, scale=dim ** -0.5), first)
+
+
+@pytest.mark.parametrize("lens", [False, True])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("b,s,a,packed", [(1, 8, 1, True), (2, 64, 3, False), (1, 65, 2, True), (2, 129, 200, True), (1, 192, 40, False), (3, 257, 70, True),
+                                          (2, 385, 80, True), (1, 1096, 33, False), (90, 200, 8, True), (1, 2049, 16, True)])
+def test_attention_forward_two_tiles_per_block(b, s, a, packed, dim, causal, lens):
+    """One unit of 64 keys and many, one query tile or two per work item, an odd number of tiles, last units of every width, fewer and
+    more work items than SMs: result and log-sum-exp against float64, the same bits again."""
+    if packed:
+        q, k, v = (t.permute(0, 2, 1, 3) for t in _rand((b, s, a, 3 * dim), 1).split(dim, -1))
+    else:
+        q, k, v = (_rand((b, a, s, dim), 1 + i) for i in range(3))
+    n = torch.tensor([max(1, s - 29 * i * i) for i in range(b)], dtype=torch.int32, device="cuda") if lens else None
+    o, lse, _ = load_ext().attn_fwd(q, k, v, causal, dim ** -0.5, n, None, None, 0.0, 0)
+    assert o.transpose(1, 2).is_contiguous()
+    for i in range(0, b, max(1, b // 3)):
+        z = q[i].double() @ k[i].double().transpose(-1, -2) * dim ** -0.5
+        keep = torch.ones(s, s, dtype=torch.bool, device="cuda")
+        keep = keep.tril() if causal else keep
+        if lens:
+            keep = keep & (torch.arange(s, device="cuda")[None] < n[i])
+        z = z.masked_fill(~keep, -math.inf)
+        prob = torch.softmax(z, -1)
+        want = prob @ v[i].double()
+        # a probability is rounded to bf16 (8 bits: by at most 2^-8 of it, so by 2^-8 of the sum of |p v|), the result once more; 2^-13 for all fp32
+        assert bool(((o[i].double() - want).abs() <= (2.0 ** -8 + 2.0 ** -13) * (prob @ v[i].double().abs() + want.abs())).all())
+        # scores are fp32 sums of `dim` products
+        assert float((lse[i].double() - torch.logsumexp(z, -1)).abs().max()) < 2.0 ** -24 * dim * max(1.0, float(z[keep.expand_as(z)].abs().max()))
+    for _ in range(2):
+        o2, lse2, _ = load_ext().attn_fwd(q, k, v, causal, dim ** -0.5, n, None, None, 0.0, 0)
+        assert torch.equal(o, o2) and torch.equal(lse, lse2)
 
 
 @pytest.mark.parametrize("rms", [False, True])
