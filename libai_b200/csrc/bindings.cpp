@@ -732,6 +732,19 @@ BiasDesc bias_desc(const c10::optional<Tensor>& bias, int B, int A, int S) {
   return d;
 }
 
+// attention without bias or dropout, o [B, S, A, D]
+void attn_fwd_plain(const void* q, const void* k, const void* v, void* o, float* lse, int B, int A, int S, int D, const long* qs, const long* ks,
+                    const long* vs, bool causal, double scale, const int* kv_lens) {
+  if ((D == 64 || D == 128) && lb_attn_fwd_pair_rule(B, A, S, D)) {
+    static WaitWord word;
+    check(lb_attn_fwd_pair(q, k, v, o, lse, B, A, S, D, qs, ks, vs, causal ? 1 : 0, (float)scale, kv_lens, word.device("attn_fwd"), cur_stream()), "attn_fwd");
+  } else {
+    check(lb_attn_fwd(q, k, v, o, lse, B, A, S, D, qs, ks, vs, causal ? 1 : 0, (float)scale, kv_lens, nullptr, nullptr, nullptr, 0.f, nullptr, nullptr,
+                      cur_stream()),
+          "attn_fwd");
+  }
+}
+
 // returns (o, lse, rng_state): rng_state int64[2] = (seed, offset) of the dropout mask (empty without dropout)
 std::tuple<Tensor, Tensor, Tensor> attn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, bool causal, double scale,
                                             const c10::optional<Tensor>& kv_lens, const c10::optional<Tensor>& bias,
@@ -765,11 +778,8 @@ std::tuple<Tensor, Tensor, Tensor> attn_fwd(const Tensor& q, const Tensor& k, co
   } else {
     rng_state = at::empty({0}, q.options().dtype(at::kLong));
   }
-  if (!drop && bd.ptr == nullptr && slopes == nullptr && (D == 64 || D == 128) && lb_attn_fwd_pair_rule(B, A, S, D)) {
-    static WaitWord word;
-    check(lb_attn_fwd_pair(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr<float>(), B, A, S, D, qs, ks, vs, causal ? 1 : 0,
-                           (float)scale, kvl, word.device("attn_fwd"), cur_stream()),
-          "attn_fwd");
+  if (!drop && bd.ptr == nullptr && slopes == nullptr) {
+    attn_fwd_plain(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr<float>(), B, A, S, D, qs, ks, vs, causal, scale, kvl);
     return std::make_tuple(o.permute({0, 2, 1, 3}), lse, rng_state);
   }
   check(lb_attn_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr<float>(), B, A, S, D, qs, ks,
@@ -961,6 +971,156 @@ std::tuple<Tensor, Tensor, Tensor> attn_decode(const Tensor& q, const Tensor& k_
 }
 
 // ---- fused collectives ---------------------------------------------------------------------------------------
+// ---- whole blocks without a graph ---------------------------------------------------------------------------------
+// The forward of a transformer block launched from here: a generation step's kernels take 2 to 9 us each, an operator call from Python 14 to
+// 25 us (views, checks, dispatch, one allocation per result), and eight modules per block as much again.  The same kernels in the same order
+// as the modules launch them, intermediate results in one allocation.  An empty answer: not of the form that these take, the caller's modules
+// run (and report what is wrong with it).
+bool block_tensor(const Tensor& t, const Tensor& x) {
+  return t.defined() && t.is_cuda() && t.device() == x.device() && t.scalar_type() == at::kBFloat16 && t.is_contiguous() &&
+         (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
+}
+bool block_vector(const Tensor& t, const Tensor& x, int64_t n) { return block_tensor(t, x) && t.dim() == 1 && t.size(0) == n; }
+bool block_matrix(const Tensor& t, const Tensor& x, int64_t n, int64_t k) {
+  return block_tensor(t, x) && t.dim() == 2 && t.size(0) == n && t.size(1) == k && n % 8 == 0 && k % 8 == 0;
+}
+// [B, A, past, d] views whose rows are whole 16-byte vectors (attention_cached's condition)
+bool block_cache(const Tensor& t, const Tensor& x, int64_t B, int64_t A, int64_t d) {
+  if (!(t.defined() && t.is_cuda() && t.device() == x.device() && t.scalar_type() == at::kBFloat16 && t.dim() == 4 && t.size(0) == B && t.size(1) == A &&
+        t.size(3) == d && t.size(2) > 0 && t.stride(3) == 1 && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0))
+    return false;
+  for (int i = 0; i < 3; ++i)
+    if (t.size(i) != 1 && (t.stride(i) <= 0 || t.stride(i) % 8 != 0)) return false;
+  return true;
+}
+
+struct BlockScratch {                       // pieces of one allocation, 256-byte aligned
+  Tensor mem;
+  int64_t bytes = 0;
+  int64_t add(int64_t n) {
+    const int64_t at = bytes;
+    bytes += (n + 255) / 256 * 256;
+    return at;
+  }
+  void make(const Tensor& x) { mem = at::empty({bytes}, x.options().dtype(at::kByte)); }
+  char* operator()(int64_t at) const { return static_cast<char*>(mem.data_ptr()) + at; }
+};
+
+// attention of the packed projection qkv [B, S, A, 3 d] into ctx [B, S, A, d]; with caches the grown ones are appended to `out`
+void block_attention(const char* qkv, char* ctx, float* lse, int64_t B, int64_t S, int64_t A, int64_t d, bool causal, double scale,
+                     const c10::optional<Tensor>& past_k, const c10::optional<Tensor>& past_v, std::vector<Tensor>& out) {
+  const long st[3] = {(long)(S * A * 3 * d), (long)(3 * d), (long)(A * 3 * d)};
+  const char *q = qkv, *k = qkv + 2 * d, *v = qkv + 4 * d;
+  if (past_k.has_value()) {
+    long ks[3], vs[3];
+    split_strides(*past_k, past_k->device(), ks);
+    split_strides(*past_v, past_v->device(), vs);
+    const int64_t past = past_k->size(2);
+    Tensor ko = at::empty({B, A, past + 1, d}, past_k->options()), vo = at::empty({B, A, past + 1, d}, past_k->options());
+    check(lb_attn_decode(q, k, v, past_k->data_ptr(), past_v->data_ptr(), ko.data_ptr(), vo.data_ptr(), ctx, (int)B, (int)A, (int)past, (int)d, st, st, st, ks,
+                         vs, (float)scale, nullptr, nullptr, 0, 0, cur_stream()),
+          "attn_decode");
+    out.push_back(ko);
+    out.push_back(vo);
+  } else if (d == 64 || d == 128) {
+    attn_fwd_plain(q, k, v, ctx, lse, (int)B, (int)A, (int)S, (int)d, st, st, st, causal, scale, nullptr);
+  } else {
+    check(lb_attn_split_fwd(q, k, v, ctx, nullptr, lse, (int)B, (int)A, (int)S, (int)S, (int)d, st, st, st, causal ? 1 : 0, (float)scale, nullptr, nullptr, 0,
+                            0, split_word().device("attn_split"), cur_stream()),
+          "attn_split_fwd");
+  }
+}
+// forms that block_attention takes
+bool block_attention_ok(const Tensor& x, int64_t A, int64_t d, double scale, const c10::optional<Tensor>& past_k, const c10::optional<Tensor>& past_v) {
+  const int64_t B = x.size(0), S = x.size(1);
+  if (x.numel() == 0 || B > 65535 || A > 65535 || B * S > (int64_t(1) << 30) || !(scale > 0)) return false;
+  if (past_k.has_value() != past_v.has_value()) return false;
+  if (past_k.has_value())
+    return S == 1 && d % 8 == 0 && d <= 256 && block_cache(*past_k, x, B, A, d) && block_cache(*past_v, x, B, A, d) && past_k->size(2) == past_v->size(2);
+  return d == 64 || d == 128 || (d % 8 == 0 && d >= 8 && d <= 64);
+}
+void block_linear(const void* x, const Tensor& w, const void* bias, int act, void* y, int64_t rows) {
+  check(lb_gemm_bf16(x, w.data_ptr(), y, (int)rows, (int)w.size(0), (int)w.size(1), (int)w.size(1), (int)w.size(1), (int)w.size(0), 0, 0, bias, act, nullptr,
+                     0, 0, cur_stream()),
+        "linear_fwd");
+}
+
+// Pre-norm block: params = norm weight, bias; qkv weight, bias; projection weight, bias; norm weight, bias; h->4h weight, bias; 4h->h weight, bias.
+// x [B, S, h] -> {y} or, against caches, {y, keys, values}
+std::vector<Tensor> block_fwd(const Tensor& x, const std::vector<Tensor>& p, int64_t heads, double eps1, double eps2, double scale, bool causal,
+                              const c10::optional<Tensor>& past_k, const c10::optional<Tensor>& past_v) {
+  if (p.size() != 12 || x.dim() != 3 || !block_tensor(x, x) || heads <= 0 || !p[2].defined() || p[2].dim() != 2 || !p[8].defined() || p[8].dim() != 2) return {};
+  const int64_t B = x.size(0), S = x.size(1), h = x.size(2), T = B * S, ad = p[2].size(0) / 3, f = p[8].size(0), d = ad / heads;
+  if (p[2].size(0) != 3 * heads * d || !block_attention_ok(x, heads, d, scale, past_k, past_v) || !block_vector(p[0], x, h) || !block_vector(p[1], x, h) ||
+      !block_matrix(p[2], x, 3 * ad, h) || !block_vector(p[3], x, 3 * ad) || !block_matrix(p[4], x, h, ad) || !block_vector(p[5], x, h) ||
+      !block_vector(p[6], x, h) || !block_vector(p[7], x, h) || !block_matrix(p[8], x, f, h) || !block_vector(p[9], x, f) || !block_matrix(p[10], x, h, f) ||
+      !block_vector(p[11], x, h))
+    return {};
+  c10::cuda::CUDAGuard guard(x.device());
+  BlockScratch s;
+  const int64_t norm = s.add(T * std::max(h, ad) * 2), wide = s.add(T * std::max(3 * ad, f) * 2), mid = s.add(T * h * 2), stats = s.add(T * std::max<int64_t>(2, heads) * 4);
+  s.make(x);
+  std::vector<Tensor> out{at::empty_like(x)};
+  float* st = reinterpret_cast<float*>(s(stats));
+  check(lb_norm_fwd(x.data_ptr(), p[0].data_ptr(), p[1].data_ptr(), s(norm), st, st + T, (int)T, (int)h, (float)eps1, 0, 0, 0, cur_stream()), "norm_fwd");
+  block_linear(s(norm), p[2], p[3].data_ptr(), 0, s(wide), T);
+  block_attention(s(wide), s(norm), st, B, S, heads, d, causal, scale, past_k, past_v, out);
+  check(lb_gemm_bf16_bias_residual(s(norm), p[4].data_ptr(), s(mid), (int)T, (int)h, (int)ad, (int)ad, (int)ad, p[5].data_ptr(), x.data_ptr(), cur_stream()),
+        "linear_bias_residual");
+  check(lb_norm_fwd(s(mid), p[6].data_ptr(), p[7].data_ptr(), s(norm), st, st + T, (int)T, (int)h, (float)eps2, 0, 0, 0, cur_stream()), "norm_fwd");
+  block_linear(s(norm), p[8], p[9].data_ptr(), 1 /* GELU */, s(wide), T);
+  check(lb_gemm_bf16_bias_residual(s(wide), p[10].data_ptr(), out[0].data_ptr(), (int)T, (int)h, (int)f, (int)f, (int)f, p[11].data_ptr(), s(mid), cur_stream()),
+        "linear_bias_residual");
+  return out;
+}
+
+// Llama block: params = norm weight; qkv weight; projection weight; norm weight; gate, up, down weights; `bias` of qkv or none.  `joint`: gate and
+// up lie side by side in memory and may be one product
+std::vector<Tensor> llama_block_fwd(const Tensor& x, const std::vector<Tensor>& p, const c10::optional<Tensor>& bias, const Tensor& cosv, const Tensor& sinv,
+                                    int64_t heads, double eps1, double eps2, double scale, bool joint, const c10::optional<Tensor>& past_k,
+                                    const c10::optional<Tensor>& past_v) {
+  if (p.size() != 7 || x.dim() != 3 || !block_tensor(x, x) || heads <= 0 || !p[1].defined() || p[1].dim() != 2 || !p[4].defined() || p[4].dim() != 2) return {};
+  const int64_t B = x.size(0), S = x.size(1), h = x.size(2), T = B * S, ad = p[1].size(0) / 3, f = p[4].size(0), d = ad / heads;
+  const int64_t at0 = past_k.has_value() && past_k->dim() == 4 ? past_k->size(2) : 0;
+  if (p[1].size(0) != 3 * heads * d || !block_attention_ok(x, heads, d, scale, past_k, past_v) || (!past_k.has_value() && d != 64 && d != 128) || d % 2 ||
+      !block_vector(p[0], x, h) || !block_matrix(p[1], x, 3 * ad, h) || !block_matrix(p[2], x, h, ad) || !block_vector(p[3], x, h) ||
+      !block_matrix(p[4], x, f, h) || !block_matrix(p[5], x, f, h) || !block_matrix(p[6], x, h, f) || (bias.has_value() && !block_vector(*bias, x, 3 * ad)))
+    return {};
+  for (const Tensor* t : {&cosv, &sinv})
+    if (!(t->defined() && t->is_cuda() && t->device() == x.device() && t->scalar_type() == at::kFloat && t->dim() == 2 && t->is_contiguous() &&
+          t->size(0) >= S + at0 && t->size(1) == d))
+      return {};
+  if (cosv.sizes() != sinv.sizes()) return {};
+  c10::cuda::CUDAGuard guard(x.device());
+  joint = joint && p[5].data_ptr() == static_cast<char*>(p[4].data_ptr()) + p[4].nbytes() && p[4].storage().data() == p[5].storage().data();
+  BlockScratch s;
+  const int64_t norm = s.add(T * std::max(h, ad) * 2), wide = s.add(T * std::max(3 * ad, 2 * f) * 2), rot = s.add(T * std::max(3 * ad, f) * 2),
+                mid = s.add(T * h * 2), add = s.add(T * h * 2), stats = s.add(T * std::max<int64_t>(1, heads) * 4);
+  s.make(x);
+  std::vector<Tensor> out{at::empty_like(x)};
+  float* st = reinterpret_cast<float*>(s(stats));
+  check(lb_norm_fwd(x.data_ptr(), p[0].data_ptr(), nullptr, s(norm), nullptr, st, (int)T, (int)h, (float)eps1, 1, 0, 0, cur_stream()), "norm_fwd");
+  block_linear(s(norm), p[1], bias.has_value() ? bias->data_ptr() : nullptr, 0, s(wide), T);
+  check(lb_rope_qkv(s(wide), cosv.data_ptr<float>(), sinv.data_ptr<float>(), s(rot), T * heads, (int)S, (int)heads, (int)d, (int)at0, 0, cur_stream()), "rope_qkv");
+  block_attention(s(rot), s(norm), st, B, S, heads, d, true, scale, past_k, past_v, out);
+  block_linear(s(norm), p[2], nullptr, 0, s(add), T);
+  check(lb_bias_residual(s(add), nullptr, x.data_ptr(), s(mid), T, (int)h, cur_stream()), "bias_residual");
+  check(lb_norm_fwd(s(mid), p[3].data_ptr(), nullptr, s(norm), nullptr, st, (int)T, (int)h, (float)eps2, 1, 0, 0, cur_stream()), "norm_fwd");
+  if (joint) {
+    check(lb_gemm_bf16(s(norm), p[4].data_ptr(), s(wide), (int)T, (int)(2 * f), (int)h, (int)h, (int)h, (int)(2 * f), 0, 0, nullptr, 0, nullptr, 0, 0, cur_stream()),
+          "gemm");
+    check(lb_swiglu_packed_fwd(s(wide), s(rot), T, f, cur_stream()), "swiglu_packed_fwd");
+  } else {
+    char* up = s(wide) + T * f * 2;
+    block_linear(s(norm), p[4], nullptr, 0, s(wide), T);
+    block_linear(s(norm), p[5], nullptr, 0, up, T);
+    check(lb_swiglu_fwd(s(wide), up, s(rot), T * f, cur_stream()), "swiglu_fwd");
+  }
+  block_linear(s(rot), p[6], nullptr, 0, s(add), T);
+  check(lb_bias_residual(s(add), nullptr, s(mid), out[0].data_ptr(), T, (int)h, cur_stream()), "bias_residual");
+  return out;
+}
+
 std::vector<long> to_longs(at::IntArrayRef v) { return std::vector<long>(v.begin(), v.end()); }
 
 const void* opt_ptr(const c10::optional<Tensor>& t) { return (t.has_value() && t->defined()) ? t->data_ptr() : nullptr; }
@@ -1085,6 +1245,8 @@ TORCH_LIBRARY(libai_b200, m) {
   m.def("masked_attention_tc(Tensor q, Tensor kmat, Tensor vmat, Tensor ext_off, Tensor nsink, Tensor cstart, Tensor? gate, bool gate_wide, Tensor seq_off, Tensor past, Tensor qt_seq, Tensor qt_start, Tensor(a!) y, int H, int G, int D, int V, int window, int chunk, float scale, float out_scale, float temp_coef, float temp_every) -> ()", &masked_attention_tc);
   m.def("latent_prompt_tc(Tensor q, Tensor kv, Tensor rot, Tensor cs, Tensor? sink, Tensor ext_off, Tensor seq_off, Tensor past, Tensor qt_seq, Tensor qt_start, Tensor(a!) y, int H, int D, int R, int V, float scale) -> ()", &latent_prompt_tc);
   m.def("linear_bias_residual(Tensor x, Tensor w, Tensor? bias, Tensor residual) -> Tensor", &linear_bias_residual);
+  m.def("block_fwd(Tensor x, Tensor[] params, int heads, float eps1, float eps2, float scale, bool causal, Tensor? past_k, Tensor? past_v) -> Tensor[]", &block_fwd);
+  m.def("llama_block_fwd(Tensor x, Tensor[] params, Tensor? bias, Tensor cos, Tensor sin, int heads, float eps1, float eps2, float scale, bool joint, Tensor? past_k, Tensor? past_v) -> Tensor[]", &llama_block_fwd);
   m.def("embedding_fwd(Tensor ids, Tensor table, int vocab_start) -> Tensor", &embedding_fwd);
   m.def("embedding_bwd(Tensor ids, Tensor gy, Tensor(a!) grad, int vocab_start) -> ()", &embedding_bwd);
   m.def("gemm_tuned(Tensor a, Tensor b, int layout, int bn, int splits, bool fp32_out) -> Tensor", &gemm_tuned);

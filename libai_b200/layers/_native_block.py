@@ -1,0 +1,59 @@
+"""Whole blocks without a graph as one native call.
+
+A generation step's kernels take 2 to 9 us each; launched module by module from Python an operator costs 14 to 25 us and a module call a few
+more.  Where nothing can tell the difference (no graph, no transform or trace, plain modules without hooks, plain bf16 parameters, one
+tensor-parallel rank, no active dropout, no mask) the block's kernels are launched in the same order from C++ (``block_fwd`` and
+``llama_block_fwd`` in ``csrc/bindings.cpp``, which look at the tensors); everything else runs through the modules as ever, so ``None`` is
+always a safe answer.  Nothing is kept from one call for the next.
+"""
+import torch
+from torch.nn import Parameter
+from torch.nn.modules import module as _module
+
+from libai_b200 import ops
+from libai_b200.ops import functional as OF
+from libai_b200.utils import distributed as dutil
+
+_FORWARDS = {}
+
+
+def remember(*classes):
+    """The forwards that a native call stands for (a class whose ``forward`` is replaced later runs through its modules)."""
+    for cls in classes:
+        _FORWARDS[cls] = cls.forward
+
+
+def applies(x) -> bool:
+    """What holds for the call as a whole."""
+    return (not torch.is_grad_enabled() and type(x) is torch.Tensor and x.dtype is torch.bfloat16 and x.dim() == 3 and ops.use_native(x)
+            and OF._plain_call() and not ops.fp8_enabled() and dutil.get_dist_util().tensor_parallel_size == 1
+            and not _module._global_forward_hooks and not _module._global_forward_pre_hooks)
+
+
+def plain(m, cls) -> bool:
+    """A module of this very class whose call is its class's ``forward`` and nothing else."""
+    return (type(m) is cls and cls.forward is _FORWARDS[cls] and not m._forward_hooks and not m._forward_pre_hooks and "forward" not in m.__dict__)
+
+
+def parameters(*pairs):
+    """``(module, name, ...)`` tuples → their parameters, or ``None`` where one is missing or of another kind (a view, a parametrization)."""
+    out = []
+    for m, *names in pairs:
+        for name in names:
+            p = m._parameters.get(name)
+            if type(p) is not Parameter:
+                return None
+            out.append(p)
+    return out
+
+
+def past_pair(past, heads: int, x):
+    """``(keys, values)`` of a cache that one new token may join in one kernel, ``(None, None)`` without one, else ``None``."""
+    if past is None:
+        return None, None
+    if len(past) != 2 or x.shape[1] != 1 or not all(type(t) is torch.Tensor and t.dim() == 4 for t in past):
+        return None
+    b = x.shape[0]
+    if b * heads < 4 and OF._cache_too_long_for_one_cluster(b * heads, past[0].shape[2], past[0].shape[3]):
+        return None
+    return past

@@ -8,11 +8,17 @@ The pipeline hand-off the reference performs inside ``forward`` (``to_global(pla
 """
 from torch import nn
 
+from libai_b200.ops import count_launch, load_ext
+
+from . import _native_block as native
 from ._param import xavier_normal_
 from .attention import AttnMaskType, MultiheadAttention
 from .droppath import DropPath
 from .layer_norm import LayerNorm
+from .linear import Linear
 from .mlp import MLP
+
+native.remember(LayerNorm, MultiheadAttention, Linear, MLP)
 
 
 class TransformerLayer(nn.Module):
@@ -89,6 +95,10 @@ class TransformerLayer(nn.Module):
     ):
         """``past_key_value``: ``(self_k, self_v[, cross_k, cross_v])``; returns hidden states, and
         the updated cache tuple when ``use_cache``."""
+        if attention_mask is None and encoder_states is None and native.applies(hidden_states):
+            done = self._native_forward(hidden_states, past_key_value, use_cache)
+            if done is not None:
+                return done
         self_past = cross_past = None
         if past_key_value is not None:
             self_past = past_key_value[:2]
@@ -135,6 +145,31 @@ class TransformerLayer(nn.Module):
         if use_cache:
             return output, presents
         return output
+
+    def _native_forward(self, x, past, use_cache):
+        """The block without a graph as one native call; ``None``: the modules have to run."""
+        if self.is_decoder or self.apply_residual_post_layernorm or not self.plain_residual or (use_cache and past is None):
+            return None
+        mods = self._modules
+        ln1, attn, ln2, mlp = mods["input_layernorm"], mods["self_attention"], mods["post_attention_layernorm"], mods["mlp"]
+        plain = native.plain
+        if not (plain(ln1, LayerNorm) and plain(attn, MultiheadAttention) and plain(ln2, LayerNorm) and plain(mlp, MLP)):
+            return None
+        qkv, dense, up, down = attn._modules.get("query_key_value"), attn._modules["dense"], mlp._modules["dense_h_to_4h"], mlp._modules["dense_4h_to_h"]
+        if (not (plain(qkv, Linear) and plain(dense, Linear) and plain(up, Linear) and plain(down, Linear))
+                or qkv.skip_bias_add or up.skip_bias_add or len(ln1.normalized_shape) != 1 or len(ln2.normalized_shape) != 1
+                or (attn.training and (attn.attention_dropout_prob > 0.0 or attn.output_dropout_prob > 0.0)) or (mlp.training and mlp.output_dropout_prob > 0.0)):
+            return None
+        both = ("weight", "bias")
+        params = native.parameters((ln1, *both), (qkv, *both), (dense, *both), (ln2, *both), (up, *both), (down, *both))
+        pair = native.past_pair(past, attn.local_heads, x)
+        if params is None or pair is None:
+            return None
+        out = load_ext().block_fwd(x, params, attn.local_heads, ln1.eps, ln2.eps, attn.softmax_scale, attn.attn_mask_type == AttnMaskType.causal, *pair)
+        if not out:
+            return None
+        count_launch(7)
+        return (out[0], tuple(out[1:])) if use_cache else out[0]
 
     def build_attention(self, is_cross_attention=False):
         return MultiheadAttention(

@@ -21,9 +21,11 @@ from torch import nn
 
 from libai_b200.config import configurable
 from libai_b200.layers import Linear, RMSLayerNorm, VocabEmbedding
+from libai_b200.layers import _native_block as native
 from libai_b200.layers._param import xavier_normal_
 from libai_b200.layers.attention import AttnMaskType
 from libai_b200.layers.embedding import get_sp_shape, set_sp_shape
+from libai_b200.ops import count_launch, load_ext
 from libai_b200.ops import functional as OF
 from libai_b200.parallel import mappings
 from libai_b200.utils import distributed as dutil
@@ -200,6 +202,10 @@ class LlamaDecoderLayer(nn.Module):
 
     def forward(self, hidden_states, attention_mask=None, past_key_value=None, cos_cached=None, sin_cached=None,
                 use_cache=False):
+        if attention_mask is None and native.applies(hidden_states):
+            done = self._native_forward(hidden_states, past_key_value, cos_cached, sin_cached, use_cache)
+            if done is not None:
+                return done
         attn = self.self_attn(self.input_layernorm(hidden_states), attention_mask=attention_mask,
                               past_key_value=past_key_value, cos_cached=cos_cached, sin_cached=sin_cached,
                               use_cache=use_cache)
@@ -209,6 +215,35 @@ class LlamaDecoderLayer(nn.Module):
         hidden_states = hidden_states + attn
         output = hidden_states + self.mlp(self.post_attention_layernorm(hidden_states))
         return (output, presents) if use_cache else output
+
+    def _native_forward(self, x, past, cos, sin, use_cache):
+        """The block without a graph as one native call; ``None``: the modules have to run."""
+        from libai_b200.ops import gated_mlp
+
+        mods = self._modules
+        ln1, attn, ln2, mlp = mods["input_layernorm"], mods["self_attn"], mods["post_attention_layernorm"], mods["mlp"]
+        plain = native.plain
+        if not (plain(ln1, RMSLayerNorm) and plain(attn, LlamaAttention) and plain(ln2, RMSLayerNorm) and plain(mlp, LlamaMLP)) or (use_cache and past is None):
+            return None
+        qkv, proj = attn._modules["query_key_value"], attn._modules["o_proj"]
+        gate, up, down = mlp._modules["gate_proj"], mlp._modules["up_proj"], mlp._modules["down_proj"]
+        if (not (plain(qkv, Linear) and plain(proj, Linear) and plain(gate, Linear) and plain(up, Linear) and plain(down, Linear))
+                or ln1.zero_centered or ln2.zero_centered or any(m.skip_bias_add for m in (qkv, proj, gate, up, down))
+                or any(m._parameters.get("bias") is not None for m in (proj, gate, up, down)) or type(cos) is not torch.Tensor or type(sin) is not torch.Tensor):
+            return None
+        params = native.parameters((ln1, "weight"), (qkv, "weight"), (proj, "weight"), (ln2, "weight"), (gate, "weight"), (up, "weight"), (down, "weight"))
+        pair = native.past_pair(past, attn.local_heads, x)
+        bias = qkv._parameters.get("bias")
+        if params is None or pair is None or (bias is not None and type(bias) is not nn.Parameter):
+            return None
+        out = load_ext().llama_block_fwd(x, params, bias, cos, sin, attn.local_heads, ln1.eps, ln2.eps, attn.norm_factor, gated_mlp.enabled(), *pair)
+        if not out:
+            return None
+        count_launch(11)                # one more where gate and up projection are two products
+        return (out[0], tuple(out[1:])) if use_cache else out[0]
+
+
+native.remember(RMSLayerNorm, LlamaAttention, Linear, LlamaMLP)
 
 
 class LlamaModel(nn.Module):

@@ -516,3 +516,113 @@ def test_attention_backward_from_tensors_saved_on_the_host(d, pin):
     with torch.autograd.graph.save_on_cpu(pin_memory=pin):
         out = OF.attention(q, k, v, causal=True)
     assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(out, (q, k, v), go), want))
+
+
+def _gpt_block(heads, dim, mask="causal", **kw):
+    from libai_b200.layers import TransformerLayer
+    from libai_b200.layers._param import param_defaults
+    from libai_b200.layers.attention import AttnMaskType
+
+    with param_defaults(dtype=BF16, device="cuda", seed=3):
+        m = TransformerLayer(heads * dim, 3 * heads * dim, heads, attn_mask_type=getattr(AttnMaskType, mask), **kw)
+    with torch.no_grad():
+        for i, p in enumerate(m.parameters()):
+            p.copy_(_rand(p.shape, i, 0.05) + (1.0 if i in (0, 6) else 0.0))
+    return m.eval()
+
+
+def _llama_block(heads, dim, joint):
+    from libai_b200.layers._param import param_defaults
+    from libai_b200.models.llama_model import LlamaDecoderLayer
+
+    with param_defaults(dtype=BF16, device="cuda", seed=3):
+        m = LlamaDecoderLayer(heads * dim, 2 * heads * dim, heads, qkv_bias=joint)
+    with torch.no_grad():
+        for i, p in enumerate(m.parameters()):
+            p.copy_(_rand(p.shape, i, 0.05) + (1.0 if p.dim() == 1 and p.shape[0] == heads * dim else 0.0))
+        if joint:                                              # side by side, as an optimizer's flat buffer has them
+            g, u = m.mlp.gate_proj, m.mlp.up_proj
+            both = torch.cat([g.weight, u.weight])
+            g.weight.data, u.weight.data = both[:g.weight.shape[0]], both[g.weight.shape[0]:]
+    return m.eval()
+
+
+def _by_modules(m, call):
+    """The same call with a hook that has to see the MLP: the modules run one by one."""
+    seen = []
+    handle = m.mlp.register_forward_hook(lambda *a: seen.append(1))
+    out = call()
+    handle.remove()
+    assert seen
+    return out
+
+
+def _flat(out):
+    return [out] if torch.is_tensor(out) else [out[0], *out[1]]
+
+
+@pytest.mark.parametrize("past", [None, 1, 70])
+@pytest.mark.parametrize("b,s,heads,dim,mask", [(1, 1, 4, 24, "causal"), (2, 37, 16, 24, "causal"), (3, 130, 3, 64, "causal"), (1, 200, 2, 128, "padding"),
+                                                (2, 65, 4, 48, "padding"), (1, 9, 1, 72, "causal")])
+def test_block_without_a_graph_in_one_call(b, s, heads, dim, mask, past):
+    """The native call and the modules: the same bits, with and without a cache; head dims that neither attention takes as well."""
+    m = _gpt_block(heads, dim, mask)
+    x = _rand((b, 1 if past else s, heads * dim), 1)
+    kv = None if past is None else tuple(_rand((b, heads, past, dim), 5 + i) for i in range(2))
+    with torch.no_grad():
+        for use_cache in (False, True):
+            call = lambda: m(x, past_key_value=kv, use_cache=use_cache)
+            for got, want in zip(_flat(call()), _flat(_by_modules(m, call))):
+                assert torch.equal(got, want) and got.stride() == want.stride() and not got.requires_grad
+        y = m(x.transpose(0, 1).contiguous().transpose(0, 1), past_key_value=kv)
+        assert torch.equal(y, m(x, past_key_value=kv))
+
+
+@pytest.mark.parametrize("joint", [False, True])
+@pytest.mark.parametrize("past", [None, 1, 70])
+@pytest.mark.parametrize("b,s,heads,dim", [(1, 1, 4, 64), (2, 70, 3, 128), (3, 33, 2, 48)])
+def test_llama_block_without_a_graph_in_one_call(b, s, heads, dim, past, joint):
+    m = _llama_block(heads, dim, joint)
+    x = _rand((b, 1 if past else s, heads * dim), 1)
+    kv = None if past is None else tuple(_rand((b, heads, past, dim), 5 + i) for i in range(2))
+    cos, sin = _ROT(128, dim)
+    with torch.no_grad():
+        for use_cache in (False, True):
+            call = lambda: m(x, past_key_value=kv, cos_cached=cos, sin_cached=sin, use_cache=use_cache)
+            for got, want in zip(_flat(call()), _flat(_by_modules(m, call))):
+                assert torch.equal(got, want) and got.stride() == want.stride() and not got.requires_grad
+
+
+def test_block_in_one_call_leaves_everything_else_to_the_modules():
+    """Masks, active dropout, replaced forwards, replaced modules, functional parameters, transforms, graph capture."""
+    from libai_b200.layers import MLP
+
+    m, x = _gpt_block(4, 64), _rand((2, 40, 256), 1)
+    with torch.no_grad():
+        base = m(x)
+        keep = torch.ones(2, 1, 40, 40, dtype=torch.bool, device="cuda").tril()
+        assert float((m(x, keep) - base).float().norm()) < 2.0 ** -7 * float(base.float().norm())
+        d = _gpt_block(4, 64, output_dropout_prob=0.5)
+        assert torch.equal(d(x), base) and not torch.equal(d.train()(x), base)
+        old, calls = MLP.forward, []
+        try:
+            MLP.forward = lambda self, *a, **k: (calls.append(1), old(self, *a, **k))[1]
+            assert torch.equal(m(x), base) and calls
+        finally:
+            MLP.forward = old
+        m.mlp.forward = lambda h, residual=None: residual
+        assert not torch.equal(m(x), base)
+        del m.mlp.forward
+        half = {k: (v * 0.5 if v.dim() == 2 else v).detach() for k, v in m.named_parameters()}
+        assert not torch.equal(torch.func.functional_call(m, half, (x,)), base)
+        assert torch.equal(torch.func.vmap(lambda t: t * 2)(x), x * 2) and torch.equal(m(x), base)
+        side = torch.cuda.Stream()
+        with torch.cuda.stream(side):
+            m(x)
+        side.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            y = m(x)
+        graph.replay()
+        assert torch.equal(y, base)
+    assert m(x).requires_grad
