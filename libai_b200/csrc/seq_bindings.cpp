@@ -11,9 +11,10 @@ int lbs_rmsnorm(const void* x, long ldx, int xdtype, const int64_t* ids, const v
 int lbs_slice_act(const void* in, long ldi, int idtype, void* out, long ldo, int odtype, long rows, int n, int act, cudaStream_t s);
 int lbs_short_conv(const void* in, long ldi, const void* w, void* tail, const int* tok_seq, const int* seq_off, const int* slots,
                    const int* past, void* out, long ldo, long tokens, int B, int C, int taps, int dtype, cudaStream_t s);
+long lbs_delta_work(long tokens, int B, long ldq, int koff, int voff, int H, int KH, int D, int V, int chan, int dtype, long longest);
 int lbs_delta_scan(const void* qkv, long ldq, int koff, int voff, const void* a, long lda, const void* bl, long ldb, const void* A_log,
                    const void* dt_bias, float* S, const int* seq_off, const int* slots, const int* past, float* out, float* work,
-                   long tokens, int B, int H, int KH, int D, int V, int chan, int dtype, cudaStream_t s);
+                   long tokens, int B, int H, int KH, int D, int V, int chan, int dtype, long shortest, long longest, cudaStream_t s);
 int lbs_gated_rmsnorm(const float* o, const void* gate, long ldg, const void* w, float eps, int act, void* y, long ldy, long rows,
                       int H, int V, int dtype, cudaStream_t s);
 int lbs_latent_gather(const void* ring, const void* cnew, const int* ext_seq, const int* ext_off, const int* seq_off, const int* slots,
@@ -86,7 +87,7 @@ void short_conv(const Tensor& in, const Tensor& w, Tensor tail, const Tensor& to
 
 void delta_scan(const Tensor& qkv, int64_t koff, int64_t voff, const Tensor& a, const Tensor& b, const Tensor& A_log,
                 const Tensor& dt_bias, Tensor S, const Tensor& seq_off, const Tensor& slots, const Tensor& past, Tensor out,
-                int64_t KH, bool chan) {
+                int64_t KH, bool chan, int64_t shortest, int64_t longest) {
   rows2d(qkv, "delta_scan qkv"); rows2d(a, "delta_scan a"); rows2d(b, "delta_scan b");
   TORCH_CHECK(S.dim() == 4 && S.is_contiguous() && S.scalar_type() == at::kFloat, "delta_scan: S must be fp32 [slots, H, D, V]");
   const int H = (int)S.size(1), D = (int)S.size(2), V = (int)S.size(3);
@@ -100,10 +101,11 @@ void delta_scan(const Tensor& qkv, int64_t koff, int64_t voff, const Tensor& a, 
   TORCH_CHECK(A_log.is_contiguous() && dt_bias.is_contiguous(), "delta_scan: contiguous constants");
   c10::cuda::CUDAGuard guard(qkv.device());
   const int64_t tokens = qkv.size(0);
-  Tensor work = at::empty({tokens * (2 * KH * D + KH + H + (chan ? (int64_t)H * D : (int64_t)H))}, out.options());
+  Tensor work = at::empty({lbs_delta_work(tokens, (int)slots.numel(), qkv.stride(0), (int)koff, (int)voff, H, (int)KH, D, V, chan ? 1 : 0, code(qkv), longest)}, out.options());
   check(lbs_delta_scan(qkv.data_ptr(), qkv.stride(0), (int)koff, (int)voff, a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0),
                        A_log.data_ptr(), dt_bias.data_ptr(), S.data_ptr<float>(), meta(seq_off), meta(slots), meta(past),
-                       out.data_ptr<float>(), work.data_ptr<float>(), tokens, (int)slots.numel(), H, (int)KH, D, V, chan ? 1 : 0, code(qkv), cur_stream()), "delta_scan");
+                       out.data_ptr<float>(), work.data_ptr<float>(), tokens, (int)slots.numel(), H, (int)KH, D, V, chan ? 1 : 0, code(qkv), shortest,
+                       longest, cur_stream()), "delta_scan");
 }
 
 void gated_rmsnorm(const Tensor& o, const Tensor& gate, const Tensor& w, double eps, int64_t act, Tensor y, int64_t H, int64_t V) {
@@ -198,7 +200,7 @@ TORCH_LIBRARY(libai_b200_seq, m) {
   m.def("rmsnorm(Tensor x, Tensor? ids, Tensor w, float offset, float eps, Tensor(a!) out) -> ()", &rmsnorm);
   m.def("slice_act(Tensor inp, Tensor(a!) out, int act) -> ()", &slice_act);
   m.def("short_conv(Tensor inp, Tensor w, Tensor(a!) tail, Tensor tok_seq, Tensor seq_off, Tensor slots, Tensor past, Tensor(b!) out) -> ()", &short_conv);
-  m.def("delta_scan(Tensor qkv, int koff, int voff, Tensor a, Tensor b, Tensor A_log, Tensor dt_bias, Tensor(a!) S, Tensor seq_off, Tensor slots, Tensor past, Tensor(b!) out, int kv_heads, bool chan) -> ()", &delta_scan);
+  m.def("delta_scan(Tensor qkv, int koff, int voff, Tensor a, Tensor b, Tensor A_log, Tensor dt_bias, Tensor(a!) S, Tensor seq_off, Tensor slots, Tensor past, Tensor(b!) out, int kv_heads, bool chan, int shortest, int longest) -> ()", &delta_scan);
   m.def("gated_rmsnorm(Tensor o, Tensor gate, Tensor w, float eps, int act, Tensor(a!) y, int H, int V) -> ()", &gated_rmsnorm);
   m.def("latent_gather(Tensor ring, Tensor cnew, Tensor ext_seq, Tensor ext_off, Tensor seq_off, Tensor slots, Tensor past, Tensor(a!) ext) -> ()", &latent_gather);
   m.def("latent_write(Tensor(a!) ring, Tensor cnew, Tensor tok_seq, Tensor seq_off, Tensor slots, Tensor past) -> ()", &latent_write);

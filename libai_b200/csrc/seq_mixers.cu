@@ -14,6 +14,8 @@
 #include <math.h>
 #include <stdint.h>
 
+typedef __nv_bfloat16 bf16;
+
 namespace {
 
 template <typename T> __device__ __forceinline__ float ldf(const T* p);
@@ -367,13 +369,14 @@ __global__ void __launch_bounds__(PAIR_THREADS)
 delta_scan_pair_kernel(const T* __restrict__ qkv, long ldq, int voff, const float* __restrict__ qn, const float* __restrict__ kn,
                        const float* __restrict__ kqs, const float* __restrict__ gs, const float* __restrict__ betas,
                        float* __restrict__ S, const int* __restrict__ seq_off, const int* __restrict__ slots,
-                       const int* __restrict__ past, float* __restrict__ out, int H, int KH, int D, int V) {
+                       const int* __restrict__ past, float* __restrict__ out, int H, int KH, int D, int V, int shorter_than) {
   constexpr int DP = 16 * D4, VB = 32 * CPT, BUF = pair_buffer_floats(DP, VB), VE = 16 / sizeof(T);
   extern __shared__ __align__(16) float sm[];
   float* scal = sm + 2 * BUF;
   const int tid = threadIdx.x, r = tid & 3, cg = tid >> 2, bit0 = r & 1;
   const int b = blockIdx.x / H, h = blockIdx.x % H, kh = h / (H / KH), j0 = blockIdx.y * VB;
   const int n = seq_off[b + 1] - seq_off[b];
+  if (n >= shorter_than) return;
   const long tok0 = seq_off[b];
   float* Sg = S + ((long)slots[b] * H + h) * (long)D * V;
   const int jc = j0 + cg * CPT;
@@ -549,6 +552,430 @@ delta_scan_pair_kernel(const T* __restrict__ qkv, long ldq, int voff, const floa
       }
     }
   }
+}
+
+// ------------------------------------------------------------------------------------------------------------------
+// The same recurrence for long bf16 sequences, CL tokens at a time on the tensor cores.  With G_t the product of the decays from the chunk's
+// start, γ(t, s) that of s+1 .. t and S0 the state before the chunk,
+//   u_t = β_t (v_t - G_t S0ᵀk_t - Σ_{s<t} γ(t, s) (k_t·k_s) u_s),   that is  U = T Y,  Y = V - G K S0,  T = (I + A)^-1 β,  A_ts = β_t γ(t, s) (k_t·k_s),
+//   o_t = G_t S0ᵀq_t + Σ_{s<=t} M_ts u_s,  M_ts = γ(t, s) (q_t·k_s),                        S <- G_L S0 + Σ_s γ(L, s) k_s u_sᵀ.
+// A first kernel makes T, M and the decays of all chunks at once, the second walks a sequence's chunks with the state.  There a warp owns 16 columns
+// of Sᵀ in registers (accumulator layout of m16n8k16, 16 x 128 fp32), everything is transposed ([16 columns, tokens]) and each result is the
+// next product's A operand, so warps share staged operands only and a chunk needs one barrier.
+// Nothing that was fp32 is rounded: q and k are the bf16 numbers as they came (their lengths go into fp32 factors per token), the state, Y, U, T and M
+// are sums of three bf16 parts (24 bits), so all products are exact; the tensor core adds up the 16 products of one step and its parts, steps are
+// added in fp32 registers with rounding to nearest (the tensor core's accumulator cuts off).  Decays are products in token order as in
+// the scan (no logarithms).  T and M end at the diagonal: 0 times what is not finite would reach earlier tokens of the column, so columns
+// with such numbers (or beyond 1e37) take these two products from plain sums over s <= t.
+// The scan in pairs is a chain of 1150 cycles per two tokens on one warp per scheduler; here a warp's chunk is 360 products
+// (192 with the state, 36 + 36 with T and M, 96 for the update), 16 cycles each on its scheduler's tensor core: 7300 cycles per 32 tokens, and
+// a sequence's chunks are a chain.  [2560 tokens of 4 sequences up to 1024, 16 heads, 128 x 128]: 334 -> 143 us with the preparations (16); eight sequences
+// of 1024: 680 -> 233.  Relative error of the read-outs against 64 bits 1.2e-7 to 1.5e-7 (pairs
+// 1.1e-7 to 1.4e-7), 1.2e-6 to 2.5e-6 for decays near one (pairs 0.7e-6 to 2.5e-6).  The same in fp32 on the FMA pipe (the inverse times
+// keys and values ahead of the scan, 4 x 4 tiles) took 333: 16-byte reads of shared memory bound it.
+// ------------------------------------------------------------------------------------------------------------------
+constexpr int CL = 32;                       // tokens per chunk
+// Sequences from here on are scanned in chunks: one of 64 tokens takes 22 us both ways, eight of 64 29 against 41, one of 128 30 against 41,
+// eight of 256 64 against 134 (16 heads of 128 x 128).
+constexpr int CL_MIN = 64;
+constexpr int CL_LD = CL + 8;                // row stride of 32 x 32 bf16 matrices in shared memory (ldmatrix without bank conflicts)
+constexpr int CL_WARPS = 4;                  // warps (of 16 columns) per block of the scan
+constexpr int CL_COLS = 16 * CL_WARPS;
+// scratch per (chunk, head), in floats: T and M as three bf16 parts each, then per token the factors of K S0, Q S0 and of u in the update, then G_L
+constexpr int CL_SCRATCH = 3 * CL * CL + 3 * CL + 32;
+
+__device__ __forceinline__ uint32_t smem_at(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t at) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at));
+}
+__device__ __forceinline__ void ldsm4_trans(uint32_t (&r)[4], uint32_t at) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at));
+}
+__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// (x, y) as the sum of three pairs of bf16 numbers, largest first
+__device__ __forceinline__ void parts3(float x, float y, uint32_t (&p)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const __nv_bfloat162 r = __floats2bfloat162_rn(x, y);
+    p[i] = *reinterpret_cast<const uint32_t*>(&r);
+    x -= __uint_as_float(p[i] << 16);
+    y -= __uint_as_float(p[i] & 0xffff0000u);
+  }
+}
+// A operand of 16 rows and the 16 columns of two neighbouring accumulator tiles, in three parts
+__device__ __forceinline__ void a_parts(const float (&l)[4], const float (&r)[4], uint32_t (&a)[3][4]) {
+  uint32_t p[3];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float x = i < 2 ? l[2 * (i & 1)] : r[2 * (i & 1)], y = i < 2 ? l[2 * (i & 1) + 1] : r[2 * (i & 1) + 1];
+    parts3(x, y, p);
+#pragma unroll
+    for (int e = 0; e < 3; ++e) a[e][i] = p[e];
+  }
+}
+
+// block = (chunk, key head); heads of a group by warps in turn
+template <int DP>
+__global__ void __launch_bounds__(128)
+delta_chunk_prep_kernel(const bf16* __restrict__ qkv, long ldq, int koff, const bf16* __restrict__ a, long lda, const bf16* __restrict__ bl, long ldb,
+                        const bf16* __restrict__ A_log, const bf16* __restrict__ dt_bias, const int* __restrict__ seq_off, float* __restrict__ scratch,
+                        int B, int H, int KH, int D) {
+  constexpr int LD = DP + 8;
+  __shared__ __align__(16) bf16 sK[CL * LD], sQ[CL * LD];
+  __shared__ float sKK[CL][CL + 1], sQK[CL][CL + 1], sA[4][CL][CL + 4];
+  __shared__ float ksc[CL], qsc[CL];
+  __shared__ int where[2];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, kh = blockIdx.y;
+  if (warp == 0) {                           // the chunk's sequence
+    int left = blockIdx.x, found = -1;
+    for (int b0 = 0; b0 < B && found < 0; b0 += 32) {
+      const int b = b0 + lane, n = b < B ? seq_off[b + 1] - seq_off[b] : 0, c = n >= CL_MIN ? (n + CL - 1) / CL : 0;
+      int sum = c;
+#pragma unroll
+      for (int m = 1; m < 32; m <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, sum, m);
+        if (lane >= m) sum += x;
+      }
+      const unsigned hit = __ballot_sync(0xffffffffu, sum > left);
+      if (hit) {
+        const int at = __ffs(hit) - 1;
+        found = b0 + at;
+        left -= __shfl_sync(0xffffffffu, sum - c, at);
+      } else {
+        left -= __shfl_sync(0xffffffffu, sum, 31);
+      }
+    }
+    if (lane == 0) { where[0] = found; where[1] = left; }
+  }
+  __syncthreads();
+  const int b = where[0];
+  if (b < 0) return;
+  const long tok0 = seq_off[b] + (long)where[1] * CL;
+  const int nt = min(CL, (int)(seq_off[b + 1] - tok0));
+  for (int t = warp; t < CL; t += 4) {       // rows as they are, their lengths apart
+    float qq = 0.f, kk = 0.f;
+    const bf16 *qr = qkv + (tok0 + t) * ldq + (long)kh * D, *kr = qr + koff;
+    for (int i = lane * 4; i < DP; i += 128) {
+      uint2 x = make_uint2(0u, 0u), y = x;
+      if (t < nt && i < D) { x = *reinterpret_cast<const uint2*>(qr + i); y = *reinterpret_cast<const uint2*>(kr + i); }
+      *reinterpret_cast<uint2*>(sQ + t * LD + i) = x;
+      *reinterpret_cast<uint2*>(sK + t * LD + i) = y;
+      const uint32_t xs[2] = {x.x, x.y}, ys[2] = {y.x, y.y};
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const float x0 = __uint_as_float(xs[e] << 16), x1 = __uint_as_float(xs[e] & 0xffff0000u);
+        const float y0 = __uint_as_float(ys[e] << 16), y1 = __uint_as_float(ys[e] & 0xffff0000u);
+        qq += x0 * x0 + x1 * x1;
+        kk += y0 * y0 + y1 * y1;
+      }
+    }
+    qq = warp_sum(qq);
+    kk = warp_sum(kk);
+    if (lane == 0) {
+      qsc[t] = (1.f / sqrtf((float)D)) / sqrtf(qq + 1e-6f);
+      ksc[t] = 1.f / sqrtf(kk + 1e-6f);
+    }
+  }
+  __syncthreads();
+  {                                          // K Kᵀ (warps 0, 1) and Q Kᵀ (2, 3), 16 rows per warp
+    const bf16* rows = warp < 2 ? sK : sQ;
+    const int r0 = (warp & 1) * 16;
+    float c[4][4] = {};
+#pragma unroll
+    for (int k0 = 0; k0 < DP; k0 += 16) {
+      uint32_t am[4];
+      ldsm4(am, smem_at(rows + (r0 + (lane & 15)) * LD + k0 + (lane >> 4) * 8));
+#pragma unroll
+      for (int n2 = 0; n2 < 2; ++n2) {
+        uint32_t bm[4];
+        ldsm4(bm, smem_at(sK + (n2 * 16 + (lane & 7) + (lane >> 4) * 8) * LD + k0 + ((lane >> 3) & 1) * 8));
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          float x[4] = {};
+          mma16816(x, am, bm[2 * i], bm[2 * i + 1]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) c[n2 * 2 + i][e] += x[e];
+        }
+      }
+    }
+    float(*dst)[CL + 1] = warp < 2 ? sKK : sQK;
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) dst[r0 + (lane >> 2) + (e >> 1) * 8][n * 8 + (lane & 3) * 2 + (e & 1)] = c[n][e];
+  }
+  __syncthreads();
+  const int group = H / KH;
+  for (int hh = warp; hh < group; hh += 4) {
+    const int h = kh * group + hh;
+    float* mine = scratch + ((long)blockIdx.x * H + h) * CL_SCRATCH;
+    bf16* Tp = reinterpret_cast<bf16*>(mine);
+    bf16* Mp = Tp + 3 * CL * CL;
+    float* fac = mine + 3 * CL * CL;
+    float g = 1.f, beta = 0.f;               // of token `lane`
+    if (lane < nt) {
+      const float rate = expf(ldf(A_log + h));
+      g = expf(-rate * softplusf_(ldf(a + (tok0 + lane) * lda + h) + ldf(dt_bias + h)));
+      beta = sigmoidf_(ldf(bl + (tok0 + lane) * ldb + h));
+    }
+    float x = 0.f, all = 1.f, G = 1.f;       // γ(t, lane); products of all decays up to t
+    const float ks = ksc[lane];
+    auto store3 = [&](bf16* p, float v) {
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        const bf16 r = __float2bfloat16_rn(v);
+        p[e * CL * CL] = r;
+        v -= __bfloat162float(r);
+      }
+    };
+#pragma unroll 4
+    for (int t = 0; t < CL; ++t) {
+      const float gt = __shfl_sync(0xffffffffu, g, t), bt = __shfl_sync(0xffffffffu, beta, t);
+      x = t == lane ? 1.f : (t > lane ? x * gt : 0.f);
+      all *= gt;
+      if (t == lane) G = all;
+      sA[warp][t][lane] = lane < t ? bt * (x * (ksc[t] * ks * sKK[t][lane])) : 0.f;
+      store3(Mp + t * CL + lane, lane <= t ? x * (qsc[t] * ks * sQK[t][lane]) : 0.f);
+    }
+    fac[lane] = G * ks;
+    fac[CL + lane] = G * qsc[lane];
+    fac[2 * CL + lane] = x * ks;             // (tokens behind the end decay by 1)
+    if (lane == 0) fac[3 * CL] = all;
+    __syncwarp();
+    float col[CL];                           // column `lane` of (I + A)^-1
+#pragma unroll
+    for (int t = 0; t < CL; ++t) {
+      float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int s = 0; s < t; ++s) acc[s & 3] += sA[warp][t][s] * col[s];
+      col[t] = t == lane ? 1.f : (t > lane ? -((acc[0] + acc[1]) + (acc[2] + acc[3])) : 0.f);
+      store3(Tp + t * CL + lane, t >= lane ? col[t] * beta : 0.f);
+    }
+    __syncwarp();
+  }
+}
+
+template <int DP>
+struct DeltaChunkStage {
+  bf16 k[CL * (DP + 8)], q[CL * (DP + 8)];
+  bf16 tm[6 * CL * CL_LD];                   // T, M: three parts each
+  bf16 v[CL * (CL_COLS + 8)];
+  float fac[3 * CL + 4];
+};
+template <int DP>
+struct DeltaChunkSmem {
+  DeltaChunkStage<DP> st[2];
+  float slow[CL_WARPS][2][16][CL + 1];       // Y and U, O of columns with numbers that are not finite
+};
+
+// block = (sequence and head, CL_COLS columns)
+template <int DP>
+__global__ void __launch_bounds__(32 * CL_WARPS)
+delta_chunk_scan_kernel(const bf16* __restrict__ qkv, long ldq, int koff, int voff, const float* __restrict__ scratch, float* __restrict__ S,
+                        const int* __restrict__ seq_off, const int* __restrict__ slots, const int* __restrict__ past, float* __restrict__ out,
+                        int H, int KH, int D, int V) {
+  constexpr int LD = DP + 8, VLD = CL_COLS + 8, THREADS = 32 * CL_WARPS;
+  extern __shared__ __align__(16) unsigned char delta_sm[];
+  DeltaChunkSmem<DP>& sm = *reinterpret_cast<DeltaChunkSmem<DP>*>(delta_sm);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q2 = (lane & 3) * 2;
+  const int b = blockIdx.x / H, h = blockIdx.x % H, kh = h / (H / KH), j0 = blockIdx.y * CL_COLS;
+  const int n = seq_off[b + 1] - seq_off[b];
+  if (n < CL_MIN) return;
+  int before = 0;                            // chunks of the sequences before this one
+  for (int i = lane; i < b; i += 32) {
+    const int m = seq_off[i + 1] - seq_off[i];
+    before += m >= CL_MIN ? (m + CL - 1) / CL : 0;
+  }
+#pragma unroll
+  for (int m = 16; m > 0; m >>= 1) before += __shfl_xor_sync(0xffffffffu, before, m);
+  const long tok0 = seq_off[b];
+  const float* base = scratch + ((long)before * H + h) * CL_SCRATCH;
+  const long step = (long)H * CL_SCRATCH;
+  float* Sg = S + ((long)slots[b] * H + h) * (long)D * V;
+  const int jc = j0 + warp * 16 + g;         // this thread's columns: jc, jc + 8
+  float st[DP / 8][4];                       // Sᵀ: rows are columns of S; n-tile i, element e: row jc + 8 (e / 2), column 8 i + q2 + e % 2
+#pragma unroll
+  for (int i = 0; i < DP / 8; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int d = 8 * i + q2 + (e & 1), col = jc + 8 * (e >> 1);
+      st[i][e] = past[b] > 0 && d < D && col < V ? Sg[(long)d * V + col] : 0.f;
+    }
+  auto stage = [&](int c) {
+    DeltaChunkStage<DP>& p = sm.st[c & 1];
+    const int nt = min(CL, n - c * CL);
+    const long tok = tok0 + c * CL;
+    const float* w = base + c * step;
+    for (int e = tid; e < CL * DP / 8; e += THREADS) {
+      const int t = e / (DP / 8), i = e % (DP / 8) * 8;
+      const int bytes = t < nt ? max(0, min(8, D - i)) * 2 : 0;
+      const bf16* src = qkv + (bytes ? (tok + t) * ldq + (long)kh * D + i : 0);
+      cp_async16(p.q + t * LD + i, src, bytes);
+      cp_async16(p.k + t * LD + i, src + (bytes ? koff : 0), bytes);
+    }
+    for (int e = tid; e < 6 * CL * CL / 8; e += THREADS)
+      cp_async16(p.tm + e / (CL / 8) * CL_LD + e % (CL / 8) * 8, reinterpret_cast<const bf16*>(w) + e * 8, 16);
+    for (int e = tid; e < CL * CL_COLS / 8; e += THREADS) {
+      const int t = e / (CL_COLS / 8), j = e % (CL_COLS / 8) * 8;
+      const bool in = t < nt && j0 + j < V;
+      cp_async16(p.v + t * VLD + j, qkv + (in ? (tok + t) * ldq + voff + (long)h * V + j0 + j : 0), in ? 16 : 0);
+    }
+    if (tid < (3 * CL + 4) / 4) cp_async16(p.fac + 4 * tid, w + 3 * CL * CL + 4 * tid, 16);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  const int chunks = (n + CL - 1) / CL;
+  stage(0);
+  for (int c = 0; c < chunks; ++c) {
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();                         // the chunk is here, and nobody reads the other stage any more
+    if (c + 1 < chunks) stage(c + 1);
+    const DeltaChunkStage<DP>& p = sm.st[c & 1];
+    const int nt = min(CL, n - c * CL);
+    // ---- S0ᵀ [Kᵀ Qᵀ]: [16, 32 + 32]
+    float x[8][4] = {};
+#pragma unroll
+    for (int kk = 0; kk < DP / 16; ++kk) {
+      uint32_t am[3][4];
+      a_parts(st[2 * kk], st[2 * kk + 1], am);
+#pragma unroll
+      for (int n2 = 0; n2 < 4; ++n2) {
+        uint32_t bm[4];
+        ldsm4(bm, smem_at((n2 < 2 ? p.k : p.q) + ((n2 & 1) * 16 + (lane & 7) + (lane >> 4) * 8) * LD + kk * 16 + ((lane >> 3) & 1) * 8));
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          float y[4] = {};
+#pragma unroll
+          for (int e = 2; e >= 0; --e) mma16816(y, am[e], bm[2 * i], bm[2 * i + 1]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) x[n2 * 2 + i][e] += y[e];
+        }
+      }
+    }
+    // ---- Y = V - G K S0; O starts with G Q S0
+    bool odd[2] = {false, false};            // columns g, g + 8 with a number that is not finite or close to that
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int t = 8 * i + q2 + (e & 1);
+        x[i][e] = __bfloat162float(p.v[t * VLD + warp * 16 + g + 8 * (e >> 1)]) - p.fac[t] * x[i][e];
+        x[4 + i][e] *= p.fac[CL + t];
+        odd[e >> 1] = odd[e >> 1] || !(fabsf(x[i][e]) < 1e37f);
+      }
+    float u[4][4] = {};
+    {
+      // D += [16, 32] (as A, three parts) times the three parts of a lower triangular matrix at `tri`
+      auto times = [&](const float (*y)[4], const bf16* tri, float (&d)[4][4]) {
+#pragma unroll
+        for (int kk = 0; kk < 2; ++kk) {
+          uint32_t am[3][4];
+          a_parts(y[2 * kk], y[2 * kk + 1], am);
+#pragma unroll
+          for (int n2 = kk; n2 < 2; ++n2) {  // tokens 16 n2 .. + 15 from 16 kk .. + 15
+            uint32_t bm[3][4];
+#pragma unroll
+            for (int e = 0; e < 3; ++e)
+              ldsm4(bm[e], smem_at(tri + (e * CL + n2 * 16 + (lane & 7) + (lane >> 4) * 8) * CL_LD + kk * 16 + ((lane >> 3) & 1) * 8));
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {    // the smaller products first
+              float z[4] = {};
+              mma16816(z, am[2], bm[0][2 * i], bm[0][2 * i + 1]);
+              mma16816(z, am[1], bm[1][2 * i], bm[1][2 * i + 1]);
+              mma16816(z, am[0], bm[2][2 * i], bm[2][2 * i + 1]);
+              mma16816(z, am[1], bm[0][2 * i], bm[0][2 * i + 1]);
+              mma16816(z, am[0], bm[1][2 * i], bm[1][2 * i + 1]);
+              mma16816(z, am[0], bm[0][2 * i], bm[0][2 * i + 1]);
+#pragma unroll
+              for (int e = 0; e < 4; ++e) d[n2 * 2 + i][e] += z[e];
+            }
+          }
+        }
+      };
+      times(x, p.tm, u);
+      float o[4][4] = {};
+      times(u, p.tm + 3 * CL * CL_LD, o);
+      const unsigned any = __ballot_sync(0xffffffffu, odd[0] || odd[1]);
+      if (any == 0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) x[4 + i][e] += o[i][e];
+      } else {
+#pragma unroll
+        for (int r = 0; r < 2; ++r) odd[r] = (__ballot_sync(0xffffffffu, odd[r]) >> (lane & ~3) & 15u) != 0;
+        float(*ys)[CL + 1] = sm.slow[warp][0];
+        float(*us)[CL + 1] = sm.slow[warp][1];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) ys[g + 8 * (e >> 1)][8 * i + q2 + (e & 1)] = x[i][e];
+        __syncwarp();
+        for (int pass = 0; pass < 2; ++pass) {       // U from Y, then the rest of O (in Y's place) from U
+          const bf16* tri = p.tm + pass * 3 * CL * CL_LD;
+          for (int at = lane; at < 16 * CL; at += 32) {
+            const int col = at & 15, t = at / 16;
+            float sum = 0.f;
+            for (int s = 0; s <= t; ++s) {
+              const float m = (__bfloat162float(tri[(2 * CL + t) * CL_LD + s]) + __bfloat162float(tri[(CL + t) * CL_LD + s])) + __bfloat162float(tri[t * CL_LD + s]);
+              sum += m * (pass ? us[col][s] : ys[col][s]);
+            }
+            if (pass) ys[col][t] = sum; else us[col][t] = sum;
+          }
+          __syncwarp();
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int t = 8 * i + q2 + (e & 1), col = g + 8 * (e >> 1);
+            if (odd[e >> 1]) u[i][e] = us[col][t];
+            x[4 + i][e] += odd[e >> 1] ? ys[col][t] : o[i][e];
+          }
+        __syncwarp();
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int t = 8 * i + q2 + (e & 1), col = jc + 8 * (e >> 1);
+        if (t < nt && col < V) out[(tok0 + c * CL + t) * (long)(H * V) + (long)h * V + col] = x[4 + i][e];
+        u[i][e] = t < nt ? u[i][e] * p.fac[2 * CL + t] : 0.f;
+      }
+    // ---- Sᵀ <- G_L Sᵀ + Uᵀ K
+    const float gl = p.fac[3 * CL];
+    uint32_t am[2][3][4];
+#pragma unroll
+    for (int kk = 0; kk < 2; ++kk) a_parts(u[2 * kk], u[2 * kk + 1], am[kk]);
+#pragma unroll
+    for (int d2 = 0; d2 < DP / 16; ++d2) {
+      float y[2][4] = {};
+#pragma unroll
+      for (int kk = 0; kk < 2; ++kk) {
+        uint32_t bm[4];
+        ldsm4_trans(bm, smem_at(p.k + (kk * 16 + (lane & 15)) * LD + d2 * 16 + (lane >> 4) * 8));
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int e = 2; e >= 0; --e) mma16816(y[i], am[kk][e], bm[2 * i], bm[2 * i + 1]);
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) st[2 * d2 + i][e] = fmaf(gl, st[2 * d2 + i][e], y[i][e]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < DP / 8; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int d = 8 * i + q2 + (e & 1), col = jc + 8 * (e >> 1);
+      if (d < D && col < V) Sg[(long)d * V + col] = st[i][e];
+    }
 }
 
 // y[tok, h, :] = o / rms(o over V) * w * act(gate[tok, h, :]);  act 0: silu, 1: sigmoid.  One warp per (token, head).
@@ -950,7 +1377,6 @@ __global__ void head_gate_kernel(const float* __restrict__ x, const T* __restric
 
 inline int cdiv(long a, long b) { return (int)((a + b - 1) / b); }
 inline int ok() { return (int)cudaGetLastError(); }
-typedef __nv_bfloat16 bf16;
 
 }  // namespace
 
@@ -1019,12 +1445,42 @@ int lbs_short_conv(const void* in, long ldi, const void* w, void* tail, const in
   return ok();
 }
 
-// work: fp32 scratch of at least tokens * (2*KH*D + KH + H + (chan ? H*D : H)) floats
+// can bf16 sequences of these sizes be scanned in chunks?  (every row of q, k and v in whole aligned vectors)
+static bool delta_chunks_apply(long ldq, int koff, int voff, int H, int D, int V, int chan, int dtype) {
+  return dtype != 0 && !chan && D <= 128 && D % 4 == 0 && V % 8 == 0 && ldq % 8 == 0 && koff % 8 == 0 && voff % 8 == 0 && H <= 65535;
+}
+// fp32 scratch of lbs_delta_scan, in floats; longest: tokens of the longest sequence
+long lbs_delta_work(long tokens, int B, long ldq, int koff, int voff, int H, int KH, int D, int V, int chan, int dtype, long longest) {
+  const long prep = (tokens * (2L * KH * D + KH + H + (chan ? (long)H * D : (long)H)) + 3) / 4 * 4;
+  return prep + (longest >= CL_MIN && delta_chunks_apply(ldq, koff, voff, H, D, V, chan, dtype) ? (tokens / CL + B) * H * CL_SCRATCH : 0);
+}
+
+// work: lbs_delta_work(...) floats; shortest, longest: tokens of the shortest and the longest sequence
 int lbs_delta_scan(const void* qkv, long ldq, int koff, int voff, const void* a, long lda, const void* bl, long ldb, const void* A_log,
                    const void* dt_bias, float* S, const int* seq_off, const int* slots, const int* past, float* out, float* work,
-                   long tokens, int B, int H, int KH, int D, int V, int chan, int dtype, cudaStream_t s) {
+                   long tokens, int B, int H, int KH, int D, int V, int chan, int dtype, long shortest, long longest, cudaStream_t s) {
   if (B == 0 || tokens == 0) return 0;
   if (D > 256 || H % KH != 0) return -1;
+  // Long sequences in chunks, the others in pairs or token by token; which one depends on a sequence's own length only.
+  int shorter_than = 0x7fffffff;
+  if (longest >= CL_MIN && delta_chunks_apply(ldq, koff, voff, H, D, V, chan, dtype) && (reinterpret_cast<uintptr_t>(qkv) & 15) == 0 &&
+      (reinterpret_cast<uintptr_t>(work) & 15) == 0 && (D % 8 == 0 || KH == 1)) {
+    float* scratch = work + (tokens * (2L * KH * D + KH + 2L * H) + 3) / 4 * 4;
+    const dim3 pg((unsigned)(tokens / CL + B), (unsigned)KH), sg((unsigned)(B * H), (unsigned)((V + CL_COLS - 1) / CL_COLS));
+#define DCH(DP)                                                                                                                          \
+  {                                                                                                                                      \
+    const int smem = (int)sizeof(DeltaChunkSmem<DP>);                                                                                    \
+    const cudaError_t e = cudaFuncSetAttribute(delta_chunk_scan_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);          \
+    if (e != cudaSuccess) return (int)e;                                                                                                 \
+    delta_chunk_prep_kernel<DP><<<pg, 128, 0, s>>>((const bf16*)qkv, ldq, koff, (const bf16*)a, lda, (const bf16*)bl, ldb, (const bf16*)A_log, \
+                                                   (const bf16*)dt_bias, seq_off, scratch, B, H, KH, D);                                 \
+    delta_chunk_scan_kernel<DP><<<sg, 32 * CL_WARPS, smem, s>>>((const bf16*)qkv, ldq, koff, voff, scratch, S, seq_off, slots, past, out, H, KH, D, V); \
+  }
+    if (D <= 64) DCH(64) else DCH(128)
+#undef DCH
+    if (shortest >= CL_MIN) return ok();
+    shorter_than = CL_MIN;
+  }
   float* qn = work;
   float* kn = qn + tokens * KH * D;
   float* kq = kn + tokens * KH * D;
@@ -1042,7 +1498,7 @@ int lbs_delta_scan(const void* qkv, long ldq, int koff, int voff, const void* a,
     const dim3 pgrid((unsigned)(B * H), (unsigned)((V + 32 * cpt - 1) / (32 * cpt)));
 #define DSP(TT, D4, CPT)                                                                                                                \
   delta_scan_pair_kernel<TT, D4, CPT><<<pgrid, PAIR_THREADS, pair_smem_floats(16 * D4, 32 * CPT) * sizeof(float), s>>>(                 \
-      (const TT*)qkv, ldq, voff, qn, kn, kq, g, beta, S, seq_off, slots, past, out, H, KH, D, V)
+      (const TT*)qkv, ldq, voff, qn, kn, kq, g, beta, S, seq_off, slots, past, out, H, KH, D, V, shorter_than)
 #define DSP4(TT)                                          \
   {                                                       \
     if (D <= 64) { if (cpt == 2) DSP(TT, 4, 2); else DSP(TT, 4, 1); } \

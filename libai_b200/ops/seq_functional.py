@@ -103,7 +103,8 @@ def delta_scan(qkv, koff: int, voff: int, a, b, A_log, dt_bias, S, rb, kv_heads:
     out = torch.empty(qkv.shape[0], H * V, dtype=torch.float32, device=qkv.device)
     if _native(qkv):
         count_launch()
-        load_seq_ext().delta_scan(qkv, koff, voff, a, b, A_log, dt_bias, S, rb.seq_off, rb.slots, rb.past, out, kv_heads, chan)
+        load_seq_ext().delta_scan(qkv, koff, voff, a, b, A_log, dt_bias, S, rb.seq_off, rb.slots, rb.past, out, kv_heads, chan,
+                                  min(rb.lens), max(rb.lens))
         return out
     rep = H // kv_heads
     rate = torch.exp(A_log.float())

@@ -361,6 +361,85 @@ def test_delta_scan_two_tokens_at_a_time(lens, heads, kv, d, v, dtype):
         at += n
 
 
+def _delta64(qkv, a, b, rate, bias, S, lens, heads, kv, d, v):
+    """The recurrence token by token in float64: read-outs, final states."""
+    out, final, at = [], [], 0
+    for i, n in enumerate(lens):
+        rows, st = qkv[at:at + n].double(), S[i].double().clone()
+        q, k, val = rows[:, :kv * d].view(n, kv, d), rows[:, kv * d:2 * kv * d].view(n, kv, d), rows[:, 2 * kv * d:].view(n, heads, v)
+        unit = lambda t: (t / torch.sqrt(t.square().sum(-1, keepdim=True) + 1e-6)).repeat_interleave(heads // kv, 1)
+        q, k = unit(q) / math.sqrt(d), unit(k)
+        beta = torch.sigmoid(b[at:at + n].double())
+        g = torch.exp(-torch.exp(rate.double()) * torch.nn.functional.softplus(a[at:at + n].double() + bias.double(), threshold=300.0))
+        for t in range(n):
+            st = st * g[t][:, None, None]
+            st = st + k[t][:, :, None] * (beta[t][:, None] * (val[t] - torch.einsum("hdv,hd->hv", st, k[t])))[:, None, :]
+            out.append(torch.einsum("hdv,hd->hv", st, q[t]).reshape(-1))
+        final.append(st)
+        at += n
+    return torch.stack(out), torch.stack(final)
+
+
+@pytest.mark.parametrize("shift", [-8.0, 0.0, 6.0])
+@pytest.mark.parametrize("lens,heads,kv,d,v", [([64], 1, 1, 8, 8), ([65, 3, 97], 2, 1, 64, 64), ([96, 33, 128], 6, 3, 104, 136), ([200, 64], 4, 2, 128, 72),
+                                               ([70], 2, 1, 12, 16), ([95, 63, 64], 16, 8, 128, 128)])
+def test_delta_scan_in_chunks(lens, heads, kv, d, v, shift):
+    """Sequences on both sides of the line between chunks and pairs in one batch, last chunks of every kind, columns and rows short of
+    the tiles, states carried over in slots of another order; decays near one, ordinary and near zero."""
+    from libai_b200.inference.ragged import RaggedBatch
+    from libai_b200.ops import seq_functional as SF
+
+    n = sum(lens)
+    qkv, a, b = _rand((n, 2 * kv * d + heads * v), 1), (_rand((n, heads), 2).float() + shift).to(BF16), _rand((n, heads), 3)
+    rate, bias = _rand((heads,), 4, 0.5), _rand((heads,), 5, 0.5)
+    slots, past = list(range(len(lens)))[::-1], [7 * (i % 2) for i in range(len(lens))]
+    S = _rand((len(lens), heads, d, v), 6, 1.0, torch.float32)
+    start = torch.stack([S[s] * (p > 0) for s, p in zip(slots, past)])
+    want, final = _delta64(qkv, a, b, rate, bias, start, lens, heads, kv, d, v)
+    rb = RaggedBatch(lens, slots, past, "cuda")
+    run = lambda st: SF.delta_scan(qkv, kv * d, 2 * kv * d, a, b, rate, bias, st, rb, kv, False)
+    first = S.clone()
+    out = run(first)
+    # all numbers are fp32 sums: 2^-24 per step of a product of `d` and of a chain whose links contract (decays near one keep every link's)
+    assert float((out.double() - want).norm() / want.norm()) < 2.0 ** -24 * (32 + (max(lens) if shift < 0 else 0))
+    assert float((first[slots].double() - final).norm() / final.norm()) < 2.0 ** -24 * (32 + (max(lens) if shift < 0 else 0))
+    second = S.clone()
+    assert torch.equal(run(second), out) and torch.equal(first, second)
+    for i, m in enumerate(lens):                              # a sequence alone gives the same bits
+        lo = sum(lens[:i])
+        st, alone = S.clone(), RaggedBatch([m], [slots[i]], [past[i]], "cuda")
+        rows = slice(lo, lo + m)
+        y = SF.delta_scan(qkv[rows], kv * d, 2 * kv * d, a[rows], b[rows], rate, bias, st, alone, kv, False)
+        assert torch.equal(y, out[rows]) and torch.equal(st[slots[i]], first[slots[i]])
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan"), 3e38])
+def test_delta_scan_in_chunks_value_that_is_not_finite(value):
+    """It reaches no earlier token, no other column and no other head."""
+    from libai_b200.inference.ragged import RaggedBatch
+    from libai_b200.ops import seq_functional as SF
+
+    heads, kv, d, v, n, at = 2, 1, 64, 72, 100, 75
+    qkv, a, b = _rand((n, 2 * kv * d + heads * v), 1), _rand((n, heads), 2), _rand((n, heads), 3)
+    rate, bias, rb = _rand((heads,), 4, 0.5), _rand((heads,), 5, 0.5), RaggedBatch([n], [0], [0], "cuda")
+
+    def run(x):
+        S = torch.zeros(1, heads, d, v, device="cuda")
+        return SF.delta_scan(x, kv * d, 2 * kv * d, a, b, rate, bias, S, rb, kv, False).view(n, heads, v), S[0]
+
+    out, S = run(qkv)
+    x = qkv.clone()
+    x[at, 2 * kv * d + v + 5] = value                         # head 1, column 5
+    got, T = run(x)
+    other = torch.ones(heads, v, dtype=torch.bool, device="cuda")
+    other[1, 5] = False
+    assert torch.equal(got[:, other], out[:, other]) and torch.equal(T.transpose(1, 2)[other], S.transpose(1, 2)[other])
+    # earlier tokens of the chunk take these sums in another order
+    near = (got[:at, 1, 5] - out[:at, 1, 5]).abs().max()
+    assert float(near) < 2.0 ** -20 * float(out[:at, 1].abs().max()) and torch.equal(got[:64, 1, 5], out[:64, 1, 5])
+    assert not torch.isfinite(got[at:, 1, 5]).all() if value != 3e38 else torch.isfinite(got[at, 1, 5])
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, BF16])
 @pytest.mark.parametrize("n", [1, 17])
 def test_delta_scan_value_that_is_not_finite(n, dtype):
