@@ -413,6 +413,47 @@ def test_delta_scan_in_chunks(lens, heads, kv, d, v, shift):
         assert torch.equal(y, out[rows]) and torch.equal(st[slots[i]], first[slots[i]])
 
 
+@pytest.mark.parametrize("taps", [2, 3, 4])
+@pytest.mark.parametrize("lens", [[173], [1, 2, 3, 4, 5, 1, 1, 160], [4, 4, 8, 130, 6, 7]])
+def test_short_convolution_in_strips(lens, taps):
+    """Many tokens: sequences that begin anywhere in a strip, shorter than the taps, with and without a past; the new tails."""
+    from libai_b200.inference.ragged import RaggedBatch
+    from libai_b200.ops import seq_functional as SF
+
+    C, n, past = 8200, sum(lens), [5 * (i % 2) for i in range(len(lens))]
+    x, w, tail = _rand((n, C + 8), 1)[:, :C], _rand((C, taps), 2), _rand((len(lens), taps - 1, C), 3)
+    slots = list(range(len(lens)))[::-1]
+    new, out = tail.clone(), torch.empty(n, C, device="cuda", dtype=BF16)
+    SF.short_conv(x, w, new, RaggedBatch(lens, slots, past, "cuda"), out)
+    at = 0
+    for m, slot, p in zip(lens, slots, past):
+        rows = torch.cat([tail[slot].double() * (p > 0), x[at:at + m].double()])
+        z = sum(rows[j:j + m] * w[:, j].double() for j in range(taps))
+        size = sum((rows[j:j + m] * w[:, j].double()).abs() for j in range(taps))
+        want = z * torch.sigmoid(z)
+        # fp32 sums of `taps` products, a slope of at most 1.1, one rounding to bf16
+        assert bool(((out[at:at + m].double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -21 * size).all())
+        assert torch.equal(new[slot].double(), rows[m:])
+        at += m
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, BF16])
+@pytest.mark.parametrize("tokens,heads,v,pad", [(1, 1, 4, 0), (37, 3, 72, 0), (200, 16, 128, 4), (5, 2, 132, 0), (3, 2, 500, 4), (9, 2, 512, 0), (9, 2, 516, 0), (9, 3, 64, 1)])
+@pytest.mark.parametrize("act", [0, 1])
+def test_gated_norm_of_read_outs(tokens, heads, v, pad, act, dtype):
+    """Widths around the vectors of a warp, rows on and off their alignment, both gates."""
+    from libai_b200.ops import seq_functional as SF
+
+    n = heads * v
+    o, gate, w, y = _rand((tokens, n), 1, 2.0, torch.float32), _rand((tokens, n + pad), 2, 1.0, dtype)[:, :n], _rand((v,), 3, 1.0, dtype), torch.empty(tokens, n + pad, device="cuda", dtype=dtype)[:, :n]
+    SF.gated_rmsnorm(o, gate, w, 1e-6, act, y, heads, v)
+    x, g = o.double().view(tokens, heads, v), gate.double().view(tokens, heads, v)
+    want = x * torch.rsqrt(x.square().mean(-1, keepdim=True) + 1e-6) * w.double() * torch.sigmoid(g) * (g if act == 0 else 1.0)
+    got = y.double().view(tokens, heads, v)
+    # a dozen fp32 roundings and a sum of v squares, then one rounding to the type
+    assert bool(((got - want).abs() <= (2.0 ** -20 + (2.0 ** -8 if dtype == BF16 else 0.0)) * want.abs() + 1e-30).all())
+
+
 @pytest.mark.parametrize("value", [float("inf"), float("nan"), 3e38])
 def test_delta_scan_in_chunks_value_that_is_not_finite(value):
     """It reaches no earlier token, no other column and no other head."""
