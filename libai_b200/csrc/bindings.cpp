@@ -52,6 +52,7 @@ int lb_ce_bwd(const void* logits, const int64_t* labels, const float* lse, const
 int lb_adamw(float* master, const float* grad, float* m, float* v, void* lp_out, const float* scale, long n, float lr,
              float b1, float b2, float eps, float wd, float bc1, float bc2, int decoupled, cudaStream_t s);
 int lb_sqnorm(const float* x, float* out, long n, cudaStream_t s);
+int lb_clip_coef(const float* sq, float grad_scale, float max_norm, float* out, cudaStream_t s);
 int lb_gemm_bf16_comm(const void* a, const void* b, void* out, int M, int N, int K, int layout, int epi,
                       const void* bias, int act, void* pre_out, const void* pre_in, float* colsum, int mode,
                       int world, int rank, const long* peer_buf, const long* peer_flags, const long* peer_done,
@@ -656,6 +657,21 @@ Tensor sqnorm(const Tensor& x) {
   c10::cuda::CUDAGuard guard(x.device());
   Tensor out = at::zeros({1}, x.options().dtype(at::kFloat));
   check(lb_sqnorm(x.data_ptr<float>(), out.data_ptr<float>(), x.numel(), cur_stream()), "sqnorm");
+  return out;
+}
+
+// out[0] += sum x^2
+void sqnorm_add(const Tensor& x, Tensor out) {
+  c10::cuda::CUDAGuard guard(x.device());
+  TORCH_CHECK(out.is_cuda() && out.device() == x.device() && out.scalar_type() == at::kFloat && out.numel() == 1, "sqnorm_add: out must be one fp32 number");
+  check(lb_sqnorm(x.data_ptr<float>(), out.data_ptr<float>(), x.numel(), cur_stream()), "sqnorm");
+}
+// {norm, clip coefficient} from a sum of squares
+Tensor clip_coef(const Tensor& sq, double grad_scale, double max_norm) {
+  c10::cuda::CUDAGuard guard(sq.device());
+  TORCH_CHECK(sq.is_cuda() && sq.scalar_type() == at::kFloat && sq.numel() == 1, "clip_coef: one fp32 number");
+  Tensor out = at::empty({2}, sq.options());
+  check(lb_clip_coef(sq.data_ptr<float>(), (float)grad_scale, (float)max_norm, out.data_ptr<float>(), cur_stream()), "clip_coef");
   return out;
 }
 
@@ -1271,6 +1287,8 @@ TORCH_LIBRARY(libai_b200, m) {
   m.def("ce_bwd(Tensor(a!) logits, Tensor labels, Tensor lse, Tensor gloss, int vocab_start) -> Tensor(a!)", &ce_bwd);
   m.def("fused_adamw(Tensor(a!) master, Tensor grad, Tensor(b!) m, Tensor(c!) v, Tensor? lp_out, Tensor scale, float lr, float b1, float b2, float eps, float wd, float bc1, float bc2, bool decoupled) -> ()", &fused_adamw);
   m.def("sqnorm(Tensor x) -> Tensor", &sqnorm);
+  m.def("sqnorm_add(Tensor x, Tensor(a!) out) -> ()", &sqnorm_add);
+  m.def("clip_coef(Tensor sq, float grad_scale, float max_norm) -> Tensor", &clip_coef);
   m.def("attn_mask_pack(Tensor mask, bool causal) -> (Tensor, Tensor)", &attn_mask_pack);
   m.def("attn_split_fwd(Tensor q, Tensor k, Tensor v, bool causal, float scale, Tensor? words, Tensor? fill, bool train) -> (Tensor, Tensor, Tensor)", &attn_split_fwd);
   m.def("attn_split_bwd(Tensor dout, Tensor q, Tensor k, Tensor v, Tensor o32, Tensor lse, Tensor(a!) dq, Tensor(b!) dk, Tensor(c!) dv, bool causal, float scale, Tensor? words, Tensor? fill) -> ()", &attn_split_bwd);

@@ -382,17 +382,21 @@ class FlatOptimizer(torch.optim.Optimizer):
         self._synced = True
 
     # ------------------------------------------------------------------ clipping
-    def _global_grad_norm(self, norm_type: float) -> torch.Tensor:
-        """Norm over *all* parameters of the model-parallel group (each logical element once)."""
+    def _global_grad_norm(self, norm_type: float, squared: bool = False) -> torch.Tensor:
+        """Norm over *all* parameters of the model-parallel group (each logical element once); ``squared``: for the 2-norm the
+        sum of squares, before ``grad_scale``."""
         topo = dutil.get_dist_util()
         dev = None
         total = None
+        def _one_pass(seg):
+            return (seg.numel() and seg.dtype == torch.float32 and seg.is_contiguous() and seg.data_ptr() % 16 == 0
+                    and use_native(seg))
+
         def _acc(seg):
             if math.isinf(norm_type):
                 return seg.abs().max() if seg.numel() else torch.zeros((), device=seg.device)
             if norm_type == 2.0:
-                if (seg.numel() and seg.dtype == torch.float32 and seg.is_contiguous() and seg.data_ptr() % 16 == 0
-                        and use_native(seg)):
+                if _one_pass(seg):
                     # one pass over the flat fp32 gradient buffer (K19); `pow(2).sum()` would write and re-read a
                     # temporary as large as the buffer (1.4 GB for the 345M-parameter benchmark model)
                     count_launch()
@@ -423,7 +427,12 @@ class FlatOptimizer(torch.optim.Optimizer):
                         acc = torch.maximum(acc, _acc(view(cur, lo)))
                     cur = max(cur, hi)
             else:
-                acc = _acc(fg.grad_shard())
+                shard = fg.grad_shard()
+                if norm_type == 2.0 and not skip and total is not None and total.device == shard.device and _one_pass(shard):
+                    count_launch()
+                    load_ext().sqnorm_add(shard, total)       # `total` is this call's own number
+                    continue
+                acc = _acc(shard)
                 if skip:
                     # ONE reduction over the packed duplicates (≈150 LayerNorm / bias segments under tensor parallelism:
                     # one kernel per segment made the step host-bound on tp_rank != 0)
@@ -447,6 +456,8 @@ class FlatOptimizer(torch.optim.Optimizer):
                 dist.all_reduce(total, op=op, group=topo.tp_group)
             if topo.pp_group is not None:
                 dist.all_reduce(total, op=op, group=topo.pp_group)
+        if squared:
+            return total
         if not math.isinf(norm_type):
             total = total.pow(1.0 / norm_type)
         return total * self.grad_scale
@@ -460,7 +471,16 @@ class FlatOptimizer(torch.optim.Optimizer):
             self._clip_coef = None
             return None
         max_norm = float(g0["clip_grad_max_norm"])
-        norm = self._global_grad_norm(float(g0["clip_grad_norm_type"]))
+        norm_type = float(g0["clip_grad_norm_type"])
+        if norm_type == 2.0 and not torch.is_tensor(self.grad_scale):
+            square = self._global_grad_norm(norm_type, squared=True)
+            if use_native(square) and square.dtype == torch.float32 and square.numel() == 1:
+                count_launch()               # square root, scale and coefficient in one kernel (seven single-number launches of PyTorch)
+                self.last_grad_norm, self._clip_coef = load_ext().clip_coef(square, float(self.grad_scale), max_norm).unbind()
+                return self.last_grad_norm
+            norm = square.sqrt() * self.grad_scale
+        else:
+            norm = self._global_grad_norm(norm_type)
         self.last_grad_norm = norm
         self._clip_coef = torch.clamp(max_norm / (norm + 1e-6), max=1.0)
         return norm
@@ -495,7 +515,9 @@ class FlatOptimizer(torch.optim.Optimizer):
             if fg is None:
                 continue
             g = self.param_groups[gi]
-            scale = coef * self.grad_scale if coef is not None else None
+            scale = coef
+            if coef is not None and (torch.is_tensor(self.grad_scale) or self.grad_scale != 1.0):
+                scale = coef * self.grad_scale
             if fg.symm is not None and hasattr(self, "_fused_zero_update"):
                 self._fused_zero_update(g, fg, self._step_count, scale)
                 continue

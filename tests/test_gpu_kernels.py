@@ -746,3 +746,26 @@ def test_block_in_one_call_leaves_everything_else_to_the_modules():
         graph.replay()
         assert torch.equal(y, base)
     assert m(x).requires_grad
+
+
+@pytest.mark.parametrize("scale", [1.0, 0.25])
+@pytest.mark.parametrize("size,poison", [(1e-3, None), (3.0, None), (3.0, float("nan")), (3.0, float("inf")), (0.0, None)])
+def test_gradient_norm_and_clip_coefficient_over_groups(size, poison, scale):
+    """One accumulator for all parameter groups, coefficient below and at one, what is not finite, a loss scale."""
+    from libai_b200.optim import AdamW, get_default_optimizer_params
+
+    m = torch.nn.Sequential(torch.nn.Linear(72, 40), torch.nn.LayerNorm(40), torch.nn.Linear(40, 8)).cuda().to(BF16)
+    opt = AdamW(get_default_optimizer_params(m, weight_decay_norm=0.0, weight_decay_bias=0.0, clip_grad_max_norm=1.0, clip_grad_norm_type=2.0), lr=1e-3)
+    opt.setup()
+    assert sum(g is not None for g in opt._groups) > 1
+    for i, p in enumerate(m.parameters()):
+        p.main_grad.copy_(_rand(p.shape, i, size, torch.float32))
+    if poison is not None:
+        next(m.parameters()).main_grad[3, 5] = poison
+    opt.grad_scale = scale
+    want = torch.sqrt(sum(p.main_grad.double().square().sum() for p in m.parameters())) * scale
+    norm = opt.clip_grad()
+    assert norm.dim() == 0 and norm.dtype == torch.float32 and opt._clip_coef.dim() == 0
+    coef = torch.clamp(1.0 / (want + 1e-6), max=1.0)
+    # sums of a few thousand squares in fp32 and a handful of roundings
+    assert torch.allclose(norm.double(), want, rtol=1e-5, equal_nan=True) and torch.allclose(opt._clip_coef.double(), coef, rtol=1e-5, equal_nan=True)
