@@ -15,7 +15,7 @@
 // next Q·Kᵀ into the same buffer, so scores are not overwritten before P has been read.  The last unit is as wide as its keys need
 // (multiples of 16).  Work items are pairs of query tiles, heaviest first within groups of heads whose keys and values stay in L2.
 //
-// [1, 8192, 16, 128] causal 334 -> 236 us, [1, 2048, 32, 128] 65 -> 42, [8, 1024, 16, 64] 55.6 -> 43.5, [64, 197, 16, 64] full 56.4 -> 41.7,
+// [1, 8192, 16, 128] causal 334 -> 236 us, [1, 2048, 32, 128] 65 -> 42, [8, 1024, 16, 64] 55.6 -> 46.5, [64, 197, 16, 64] full 56.4 -> 43.4,
 // [1, 8192, 16, 64] 295 -> 204.  What bounds it are the softmax warps, not the products (without those 6 to 14 % less): a unit takes its warp 1500 to
 // 1700 cycles, 850 to 1000 of them exponentials (512 of a warp alone), the rest waiting for the scores' barrier (120), reading them (65), the
 // maximum (340), storing P and handing it over (190), and two warps per scheduler do not fill each other's gaps.  Measured and not kept:
@@ -309,6 +309,31 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       // keys [0, key_lim) are visible to this row, [0, lim_lo) to all rows of this warp
       const int key_lim = p.causal ? min(w.kv_len, q_idx + 1) : w.kv_len, lim_lo = p.causal ? min(w.kv_len, q_warp + 1) : w.kv_len;
       float m_run = -INFINITY, l_run = 0.f;
+      // The first reference is the maximum of 128 keys: the largest probability is 1 and not rounded (with that of 64, results of 100 to 200 keys
+      // are 2 to 4 % further off; 1.7 us of [64, 197, 16, 64]).
+      if (n > 1) {
+        uint32_t x[4][32];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const uint32_t b = (sn + c / 2) & 1;
+          if (c % 2 == 0) {
+            ready(&s_full[t * 2 + b], ((sn + c / 2) >> 1) & 1);
+            __syncwarp();
+            tc_fence_after_sync();
+          }
+          tmem_ld_32x32b_x32(s_tile + b * 64 + c % 2 * 32, x[c]);
+        }
+        tmem_ld_wait();
+        float top[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        if (lim_lo >= 128) {
+#pragma unroll
+          for (int i = 0; i < 128; i += 2) top[(i >> 1) & 3] = max3(top[(i >> 1) & 3], __uint_as_float(x[i / 32][i % 32]), __uint_as_float(x[i / 32][i % 32 + 1]));
+        } else {
+#pragma unroll
+          for (int i = 0; i < 128; ++i) top[i & 3] = fmaxf(top[i & 3], i < key_lim ? __uint_as_float(x[i / 32][i % 32]) : -INFINITY);
+        }
+        m_run = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3])) * p.scale_log2;
+      }
       bool fine = true;
       for (int u = 0; u < n; ++u, ++sn) {
         fine = ready(&s_full[t * 2 + (sn & 1)], (sn >> 1) & 1);
