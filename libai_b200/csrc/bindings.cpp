@@ -1111,7 +1111,7 @@ std::vector<Tensor> llama_block_fwd(const Tensor& x, const std::vector<Tensor>& 
   joint = joint && p[5].data_ptr() == static_cast<char*>(p[4].data_ptr()) + p[4].nbytes() && p[4].storage().data() == p[5].storage().data();
   BlockScratch s;
   const int64_t norm = s.add(T * std::max(h, ad) * 2), wide = s.add(T * std::max(3 * ad, 2 * f) * 2), rot = s.add(T * std::max(3 * ad, f) * 2),
-                mid = s.add(T * h * 2), add = s.add(T * h * 2), stats = s.add(T * std::max<int64_t>(1, heads) * 4);
+                mid = s.add(T * h * 2), stats = s.add(T * std::max<int64_t>(1, heads) * 4);
   s.make(x);
   std::vector<Tensor> out{at::empty_like(x)};
   float* st = reinterpret_cast<float*>(s(stats));
@@ -1119,8 +1119,8 @@ std::vector<Tensor> llama_block_fwd(const Tensor& x, const std::vector<Tensor>& 
   block_linear(s(norm), p[1], bias.has_value() ? bias->data_ptr() : nullptr, 0, s(wide), T);
   check(lb_rope_qkv(s(wide), cosv.data_ptr<float>(), sinv.data_ptr<float>(), s(rot), T * heads, (int)S, (int)heads, (int)d, (int)at0, 0, cur_stream()), "rope_qkv");
   block_attention(s(rot), s(norm), st, B, S, heads, d, true, scale, past_k, past_v, out);
-  block_linear(s(norm), p[2], nullptr, 0, s(add), T);
-  check(lb_bias_residual(s(add), nullptr, x.data_ptr(), s(mid), T, (int)h, cur_stream()), "bias_residual");
+  check(lb_gemm_bf16_bias_residual(s(norm), p[2].data_ptr(), s(mid), (int)T, (int)h, (int)ad, (int)ad, (int)ad, nullptr, x.data_ptr(), cur_stream()),
+        "linear_bias_residual");
   check(lb_norm_fwd(s(mid), p[3].data_ptr(), nullptr, s(norm), nullptr, st, (int)T, (int)h, (float)eps2, 1, 0, 0, cur_stream()), "norm_fwd");
   if (joint) {
     check(lb_gemm_bf16(s(norm), p[4].data_ptr(), s(wide), (int)T, (int)(2 * f), (int)h, (int)h, (int)h, (int)(2 * f), 0, 0, nullptr, 0, nullptr, 0, 0, cur_stream()),
@@ -1132,8 +1132,8 @@ std::vector<Tensor> llama_block_fwd(const Tensor& x, const std::vector<Tensor>& 
     block_linear(s(norm), p[5], nullptr, 0, up, T);
     check(lb_swiglu_fwd(s(wide), up, s(rot), T * f, cur_stream()), "swiglu_fwd");
   }
-  block_linear(s(rot), p[6], nullptr, 0, s(add), T);
-  check(lb_bias_residual(s(add), nullptr, s(mid), out[0].data_ptr(), T, (int)h, cur_stream()), "bias_residual");
+  check(lb_gemm_bf16_bias_residual(s(rot), p[6].data_ptr(), out[0].data_ptr(), (int)T, (int)h, (int)f, (int)f, (int)f, nullptr, s(mid), cur_stream()),
+        "linear_bias_residual");
   return out;
 }
 

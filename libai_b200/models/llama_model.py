@@ -78,13 +78,15 @@ class LlamaMLP(nn.Module):
         self.down_proj = Linear(intermediate_size, hidden_size, bias=False, parallel="row",
                                 init_method=output_layer_init_method, layer_idx=layer_idx)
 
-    def forward(self, hidden_states):
-        y = self._forward_fused_gate_up(hidden_states)
+    def forward(self, hidden_states, residual=None):
+        """``residual`` (optional) is added to the result, in the down projection's epilogue where that is a kernel of its own."""
+        y = self._forward_fused_gate_up(hidden_states, residual)
         if y is not None:
             return y
-        return self.down_proj(OF.swiglu(self.gate_proj(hidden_states), self.up_proj(hidden_states)))
+        h = OF.swiglu(self.gate_proj(hidden_states), self.up_proj(hidden_states))
+        return self.down_proj(h) if residual is None else _plus_residual(self.down_proj, h, residual)
 
-    def _forward_fused_gate_up(self, x):
+    def _forward_fused_gate_up(self, x, residual=None):
         """Gate and up projection as ONE GEMM against the ``[2F, K]`` view over both weights (they are adjacent once the
         optimizer owns the parameters) — ``ops/gated_mlp.py``; ``None`` = not applicable, take the two-GEMM path."""
         from libai_b200.ops import gated_mlp, use_native
@@ -99,7 +101,9 @@ class LlamaMLP(nn.Module):
         topo = dutil.get_dist_util()
         t = topo.tensor_parallel_size
         if t == 1:
-            return gated_mlp.gated_mlp(x, wg, wu, wd)
+            fits = residual is None or (residual.dtype == torch.bfloat16 and residual.shape == x.shape and wd.shape[0] == x.shape[-1])
+            y = gated_mlp.gated_mlp(x, wg, wu, wd, residual if fits else None)
+            return y if fits else residual + y
         if not (topo.fused_tp_comm and topo.sequence_parallel and x.dim() == 2):
             return None
         from libai_b200.ops import comm_gemm
@@ -107,7 +111,17 @@ class LlamaMLP(nn.Module):
         M, K = x.shape[0] * t, x.shape[1]
         if not (comm_gemm.fused_supported(M, 2 * wg.shape[0], K, t) and comm_gemm.fused_supported(M, wd.shape[0], wg.shape[0], t)):
             return None
-        return gated_mlp.tp_gated_mlp(x.contiguous(), wg, wu, wd, None, topo.tp_group)
+        y = gated_mlp.tp_gated_mlp(x.contiguous(), wg, wu, wd, None, topo.tp_group)
+        return y if residual is None else residual + y
+
+
+def _plus_residual(proj, x, residual):
+    """``residual + proj(x)``; one kernel where ``proj`` is a plain linear layer of one tensor-parallel rank without a bias."""
+    w = proj._parameters.get("weight") if native.plain(proj, Linear) else None
+    if (w is not None and proj.bias is None and not proj.skip_bias_add and dutil.get_dist_util().tensor_parallel_size == 1 and x.dtype == torch.bfloat16
+            and residual.shape == (*x.shape[:-1], w.shape[0])):
+        return OF.linear_bias_residual(x, w, None, residual)
+    return residual + proj(x)
 
 
 class LlamaAttention(nn.Module):
@@ -129,7 +143,8 @@ class LlamaAttention(nn.Module):
                              init_method=output_layer_init_method, layer_idx=layer_idx)
 
     def forward(self, hidden_states, attention_mask=None, past_key_value=None, cos_cached=None, sin_cached=None,
-                use_cache=False):
+                use_cache=False, residual=None):
+        """``residual`` (optional) is added to the output projection's result."""
         sp = dutil.get_dist_util().sequence_parallel and hidden_states.dim() == 2
         a, d = self.local_heads, self.head_size
         bsz, tgt_len = get_sp_shape() if sp else hidden_states.shape[:2]
@@ -163,7 +178,7 @@ class LlamaAttention(nn.Module):
                 context = context.transpose(1, 2).reshape(bsz, -1, a * d)
         if sp:
             context = context.reshape(-1, a * d)
-        output = self.o_proj(context)
+        output = self.o_proj(context) if residual is None else _plus_residual(self.o_proj, context, residual)
         return (output, past_key_value) if use_cache else output
 
 
@@ -206,15 +221,27 @@ class LlamaDecoderLayer(nn.Module):
             done = self._native_forward(hidden_states, past_key_value, cos_cached, sin_cached, use_cache)
             if done is not None:
                 return done
-        attn = self.self_attn(self.input_layernorm(hidden_states), attention_mask=attention_mask,
-                              past_key_value=past_key_value, cos_cached=cos_cached, sin_cached=sin_cached,
-                              use_cache=use_cache)
+        ln, skip = self._norm(self.input_layernorm, hidden_states)
+        call = dict(attention_mask=attention_mask, past_key_value=past_key_value, cos_cached=cos_cached, sin_cached=sin_cached, use_cache=use_cache)
         presents = None
-        if use_cache:
-            attn, presents = attn
-        hidden_states = hidden_states + attn
-        output = hidden_states + self.mlp(self.post_attention_layernorm(hidden_states))
+        if native.plain(self.self_attn, LlamaAttention):
+            attn = self.self_attn(ln, residual=skip, **call)
+            hidden_states, presents = attn if use_cache else (attn, None)
+        else:
+            attn = self.self_attn(ln, **call)
+            if use_cache:
+                attn, presents = attn
+            hidden_states = skip + attn
+        ln, skip = self._norm(self.post_attention_layernorm, hidden_states)
+        output = self.mlp(ln, residual=skip) if native.plain(self.mlp, LlamaMLP) else skip + self.mlp(ln)
         return (output, presents) if use_cache else output
+
+    @staticmethod
+    def _norm(norm, x):
+        """``(norm(x), x)``; the skip connection's gradient joins inside the norm's backward kernel where ``norm`` is a plain one."""
+        if native.plain(norm, RMSLayerNorm) and not norm.zero_centered:
+            return OF.rms_norm_with_skip(x, norm.weight, norm.eps)
+        return norm(x), x
 
     def _native_forward(self, x, past, cos, sin, use_cache):
         """The block without a graph as one native call; ``None``: the modules have to run."""
@@ -239,7 +266,7 @@ class LlamaDecoderLayer(nn.Module):
         out = load_ext().llama_block_fwd(x, params, bias, cos, sin, attn.local_heads, ln1.eps, ln2.eps, attn.norm_factor, gated_mlp.enabled(), *pair)
         if not out:
             return None
-        count_launch(11)                # one more where gate and up projection are two products
+        count_launch(9)                 # one more where gate and up projection are two products
         return (out[0], tuple(out[1:])) if use_cache else out[0]
 
 

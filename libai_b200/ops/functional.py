@@ -399,6 +399,13 @@ def layer_norm(x, weight, bias, eps: float = 1e-5):
     return F.layer_norm(x.float(), (x.shape[-1],), w, b, eps).to(x.dtype)
 
 
+def rms_norm_with_skip(x, weight, eps: float = 1e-6):
+    """``(rms_norm(x), x)``; the gradient of the second output is added inside the norm's backward kernel (see ``_LayerNormFn``)."""
+    if use_native(x) and x.dtype in (torch.bfloat16, torch.float32) and x.requires_grad:
+        return _call(_LayerNormFn, x, weight, None, eps, True, True)
+    return rms_norm(x, weight, eps), x
+
+
 def rms_norm(x, weight, eps: float = 1e-6):
     if use_native(x) and x.dtype in (torch.bfloat16, torch.float32):
         return _call(_LayerNormFn, x, weight, None, eps, True)

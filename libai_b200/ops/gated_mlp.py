@@ -67,7 +67,7 @@ class GatedMLPFn(torch.autograd.Function):
     """Single-GPU / data-parallel form: ``y = (silu(x Wgᵀ) * (x Wuᵀ)) Wdᵀ`` with ``[Wg; Wu]`` as one GEMM operand."""
 
     @staticmethod
-    def forward(ctx, x, wg, wu, wd):
+    def forward(ctx, x, wg, wu, wd, residual=None):
         ext = load_ext()
         w, _ = fused_gate_up_views(wg, wu)
         x2 = x.reshape(-1, x.shape[-1])
@@ -75,10 +75,13 @@ class GatedMLPFn(torch.autograd.Function):
             x2 = x2.contiguous()
         gu = ext.gemm(x2, w, 0, None, None, False, torch.bfloat16)
         h = ext.swiglu_packed_fwd(gu)
-        y = ext.gemm(h, wd, 0, None, None, False, torch.bfloat16)
+        if residual is None:
+            y = ext.gemm(h, wd, 0, None, None, False, torch.bfloat16)
+        else:                                  # the residual add rides in the epilogue of the down projection
+            y = ext.linear_bias_residual(h, wd, None, residual.reshape(-1, wd.shape[0]).contiguous())
         count_launch(3)
         ctx.save_for_backward(x2, gu, h)
-        ctx.params = (wg, wu, wd)
+        ctx.params, ctx.has_res = (wg, wu, wd), residual is not None
         return y.view(*x.shape[:-1], wd.shape[0])
 
     @staticmethod
@@ -111,7 +114,7 @@ class GatedMLPFn(torch.autograd.Function):
                 gwg, gwu = _finish_wgrad(wg, wu, None, ext.gemm(dgu, x2, 2, None, None, False, torch.float32))
             count_launch()
         count_launch(3)
-        return gx, gwg, gwu, gwd
+        return gx, gwg, gwu, gwd, (gy if ctx.has_res else None)
 
 
 class TPGatedMLPFused(torch.autograd.Function):
@@ -159,8 +162,10 @@ class TPGatedMLPFused(torch.autograd.Function):
         return gx, gwg, gwu, gwd, (gy_shard if ctx.has_res else None), None
 
 
-def gated_mlp(x, wg, wu, wd):
-    return _call(GatedMLPFn, x, wg, wu, wd)
+def gated_mlp(x, wg, wu, wd, residual=None):
+    if residual is None:
+        return _call(GatedMLPFn, x, wg, wu, wd)
+    return _call(GatedMLPFn, x, wg, wu, wd, residual)
 
 
 def tp_gated_mlp(x_shard, wg, wu, wd, residual, group):

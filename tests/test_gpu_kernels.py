@@ -668,9 +668,9 @@ def _llama_block(heads, dim, joint):
 
 
 def _by_modules(m, call):
-    """The same call with a hook that has to see the MLP: the modules run one by one."""
+    """The same call with a hook that has to see a module (one without a residual of its own): the modules run one by one."""
     seen = []
-    handle = m.mlp.register_forward_hook(lambda *a: seen.append(1))
+    handle = (m.mlp if hasattr(m, "self_attention") else m.post_attention_layernorm).register_forward_hook(lambda *a: seen.append(1))
     out = call()
     handle.remove()
     assert seen
@@ -711,6 +711,28 @@ def test_llama_block_without_a_graph_in_one_call(b, s, heads, dim, past, joint):
             call = lambda: m(x, past_key_value=kv, cos_cached=cos, sin_cached=sin, use_cache=use_cache)
             for got, want in zip(_flat(call()), _flat(_by_modules(m, call))):
                 assert torch.equal(got, want) and got.stride() == want.stride() and not got.requires_grad
+
+
+@pytest.mark.parametrize("joint", [False, True])
+@pytest.mark.parametrize("b,s,heads,dim", [(1, 40, 4, 64), (2, 130, 2, 128)])
+def test_llama_block_residuals_in_the_epilogues(b, s, heads, dim, joint):
+    """Residual adds in the projections' epilogues and skip gradients in the norms' backward against additions of their own (hooks on
+    attention and MLP keep those)."""
+    m, (cos, sin) = _llama_block(heads, dim, joint), _ROT(256, dim)
+    x, gy = _rand((b, s, heads * dim), 1), _rand((b, s, heads * dim), 2)
+
+    def run():
+        xi = x.clone().requires_grad_(True)
+        y = m(xi, cos_cached=cos, sin_cached=sin)
+        return [y, *torch.autograd.grad(y, [xi, *m.parameters()], gy)]
+
+    got = run()
+    hooks = [k.register_forward_hook(lambda *a: None) for k in (m.self_attn, m.mlp, m.input_layernorm, m.post_attention_layernorm)]
+    for u, v in zip(got, run()):
+        # bf16 roundings of the sums (2^-8 each) that are not taken any more, through one block
+        assert u.shape == v.shape and float((u.detach().double() - v.detach().double()).norm()) < 2.0 ** -6 * float(v.detach().double().norm())
+    for h in hooks:
+        h.remove()
 
 
 def test_block_in_one_call_leaves_everything_else_to_the_modules():
