@@ -101,6 +101,7 @@ attn_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  chain_next();
 
   // phases are taken in order, so one that is there needs no look at *stop (30 cycles, up to six times per tile)
   auto ready = [&](uint64_t* bar, uint32_t parity) { return mbar_try_wait(bar, parity) || tc_wait(bar, parity, stop); };
@@ -342,6 +343,8 @@ __global__ void __launch_bounds__(256)
 attn_bwd128_stats_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ o, const float* __restrict__ lse,
                          float* __restrict__ stats, int A, int S, long bh_count, long sb, long sa, long ss, float scale,
                          float4* __restrict__ zero_fill, long zero_n4) {
+  chain_wait(dout, o, lse, zero_fill);
+  chain_next();
   const long gid = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x, threads = static_cast<long>(gridDim.x) * blockDim.x;
   for (long z = gid; z < zero_n4; z += threads) zero_fill[z] = make_float4(0.f, 0.f, 0.f, 0.f);
   const int nq = (S + 63) / 64, sub = threadIdx.x % 16;
@@ -401,7 +404,7 @@ extern "C" int lb_attn_bwd128(const void* dout, const void* q, const void* k, co
   const long rows = (long)B * A * ((S + 63) / 64) * 64;
   long blocks = (rows * 16 + 255) / 256;
   if (blocks > 148L * 16) blocks = 148L * 16;
-  lb::attn_bwd128_stats_kernel<<<(unsigned)blocks, 256, 0, s>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)o, lse, stats, A, S, (long)B * A, dos[0],
+  lb_host::launch_chained(lb::attn_bwd128_stats_kernel, dim3((unsigned)blocks), dim3(256), 0, s, 0, (const __nv_bfloat16*)dout, (const __nv_bfloat16*)o, lse, stats, A, S, (long)B * A, dos[0],
                                                                 dos[1], dos[2], scale, (float4*)dq_acc, (long)B * A * S * 32);
   lb::Bwd128Params p{};
   p.stats = stats;

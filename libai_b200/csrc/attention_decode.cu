@@ -59,6 +59,8 @@ attn_decode_kernel(const DecodeParams p) {
     const float2 a = unpack_bf16(w.x), b = unpack_bf16(w.y), c = unpack_bf16(w.z), e = unpack_bf16(w.w);
     v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = c.x; v[5] = c.y; v[6] = e.x; v[7] = e.y;
   };
+  chain_wait();
+  chain_next();
   float q[8];
   unpack8(col_ok ? *reinterpret_cast<const uint4*>(p.q + batch * p.q_st[0] + head * p.q_st[1] + sub * 8) : make_uint4(0, 0, 0, 0), q);
   const __nv_bfloat16* kp = p.k_past + batch * p.kp_st[0] + head * p.kp_st[1] + sub * 8;
@@ -175,18 +177,8 @@ attn_decode_kernel(const DecodeParams p) {
 
 template <int LPR>
 cudaError_t launch_attn_decode(const DecodeParams& p, int B, int cluster, cudaStream_t s) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)cluster, (unsigned)p.A, (unsigned)B);
-  cfg.blockDim = dim3(ADEC_THREADS);
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)cluster;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return p.mask != nullptr ? cudaLaunchKernelEx(&cfg, attn_decode_kernel<LPR, true>, p) : cudaLaunchKernelEx(&cfg, attn_decode_kernel<LPR, false>, p);
+  const dim3 grid((unsigned)cluster, (unsigned)p.A, (unsigned)B);
+  return lb_host::launch_chained(p.mask != nullptr ? attn_decode_kernel<LPR, true> : attn_decode_kernel<LPR, false>, grid, dim3(ADEC_THREADS), 0, s, (unsigned)cluster, p);
 }
 
 }  // namespace lb

@@ -166,6 +166,8 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  chain_wait();
+  chain_next();
   auto ready = [&](uint64_t* bar, uint32_t parity) { return mbar_try_wait(bar, parity) || tc_wait(bar, parity, stop); };
 
   if (warp_idx < 4) {
@@ -462,8 +464,7 @@ int launch_fwd_pair(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensor
     if (e != cudaSuccess) return (int)e;
     done.fetch_or(bit, std::memory_order_relaxed);
   }
-  kern<<<p.parts * p.BA, lb::FA_THREADS, lb::FaCfg<D>::SMEM, s>>>(tq, tk, tv, p);
-  return (int)cudaGetLastError();
+  return (int)lb_host::launch_chained(kern, dim3((unsigned)(p.parts * p.BA)), dim3(lb::FA_THREADS), lb::FaCfg<D>::SMEM, s, 0, tq, tk, tv, p);
 }
 }  // namespace
 

@@ -144,6 +144,8 @@ attn_fwd_v2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  chain_wait();
+  chain_next();
 
   if (warp_idx == 0) {
     if (elect_one()) {
@@ -450,8 +452,7 @@ cudaError_t launch_fwd_v2_t(const CUtensorMap& tq, const CUtensorMap& tk, const 
     configured = true;
   }
   dim3 grid((p.S + lb::ATT_BM - 1) / lb::ATT_BM, p.A, p.B);
-  kern<<<grid, lb::ATT_FWD2_THREADS, Cfg::SMEM_BYTES, s>>>(tq, tk, tv, p);
-  return cudaGetLastError();
+  return lb_host::launch_chained(kern, grid, dim3(lb::ATT_FWD2_THREADS), Cfg::SMEM_BYTES, s, 0, tq, tk, tv, p);
 }
 
 template <int D>
@@ -615,6 +616,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  chain_wait();
+  chain_next();
 
   if (warp_idx == 0) {
     if (elect_one()) {
@@ -1019,6 +1022,8 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  chain_wait();
+  chain_next();
   constexpr int CW0 = REGS ? 4 : 2;    // first softmax warp
   if constexpr (REGS) {
     if (warp_idx < CW0) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;\n");
@@ -1339,6 +1344,8 @@ template <int D>
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ o, float* __restrict__ delta,
                   int B, int A, int S, long sb, long sa, long ss, float4* __restrict__ zero_fill, long zero_n4) {
+  chain_wait(dout, o, zero_fill);
+  chain_next();
   constexpr int LPR = D / 8;  // lanes per row
   const long total = static_cast<long>(B) * A * S;
   const long gid = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
@@ -1379,6 +1386,8 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* _
 __global__ void __launch_bounds__(256)
 attn_dq_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, int B, int A, int S, int D, long sb,
                        long sa, long ss) {
+  chain_wait(acc);
+  chain_next();
   const long nvec = static_cast<long>(B) * A * S * D / 8;
   const long stride = static_cast<long>(gridDim.x) * blockDim.x;
   for (long i0 = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i0 < nvec; i0 += 2 * stride) {
@@ -1387,8 +1396,8 @@ attn_dq_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict_
     for (int u = 0; u < 2; ++u) {
       const long i = i0 + u * stride;
       if (i < nvec) {
-        lo[u] = reinterpret_cast<const float4*>(acc)[2 * i];
-        hi[u] = reinterpret_cast<const float4*>(acc)[2 * i + 1];
+        lo[u] = __ldg(reinterpret_cast<const float4*>(acc) + 2 * i);
+        hi[u] = __ldg(reinterpret_cast<const float4*>(acc) + 2 * i + 1);
       }
     }
 #pragma unroll
@@ -1422,8 +1431,7 @@ cudaError_t launch_bwd_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUt
     configured = true;
   }
   dim3 grid((p.S + 127) / 128, p.A, p.B);
-  kern<<<grid, lb::ATT_BWD_THREADS, Cfg::SMEM_BYTES, s>>>(tq, tk, tv, tdo, tdq, p);
-  return cudaGetLastError();
+  return lb_host::launch_chained(kern, grid, dim3(lb::ATT_BWD_THREADS), Cfg::SMEM_BYTES, s, 0, tq, tk, tv, tdo, tdq, p);
 }
 template <int BIAS, bool DROP, bool REGS>
 cudaError_t launch_bwd_pipe_r(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
@@ -1436,8 +1444,7 @@ cudaError_t launch_bwd_pipe_r(const CUtensorMap& tq, const CUtensorMap& tk, cons
     configured = true;
   }
   dim3 grid((p.S + 127) / 128, p.A, p.B);
-  kern<<<grid, lb::att_bwdp_threads<REGS>(), lb::ATT_BWDP_SMEM, s>>>(tq, tk, tv, tdo, tdq, p);
-  return cudaGetLastError();
+  return lb_host::launch_chained(kern, grid, dim3(lb::att_bwdp_threads<REGS>()), lb::ATT_BWDP_SMEM, s, 0, tq, tk, tv, tdo, tdq, p);
 }
 // LIBAI_B200_ATTN_BWD_PIPE: 0 = sequential kernel, 1 (default) = pipelined, 2 = pipelined + setmaxnreg (experimental:
 // the first version, 64/112 registers = the whole register file, never got its TRY_ALLOC granted and hung)
@@ -1483,7 +1490,7 @@ extern "C" int lb_attn_dq_convert(const float* acc, void* dq, int B, int A, int 
   const long nvec = (long)B * A * S * D / 8;
   int blocks = (int)((nvec + 511) / 512);
   if (blocks > 148 * 8) blocks = 148 * 8;
-  lb::attn_dq_convert_kernel<<<blocks, 256, 0, s>>>(acc, (__nv_bfloat16*)dq, B, A, S, D, st[0], st[1], st[2]);
+  lb_host::launch_chained(lb::attn_dq_convert_kernel, dim3(blocks), dim3(256), 0, s, 0, acc, (__nv_bfloat16*)dq, B, A, S, D, st[0], st[1], st[2]);
   return (int)cudaGetLastError();
 }
 
@@ -1525,11 +1532,11 @@ extern "C" int lb_attn_bwd(const void* dout, const void* q, const void* k, const
     long blocks = (groups * lpr + 255) / 256;
     if (blocks > 148L * 16) blocks = 148L * 16;
     if (D == 64)
-      lb::attn_delta_kernel<64><<<(unsigned)blocks, 256, 0, s>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)o, delta, B,
+      lb_host::launch_chained(lb::attn_delta_kernel<64>, dim3((unsigned)blocks), dim3(256), 0, s, 0, (const __nv_bfloat16*)dout, (const __nv_bfloat16*)o, delta, B,
                                                                    A, S, do_strides[0], do_strides[1], do_strides[2],
                                                                    reinterpret_cast<float4*>(dq_accum), rows * D / 4);
     else
-      lb::attn_delta_kernel<128><<<(unsigned)blocks, 256, 0, s>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)o, delta, B,
+      lb_host::launch_chained(lb::attn_delta_kernel<128>, dim3((unsigned)blocks), dim3(256), 0, s, 0, (const __nv_bfloat16*)dout, (const __nv_bfloat16*)o, delta, B,
                                                                     A, S, do_strides[0], do_strides[1], do_strides[2],
                                                                     reinterpret_cast<float4*>(dq_accum), rows * D / 4);
   }

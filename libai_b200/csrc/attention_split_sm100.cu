@@ -67,6 +67,8 @@ template <typename U>
 __global__ void __launch_bounds__(256)
 attn_mask_pack_kernel(const U* __restrict__ mask, unsigned long long and_mask, int Bm, int Am, int Sq, int Sk, long sb, long sa, long sq,
                       long sk, int causal, int off, uint32_t* __restrict__ words, float* __restrict__ fill, int pitch) {
+  chain_wait(mask);
+  chain_next();
   const long rows = static_cast<long>(Bm) * Am * Sq;
   const int lane = threadIdx.x % 32;
   const U keep_bits = static_cast<U>(and_mask);
@@ -142,6 +144,8 @@ attn_split_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  chain_wait();
+  chain_next();
 
   // The block's chain is serial whoever issues it (the other CTA of the SM fills its gaps), so a thread of the softmax warps does.  K(j+1) and
   // V(j+1) go where K(j-1) and V(j-1) were, and o_full(j-1) has said that nothing reads those any more.
@@ -406,6 +410,8 @@ attn_split_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  chain_wait();
+  chain_next();
 
   if (warp_idx == 0) {
     if (elect_one()) {
@@ -650,6 +656,8 @@ attn_split_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 __global__ void __launch_bounds__(256)
 attn_split_delta_kernel(const __nv_bfloat16* __restrict__ dout, long sb, long sa, long ss, const float* __restrict__ o32,
                         float* __restrict__ delta, int B, int A, int S, int d) {
+  chain_wait(dout, o32);
+  chain_next();
   const long total = static_cast<long>(B) * A * S;
   const long gid = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x, threads = static_cast<long>(gridDim.x) * blockDim.x;
   const int sub = threadIdx.x % 8;
@@ -676,6 +684,7 @@ attn_split_delta_kernel(const __nv_bfloat16* __restrict__ dout, long sb, long sa
 __global__ void __launch_bounds__(256)
 attn_split_dq_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, int B, int A, int S, int d, long sb, long sa, long ss,
                      int key_blocks, int causal, int off) {
+  chain_next();
   const long nvec = static_cast<long>(B) * A * S * d / 8;
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < nvec; i += static_cast<long>(gridDim.x) * blockDim.x) {
     const long row = i * 8 / d;
@@ -745,7 +754,7 @@ extern "C" int lb_attn_mask_pack(const void* mask, int elem, unsigned long long 
   const int pitch = (Sk + 127) / 128 * 4;
   long blocks = (rows + 7) / 8;
   if (blocks > 148L * 8) blocks = 148L * 8;
-#define LB_GO(U) lb::attn_mask_pack_kernel<U><<<(unsigned)blocks, 256, 0, s>>>((const U*)mask, and_mask, Bm, Am, Sq, Sk, strides[0], strides[1], strides[2], strides[3], causal, off, words, fill, pitch)
+#define LB_GO(U) lb_host::launch_chained(lb::attn_mask_pack_kernel<U>, dim3((unsigned)blocks), dim3(256), 0, s, 0, (const U*)mask, and_mask, Bm, Am, Sq, Sk, strides[0], strides[1], strides[2], strides[3], causal, off, words, fill, pitch)
   if (elem == 1) LB_GO(uint8_t);
   else if (elem == 2) LB_GO(uint16_t);
   else if (elem == 4) LB_GO(uint32_t);
@@ -768,9 +777,8 @@ extern "C" int lb_attn_split_fwd(const void* q, const void* k, const void* v, vo
   const dim3 grid((Sq + 127) / 128, A, B);
   cudaError_t e = mask ? split_configure(lb::attn_split_fwd_kernel<true>, lb::SPL_FWD_SMEM, c1) : split_configure(lb::attn_split_fwd_kernel<false>, lb::SPL_FWD_SMEM, c0);
   if (e != cudaSuccess) return (int)e;
-  if (mask) lb::attn_split_fwd_kernel<true><<<grid, lb::SPL_FWD_THREADS, lb::SPL_FWD_SMEM, s>>>(tq, tk, tv, p);
-  else lb::attn_split_fwd_kernel<false><<<grid, lb::SPL_FWD_THREADS, lb::SPL_FWD_SMEM, s>>>(tq, tk, tv, p);
-  return (int)cudaGetLastError();
+  return (int)lb_host::launch_chained(mask ? lb::attn_split_fwd_kernel<true> : lb::attn_split_fwd_kernel<false>, grid, dim3(lb::SPL_FWD_THREADS), lb::SPL_FWD_SMEM, s, 0,
+                                      tq, tk, tv, p);
 }
 
 // dq / dk / dv: [B, A, S, d] views; delta fp32 [B, A, Sq] and dq_acc fp32 [ceil(Sk / 128), B, A, Sq, d] are scratch
@@ -797,7 +805,7 @@ extern "C" int lb_attn_split_bwd(const void* dout, const void* q, const void* k,
   const long rows = (long)B * A * Sq;
   long blocks = (rows * 8 + 255) / 256;
   if (blocks > 148L * 16) blocks = 148L * 16;
-  lb::attn_split_delta_kernel<<<(unsigned)blocks, 256, 0, s>>>((const __nv_bfloat16*)dout, dos[0], dos[1], dos[2], o32, delta, B, A, Sq, d);
+  lb_host::launch_chained(lb::attn_split_delta_kernel, dim3((unsigned)blocks), dim3(256), 0, s, 0, (const __nv_bfloat16*)dout, dos[0], dos[1], dos[2], o32, delta, B, A, Sq, d);
   lb::SplitParams p = split_params(B, A, Sq, Sk, d, causal, scale, mask, fill, mask_b, mask_a, err);
   p.lse = const_cast<float*>(lse);
   p.delta = delta;
@@ -807,13 +815,13 @@ extern "C" int lb_attn_split_bwd(const void* dout, const void* q, const void* k,
   const dim3 grid(key_blocks, A, B);
   cudaError_t e = mask ? split_configure(lb::attn_split_bwd_kernel<true>, lb::SPL_BWD_SMEM, c1) : split_configure(lb::attn_split_bwd_kernel<false>, lb::SPL_BWD_SMEM, c0);
   if (e != cudaSuccess) return (int)e;
-  if (mask) lb::attn_split_bwd_kernel<true><<<grid, lb::SPL_THREADS, lb::SPL_BWD_SMEM, s>>>(tq, tk, tv, tdo, tdq, p);
-  else lb::attn_split_bwd_kernel<false><<<grid, lb::SPL_THREADS, lb::SPL_BWD_SMEM, s>>>(tq, tk, tv, tdo, tdq, p);
+  lb_host::launch_chained(mask ? lb::attn_split_bwd_kernel<true> : lb::attn_split_bwd_kernel<false>, grid, dim3(lb::SPL_THREADS), lb::SPL_BWD_SMEM, s, 0, tq, tk, tv, tdo,
+                          tdq, p);
   e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
   blocks = (rows * d / 8 + 255) / 256;
   if (blocks > 148L * 8) blocks = 148L * 8;
-  lb::attn_split_dq_kernel<<<(unsigned)blocks, 256, 0, s>>>(dq_acc, (__nv_bfloat16*)dq, B, A, Sq, d, dqs[0], dqs[1], dqs[2], key_blocks,
+  lb::attn_split_dq_kernel<<<dim3((unsigned)blocks), 256, 0, s>>>(dq_acc, (__nv_bfloat16*)dq, B, A, Sq, d, dqs[0], dqs[1], dqs[2], key_blocks,
                                                               causal, Sk - Sq);
   return (int)cudaGetLastError();
 }

@@ -7,6 +7,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <initializer_list>
+
 namespace lb {
 
 #define LB_DEVICE __device__ __forceinline__
@@ -98,6 +100,25 @@ LB_DEVICE uint4 philox4x32_7(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3,
   }
   return make_uint4(c0, c1, c2, c3);
 }
+
+// ---------------------------------------------------------------------------------------------
+// Launches that overlap the end of the kernel before them (lb_host::launch_chained below).  chain_wait() returns once that kernel has completed and
+// its writes can be seen: before it a kernel touches no global memory.  It takes the pointers that the kernel loads from through
+// `const __restrict__` parameters, whose loads the compiler could move in front of it otherwise.  chain_next() lets the next
+// kernel's blocks start, as soon as every block of this one has got there: behind a block's allocation of TMEM, which the next kernel's blocks
+// must not take from it.  A kernel that waits for other ranks or streams never calls it (the next one would hold an SM meanwhile).
+// What it gives: 1 to 3 us per launch (block of GPT-2 against a cache, 7 launches: 58 -> 45 us; block of Llama, 10 launches: 170 -> 150 us; [8, 1024] GPT-2
+// block forward and backward: 858 -> 809 us of GPU time).  What it takes: blocks are handed out while the SMs come free one after the other, so the
+// first ones get as many as fit.  Kernels that plan for an even spread lose more than they gain and are launched in order, without chain_wait(): norms
+// whose blocks take several rows in turn, norm backward ([12608, 1024] 25 us, chained 29), gated products ([2048, 11008] backward 40, chained 47),
+// attention backward with 512 blocks, longest first (185, chained 201), the sum over dQ's layers (22.1, chained 23.7).
+// ---------------------------------------------------------------------------------------------
+template <typename... P>
+LB_DEVICE void chain_wait(P&... loaded) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  (void)std::initializer_list<int>{(([&] { asm volatile("" : "+l"(loaded)); }()), 0)..., 0};
+}
+LB_DEVICE void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------------------------
 // mbarrier
@@ -497,4 +518,33 @@ bool make_tmap_typed(CUtensorMap* out, CUtensorMapDataType dtype, const void* ba
                      const uint64_t* strides_bytes, const uint32_t* box, CUtensorMapSwizzle swizzle);
 bool make_tmap_bf16(CUtensorMap* out, const void* base, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
                     const uint32_t* box, CUtensorMapSwizzle swizzle);
+
+// Launch of a kernel that begins with chain_wait(): its blocks start while the kernel before it in the stream ends, and set up their barriers and
+// TMEM meanwhile.  `cluster` CTAs along x, 0: no clusters.  While a graph is captured the launch is an ordinary one.
+template <typename... P, typename... A>
+cudaError_t launch_chained(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, unsigned cluster, const A&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (cluster > 0) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = cluster;
+    attr[n].val.clusterDim.y = 1;
+    attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n].val.programmaticStreamSerializationAllowed = 1;
+    ++n;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
 }  // namespace lb_host

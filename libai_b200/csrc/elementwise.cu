@@ -13,7 +13,7 @@
 namespace lb {
 
 LB_DEVICE void ld8(const __nv_bfloat16* p, float (&v)[8]) {
-  uint4 q = *reinterpret_cast<const uint4*>(p);
+  uint4 q = __ldg(reinterpret_cast<const uint4*>(p));
   float2 a = unpack_bf16(q.x), b = unpack_bf16(q.y), c = unpack_bf16(q.z), d = unpack_bf16(q.w);
   v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = c.x; v[5] = c.y; v[6] = d.x; v[7] = d.y;
 }
@@ -64,6 +64,8 @@ __global__ void bias_act_bwd_kernel(const __nv_bfloat16* __restrict__ gy, const 
 __global__ void bias_residual_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ bias,
                                      const __nv_bfloat16* __restrict__ res, __nv_bfloat16* __restrict__ y,
                                      size_t total_vec, int nvec_per_row) {
+  chain_wait(x, bias, res);
+  chain_next();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total_vec; i += (size_t)gridDim.x * blockDim.x) {
     float v[8];
     ld8(x + i * 8, v);
@@ -134,6 +136,7 @@ bias_dropout_residual_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfl
 
 __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __restrict__ up,
                                   __nv_bfloat16* __restrict__ y, size_t total_vec) {
+  chain_next();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total_vec; i += (size_t)gridDim.x * blockDim.x) {
     float g[8], u[8];
     ld8(gate + i * 8, g);
@@ -147,6 +150,7 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gate, const 
 // packed form: gu [T, 2F] = [gate | up] (the output of ONE GEMM against the stacked gate/up weights) -> y [T, F]
 __global__ void swiglu_packed_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ y, size_t rows,
                                          size_t fvec /* F / 8 */) {
+  chain_next();
   const size_t total = rows * fvec;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const size_t r = i / fvec, c = i % fvec;
@@ -161,6 +165,7 @@ __global__ void swiglu_packed_fwd_kernel(const __nv_bfloat16* __restrict__ gu, _
 // dgu [T, 2F] = [d gate | d up] from gy [T, F] and the saved gu
 __global__ void swiglu_packed_bwd_kernel(const __nv_bfloat16* __restrict__ gy, const __nv_bfloat16* __restrict__ gu,
                                          __nv_bfloat16* __restrict__ dgu, size_t rows, size_t fvec) {
+  chain_next();
   const size_t total = rows * fvec;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const size_t r = i / fvec, c = i % fvec;
@@ -182,6 +187,7 @@ __global__ void swiglu_packed_bwd_kernel(const __nv_bfloat16* __restrict__ gy, c
 __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gy, const __nv_bfloat16* __restrict__ gate,
                                   const __nv_bfloat16* __restrict__ up, __nv_bfloat16* __restrict__ dgate,
                                   __nv_bfloat16* __restrict__ dup, size_t total_vec) {
+  chain_next();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total_vec; i += (size_t)gridDim.x * blockDim.x) {
     float g[8], u[8], d[8], dg[8], du[8];
     ld8(gate + i * 8, g);
@@ -234,6 +240,8 @@ __global__ void rope_kernel(const __nv_bfloat16* __restrict__ x, const float* __
 __global__ void __launch_bounds__(256)
 rope_qkv_vec_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ cosv, const float* __restrict__ sinv,
                     __nv_bfloat16* __restrict__ y, int tokens, int S, int A, int D, int pos_offset, int backward, int copy_v) {
+  chain_wait(x, cosv, sinv);
+  chain_next();
   const int half = D / 2, vh = half / 8;            // vectors per half head
   const int c = (static_cast<int>(threadIdx.x) % vh) * 8, lane_row = threadIdx.x / vh, rows_per_pass = blockDim.x / vh;
   if (lane_row >= rows_per_pass) return;            // blockDim not a multiple of vh: the last threads own no vector
@@ -323,6 +331,8 @@ __global__ void rope_qkv_kernel(const __nv_bfloat16* __restrict__ x, const float
 // and serialised on 256-way contended addresses).
 __global__ void __launch_bounds__(256) colsum_vec_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ out,
                                                          int M, int N, int rows_per_block) {
+  chain_wait(x);
+  chain_next();
   __shared__ float sm[8][32][9];
   const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;
   const int c8 = (blockIdx.x * 32 + tx) * 8;
@@ -415,6 +425,8 @@ template <typename T>
 __global__ void __launch_bounds__(256) ce_stats_kernel(const T* __restrict__ logits, const int64_t* __restrict__ labels,
                                                        float* __restrict__ mx_out, float* __restrict__ se_out,
                                                        float* __restrict__ tgt_out, int V, int64_t vocab_start) {
+  chain_wait(logits, labels);
+  chain_next();
   __shared__ float sm[8], ss[8];
   const int row = blockIdx.x;
   const T* lr = logits + static_cast<size_t>(row) * V;
@@ -473,6 +485,8 @@ template <typename T>
 __global__ void __launch_bounds__(256) ce_bwd_kernel(const T* __restrict__ logits, const int64_t* __restrict__ labels,
                                                      const float* __restrict__ lse, const float* __restrict__ gloss,
                                                      T* __restrict__ dlogits, int V, int64_t vocab_start) {
+  chain_wait(logits, labels, lse, gloss);
+  chain_next();
   const int row = blockIdx.x;
   const T* lr = logits + static_cast<size_t>(row) * V;
   T* dr = dlogits + static_cast<size_t>(row) * V;
@@ -570,6 +584,8 @@ __global__ void clip_coef_kernel(const float* __restrict__ sq, float grad_scale,
 // out[t, :] = table[ids[t] - vocab_start, :]  (zero row when the id belongs to another vocabulary shard)
 __global__ void __launch_bounds__(128) embedding_fwd_kernel(const int64_t* __restrict__ ids, const __nv_bfloat16* __restrict__ table,
                                                             __nv_bfloat16* __restrict__ out, int H, long vocab_start, long rows) {
+  chain_wait(ids, table);
+  chain_next();
   const long t = blockIdx.x;
   const long r = ids[t] - vocab_start;
   const bool inside = r >= 0 && r < rows;
@@ -631,7 +647,7 @@ extern "C" int lb_bias_residual(const void* x, const void* bias, const void* res
   if (N % 8) return -1;
   const size_t tv = (size_t)rows * N / 8;
   if (tv == 0) return 0;
-  lb::bias_residual_kernel<<<ew_grid(tv, 256), 256, 0, s>>>((const bf16*)x, (const bf16*)bias, (const bf16*)res,
+  lb_host::launch_chained(lb::bias_residual_kernel, dim3(ew_grid(tv, 256)), dim3(256), 0, s, 0, (const bf16*)x, (const bf16*)bias, (const bf16*)res,
                                                             (bf16*)y, tv, N / 8);
   return (int)cudaGetLastError();
 }
@@ -655,27 +671,27 @@ extern "C" int lb_bias_dropout_residual(const void* x, const void* bias, const v
 extern "C" int lb_swiglu_fwd(const void* gate, const void* up, void* y, long n, cudaStream_t s) {
   if (n % 8) return -1;
   if (n == 0) return 0;
-  lb::swiglu_fwd_kernel<<<ew_grid(n / 8, 256), 256, 0, s>>>((const bf16*)gate, (const bf16*)up, (bf16*)y, n / 8);
+  lb::swiglu_fwd_kernel<<<dim3(ew_grid(n / 8, 256)), 256, 0, s>>>((const bf16*)gate, (const bf16*)up, (bf16*)y, n / 8);
   return (int)cudaGetLastError();
 }
 extern "C" int lb_swiglu_bwd(const void* gy, const void* gate, const void* up, void* dgate, void* dup, long n,
                              cudaStream_t s) {
   if (n % 8) return -1;
   if (n == 0) return 0;
-  lb::swiglu_bwd_kernel<<<ew_grid(n / 8, 256), 256, 0, s>>>((const bf16*)gy, (const bf16*)gate, (const bf16*)up,
+  lb::swiglu_bwd_kernel<<<dim3(ew_grid(n / 8, 256)), 256, 0, s>>>((const bf16*)gy, (const bf16*)gate, (const bf16*)up,
                                                             (bf16*)dgate, (bf16*)dup, n / 8);
   return (int)cudaGetLastError();
 }
 extern "C" int lb_swiglu_packed_fwd(const void* gu, void* y, long rows, long F, cudaStream_t s) {
   if (F % 8) return -1;
   if (rows == 0) return 0;
-  lb::swiglu_packed_fwd_kernel<<<ew_grid(rows * F / 8, 256), 256, 0, s>>>((const bf16*)gu, (bf16*)y, (size_t)rows, (size_t)(F / 8));
+  lb::swiglu_packed_fwd_kernel<<<dim3(ew_grid(rows * F / 8, 256)), 256, 0, s>>>((const bf16*)gu, (bf16*)y, (size_t)rows, (size_t)(F / 8));
   return (int)cudaGetLastError();
 }
 extern "C" int lb_swiglu_packed_bwd(const void* gy, const void* gu, void* dgu, long rows, long F, cudaStream_t s) {
   if (F % 8) return -1;
   if (rows == 0) return 0;
-  lb::swiglu_packed_bwd_kernel<<<ew_grid(rows * F / 8, 256), 256, 0, s>>>((const bf16*)gy, (const bf16*)gu, (bf16*)dgu,
+  lb::swiglu_packed_bwd_kernel<<<dim3(ew_grid(rows * F / 8, 256)), 256, 0, s>>>((const bf16*)gy, (const bf16*)gu, (bf16*)dgu,
                                                                          (size_t)rows, (size_t)(F / 8));
   return (int)cudaGetLastError();
 }
@@ -697,7 +713,7 @@ extern "C" int lb_rope_qkv(const void* x, const float* cosv, const float* sinv, 
     const int gx = (int)(tokens < 148L * 8 ? tokens : 148L * 8);      // eight blocks of 256 threads per SM
     const int rows_per_pass = 256 / (D / 16), passes = (A * (copy_v ? 3 : 2) + rows_per_pass - 1) / rows_per_pass;
     const int room = 148 * 8 / gx, gy = passes < room ? passes : room;
-    lb::rope_qkv_vec_kernel<<<dim3((unsigned)gx, (unsigned)gy), 256, 0, s>>>((const bf16*)x, cosv, sinv, (bf16*)y, (int)tokens, S, A, D, pos_offset, backward, copy_v);
+    lb_host::launch_chained(lb::rope_qkv_vec_kernel, dim3((unsigned)gx, (unsigned)gy), dim3(256), 0, s, 0, (const bf16*)x, cosv, sinv, (bf16*)y, (int)tokens, S, A, D, pos_offset, backward, copy_v);
     return (int)cudaGetLastError();
   }
   lb::rope_qkv_kernel<<<ew_grid((size_t)heads * (copy_v ? 3 : 2) * D / 2, 256), 256, 0, s>>>(
@@ -716,7 +732,8 @@ extern "C" int lb_colsum(const void* x, float* out, int M, int N, int accumulate
     if (row_blocks < 1) row_blocks = 1;
     const int rpb = (M + row_blocks - 1) / row_blocks;
     dim3 grid(col_blocks, (M + rpb - 1) / rpb);
-    lb::colsum_vec_kernel<<<grid, 256, 0, s>>>((const bf16*)x, out, M, N, rpb);
+    // (36 KB that nobody uses keep it to 4 blocks per SM: started while the SMs come free one after the other, eight would go to the first)
+    lb_host::launch_chained(lb::colsum_vec_kernel, dim3(grid), dim3(256), 36 * 1024, s, 0, (const bf16*)x, out, M, N, rpb);
     return (int)cudaGetLastError();
   }
   const int rpb = 128;
@@ -728,18 +745,18 @@ extern "C" int lb_ce_stats(const void* logits, const int64_t* labels, float* mx,
                            long vocab_start, int dtype, cudaStream_t s) {
   if (T == 0) return 0;
   if (dtype == 0)
-    lb::ce_stats_kernel<bf16><<<T, 256, 0, s>>>((const bf16*)logits, labels, mx, se, tgt, V, vocab_start);
+    lb_host::launch_chained(lb::ce_stats_kernel<bf16>, dim3(T), dim3(256), 0, s, 0, (const bf16*)logits, labels, mx, se, tgt, V, vocab_start);
   else
-    lb::ce_stats_kernel<float><<<T, 256, 0, s>>>((const float*)logits, labels, mx, se, tgt, V, vocab_start);
+    lb_host::launch_chained(lb::ce_stats_kernel<float>, dim3(T), dim3(256), 0, s, 0, (const float*)logits, labels, mx, se, tgt, V, vocab_start);
   return (int)cudaGetLastError();
 }
 extern "C" int lb_ce_bwd(const void* logits, const int64_t* labels, const float* lse, const float* gloss, void* dlogits,
                          int T, int V, long vocab_start, int dtype, cudaStream_t s) {
   if (T == 0) return 0;
   if (dtype == 0)
-    lb::ce_bwd_kernel<bf16><<<T, 256, 0, s>>>((const bf16*)logits, labels, lse, gloss, (bf16*)dlogits, V, vocab_start);
+    lb_host::launch_chained(lb::ce_bwd_kernel<bf16>, dim3(T), dim3(256), 0, s, 0, (const bf16*)logits, labels, lse, gloss, (bf16*)dlogits, V, vocab_start);
   else
-    lb::ce_bwd_kernel<float><<<T, 256, 0, s>>>((const float*)logits, labels, lse, gloss, (float*)dlogits, V,
+    lb_host::launch_chained(lb::ce_bwd_kernel<float>, dim3(T), dim3(256), 0, s, 0, (const float*)logits, labels, lse, gloss, (float*)dlogits, V,
                                                vocab_start);
   return (int)cudaGetLastError();
 }
@@ -756,7 +773,7 @@ extern "C" int lb_embedding_fwd(const int64_t* ids, const void* table, void* out
                                 cudaStream_t s) {
   if (T == 0) return 0;
   if (H % 8) return -1;
-  lb::embedding_fwd_kernel<<<(unsigned)T, 128, 0, s>>>(ids, (const bf16*)table, (bf16*)out, H, vocab_start, rows);
+  lb_host::launch_chained(lb::embedding_fwd_kernel, dim3((unsigned)T), dim3(128), 0, s, 0, ids, (const bf16*)table, (bf16*)out, H, vocab_start, rows);
   return (int)cudaGetLastError();
 }
 extern "C" int lb_embedding_bwd(const int64_t* ids, const void* gy, float* grad, long T, int H, long vocab_start, long rows,

@@ -77,6 +77,8 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  chain_wait();
+  chain_next();
 
   if (warp_idx == 0) {
     if (elect_one()) {
@@ -202,19 +204,8 @@ cudaError_t launch_gemm_small_r(const CUtensorMap& tw, const CUtensorMap& tx, Ge
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)RANKS, (unsigned)((p.N + 127) / 128), (unsigned)((p.M + NT - 1) / NT));
-  cfg.blockDim = dim3(GS_THREADS);
-  cfg.dynamicSmemBytes = (size_t)smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)RANKS;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, tw, tx, p);
+  return lb_host::launch_chained(kern, dim3((unsigned)RANKS, (unsigned)((p.N + 127) / 128), (unsigned)((p.M + NT - 1) / NT)), dim3(GS_THREADS), (size_t)smem, s,
+                                 (unsigned)RANKS, tw, tx, p);
 }
 template <int NT>
 cudaError_t launch_gemm_small(const CUtensorMap& tw, const CUtensorMap& tx, const GemmSmallParams& p, int ranks, cudaStream_t s) {

@@ -17,7 +17,7 @@ struct Vec8;
 template <>
 struct Vec8<__nv_bfloat16> {
   static LB_DEVICE void load(const __nv_bfloat16* p, float (&v)[8]) {
-    uint4 q = *reinterpret_cast<const uint4*>(p);
+    uint4 q = __ldg(reinterpret_cast<const uint4*>(p));
     float2 a = unpack_bf16(q.x), b = unpack_bf16(q.y), c = unpack_bf16(q.z), d = unpack_bf16(q.w);
     v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = c.x; v[5] = c.y; v[6] = d.x; v[7] = d.y;
   }
@@ -29,7 +29,7 @@ struct Vec8<__nv_bfloat16> {
 template <>
 struct Vec8<float> {
   static LB_DEVICE void load(const float* p, float (&v)[8]) {
-    float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+    float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p + 4));
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
   }
   static LB_DEVICE void store(float* p, const float (&v)[8]) {
@@ -46,6 +46,8 @@ template <typename T, typename W, int VPL, bool RMS, bool TAIL>
 __global__ void __launch_bounds__(NORM_WARPS * 32)
 norm_fwd_kernel(const T* __restrict__ x, const W* __restrict__ gamma, const W* __restrict__ beta, T* __restrict__ y,
                 float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, float eps, int h_tail) {
+  chain_wait(x, gamma, beta);
+  chain_next();
   const int H = TAIL ? h_tail : VPL * 256;
   const float inv_h = 1.0f / static_cast<float>(H);
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
@@ -104,6 +106,7 @@ norm_bwd_kernel(const T* __restrict__ gy, const T* __restrict__ x, const W* __re
                 const float* __restrict__ mean_in, const float* __restrict__ rstd_in, T* __restrict__ gx,
                 float* __restrict__ part_dgamma, float* __restrict__ part_dbeta, int rows,
                 const T* __restrict__ gadd /* optional [rows, H]: gradient of the residual path, added to gx */) {
+  chain_next();
   constexpr int H = VPL * 256;
   __shared__ float red[NORM_WARPS][32 * 8 + 8];
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
@@ -188,6 +191,7 @@ norm_bwd_bf16_kernel(const __nv_bfloat16* __restrict__ gy, const __nv_bfloat16* 
                      float* __restrict__ part_dgamma, float* __restrict__ part_dbeta, int rows,
                      const __nv_bfloat16* __restrict__ gadd, float* __restrict__ acc_dgamma, float* __restrict__ acc_dbeta,
                      int h_tail) {
+  chain_next();
   const int H = TAIL ? h_tail : VPL * 256;       // TAIL: lanes behind the row's end neither load nor store
   const float inv_h = 1.0f / static_cast<float>(H);
   __shared__ float red[NORM_BWD_WARPS][32 * 8 + 8];
@@ -321,6 +325,8 @@ __global__ void __launch_bounds__(NORM_WIDE_THREADS)
 norm_fwd_wide_kernel(const __nv_bfloat16* __restrict__ x, const W* __restrict__ gamma, const W* __restrict__ beta,
                      __nv_bfloat16* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int H,
                      float eps) {
+  chain_wait(x, gamma, beta);
+  chain_next();
   __shared__ float2 red[2][NORM_WIDE_THREADS / 32];
   int buf = 0;
   const float inv_h = 1.0f / static_cast<float>(H);
@@ -330,7 +336,7 @@ norm_fwd_wide_kernel(const __nv_bfloat16* __restrict__ x, const W* __restrict__ 
 #pragma unroll
     for (int i = 0; i < V; ++i) {
       const int c = (i * NORM_WIDE_THREADS + threadIdx.x) * 8;
-      q[i] = c < H ? *reinterpret_cast<const uint4*>(x + base + c) : make_uint4(0, 0, 0, 0);
+      q[i] = c < H ? __ldg(reinterpret_cast<const uint4*>(x + base + c)) : make_uint4(0, 0, 0, 0);
     }
     float mean = 0.f;
     if (!RMS) {
@@ -384,6 +390,7 @@ norm_bwd_wide_kernel(const __nv_bfloat16* __restrict__ gy, const __nv_bfloat16* 
                      const float* __restrict__ mean_in, const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ gx,
                      float* __restrict__ part_dgamma, float* __restrict__ part_dbeta, int rows, int H,
                      const __nv_bfloat16* __restrict__ gadd) {
+  chain_next();
   __shared__ float2 red[2][NORM_WIDE_THREADS / 32];
   int buf = 0;
   const float inv_h = 1.0f / static_cast<float>(H);
@@ -459,6 +466,8 @@ norm_bwd_wide_kernel(const __nv_bfloat16* __restrict__ gy, const __nv_bfloat16* 
 __global__ void __launch_bounds__(256) colreduce_kernel(const float* __restrict__ part0, float* __restrict__ out0,
                                                         const float* __restrict__ part1, float* __restrict__ out1,
                                                         int nrows, int H, int accumulate) {
+  chain_wait(part0, out0, part1, out1);
+  chain_next();
   const float* __restrict__ part = blockIdx.y == 0 ? part0 : part1;
   float* __restrict__ out = blockIdx.y == 0 ? out0 : out1;
   __shared__ float sm[8][33];
@@ -596,13 +605,20 @@ bool norm_bwd_by_warp(int rows, int H) {
 }
 
 // fp32 activations: H = 256 VPL
+// Chained where every row has its own warp or block.  Where blocks take several rows in turn, the first SMs to come free would get the blocks with one row
+// more: [12608, 1024] 10.9 us in order, 13.0 chained.
+template <typename... P, typename... A>
+void launch_norm(bool chain, void (*kern)(P...), int grid, int threads, cudaStream_t s, const A&... args) {
+  if (chain) lb_host::launch_chained(kern, dim3(grid), dim3(threads), 0, s, 0, args...);
+  else kern<<<grid, threads, 0, s>>>(static_cast<P>(args)...);
+}
 template <bool RMS>
 bool fwd_dispatch_f32(int vpl, const float* x, const float* g, const float* b, float* y, float* mean, float* rstd, int rows,
                       float eps, cudaStream_t s) {
   const int grid = norm_fwd_grid(rows);
 #define LB_CASE(V)                                                                                                            \
   case V:                                                                                                                     \
-    lb::norm_fwd_kernel<float, float, V, RMS, false><<<grid, lb::NORM_WARPS * 32, 0, s>>>(x, g, b, y, mean, rstd, rows, eps, 0); \
+    launch_norm(rows <= grid * lb::NORM_WARPS, lb::norm_fwd_kernel<float, float, V, RMS, false>, grid, lb::NORM_WARPS * 32, s, x, g, b, y, mean, rstd, rows, eps, 0); \
     return true;
   switch (vpl) {
     LB_CASE(1) LB_CASE(2) LB_CASE(3) LB_CASE(4) LB_CASE(5) LB_CASE(6) LB_CASE(8) LB_CASE(10) LB_CASE(12) LB_CASE(16)
@@ -621,9 +637,9 @@ void fwd_dispatch_bf16(int H, const __nv_bfloat16* x, const W* g, const W* b, __
 #define LB_CASE(V)                                                                                                                  \
   case V:                                                                                                                           \
     if (H % 256 == 0)                                                                                                               \
-      lb::norm_fwd_kernel<__nv_bfloat16, W, V, RMS, false><<<grid, lb::NORM_WARPS * 32, 0, s>>>(x, g, b, y, mean, rstd, rows, eps, H); \
+      launch_norm(rows <= grid * lb::NORM_WARPS, lb::norm_fwd_kernel<__nv_bfloat16, W, V, RMS, false>, grid, lb::NORM_WARPS * 32, s, x, g, b, y, mean, rstd, rows, eps, H); \
     else                                                                                                                            \
-      lb::norm_fwd_kernel<__nv_bfloat16, W, V, RMS, true><<<grid, lb::NORM_WARPS * 32, 0, s>>>(x, g, b, y, mean, rstd, rows, eps, H);  \
+      launch_norm(rows <= grid * lb::NORM_WARPS, lb::norm_fwd_kernel<__nv_bfloat16, W, V, RMS, true>, grid, lb::NORM_WARPS * 32, s, x, g, b, y, mean, rstd, rows, eps, H);  \
     break;
     switch ((H + 255) / 256) { LB_CASE(1) LB_CASE(2) LB_CASE(3) LB_CASE(4) }
 #undef LB_CASE
@@ -633,7 +649,7 @@ void fwd_dispatch_bf16(int H, const __nv_bfloat16* x, const W* g, const W* b, __
     const int grid = norm_fwd_grid(rows);
 #define LB_CASE(V)                                                                                                                  \
   case V:                                                                                                                           \
-    lb::norm_fwd_kernel<__nv_bfloat16, W, V, RMS, false><<<grid, lb::NORM_WARPS * 32, 0, s>>>(x, g, b, y, mean, rstd, rows, eps, H); \
+    launch_norm(rows <= grid * lb::NORM_WARPS, lb::norm_fwd_kernel<__nv_bfloat16, W, V, RMS, false>, grid, lb::NORM_WARPS * 32, s, x, g, b, y, mean, rstd, rows, eps, H); \
     break;
     switch (H / 256) { LB_CASE(5) LB_CASE(6) LB_CASE(8) LB_CASE(10) }
 #undef LB_CASE
@@ -642,7 +658,7 @@ void fwd_dispatch_bf16(int H, const __nv_bfloat16* x, const W* g, const W* b, __
   const int grid = norm_fwd_wide_grid(rows);
 #define LB_CASE(V)                                                                                                             \
   case V:                                                                                                                      \
-    lb::norm_fwd_wide_kernel<W, V, RMS><<<grid, lb::NORM_WIDE_THREADS, 0, s>>>(x, g, b, y, mean, rstd, rows, H, eps);          \
+    launch_norm(rows <= grid, lb::norm_fwd_wide_kernel<W, V, RMS>, grid, lb::NORM_WIDE_THREADS, s, x, g, b, y, mean, rstd, rows, H, eps);          \
     break;
   switch ((H + 2047) / 2048) { LB_CASE(1) LB_CASE(2) LB_CASE(3) LB_CASE(4) }
 #undef LB_CASE
@@ -787,7 +803,7 @@ extern "C" int lb_norm_bwd(const void* gy, const void* x, const void* gamma, con
     else { if (rms) LB_GO(float, true); else LB_GO(float, false); }
 #undef LB_GO
     if (!direct)
-      lb::colreduce_kernel<<<dim3((H + 31) / 32, dbeta != nullptr ? 2 : 1), 256, 0, s>>>(pdg, dgamma, pdb, dbeta, grid, H, accumulate);
+      lb_host::launch_chained(lb::colreduce_kernel, dim3((H + 31) / 32, dbeta != nullptr ? 2 : 1), dim3(256), 0, s, 0, pdg, dgamma, pdb, dbeta, grid, H, accumulate);
   } else if (dtype == 1 && wdtype == 1) {
     const int grid = norm_grid(rows);
     float* pdg = workspace;
@@ -797,7 +813,7 @@ extern "C" int lb_norm_bwd(const void* gy, const void* x, const void* gamma, con
       done = rms ? bwd_dispatch_f32<true>(H / 256, (const float*)gy, (const float*)x, (const float*)gamma, mean, rstd, (float*)gx, pdg, pdb, rows, grid, s, (const float*)gadd)
                  : bwd_dispatch_f32<false>(H / 256, (const float*)gy, (const float*)x, (const float*)gamma, mean, rstd, (float*)gx, pdg, pdb, rows, grid, s, (const float*)gadd);
     if (done)
-      lb::colreduce_kernel<<<dim3((H + 31) / 32, dbeta != nullptr ? 2 : 1), 256, 0, s>>>(pdg, dgamma, pdb, dbeta, grid, H, accumulate);
+      lb_host::launch_chained(lb::colreduce_kernel, dim3((H + 31) / 32, dbeta != nullptr ? 2 : 1), dim3(256), 0, s, 0, pdg, dgamma, pdb, dbeta, grid, H, accumulate);
     else
       norm_bwd_any<float, float>(gy, x, gamma, mean, rstd, gx, dgamma, dbeta, rows, H, rms, accumulate, s);
   } else {

@@ -791,3 +791,58 @@ def test_gradient_norm_and_clip_coefficient_over_groups(size, poison, scale):
     coef = torch.clamp(1.0 / (want + 1e-6), max=1.0)
     # sums of a few thousand squares in fp32 and a handful of roundings
     assert torch.allclose(norm.double(), want, rtol=1e-5, equal_nan=True) and torch.allclose(opt._clip_coef.double(), coef, rtol=1e-5, equal_nan=True)
+
+
+@pytest.mark.parametrize("where", ["stream", "side stream", "capture"])
+@pytest.mark.parametrize("make,b,s", [(lambda: _gpt_block(16, 24, "causal"), 1, 40), (lambda: _gpt_block(4, 64, "causal"), 3, 260),
+                                      (lambda: _gpt_block(6, 48, "padding"), 2, 150), (lambda: _llama_block(4, 64, True), 2, 130)])
+def test_launches_that_start_before_the_last_one_ends(make, b, s, where):
+    """Ten passes in a row, each on the last one's output and in memory that the one before left, and one backward pass: the same bits as with a wait after
+    every operator (the operators' sums have one order; only weight gradients do not)."""
+    m = make()
+    h = next(m.parameters()).numel()
+    x = _rand((b, s, h), 1)
+    kw = {}
+    if type(m).__name__ == "LlamaDecoderLayer":
+        kw = dict(zip(("cos_cached", "sin_cached"), _ROT(512, 64)))
+
+    class Waiting(torch.utils._python_dispatch.TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            out = func(*args, **(kwargs or {}))
+            torch.cuda.synchronize()
+            return out
+
+    def forward():
+        y = x
+        for _ in range(10):
+            y = m(y, **kw)
+        return y
+
+    def backward():
+        xi = x.clone().requires_grad_(True)
+        return torch.autograd.grad(m(xi, **kw), xi, x)[0]
+
+    with torch.no_grad(), Waiting():
+        want = forward()
+    stream = torch.cuda.current_stream() if where == "stream" else torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.no_grad(), torch.cuda.stream(stream):
+        for _ in range(3):
+            got = forward()
+        if where == "capture":
+            stream.synchronize()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=stream):
+                got = forward()
+            for _ in range(3):
+                got.zero_()
+                graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+    if x.shape[-1] == 6 * 48:                       # (attention that adds dQ up in one order)
+        with Waiting():
+            want = backward()
+        with torch.cuda.stream(stream):
+            got = backward()
+        torch.cuda.synchronize()
+        assert torch.equal(got, want)
