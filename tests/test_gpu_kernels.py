@@ -846,3 +846,23 @@ def test_launches_that_start_before_the_last_one_ends(make, b, s, where):
             got = backward()
         torch.cuda.synchronize()
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("vocab", [8, 2056, 8184, 8192, 8200, 18440, 50304, 1003])
+def test_cross_entropy_statistics_in_groups_of_loads(vocab):
+    """Maxima are exact.  A thread adds up ``vocab / 256`` terms in two sums, 13 more come from the other threads: as many roundings of 2^-24 at most, and each
+    exponential is off by 2 ulp and the rounding of its argument, up to 2^-24 of 60.  A row may be minus infinity almost everywhere."""
+    x = _rand((5, vocab), 1, 4.0)
+    x[1] -= 40.0
+    x[2, : vocab // 2] = float("-inf")
+    x[2, vocab // 3] = 1.0
+    x[3, vocab - 1] = 50.0
+    labels = torch.tensor([0, vocab - 1, vocab, -1, vocab // 2], device="cuda")
+    mx, se, tgt = load_ext().ce_stats(x, labels, 0)
+    d = x.double()
+    want = (d - d.amax(1, keepdim=True)).exp().sum(1)
+    assert torch.equal(mx, x.float().amax(1))
+    assert torch.equal(tgt, torch.stack([x[0, 0], x[1, -1], x.new_zeros(()), x.new_zeros(()), x[4, vocab // 2]]).float())
+    assert float(((se.double() - want).abs() / want).max()) <= (vocab / 256 + 13 + 4 + 60) * 2.0 ** -24
+    x[4, vocab // 3] = float("nan")
+    assert bool(load_ext().ce_stats(x, labels, 0)[1][4].isnan())
