@@ -14,6 +14,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "common.cuh"
+
 typedef __nv_bfloat16 bf16;
 
 namespace {
@@ -175,6 +177,7 @@ __global__ void __launch_bounds__(128)
 short_conv_strip_kernel(const __nv_bfloat16* __restrict__ in, long ldi, const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ tail,
                         const int* __restrict__ tok_seq, const int* __restrict__ seq_off, const int* __restrict__ slots, const int* __restrict__ past,
                         __nv_bfloat16* __restrict__ out, long ldo, long tokens, int C) {
+  lb::chain_next();
   const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
   const int C8 = C >> 3;
   const long tok0 = idx / C8 * CONV_STRIP;
@@ -232,6 +235,8 @@ short_conv_strip_kernel(const __nv_bfloat16* __restrict__ in, long ldi, const __
 template <typename T>
 __global__ void conv_tail_kernel(const T* __restrict__ in, long ldi, T* __restrict__ tail, const int* __restrict__ seq_off,
                                  const int* __restrict__ slots, const int* __restrict__ past, int B, int C, int taps) {
+  lb::chain_wait(in, tail, seq_off, slots, past);
+  lb::chain_next();
   const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long)B * C) return;
   const int b = (int)(idx / C), c = (int)(idx - (long)b * C);
@@ -687,6 +692,7 @@ __global__ void __launch_bounds__(128)
 delta_chunk_prep_kernel(const bf16* __restrict__ qkv, long ldq, int koff, const bf16* __restrict__ a, long lda, const bf16* __restrict__ bl, long ldb,
                         const bf16* __restrict__ A_log, const bf16* __restrict__ dt_bias, const int* __restrict__ seq_off, float* __restrict__ scratch,
                         int B, int H, int KH, int D) {
+  lb::chain_next();
   constexpr int LD = DP + 8;
   __shared__ __align__(16) bf16 sK[CL * LD], sQ[CL * LD];
   __shared__ float sKK[CL][CL + 1], sQK[CL][CL + 1], sA[4][CL][CL + 4];
@@ -841,6 +847,7 @@ __global__ void __launch_bounds__(32 * CL_WARPS)
 delta_chunk_scan_kernel(const bf16* __restrict__ qkv, long ldq, int koff, int voff, const float* __restrict__ scratch, float* __restrict__ S,
                         const int* __restrict__ seq_off, const int* __restrict__ slots, const int* __restrict__ past, float* __restrict__ out,
                         int H, int KH, int D, int V) {
+  lb::chain_next();
   constexpr int LD = DP + 8, VLD = CL_COLS + 8, THREADS = 32 * CL_WARPS;
   extern __shared__ __align__(16) unsigned char delta_sm[];
   DeltaChunkSmem<DP>& sm = *reinterpret_cast<DeltaChunkSmem<DP>*>(delta_sm);
@@ -1077,6 +1084,8 @@ template <typename T, int R>
 __global__ void __launch_bounds__(256)
 gated_rmsnorm_vec_kernel(const float* __restrict__ o, const T* __restrict__ gate, long ldg, const T* __restrict__ w, float eps, int act, T* __restrict__ y,
                          long ldy, long rows, int H, int V) {
+  lb::chain_wait(o, gate, w);
+  lb::chain_next();
   const long wid = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (wid >= rows * H) return;
@@ -1550,14 +1559,14 @@ int lbs_short_conv(const void* in, long ldi, const void* w, void* tail, const in
                                                     (bf16*)out, ldo, tokens, C)
     if (taps == 2) { SC(2); } else if (taps == 3) { SC(3); } else { SC(4); }
 #undef SC
-    conv_tail_kernel<bf16><<<cdiv((long)B * C, 256), 256, 0, s>>>((const bf16*)in, ldi, (bf16*)tail, seq_off, slots, past, B, C, taps);
+    lb_host::launch_chained(conv_tail_kernel<bf16>, dim3(cdiv((long)B * C, 256)), dim3(256), 0, s, 0, (const bf16*)in, ldi, (bf16*)tail, seq_off, slots, past, B, C, taps);
     return ok();
   }
   DISPATCH(dtype, {
     short_conv_kernel<T><<<cdiv(tokens * C, 256), 256, 0, s>>>((const T*)in, ldi, (const T*)w, (const T*)tail, tok_seq, seq_off, slots,
                                                                 past, (T*)out, ldo, tokens, C, taps);
     if (taps > 1)
-      conv_tail_kernel<T><<<cdiv((long)B * C, 256), 256, 0, s>>>((const T*)in, ldi, (T*)tail, seq_off, slots, past, B, C, taps);
+      lb_host::launch_chained(conv_tail_kernel<T>, dim3(cdiv((long)B * C, 256)), dim3(256), 0, s, 0, (const T*)in, ldi, (T*)tail, seq_off, slots, past, B, C, taps);
   });
   return ok();
 }
@@ -1653,7 +1662,7 @@ int lbs_gated_rmsnorm(const float* o, const void* gate, long ldg, const void* w,
   const uintptr_t vec = dtype == 0 ? 16 : 8;                    // bytes of four elements
   if (V % 4 == 0 && V <= 512 && ldg % 4 == 0 && ldy % 4 == 0 && (reinterpret_cast<uintptr_t>(o) & 15) == 0 &&
       ((reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) & (vec - 1)) == 0) {
-#define GRV(R) DISPATCH(dtype, gated_rmsnorm_vec_kernel<T, R><<<cdiv(rows * H * 32, 256), 256, 0, s>>>(o, (const T*)gate, ldg, (const T*)w, eps, act, (T*)y, ldy, rows, H, V))
+#define GRV(R) DISPATCH(dtype, lb_host::launch_chained(gated_rmsnorm_vec_kernel<T, R>, dim3(cdiv(rows * H * 32, 256)), dim3(256), 0, s, 0, o, (const T*)gate, ldg, (const T*)w, eps, act, (T*)y, ldy, rows, H, V))
     if (V <= 128) { GRV(1); } else if (V <= 256) { GRV(2); } else { GRV(4); }
 #undef GRV
     return ok();
