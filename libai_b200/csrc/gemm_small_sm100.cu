@@ -253,8 +253,11 @@ int* small_wait_word() {
 // 46.6), not many tiles ([64, 1024] x [50304, 1024] 27.3 against 23.4 us, [2048, 5120] x [1280, 5120] 39.6 against 29.3) and not a short K
 // ([256, 384] x [1536, 384] 6.2 against 5.8).  Clusters of 4 and 8 are kept to 264 CTAs: the SMs of a GPC do not divide by them, and 72
 // clusters of 4 with two CTAs per SM ran in two waves ([96, 1024] x [3072, 1024] 10.2 against 8.2 us).
+// More than 2048 rows only against one tile of 16 to 128 columns (the gates of a mixer), where the other kernel walks all of K in one CTA:
+// [2560, 2048] x [16, 2048] 9.6 against 11.1 us, x [128, 2048] 9.2 against 11.4, [4096, 4096] x [32, 4096] 9.8 against 18.6, [8192, 4096] x [64, 4096]
+// 14.0 against 19.3; with 8 columns [8192, 4096] 19.7 against 18.9, and [16384, 2048] x [64, 2048] 15.5 against 12.1.
 extern "C" int lb_gemm_small_rule(int M, int N, int K, int* nt, int* ranks) {
-  if (M > 2048) return 0;
+  if (M > (N < 16 || N > 128 ? 2048 : 8192)) return 0;
   const int kb = (K + 63) / 64, tiles_n = (N + 127) / 128;
   const double w_us = (double)N * K * 2 / 6e6;
   const double block_us[4] = {0.28, 0.34, 0.34, 0.38};

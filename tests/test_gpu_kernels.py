@@ -866,3 +866,15 @@ def test_cross_entropy_statistics_in_groups_of_loads(vocab):
     assert float(((se.double() - want).abs() / want).max()) <= (vocab / 256 + 13 + 4 + 60) * 2.0 ** -24
     x[4, vocab // 3] = float("nan")
     assert bool(load_ext().ce_stats(x, labels, 0)[1][4].isnan())
+
+
+@pytest.mark.parametrize("m,n,k", [(2049, 16, 2048), (2560, 128, 2048), (8192, 64, 4096), (8193, 64, 4096), (4096, 8, 4096), (4097, 24, 4104), (2560, 136, 2048)])
+def test_many_rows_against_one_tile_of_columns(m, n, k):
+    """Both sides of the rule that gives such products to clusters along K: bf16 results within the rounding of the result (2^-8 of it) and of ``k`` fp32
+    additions (``k * 2^-24`` of the sum of magnitudes; the tensor core truncates, twice that)."""
+    x, w, b = _rand((m, k), 1), _rand((n, k), 2), _rand((n,), 3)
+    y = load_ext().linear_fwd(x, w, b, 0, False)[0]
+    want = x.double() @ w.double().T + b.double()
+    bound = want.abs() * 2.0 ** -8 + (x.double().abs() @ w.double().abs().T + b.double().abs()) * k * 2.0 ** -23
+    assert bool(((y.double() - want).abs() <= bound).all())
+    assert float((y.double() - want).norm() / want.norm()) < 2.0 ** -8
