@@ -15,6 +15,7 @@ from libai_b200.ops import functional as OF
 from libai_b200.utils import distributed as dutil
 
 _FORWARDS = {}
+_CALL = torch.nn.Module.__call__
 
 
 def remember(*classes):
@@ -26,13 +27,24 @@ def remember(*classes):
 def applies(x) -> bool:
     """What holds for the call as a whole."""
     return (not torch.is_grad_enabled() and type(x) is torch.Tensor and x.dtype is torch.bfloat16 and x.dim() == 3 and ops.use_native(x)
-            and OF._plain_call() and not ops.fp8_enabled() and dutil.get_dist_util().tensor_parallel_size == 1
-            and not _module._global_forward_hooks and not _module._global_forward_pre_hooks)
+            and OF._plain_call() and not ops.fp8_enabled() and dutil.get_dist_util().tensor_parallel_size == 1 and not _calls_are_seen())
+
+
+def _calls_are_seen() -> bool:
+    """Does anything look at the call of every module: global hooks, a replaced ``Module.__call__``?"""
+    return bool(_module._global_forward_hooks or _module._global_forward_pre_hooks or _module._global_backward_hooks or _module._global_backward_pre_hooks
+                or torch.nn.Module.__call__ is not _CALL)
 
 
 def plain(m, cls) -> bool:
-    """A module of this very class whose call is its class's ``forward`` and nothing else."""
-    return (type(m) is cls and cls.forward is _FORWARDS[cls] and not m._forward_hooks and not m._forward_pre_hooks and "forward" not in m.__dict__)
+    """A module of this very class whose call is its class's ``forward`` and nothing else (``alone`` asks for what holds for all modules, too)."""
+    return (type(m) is cls and cls.forward is _FORWARDS[cls] and not m._forward_hooks and not m._forward_pre_hooks and not m._backward_hooks
+            and not m._backward_pre_hooks and m._compiled_call_impl is None and "forward" not in m.__dict__)
+
+
+def alone(m, cls) -> bool:
+    """Would nobody notice if this module were passed by, its work joined with a neighbour's, graph or not?"""
+    return plain(m, cls) and not _calls_are_seen()
 
 
 def parameters(*pairs):

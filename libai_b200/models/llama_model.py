@@ -117,7 +117,7 @@ class LlamaMLP(nn.Module):
 
 def _plus_residual(proj, x, residual):
     """``residual + proj(x)``; one kernel where ``proj`` is a plain linear layer of one tensor-parallel rank without a bias."""
-    w = proj._parameters.get("weight") if native.plain(proj, Linear) else None
+    w = proj._parameters.get("weight") if native.alone(proj, Linear) else None
     if (w is not None and proj.bias is None and not proj.skip_bias_add and dutil.get_dist_util().tensor_parallel_size == 1 and x.dtype == torch.bfloat16
             and residual.shape == (*x.shape[:-1], w.shape[0])):
         return OF.linear_bias_residual(x, w, None, residual)
@@ -224,7 +224,7 @@ class LlamaDecoderLayer(nn.Module):
         ln, skip = self._norm(self.input_layernorm, hidden_states)
         call = dict(attention_mask=attention_mask, past_key_value=past_key_value, cos_cached=cos_cached, sin_cached=sin_cached, use_cache=use_cache)
         presents = None
-        if native.plain(self.self_attn, LlamaAttention):
+        if native.alone(self.self_attn, LlamaAttention):
             attn = self.self_attn(ln, residual=skip, **call)
             hidden_states, presents = attn if use_cache else (attn, None)
         else:
@@ -233,13 +233,13 @@ class LlamaDecoderLayer(nn.Module):
                 attn, presents = attn
             hidden_states = skip + attn
         ln, skip = self._norm(self.post_attention_layernorm, hidden_states)
-        output = self.mlp(ln, residual=skip) if native.plain(self.mlp, LlamaMLP) else skip + self.mlp(ln)
+        output = self.mlp(ln, residual=skip) if native.alone(self.mlp, LlamaMLP) else skip + self.mlp(ln)
         return (output, presents) if use_cache else output
 
     @staticmethod
     def _norm(norm, x):
         """``(norm(x), x)``; the skip connection's gradient joins inside the norm's backward kernel where ``norm`` is a plain one."""
-        if native.plain(norm, RMSLayerNorm) and not norm.zero_centered:
+        if native.alone(norm, RMSLayerNorm) and not norm.zero_centered:
             return OF.rms_norm_with_skip(x, norm.weight, norm.eps)
         return norm(x), x
 

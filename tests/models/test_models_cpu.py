@@ -92,3 +92,63 @@ def test_vision_models_with_mixup(recipe, overrides, size):
     _check(model, out["losses"])
     model.eval()
     assert model(images)["prediction_scores"].shape == (4, 10)
+
+
+def _small_block(kind, dtype):
+    from libai_b200.layers import TransformerLayer
+    from libai_b200.layers._param import param_defaults
+    from libai_b200.models.llama_model import LlamaDecoderLayer, rotary_tables
+
+    with param_defaults(dtype=dtype, seed=5):
+        m = LlamaDecoderLayer(32, 64, 4) if kind == "llama" else TransformerLayer(32, 64, 4)
+    tables = dict(zip(("cos_cached", "sin_cached"), rotary_tables(8, 16))) if kind == "llama" else {}
+    x = torch.randn(2, 6, 32, generator=torch.Generator().manual_seed(1)).to(dtype).requires_grad_(True)
+    return m, x, lambda: m(x, **tables)
+
+
+# what a block calls as modules (the GPT block's norms and, in bf16, its projections have always been joined with their neighbours)
+SEEN = {"llama": {"input_layernorm", "self_attn", "self_attn.query_key_value", "self_attn.o_proj", "post_attention_layernorm", "mlp", "mlp.gate_proj",
+                  "mlp.up_proj", "mlp.down_proj"},
+        "gpt": {"self_attention", "self_attention.query_key_value", "self_attention.dense", "mlp"}}
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("kind", ["llama", "gpt"])
+@pytest.mark.parametrize("how", ["backward", "backward_pre", "global_forward", "global_forward_pre", "global_backward"])
+def test_hooks_see_the_modules_of_a_block(kind, how, dtype):
+    """Residual adds in epilogues and skip gradients in the norms' backward pass modules by: not while anything looks at their calls."""
+    from torch.nn.modules import module as hooks
+
+    m, x, call = _small_block(kind, dtype)
+    names, seen, handles = {k: n for n, k in m.named_modules()}, set(), []
+    note = lambda mod, *a: seen.add(names[mod])
+    if how.startswith("global"):
+        register = {"global_forward": hooks.register_module_forward_hook, "global_forward_pre": hooks.register_module_forward_pre_hook,
+                    "global_backward": hooks.register_module_full_backward_hook}[how]
+        handles.append(register(note))
+    else:
+        for n, k in m.named_modules():
+            if n:
+                handles.append(k.register_full_backward_hook(note) if how == "backward" else k.register_full_backward_pre_hook(note))
+    try:
+        call().sum().backward()
+    finally:
+        for h in handles:
+            h.remove()
+    joined = {"self_attention.dense"} if kind == "gpt" and dtype == torch.bfloat16 else set()
+    assert seen - {""} == SEEN[kind] - joined
+
+
+@pytest.mark.parametrize("name", ["input_layernorm", "post_attention_layernorm", "self_attn", "self_attn.o_proj", "mlp", "mlp.down_proj"])
+def test_backward_hooks_of_a_llama_block_change_their_branch_only(name):
+    """A hook that drops the gradient at a module's output drops that branch and keeps the skip connection."""
+    m, x, call = _small_block("llama", torch.bfloat16)
+    whole = torch.autograd.grad(call().sum(), x)[0]
+    h = m.get_submodule(name).register_full_backward_pre_hook(lambda mod, gy: tuple(torch.zeros_like(g) for g in gy))
+    cut = torch.autograd.grad(call().sum(), x)[0]
+    h.remove()
+    branch = m.self_attn if name in ("input_layernorm", "self_attn", "self_attn.o_proj") else m.mlp
+    forward = branch.forward
+    branch.forward = lambda *a, **k: forward(*a, **k).detach()               # the same by hand
+    want = torch.autograd.grad(call().sum(), x)[0]
+    assert torch.equal(cut, want) and not torch.equal(cut, whole)
