@@ -634,7 +634,7 @@ delta_scan_pair_kernel(const T* __restrict__ qkv, long ldq, int voff, const floa
 // are sums of three bf16 parts (24 bits), so all products are exact; the tensor core adds up the 16 products of one step and its parts, steps are
 // added in fp32 registers with rounding to nearest (the tensor core's accumulator cuts off).  Decays are products in token order as in
 // the scan (no logarithms).  T and M end at the diagonal: 0 times what is not finite would reach earlier tokens of the column, so columns
-// with such numbers (or beyond 1e37) take these two products from plain sums over s <= t.
+// where Y or U has such numbers (or beyond 1e37) take these two products from plain sums over s <= t.
 // The scan in pairs is a chain of 1150 cycles per two tokens on one warp per scheduler; here a warp's chunk is 360 products
 // (192 with the state, 36 + 36 with T and M, 96 for the update), 16 cycles each on its scheduler's tensor core: 7300 cycles per 32 tokens, and
 // a sequence's chunks are a chain.  [2560 tokens of 4 sequences up to 1024, 16 heads, 128 x 128]: 334 -> 143 us with the preparations (16); eight sequences
@@ -966,6 +966,10 @@ delta_chunk_scan_kernel(const bf16* __restrict__ qkv, long ldq, int koff, int vo
         }
       };
       times(x, p.tm, u);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) odd[e >> 1] = odd[e >> 1] || !(fabsf(u[i][e]) < 1e37f);
       float o[4][4] = {};
       times(u, p.tm + 3 * CL * CL_LD, o);
       const unsigned any = __ballot_sync(0xffffffffu, odd[0] || odd[1]);

@@ -481,6 +481,45 @@ def test_delta_scan_in_chunks_value_that_is_not_finite(value):
     assert not torch.isfinite(got[at:, 1, 5]).all() if value != 3e38 else torch.isfinite(got[at, 1, 5])
 
 
+def _delta_case(lens, heads, kv, d, v, shift):
+    n = sum(lens)
+    return (_rand((n, 2 * kv * d + heads * v), 1), (_rand((n, heads), 2).float() + shift).to(BF16), _rand((n, heads), 3), _rand((heads,), 4, 0.5),
+            _rand((heads,), 5, 0.5))
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("where", ["a", "b", "key", "query"])
+def test_delta_scan_in_chunks_input_that_is_not_finite(where, value):
+    """A gate, key or query that is not finite reaches no earlier token and no head that does not read it."""
+    from libai_b200.inference.ragged import RaggedBatch
+    from libai_b200.ops import seq_functional as SF
+
+    heads, kv, d, v, lens, at = 4, 2, 64, 72, [100, 90], 75
+    qkv, a, b, rate, bias = _delta_case(lens, heads, kv, d, v, 0.0)
+    rb = RaggedBatch(lens, [0, 1], [0, 0], "cuda")
+
+    def run(qkv, a, b):
+        S = torch.zeros(2, heads, d, v, device="cuda")
+        return SF.delta_scan(qkv, kv * d, 2 * kv * d, a, b, rate, bias, S, rb, kv, False).view(-1, heads, v), S
+
+    out, S = run(qkv, a, b)
+    x, ga, gb = qkv.clone(), a.clone(), b.clone()
+    hit = [2, 3]                                              # the second key head's
+    if where == "a":
+        ga[at, 2], hit = value, [2]
+    elif where == "b":
+        gb[at, 2], hit = -value, [2]
+    else:
+        x[at, (d if where == "query" else kv * d + d) + 5] = value
+    got, T = run(x, ga, gb)
+    rest = [h for h in range(heads) if h not in hit]
+    assert torch.equal(got[:, rest], out[:, rest]) and torch.equal(T[:, rest], S[:, rest])           # other heads
+    assert torch.equal(got[100:], out[100:]) and torch.equal(T[1], S[1])                             # the other sequence
+    assert torch.equal(got[:64], out[:64])                                                           # earlier chunks
+    # earlier tokens of the chunk may take their sums in another order
+    assert float((got[64:at, hit] - out[64:at, hit]).abs().max()) < 2.0 ** -20 * float(out[64:at].abs().max())
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, BF16])
 @pytest.mark.parametrize("n", [1, 17])
 def test_delta_scan_value_that_is_not_finite(n, dtype):
