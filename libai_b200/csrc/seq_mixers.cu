@@ -630,17 +630,22 @@ delta_scan_pair_kernel(const T* __restrict__ qkv, long ldq, int voff, const floa
 // A first kernel makes T, M and the decays of all chunks at once, the second walks a sequence's chunks with the state.  There a warp owns 16 columns
 // of Sᵀ in registers (accumulator layout of m16n8k16, 16 x 128 fp32), everything is transposed ([16 columns, tokens]) and each result is the
 // next product's A operand, so warps share staged operands only and a chunk needs one barrier.
-// Nothing that was fp32 is rounded: q and k are the bf16 numbers as they came (their lengths go into fp32 factors per token), the state, Y, U, T and M
-// are sums of three bf16 parts (24 bits), so all products are exact; the tensor core adds up the 16 products of one step and its parts, steps are
-// added in fp32 registers with rounding to nearest (the tensor core's accumulator cuts off).  Decays are products in token order as in
-// the scan (no logarithms).  T and M end at the diagonal: 0 times what is not finite would reach earlier tokens of the column, so columns
-// where Y or U has such numbers (or beyond 1e37) take these two products from plain sums over s <= t.
-// The scan in pairs is a chain of 1150 cycles per two tokens on one warp per scheduler; here a warp's chunk is 360 products
-// (192 with the state, 36 + 36 with T and M, 96 for the update), 16 cycles each on its scheduler's tensor core: 7300 cycles per 32 tokens, and
-// a sequence's chunks are a chain.  [2560 tokens of 4 sequences up to 1024, 16 heads, 128 x 128]: 334 -> 143 us with the preparations (16); eight sequences
-// of 1024: 680 -> 233.  Relative error of the read-outs against 64 bits 1.2e-7 to 1.5e-7 (pairs
-// 1.1e-7 to 1.4e-7), 1.2e-6 to 2.5e-6 for decays near one (pairs 0.7e-6 to 2.5e-6).  The same in fp32 on the FMA pipe (the inverse times
-// keys and values ahead of the scan, 4 x 4 tiles) took 333: 16-byte reads of shared memory bound it.
+// Precision.  q and k are the bf16 numbers as they came; the state, Y, U, T and M are sums of three bf16 parts (24 bits).  The tensor core cuts
+// its sums off at 24 bits instead of rounding them, which in a chain of such sums cost more than the scan's roundings.  So the products of
+// first parts leave it step by step and are added in fp32 registers with rounding to nearest, and only those of the smaller parts (2^-8 and below;
+// of two matrices in parts the last, 2^-32, is left out) are chained; T's diagonal, the largest term where decays are strong, is a
+// product on the FMA pipe with its error, and U stays two numbers until it is split.  Lengths, decays, their products, beta and the entries of T and M
+// are made once per chunk in 64 bits (1 / |k_t| is a factor of T's row t, so that U can be taken with the keys as they came).  Relative error against 64 bits, decays from strong to
+// near one, 64 to 1024 tokens: read-outs 0.7e-7 to 1.2e-7, states 0.4e-7 to 1.3e-7 (pairs 1.0e-7 to 2.6e-6, 0.7e-7 to 3.6e-6).
+// T and M end at the diagonal: 0 times what is not finite would reach earlier tokens of the column, so columns where Y or U has
+// such numbers (or beyond 1e37) take these two products from plain sums over s <= t.
+// The scan in pairs is a chain of 1150 cycles per two tokens on one warp per scheduler; here a warp's chunk is 384 products (192 with the state,
+// 48 + 48 with T and M, 96 for the update), 6150 cycles on its scheduler's tensor core at 16 each, of 9800 that a chunk takes: the rest are
+// the parts, sums and roundings between products that wait for one another, and a sequence's chunks are a chain.
+// [2560 tokens of 4 sequences up to 1024, 16 heads, 128 x 128]: 339 -> 201 us with the preparations (26) and inputs from memory; eight sequences of 1024:
+// 536 -> 269.  (All sums in the tensor core and the factors in fp32 took 158 and 237.)  Q S0 with the state's update instead of K S0: 184
+// instead of 166 us (registers).  The same in fp32 on the FMA pipe (the inverse times keys and values ahead of the scan, 4 x 4 tiles) took 333: 16-byte
+// reads of shared memory bound it.
 // ------------------------------------------------------------------------------------------------------------------
 constexpr int CL = 32;                       // tokens per chunk
 // Sequences from here on are scanned in chunks: one of 64 tokens takes 22 us both ways, eight of 64 29 against 41, one of 128 30 against 41,
@@ -649,8 +654,9 @@ constexpr int CL_MIN = 64;
 constexpr int CL_LD = CL + 8;                // row stride of 32 x 32 bf16 matrices in shared memory (ldmatrix without bank conflicts)
 constexpr int CL_WARPS = 4;                  // warps (of 16 columns) per block of the scan
 constexpr int CL_COLS = 16 * CL_WARPS;
-// scratch per (chunk, head), in floats: T and M as three bf16 parts each, then per token the factors of K S0, Q S0 and of u in the update, then G_L
-constexpr int CL_SCRATCH = 3 * CL * CL + 3 * CL + 32;
+// scratch per (chunk, head), in floats: T and M as three bf16 parts each, then per token the factors of K S0,
+// Q S0 and of u in the update and T's diagonal with its rest, then G_L
+constexpr int CL_SCRATCH = 3 * CL * CL + 5 * CL + 32;
 
 __device__ __forceinline__ uint32_t smem_at(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t at) {
@@ -660,27 +666,46 @@ __device__ __forceinline__ void ldsm4_trans(uint32_t (&r)[4], uint32_t at) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at));
 }
 __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// (x, y) as the sum of three pairs of bf16 numbers, largest first
-__device__ __forceinline__ void parts3(float x, float y, uint32_t (&p)[3]) {
+// a product by itself
+__device__ __forceinline__ void mma16816_new(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+// added to c with rounding to nearest (the tensor core's accumulator cuts off)
+__device__ __forceinline__ void add_mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  float y[4];
+  mma16816_new(y, a, b0, b1);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) c[e] += y[e];
+}
+// (x + xr, y + yr) as the sum of three pairs of bf16 numbers, largest first; the rests are small
+__device__ __forceinline__ void parts3(float x, float y, float xr, float yr, uint32_t (&p)[3]) {
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     const __nv_bfloat162 r = __floats2bfloat162_rn(x, y);
     p[i] = *reinterpret_cast<const uint32_t*>(&r);
     x -= __uint_as_float(p[i] << 16);
     y -= __uint_as_float(p[i] & 0xffff0000u);
+    if (i == 0) {
+      x += xr;
+      y += yr;
+    }
   }
 }
-// A operand of 16 rows and the 16 columns of two neighbouring accumulator tiles, in three parts
-__device__ __forceinline__ void a_parts(const float (&l)[4], const float (&r)[4], uint32_t (&a)[3][4]) {
+// A operand of 16 rows and the 16 columns of two neighbouring accumulator tiles (and their rests), in three parts
+__device__ __forceinline__ void a_parts(const float (&l)[4], const float (&r)[4], uint32_t (&a)[3][4], const float (&lr)[4] = {0.f, 0.f, 0.f, 0.f},
+                                        const float (&rr)[4] = {0.f, 0.f, 0.f, 0.f}) {
   uint32_t p[3];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const float x = i < 2 ? l[2 * (i & 1)] : r[2 * (i & 1)], y = i < 2 ? l[2 * (i & 1) + 1] : r[2 * (i & 1) + 1];
-    parts3(x, y, p);
+    const int at = 2 * (i & 1);
+    if (i < 2) parts3(l[at], l[at + 1], lr[at], lr[at + 1], p);
+    else parts3(r[at], r[at + 1], rr[at], rr[at + 1], p);
 #pragma unroll
     for (int e = 0; e < 3; ++e) a[e][i] = p[e];
   }
@@ -696,7 +721,7 @@ delta_chunk_prep_kernel(const bf16* __restrict__ qkv, long ldq, int koff, const 
   constexpr int LD = DP + 8;
   __shared__ __align__(16) bf16 sK[CL * LD], sQ[CL * LD];
   __shared__ float sKK[CL][CL + 1], sQK[CL][CL + 1], sA[4][CL][CL + 4];
-  __shared__ float ksc[CL], qsc[CL];
+  __shared__ double ksc[CL], qsc[CL];
   __shared__ int where[2];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, kh = blockIdx.y;
   if (warp == 0) {                           // the chunk's sequence
@@ -725,10 +750,11 @@ delta_chunk_prep_kernel(const bf16* __restrict__ qkv, long ldq, int koff, const 
   if (b < 0) return;
   const long tok0 = seq_off[b] + (long)where[1] * CL;
   const int nt = min(CL, (int)(seq_off[b + 1] - tok0));
-  for (int t = warp; t < CL; t += 4) {       // rows as they are, their lengths apart
-    float qq = 0.f, kk = 0.f;
+  for (int t = tid >> 3; t < CL; t += 16) {  // rows as they are, their lengths apart; eight lanes per row
+    double qq = 0.0, kk = 0.0;
     const bf16 *qr = qkv + (tok0 + t) * ldq + (long)kh * D, *kr = qr + koff;
-    for (int i = lane * 4; i < DP; i += 128) {
+#pragma unroll
+    for (int i = (tid & 7) * 4; i < DP; i += 32) {
       uint2 x = make_uint2(0u, 0u), y = x;
       if (t < nt && i < D) { x = *reinterpret_cast<const uint2*>(qr + i); y = *reinterpret_cast<const uint2*>(kr + i); }
       *reinterpret_cast<uint2*>(sQ + t * LD + i) = x;
@@ -736,20 +762,27 @@ delta_chunk_prep_kernel(const bf16* __restrict__ qkv, long ldq, int koff, const 
       const uint32_t xs[2] = {x.x, x.y}, ys[2] = {y.x, y.y};
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const float x0 = __uint_as_float(xs[e] << 16), x1 = __uint_as_float(xs[e] & 0xffff0000u);
-        const float y0 = __uint_as_float(ys[e] << 16), y1 = __uint_as_float(ys[e] & 0xffff0000u);
+        const double x0 = __uint_as_float(xs[e] << 16), x1 = __uint_as_float(xs[e] & 0xffff0000u);
+        const double y0 = __uint_as_float(ys[e] << 16), y1 = __uint_as_float(ys[e] & 0xffff0000u);
         qq += x0 * x0 + x1 * x1;
         kk += y0 * y0 + y1 * y1;
       }
     }
-    qq = warp_sum(qq);
-    kk = warp_sum(kk);
-    if (lane == 0) {
-      qsc[t] = (1.f / sqrtf((float)D)) / sqrtf(qq + 1e-6f);
-      ksc[t] = 1.f / sqrtf(kk + 1e-6f);
+#pragma unroll
+    for (int m = 4; m > 0; m >>= 1) {
+      qq += __shfl_xor_sync(0xffffffffu, qq, m);
+      kk += __shfl_xor_sync(0xffffffffu, kk, m);
+    }
+    if ((tid & 7) == 0) {
+      qsc[t] = qq;
+      ksc[t] = kk;
     }
   }
   __syncthreads();
+  if (tid < 2 * CL) {
+    double& sc = tid < CL ? qsc[tid] : ksc[tid - CL];
+    sc = 1.0 / sqrt((tid < CL ? D : 1) * (sc + 1e-6));
+  }
   {                                          // K Kᵀ (warps 0, 1) and Q Kᵀ (2, 3), 16 rows per warp
     const bf16* rows = warp < 2 ? sK : sQ;
     const int r0 = (warp & 1) * 16;
@@ -785,35 +818,41 @@ delta_chunk_prep_kernel(const bf16* __restrict__ qkv, long ldq, int koff, const 
     bf16* Tp = reinterpret_cast<bf16*>(mine);
     bf16* Mp = Tp + 3 * CL * CL;
     float* fac = mine + 3 * CL * CL;
-    float g = 1.f, beta = 0.f;               // of token `lane`
+    double g = 1.0, beta = 0.0;              // of token `lane`
     if (lane < nt) {
-      const float rate = expf(ldf(A_log + h));
-      g = expf(-rate * softplusf_(ldf(a + (tok0 + lane) * lda + h) + ldf(dt_bias + h)));
-      beta = sigmoidf_(ldf(bl + (tok0 + lane) * ldb + h));
+      const double z = static_cast<double>(ldf(a + (tok0 + lane) * lda + h)) + ldf(dt_bias + h);
+      g = exp(-exp(static_cast<double>(ldf(A_log + h))) * (z > 40.0 ? z : log1p(exp(z))));
+      beta = 1.0 / (1.0 + exp(-static_cast<double>(ldf(bl + (tok0 + lane) * ldb + h))));
     }
-    float x = 0.f, all = 1.f, G = 1.f;       // γ(t, lane); products of all decays up to t
-    const float ks = ksc[lane];
-    auto store3 = [&](bf16* p, float v) {
+    double x = 0.0, all = 1.0, G = 1.0;      // γ(t, lane); products of all decays up to t
+    const double ks = ksc[lane];
+    auto store3 = [&](bf16* p, double v) {
+      float x = static_cast<float>(v);
+      const float rest = static_cast<float>(v - x);
 #pragma unroll
       for (int e = 0; e < 3; ++e) {
-        const bf16 r = __float2bfloat16_rn(v);
+        const bf16 r = __float2bfloat16_rn(x);
         p[e * CL * CL] = r;
-        v -= __bfloat162float(r);
+        x -= __bfloat162float(r);
+        if (e == 0) x += rest;
       }
     };
 #pragma unroll 4
     for (int t = 0; t < CL; ++t) {
-      const float gt = __shfl_sync(0xffffffffu, g, t), bt = __shfl_sync(0xffffffffu, beta, t);
-      x = t == lane ? 1.f : (t > lane ? x * gt : 0.f);
+      const double gt = __shfl_sync(0xffffffffu, g, t), bt = __shfl_sync(0xffffffffu, beta, t);
+      x = t == lane ? 1.0 : (t > lane ? x * gt : 0.0);
       all *= gt;
       if (t == lane) G = all;
-      sA[warp][t][lane] = lane < t ? bt * (x * (ksc[t] * ks * sKK[t][lane])) : 0.f;
-      store3(Mp + t * CL + lane, lane <= t ? x * (qsc[t] * ks * sQK[t][lane]) : 0.f);
+      sA[warp][t][lane] = lane < t ? static_cast<float>(bt * x * (ksc[t] * ks) * sKK[t][lane]) : 0.f;
+      store3(Mp + t * CL + lane, lane <= t ? x * qsc[t] * sQK[t][lane] : 0.0);
     }
-    fac[lane] = G * ks;
-    fac[CL + lane] = G * qsc[lane];
-    fac[2 * CL + lane] = x * ks;             // (tokens behind the end decay by 1)
-    if (lane == 0) fac[3 * CL] = all;
+    fac[lane] = static_cast<float>(G * ks);
+    fac[CL + lane] = static_cast<float>(G * qsc[lane]);
+    fac[2 * CL + lane] = static_cast<float>(x);        // (tokens behind the end decay by 1)
+    const double diag = beta * ks;
+    fac[3 * CL + lane] = static_cast<float>(diag);
+    fac[4 * CL + lane] = static_cast<float>(diag - static_cast<float>(diag));
+    if (lane == 0) fac[5 * CL] = static_cast<float>(all);
     __syncwarp();
     float col[CL];                           // column `lane` of (I + A)^-1
 #pragma unroll
@@ -822,7 +861,7 @@ delta_chunk_prep_kernel(const bf16* __restrict__ qkv, long ldq, int koff, const 
 #pragma unroll
       for (int s = 0; s < t; ++s) acc[s & 3] += sA[warp][t][s] * col[s];
       col[t] = t == lane ? 1.f : (t > lane ? -((acc[0] + acc[1]) + (acc[2] + acc[3])) : 0.f);
-      store3(Tp + t * CL + lane, t >= lane ? col[t] * beta : 0.f);
+      store3(Tp + t * CL + lane, t > lane ? ksc[t] * col[t] * beta : 0.0);
     }
     __syncwarp();
   }
@@ -833,7 +872,7 @@ struct DeltaChunkStage {
   bf16 k[CL * (DP + 8)], q[CL * (DP + 8)];
   bf16 tm[6 * CL * CL_LD];                   // T, M: three parts each
   bf16 v[CL * (CL_COLS + 8)];
-  float fac[3 * CL + 4];
+  float fac[5 * CL + 4];
 };
 template <int DP>
 struct DeltaChunkSmem {
@@ -894,7 +933,7 @@ delta_chunk_scan_kernel(const bf16* __restrict__ qkv, long ldq, int koff, int vo
       const bool in = t < nt && j0 + j < V;
       cp_async16(p.v + t * VLD + j, qkv + (in ? (tok + t) * ldq + voff + (long)h * V + j0 + j : 0), in ? 16 : 0);
     }
-    if (tid < (3 * CL + 4) / 4) cp_async16(p.fac + 4 * tid, w + 3 * CL * CL + 4 * tid, 16);
+    if (tid < (5 * CL + 4) / 4) cp_async16(p.fac + 4 * tid, w + 3 * CL * CL + 4 * tid, 16);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
   const int chunks = (n + CL - 1) / CL;
@@ -906,7 +945,7 @@ delta_chunk_scan_kernel(const bf16* __restrict__ qkv, long ldq, int koff, int vo
     const DeltaChunkStage<DP>& p = sm.st[c & 1];
     const int nt = min(CL, n - c * CL);
     // ---- S0ᵀ [Kᵀ Qᵀ]: [16, 32 + 32]
-    float x[8][4] = {};
+    float x[8][4] = {}, xl[8][4] = {};       // sums of the first parts; of the smaller ones
 #pragma unroll
     for (int kk = 0; kk < DP / 16; ++kk) {
       uint32_t am[3][4];
@@ -916,15 +955,17 @@ delta_chunk_scan_kernel(const bf16* __restrict__ qkv, long ldq, int koff, int vo
         uint32_t bm[4];
         ldsm4(bm, smem_at((n2 < 2 ? p.k : p.q) + ((n2 & 1) * 16 + (lane & 7) + (lane >> 4) * 8) * LD + kk * 16 + ((lane >> 3) & 1) * 8));
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          float y[4] = {};
+        for (int i = 0; i < 2; ++i) mma16816(xl[n2 * 2 + i], am[2], bm[2 * i], bm[2 * i + 1]);
 #pragma unroll
-          for (int e = 2; e >= 0; --e) mma16816(y, am[e], bm[2 * i], bm[2 * i + 1]);
+        for (int i = 0; i < 2; ++i) add_mma16816(x[n2 * 2 + i], am[0], bm[2 * i], bm[2 * i + 1]);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) x[n2 * 2 + i][e] += y[e];
-        }
+        for (int i = 0; i < 2; ++i) mma16816(xl[n2 * 2 + i], am[1], bm[2 * i], bm[2 * i + 1]);
       }
     }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[i][e] += xl[i][e];
     // ---- Y = V - G K S0; O starts with G Q S0
     bool odd[2] = {false, false};            // columns g, g + 8 with a number that is not finite or close to that
 #pragma unroll
@@ -932,14 +973,13 @@ delta_chunk_scan_kernel(const bf16* __restrict__ qkv, long ldq, int koff, int vo
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int t = 8 * i + q2 + (e & 1);
-        x[i][e] = __bfloat162float(p.v[t * VLD + warp * 16 + g + 8 * (e >> 1)]) - p.fac[t] * x[i][e];
-        x[4 + i][e] *= p.fac[CL + t];
+        x[i][e] = fmaf(-p.fac[t], x[i][e], __bfloat162float(p.v[t * VLD + warp * 16 + g + 8 * (e >> 1)]));
         odd[e >> 1] = odd[e >> 1] || !(fabsf(x[i][e]) < 1e37f);
       }
-    float u[4][4] = {};
+    float u[4][4] = {}, ur[4][4] = {};       // U and what its rounding left
     {
-      // D += [16, 32] (as A, three parts) times the three parts of a lower triangular matrix at `tri`
-      auto times = [&](const float (*y)[4], const bf16* tri, float (&d)[4][4]) {
+      // D + R = [16, 32] (as A, three parts) times the three parts of a lower triangular matrix at `tri`; R is small
+      auto times = [&](const float (*y)[4], const bf16* tri, float (&d)[4][4], float (&r)[4][4]) {
 #pragma unroll
         for (int kk = 0; kk < 2; ++kk) {
           uint32_t am[3][4];
@@ -951,33 +991,48 @@ delta_chunk_scan_kernel(const bf16* __restrict__ qkv, long ldq, int koff, int vo
             for (int e = 0; e < 3; ++e)
               ldsm4(bm[e], smem_at(tri + (e * CL + n2 * 16 + (lane & 7) + (lane >> 4) * 8) * CL_LD + kk * 16 + ((lane >> 3) & 1) * 8));
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {    // the smaller products first
-              float z[4] = {};
-              mma16816(z, am[2], bm[0][2 * i], bm[0][2 * i + 1]);
-              mma16816(z, am[1], bm[1][2 * i], bm[1][2 * i + 1]);
-              mma16816(z, am[0], bm[2][2 * i], bm[2][2 * i + 1]);
-              mma16816(z, am[1], bm[0][2 * i], bm[0][2 * i + 1]);
-              mma16816(z, am[0], bm[1][2 * i], bm[1][2 * i + 1]);
-              mma16816(z, am[0], bm[0][2 * i], bm[0][2 * i + 1]);
+            for (int i = 0; i < 2; ++i) add_mma16816(d[n2 * 2 + i], am[0], bm[0][2 * i], bm[0][2 * i + 1]);
 #pragma unroll
-              for (int e = 0; e < 4; ++e) d[n2 * 2 + i][e] += z[e];
-            }
+            for (int order = 3; order > 0; --order)          // the smaller products first
+#pragma unroll
+              for (int e = 2; e >= 0; --e)
+                if (order - e >= 0 && order - e <= 2) {
+#pragma unroll
+                  for (int i = 0; i < 2; ++i) mma16816(r[n2 * 2 + i], am[e], bm[order - e][2 * i], bm[order - e][2 * i + 1]);
+                }
           }
         }
       };
-      times(x, p.tm, u);
+      times(x, p.tm, u, ur);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) odd[e >> 1] = odd[e >> 1] || !(fabsf(u[i][e]) < 1e37f);
+        for (int e = 0; e < 4; ++e) {        // the diagonal, exact; sum with its rounding error
+          const int t = 8 * i + q2 + (e & 1);
+          const float own = p.fac[3 * CL + t] * x[i][e], sum = u[i][e] + own, back = sum - u[i][e];
+          ur[i][e] += fmaf(p.fac[3 * CL + t], x[i][e], -own) + p.fac[4 * CL + t] * x[i][e] + ((u[i][e] - (sum - back)) + (own - back));
+          u[i][e] = sum;
+          odd[e >> 1] = odd[e >> 1] || !(fabsf(sum) < 1e37f);
+        }
       float o[4][4] = {};
-      times(u, p.tm + 3 * CL * CL_LD, o);
+      {
+        float y[4][4], low[4][4] = {};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) y[i][e] = u[i][e] + ur[i][e];
+        times(y, p.tm + 3 * CL * CL_LD, o, low);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) o[i][e] += low[i][e];
+      }
       const unsigned any = __ballot_sync(0xffffffffu, odd[0] || odd[1]);
       if (any == 0) {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) x[4 + i][e] += o[i][e];
+          for (int e = 0; e < 4; ++e) x[4 + i][e] = fmaf(p.fac[CL + 8 * i + q2 + (e & 1)], x[4 + i][e], o[i][e]);
       } else {
 #pragma unroll
         for (int r = 0; r < 2; ++r) odd[r] = (__ballot_sync(0xffffffffu, odd[r]) >> (lane & ~3) & 15u) != 0;
@@ -994,7 +1049,8 @@ delta_chunk_scan_kernel(const bf16* __restrict__ qkv, long ldq, int koff, int vo
             const int col = at & 15, t = at / 16;
             float sum = 0.f;
             for (int s = 0; s <= t; ++s) {
-              const float m = (__bfloat162float(tri[(2 * CL + t) * CL_LD + s]) + __bfloat162float(tri[(CL + t) * CL_LD + s])) + __bfloat162float(tri[t * CL_LD + s]);
+              const float m = !pass && s == t ? p.fac[3 * CL + t]
+                                              : (__bfloat162float(tri[(2 * CL + t) * CL_LD + s]) + __bfloat162float(tri[(CL + t) * CL_LD + s])) + __bfloat162float(tri[t * CL_LD + s]);
               sum += m * (pass ? us[col][s] : ys[col][s]);
             }
             if (pass) ys[col][t] = sum; else us[col][t] = sum;
@@ -1006,8 +1062,11 @@ delta_chunk_scan_kernel(const bf16* __restrict__ qkv, long ldq, int koff, int vo
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const int t = 8 * i + q2 + (e & 1), col = g + 8 * (e >> 1);
-            if (odd[e >> 1]) u[i][e] = us[col][t];
-            x[4 + i][e] += odd[e >> 1] ? ys[col][t] : o[i][e];
+            if (odd[e >> 1]) {
+              u[i][e] = us[col][t];
+              ur[i][e] = 0.f;
+            }
+            x[4 + i][e] = fmaf(p.fac[CL + t], x[4 + i][e], odd[e >> 1] ? ys[col][t] : o[i][e]);
           }
         __syncwarp();
       }
@@ -1018,29 +1077,38 @@ delta_chunk_scan_kernel(const bf16* __restrict__ qkv, long ldq, int koff, int vo
       for (int e = 0; e < 4; ++e) {
         const int t = 8 * i + q2 + (e & 1), col = jc + 8 * (e >> 1);
         if (t < nt && col < V) out[(tok0 + c * CL + t) * (long)(H * V) + (long)h * V + col] = x[4 + i][e];
-        u[i][e] = t < nt ? u[i][e] * p.fac[2 * CL + t] : 0.f;
+        const float f = p.fac[2 * CL + t], w = u[i][e] * f, wr = fmaf(u[i][e], f, -w) + ur[i][e] * f;
+        u[i][e] = t < nt ? w : 0.f;
+        ur[i][e] = t < nt && fabsf(w) < 1e37f ? wr : 0.f;
       }
     // ---- Sᵀ <- G_L Sᵀ + Uᵀ K
-    const float gl = p.fac[3 * CL];
+    const float gl = p.fac[5 * CL];
     uint32_t am[2][3][4];
 #pragma unroll
-    for (int kk = 0; kk < 2; ++kk) a_parts(u[2 * kk], u[2 * kk + 1], am[kk]);
+    for (int kk = 0; kk < 2; ++kk) a_parts(u[2 * kk], u[2 * kk + 1], am[kk], ur[2 * kk], ur[2 * kk + 1]);
 #pragma unroll
     for (int d2 = 0; d2 < DP / 16; ++d2) {
-      float y[2][4] = {};
+      uint32_t bm[2][4];
 #pragma unroll
-      for (int kk = 0; kk < 2; ++kk) {
-        uint32_t bm[4];
-        ldsm4_trans(bm, smem_at(p.k + (kk * 16 + (lane & 15)) * LD + d2 * 16 + (lane >> 4) * 8));
+      for (int kk = 0; kk < 2; ++kk) ldsm4_trans(bm[kk], smem_at(p.k + (kk * 16 + (lane & 15)) * LD + d2 * 16 + (lane >> 4) * 8));
+      // the smaller parts and the earlier tokens, the state, then the later tokens
+      float y[2][4], z[2][4];
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+      for (int i = 0; i < 2; ++i) mma16816_new(z[i], am[1][0], bm[1][2 * i], bm[1][2 * i + 1]);
 #pragma unroll
-          for (int e = 2; e >= 0; --e) mma16816(y[i], am[kk][e], bm[2 * i], bm[2 * i + 1]);
-      }
+      for (int i = 0; i < 2; ++i) mma16816_new(y[i], am[0][2], bm[0][2 * i], bm[0][2 * i + 1]);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) mma16816(y[i], am[1][2], bm[1][2 * i], bm[1][2 * i + 1]);
+#pragma unroll
+      for (int kk = 1; kk >= 0; --kk)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) mma16816(y[i], am[kk][1], bm[kk][2 * i], bm[kk][2 * i + 1]);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) mma16816(y[i], am[0][0], bm[0][2 * i], bm[0][2 * i + 1]);
 #pragma unroll
       for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) st[2 * d2 + i][e] = fmaf(gl, st[2 * d2 + i][e], y[i][e]);
+        for (int e = 0; e < 4; ++e) st[2 * d2 + i][e] = fmaf(gl, st[2 * d2 + i][e], y[i][e]) + z[i][e];
     }
   }
 #pragma unroll

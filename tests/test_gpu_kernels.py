@@ -487,6 +487,27 @@ def _delta_case(lens, heads, kv, d, v, shift):
             _rand((heads,), 5, 0.5))
 
 
+@pytest.mark.parametrize("shift", [-8.0, -3.0, 0.0, 5.0])
+@pytest.mark.parametrize("lens,heads,kv,d,v", [([257, 130], 4, 2, 128, 128), ([88, 96, 97, 640], 2, 2, 64, 64)])
+def test_delta_scan_in_chunks_is_as_exact_as_token_by_token(lens, heads, kv, d, v, shift):
+    """The same numbers in rows off the vectors' alignment are scanned token by token in fp32: chunks are no further from 64 bits."""
+    from libai_b200.inference.ragged import RaggedBatch
+    from libai_b200.ops import seq_functional as SF
+
+    qkv, a, b, rate, bias = _delta_case(lens, heads, kv, d, v, shift)
+    start = _rand((len(lens), heads, d, v), 6, 1.0, torch.float32)
+    want, final = _delta64(qkv, a, b, rate, bias, start, lens, heads, kv, d, v)
+    rb = RaggedBatch(lens, list(range(len(lens))), [1] * len(lens), "cuda")
+    wide = torch.zeros(qkv.shape[0], qkv.shape[1] + 3, device="cuda", dtype=BF16)
+    wide[:, :-3] = qkv
+    errors = []
+    for rows in (qkv, wide[:, :-3]):
+        S = start.clone()
+        out = SF.delta_scan(rows, kv * d, 2 * kv * d, a, b, rate, bias, S, rb, kv, False)
+        errors.append((float((out.double() - want).norm() / want.norm()), float((S.double() - final).norm() / final.norm())))
+    assert errors[0][0] <= errors[1][0] and errors[0][1] <= errors[1][1], errors
+
+
 @pytest.mark.parametrize("value", [float("nan"), float("inf")])
 @pytest.mark.parametrize("where", ["a", "b", "key", "query"])
 def test_delta_scan_in_chunks_input_that_is_not_finite(where, value):
