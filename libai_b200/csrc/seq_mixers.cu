@@ -11,6 +11,7 @@
 // arithmetic is fp32.  This file is built WITHOUT fast-math: the fp32 mode is meant to be exact to rounding.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+#include <float.h>
 #include <math.h>
 #include <stdint.h>
 
@@ -773,15 +774,21 @@ delta_chunk_prep_kernel(const bf16* __restrict__ qkv, long ldq, int koff, const 
       qq += __shfl_xor_sync(0xffffffffu, qq, m);
       kk += __shfl_xor_sync(0xffffffffu, kk, m);
     }
+    // lengths beyond what fp32 squares hold: such a vector counts as zero, as in the scan token by token (not where an element is infinite)
+    const bool q0 = qq > FLT_MAX && qq < INFINITY, k0 = kk > FLT_MAX && kk < INFINITY;
+    for (int i = (tid & 7) * 4; i < DP; i += 32) {
+      if (q0) *reinterpret_cast<uint2*>(sQ + t * LD + i) = make_uint2(0u, 0u);
+      if (k0) *reinterpret_cast<uint2*>(sK + t * LD + i) = make_uint2(0u, 0u);
+    }
     if ((tid & 7) == 0) {
-      qsc[t] = qq;
-      ksc[t] = kk;
+      qsc[t] = q0 ? -1.0 : qq;
+      ksc[t] = k0 ? -1.0 : kk;
     }
   }
   __syncthreads();
-  if (tid < 2 * CL) {
+  if (tid < 2 * CL) {                        // -0: counts as zero
     double& sc = tid < CL ? qsc[tid] : ksc[tid - CL];
-    sc = 1.0 / sqrt((tid < CL ? D : 1) * (sc + 1e-6));
+    sc = sc < 0.0 ? -0.0 : 1.0 / sqrt((tid < CL ? D : 1) * (sc + 1e-6));
   }
   {                                          // K Kᵀ (warps 0, 1) and Q Kᵀ (2, 3), 16 rows per warp
     const bf16* rows = warp < 2 ? sK : sQ;
@@ -973,7 +980,9 @@ delta_chunk_scan_kernel(const bf16* __restrict__ qkv, long ldq, int koff, int vo
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int t = 8 * i + q2 + (e & 1);
+        if (__float_as_uint(p.fac[t]) == 0x80000000u) x[i][e] = 0.f;
         x[i][e] = fmaf(-p.fac[t], x[i][e], __bfloat162float(p.v[t * VLD + warp * 16 + g + 8 * (e >> 1)]));
+        if (__float_as_uint(p.fac[CL + t]) == 0x80000000u) x[4 + i][e] = 0.f;
         odd[e >> 1] = odd[e >> 1] || !(fabsf(x[i][e]) < 1e37f);
       }
     float u[4][4] = {}, ur[4][4] = {};       // U and what its rounding left

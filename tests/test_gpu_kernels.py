@@ -541,6 +541,23 @@ def test_delta_scan_in_chunks_input_that_is_not_finite(where, value):
     assert float((got[64:at, hit] - out[64:at, hit]).abs().max()) < 2.0 ** -20 * float(out[64:at].abs().max())
 
 
+def test_delta_scan_in_chunks_vectors_beyond_fp32_squares():
+    """A key or query whose squares overflow counts as zero, as in the scan token by token."""
+    from libai_b200.inference.ragged import RaggedBatch
+    from libai_b200.ops import seq_functional as SF
+
+    heads, kv, d, v, n = 2, 1, 128, 64, 110
+    qkv, a, b, rate, bias = _delta_case([n], heads, kv, d, v, 0.0)
+    rb, results = RaggedBatch([n], [0], [1], "cuda"), []
+    for size in (0.0, 2e38):
+        x = qkv.clone()
+        x[40, d:2 * d] = size                                 # key
+        x[70, :d] = -size                                     # query
+        S = _rand((1, heads, d, v), 6, 1.0, torch.float32)
+        results.append((SF.delta_scan(x, kv * d, 2 * kv * d, a, b, rate, bias, S, rb, kv, False), S))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, BF16])
 @pytest.mark.parametrize("n", [1, 17])
 def test_delta_scan_value_that_is_not_finite(n, dtype):
