@@ -649,9 +649,10 @@ delta_scan_pair_kernel(const T* __restrict__ qkv, long ldq, int voff, const floa
 // reads of shared memory bound it.
 // ------------------------------------------------------------------------------------------------------------------
 constexpr int CL = 32;                       // tokens per chunk
-// Sequences from here on are scanned in chunks: one of 64 tokens takes 22 us both ways, eight of 64 29 against 41, one of 128 30 against 41,
-// eight of 256 64 against 134 (16 heads of 128 x 128).
-constexpr int CL_MIN = 64;
+// Sequences from here on are scanned in chunks.  Three chunks take what pairs take for 85 to 88 tokens where a batch is small: one sequence of 80 tokens 28.2
+// against 26.9 us, of 96 28.3 against 31.2 (16 heads of 128 x 128); 21.3 against 19.7, 21.5 against 22.8 (8 of 64 x 64).  Of many the chunks are
+// ahead from 64 on (32 of 64: 82 against 130), but a sequence's result must not depend on the others.
+constexpr int CL_MIN = 88;
 constexpr int CL_LD = CL + 8;                // row stride of 32 x 32 bf16 matrices in shared memory (ldmatrix without bank conflicts)
 constexpr int CL_WARPS = 4;                  // warps (of 16 columns) per block of the scan
 constexpr int CL_COLS = 16 * CL_WARPS;
