@@ -116,9 +116,6 @@ attn_fwd_v2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   const int q_blk = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x);
   const int head = blockIdx.y, batch = blockIdx.z;
   const int q0 = q_blk * ATT_BM;
-  const int kv_len = p.kv_lens != nullptr ? max(1, min(p.S, p.kv_lens[batch])) : p.S;
-  int nkv = (kv_len + ATT_BN - 1) / ATT_BN;
-  if (p.causal) nkv = min(nkv, q_blk + 1);
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmap_q);
@@ -144,8 +141,11 @@ attn_fwd_v2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
-  chain_wait();
+  chain_wait();                      // (the lengths may be what the kernel before wrote: every warp has to see the same trip counts)
   chain_next();
+  const int kv_len = p.kv_lens != nullptr ? max(1, min(p.S, p.kv_lens[batch])) : p.S;
+  int nkv = (kv_len + ATT_BN - 1) / ATT_BN;
+  if (p.causal) nkv = min(nkv, q_blk + 1);
 
   if (warp_idx == 0) {
     if (elect_one()) {
@@ -587,7 +587,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   const int warp_idx = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int kv_blk = blockIdx.x, head = blockIdx.y, batch = blockIdx.z;
   const int k0 = kv_blk * 128;
-  const int kv_len = p.kv_lens != nullptr ? max(1, min(p.S, p.kv_lens[batch])) : p.S;
   const int nq = (p.S + 127) / 128;
   const int i_begin = p.causal ? kv_blk : 0;
   const int iters = nq - i_begin;
@@ -618,6 +617,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   const uint32_t tmem_base = *tmem_ptr_smem;
   chain_wait();
   chain_next();
+  const int kv_len = p.kv_lens != nullptr ? max(1, min(p.S, p.kv_lens[batch])) : p.S;
 
   if (warp_idx == 0) {
     if (elect_one()) {
@@ -988,7 +988,6 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   const int warp_idx = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int kv_blk = blockIdx.x, head = blockIdx.y, batch = blockIdx.z;
   const int k0 = kv_blk * 128;
-  const int kv_len = p.kv_lens != nullptr ? max(1, min(p.S, p.kv_lens[batch])) : p.S;
   const int nq = (p.S + 127) / 128;
   const int i_begin = p.causal ? kv_blk : 0;
   const int iters = nq - i_begin;
@@ -1024,6 +1023,7 @@ attn_bwd_pipe_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   const uint32_t tmem_base = *tmem_ptr_smem;
   chain_wait();
   chain_next();
+  const int kv_len = p.kv_lens != nullptr ? max(1, min(p.S, p.kv_lens[batch])) : p.S;
   constexpr int CW0 = REGS ? 4 : 2;    // first softmax warp
   if constexpr (REGS) {
     if (warp_idx < CW0) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;\n");

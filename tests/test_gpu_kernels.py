@@ -955,3 +955,36 @@ def test_many_rows_against_one_tile_of_columns(m, n, k):
     bound = want.abs() * 2.0 ** -8 + (x.double().abs() @ w.double().abs().T + b.double().abs()) * k * 2.0 ** -23
     assert bool(((y.double() - want).abs() <= bound).all())
     assert float((y.double() - want).norm() / want.norm()) < 2.0 ** -8
+
+
+@pytest.mark.parametrize("dim,b,s,a,biased,causal", [(64, 3, 100, 4, False, False), (64, 5, 128, 2, False, True), (128, 2, 384, 4, False, False), (64, 2, 304, 3, True, False),
+                                                     (128, 2, 264, 2, True, True), (64, 4, 520, 2, False, False)])
+def test_attention_lengths_written_by_the_launch_before(dim, b, s, a, biased, causal):
+    """Key lengths, and the memory they are in, change right before the kernel that reads them: the same bits as with a wait in between, forward and
+    backward (without a bias), one and two tiles per block."""
+    qkv = _rand((b, s, a, 3 * dim), 1)
+    q, k, v = (t.permute(0, 2, 1, 3) for t in qkv.split(dim, -1))
+    bias = _rand((b, a, s, s), 2) if biased else None
+    go, base, n = _rand((b, s, a, dim), 3), torch.arange(b, device="cuda", dtype=torch.int32) * 17, torch.empty(b, device="cuda", dtype=torch.int32)
+
+    def run(wait):
+        out = []
+        for i in range(6):
+            torch.add(base, 1 + s * i // 6, out=n)
+            if wait:
+                torch.cuda.synchronize()
+            if biased:
+                o, lse, _ = load_ext().attn_fwd(q, k, v, causal, dim ** -0.5, n, bias, None, 0.0, 0)
+                out += [o, lse]
+            else:
+                x = qkv.detach().requires_grad_(True)
+                o = OF.attention_qkvpacked(x, causal=causal, scale=dim ** -0.5, kv_lens=n)
+                out += [o.detach(), *(torch.autograd.grad(o, x, go)[0].split(dim, -1)[1:])]           # dK and dV have a fixed order
+            if wait:
+                torch.cuda.synchronize()
+        return out
+
+    want = run(True)
+    for _ in range(3):
+        assert all(torch.equal(x, y) for x, y in zip(run(False), want))
+    assert not torch.equal(want[0], want[-2 if biased else -3])
