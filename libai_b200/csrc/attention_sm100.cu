@@ -1396,8 +1396,8 @@ attn_dq_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict_
     for (int u = 0; u < 2; ++u) {
       const long i = i0 + u * stride;
       if (i < nvec) {
-        lo[u] = __ldg(reinterpret_cast<const float4*>(acc) + 2 * i);
-        hi[u] = __ldg(reinterpret_cast<const float4*>(acc) + 2 * i + 1);
+        lo[u] = reinterpret_cast<const float4*>(acc)[2 * i];
+        hi[u] = reinterpret_cast<const float4*>(acc)[2 * i + 1];
       }
     }
 #pragma unroll

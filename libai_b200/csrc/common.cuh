@@ -104,7 +104,8 @@ LB_DEVICE uint4 philox4x32_7(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3,
 // ---------------------------------------------------------------------------------------------
 // Launches that overlap the end of the kernel before them (lb_host::launch_chained below).  chain_wait() returns once that kernel has completed and
 // its writes can be seen: before it a kernel touches no global memory.  It takes the pointers that the kernel loads from through
-// `const __restrict__` parameters, whose loads the compiler could move in front of it otherwise.  chain_next() lets the next
+// `const __restrict__` parameters: the compiler could otherwise move their loads in front of it or make them ld.global.nc, which wants memory that
+// nobody writes while the kernel runs, and a chained kernel runs while the one before still writes (so no __ldg in one either).  chain_next() lets the next
 // kernel's blocks start, as soon as every block of this one has got there: behind a block's allocation of TMEM, which the next kernel's blocks
 // must not take from it.  A kernel that waits for other ranks or streams never calls it (the next one would hold an SM meanwhile).
 // What it gives: 1 to 3 us per launch (block of GPT-2 against a cache, 7 launches: 58 -> 45 us; block of Llama, 10 launches: 170 -> 150 us; [8, 1024] GPT-2

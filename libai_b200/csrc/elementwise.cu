@@ -13,7 +13,7 @@
 namespace lb {
 
 LB_DEVICE void ld8(const __nv_bfloat16* p, float (&v)[8]) {
-  uint4 q = __ldg(reinterpret_cast<const uint4*>(p));
+  const uint4 q = *reinterpret_cast<const uint4*>(p);
   float2 a = unpack_bf16(q.x), b = unpack_bf16(q.y), c = unpack_bf16(q.z), d = unpack_bf16(q.w);
   v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = c.x; v[5] = c.y; v[6] = d.x; v[7] = d.y;
 }
@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(256) ce_stats_kernel(const T* __restrict__ log
       for (; c + (G - 1) * STEP < V; c += G * STEP) {
         uint4 q[G];
 #pragma unroll
-        for (int k = 0; k < G; ++k) q[k] = __ldg(reinterpret_cast<const uint4*>(lr + c + k * STEP));
+        for (int k = 0; k < G; ++k) q[k] = *reinterpret_cast<const uint4*>(lr + c + k * STEP);
         __nv_bfloat162 pm = *reinterpret_cast<const __nv_bfloat162*>(&q[0].x);
 #pragma unroll
         for (int k = 0; k < G; ++k) {

@@ -547,7 +547,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     int acc = 0;
     uint32_t acc_phase = 0;
     float alpha = 1.0f;
-    if constexpr (FP8) alpha = __ldg(p.deq_a) * __ldg(p.deq_b);
+    if constexpr (FP8) alpha = *p.deq_a * *p.deq_b;       // (written by the launches before: ordinary loads behind chain_wait)
     if (cp.mode == COMM_RS) {
       // write-after-read on the owners' staging buffers: every owner must have retired its previous call on this
       // buffer set (its reduce phase read what we stored then) before the first partial tile of this call lands

@@ -17,7 +17,7 @@ struct Vec8;
 template <>
 struct Vec8<__nv_bfloat16> {
   static LB_DEVICE void load(const __nv_bfloat16* p, float (&v)[8]) {
-    uint4 q = __ldg(reinterpret_cast<const uint4*>(p));
+    const uint4 q = *reinterpret_cast<const uint4*>(p);
     float2 a = unpack_bf16(q.x), b = unpack_bf16(q.y), c = unpack_bf16(q.z), d = unpack_bf16(q.w);
     v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = c.x; v[5] = c.y; v[6] = d.x; v[7] = d.y;
   }
@@ -29,7 +29,7 @@ struct Vec8<__nv_bfloat16> {
 template <>
 struct Vec8<float> {
   static LB_DEVICE void load(const float* p, float (&v)[8]) {
-    float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p + 4));
+    const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
   }
   static LB_DEVICE void store(float* p, const float (&v)[8]) {
@@ -336,7 +336,7 @@ norm_fwd_wide_kernel(const __nv_bfloat16* __restrict__ x, const W* __restrict__ 
 #pragma unroll
     for (int i = 0; i < V; ++i) {
       const int c = (i * NORM_WIDE_THREADS + threadIdx.x) * 8;
-      q[i] = c < H ? __ldg(reinterpret_cast<const uint4*>(x + base + c)) : make_uint4(0, 0, 0, 0);
+      q[i] = c < H ? *reinterpret_cast<const uint4*>(x + base + c) : make_uint4(0, 0, 0, 0);
     }
     float mean = 0.f;
     if (!RMS) {

@@ -988,3 +988,67 @@ def test_attention_lengths_written_by_the_launch_before(dim, b, s, a, biased, ca
     for _ in range(3):
         assert all(torch.equal(x, y) for x, y in zip(run(False), want))
     assert not torch.equal(want[0], want[-2 if biased else -3])
+
+
+def _waiting():
+    """Mode that waits for the device after every operator."""
+    class Waiting(torch.utils._python_dispatch.TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            out = func(*args, **(kwargs or {}))
+            torch.cuda.synchronize()
+            return out
+
+    return Waiting()
+
+
+def _chain_fp8():
+    out, w = [], _rand((264, 512), 9)
+    for i, (m, size) in enumerate([(300, 1.0), (300, 40.0), (64, 0.01), (300, 7.0), (2000, 300.0)]):
+        xq, dx = load_ext().quantize_e4m3(_rand((m, 512), i, size))
+        wq, dw = load_ext().quantize_e4m3(w * (i + 1))
+        out.append(load_ext().linear_fp8_fwd(xq, wq, dx, dw, None, 0, False, None)[0])
+    return out
+
+
+def _chain_loss():
+    from libai_b200.layers import LMLogits, ParallelCrossEntropyLoss
+
+    out, w = [], _rand((4104, 256), 1, 0.05).requires_grad_(True)
+    for i, m in enumerate([700, 33, 700, 1500]):
+        x = _rand((1, m, 256), 2 + i).requires_grad_(True)
+        labels = torch.randint(0, 4104, (1, m), device="cuda", generator=torch.Generator("cuda").manual_seed(i))
+        loss = ParallelCrossEntropyLoss()(LMLogits(4104)(x, w), labels)
+        out += [loss.detach(), torch.autograd.grad(loss.sum(), x)[0]]
+    return out
+
+
+def _chain_attention(drop):
+    out = []
+    for i, (s, d) in enumerate([(136, 64), (264, 128), (520, 64), (136, 64)]):
+        torch.manual_seed(i)
+        q, k, v = (t + 0.25 for t in _rand((2, 4, 3 * s, d), i).split(s, 2))
+        bias = None if drop else _rand((1, 4, s, s), 7 + i) * 2.0
+        out.append(OF.attention(q, k, v, causal=True, bias=bias, dropout_p=0.2 * drop, training=bool(drop)))
+    return out
+
+
+def _chain_block(dim):
+    m, x, out = _gpt_block(4, dim), _rand((3, 200, 4 * dim), 1).requires_grad_(True), []
+    y = x
+    for _ in range(4):
+        y = m(y)
+        out.append(y.detach())
+    y.sum().backward()                              # the kernels in a row; its sums over blocks have no fixed order
+    return out
+
+
+@pytest.mark.parametrize("chain", [_chain_fp8, _chain_loss, lambda: _chain_attention(0), lambda: _chain_attention(1), lambda: _chain_block(64),
+                                   lambda: _chain_block(128)], ids=["fp8", "loss", "bias", "dropout", "block 64", "block 128"])
+def test_inputs_written_by_the_launch_before(chain):
+    """Scales, logits, scores' bias and activations straight from the kernel before, in memory that was something else a moment ago: the same bits as
+    with a wait after every operator."""
+    with _waiting():
+        want = chain()
+    for _ in range(3):
+        got = chain()
+        assert len(got) == len(want) and all(torch.equal(a, b) for a, b in zip(got, want))
