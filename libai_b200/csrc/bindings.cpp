@@ -316,6 +316,9 @@ Tensor dgrad_actgrad(const Tensor& gy, const Tensor& w, const Tensor& pre, int64
   return out;
 }
 
+// The GEMM's epilogue loads a residual in vectors of 16 bytes; a block's input may be a view that begins anywhere.
+Tensor in_vectors(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) != 0 ? t.clone() : t; }
+
 // y = x @ w^T + bias + residual (one kernel)
 Tensor linear_bias_residual(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& bias, const Tensor& residual) {
   TORCH_CHECK(x.is_cuda() && x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1), "linear_bias_residual: shape mismatch");
@@ -325,6 +328,7 @@ Tensor linear_bias_residual(const Tensor& x, const Tensor& w, const c10::optiona
   const int64_t M = x.size(0), K = x.size(1), N = w.size(0);
   TORCH_CHECK(residual.dim() == 2 && residual.size(0) == M && residual.size(1) == N, "linear_bias_residual: residual must be [M, N]");
   c10::cuda::CUDAGuard guard(x.device());
+  const Tensor res = in_vectors(residual);
   Tensor y = at::empty({M, N}, x.options());
   const void* bias_ptr = nullptr;
   if (bias.has_value() && bias->defined()) {
@@ -332,7 +336,7 @@ Tensor linear_bias_residual(const Tensor& x, const Tensor& w, const c10::optiona
     bias_ptr = bias->data_ptr();
   }
   check(lb_gemm_bf16_bias_residual(x.data_ptr(), w.data_ptr(), y.data_ptr(), (int)M, (int)N, (int)K, (int)x.stride(0),
-                                   (int)w.stride(0), bias_ptr, residual.data_ptr(), cur_stream()),
+                                   (int)w.stride(0), bias_ptr, res.data_ptr(), cur_stream()),
         "linear_bias_residual");
   return y;
 }
@@ -393,14 +397,14 @@ std::tuple<Tensor, Tensor> linear_fp8_fwd(const Tensor& xq, const Tensor& wq, co
     TORCH_CHECK(bias->scalar_type() == at::kBFloat16 && bias->numel() == N, "linear_fp8_fwd: bias must be bf16 [N]");
     bias_ptr = bias->data_ptr();
   }
-  const void* res_ptr = nullptr;
+  Tensor res;
   if (residual.has_value() && residual->defined()) {
     TORCH_CHECK(residual->scalar_type() == at::kBFloat16 && residual->is_contiguous() && residual->numel() == M * N,
                 "linear_fp8_fwd: residual must be contiguous bf16 [M, N]");
-    res_ptr = residual->data_ptr();
+    res = in_vectors(*residual);
   }
   check(lb_gemm_fp8(xq.data_ptr(), wq.data_ptr(), y.data_ptr(), (int)M, (int)N, (int)K, bias_ptr, (int)act,
-                    pre.defined() ? pre.data_ptr() : nullptr, res_ptr, deq_x.data_ptr<float>(), deq_w.data_ptr<float>(),
+                    pre.defined() ? pre.data_ptr() : nullptr, res.defined() ? res.data_ptr() : nullptr, deq_x.data_ptr<float>(), deq_w.data_ptr<float>(),
                     cur_stream()),
         "linear_fp8_fwd");
   return std::make_tuple(y, pre.defined() ? pre : at::empty({0}, opts));

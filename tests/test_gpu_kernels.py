@@ -1052,3 +1052,26 @@ def test_inputs_written_by_the_launch_before(chain):
     for _ in range(3):
         got = chain()
         assert len(got) == len(want) and all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("rows", [3, 200, 2100])
+def test_residual_that_begins_anywhere(rows):
+    """A block's input may be a view off the vectors of 16 bytes that the epilogue loads: few rows and many, fp8, and a whole block forward and backward."""
+    h, k = 192, 256
+    x, w, b, flat = _rand((rows, k), 1), _rand((h, k), 2, 0.1), _rand((h,), 3), _rand((rows * h + 8,), 4)
+    xq, dx = load_ext().quantize_e4m3(x)
+    wq, dw = load_ext().quantize_e4m3(w)
+    for off in (1, 2, 4):
+        view = flat[off:off + rows * h].view(rows, h)
+        assert view.data_ptr() % 16
+        assert torch.equal(load_ext().linear_bias_residual(x, w, b, view), load_ext().linear_bias_residual(x, w, b, view.clone()))
+        assert torch.equal(load_ext().linear_fp8_fwd(xq, wq, dx, dw, b, 0, False, view)[0], load_ext().linear_fp8_fwd(xq, wq, dx, dw, b, 0, False, view.clone())[0])
+    if rows == 200:
+        m, (cos, sin) = _llama_block(3, 64, False), _ROT(256, 64)
+        results = []
+        for x in (flat[3:3 + rows * h].view(1, rows, h), flat[3:3 + rows * h].view(1, rows, h).clone()):
+            x = x.detach().requires_grad_(True)
+            y = m(x, cos_cached=cos, sin_cached=sin)
+            results.append((y.detach().double(), torch.autograd.grad(y, x, y.detach())[0].double()))
+        for got, want in zip(*results):              # another norm kernel reads rows off their alignment: roundings of its result (2^-8) through the block
+            assert float((got - want).norm()) < 2.0 ** -6 * float(want.norm())
