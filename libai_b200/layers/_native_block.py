@@ -37,14 +37,14 @@ def _calls_are_seen() -> bool:
 
 
 def plain(m, cls) -> bool:
-    """A module of this very class whose call is its class's ``forward`` and nothing else (``alone`` asks for what holds for all modules, too)."""
-    return (type(m) is cls and cls.forward is _FORWARDS[cls] and not m._forward_hooks and not m._forward_pre_hooks and not m._backward_hooks
-            and not m._backward_pre_hooks and m._compiled_call_impl is None and "forward" not in m.__dict__)
+    """A module of this very class whose call without a graph is its class's ``forward`` and nothing else."""
+    return (type(m) is cls and cls.forward is _FORWARDS[cls] and not m._forward_hooks and not m._forward_pre_hooks and m._compiled_call_impl is None
+            and "forward" not in m.__dict__)
 
 
 def alone(m, cls) -> bool:
-    """Would nobody notice if this module were passed by, its work joined with a neighbour's, graph or not?"""
-    return plain(m, cls) and not _calls_are_seen()
+    """Would nobody notice if this module were passed by, its work joined with a neighbour's, with a graph or without?"""
+    return plain(m, cls) and not m._backward_hooks and not m._backward_pre_hooks and not _calls_are_seen()
 
 
 def parameters(*pairs):
