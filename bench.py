@@ -1,8 +1,8 @@
 #!/usr/bin/env python
 """Headline benchmark: GPT-2 pre-training throughput (tokens/s) on N B200 GPUs of one node.
 
-Model/config = the reference's published GPT-2 benchmark (docs Benchmark.md:20-26, BASELINE.md rows
-6-8: 24 layers, hidden 1024, 16 heads, seq 1024, data parallel, micro-batch per GPU fixed → weak
+Model/config = the reference's published GPT-2 benchmark (docs Benchmark.md:20-26:
+24 layers, hidden 1024, 16 heads, seq 1024, data parallel, micro-batch per GPU fixed → weak
 scaling), bf16 compute with fp32 master weights, synthetic tokens, random-init weights.
 
     python bench.py --gpus 1 --steps 20 --warmup 5
@@ -29,10 +29,10 @@ import time
 REPO = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, REPO)
 
-# published LiBai numbers for the GPT-2 data-parallel rows (samples/s × 1024 tokens), BASELINE.md #6-#8
+# published LiBai numbers for the GPT-2 data-parallel rows (samples/s × 1024 tokens)
 PUBLISHED_TOKENS_PER_S = {1: 17940.0, 4: 64973.0, 8: 128655.0}
 
-# benchmark models: the headline (gpt2 = the reference's benchmark GPT-2) and the other BASELINE.json configs
+# benchmark models: the headline (gpt2 = the reference's benchmark GPT-2) and the other recipes
 MODELS = {
     "gpt2": dict(cfg="configs/gpt2_synthetic.py", layers=24, hidden=1024, heads=16, seq=1024, micro=8, unit="tokens/s",
                  name="GPT-2 nl{layers} h{hidden} a{heads} (reference benchmark model, ~355M params)"),
@@ -55,7 +55,7 @@ def parse_args():
     ap.add_argument("--impl", default="native", choices=["native", "ref", "reference"])
     ap.add_argument("--model", default="gpt2", choices=sorted(MODELS),
                     help="gpt2 (default, the headline: reference benchmark GPT-2 nl24 h1024) | gpt2_large | bert_large | "
-                         "llama7b | vit_l — the other BASELINE.json configs; metric stays tokens/s (images/s for vit_l)")
+                         "llama7b | vit_l — the other recipes; metric stays tokens/s (images/s for vit_l)")
     ap.add_argument("--micro-batch", type=int, default=0, help="samples per GPU per step (0 = the model's default)")
     ap.add_argument("--layers", type=int, default=0)
     ap.add_argument("--hidden", type=int, default=0)
@@ -661,10 +661,9 @@ def main():
         watch.idle()
 
     if args.extras and args.impl == "native" and args.model == "gpt2" and not args.layout and args.tp == 1 and args.pp == 1:
-        # the model-parallel layouts that fit this GPU count, same global batch, same launch (
-        # "TP=2 DP=4", "TP=2 PP=2 DP=2 + ZeRO-1").  They run LAST and under a watchdog: the headline measurement above
-        # is already complete, and a failure (or a hang) in an extra layout on any rank ends every rank cleanly with
-        # the line printed — it must never take the headline down.
+        # the model-parallel layouts that fit this GPU count, same global batch, same launch ("TP=2 DP=4", "TP=2 PP=2 DP=2 +
+        # ZeRO-1").  They run LAST and under a watchdog: the headline measurement above is already complete, and a failure (or a
+        # hang) in an extra layout on any rank ends every rank cleanly with the line printed — it must never take the headline down.
         names = {2: ["tp2"], 4: ["tp2", "3d"], 8: ["tp2", "3d"]}.get(world, [])
         for name in names:
             lay = layout_of(args, world, name)

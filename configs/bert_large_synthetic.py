@@ -1,5 +1,5 @@
 """BERT-large pre-training on synthetic tokens: the reference's benchmark BERT (docs Benchmark.md:13-19: 24 layers,
-hidden 1024, 16 heads, seq 512; BASELINE.json config "BERT-large pretrain TP=2 DP=4 bf16") with random-init weights."""
+hidden 1024, 16 heads, seq 512; "BERT-large pretrain TP=2 DP=4 bf16") with random-init weights."""
 from libai_b200.config import LazyCall, OmegaConf
 from libai_b200.data import build_nlp_test_loader, build_nlp_train_loader
 from libai_b200.data.datasets import SyntheticBertDataset

@@ -1,4 +1,4 @@
-"""ViT-Large/16 on synthetic 224×224 images (BASELINE.json config "ViT-Large configs/vit_imagenet.py DP=8 synthetic
+"""ViT-Large/16 on synthetic 224×224 images ("ViT-Large configs/vit_imagenet.py DP=8 synthetic
 224×224 images/sec"): the vit_imagenet recipe with ``vit_large_patch16_224`` and generated data."""
 from libai_b200.config import LazyCall, OmegaConf
 from libai_b200.data.build import build_image_test_loader, build_image_train_loader

@@ -928,7 +928,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 
 // =================================================================================================
 // Backward, pipelined variant (D = 64).  Same maths and the same tiles as attn_bwd_kernel; what changes is who waits
-// for whom.  ncu of the kernel above (profiles/r17_ncu_summary.md): tensor pipe 17 %, issue slots 18 % — the chain
+// for whom.  ncu of the kernel above: tensor pipe 17 %, issue slots 18 % — the chain
 // S,dP → softmax → dV,dK,dQ → dQ drain → next S,dP ran strictly in sequence.  Here
 //   * 16 softmax warps (4 per TMEM lane quadrant, 32 key columns each): a thread holds its whole share of S and dP in
 //     64 registers, so the S/dP columns are handed back to the MMA warp right after the two tcgen05.ld — the tensor core

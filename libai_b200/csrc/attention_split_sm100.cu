@@ -821,7 +821,7 @@ extern "C" int lb_attn_split_bwd(const void* dout, const void* q, const void* k,
   if (e != cudaSuccess) return (int)e;
   blocks = (rows * d / 8 + 255) / 256;
   if (blocks > 148L * 8) blocks = 148L * 8;
-  lb::attn_split_dq_kernel<<<dim3((unsigned)blocks), 256, 0, s>>>(dq_acc, (__nv_bfloat16*)dq, B, A, Sq, d, dqs[0], dqs[1], dqs[2], key_blocks,
+  lb::attn_split_dq_kernel<<<(unsigned)blocks, 256, 0, s>>>(dq_acc, (__nv_bfloat16*)dq, B, A, Sq, d, dqs[0], dqs[1], dqs[2], key_blocks,
                                                               causal, Sk - Sq);
   return (int)cudaGetLastError();
 }

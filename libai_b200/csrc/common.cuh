@@ -30,7 +30,7 @@ LB_DEVICE bool elect_one() {
 
 // ---------------------------------------------------------------------------------------------
 // cross-GPU flag waits (NVLink peer memory).  Every wait is BOUNDED: a dead or wedged peer must not hang the GPU
-// forever (SURVEY §5.3) — after `timeout_ns` the waiter prints who/what it was waiting for and traps, which surfaces
+// forever — after `timeout_ns` the waiter prints who/what it was waiting for and traps, which surfaces
 // as a CUDA error on the host (the trainer's emergency path / the launcher's restart then take over).
 // ---------------------------------------------------------------------------------------------
 LB_DEVICE unsigned long long globaltimer_ns() {
@@ -249,7 +249,7 @@ LB_DEVICE void tmem_dealloc_2cta(uint32_t taddr) {
 }
 // arrive (count 1) on the mbarrier at the same shared-memory offset in CTA `cta` of the cluster (the form CUTLASS'
 // ClusterBarrier::arrive(cta_id) uses; with an explicit `.release.cluster` per arrival the peer's TMA producer was measured
-// throttled to one k-block per arrival: profiles/r2_10_ncu_gemm_2cta_first.txt)
+// throttled to one k-block per arrival)
 LB_DEVICE void mbar_arrive_cluster(uint64_t* bar, uint32_t cta) {
   asm volatile(
       "{\n\t.reg .b32 ra;\n\t"

@@ -708,27 +708,27 @@ extern "C" int lb_bias_dropout_residual(const void* x, const void* bias, const v
 extern "C" int lb_swiglu_fwd(const void* gate, const void* up, void* y, long n, cudaStream_t s) {
   if (n % 8) return -1;
   if (n == 0) return 0;
-  lb::swiglu_fwd_kernel<<<dim3(ew_grid(n / 8, 256)), 256, 0, s>>>((const bf16*)gate, (const bf16*)up, (bf16*)y, n / 8);
+  lb::swiglu_fwd_kernel<<<ew_grid(n / 8, 256), 256, 0, s>>>((const bf16*)gate, (const bf16*)up, (bf16*)y, n / 8);
   return (int)cudaGetLastError();
 }
 extern "C" int lb_swiglu_bwd(const void* gy, const void* gate, const void* up, void* dgate, void* dup, long n,
                              cudaStream_t s) {
   if (n % 8) return -1;
   if (n == 0) return 0;
-  lb::swiglu_bwd_kernel<<<dim3(ew_grid(n / 8, 256)), 256, 0, s>>>((const bf16*)gy, (const bf16*)gate, (const bf16*)up,
+  lb::swiglu_bwd_kernel<<<ew_grid(n / 8, 256), 256, 0, s>>>((const bf16*)gy, (const bf16*)gate, (const bf16*)up,
                                                             (bf16*)dgate, (bf16*)dup, n / 8);
   return (int)cudaGetLastError();
 }
 extern "C" int lb_swiglu_packed_fwd(const void* gu, void* y, long rows, long F, cudaStream_t s) {
   if (F % 8) return -1;
   if (rows == 0) return 0;
-  lb::swiglu_packed_fwd_kernel<<<dim3(ew_grid(rows * F / 8, 256)), 256, 0, s>>>((const bf16*)gu, (bf16*)y, (size_t)rows, (size_t)(F / 8));
+  lb::swiglu_packed_fwd_kernel<<<ew_grid(rows * F / 8, 256), 256, 0, s>>>((const bf16*)gu, (bf16*)y, (size_t)rows, (size_t)(F / 8));
   return (int)cudaGetLastError();
 }
 extern "C" int lb_swiglu_packed_bwd(const void* gy, const void* gu, void* dgu, long rows, long F, cudaStream_t s) {
   if (F % 8) return -1;
   if (rows == 0) return 0;
-  lb::swiglu_packed_bwd_kernel<<<dim3(ew_grid(rows * F / 8, 256)), 256, 0, s>>>((const bf16*)gy, (const bf16*)gu, (bf16*)dgu,
+  lb::swiglu_packed_bwd_kernel<<<ew_grid(rows * F / 8, 256), 256, 0, s>>>((const bf16*)gy, (const bf16*)gu, (bf16*)dgu,
                                                                          (size_t)rows, (size_t)(F / 8));
   return (int)cudaGetLastError();
 }

@@ -297,7 +297,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     // pushes of call n-1, which we issue after our call n-2 kernel ended, so nobody still reads parity (n-2).
     // `copy_rings` independent engines per copy CTA (lane 0 of the first warps), each with its own slice of the
     // (otherwise idle) pipeline smem as a 6-slot ring and its own mbarriers: one engine alone is latency bound
-    // (~1.6 us per 32 KB chunk, ~20 GB/s — profiles/r2_04_comm_bench_2gpu.json).
+    // (~1.6 us per 32 KB chunk, ~20 GB/s).
     const int n_rings = cp.copy_rings > 0 ? cp.copy_rings : 1;
     if (lane == 0 && warp_idx < n_rings) {
       // 12 slots; at most LOADS_AHEAD loads (local, L2-resident source: fast) and up to NSLOT - LOADS_AHEAD stores (the
@@ -651,7 +651,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
             // partial tile -> this rank's OWN partial-product buffer [M, N] (peer-mapped): the epilogue runs at local
             // HBM speed; the owners pull the rows they own during their reduce phase with wide coalesced loads and the
             // whole GPU's memory-level parallelism (P2P stores of 64-byte row segments from the epilogue throttled the
-            // GEMM itself: profiles/r2_04_comm_bench_2gpu.json)
+            // GEMM itself)
             slab = cp.peer_buf[cp.rank] + cp.staging_parity_off + static_cast<size_t>(slab_row0) * p.N + col0;
             ld = static_cast<size_t>(p.N);
           }
@@ -731,7 +731,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     // ---------------- reduce phase: out[r, :] = sum_src staging[src][r, :] (+ bias) (+ residual) ----------------
     // Bandwidth bound (world + 2 streams of rows_per_rank x N bf16), one CTA per SM: every thread keeps UNR row
     // vectors x (sources + residual) 16-byte loads in flight — with one vector at a time this phase was latency bound
-    // and cost more than the GEMM it follows (profiles/r2_04_comm_bench_2gpu.json).
+    // and cost more than the GEMM it follows.
     constexpr int UNR = 4;
     const int col_groups = (p.N + 255) / 256;
     const int units = mbpr * col_groups;
@@ -1114,7 +1114,7 @@ static int gemm_impl(const void* a, const void* b, void* out, int M, int N, int 
   if (epi == 2 && p.k_splits == 1 && wgrad_rmw()) {
     // a single K partition owns the whole tile: accumulate with a plain read-modify-write instead of L2 atomics.
     // Off by default since the epilogue became coalesced: `red.add.v4` is fire-and-forget, while the read of the old
-    // tile sits exposed at the end of a one-tile-per-CTA GEMM (profiles/r28_wgrad_sweep.json: 4096x1024x8192
+    // tile sits exposed at the end of a one-tile-per-CTA GEMM (4096x1024x8192
     // 2-way split with red.add 54 us vs single partition with rmw 67 us).  LIBAI_B200_WGRAD_RMW=1 restores it.
     epi = 1;
     p.rmw = 1;
@@ -1132,7 +1132,7 @@ static int gemm_impl(const void* a, const void* b, void* out, int M, int N, int 
 
   // CTA pairs (cta_group::2, 256 x 256 tiles, each CTA stages half of B) for the plain bf16 GEMMs whose tile width is
   // 256: 10-27 % faster than the single-CTA tiles on the benchmark shapes (8192^3 0.71 vs 0.81 ms, LM head 0.64 vs
-  // 0.81 ms, profiles/r2_11_kernel_check_gemm_2cta.json).  LIBAI_B200_GEMM_2CTA=0 keeps everything on single-CTA tiles.
+  // 0.81 ms).  LIBAI_B200_GEMM_2CTA=0 keeps everything on single-CTA tiles.
   const int allow_2cta = gemm_allow_2cta();
   // (fused collectives: shards must hold whole 256-row pair tiles and the copy CTAs come in pairs)
   const bool comm_ok = cp.mode == lb::COMM_NONE ||

@@ -179,7 +179,7 @@ norm_bwd_kernel(const T* __restrict__ gy, const T* __restrict__ x, const W* __re
 // bf16 activations, bandwidth-oriented variant of the kernel above (same maths, same outputs).  The first version kept
 // x̂ and g·γ of a row as 2 x VPL x 8 floats across the two warp reductions and fetched the residual gradient afterwards:
 // 191 registers → one 8-warp block per SM, and three dependent memory phases per row — 19 µs for [8192, 1024] where
-// the 64 MB it moves take 9 µs (profiles/r2_20_step_breakdown.md).  Here a row's x, gy and residual gradient are
+// the 64 MB it moves take 9 µs.  Here a row's x, gy and residual gradient are
 // fetched together as raw 16-byte vectors (3 x VPL x 4 registers), unpacked twice (before and after the reductions:
 // ALU is free here), and blocks are 4 warps at <= 168 registers → 12 warps per SM with 12 loads each in flight.
 constexpr int NORM_BWD_WARPS = 4;

@@ -175,8 +175,8 @@ class StepTrainer(TrainerBase):
         pass of the last micro-batch (the fused NVLink reduce-scatter of the already-final part of the gradient buffer
         starts at a few block boundaries).  Measured on B200 it does NOT pay for the 345M benchmark model: the
         end-of-step reduction costs ~1 ms at 8 GPUs (97 % weak scaling without overlap), while the extra side-stream
-        kernels, their flag exchanges and the added host work cost more (2 GPUs 29.4 → 30.0 ms, 8 GPUs 29.9 → 35.3 ms;
-        `profiles/r20_*`, `profiles/r21_*`).  Kept for models whose gradient volume per step is much larger."""
+        kernels, their flag exchanges and the added host work cost more (2 GPUs 29.4 → 30.0 ms, 8 GPUs 29.9 →
+        35.3 ms).  Kept for models whose gradient volume per step is much larger."""
         if not hasattr(self, "_overlap_layers"):
             self._overlap_layers = ()
             model = self.model.module if hasattr(self.model, "module") else self.model

@@ -47,7 +47,7 @@ def impl() -> str:
 class _FastOps:
     """``torch.ops.libai_b200`` with every operator resolved once to its ``.default`` overload.  Calling the
     ``OpOverloadPacket`` (what ``torch.ops.ns.name(...)`` is) re-resolves the overload on every call — a few
-    microseconds of Python per kernel launch, ~600 times per training step (``profiles/r23_host_profile.txt``)."""
+    microseconds of Python per kernel launch, ~600 times per training step."""
 
     def __init__(self, namespace):
         self._ns = namespace
@@ -208,7 +208,7 @@ def bump_fp8_weight_epoch() -> None:
 # --------------------------------------------------------------------------------------
 # bias gradient of the MLP's first linear inside the dgrad epilogue (GEMM column sums via red.add)
 # --------------------------------------------------------------------------------------
-_FUSED_BIAS_GRAD = os.environ.get("LIBAI_B200_FUSED_BIAS_GRAD", "1") == "1"   # +0.8 % on the step in a same-box A/B (profiles/r2_28_*)
+_FUSED_BIAS_GRAD = os.environ.get("LIBAI_B200_FUSED_BIAS_GRAD", "1") == "1"   # +0.8 % on the step in a same-box A/B
 
 
 def fused_bias_grad() -> bool:

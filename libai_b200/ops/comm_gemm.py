@@ -29,7 +29,7 @@ _BM = 128
 
 def _n_comm_ctas(world: int) -> int:
     """Copy CTAs of the AG kernels: each streams ~200 KB in flight through its TMA ring; more destinations → more CTAs."""
-    return 24 if world <= 4 else 32      # measured: profiles/r2_04_comm_bench_2gpu.json (8: 132 us, 16: 71, 24: 69, 32: 65, 48: 73)
+    return 24 if world <= 4 else 32      # measured on two GPUs (8: 132 us, 16: 71, 24: 69, 32: 65, 48: 73)
 
 
 class _TPState:
@@ -88,7 +88,7 @@ def fused_supported(M: int, N: int, K: int, world: int) -> bool:
 
 # Keep all_gather(x) of the forward for the weight gradient (one device copy of [tokens, h] per column-parallel linear
 # and layer) instead of gathering x a second time inside the wgrad kernel: trades b·s·h·2 bytes of activation memory per
-# column-parallel linear for ~35 us of exposed NVLink synchronisation per wgrad (profiles/r2_06_comm_bench_2gpu.json:
+# column-parallel linear for ~35 us of exposed NVLink synchronisation per wgrad (two GPUs:
 # AG->wgrad 80 us vs plain wgrad 42 us at 16k tokens).  ``LIBAI_B200_SP_SAVE_GATHERED=0`` restores the re-gather
 # (Megatron's sequence-parallel memory profile).
 import os as _os
@@ -139,7 +139,7 @@ def ag_gemm(x_shard: torch.Tensor, w: torch.Tensor, bias, act, group, layout: in
     if fill_local:
         # the local rows of the gathered buffer are only needed by LATER kernels of this stream (the wgrad that reuses
         # all_gather(dy)): a plain device copy at HBM speed (~6 us per 16 MB) instead of a second job for the copy
-        # CTAs, whose throughput is what the kernel waits for (profiles/r2_04_comm_bench_2gpu.json)
+        # CTAs, whose throughput is what the kernel waits for
         gathered[st.rank * rows : (st.rank + 1) * rows].copy_(x_shard)
         count_launch()
     y, pre = ext.ag_gemm(

@@ -2,7 +2,7 @@
 
 Each function dispatches to the native sm_100a kernels for CUDA tensors and to the PyTorch
 reference otherwise (see :mod:`libai_b200.ops`).  The reference call sites these replace are the
-OneFlow fused ops listed in SURVEY.md §2.4: ``flow._C.layer_norm_affine`` / ``rms_norm``
+OneFlow fused ops ``flow._C.layer_norm_affine`` / ``rms_norm``
 (libai/layers/layer_norm.py:78-131), ``fused_bias_add_gelu`` (libai/layers/mlp.py:95),
 ``fused_bias_add_dropout`` (libai/layers/mlp.py:104, attention.py:265),
 ``fused_scale_mask_softmax_dropout`` / ``fused_scale_tril_softmax_mask_scale``
@@ -455,7 +455,7 @@ def bias_gelu(x, bias):
 
 
 def tp_rng_salt(sharded: bool) -> int:
-    """Salt of the dropout RNG stream (TP-aware RNG).  All tensor-parallel ranks of a model replica share
+    """Salt of the dropout RNG stream (tensor-parallel aware).  All tensor-parallel ranks of a model replica share
     one (seed, offset) sequence (``dutil.model_parallel_seed``); activations that are *sharded* over the TP group
     (attention heads, token shards under sequence parallelism) must see different masks on different ranks → the TP
     rank is mixed into the Philox key; *replicated* activations (salt 0) get identical masks everywhere."""

@@ -63,7 +63,7 @@ class _Group:
             # in-switch sums (multimem.ld_reduce), the parameter all-gather is one multimem.st per vector.  Off by default:
             # a reduce-SCATTER through the switch still has every GPU send its whole buffer (only the inbound side
             # shrinks), so it cannot beat the unicast pull on full-duplex links; measured on 2 GPUs 26.9 vs 26.2 ms per
-            # step (profiles/r2_26_*), bit-identical results.
+            # step, bit-identical results.
             nvls = os.environ.get("LIBAI_B200_NVLS", "0") == "1" and self.dtype == torch.bfloat16
             pbuf = symm_ws.buffer(("zero_param", index, self.numel, nvls), self.numel * params[0].element_size(), multicast=nvls)
             gbuf = symm_ws.buffer(("zero_grad", index, self.numel, nvls), self.numel * 4, multicast=nvls)

@@ -1,4 +1,4 @@
-"""Llama-2 7B shaped pre-training on synthetic tokens (BASELINE.json config "Llama-2 7B projects/Llama TP=4 DP=2 +
+"""Llama-2 7B shaped pre-training on synthetic tokens ("Llama-2 7B projects/Llama TP=4 DP=2 +
 ZeRO-2"): 32 layers, hidden 4096, 32 heads, SwiGLU 11008, seq 2048, random-init weights."""
 from libai_b200.config import LazyCall, OmegaConf
 from libai_b200.data import build_nlp_test_loader, build_nlp_train_loader
