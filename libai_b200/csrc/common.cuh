@@ -112,8 +112,8 @@ LB_DEVICE uint4 philox4x32_7(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3,
 // block forward and backward: 858 -> 809 us of GPU time).  What it takes: blocks are handed out while the SMs come free one after the other, so the
 // first ones get as many as fit.  Kernels that plan for an even spread lose more than they gain and are launched in order, without chain_wait(): norms
 // whose blocks take several rows in turn, norm backward ([12608, 1024] 25 us, chained 29), gated products ([2048, 11008] backward 40, chained 47),
-// attention backward with 512 blocks, longest first (185, chained 201), the sum over dQ's layers (22.1, chained 23.7), the delta rule's scan over chunks (133, chained
-// 192: two long sequences on one SM).
+// attention backward with 512 blocks, longest first (185, chained 201), the sum over dQ's layers (22.1, chained 23.7), the delta rule's scan over chunks (133 in its
+// first form, chained 192: two long sequences on one SM).
 // ---------------------------------------------------------------------------------------------
 template <typename... P>
 LB_DEVICE void chain_wait(P&... loaded) {
