@@ -635,30 +635,30 @@ delta_scan_pair_kernel(const T* __restrict__ qkv, long ldq, int voff, const floa
 // its sums off at 24 bits instead of rounding them, which in a chain of such sums cost more than the scan's roundings.  So the products of
 // first parts leave it step by step and are added in fp32 registers with rounding to nearest, and only those of the smaller parts (2^-8 and below;
 // of two matrices in parts the last, 2^-32, is left out) are chained; T's diagonal, the largest term where decays are strong, is a
-// product on the FMA pipe with its error, and U stays two numbers until it is split.  Lengths, decays, their products, beta and the entries of T and M
-// are made once per chunk in 64 bits (1 / |k_t| is a factor of T's row t, so that U can be taken with the keys as they came).  Relative error against 64 bits, decays from strong to
-// near one, 64 to 1024 tokens: read-outs 0.7e-7 to 1.2e-7, states 0.4e-7 to 1.3e-7 (pairs 1.0e-7 to 2.6e-6, 0.7e-7 to 3.6e-6).
+// product on the FMA pipe.  Lengths, decays, their products, beta and the entries of T and M are made once per chunk in 64 bits (1 / |k_t| is a factor of
+// T's row t, so that U can be taken with the keys as they came).  Relative error against 64 bits, decays from strong to
+// near one, 100 to 1024 tokens: read-outs 0.8e-7 to 1.4e-7, states 0.5e-7 to 1.4e-7 (pairs 1.0e-7 to 2.6e-6, 0.7e-7 to 3.6e-6).  With the diagonal's
+// error and U as two numbers 0.7e-7 to 1.2e-7 and 0.4e-7 to 1.3e-7, but 166 instead of 128 us (registers).
 // T and M end at the diagonal: 0 times what is not finite would reach earlier tokens of the column, so columns where Y or U has
 // such numbers (or beyond 1e37) take these two products from plain sums over s <= t.
 // The scan in pairs is a chain of 1150 cycles per two tokens on one warp per scheduler; here a warp's chunk is 384 products (192 with the state,
-// 48 + 48 with T and M, 96 for the update), 6150 cycles on its scheduler's tensor core at 16 each, of 9800 that a chunk takes: the rest are
+// 48 + 48 with T and M, 96 for the update), 6150 cycles on its scheduler's tensor core at 16 each, of 7900 that a chunk takes: the rest are
 // the parts, sums and roundings between products that wait for one another, and a sequence's chunks are a chain.
-// [2560 tokens of 4 sequences up to 1024, 16 heads, 128 x 128]: 339 -> 201 us with the preparations (26) and inputs from memory; eight sequences of 1024:
-// 536 -> 269.  (All sums in the tensor core and the factors in fp32 took 158 and 237.)  Q S0 with the state's update instead of K S0: 184
-// instead of 166 us (registers).  The same in fp32 on the FMA pipe (the inverse times keys and values ahead of the scan, 4 x 4 tiles) took 333: 16-byte
-// reads of shared memory bound it.
+// [2560 tokens of 4 sequences up to 1024, 16 heads, 128 x 128]: 339 -> 165 us with the preparations (25) and inputs from memory; eight sequences of 1024:
+// 536 -> 248.  Q S0 with the state's update instead of K S0 was slower (registers).  The same in fp32 on the FMA pipe (the inverse times keys
+// and values ahead of the scan, 4 x 4 tiles) took 333: 16-byte reads of shared memory bound it.
 // ------------------------------------------------------------------------------------------------------------------
 constexpr int CL = 32;                       // tokens per chunk
-// Sequences from here on are scanned in chunks.  Three chunks take what pairs take for 85 to 88 tokens where a batch is small: one sequence of 80 tokens 28.2
-// against 26.9 us, of 96 28.3 against 31.2 (16 heads of 128 x 128); 21.3 against 19.7, 21.5 against 22.8 (8 of 64 x 64).  Of many the chunks are
-// ahead from 64 on (32 of 64: 82 against 130), but a sequence's result must not depend on the others.
+// Sequences from here on are scanned in chunks: the first length at which they are ahead or level at every size and batch.  Three chunks take what pairs
+// take for 81 tokens (one sequence, 16 heads of 128 x 128: 80 tokens 26.7 in pairs, 96 31.2, three chunks 27.0 us) to 88 (8 heads of 64 x 64: 19.6, 22.8 and 21.5).
+// Of many the chunks are ahead from 64 on (32 of 64: 71 against 130), but a sequence's result must not depend on the others.
 constexpr int CL_MIN = 88;
 constexpr int CL_LD = CL + 8;                // row stride of 32 x 32 bf16 matrices in shared memory (ldmatrix without bank conflicts)
 constexpr int CL_WARPS = 4;                  // warps (of 16 columns) per block of the scan
 constexpr int CL_COLS = 16 * CL_WARPS;
 // scratch per (chunk, head), in floats: T and M as three bf16 parts each, then per token the factors of K S0,
-// Q S0 and of u in the update and T's diagonal with its rest, then G_L
-constexpr int CL_SCRATCH = 3 * CL * CL + 5 * CL + 32;
+// Q S0 and of u in the update and T's diagonal, then G_L
+constexpr int CL_SCRATCH = 3 * CL * CL + 4 * CL + 32;
 
 __device__ __forceinline__ uint32_t smem_at(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t at) {
@@ -685,29 +685,23 @@ __device__ __forceinline__ void add_mma16816(float (&c)[4], const uint32_t (&a)[
 #pragma unroll
   for (int e = 0; e < 4; ++e) c[e] += y[e];
 }
-// (x + xr, y + yr) as the sum of three pairs of bf16 numbers, largest first; the rests are small
-__device__ __forceinline__ void parts3(float x, float y, float xr, float yr, uint32_t (&p)[3]) {
+// (x, y) as the sum of three pairs of bf16 numbers, largest first
+__device__ __forceinline__ void parts3(float x, float y, uint32_t (&p)[3]) {
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     const __nv_bfloat162 r = __floats2bfloat162_rn(x, y);
     p[i] = *reinterpret_cast<const uint32_t*>(&r);
     x -= __uint_as_float(p[i] << 16);
     y -= __uint_as_float(p[i] & 0xffff0000u);
-    if (i == 0) {
-      x += xr;
-      y += yr;
-    }
   }
 }
-// A operand of 16 rows and the 16 columns of two neighbouring accumulator tiles (and their rests), in three parts
-__device__ __forceinline__ void a_parts(const float (&l)[4], const float (&r)[4], uint32_t (&a)[3][4], const float (&lr)[4] = {0.f, 0.f, 0.f, 0.f},
-                                        const float (&rr)[4] = {0.f, 0.f, 0.f, 0.f}) {
+// A operand of 16 rows and the 16 columns of two neighbouring accumulator tiles, in three parts
+__device__ __forceinline__ void a_parts(const float (&l)[4], const float (&r)[4], uint32_t (&a)[3][4]) {
   uint32_t p[3];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int at = 2 * (i & 1);
-    if (i < 2) parts3(l[at], l[at + 1], lr[at], lr[at + 1], p);
-    else parts3(r[at], r[at + 1], rr[at], rr[at + 1], p);
+    const float x = i < 2 ? l[2 * (i & 1)] : r[2 * (i & 1)], y = i < 2 ? l[2 * (i & 1) + 1] : r[2 * (i & 1) + 1];
+    parts3(x, y, p);
 #pragma unroll
     for (int e = 0; e < 3; ++e) a[e][i] = p[e];
   }
@@ -857,10 +851,8 @@ delta_chunk_prep_kernel(const bf16* __restrict__ qkv, long ldq, int koff, const 
     fac[lane] = static_cast<float>(G * ks);
     fac[CL + lane] = static_cast<float>(G * qsc[lane]);
     fac[2 * CL + lane] = static_cast<float>(x);        // (tokens behind the end decay by 1)
-    const double diag = beta * ks;
-    fac[3 * CL + lane] = static_cast<float>(diag);
-    fac[4 * CL + lane] = static_cast<float>(diag - static_cast<float>(diag));
-    if (lane == 0) fac[5 * CL] = static_cast<float>(all);
+    fac[3 * CL + lane] = static_cast<float>(beta * ks);
+    if (lane == 0) fac[4 * CL] = static_cast<float>(all);
     __syncwarp();
     float col[CL];                           // column `lane` of (I + A)^-1
 #pragma unroll
@@ -880,7 +872,7 @@ struct DeltaChunkStage {
   bf16 k[CL * (DP + 8)], q[CL * (DP + 8)];
   bf16 tm[6 * CL * CL_LD];                   // T, M: three parts each
   bf16 v[CL * (CL_COLS + 8)];
-  float fac[5 * CL + 4];
+  float fac[4 * CL + 4];
 };
 template <int DP>
 struct DeltaChunkSmem {
@@ -941,7 +933,7 @@ delta_chunk_scan_kernel(const bf16* __restrict__ qkv, long ldq, int koff, int vo
       const bool in = t < nt && j0 + j < V;
       cp_async16(p.v + t * VLD + j, qkv + (in ? (tok + t) * ldq + voff + (long)h * V + j0 + j : 0), in ? 16 : 0);
     }
-    if (tid < (5 * CL + 4) / 4) cp_async16(p.fac + 4 * tid, w + 3 * CL * CL + 4 * tid, 16);
+    if (tid < (4 * CL + 4) / 4) cp_async16(p.fac + 4 * tid, w + 3 * CL * CL + 4 * tid, 16);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
   const int chunks = (n + CL - 1) / CL;
@@ -986,10 +978,11 @@ delta_chunk_scan_kernel(const bf16* __restrict__ qkv, long ldq, int koff, int vo
         if (__float_as_uint(p.fac[CL + t]) == 0x80000000u) x[4 + i][e] = 0.f;
         odd[e >> 1] = odd[e >> 1] || !(fabsf(x[i][e]) < 1e37f);
       }
-    float u[4][4] = {}, ur[4][4] = {};       // U and what its rounding left
+    float u[4][4] = {};
     {
-      // D + R = [16, 32] (as A, three parts) times the three parts of a lower triangular matrix at `tri`; R is small
-      auto times = [&](const float (*y)[4], const bf16* tri, float (&d)[4][4], float (&r)[4][4]) {
+      // D = [16, 32] (as A, three parts) times the three parts of a lower triangular matrix at `tri`
+      auto times = [&](const float (*y)[4], const bf16* tri, float (&d)[4][4]) {
+        float r[4][4] = {};
 #pragma unroll
         for (int kk = 0; kk < 2; ++kk) {
           uint32_t am[3][4];
@@ -1012,31 +1005,21 @@ delta_chunk_scan_kernel(const bf16* __restrict__ qkv, long ldq, int koff, int vo
                 }
           }
         }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) d[i][e] += r[i][e];
       };
-      times(x, p.tm, u, ur);
+      times(x, p.tm, u);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {        // the diagonal, exact; sum with its rounding error
-          const int t = 8 * i + q2 + (e & 1);
-          const float own = p.fac[3 * CL + t] * x[i][e], sum = u[i][e] + own, back = sum - u[i][e];
-          ur[i][e] += fmaf(p.fac[3 * CL + t], x[i][e], -own) + p.fac[4 * CL + t] * x[i][e] + ((u[i][e] - (sum - back)) + (own - back));
-          u[i][e] = sum;
-          odd[e >> 1] = odd[e >> 1] || !(fabsf(sum) < 1e37f);
+        for (int e = 0; e < 4; ++e) {        // the diagonal
+          u[i][e] = fmaf(p.fac[3 * CL + 8 * i + q2 + (e & 1)], x[i][e], u[i][e]);
+          odd[e >> 1] = odd[e >> 1] || !(fabsf(u[i][e]) < 1e37f);
         }
       float o[4][4] = {};
-      {
-        float y[4][4], low[4][4] = {};
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) y[i][e] = u[i][e] + ur[i][e];
-        times(y, p.tm + 3 * CL * CL_LD, o, low);
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) o[i][e] += low[i][e];
-      }
+      times(u, p.tm + 3 * CL * CL_LD, o);
       const unsigned any = __ballot_sync(0xffffffffu, odd[0] || odd[1]);
       if (any == 0) {
 #pragma unroll
@@ -1072,10 +1055,7 @@ delta_chunk_scan_kernel(const bf16* __restrict__ qkv, long ldq, int koff, int vo
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const int t = 8 * i + q2 + (e & 1), col = g + 8 * (e >> 1);
-            if (odd[e >> 1]) {
-              u[i][e] = us[col][t];
-              ur[i][e] = 0.f;
-            }
+            if (odd[e >> 1]) u[i][e] = us[col][t];
             x[4 + i][e] = fmaf(p.fac[CL + t], x[4 + i][e], odd[e >> 1] ? ys[col][t] : o[i][e]);
           }
         __syncwarp();
@@ -1087,24 +1067,24 @@ delta_chunk_scan_kernel(const bf16* __restrict__ qkv, long ldq, int koff, int vo
       for (int e = 0; e < 4; ++e) {
         const int t = 8 * i + q2 + (e & 1), col = jc + 8 * (e >> 1);
         if (t < nt && col < V) out[(tok0 + c * CL + t) * (long)(H * V) + (long)h * V + col] = x[4 + i][e];
-        const float f = p.fac[2 * CL + t], w = u[i][e] * f, wr = fmaf(u[i][e], f, -w) + ur[i][e] * f;
-        u[i][e] = t < nt ? w : 0.f;
-        ur[i][e] = t < nt && fabsf(w) < 1e37f ? wr : 0.f;
+        u[i][e] = t < nt ? u[i][e] * p.fac[2 * CL + t] : 0.f;
       }
     // ---- Sᵀ <- G_L Sᵀ + Uᵀ K
-    const float gl = p.fac[5 * CL];
+    const float gl = p.fac[4 * CL];
     uint32_t am[2][3][4];
 #pragma unroll
-    for (int kk = 0; kk < 2; ++kk) a_parts(u[2 * kk], u[2 * kk + 1], am[kk], ur[2 * kk], ur[2 * kk + 1]);
+    for (int kk = 0; kk < 2; ++kk) a_parts(u[2 * kk], u[2 * kk + 1], am[kk]);
 #pragma unroll
     for (int d2 = 0; d2 < DP / 16; ++d2) {
       uint32_t bm[2][4];
 #pragma unroll
       for (int kk = 0; kk < 2; ++kk) ldsm4_trans(bm[kk], smem_at(p.k + (kk * 16 + (lane & 15)) * LD + d2 * 16 + (lane >> 4) * 8));
       // the smaller parts and the earlier tokens, the state, then the later tokens
-      float y[2][4], z[2][4];
+      float y[2][4], z[2][2][4];
 #pragma unroll
-      for (int i = 0; i < 2; ++i) mma16816_new(z[i], am[1][0], bm[1][2 * i], bm[1][2 * i + 1]);
+      for (int kk = 0; kk < 2; ++kk)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) mma16816_new(z[kk][i], am[kk][0], bm[kk][2 * i], bm[kk][2 * i + 1]);
 #pragma unroll
       for (int i = 0; i < 2; ++i) mma16816_new(y[i], am[0][2], bm[0][2 * i], bm[0][2 * i + 1]);
 #pragma unroll
@@ -1114,11 +1094,9 @@ delta_chunk_scan_kernel(const bf16* __restrict__ qkv, long ldq, int koff, int vo
 #pragma unroll
         for (int i = 0; i < 2; ++i) mma16816(y[i], am[kk][1], bm[kk][2 * i], bm[kk][2 * i + 1]);
 #pragma unroll
-      for (int i = 0; i < 2; ++i) mma16816(y[i], am[0][0], bm[0][2 * i], bm[0][2 * i + 1]);
-#pragma unroll
       for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) st[2 * d2 + i][e] = fmaf(gl, st[2 * d2 + i][e], y[i][e]) + z[i][e];
+        for (int e = 0; e < 4; ++e) st[2 * d2 + i][e] = fmaf(gl, st[2 * d2 + i][e], y[i][e] + z[0][i][e]) + z[1][i][e];
     }
   }
 #pragma unroll
