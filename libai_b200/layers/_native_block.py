@@ -38,8 +38,10 @@ def _calls_are_seen() -> bool:
 
 def plain(m, cls) -> bool:
     """A module of this very class whose call without a graph is its class's ``forward`` and nothing else."""
-    return (type(m) is cls and cls.forward is _FORWARDS[cls] and not m._forward_hooks and not m._forward_pre_hooks and m._compiled_call_impl is None
-            and "forward" not in m.__dict__)
+    if type(m) is not cls or cls.forward is not _FORWARDS[cls]:
+        return False
+    own = m.__dict__                     # (a lookup each where the attribute takes three)
+    return not own["_forward_hooks"] and not own["_forward_pre_hooks"] and "_compiled_call_impl" not in own and "forward" not in own
 
 
 def alone(m, cls) -> bool:

@@ -152,3 +152,18 @@ def test_backward_hooks_of_a_llama_block_change_their_branch_only(name):
     branch.forward = lambda *a, **k: forward(*a, **k).detach()               # the same by hand
     want = torch.autograd.grad(call().sum(), x)[0]
     assert torch.equal(cut, want) and not torch.equal(cut, whole)
+
+
+def test_modules_with_another_call_are_not_passed_by(monkeypatch):
+    from libai_b200.layers import RMSLayerNorm
+    from libai_b200.layers import _native_block as native
+
+    m = _small_block("llama", torch.float32)[0].input_layernorm
+    assert native.alone(m, RMSLayerNorm)
+    call = torch.nn.Module.__call__
+    with monkeypatch.context() as patch:                      # as tracers and profilers do
+        patch.setattr(torch.nn.Module, "__call__", lambda self, *a, **k: call(self, *a, **k))
+        assert not native.alone(m, RMSLayerNorm)
+    assert native.alone(m, RMSLayerNorm)
+    m.compile(backend="eager")
+    assert not native.plain(m, RMSLayerNorm)
