@@ -1022,7 +1022,7 @@ static int gemm_impl(const void* a, const void* b, void* out, int M, int N, int 
       if (rc != -1) return rc;
     }
   }
-  if ((reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(pre_in) | reinterpret_cast<uintptr_t>(pre_out)) & 15) return -8;   // vectors of the epilogue
+  if (epi == 0 && ((reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(pre_in) | reinterpret_cast<uintptr_t>(pre_out)) & 15)) return -8;   // vectors of the bf16 epilogue
   const bool a_mn = (layout == 2);
   const bool b_mn = (layout != 0);
   const int sms = num_sms();
