@@ -196,6 +196,12 @@ LB_DEVICE void tma_store_4d(const CUtensorMap* map, const void* smem_src, int32_
                "r"(smem_u32(smem_src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
                : "memory");
 }
+// out[box] += shared memory, in the element type of the map
+LB_DEVICE void tma_reduce_add_2d(const CUtensorMap* map, const void* smem_src, int32_t c0, int32_t c1) {
+  asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];\n" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c0),
+               "r"(c1), "r"(smem_u32(smem_src))
+               : "memory");
+}
 LB_DEVICE void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;\n" ::: "memory"); }
 template <int N>
 LB_DEVICE void tma_store_wait_read() {

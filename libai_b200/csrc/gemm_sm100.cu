@@ -4,7 +4,7 @@
 //   D[M,N] = A · Bᵀ   with three operand layouts (all row-major tensors in global memory):
 //     NT: A[M,K], B[N,K]   (forward  : y  = x · Wᵀ)
 //     NN: A[M,K], B[K,N]   (dgrad    : dx = dy · W,   B is "MN-major")
-//     TN: A[K,M], B[K,N]   (wgrad    : dW = dyᵀ · x,  both "MN-major"; split-K + fp32 red.add)
+//     TN: A[K,M], B[K,N]   (wgrad    : dW = dyᵀ · x,  both "MN-major"; split-K + fp32 TMA reductions)
 //
 // Replaces the cuBLAS matmuls behind libai/layers/linear.py:123-157 and the separate
 // fused_bias_add_gelu kernel (libai/layers/mlp.py:95) of the reference.
@@ -109,14 +109,16 @@ LB_DEVICE uint32_t ld_acquire_gpu_u32(const uint32_t* a) {
   return v;
 }
 
-template <int BLOCK_N, int CTAS = 1>
+template <int BLOCK_N, int CTAS = 1, bool REDUCE = false>
 struct StageCfg {
   static constexpr int A_BYTES = BLOCK_M * BLOCK_K * 2;
   static constexpr int B_BYTES = (BLOCK_N / CTAS) * BLOCK_K * 2;   // CTA pair: each CTA stages half of the B tile
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int NUM_STAGES = CTAS == 2 ? 6 : ((BLOCK_N == 256) ? 4 : (BLOCK_N == 192 ? 5 : (BLOCK_N == 128 ? 6 : 8)));
-  static constexpr int STAGING_BYTES = 8 * 2048;  // one 32x32 bf16 chunk (32 rows x 64 B) per epilogue warp
+  static constexpr int NUM_STAGES = CTAS == 2 ? 6 : ((BLOCK_N == 256) ? 4 : (BLOCK_N == 192 ? (REDUCE ? 4 : 5) : (BLOCK_N == 128 ? 6 : 8)));
+  static constexpr int STAGING_SLOT = REDUCE ? 4096 : 2048;   // per epilogue warp: a 32 x 32 chunk in fp32 (box of a TMA reduction) or bf16
+  static constexpr int STAGING_BYTES = 8 * STAGING_SLOT;
   static constexpr int SMEM_BYTES = NUM_STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/ + STAGING_BYTES;
+  static_assert(SMEM_BYTES <= 232448, "shared memory of one CTA");
   static constexpr uint32_t TMEM_COLS = (2 * BLOCK_N <= 32) ? 32 : (2 * BLOCK_N <= 64 ? 64 : (2 * BLOCK_N <= 128 ? 128 : (2 * BLOCK_N <= 256 ? 256 : 512)));
 };
 
@@ -190,20 +192,20 @@ LB_DEVICE void stg_store_chunk(uint8_t* stg, int lane, const float (&v)[32], __n
 template <int BLOCK_N, bool A_MN, bool B_MN, int EPI, bool FP8 = false, int CTAS = 1>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-            const __grid_constant__ CUtensorMap tmap_g /* COMM_AG: the local shard of the gathered operand */, GemmParams p,
-            CommParams cp) {
-  using Cfg = StageCfg<BLOCK_N, CTAS>;
+            const __grid_constant__ CUtensorMap tmap_g /* COMM_AG: the local shard of the gathered operand */,
+            const __grid_constant__ CUtensorMap tmap_o /* EPI_ATOMIC_F32: the output in boxes of 32 x 32 */, GemmParams p, CommParams cp) {
+  using Cfg = StageCfg<BLOCK_N, CTAS, EPI == EPI_ATOMIC_F32>;
   constexpr int NS = Cfg::NUM_STAGES;
   static_assert(CTAS == 1 || (CTAS == 2 && BLOCK_N == 256 && !FP8), "CTA-pair mode: 256-wide bf16 tiles only");
   const int cta_rank = CTAS == 2 ? static_cast<int>(cluster_ctarank()) : 0;   // 0 = leader of the pair
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + NS * Cfg::STAGE_BYTES);
+  uint8_t* staging = smem + NS * Cfg::STAGE_BYTES;        // one slot per epilogue warp (on 1024 bytes: swizzled boxes)
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(staging + Cfg::STAGING_BYTES);
   uint64_t* empty_bar = full_bar + NS;
   uint64_t* tmem_full = empty_bar + NS;
   uint64_t* tmem_empty = tmem_full + 2;
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(tmem_empty + 2);
-  uint8_t* staging = smem + NS * Cfg::STAGE_BYTES + 256;  // 8 x 2 KB, one slot per epilogue warp
 
   const int warp_idx = threadIdx.x / 32;
   const int lane = threadIdx.x % 32;
@@ -228,7 +230,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     const int owner = (cp.rank + shift + m_seq / upr) % cp.world;
     return owner * upr + m_seq % upr;
   };
-  // work item -> (output tile, K partition).  Default: partitions of one tile are neighbours (their red.adds hit L2
+  // work item -> (output tile, K partition).  Default: partitions of one tile are neighbours (their reductions hit L2
   // together).  Gathered-B wgrad: partition-major, starting with the partitions that lie in the local shard (the host
   // makes k_splits a multiple of world and partitions never straddle a shard boundary), so every CTA has local work
   // while the remote shards are still in flight.
@@ -256,6 +258,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
     if (cp.mode == COMM_AG) tma_prefetch_desc(&tmap_g);
+    if constexpr (EPI == EPI_ATOMIC_F32) tma_prefetch_desc(&tmap_o);
 #pragma unroll
     for (int i = 0; i < NS; ++i) {
       mbar_init(&full_bar[i], CTAS);   // pair: the leader's barrier collects one arrival per CTA (+ both CTAs' bytes)
@@ -657,11 +660,30 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           }
           stg_store_chunk(stg, lane, v, slab, ld, rows_valid, cols_valid,
                           (p.colsum != nullptr && cp.mode != COMM_RS) ? p.colsum + col0 : nullptr);
+        } else if constexpr (EPI == EPI_ATOMIC_F32) {
+          // ---- accumulation into fp32 (wgrad into main_grad, split-K): the chunk goes through shared memory and one TMA reduction.
+          // One instruction per 4 KB and none that waits: the 8 rows x 64 bytes of red.global.add.v4 per instruction that this took before
+          // cost [2048, 22016]ᵀ x [2048, 4096] 290 us, now 280 (bf16 results 232: the difference is 540 MB more to and from HBM), [2048, 4096]ᵀ x [2048, 11008]
+          // 149.6 -> 145.7, [8192, 50304]ᵀ x [8192, 1024] 582 -> 570, [8192, 1024]ᵀ x [8192, 3072] 39.7 -> 38.4.  The output ahead into L2
+          // (cp.async.bulk.prefetch) makes it slower, 283 and 158 us; an evict-first policy changes nothing.
+          uint8_t* stg = staging + (warp_idx - 2) * Cfg::STAGING_SLOT;
+          if (lane == 0) tma_store_wait_read<0>();          // the reduction before has read the slot
+          tmem_ld_wait();
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 8; ++i)                       // row `lane` of the box, its 16-byte pieces where the 128-byte swizzle has them
+            *reinterpret_cast<uint4*>(stg + lane * 128 + ((i ^ (lane & 7)) << 4)) = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
+          fence_proxy_async();
+          __syncwarp();
+          const int row0 = m_blk * BLOCK_M + quad * 32;
+          if (lane == 0 && row0 < p.M) {                    // (rows and columns behind the end are left out by the map)
+            tma_reduce_add_2d(&tmap_o, stg, col0, row0);
+            tma_store_commit();
+          }
         } else {
-          // ---- fp32 outputs (wgrad: plain store / read-modify-write into main_grad, or red.add for split-K): the
+          // ---- fp32 outputs (plain store or read-modify-write): the
           // same staging slot, 16 columns (64 B per row) at a time, so every global instruction covers 8 rows x 64
-          // contiguous bytes instead of 32 rows x 16 B.  With <= 148 tiles there is no next tile whose MMAs could hide
-          // this epilogue, so its LSU wavefront count is on the critical path.
+          // contiguous bytes instead of 32 rows x 16 B.
           tmem_ld_wait();
           uint8_t* stg = staging + (warp_idx - 2) * 2048;
           const int slab_row0 = m_blk * BLOCK_M + quad * 32;
@@ -683,16 +705,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
                   float* dst = slab + static_cast<size_t>(rr) * p.ldo + c;
                   float4 o4 = make_float4(__uint_as_float(quadv[j].x), __uint_as_float(quadv[j].y), __uint_as_float(quadv[j].z),
                                           __uint_as_float(quadv[j].w));
-                  if constexpr (EPI == EPI_F32) {
-                    if (p.rmw) {
-                      const float4 old = *reinterpret_cast<const float4*>(dst);
-                      o4.x += old.x; o4.y += old.y; o4.z += old.z; o4.w += old.w;
-                    }
-                    *reinterpret_cast<float4*>(dst) = o4;
-                  } else {
-                    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"l"(dst), "f"(o4.x), "f"(o4.y), "f"(o4.z), "f"(o4.w)
-                                 : "memory");
+                  if (p.rmw) {
+                    const float4 old = *reinterpret_cast<const float4*>(dst);
+                    o4.x += old.x; o4.y += old.y; o4.z += old.z; o4.w += old.w;
                   }
+                  *reinterpret_cast<float4*>(dst) = o4;
                 }
               }
             }
@@ -724,6 +741,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         acc = 0;
         acc_phase ^= 1;
       }
+    }
+    if constexpr (EPI == EPI_ATOMIC_F32) {
+      if (lane == 0) tma_store_wait<0>();
+      __syncwarp();
     }
   }
 
@@ -921,9 +942,9 @@ bool chained(const lb::GemmParams& p, const lb::CommParams& cp) { return cp.mode
 
 // CTA-pair (cta_group::2) variant: clusters of 2, 256 x 256 tiles
 template <bool AMN, bool BMN, int EPI>
-cudaError_t launch_2cta(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tg, const lb::GemmParams& p,
+cudaError_t launch_2cta(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tg, const CUtensorMap& to, const lb::GemmParams& p,
                         const lb::CommParams& cp, int grid, cudaStream_t stream) {
-  using Cfg = lb::StageCfg<256, 2>;
+  using Cfg = lb::StageCfg<256, 2, EPI == lb::EPI_ATOMIC_F32>;
   auto kern = lb::gemm_kernel<256, AMN, BMN, EPI, false, 2>;
   static bool configured = false;
   if (!configured) {
@@ -931,7 +952,7 @@ cudaError_t launch_2cta(const CUtensorMap& ta, const CUtensorMap& tb, const CUte
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  if (chained(p, cp)) return lb_host::launch_chained(kern, dim3((unsigned)grid), dim3(lb::NUM_THREADS), Cfg::SMEM_BYTES, stream, 2, ta, tb, tg, p, cp);
+  if (chained(p, cp)) return lb_host::launch_chained(kern, dim3((unsigned)grid), dim3(lb::NUM_THREADS), Cfg::SMEM_BYTES, stream, 2, ta, tb, tg, to, p, cp);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3(lb::NUM_THREADS);
@@ -944,13 +965,13 @@ cudaError_t launch_2cta(const CUtensorMap& ta, const CUtensorMap& tb, const CUte
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, ta, tb, tg, p, cp);
+  return cudaLaunchKernelEx(&cfg, kern, ta, tb, tg, to, p, cp);
 }
 
 template <int BN, bool AMN, bool BMN, int EPI, bool FP8 = false>
-cudaError_t launch_cfg(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tg, const lb::GemmParams& p,
+cudaError_t launch_cfg(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tg, const CUtensorMap& to, const lb::GemmParams& p,
                        const lb::CommParams& cp, int grid, cudaStream_t stream) {
-  using Cfg = lb::StageCfg<BN>;
+  using Cfg = lb::StageCfg<BN, 1, EPI == lb::EPI_ATOMIC_F32>;
   auto kern = lb::gemm_kernel<BN, AMN, BMN, EPI, FP8>;
   static bool configured = false;
   if (!configured) {
@@ -958,23 +979,23 @@ cudaError_t launch_cfg(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  if (chained(p, cp)) return lb_host::launch_chained(kern, dim3((unsigned)grid), dim3(lb::NUM_THREADS), Cfg::SMEM_BYTES, stream, 0, ta, tb, tg, p, cp);
-  kern<<<grid, lb::NUM_THREADS, Cfg::SMEM_BYTES, stream>>>(ta, tb, tg, p, cp);
+  if (chained(p, cp)) return lb_host::launch_chained(kern, dim3((unsigned)grid), dim3(lb::NUM_THREADS), Cfg::SMEM_BYTES, stream, 0, ta, tb, tg, to, p, cp);
+  kern<<<grid, lb::NUM_THREADS, Cfg::SMEM_BYTES, stream>>>(ta, tb, tg, to, p, cp);
   return cudaGetLastError();
 }
 
 template <bool AMN, bool BMN, int EPI, bool FP8 = false>
-cudaError_t launch_bn(int bn, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tg, const lb::GemmParams& p,
+cudaError_t launch_bn(int bn, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tg, const CUtensorMap& to, const lb::GemmParams& p,
                       const lb::CommParams& cp, int grid, cudaStream_t s) {
   switch (bn) {
     case 256:
-      return launch_cfg<256, AMN, BMN, EPI, FP8>(ta, tb, tg, p, cp, grid, s);
+      return launch_cfg<256, AMN, BMN, EPI, FP8>(ta, tb, tg, to, p, cp, grid, s);
     case 192:
-      return launch_cfg<192, AMN, BMN, EPI, FP8>(ta, tb, tg, p, cp, grid, s);
+      return launch_cfg<192, AMN, BMN, EPI, FP8>(ta, tb, tg, to, p, cp, grid, s);
     case 128:
-      return launch_cfg<128, AMN, BMN, EPI, FP8>(ta, tb, tg, p, cp, grid, s);
+      return launch_cfg<128, AMN, BMN, EPI, FP8>(ta, tb, tg, to, p, cp, grid, s);
     default:
-      return launch_cfg<64, AMN, BMN, EPI, FP8>(ta, tb, tg, p, cp, grid, s);
+      return launch_cfg<64, AMN, BMN, EPI, FP8>(ta, tb, tg, to, p, cp, grid, s);
   }
 }
 
@@ -1085,7 +1106,7 @@ static int gemm_impl(const void* a, const void* b, void* out, int M, int N, int 
     } else if (splits <= 0) {
       // Persistent CTAs take work items round-robin, so the kernel lasts ceil(items / SMs) rounds of one K partition
       // each: pick the split count that minimises rounds x (k-blocks per partition + a fixed per-item cost for
-      // pipeline fill and the fp32 red.add epilogue).  (A plain ceil(SMs / tiles) overshoots into a second round:
+      // pipeline fill and the epilogue).  (A plain ceil(SMs / tiles) overshoots into a second round:
       // 32 tiles x 5 splits = 160 items on 148 SMs took 2 x 26 k-blocks where 4 splits take 1 x 32.)
       const long tiles = (long)m_blocks * n_blocks;
       double best = 1e30;
@@ -1113,9 +1134,9 @@ static int gemm_impl(const void* a, const void* b, void* out, int M, int N, int 
   p.rmw = 0;
   if (epi == 2 && p.k_splits == 1 && wgrad_rmw()) {
     // a single K partition owns the whole tile: accumulate with a plain read-modify-write instead of L2 atomics.
-    // Off by default since the epilogue became coalesced: `red.add.v4` is fire-and-forget, while the read of the old
+    // Off by default: a reduction is not waited for, while the read of the old
     // tile sits exposed at the end of a one-tile-per-CTA GEMM (4096x1024x8192
-    // 2-way split with red.add 54 us vs single partition with rmw 67 us).  LIBAI_B200_WGRAD_RMW=1 restores it.
+    // 2-way split with reductions 50 us vs single partition with rmw 63 us; [22016,4096] 280 vs 367).  LIBAI_B200_WGRAD_RMW=1 restores it.
     epi = 1;
     p.rmw = 1;
   }
@@ -1151,10 +1172,16 @@ static int gemm_impl(const void* a, const void* b, void* out, int M, int N, int 
     const double in_flight = two_cta ? sms / 2 : sms, side = two_cta ? 1.0 : (double)bn / lb::BLOCK_M;
     p.group_m = (int)(std::sqrt(in_flight * side) + 0.5);
   }
-  CUtensorMap ta, tb, tg;
+  CUtensorMap ta, tb, tg, to;
   if (!operand_tmap(&ta, a, a_mn, M, K, lda, lb::BLOCK_M)) return -2;
   if (!operand_tmap(&tb, b, b_mn, tile_group ? N * groups : N, K, ldb, two_cta ? bn / 2 : bn)) return -2;
-  tg = ta;
+  tg = to = ta;
+  if (epi == 2) {
+    if (reinterpret_cast<uintptr_t>(out) & 15) return -8;
+    const uint64_t dims[2] = {(uint64_t)N, (uint64_t)M}, strides[2] = {4, (uint64_t)ldo * 4};
+    const uint32_t box[2] = {32u, 32u};
+    if (!lb_host::make_tmap_typed(&to, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, out, 2, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B)) return -2;
+  }
   if (cp.mode == lb::COMM_AG) {
     // tensor map of the local shard of the gathered operand: [rows_per_rank, K] rows of A (NT/NN), or rows_per_rank
     // reduction rows of B (TN)
@@ -1184,35 +1211,35 @@ static int gemm_impl(const void* a, const void* b, void* out, int M, int N, int 
   cudaError_t e;
   if (two_cta) {
     if (layout == 0) {
-      if (epi == 0) e = launch_2cta<false, false, lb::EPI_BF16>(ta, tb, tg, p, cp, grid, stream);
-      else if (epi == 1) e = launch_2cta<false, false, lb::EPI_F32>(ta, tb, tg, p, cp, grid, stream);
-      else e = launch_2cta<false, false, lb::EPI_ATOMIC_F32>(ta, tb, tg, p, cp, grid, stream);
+      if (epi == 0) e = launch_2cta<false, false, lb::EPI_BF16>(ta, tb, tg, to, p, cp, grid, stream);
+      else if (epi == 1) e = launch_2cta<false, false, lb::EPI_F32>(ta, tb, tg, to, p, cp, grid, stream);
+      else e = launch_2cta<false, false, lb::EPI_ATOMIC_F32>(ta, tb, tg, to, p, cp, grid, stream);
     } else if (layout == 1) {
-      if (epi == 0) e = launch_2cta<false, true, lb::EPI_BF16>(ta, tb, tg, p, cp, grid, stream);
-      else if (epi == 1) e = launch_2cta<false, true, lb::EPI_F32>(ta, tb, tg, p, cp, grid, stream);
-      else e = launch_2cta<false, true, lb::EPI_ATOMIC_F32>(ta, tb, tg, p, cp, grid, stream);
+      if (epi == 0) e = launch_2cta<false, true, lb::EPI_BF16>(ta, tb, tg, to, p, cp, grid, stream);
+      else if (epi == 1) e = launch_2cta<false, true, lb::EPI_F32>(ta, tb, tg, to, p, cp, grid, stream);
+      else e = launch_2cta<false, true, lb::EPI_ATOMIC_F32>(ta, tb, tg, to, p, cp, grid, stream);
     } else {
-      if (epi == 0) e = launch_2cta<true, true, lb::EPI_BF16>(ta, tb, tg, p, cp, grid, stream);
-      else if (epi == 1) e = launch_2cta<true, true, lb::EPI_F32>(ta, tb, tg, p, cp, grid, stream);
-      else e = launch_2cta<true, true, lb::EPI_ATOMIC_F32>(ta, tb, tg, p, cp, grid, stream);
+      if (epi == 0) e = launch_2cta<true, true, lb::EPI_BF16>(ta, tb, tg, to, p, cp, grid, stream);
+      else if (epi == 1) e = launch_2cta<true, true, lb::EPI_F32>(ta, tb, tg, to, p, cp, grid, stream);
+      else e = launch_2cta<true, true, lb::EPI_ATOMIC_F32>(ta, tb, tg, to, p, cp, grid, stream);
     }
     return (int)e;
   }
   if (p.fp8) {
     if (layout != 0 || epi != 0 || cp.mode != lb::COMM_NONE) return -7;
-    e = launch_bn<false, false, lb::EPI_BF16, true>(bn, ta, tb, tg, p, cp, grid, stream);
+    e = launch_bn<false, false, lb::EPI_BF16, true>(bn, ta, tb, tg, to, p, cp, grid, stream);
   } else if (layout == 0) {
-    if (epi == 0) e = launch_bn<false, false, lb::EPI_BF16>(bn, ta, tb, tg, p, cp, grid, stream);
-    else if (epi == 1) e = launch_bn<false, false, lb::EPI_F32>(bn, ta, tb, tg, p, cp, grid, stream);
-    else e = launch_bn<false, false, lb::EPI_ATOMIC_F32>(bn, ta, tb, tg, p, cp, grid, stream);
+    if (epi == 0) e = launch_bn<false, false, lb::EPI_BF16>(bn, ta, tb, tg, to, p, cp, grid, stream);
+    else if (epi == 1) e = launch_bn<false, false, lb::EPI_F32>(bn, ta, tb, tg, to, p, cp, grid, stream);
+    else e = launch_bn<false, false, lb::EPI_ATOMIC_F32>(bn, ta, tb, tg, to, p, cp, grid, stream);
   } else if (layout == 1) {
-    if (epi == 0) e = launch_bn<false, true, lb::EPI_BF16>(bn, ta, tb, tg, p, cp, grid, stream);
-    else if (epi == 1) e = launch_bn<false, true, lb::EPI_F32>(bn, ta, tb, tg, p, cp, grid, stream);
-    else e = launch_bn<false, true, lb::EPI_ATOMIC_F32>(bn, ta, tb, tg, p, cp, grid, stream);
+    if (epi == 0) e = launch_bn<false, true, lb::EPI_BF16>(bn, ta, tb, tg, to, p, cp, grid, stream);
+    else if (epi == 1) e = launch_bn<false, true, lb::EPI_F32>(bn, ta, tb, tg, to, p, cp, grid, stream);
+    else e = launch_bn<false, true, lb::EPI_ATOMIC_F32>(bn, ta, tb, tg, to, p, cp, grid, stream);
   } else {
-    if (epi == 0) e = launch_bn<true, true, lb::EPI_BF16>(bn, ta, tb, tg, p, cp, grid, stream);
-    else if (epi == 1) e = launch_bn<true, true, lb::EPI_F32>(bn, ta, tb, tg, p, cp, grid, stream);
-    else e = launch_bn<true, true, lb::EPI_ATOMIC_F32>(bn, ta, tb, tg, p, cp, grid, stream);
+    if (epi == 0) e = launch_bn<true, true, lb::EPI_BF16>(bn, ta, tb, tg, to, p, cp, grid, stream);
+    else if (epi == 1) e = launch_bn<true, true, lb::EPI_F32>(bn, ta, tb, tg, to, p, cp, grid, stream);
+    else e = launch_bn<true, true, lb::EPI_ATOMIC_F32>(bn, ta, tb, tg, to, p, cp, grid, stream);
   }
   return (int)e;
 }
@@ -1280,7 +1307,7 @@ extern "C" int lb_gemm_bf16_bias_residual(const void* x, const void* w, void* ou
 //           CTAs), local_shard = this rank's [M/world, K] rows, out [M, N] bf16 (+bias, +act with pre-activation copy,
 //           or x act'(pre_in) for a dgrad fused with the activation backward, + column sums for the bias gradient)
 //   mode 1, layout 2 (gathered-B wgrad): a = dy [T, M] (T tokens), b = local gathered buffer [T, N], local_shard =
-//           this rank's [T/world, N] rows of it, out [M, N] fp32: epi 2 accumulates (red.add), epi 1 stores
+//           this rank's [T/world, N] rows of it, out [M, N] fp32: epi 2 accumulates, epi 1 stores
 //   mode 2 (GEMM->RS), layout 0/1: a = local [M, K_shard]; partial tiles go to the owners' staging buffers;
 //           rs_out [M/world, N] = sum over ranks (+bias +residual)
 static unsigned long long spin_timeout_ns() {

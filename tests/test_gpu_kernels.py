@@ -1075,3 +1075,20 @@ def test_residual_that_begins_anywhere(rows):
             results.append((y.detach().double(), torch.autograd.grad(y, x, y.detach())[0].double()))
         for got, want in zip(*results):              # another norm kernel reads rows off their alignment: roundings of its result (2^-8) through the block
             assert float((got - want).norm()) < 2.0 ** -6 * float(want.norm())
+
+
+@pytest.mark.parametrize("m,n,k", [(8, 8, 64), (24, 264, 72), (128, 256, 512), (200, 72, 2664), (384, 1160, 2048), (1152, 384, 4096), (4104, 1024, 520)])
+def test_weight_gradient_accumulates_in_boxes(m, n, k):
+    """dW += dyᵀ x through boxes of 32 x 32 with rows and columns behind the end, split along K and not, into a slice of a larger buffer
+    whose other elements stay as they are."""
+    a, b = _rand((k, m), 1), _rand((k, n), 2)
+    buf = _rand((m + 2, n + 8), 3, dtype=torch.float32)
+    before = buf.clone()
+    load_ext().gemm(a, b, 2, None, buf[1:m + 1, 4:n + 4], True, torch.float32)
+    old = before[1:m + 1, 4:n + 4].double()
+    want = old + a.double().t() @ b.double()
+    # k products and k / 16 additions, none of which is more than one unit of 24 bits of the sum of magnitudes off
+    bound = (k / 16 + 2) * 2.0 ** -23 * (old.abs() + a.double().abs().t() @ b.double().abs())
+    assert bool(((buf[1:m + 1, 4:n + 4].double() - want).abs() <= bound).all())
+    buf[1:m + 1, 4:n + 4] = before[1:m + 1, 4:n + 4]
+    assert torch.equal(buf, before)
