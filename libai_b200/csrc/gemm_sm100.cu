@@ -109,12 +109,15 @@ LB_DEVICE uint32_t ld_acquire_gpu_u32(const uint32_t* a) {
   return v;
 }
 
-template <int BLOCK_N, int CTAS = 1, bool REDUCE = false>
+template <int BLOCK_N, int CTAS = 1, bool REDUCE = false, bool B_MN = false>
 struct StageCfg {
   static constexpr int A_BYTES = BLOCK_M * BLOCK_K * 2;
-  static constexpr int B_BYTES = (BLOCK_N / CTAS) * BLOCK_K * 2;   // CTA pair: each CTA stages half of the B tile
+  // CTA pair: each CTA stages half of the B tile (where that lies along rows, in whole boxes of 64 columns, of which the last may hold more than the half)
+  static constexpr int B_COLS = B_MN ? (BLOCK_N / CTAS + 63) / 64 * 64 : BLOCK_N / CTAS;
+  static constexpr int B_BYTES = B_COLS * BLOCK_K * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int NUM_STAGES = CTAS == 2 ? 6 : ((BLOCK_N == 256) ? 4 : (BLOCK_N == 192 ? (REDUCE ? 4 : 5) : (BLOCK_N == 128 ? 6 : 8)));
+  static constexpr int NUM_STAGES = CTAS == 2 ? (BLOCK_N == 128 ? 8 : (B_COLS == 96 ? 7 : 6))
+                                              : ((BLOCK_N == 256) ? 4 : (BLOCK_N == 192 ? (REDUCE ? 4 : 5) : (BLOCK_N == 128 ? 6 : 8)));
   static constexpr int STAGING_SLOT = REDUCE ? 4096 : 2048;   // per epilogue warp: a 32 x 32 chunk in fp32 (box of a TMA reduction) or bf16
   static constexpr int STAGING_BYTES = 8 * STAGING_SLOT;
   static constexpr int SMEM_BYTES = NUM_STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/ + STAGING_BYTES;
@@ -194,9 +197,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
             const __grid_constant__ CUtensorMap tmap_g /* COMM_AG: the local shard of the gathered operand */,
             const __grid_constant__ CUtensorMap tmap_o /* EPI_ATOMIC_F32: the output in boxes of 32 x 32 */, GemmParams p, CommParams cp) {
-  using Cfg = StageCfg<BLOCK_N, CTAS, EPI == EPI_ATOMIC_F32>;
+  using Cfg = StageCfg<BLOCK_N, CTAS, EPI == EPI_ATOMIC_F32, B_MN>;
   constexpr int NS = Cfg::NUM_STAGES;
-  static_assert(CTAS == 1 || (CTAS == 2 && BLOCK_N == 256 && !FP8), "CTA-pair mode: 256-wide bf16 tiles only");
+  static_assert(CTAS == 1 || (CTAS == 2 && BLOCK_N >= 128 && !FP8), "CTA-pair mode: bf16 tiles of 128 columns and more");
   const int cta_rank = CTAS == 2 ? static_cast<int>(cluster_ctarank()) : 0;   // 0 = leader of the pair
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -456,7 +459,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
               tma_load_2d_2cta(sb, &tmap_b, &full_bar[stage], kb * BLOCK_K, n_row);
             } else {
 #pragma unroll
-              for (int a = 0; a < (BLOCK_N / 2) / 64; ++a)
+              for (int a = 0; a < Cfg::B_COLS / 64; ++a)
                 tma_load_2d_2cta(sb + a * (BLOCK_K * 128), map_b, &full_bar[stage], n_row + a * 64, k_row);
             }
             if (++stage == NS) {
@@ -940,12 +943,12 @@ bool operand_tmap(CUtensorMap* m, const void* ptr, bool mn_major, int rows_or_co
 // start one by one take the tiles in another order, and rows of the two inputs are read twice); without it the chain is 2 to 3 us ahead.
 bool chained(const lb::GemmParams& p, const lb::CommParams& cp) { return cp.mode == lb::COMM_NONE && (p.pre_in == nullptr || p.act == lb::ACT_RESADD); }
 
-// CTA-pair (cta_group::2) variant: clusters of 2, 256 x 256 tiles
-template <bool AMN, bool BMN, int EPI>
+// CTA-pair (cta_group::2) variant: clusters of 2, 256 x BN tiles
+template <int BN, bool AMN, bool BMN, int EPI>
 cudaError_t launch_2cta(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tg, const CUtensorMap& to, const lb::GemmParams& p,
                         const lb::CommParams& cp, int grid, cudaStream_t stream) {
-  using Cfg = lb::StageCfg<256, 2, EPI == lb::EPI_ATOMIC_F32>;
-  auto kern = lb::gemm_kernel<256, AMN, BMN, EPI, false, 2>;
+  using Cfg = lb::StageCfg<BN, 2, EPI == lb::EPI_ATOMIC_F32, BMN>;
+  auto kern = lb::gemm_kernel<BN, AMN, BMN, EPI, false, 2>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
@@ -971,7 +974,7 @@ cudaError_t launch_2cta(const CUtensorMap& ta, const CUtensorMap& tb, const CUte
 template <int BN, bool AMN, bool BMN, int EPI, bool FP8 = false>
 cudaError_t launch_cfg(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tg, const CUtensorMap& to, const lb::GemmParams& p,
                        const lb::CommParams& cp, int grid, cudaStream_t stream) {
-  using Cfg = lb::StageCfg<BN, 1, EPI == lb::EPI_ATOMIC_F32>;
+  using Cfg = lb::StageCfg<BN, 1, EPI == lb::EPI_ATOMIC_F32, BMN>;
   auto kern = lb::gemm_kernel<BN, AMN, BMN, EPI, FP8>;
   static bool configured = false;
   if (!configured) {
@@ -1023,6 +1026,88 @@ static int gemm_allow_2cta() {
   return v;
 }
 
+// Time of a product with bf16 results by its tiles, in us: fixed + waves x (per wave + k-blocks x per k-block), but not below w at 6 TB/s.  Fitted over 290
+// products, layouts NT and NN, M = 256 .. 12608, N and K = 384 .. 5120 (3 to 5 % rms per kind).  A pair's tile takes half of B from L2 per SM: 256 x 192 a k-block in
+// 0.235 us on two SMs where two single 128 x 192 tiles take 0.29.  B along rows comes in boxes of 64 columns, of which the 96 of a pair's half take two: 192 wide tiles are dearer
+// there.  Single and pair, us: [8192, 768] x K = 3072 34.8 -> 30.4, [2560, 2048] x 2048 24.9 -> 20.9 (NN 21.8), [2048, 1024] x 4096 21.8 -> 18.1, [12608, 512] x 2048 31.3 -> 25.8.
+// A pair's narrower tile has to be 4 % ahead: it leaves more SMs without work where tiles are few ([180, 1912] x [1912, 1712] 12.0 us in 54 single tiles, 13.3 in 14 of pairs),
+// and against one tile of columns single CTAs are kept ([5997, 2040] x [104, 2040] 13.4 against 14.7).  Beyond four waves the last one matters less than the traffic and power
+// per product ([2048, 4096] x [12288, 4096] 135.8 us 256 wide in six waves, 139.7 192 wide in seven).  256 wide single tiles are for up to 128 rows against much of w.
+struct TileKind {
+  int bn;
+  bool pair;
+  double fixed, wave, block;
+};
+static const TileKind kTileKinds[2][7] = {
+    {{256, true, 5.50, 0.78, 0.302}, {192, true, 5.22, 0.76, 0.239}, {128, true, 5.06, 0.62, 0.202}, {256, false, 4.20, 1.20, 0.360}, {192, false, 4.16, 0.87, 0.293},
+     {128, false, 4.39, 0.47, 0.261}, {64, false, 3.96, 0.43, 0.237}},
+    {{256, true, 5.50, 0.78, 0.302}, {192, true, 4.70, 1.25, 0.249}, {128, true, 5.06, 0.62, 0.202}, {256, false, 4.20, 1.20, 0.360}, {192, false, 4.16, 0.87, 0.293},
+     {128, false, 4.39, 0.47, 0.261}, {64, false, 3.96, 0.43, 0.237}}};
+static double tile_choice(int M, int N, int K, bool nn, int* bn, bool* pair) {
+  const int sms = num_sms(), kb = (K + lb::BLOCK_K - 1) / lb::BLOCK_K;
+  const bool pairs = M > lb::BLOCK_M && gemm_allow_2cta();
+  const double w_us = (double)N * K * 2 / 6e6;
+  double best = 1e30, time = 1e30;
+  for (const TileKind& t : kTileKinds[nn]) {
+    if ((t.bn > 64 && N <= t.bn / 2) || (t.pair ? !pairs || N <= 128 : t.bn == 256 && pairs)) continue;
+    const int rows = t.pair ? 2 * lb::BLOCK_M : lb::BLOCK_M, slots = t.pair ? sms / 2 : sms;
+    const int tiles = (M + rows - 1) / rows * ((N + t.bn - 1) / t.bn), waves = (tiles + slots - 1) / slots;
+    if (t.pair && t.bn < 256 && waves > 4) continue;
+    const double us = waves * (t.wave + kb * t.block), all = t.fixed + (us > w_us ? us : w_us), order = all + 0.06 * us;
+    if (order < best - 1e-9) {
+      best = order;
+      time = all;
+      *bn = t.bn;
+      *pair = t.pair;
+    }
+  }
+  return time;
+}
+extern "C" double lb_gemm_tile_us(int M, int N, int K) {
+  int bn;
+  bool pair;
+  return tile_choice(M, N, K, false, &bn, &pair);
+}
+
+// Partitions of K for an accumulation with tiles of bn columns: persistent CTAs take work items round-robin, so the kernel lasts ceil(items / SMs) rounds of one K partition
+// each; the count that minimises rounds x (k-blocks per partition + a fixed per-item cost for pipeline fill and the epilogue).  (A plain ceil(SMs / tiles)
+// overshoots into a second round: 32 tiles x 5 splits = 160 items on 148 SMs took 2 x 26 k-blocks where 4 splits take 1 x 32.)
+static int split_choice(long tiles, int k_blocks, int sms) {
+  double best = 1e30;
+  int splits = 1;
+  for (int c = 1; c <= 16 && c <= k_blocks; ++c) {
+    if (c > 1 && k_blocks / c < 4) break;  // keep at least 4 k-blocks per split so the pipeline fills
+    const long rounds = (tiles * c + sms - 1) / sms;
+    const int kps = (k_blocks + c - 1) / c;
+    const double cost = (double)rounds * (kps + (c > 1 ? 6.0 : 3.0));
+    if (cost < best - 1e-9) {
+      best = cost;
+      splits = c;
+    }
+  }
+  return splits;
+}
+// Width of the pair tiles of an accumulation (weight gradients): fixed + rounds x (per round + k-blocks x per k-block) + bytes added.  Fitted over 48 products of up to
+// [3072, 1024], K = 512 .. 8192 (2.5 to 5 % rms; the narrow ones have to be 3 % ahead).  256 wide and the chosen width, us: [1152, 384] x K = 2048 9.9 -> 8.1, [1536, 384] x 2048 9.1 -> 7.4,
+// [2304, 768] x 5000 19.2 -> 16.7, [1280, 1280] x 5000 19.3 -> 16.2, [1024, 1024] x 512 8.4 -> 6.8; [3072, 1024] x 8192 and larger keep 256.
+static int wgrad_tile_choice(int M, int N, int K, int sms) {
+  static const struct { int bn; double fixed, round, block, mb; } kinds[3] = {{256, 6.56, 0.0, 0.322, 0.061}, {192, 5.25, 0.90, 0.273, 0.049}, {128, 6.10, 0.0, 0.207, 0.0129}};
+  const int kb = (K + lb::BLOCK_K - 1) / lb::BLOCK_K, m_blocks = (M + lb::BLOCK_M - 1) / lb::BLOCK_M;
+  double best = 1e30;
+  int bn = 256;
+  for (const auto& t : kinds) {
+    const long cols = (N + t.bn - 1) / t.bn;
+    const int c = split_choice(m_blocks * cols, kb, sms), kps = (kb + c - 1) / c, splits = (kb + kps - 1) / kps;
+    const long rounds = ((m_blocks + 1) / 2 * cols * splits + sms / 2 - 1) / (sms / 2);
+    const double us = t.fixed + rounds * (t.round + kps * t.block) + t.mb * splits * ((double)M * N * 4e-6);
+    if (us < best - 1e-9) {
+      best = us;
+      bn = t.bn;
+    }
+  }
+  return bn;
+}
+
 extern "C" int lb_gemm_small_rule(int M, int N, int K, int* nt, int* ranks);
 extern "C" int lb_gemm_small(const void* x, const void* w, void* out, int M, int N, int K, int ldx, int ldw, int ldo, const void* bias, int act,
                              void* pre_out, const void* residual, int nt, int ranks, cudaStream_t s);
@@ -1048,13 +1133,23 @@ static int gemm_impl(const void* a, const void* b, void* out, int M, int N, int 
   const bool b_mn = (layout != 0);
   const int sms = num_sms();
   const int m_blocks = (M + lb::BLOCK_M - 1) / lb::BLOCK_M;
-  // ---- tile-N heuristic: fewest waves, ties -> wider tile (less smem traffic per flop)
+  // ---- tiles: a CTA pair's 256 x bn or one CTA's 128 x bn
+  const bool pairs_ok = gemm_allow_2cta() && M > lb::BLOCK_M && deq_a == nullptr && !tile_group;
+  const bool plain = cp.mode == lb::COMM_NONE && deq_a == nullptr && !tile_group;
   int bn = force_bn;
-  if (bn == 0 && epi == 2) {
-    // split-K fills the machine for the accumulate (wgrad) epilogue: always take the widest tile that fits N
+  bool pair = force_bn == 256;
+  if (force_bn < 0) {                       // (timing: a pair's tile of that width)
+    bn = -force_bn;
+    pair = true;
+  } else if (force_bn == 0 && epi == 2) {
+    // split-K fills the machine for the accumulate (wgrad) epilogue: the widest tile that fits N, on pairs the width that is estimated best
     bn = N >= 192 ? 256 : (N >= 96 ? 128 : 64);
-  }
-  if (bn == 0) {
+    if (plain && pairs_ok && layout == 2 && N >= 96) bn = wgrad_tile_choice(M, N, K, sms);
+    pair = bn == 256 || (plain && pairs_ok && layout == 2 && N >= 96);
+  } else if (force_bn == 0 && plain && epi == 0 && layout != 2) {
+    tile_choice(M, N, K, layout == 1, &bn, &pair);
+  } else if (force_bn == 0) {
+    // collectives, fp8, groups, fp32 results: fewest waves, ties -> wider tile (less smem traffic per flop)
     double best = 1e30;
     const int cands[4] = {256, 192, 128, 64};
     for (int c : cands) {
@@ -1064,7 +1159,7 @@ static int gemm_impl(const void* a, const void* b, void* out, int M, int N, int 
       // cost ~ waves * per-tile time (proportional to c, narrower tiles pay more shared-memory traffic per
       // flop, plus a fixed prologue/epilogue overhead per tile)
       double eff = c == 256 ? 1.0 : (c == 192 ? 1.03 : (c == 128 ? 1.08 : 1.2));
-      if (c == 256 && cp_in.mode == lb::COMM_NONE && deq_a == nullptr && M > lb::BLOCK_M && gemm_allow_2cta() && !tile_group) {
+      if (c == 256 && plain && pairs_ok) {
         // 256-wide tiles run on CTA pairs (256 x 256 per pair, half the B traffic per SM): measured ~12 % faster per
         // tile row, scheduled over sms / 2 pairs
         tiles = (long)((m_blocks + 1) / 2) * ((N + c - 1) / c);
@@ -1075,6 +1170,7 @@ static int gemm_impl(const void* a, const void* b, void* out, int M, int N, int 
       if (cost < best - 1e-9) {
         best = cost;
         bn = c;
+        pair = c == 256;
       }
     }
   }
@@ -1104,22 +1200,7 @@ static int gemm_impl(const void* a, const void* b, void* out, int M, int N, int 
         }
       }
     } else if (splits <= 0) {
-      // Persistent CTAs take work items round-robin, so the kernel lasts ceil(items / SMs) rounds of one K partition
-      // each: pick the split count that minimises rounds x (k-blocks per partition + a fixed per-item cost for
-      // pipeline fill and the epilogue).  (A plain ceil(SMs / tiles) overshoots into a second round:
-      // 32 tiles x 5 splits = 160 items on 148 SMs took 2 x 26 k-blocks where 4 splits take 1 x 32.)
-      const long tiles = (long)m_blocks * n_blocks;
-      double best = 1e30;
-      for (int c = 1; c <= 16 && c <= k_blocks; ++c) {
-        if (c > 1 && k_blocks / c < 4) break;  // keep at least 4 k-blocks per split so the pipeline fills
-        const long rounds = (tiles * c + sms - 1) / sms;
-        const int kps = (k_blocks + c - 1) / c;
-        const double cost = (double)rounds * (kps + (c > 1 ? 6.0 : 3.0));
-        if (cost < best - 1e-9) {
-          best = cost;
-          splits = c;
-        }
-      }
+      splits = split_choice((long)m_blocks * n_blocks, k_blocks, sms);
     }
     if (splits > k_blocks) splits = k_blocks;
   }
@@ -1151,14 +1232,11 @@ static int gemm_impl(const void* a, const void* b, void* out, int M, int N, int 
   p.deq_b = deq_b;
   p.tile_group = tile_group;
 
-  // CTA pairs (cta_group::2, 256 x 256 tiles, each CTA stages half of B) for the plain bf16 GEMMs whose tile width is
-  // 256: 10-27 % faster than the single-CTA tiles on the benchmark shapes (8192^3 0.71 vs 0.81 ms, LM head 0.64 vs
-  // 0.81 ms).  LIBAI_B200_GEMM_2CTA=0 keeps everything on single-CTA tiles.
-  const int allow_2cta = gemm_allow_2cta();
+  // CTA pairs (cta_group::2, 256 rows x bn columns, each CTA stages half of B).  LIBAI_B200_GEMM_2CTA=0 keeps everything on single-CTA tiles.
   // (fused collectives: shards must hold whole 256-row pair tiles and the copy CTAs come in pairs)
   const bool comm_ok = cp.mode == lb::COMM_NONE ||
                        (cp.rows_per_rank % (2 * lb::BLOCK_M) == 0 && cp.n_comm % 2 == 0 && gemm_allow_2cta() >= 2);
-  const bool two_cta = allow_2cta && bn == 256 && comm_ok && !p.fp8 && M > lb::BLOCK_M && !tile_group;
+  const bool two_cta = pair && pairs_ok && comm_ok;
   // Order of the tiles.  Row by row, the CTAs in flight hold one or two row blocks of A and up to 74 column blocks of B: a B that does
   // not stay in L2 beside the output is read from HBM again for (nearly) every row block (LM head [8192, 1024] x [50304, 1024]: 32 x
   // 103 MB).  In bands of G row blocks they hold G of A and C / G of B, the least bytes at equal sides: G = sqrt(C * columns / rows of a
@@ -1169,7 +1247,7 @@ static int gemm_impl(const void* a, const void* b, void* out, int M, int N, int 
   // ([2048, 4096]ᵀ x [2048, 11008] 152 against 158 us) and keeps the old order.
   p.group_m = 1;
   if (cp.mode == lb::COMM_NONE && !tile_group && epi == 0 && (long)N * K * 2 >= (48L << 20)) {
-    const double in_flight = two_cta ? sms / 2 : sms, side = two_cta ? 1.0 : (double)bn / lb::BLOCK_M;
+    const double in_flight = two_cta ? sms / 2 : sms, side = (double)bn / (two_cta ? 2 * lb::BLOCK_M : lb::BLOCK_M);
     p.group_m = (int)(std::sqrt(in_flight * side) + 0.5);
   }
   CUtensorMap ta, tb, tg, to;
@@ -1210,18 +1288,25 @@ static int gemm_impl(const void* a, const void* b, void* out, int M, int N, int 
 
   cudaError_t e;
   if (two_cta) {
-    if (layout == 0) {
-      if (epi == 0) e = launch_2cta<false, false, lb::EPI_BF16>(ta, tb, tg, to, p, cp, grid, stream);
-      else if (epi == 1) e = launch_2cta<false, false, lb::EPI_F32>(ta, tb, tg, to, p, cp, grid, stream);
-      else e = launch_2cta<false, false, lb::EPI_ATOMIC_F32>(ta, tb, tg, to, p, cp, grid, stream);
+    if (epi == 0 && layout != 2 && bn != 256) {
+      if (layout == 0) e = bn == 192 ? launch_2cta<192, false, false, lb::EPI_BF16>(ta, tb, tg, to, p, cp, grid, stream)
+                                     : launch_2cta<128, false, false, lb::EPI_BF16>(ta, tb, tg, to, p, cp, grid, stream);
+      else e = bn == 192 ? launch_2cta<192, false, true, lb::EPI_BF16>(ta, tb, tg, to, p, cp, grid, stream)
+                         : launch_2cta<128, false, true, lb::EPI_BF16>(ta, tb, tg, to, p, cp, grid, stream);
+    } else if (layout == 0) {
+      if (epi == 0) e = launch_2cta<256, false, false, lb::EPI_BF16>(ta, tb, tg, to, p, cp, grid, stream);
+      else if (epi == 1) e = launch_2cta<256, false, false, lb::EPI_F32>(ta, tb, tg, to, p, cp, grid, stream);
+      else e = launch_2cta<256, false, false, lb::EPI_ATOMIC_F32>(ta, tb, tg, to, p, cp, grid, stream);
     } else if (layout == 1) {
-      if (epi == 0) e = launch_2cta<false, true, lb::EPI_BF16>(ta, tb, tg, to, p, cp, grid, stream);
-      else if (epi == 1) e = launch_2cta<false, true, lb::EPI_F32>(ta, tb, tg, to, p, cp, grid, stream);
-      else e = launch_2cta<false, true, lb::EPI_ATOMIC_F32>(ta, tb, tg, to, p, cp, grid, stream);
+      if (epi == 0) e = launch_2cta<256, false, true, lb::EPI_BF16>(ta, tb, tg, to, p, cp, grid, stream);
+      else if (epi == 1) e = launch_2cta<256, false, true, lb::EPI_F32>(ta, tb, tg, to, p, cp, grid, stream);
+      else e = launch_2cta<256, false, true, lb::EPI_ATOMIC_F32>(ta, tb, tg, to, p, cp, grid, stream);
     } else {
-      if (epi == 0) e = launch_2cta<true, true, lb::EPI_BF16>(ta, tb, tg, to, p, cp, grid, stream);
-      else if (epi == 1) e = launch_2cta<true, true, lb::EPI_F32>(ta, tb, tg, to, p, cp, grid, stream);
-      else e = launch_2cta<true, true, lb::EPI_ATOMIC_F32>(ta, tb, tg, to, p, cp, grid, stream);
+      if (epi == 0) e = launch_2cta<256, true, true, lb::EPI_BF16>(ta, tb, tg, to, p, cp, grid, stream);
+      else if (epi == 1) e = launch_2cta<256, true, true, lb::EPI_F32>(ta, tb, tg, to, p, cp, grid, stream);
+      else if (bn == 192) e = launch_2cta<192, true, true, lb::EPI_ATOMIC_F32>(ta, tb, tg, to, p, cp, grid, stream);
+      else if (bn == 128) e = launch_2cta<128, true, true, lb::EPI_ATOMIC_F32>(ta, tb, tg, to, p, cp, grid, stream);
+      else e = launch_2cta<256, true, true, lb::EPI_ATOMIC_F32>(ta, tb, tg, to, p, cp, grid, stream);
     }
     return (int)e;
   }

@@ -245,17 +245,17 @@ int* small_wait_word() {
 //   this kernel:     3.4 us + 0.03 us per row of the tile + the merge of a cluster (0.1 us of 2, 0.2 us of 4 CTAs, 8 ns per row of the tile
 //                    of 8) + the larger of: the k-blocks of a CTA (0.28 us each with 16 rows, 0.34 with 32 and 64, 0.38 with 128; up to 1.8
 //                    times that where two CTAs share an SM), w at 6 TB/s
-//   gemm_sm100.cu:   4.5 us + the larger of: waves x k-blocks x 0.235 us (64-wide tiles; 0.29 us 128-wide, 0.31 us 192-wide, 0.36 us 256 x 256
-//                    on CTA pairs), w at 6 TB/s
+//   gemm_sm100.cu:   lb_gemm_tile_us
 // Fitted over 350 products, M = 1 .. 2048 and w from [384, 384] to [50304, 1024] and [4096, 11008] (7 % and 3 % rms).  Up to 32 rows this
 // kernel was the better one everywhere (nearest: [32, 1024] x [50304, 1024] 24.8 against 25.3 us); above that it is taken where the estimate
-// is 8 % and 0.5 us ahead: few tiles and a long K ([128, 4096] x [1024, 4096] 9.3 against 19.9 us, [200, 11008] x [4096, 11008] 28.6 against
+// is 4 % and 0.5 us ahead: few tiles and a long K ([128, 4096] x [1024, 4096] 9.3 against 19.9 us, [200, 11008] x [4096, 11008] 28.6 against
 // 46.6), not many tiles ([64, 1024] x [50304, 1024] 27.3 against 23.4 us, [2048, 5120] x [1280, 5120] 39.6 against 29.3) and not a short K
 // ([256, 384] x [1536, 384] 6.2 against 5.8).  Clusters of 4 and 8 are kept to 264 CTAs: the SMs of a GPC do not divide by them, and 72
 // clusters of 4 with two CTAs per SM ran in two waves ([96, 1024] x [3072, 1024] 10.2 against 8.2 us).
 // More than 2048 rows only against one tile of 16 to 128 columns (the gates of a mixer), where the other kernel walks all of K in one CTA:
 // [2560, 2048] x [16, 2048] 9.6 against 11.1 us, x [128, 2048] 9.2 against 11.4, [4096, 4096] x [32, 4096] 9.8 against 18.6, [8192, 4096] x [64, 4096]
 // 14.0 against 19.3; with 8 columns [8192, 4096] 19.7 against 18.9, and [16384, 2048] x [64, 2048] 15.5 against 12.1.
+extern "C" double lb_gemm_tile_us(int M, int N, int K);
 extern "C" int lb_gemm_small_rule(int M, int N, int K, int* nt, int* ranks) {
   if (M > (N < 16 || N > 128 ? 2048 : 8192)) return 0;
   const int kb = (K + 63) / 64, tiles_n = (N + 127) / 128;
@@ -284,18 +284,8 @@ extern "C" int lb_gemm_small_rule(int M, int N, int K, int* nt, int* ranks) {
     }
   }
   if (M <= 32) return 1;
-  double old_us = 1e30;
-  const int bns[4] = {64, 128, 192, 256};
-  const double slope[4] = {0.235, 0.29, 0.31, 0.36};
-  for (int i = 0; i < 4; ++i) {
-    const long tiles = i == 3 ? (long)((M + 255) / 256) * ((N + 255) / 256) : (long)((M + 127) / 128) * ((N + bns[i] - 1) / bns[i]);
-    const long slots = i == 3 ? 74 : 148;
-    const double us = (double)((tiles + slots - 1) / slots) * kb * slope[i];
-    if (us < old_us) old_us = us;
-  }
-  if (w_us > old_us) old_us = w_us;
-  old_us += 4.5;
-  return best * 1.08 < old_us && best + 0.5 < old_us;
+  const double old_us = lb_gemm_tile_us(M, N, K);
+  return best * 1.04 < old_us && best + 0.5 < old_us;
 }
 
 // Returns 0, a cudaError_t, or a negative code for unsupported arguments (-20: an earlier launch's wait ran out).

@@ -1092,3 +1092,27 @@ def test_weight_gradient_accumulates_in_boxes(m, n, k):
     assert bool(((buf[1:m + 1, 4:n + 4].double() - want).abs() <= bound).all())
     buf[1:m + 1, 4:n + 4] = before[1:m + 1, 4:n + 4]
     assert torch.equal(buf, before)
+
+
+@pytest.mark.parametrize("bn", [64, 128, 192, -128, -192, -256])
+@pytest.mark.parametrize("layout", [0, 1, 2])
+@pytest.mark.parametrize("m,n,k", [(129, 136, 64), (256, 192, 72), (300, 200, 840), (1400, 1160, 136), (2500, 776, 264)])
+def test_gemm_tiles_of_every_width(bn, layout, m, n, k):
+    """Single CTAs' tiles and CTA pairs' (negative), whatever the rule picks: rows and columns that end inside a tile and inside a pair's half, one wave and
+    several, nothing written behind the last column.  Whole numbers, exact in every format."""
+    if layout == 2:
+        m = (m + 7) // 8 * 8
+    if layout == 2 and bn in (64, 128, 192) and n < bn // 2:
+        pytest.skip("not a tile for so few columns")
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    ints = lambda *s: (torch.rand(*s, generator=g, device="cuda") < 0.2).to(BF16) * torch.randint(-1, 2, s, generator=g, device="cuda").to(BF16)
+    a, b = ints(*((k, m) if layout == 2 else (m, k))), ints(*((n, k) if layout == 0 else (k, n)))
+    out = torch.full((m, n + 8), 3.0, device="cuda", dtype=torch.float32 if layout == 2 else BF16)
+    lib = ctypes.CDLL(so_path())
+    ptr = lambda t: ctypes.c_void_p(t.data_ptr())
+    rc = lib.lb_gemm_bf16(ptr(a), ptr(b), ptr(out), m, n, k, a.shape[1], b.shape[1], n + 8, layout, 2 if layout == 2 else 0, ctypes.c_void_p(0), 0,
+                          ctypes.c_void_p(0), bn, 0, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    want = (a.float().t() if layout == 2 else a.float()) @ (b.float().t() if layout == 0 else b.float())
+    assert want.abs().max() < 256
+    assert torch.equal(out[:, :n].float(), want + (3.0 if layout == 2 else 0.0)) and bool((out[:, n:] == 3).all())
