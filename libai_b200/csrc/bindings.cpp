@@ -1,6 +1,5 @@
 // torch.ops.libai_b200.* : thin argument-checking wrappers around the extern "C" kernel launchers.
-// Registered with TORCH_LIBRARY so the in-tree `_C.so` is loaded by torch.ops.load_library (no
-// python ABI dependency).
+// Registered with TORCH_LIBRARY so the in-tree `_C.so` is loaded by torch.ops.load_library.
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAGeneratorImpl.h>
 #include <cstring>
@@ -10,6 +9,8 @@
 #include <torch/torch.h>
 
 #include <tuple>
+
+#include "ops.h"
 
 extern "C" {
 int lb_gemm_bf16(const void* a, const void* b, void* out, int M, int N, int K, int lda, int ldb, int ldo, int layout,
@@ -114,7 +115,7 @@ int lb_bias_dropout_residual(const void* x, const void* bias, const void* res, v
                              const LbRngArgs* rng, const long long* rng_in, long long* rng_out, cudaStream_t s);
 }
 
-namespace {
+namespace lb_ops {       // (autograd_nodes.cpp calls these too: ops.h)
 
 using at::Tensor;
 
@@ -1249,9 +1250,10 @@ void p2p_allgather(const Tensor& shard, at::IntArrayRef out_ptrs, at::IntArrayRe
         "p2p_allgather");
 }
 
-}  // namespace
+}  // namespace lb_ops
 
 TORCH_LIBRARY(libai_b200, m) {
+  using namespace lb_ops;
   m.def("ag_gemm(Tensor gathered, Tensor shard, Tensor w, int layout, Tensor? bias, int act, bool need_pre, Tensor? pre_in, Tensor(a!)? colsum, bool fill_local, int world, int rank, int[] peer_buf, int[] peer_flags, int[] peer_done, Tensor(b!) state, int n_comm) -> (Tensor, Tensor)", &ag_gemm);
   m.def("ag_wgrad(Tensor gy, Tensor gathered, Tensor shard, Tensor(a!) out, bool accumulate, int world, int rank, int[] peer_buf, int[] peer_flags, int[] peer_done, Tensor(b!) state, int n_comm) -> ()", &ag_wgrad);
   m.def("gemm_rs(Tensor x, Tensor w, int layout, Tensor? bias, Tensor? residual, int world, int rank, int[] peer_buf, int[] peer_flags, int[] peer_done, Tensor(a!) state, int staging_parity_off) -> Tensor", &gemm_rs);

@@ -30,6 +30,14 @@ def applies(x) -> bool:
             and OF._plain_call() and not ops.fp8_enabled() and dutil.get_dist_util().tensor_parallel_size == 1 and not _calls_are_seen())
 
 
+def applies_with_graph(x) -> bool:
+    """The same for a call with a graph: a block's nodes made in one call (``block_nodes``, ``llama_block_nodes`` in ``csrc/autograd_nodes.cpp``)."""
+    if not (OF._graph_node(x) and x.dtype is torch.bfloat16 and x.dim() == 3 and ops.use_native(x)) or _calls_are_seen():
+        return False
+    topo = dutil.get_dist_util()
+    return topo.tensor_parallel_size == 1 and not topo.sequence_parallel and not topo.fused_tp_comm
+
+
 def _calls_are_seen() -> bool:
     """Does anything look at the call of every module: global hooks, a replaced ``Module.__call__``?"""
     return bool(_module._global_forward_hooks or _module._global_forward_pre_hooks or _module._global_backward_hooks or _module._global_backward_pre_hooks
@@ -44,9 +52,14 @@ def plain(m, cls) -> bool:
     return not own["_forward_hooks"] and not own["_forward_pre_hooks"] and "_compiled_call_impl" not in own and "forward" not in own
 
 
+def plain_with_graph(m, cls) -> bool:
+    """The same for a call with a graph, where the module's backward hooks count too."""
+    return plain(m, cls) and not m._backward_hooks and not m._backward_pre_hooks
+
+
 def alone(m, cls) -> bool:
     """Would nobody notice if this module were passed by, its work joined with a neighbour's, with a graph or without?"""
-    return plain(m, cls) and not m._backward_hooks and not m._backward_pre_hooks and not _calls_are_seen()
+    return plain_with_graph(m, cls) and not _calls_are_seen()
 
 
 def parameters(*pairs):

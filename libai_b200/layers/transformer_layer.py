@@ -8,11 +8,11 @@ The pipeline hand-off the reference performs inside ``forward`` (``to_global(pla
 """
 from torch import nn
 
-from libai_b200.ops import count_launch, load_ext
+from libai_b200.ops import count_launch, functional as OF, fused_bias_grad, load_ext
 
 from . import _native_block as native
 from ._param import xavier_normal_
-from .attention import AttnMaskType, MultiheadAttention
+from .attention import AttnMaskType, KeyPaddingMask, MultiheadAttention
 from .droppath import DropPath
 from .layer_norm import LayerNorm
 from .linear import Linear
@@ -99,6 +99,10 @@ class TransformerLayer(nn.Module):
             done = self._native_forward(hidden_states, past_key_value, use_cache)
             if done is not None:
                 return done
+        elif past_key_value is None and not use_cache and native.applies_with_graph(hidden_states):
+            done = self._graph_forward(hidden_states, attention_mask, encoder_states, encoder_attention_mask)
+            if done is not None:
+                return done
         self_past = cross_past = None
         if past_key_value is not None:
             self_past = past_key_value[:2]
@@ -170,6 +174,61 @@ class TransformerLayer(nn.Module):
             return None
         count_launch(7)
         return (out[0], tuple(out[1:])) if use_cache else out[0]
+
+    def _graph_forward(self, x, mask, enc, cross_mask):
+        """The block's graph as one native call; ``None``: the modules have to run."""
+        if self.apply_residual_post_layernorm or not self.plain_residual or self.is_decoder != (enc is not None):
+            return None
+        mods = self._modules
+        plain = native.plain_with_graph
+        attn, mlp = mods["self_attention"], mods["mlp"]
+        if not (plain(attn, MultiheadAttention) and plain(mlp, MLP)) or (mlp.training and mlp.output_dropout_prob > 0.0):
+            return None
+        parts = [(mods["input_layernorm"], LayerNorm), (attn._modules.get("query_key_value"), Linear), (attn._modules["dense"], Linear)]
+        cross = None
+        if enc is not None:
+            cross = mods["cross_attention"]
+            if not plain(cross, MultiheadAttention) or not OF._graph_node(enc) or enc.dim() != 3 or cross.local_heads != attn.local_heads:
+                return None
+            parts += [(mods["post_attention_layernorm"], LayerNorm), (cross._modules.get("query"), Linear), (cross._modules.get("key_value"), Linear),
+                      (cross._modules["dense"], Linear), (mods["post_cross_attention_layernorm"], LayerNorm)]
+        else:
+            parts.append((mods["post_attention_layernorm"], LayerNorm))
+        parts += [(mlp._modules["dense_h_to_4h"], Linear), (mlp._modules["dense_4h_to_h"], Linear)]
+        for m, cls in parts:
+            if m is None or not plain(m, cls) or (cls is LayerNorm and len(m.normalized_shape) != 1):
+                return None
+        if attn._modules["query_key_value"].skip_bias_add or mlp._modules["dense_h_to_4h"].skip_bias_add:
+            return None
+        for a in (attn, cross):
+            if a is not None and a.training and (a.attention_dropout_prob > 0.0 or a.output_dropout_prob > 0.0):
+                return None
+        params = native.parameters(*((m, "weight", "bias") for m, _ in parts))
+        if params is None:
+            return None
+        # the kernels that ``MultiheadAttention.forward`` would pick: flash (head dims 64 and 128, lengths of a right-padded batch) or with 32-bit probabilities
+        (b, s, _), heads, d, lens = x.shape, attn.local_heads, attn.head_size, None
+        causal = attn.attn_mask_type == AttnMaskType.causal
+        if isinstance(mask, KeyPaddingMask):
+            if d in (64, 128) and mask.is_prefix():
+                mask, lens = None, mask.lengths
+            else:
+                mask = mask.dense()
+        if ((mask is not None or d not in (64, 128)) and not self._split_attention_takes(x, mask, (b, heads, s), s, d, attn.softmax_scale, causal and mask is None)
+                or not OF._graph_node(mask, lens)):
+            return None
+        if cross is not None:
+            if isinstance(cross_mask, KeyPaddingMask):
+                cross_mask = cross_mask.dense()
+            if not self._split_attention_takes(x, cross_mask, (b, heads, s), enc.shape[1], cross.head_size, cross.softmax_scale, False) or not OF._graph_node(cross_mask):
+                return None
+        out = load_ext().block_nodes(x, params, heads, [m.eps for m, cls in parts if cls is LayerNorm], float(attn.softmax_scale), causal, lens, mask, enc, cross_mask,
+                                     0.0 if cross is None else float(cross.softmax_scale), fused_bias_grad())
+        return out[0] if out else None
+
+    @staticmethod
+    def _split_attention_takes(x, mask, q_sizes, keys, d, scale, causal):
+        return OF._split_sizes_ok(*q_sizes, keys, d, scale, causal) and (mask is None or OF._mask_supported(mask, q_sizes, x.device, keys))
 
     def build_attention(self, is_cross_attention=False):
         return MultiheadAttention(

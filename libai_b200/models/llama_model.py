@@ -221,6 +221,10 @@ class LlamaDecoderLayer(nn.Module):
             done = self._native_forward(hidden_states, past_key_value, cos_cached, sin_cached, use_cache)
             if done is not None:
                 return done
+        elif attention_mask is None and past_key_value is None and not use_cache and native.applies_with_graph(hidden_states):
+            done = self._graph_forward(hidden_states, cos_cached, sin_cached)
+            if done is not None:
+                return done
         ln, skip = self._norm(self.input_layernorm, hidden_states)
         call = dict(attention_mask=attention_mask, past_key_value=past_key_value, cos_cached=cos_cached, sin_cached=sin_cached, use_cache=use_cache)
         presents = None
@@ -243,14 +247,11 @@ class LlamaDecoderLayer(nn.Module):
             return OF.rms_norm_with_skip(x, norm.weight, norm.eps)
         return norm(x), x
 
-    def _native_forward(self, x, past, cos, sin, use_cache):
-        """The block without a graph as one native call; ``None``: the modules have to run."""
-        from libai_b200.ops import gated_mlp
-
+    def _native_parts(self, plain, cos, sin):
+        """``(attention, its norm, the other norm, seven weights, bias of qkv)`` where a native call can stand for the modules, else ``None``."""
         mods = self._modules
         ln1, attn, ln2, mlp = mods["input_layernorm"], mods["self_attn"], mods["post_attention_layernorm"], mods["mlp"]
-        plain = native.plain
-        if not (plain(ln1, RMSLayerNorm) and plain(attn, LlamaAttention) and plain(ln2, RMSLayerNorm) and plain(mlp, LlamaMLP)) or (use_cache and past is None):
+        if not (plain(ln1, RMSLayerNorm) and plain(attn, LlamaAttention) and plain(ln2, RMSLayerNorm) and plain(mlp, LlamaMLP)):
             return None
         qkv, proj = attn._modules["query_key_value"], attn._modules["o_proj"]
         gate, up, down = mlp._modules["gate_proj"], mlp._modules["up_proj"], mlp._modules["down_proj"]
@@ -259,10 +260,31 @@ class LlamaDecoderLayer(nn.Module):
                 or any(m._parameters.get("bias") is not None for m in (proj, gate, up, down)) or type(cos) is not torch.Tensor or type(sin) is not torch.Tensor):
             return None
         params = native.parameters((ln1, "weight"), (qkv, "weight"), (proj, "weight"), (ln2, "weight"), (gate, "weight"), (up, "weight"), (down, "weight"))
-        pair = native.past_pair(past, attn.local_heads, x)
         bias = qkv._parameters.get("bias")
-        if params is None or pair is None or (bias is not None and type(bias) is not nn.Parameter):
+        if params is None or (bias is not None and type(bias) is not nn.Parameter):
             return None
+        return attn, ln1, ln2, params, bias
+
+    def _graph_forward(self, x, cos, sin):
+        """The block's graph as one native call; ``None``: the modules have to run."""
+        from libai_b200.ops import gated_mlp
+
+        parts = self._native_parts(native.plain_with_graph, cos, sin) if gated_mlp.enabled() else None
+        if parts is None or not OF._graph_node(cos, sin):
+            return None
+        attn, ln1, ln2, params, bias = parts
+        out = load_ext().llama_block_nodes(x, params, bias, cos, sin, attn.local_heads, ln1.eps, ln2.eps, attn.norm_factor)
+        return out[0] if out else None
+
+    def _native_forward(self, x, past, cos, sin, use_cache):
+        """The block without a graph as one native call; ``None``: the modules have to run."""
+        from libai_b200.ops import gated_mlp
+
+        parts = None if use_cache and past is None else self._native_parts(native.plain, cos, sin)
+        pair = None if parts is None else native.past_pair(past, parts[0].local_heads, x)
+        if pair is None:
+            return None
+        attn, ln1, ln2, params, bias = parts
         out = load_ext().llama_block_fwd(x, params, bias, cos, sin, attn.local_heads, ln1.eps, ln2.eps, attn.norm_factor, gated_mlp.enabled(), *pair)
         if not out:
             return None

@@ -167,13 +167,15 @@ def count_launch(n: int = 1) -> None:
 
 
 def launch_count() -> int:
-    """Number of native kernel launches issued through the python wrappers (bench bookkeeping)."""
-    return _LAUNCH_COUNT
+    """Number of native kernel launches issued through the python wrappers and the C++ graph nodes (bench bookkeeping)."""
+    return _LAUNCH_COUNT + (0 if _EXT is None else _EXT.launched(False))
 
 
 def reset_launch_count() -> None:
     global _LAUNCH_COUNT
     _LAUNCH_COUNT = 0
+    if _EXT is not None:
+        _EXT.launched(True)
 
 
 # --------------------------------------------------------------------------------------

@@ -16,6 +16,7 @@ import hashlib
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -26,7 +27,7 @@ CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 NVCC = os.path.join(CUDA_HOME, "bin", "nvcc")
 
 CU_SOURCES = ["gemm_sm100.cu", "gemm_small_sm100.cu", "norm.cu", "elementwise.cu", "attention_sm100.cu", "attention_fwd_sm100.cu", "attention_bwd128_sm100.cu", "attention_split_sm100.cu", "attention_decode.cu", "latent_attention_sm100.cu", "masked_attention_sm100.cu", "comm_kernels.cu"]
-CPP_SOURCES = ["bindings.cpp", "symm_mem.cpp"]
+CPP_SOURCES = ["bindings.cpp", "autograd_nodes.cpp", "symm_mem.cpp"]
 SEQ_SO_PATH = os.path.join(ROOT, "_C_seq.so")
 SEQ_CU_SOURCES = ["seq_mixers.cu"]
 SEQ_CPP_SOURCES = ["seq_bindings.cpp"]
@@ -90,7 +91,7 @@ def _build_lib(SO_PATH, CU_SOURCES, CPP_SOURCES, NVCC_FLAGS, ext_name, force, ve
         objs.append(obj)
         if force or _stale(src, obj, headers):
             jobs.append((s, [NVCC, *NVCC_FLAGS, "-I", CSRC, "-c", src, "-o", obj]))
-    inc = []
+    inc = ["-isystem", sysconfig.get_paths()["include"]]
     for p in cpp_extension.include_paths(device_type="cuda"):
         inc += ["-isystem", p]
     abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
@@ -113,7 +114,7 @@ def _build_lib(SO_PATH, CU_SOURCES, CPP_SOURCES, NVCC_FLAGS, ext_name, force, ve
         tlib = os.path.join(os.path.dirname(torch.__file__), "lib")
         tmp_so = f"{SO_PATH}.{os.getpid()}.tmp"         # link beside the target, then rename: a reader never sees half a file
         _run(["g++", "-shared", "-o", tmp_so, *objs, f"-L{tlib}", "-lc10", "-ltorch_cpu", "-ltorch", "-lc10_cuda",
-              "-ltorch_cuda", f"-L{os.path.join(CUDA_HOME, 'lib64')}", "-lcudart",
+              "-ltorch_cuda", *(["-ltorch_python"] if "autograd_nodes.cpp" in cpp else []), f"-L{os.path.join(CUDA_HOME, 'lib64')}", "-lcudart",
               f"-Wl,-rpath,{tlib}", f"-Wl,-rpath,{os.path.join(CUDA_HOME, 'lib64')}"], verbose)
         os.replace(tmp_so, SO_PATH)
     return SO_PATH

@@ -46,6 +46,20 @@ def _call(fn, *args):
     return fn.forward(_NoGradContext(), *args)
 
 
+_PLAIN_TYPES = (torch.Tensor, torch.nn.Parameter)
+
+
+def _graph_node(*tensors) -> bool:
+    """Does this call record a graph that the C++ nodes (csrc/autograd_nodes.cpp) can stand for?  Not where a call is transformed, traced or compiled or a
+    dispatch mode looks at its operators, not for subclasses, not for fp8 products: those take the autograd functions below."""
+    if not torch.is_grad_enabled() or ops.fp8_enabled() or not _plain_call() or torch._C._len_torch_dispatch_stack() or torch.compiler.is_compiling():
+        return False
+    for t in tensors:
+        if t is not None and (type(t) not in _PLAIN_TYPES or not t.is_cuda):
+            return False
+    return True
+
+
 # --------------------------------------------------------------------------------------
 # activations (reference math)
 # --------------------------------------------------------------------------------------
@@ -201,6 +215,8 @@ class _LinearFn(torch.autograd.Function):
 def linear(x, w, bias=None, act: Optional[str] = None):
     """``act(x @ w.T + bias)``; ``w`` is ``[out, in]``."""
     if use_native(x, w) and _gemm_ok(x, w):
+        if _graph_node(x, w, bias):
+            return load_ext().linear_node(x, w, bias, _ACT_IDS[act])
         return _call(_LinearFn, x, w, bias, act)
     y = F.linear(x, w.to(x.dtype) if w.dtype != x.dtype else w, None if bias is None else bias.to(x.dtype))
     return _act_ref(y, act)
@@ -279,6 +295,8 @@ def mlp(x, w1, b1, w2, act: str = "gelu", b2=None, residual=None):
     """``act(x @ w1ᵀ + b1) @ w2ᵀ``; with ``residual`` also ``+ b2 + residual`` in the second GEMM's epilogue
     (without it the second bias is left to the fused bias+dropout+residual op)."""
     if use_native(x, w1) and _gemm_ok(x, w1) and _gemm_ok(x.new_empty(1, w1.shape[0]), w2):
+        if _graph_node(x, w1, b1, w2, b2, residual):
+            return load_ext().mlp_node(x, w1, b1, w2, _ACT_IDS[act], None if residual is None else b2, residual, ops.fused_bias_grad())
         if residual is not None:
             return _call(_MLPFn, x, w1, b1, w2, act, b2, residual)
         return _call(_MLPFn, x, w1, b1, w2, act)
@@ -328,6 +346,8 @@ class _LinearResidualFn(torch.autograd.Function):
 def linear_bias_residual(x, w, bias, residual):
     """``x @ wᵀ + bias + residual`` (output projection of a block, dropout-free)."""
     if use_native(x, w) and _gemm_ok(x, w) and residual is not None and residual.dtype == torch.bfloat16:
+        if _graph_node(x, w, bias, residual):
+            return load_ext().linear_residual_node(x, w, bias, residual)
         return _call(_LinearResidualFn, x, w, bias, residual)
     y = linear(x, w, bias)
     return y if residual is None else y + residual
@@ -387,12 +407,16 @@ class _LayerNormFn(torch.autograd.Function):
 def layer_norm_with_skip(x, weight, bias, eps: float = 1e-5):
     """``(layer_norm(x), x)`` where the second output carries the skip connection (see ``_LayerNormFn``)."""
     if use_native(x) and x.dtype in (torch.bfloat16, torch.float32) and weight is not None and x.requires_grad:
+        if _graph_node(x, weight, bias):
+            return load_ext().norm_skip_node(x, weight, bias, eps, False)
         return _call(_LayerNormFn, x, weight, bias, eps, False, True)
     return layer_norm(x, weight, bias, eps), x
 
 
 def layer_norm(x, weight, bias, eps: float = 1e-5):
     if use_native(x) and x.dtype in (torch.bfloat16, torch.float32) and weight is not None:
+        if _graph_node(x, weight, bias):
+            return load_ext().norm_node(x, weight, bias, eps, False)
         return _call(_LayerNormFn, x, weight, bias, eps, False)
     w = None if weight is None else weight.float()
     b = None if bias is None else bias.float()
@@ -402,12 +426,16 @@ def layer_norm(x, weight, bias, eps: float = 1e-5):
 def rms_norm_with_skip(x, weight, eps: float = 1e-6):
     """``(rms_norm(x), x)``; the gradient of the second output is added inside the norm's backward kernel (see ``_LayerNormFn``)."""
     if use_native(x) and x.dtype in (torch.bfloat16, torch.float32) and x.requires_grad:
+        if _graph_node(x, weight):
+            return load_ext().norm_skip_node(x, weight, None, eps, True)
         return _call(_LayerNormFn, x, weight, None, eps, True, True)
     return rms_norm(x, weight, eps), x
 
 
 def rms_norm(x, weight, eps: float = 1e-6):
     if use_native(x) and x.dtype in (torch.bfloat16, torch.float32):
+        if _graph_node(x, weight):
+            return load_ext().norm_node(x, weight, None, eps, True)
         return _call(_LayerNormFn, x, weight, None, eps, True)
     xf = x.float()
     y = xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + eps)
@@ -686,6 +714,17 @@ def _split_supported(q, k, v, scale, causal, mask) -> bool:
             and (mask is None or _mask_supported(mask, q.shape[:3], q.device, k.shape[2])) and type(q) is not FakeTensor and _plain_call())
 
 
+def _split_graph_backward(go, layout: str, causal: bool, scale: float, mask, ts, needed) -> list:
+    """Gradients of ``ts`` with a graph of their own: the unfused form is differentiated."""
+    out = attention_ref(*_split_views(layout, ts), causal=causal, scale=scale, mask=mask)
+    out = out if layout == "q_k_v" else out.permute(0, 2, 1, 3)
+    grads = iter(torch.autograd.grad(out, [t for t, n in zip(ts, needed) if n], go, create_graph=True))
+    return [next(grads) if n else None for n in needed]
+
+
+_SPLIT_LAYOUTS = {"qkv": 0, "q_kv": 1, "q_k_v": 2}
+
+
 class _SplitAttnFn(torch.autograd.Function):
     """Attention whose probabilities reach the tensor core as two bf16 parts (``layout``: see :func:`_split_views`)."""
 
@@ -707,12 +746,8 @@ class _SplitAttnFn(torch.autograd.Function):
     def backward(ctx, go):
         o32, lse, words, fill, *ts = ctx.saved_tensors
         q, k, v = _split_views(ctx.layout, ts)
-        if torch.is_grad_enabled():            # a graph of the gradients is wanted: differentiate the unfused form
-            out = attention_ref(q, k, v, causal=ctx.causal, scale=ctx.scale, mask=ctx.mask)
-            out = out if ctx.layout == "q_k_v" else out.permute(0, 2, 1, 3)
-            need = [t for t, n in zip(ts, ctx.needs_input_grad[4:]) if n]
-            grads = iter(torch.autograd.grad(out, need, go, create_graph=True))
-            return (None,) * 4 + tuple(next(grads) if n else None for n in ctx.needs_input_grad[4:])
+        if torch.is_grad_enabled():
+            return (None,) * 4 + tuple(_split_graph_backward(go, ctx.layout, ctx.causal, ctx.scale, ctx.mask, ts, ctx.needs_input_grad[4:]))
         if ctx.layout == "q_k_v":              # gradients backed by [b, s, a, d], as the projections around an attention read them
             gs = [torch.empty(t.shape[0], t.shape[2], t.shape[1], t.shape[3], dtype=t.dtype, device=t.device).permute(0, 2, 1, 3) for t in ts]
         else:
@@ -734,6 +769,8 @@ def attention_packed(layout: str, ts, *, causal: bool, scale: float, mask=None, 
             or (layout == "q_kv" and y.shape != (b, y.shape[1], a, 2 * d)) or (layout == "qkv" and x.shape[3] != 3 * d)
             or (mask is not None and not _mask_supported(mask, (b, a, sq), x.device, y.shape[1]))):
         return None
+    if _graph_node(mask, *ts):
+        return load_ext().split_attention_node(list(ts), causal, float(scale), mask, _SPLIT_LAYOUTS[layout])
     return _call(_SplitAttnFn, layout, causal, float(scale), mask, *ts)
 
 
@@ -785,6 +822,8 @@ def attention_qkvpacked(qkv, *, causal: bool, scale: float, kv_lens=None, dropou
     of a right-padded batch (keys beyond it are masked inside the kernel); ``dropout_p`` > 0 in training drops
     attention probabilities inside the kernel (Philox, TP-rank salted)."""
     p = float(dropout_p) if training else 0.0
+    if _graph_node(qkv, kv_lens, alibi_slopes):
+        return load_ext().flash_packed_node(qkv, causal, float(scale), kv_lens, p, alibi_slopes, tp_rng_salt(True) if p > 0 else 0)
     return _call(_FlashAttnPackedFn, qkv, causal, float(scale), kv_lens, p, alibi_slopes)
 
 
@@ -812,6 +851,8 @@ def attention(q, k, v, *, causal: bool = False, scale: Optional[float] = None, m
             and _split_supported(q, k, v, scale, causal, mask)):
         ts = [t if _rows_of_vectors(t) else t.contiguous() for t in (q, k, v)]
         if all(_rows_of_vectors(t) for t in ts):
+            if _graph_node(mask, *ts):
+                return load_ext().split_attention_node(ts, causal, float(scale), mask, 2)
             return _call(_SplitAttnFn, "q_k_v", causal, float(scale), mask, *ts)
     if alibi_slopes is not None:
         sq, sk = q.shape[-2], k.shape[-2]
@@ -883,8 +924,11 @@ class _VocabParallelCE(torch.autograd.Function):
 def vocab_parallel_cross_entropy(logits, labels, vocab_start: int = 0, group=None):
     """logits ``[..., V/t]``, labels ``[...]`` (global ids) → per-token loss ``[...]`` (fp32)."""
     shp = labels.shape
-    out = _call(_VocabParallelCE, logits.reshape(-1, logits.shape[-1]), labels.reshape(-1), vocab_start, group)
-    return out.view(shp)
+    rows, flat = logits.reshape(-1, logits.shape[-1]), labels.reshape(-1)
+    if (_graph_node(logits, labels) and (group is None or dist.get_world_size(group) == 1) and use_native(logits)
+            and logits.dtype in (torch.bfloat16, torch.float32)):
+        return load_ext().cross_entropy_node(rows, flat, int(vocab_start)).view(shp)
+    return _call(_VocabParallelCE, rows, flat, vocab_start, group).view(shp)
 
 
 # --------------------------------------------------------------------------------------
@@ -994,6 +1038,8 @@ def apply_rotary_qkv(qkv, cos, sin, pos_offset: int = 0):
     """qkv ``[b, s, a, 3d]`` (per-head ``[q|k|v]``); cos/sin fp32 ``[max_pos, d]``; token ``i`` of the
     sequence uses position ``i + pos_offset``."""
     if use_native(qkv) and qkv.dtype == torch.bfloat16 and cos.dtype == torch.float32 and qkv.is_contiguous():
+        if _graph_node(qkv, cos, sin):
+            return load_ext().rope_qkv_node(qkv, cos, sin, int(pos_offset))
         return _call(_RopeQKVFn, qkv, cos, sin, int(pos_offset))
     d = qkv.shape[-1] // 3
     s_len = qkv.shape[1]

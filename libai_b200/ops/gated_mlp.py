@@ -19,7 +19,7 @@ from typing import Optional, Tuple
 import torch
 
 from libai_b200.ops import count_launch, load_ext
-from libai_b200.ops.functional import _call
+from libai_b200.ops.functional import _call, _graph_node
 
 _ENABLED = os.environ.get("LIBAI_B200_FUSED_GATE_UP", "1") == "1"
 
@@ -163,6 +163,8 @@ class TPGatedMLPFused(torch.autograd.Function):
 
 
 def gated_mlp(x, wg, wu, wd, residual=None):
+    if _graph_node(x, wg, wu, wd, residual):
+        return load_ext().gated_mlp_node(x, wg, wu, wd, residual)
     if residual is None:
         return _call(GatedMLPFn, x, wg, wu, wd)
     return _call(GatedMLPFn, x, wg, wu, wd, residual)

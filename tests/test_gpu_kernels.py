@@ -1116,3 +1116,103 @@ def test_gemm_tiles_of_every_width(bn, layout, m, n, k):
     want = (a.float().t() if layout == 2 else a.float()) @ (b.float().t() if layout == 0 else b.float())
     assert want.abs().max() < 256
     assert torch.equal(out[:, :n].float(), want + (3.0 if layout == 2 else 0.0)) and bool((out[:, n:] == 3).all())
+
+
+def _train_block(kind, dim, with_main_grad):
+    """A block, its call and its inputs: causal, right-padded, without a mask, T5 decoder, Llama."""
+    from libai_b200.layers import TransformerLayer
+    from libai_b200.layers._param import param_defaults
+    from libai_b200.layers.attention import AttnMaskType, KeyPaddingMask
+    from libai_b200.models.llama_model import LlamaDecoderLayer, rotary_tables
+    from libai_b200.optim import AdamW, get_default_optimizer_params
+
+    heads, s = 4, 40
+    hidden = heads * dim
+    with param_defaults(dtype=BF16, device="cuda", seed=1):
+        if kind == "llama":
+            layer = LlamaDecoderLayer(hidden, 256, heads, rms_norm_eps=1e-6, max_position_embeddings=64)
+        else:
+            layer = TransformerLayer(hidden, 2 * hidden, heads, is_decoder=kind == "decoder",
+                                     attn_mask_type=AttnMaskType.causal if kind == "causal" else AttnMaskType.padding)
+        for i, p in enumerate(layer.parameters()):
+            p.data.copy_(_rand(p.shape, 10 + i, 0.05 if p.dim() > 1 else 0.1) + (p.dim() == 1))
+    if with_main_grad or kind == "llama":       # (one buffer: gate and up weights side by side)
+        opt = AdamW(get_default_optimizer_params(layer), lr=1e-3)
+        opt.setup()
+    x = _rand((3, s, hidden), 2).requires_grad_(True)
+    if kind == "llama":
+        cos, sin = rotary_tables(dim, 64, device="cuda")
+        return layer, lambda: layer(x, cos_cached=cos, sin_cached=sin), [x]
+    if kind == "decoder":
+        enc = _rand((3, 24, hidden), 3).requires_grad_(True)
+        m = torch.ones(3, 1, s, s, dtype=torch.bool, device="cuda").tril()
+        cm = (torch.arange(24, device="cuda") < 20).expand(3, 1, s, 24)
+        return layer, lambda: layer(x, m, enc, cm), [x, enc]
+    mask = KeyPaddingMask((torch.arange(s, device="cuda")[None] < torch.tensor([[s], [17], [1]], device="cuda")).long()) if kind == "padded" else None
+    return layer, lambda: layer(x, mask), [x]
+
+
+@pytest.mark.parametrize("main_grad", [False, True])
+@pytest.mark.parametrize("kind,dim", [("causal", 64), ("causal", 24), ("padded", 128), ("padded", 48), ("none", 32), ("decoder", 32), ("decoder", 64), ("llama", 128)])
+def test_block_graph_in_one_call(kind, dim, main_grad):
+    """One node per block, one per operator (a hook on a module) and the Python functions (a dispatch mode looks on) launch the same kernels: outputs to
+    the bit, gradients up to the order of their sums; a second backward pass, checkpointing, frozen parameters and a graph of the gradients work as with the modules."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+    from torch.utils.checkpoint import checkpoint
+
+    class Look(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    def grads(how):
+        layer, call, inputs = _train_block(kind, dim, main_grad)
+        params = list(layer.parameters())
+        if how == "nodes":
+            layer.input_layernorm.register_forward_hook(lambda *a: None)
+        if how == "python":
+            with Look():
+                y = call()
+        elif how == "checkpoint":
+            y = checkpoint(lambda *_: call(), *inputs, use_reentrant=False)
+        else:
+            y = call()
+        assert ("Block" in type(y.grad_fn).__name__ or "Block" in y.grad_fn.name()) == (how in ("block", "checkpoint")), y.grad_fn.name()
+        gy = _rand(y.shape, 5)
+        y.backward(gy, retain_graph=True)
+        if how == "block":
+            y.backward(gy)                       # twice: all gradients double
+        out = [t.grad for t in inputs] + [p.main_grad if getattr(p, "main_grad", None) is not None else p.grad for p in params]
+        assert all(g is not None for g in out) and all(p.grad_added_to_main_grad for p in params if getattr(p, "main_grad", None) is not None)
+        return y.detach(), [g.double() / (2 if how == "block" else 1) for g in out]
+
+    want, wg = grads("python")
+    for how in ("block", "nodes", "checkpoint"):
+        y, got = grads(how)
+        assert torch.equal(y, want)
+        for a, b in zip(got, wg):
+            # one bf16 rounding of an operator's result (2^-9) where sums met in another order, a few operators deep
+            assert float((a - b).norm()) <= 2.0 ** -7 * float(b.norm()), how
+    layer, call, inputs = _train_block(kind, dim, main_grad)
+    for p in layer.mlp.parameters():
+        p.requires_grad_(False)
+    y = call()
+    assert "Block" not in y.grad_fn.name()
+    y.backward(_rand(y.shape, 5))
+    assert float((inputs[0].grad.double() - wg[0]).norm()) <= 2.0 ** -7 * float(wg[0].norm())
+    layer, call, inputs = _train_block(kind, dim, main_grad)
+    y = call()
+    g = torch.autograd.grad(y, inputs, _rand(y.shape, 5), create_graph=True)
+    assert float((g[0].double() - wg[0]).norm()) <= 2.0 ** -7 * float(wg[0].norm())
+
+
+def test_block_graph_refuses_what_changed_in_between():
+    layer, call, inputs = _train_block("causal", 64, True)
+    y = call()
+    with torch.no_grad():
+        layer.mlp.dense_4h_to_h.weight.add_(1)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        y.backward(_rand(y.shape, 5))
+    y = call()
+    y.backward(_rand(y.shape, 5))
+    with pytest.raises(RuntimeError, match="second time"):
+        y.backward(_rand(y.shape, 5))
