@@ -17,9 +17,9 @@
 // whatever the constant (0 keeps its log-sum-exp small and exact).
 //
 // Bounded by the softmax threads (two passes over S, three roundings per probability), not by the tensor core or memory: key tiles of
-// 128, two forward CTAs per SM.  Measured: [16, 512] BERT block with 16 heads of 48 and a padding mask, attention kernels 334 us (199
-// backward, 96 forward, 39 around them; 294 us with two parts and unordered sums) where the unfused form took 2470 us; the block 3100 us with
-// the unfused form, 877 us with two parts, 918 us now.
+// 128, two forward CTAs per SM.  Measured: [16, 512] BERT block with 16 heads of 48 and a padding mask, attention kernels 285 us (168
+// backward, 78 forward, 39 around them) where the unfused form took 2470 us; forward 101 -> 78 us since rows of the mask that are all visible or all masked for a warp's
+// keys take no look at single bits, the largest score is scaled once and remainders need no unpacking (without a mask 152 -> 144, [4, 2048] 16 x 48 causal).
 // Every wait on an mbarrier is bounded (attention_tc.cuh).
 #include "attention_tc.cuh"
 
@@ -27,7 +27,7 @@
 
 namespace lb {
 
-constexpr int SPL_THREADS = 320;                 // backward: TMA warp, MMA warp, 8 softmax warps
+constexpr int SPL_THREADS = 384;                 // backward: TMA warp, MMA warp, two that keep their warpgroup whole, 8 softmax warps
 constexpr int SPL_FWD_THREADS = 256;             // forward: 8 softmax warps, one thread of which issues loads and MMAs: two CTAs of more warps get 96 registers, and spill
 constexpr int SPL_TILE = 128 * 64 * 2;           // one [128, 64] bf16 tile, 128-byte rows, swizzled
 constexpr float SPL_LOG2E = 1.4426950408889634f;
@@ -51,14 +51,50 @@ struct SplitParams {
 };
 
 // two fp32 numbers as three bf16 parts each, h + m + l = x to the last bit (8 + 8 + 8 bits of significand; normal range)
+// x0 - the lower, x1 - the upper bf16 of h, exactly (the multiply-add takes a bf16 factor as it is: no unpacking)
+LB_DEVICE void minus_bf16x2(float& x0, float& x1, uint32_t h) {
+  asm("{\n\t.reg .b16 a, b, m;\n\tmov.b32 {a, b}, %2;\n\tmov.b16 m, 0xBF80;\n\t"
+      "fma.rn.f32.bf16 %0, a, m, %0;\n\tfma.rn.f32.bf16 %1, b, m, %1;\n\t}\n"
+      : "+f"(x0), "+f"(x1)
+      : "r"(h));
+}
 LB_DEVICE void split3(float x0, float x1, uint32_t& h, uint32_t& m, uint32_t& l) {
   h = pack_bf16(x0, x1);
-  const float2 a = unpack_bf16(h);
-  x0 -= a.x;
-  x1 -= a.y;
+  minus_bf16x2(x0, x1, h);
   m = pack_bf16(x0, x1);
-  const float2 b = unpack_bf16(m);
-  l = pack_bf16(x0 - b.x, x1 - b.y);
+  minus_bf16x2(x0, x1, m);
+  l = pack_bf16(x0, x1);
+}
+
+// two numbers per instruction: x * f + c and x * y
+LB_DEVICE float2 fma2(float x0, float x1, float f, float c0, float c1) {
+  float2 r;
+  asm("{\n\t.reg .b64 x, f, c;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 f, {%4, %4};\n\tmov.b64 c, {%5, %6};\n\tfma.rn.f32x2 x, x, f, c;\n\tmov.b64 {%0, %1}, x;\n\t}\n"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(x0), "f"(x1), "f"(f), "f"(c0), "f"(c1));
+  return r;
+}
+LB_DEVICE float2 mul2(float x0, float x1, float2 y) {
+  float2 r;
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmul.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}\n"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(x0), "f"(x1), "f"(y.x), "f"(y.y));
+  return r;
+}
+// a 32 x 32 matrix of bits, one row per lane, transposed
+LB_DEVICE uint32_t transpose_bits(uint32_t x, int lane) {
+#pragma unroll
+  for (int j = 16; j > 0; j >>= 1) {
+    const uint32_t m = j == 16 ? 0x0000ffffu : j == 8 ? 0x00ff00ffu : j == 4 ? 0x0f0f0f0fu : j == 2 ? 0x33333333u : 0x55555555u;
+    const uint32_t y = __shfl_xor_sync(0xffffffffu, x, j);
+    x = (lane & j) ? (x & ~m) | ((y & ~m) >> j) : (x & m) | ((y & m) << j);
+  }
+  return x;
+}
+// bits [lo, hi) of a word
+LB_DEVICE uint32_t bit_range(int lo, int hi) {
+  const uint32_t below_hi = hi >= 32 ? 0xffffffffu : hi <= 0 ? 0u : (1u << hi) - 1u, below_lo = lo >= 32 ? 0xffffffffu : lo <= 0 ? 0u : (1u << lo) - 1u;
+  return below_hi & ~below_lo;
 }
 
 // ------------------------------------------------------------------------------------------------------------ mask -> bits
@@ -170,7 +206,7 @@ attn_split_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     if (j + 1 < nkv) load(j + 1);
   };
   auto values = [&](int j) {                                         // P(j)·V(j)
-    constexpr uint32_t idesc = make_idesc_bf16(128, 64, false, true);
+    const uint32_t idesc = make_idesc_bf16(128, ksteps * 16, false, true);
     const int b = j & 1;
     if (!tc_wait(p_full, j & 1, stop) || !tc_wait(&v_full[b], (j >> 1) & 1, stop)) return;
     tc_fence_after_sync();
@@ -220,9 +256,15 @@ attn_split_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       tc_fence_after_sync();
       const int k0 = j * 128 + half * 64;
       const bool edge = j * 128 + 128 > p.Sk || (p.causal && j * 128 + 127 > q0 + p.off);
+      // MASK: a warp's 32 queries and 64 keys are looked at one by one (1), all masked (2) or all visible (0)
       float mx = -INFINITY;
-      auto pass1 = [&](auto edge_tag) {
+      auto pass1 = [&](auto edge_tag, auto mask_tag) {
         constexpr bool EDGE = decltype(edge_tag)::value;
+        constexpr int MASK = decltype(mask_tag)::value;
+        if constexpr (MASK == 2) {
+          mx = fill;
+          return;
+        }
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           uint32_t t[16];
@@ -231,14 +273,36 @@ attn_split_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
           [[maybe_unused]] const uint32_t word = (c < 2 ? bits.x : bits.y) >> ((c & 1) * 16);
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
-            float x = __uint_as_float(t[i]) * p.scale_log2;
-            if constexpr (MASKED) x = (word >> i) & 1u ? x : fill;
+            float x = __uint_as_float(t[i]);
+            if constexpr (MASK == 1) x = word & (1u << i) ? x : -INFINITY;
             if constexpr (EDGE) x = k0 + c * 16 + i < key_lim ? x : -INFINITY;
             mx = fmaxf(mx, x);
           }
         }
+        mx *= p.scale_log2;                      // (scale > 0: the largest product)
+        if constexpr (MASK == 1) {               // a masked key within the sequence counts with its fill
+          const int keys = EDGE ? min(64, key_lim - k0) : 64;
+          const bool any = ((~bits.x & bit_range(0, keys)) | (~bits.y & bit_range(0, keys - 32))) != 0u;
+          mx = any ? fmaxf(mx, fill) : mx;
+        }
       };
-      if (edge) pass1(std::true_type{}); else pass1(std::false_type{});
+      using std::integral_constant;
+      [[maybe_unused]] int mode = 0;
+      if constexpr (MASKED) {
+        const bool on = __all_sync(0xffffffffu, (bits.x & bits.y) == 0xffffffffu), off = __all_sync(0xffffffffu, (bits.x | bits.y) == 0u);
+        mode = edge ? 1 : on ? 0 : off ? 2 : 1;
+      }
+      auto by_mode = [&](auto f) {
+        if constexpr (MASKED) {
+          if (edge) f(std::true_type{}, integral_constant<int, 1>{});
+          else if (mode == 0) f(std::false_type{}, integral_constant<int, 0>{});
+          else if (mode == 2) f(std::false_type{}, integral_constant<int, 2>{});
+          else f(std::false_type{}, integral_constant<int, 1>{});
+        } else {
+          if (edge) f(std::true_type{}, integral_constant<int, 0>{}); else f(std::false_type{}, integral_constant<int, 0>{});
+        }
+      };
+      by_mode(pass1);
       float* xch = sXchg + (j & 1) * 256;
       xch[half * 128 + r] = mx;
       tc_pair_sync(quad);
@@ -249,31 +313,39 @@ attn_split_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       if (bump) { alpha = fast_exp2(m_run - m_cand); m_run = m_cand; }                            // 0 on the first tile
       const float m_use = m_run == -INFINITY ? 0.f : m_run;
       float rowsum = 0.f;
-      auto pass2 = [&](auto edge_tag) {
+      auto pass2 = [&](auto edge_tag, auto mask_tag) {
         constexpr bool EDGE = decltype(edge_tag)::value;
+        constexpr int MASK = decltype(mask_tag)::value;
+        [[maybe_unused]] float masked = 0.f;     // probability of a masked key
+        if constexpr (MASK != 0) masked = fast_exp2(fill - m_use);
         float rs0 = 0.f, rs1 = 0.f;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {          // 16 keys at a time: 32 would spill
           uint32_t t[16], part[3][8];
-          tmem_ld_32x32b_x16(s_addr + c * 16, t);
-          tmem_ld_wait();
+          if constexpr (MASK != 2) {
+            tmem_ld_32x32b_x16(s_addr + c * 16, t);
+            tmem_ld_wait();
+          }
           [[maybe_unused]] const uint32_t word = (c < 2 ? bits.x : bits.y) >> ((c & 1) * 16);
 #pragma unroll
           for (int i = 0; i < 16; i += 2) {
-            float x0 = __uint_as_float(t[i]) * p.scale_log2, x1 = __uint_as_float(t[i + 1]) * p.scale_log2;
-            if constexpr (MASKED) {
-              x0 = (word >> i) & 1u ? x0 : fill;
-              x1 = (word >> (i + 1)) & 1u ? x1 : fill;
+            float2 x = make_float2(masked, masked);
+            if constexpr (MASK != 2) {
+              x = fma2(__uint_as_float(t[i]), __uint_as_float(t[i + 1]), p.scale_log2, -m_use, -m_use);
+              x.x = fast_exp2(x.x);
+              x.y = fast_exp2(x.y);
             }
-            x0 = fast_exp2(x0 - m_use);
-            x1 = fast_exp2(x1 - m_use);
+            if constexpr (MASK == 1) {
+              x.x = word & (1u << i) ? x.x : masked;
+              x.y = word & (2u << i) ? x.y : masked;
+            }
             if constexpr (EDGE) {
-              x0 = k0 + c * 16 + i < key_lim ? x0 : 0.f;
-              x1 = k0 + c * 16 + i + 1 < key_lim ? x1 : 0.f;
+              x.x = k0 + c * 16 + i < key_lim ? x.x : 0.f;
+              x.y = k0 + c * 16 + i + 1 < key_lim ? x.y : 0.f;
             }
-            rs0 += x0;
-            rs1 += x1;
-            split3(x0, x1, part[0][i / 2], part[1][i / 2], part[2][i / 2]);
+            rs0 += x.x;
+            rs1 += x.y;
+            split3(x.x, x.y, part[0][i / 2], part[1][i / 2], part[2][i / 2]);
           }
           // (S(j) follows the completion of P(j-1)·V(j-1): all columns are free; the last two parts cover S columns read above)
           tmem_st_32x32b_x8(p_addr + c * 8, part[0]);
@@ -282,7 +354,7 @@ attn_split_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         }
         rowsum = rs0 + rs1;
       };
-      if (edge) pass2(std::true_type{}); else pass2(std::false_type{});
+      by_mode(pass2);
       l_run = l_run * alpha + rowsum;
       tmem_st_wait();
       tc_fence_before_sync();
@@ -347,19 +419,26 @@ attn_split_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 }
 
 // ----------------------------------------------------------------------------------------------------------------- backward
-// One CTA per (128 keys, head, batch), looping over the query blocks that see them, with the keys on the M side:
+// Work items of (128 keys, head, batch), looping over the query blocks that see them, with the keys on the M side:
 //   Sᵀ = K·Qᵀ, dPᵀ = V·dOᵀ;  P = exp(S - lse), dS = P ∘ (dP - δ) · scale, in three bf16 parts each;
 //   dV += Pᵀ·dO with Pᵀ from TMEM, dK += dSᵀ·Q and dQ_i = dS·K with dSᵀ from shared memory.
 // dQ_i goes out in fp32, one layer per key block (attn_split_dq_kernel adds the layers up in order): the unfused product had a fixed order,
 // and additions into one accumulator by several CTAs have none.
 // Six tiles of parts do not fit shared memory beside the operands, so Pᵀ stays in TMEM, which wants it as [keys, queries]: the first part in
 // columns of its own, the second and third of 16 queries over the 16 Sᵀ columns that their thread has read.
-// Shared memory: K, V, Q, dO 64 KB, three dSᵀ tiles 96 KB, dQ staging 32 KB, two stages of what a query's thread row needs: log-sum-exp, δ, the
-// probability of a masked key and the mask bits, one word per (32 keys, query).
+// Shared memory: K, V 32 KB, two stages of Q and dO 64 KB, three dSᵀ tiles 96 KB, dQ staging 32 KB, what a query's thread row needs: log-sum-exp, δ, the
+// probability of a masked key (mask words are transposed between the lanes).
+// Bounded by the softmax threads' instructions (1700 per warp and block of 128 x 128, 3400 cycles on their schedulers) and the 72 small products (26 to 60 cycles
+// each: their A operands are 4 KB for 128 x 64 results).  So the two run side by side as far as the one buffer of dSᵀ allows: P is made first and dV runs while dS
+// is made from the probabilities kept in registers; Sᵀ and dPᵀ of the next block go out as soon as dS is there, in front of dK and dQ, Sᵀ to where dPᵀ was and the other way
+// round; the threads make the next P meanwhile and wait for dQ before they write its dSᵀ.  CTAs stay for several work items: the next one's Q and dO are loaded and its numbers
+// fetched while this one ends.  A block took 14200 cycles with everything in turn, now 8000.  Rows of the mask that are all visible or all masked for a warp's keys take
+// no look at single bits.  The split into three parts takes its remainders with a multiply-add that reads bf16 factors (310 -> 283 us; 2048 below), scales two scores per instruction.
+// Measured, us: [16, 512] 16 heads of 48 with a padding mask 201 -> 169, [4, 2048] 16 x 48 causal 375 -> 280, [8, 1024] 16 x 24 causal 211 -> 156, [1, 1024] 16 x 48 47 -> 38,
+// [64, 128] 16 x 32 63 -> 54, 128 queries against 512 keys (16, 12 x 32, masked) 53 -> 46; [16, 128] 12 x 32 masked 19.5 -> 20.5 (192 items, two for some CTAs).
 constexpr int SPL_PS = 128 * 128 * 2;
 constexpr int SPL_DQ_BOX = 32 * 128;
-constexpr int SPL_STAT = (3 + 4) * 128;                              // 32-bit words per stage
-constexpr int SPL_BWD_SMEM = 4 * SPL_TILE + 3 * SPL_PS + 8 * SPL_DQ_BOX + 2 * SPL_STAT * 4 + 1024 + 256;
+constexpr int SPL_BWD_SMEM = 6 * SPL_TILE + 3 * SPL_PS + 8 * SPL_DQ_BOX + 3 * 128 * 4 + 1024 + 128;
 static_assert(SPL_BWD_SMEM <= 232448, "split attention backward: shared memory");
 
 template <bool MASKED>
@@ -367,32 +446,45 @@ __global__ void __launch_bounds__(SPL_THREADS, 1)
 attn_split_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                       const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
                       const __grid_constant__ CUtensorMap tmap_dq, SplitParams p) {
-  constexpr uint32_t S_COL = 0, DP_COL = 128, DV_COL = 256, DK_COL = 320, DQ_COL = 384, P_COL = 448;
+  constexpr uint32_t DV_COL = 256, DK_COL = 320, DQ_COL = 384, P_COL = 448;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sK = smem;
   uint8_t* sV = sK + SPL_TILE;
-  uint8_t* sQ = sV + SPL_TILE;
-  uint8_t* sDO = sQ + SPL_TILE;
-  uint8_t* sDS = sDO + SPL_TILE;                // three parts: two chunks of 64 queries, 128 key rows x 128 bytes each
+  uint8_t* sQ = sV + SPL_TILE;                  // 2
+  uint8_t* sDO = sQ + 2 * SPL_TILE;             // 2
+  uint8_t* sDS = sDO + 2 * SPL_TILE;            // three parts: two chunks of 64 queries, 128 key rows x 128 bytes each
   uint8_t* sDQ = sDS + 3 * SPL_PS;
   uint32_t* sStat = reinterpret_cast<uint32_t*>(sDQ + 8 * SPL_DQ_BOX);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + 2 * SPL_STAT);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + 3 * 128);
   uint64_t* kv_full = bars;
-  uint64_t* qdo_full = bars + 1;
-  uint64_t* qdo_empty = bars + 2;               // also: the parts of P and dS may be written again (and, with dq_empty, the dQ columns)
-  uint64_t* sdp_full = bars + 3;
-  uint64_t* pds_full = bars + 4;
-  uint64_t* dq_full = bars + 5;
-  uint64_t* dq_empty = bars + 6;
-  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 8);
-  volatile int* stop = reinterpret_cast<volatile int*>(bars + 9);
+  uint64_t* sdp_full = bars + 1;
+  uint64_t* p_full = bars + 2;
+  uint64_t* ds_full = bars + 10;                // and dPᵀ and the dQ of the block before are read
+  uint64_t* dv_done = bars + 3;
+  uint64_t* dq_done = bars + 4;                 // and everything issued before: dS may be written again
+  uint64_t* qdo_full = bars + 5;                // 2
+  uint64_t* qdo_empty = bars + 7;               // 2
+  uint64_t* kv_empty = bars + 9;
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 11);
+  volatile int* stop = reinterpret_cast<volatile int*>(bars + 12);
 
   const int warp_idx = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int head = blockIdx.y, batch = blockIdx.z, k0 = blockIdx.x * 128;
-  const int nq = (p.Sq + 127) / 128;
-  const int i_begin = p.causal ? max(0, k0 - p.off) / 128 : 0;      // the first query that sees key k0 is k0 - off
-  const int iters = nq - i_begin;                                    // >= 1: off >= 0 under the causal mask
+  // work items: blocks of 128 keys of a head, those with the most query blocks first; CTA c takes c, c + CTAs, ..
+  const int heads = p.A * p.B, items = (p.Sk + 127) / 128 * heads, nq = (p.Sq + 127) / 128;
+  struct Item {
+    int k0, head, batch, i_begin, iters;
+  };
+  auto item_of = [&](int item) {
+    Item w;
+    const int bh = item % heads;
+    w.k0 = item / heads * 128;
+    w.head = bh % p.A;
+    w.batch = bh / p.A;
+    w.i_begin = p.causal ? max(0, w.k0 - p.off) / 128 : 0;           // the first query that sees key k0 is k0 - off
+    w.iters = nq - w.i_begin;                                        // >= 1: off >= 0 under the causal mask
+    return w;
+  };
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmap_q);
@@ -400,7 +492,7 @@ attn_split_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     tma_prefetch_desc(&tmap_v);
     tma_prefetch_desc(&tmap_do);
     tma_prefetch_desc(&tmap_dq);
-    for (int i = 0; i < 7; ++i) mbar_init(bars + i, (i == 4 || i == 6) ? 8 : 1);
+    for (int i = 0; i < 11; ++i) mbar_init(bars + i, i == 2 || i == 10 ? 8 : 1);
     *stop = 0;
     fence_barrier_init();
     fence_proxy_async();
@@ -412,232 +504,324 @@ attn_split_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   const uint32_t tmem_base = *tmem_ptr_smem;
   chain_wait();
   chain_next();
-
-  if (warp_idx == 0) {
-    if (elect_one()) {
-      mbar_arrive_expect_tx(kv_full, 2 * SPL_TILE);
-      tma_load_4d(sK, &tmap_k, kv_full, 0, k0, head, batch);
-      tma_load_4d(sV, &tmap_v, kv_full, 0, k0, head, batch);
-      for (int it = 0; it < iters; ++it) {
-        if (!tc_wait(qdo_empty, (it & 1) ^ 1, stop)) continue;
-        mbar_arrive_expect_tx(qdo_full, 2 * SPL_TILE);
-        tma_load_4d(sQ, &tmap_q, qdo_full, 0, (i_begin + it) * 128, head, batch);
-        tma_load_4d(sDO, &tmap_do, qdo_full, 0, (i_begin + it) * 128, head, batch);
+  // The softmax threads hold a block's probabilities: 3 x 168 registers as launched, 88 + 2 x 208 from here on.
+  if (warp_idx < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 88;\n");
+    if (warp_idx == 0) {
+      if (elect_one()) {
+        int t = 0, n = 0;                                              // blocks and items so far
+        for (int item = blockIdx.x; item < items; item += gridDim.x, ++n) {
+          const Item w = item_of(item);
+          for (int it = 0; it < w.iters; ++it, ++t) {
+            const int b = t & 1, q = (w.i_begin + it) * 128;
+            if (!tc_wait(&qdo_empty[b], ((t >> 1) & 1) ^ 1, stop)) continue;
+            mbar_arrive_expect_tx(&qdo_full[b], 2 * SPL_TILE);
+            tma_load_4d(sQ + b * SPL_TILE, &tmap_q, &qdo_full[b], 0, q, w.head, w.batch);
+            tma_load_4d(sDO + b * SPL_TILE, &tmap_do, &qdo_full[b], 0, q, w.head, w.batch);
+            if (it == 0 && tc_wait(kv_empty, (n & 1) ^ 1, stop)) {     // (the item's first Q and dO do not wait for this)
+              mbar_arrive_expect_tx(kv_full, 2 * SPL_TILE);
+              tma_load_4d(sK, &tmap_k, kv_full, 0, w.k0, w.head, w.batch);
+              tma_load_4d(sV, &tmap_v, kv_full, 0, w.k0, w.head, w.batch);
+            }
+          }
+        }
       }
-    }
-    __syncwarp();
-  } else if (warp_idx == 1) {
-    constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);   // K·Qᵀ, V·dOᵀ
-    constexpr uint32_t idesc_t = make_idesc_bf16(128, 64, false, true);     // Pᵀ·dO, dSᵀ·Q
-    constexpr uint32_t idesc_q = make_idesc_bf16(128, 64, true, true);      // dS·K
-    const uint32_t k_addr = smem_u32(sK), v_addr = smem_u32(sV), q_addr = smem_u32(sQ), do_addr = smem_u32(sDO), ds_addr = smem_u32(sDS);
-    const int ksteps = (p.d + 15) / 16;
-    bool ok = __all_sync(0xffffffffu, tc_wait(kv_full, 0, stop));
-    for (int it = 0; it < iters; ++it) {
-      ok = __all_sync(0xffffffffu, ok && tc_wait(qdo_full, it & 1, stop));
-      tc_fence_after_sync();
-      if (ok && elect_one()) {
+      __syncwarp();
+    } else if (warp_idx == 1) {
+      constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);   // K·Qᵀ, V·dOᵀ
+      const int dcols = (p.d + 15) / 16 * 16;                                 // columns of the products with d (those behind d are zeros, and not stored)
+      const uint32_t idesc_t = make_idesc_bf16(128, dcols, false, true);      // Pᵀ·dO, dSᵀ·Q
+      const uint32_t idesc_q = make_idesc_bf16(128, dcols, true, true);       // dS·K
+      const uint32_t k_addr = smem_u32(sK), v_addr = smem_u32(sV), ds_addr = smem_u32(sDS);
+      const int ksteps = (p.d + 15) / 16;
+      auto s_col = [&](int t) { return tmem_base + (t & 1) * 128; };          // Sᵀ of block t, dPᵀ of the block before
+      auto scores = [&](int t) {                       // Sᵀ and dPᵀ of block t
+        const uint32_t q_addr = smem_u32(sQ + (t & 1) * SPL_TILE), do_addr = smem_u32(sDO + (t & 1) * SPL_TILE);
         for (int kk = 0; kk < ksteps; ++kk)
-          umma_f16_ss(tmem_base + S_COL, make_smem_desc_sw128(k_addr + kk * 32, 0, 1024), make_smem_desc_sw128(q_addr + kk * 32, 0, 1024), idesc_s,
+          umma_f16_ss(s_col(t), make_smem_desc_sw128(k_addr + kk * 32, 0, 1024), make_smem_desc_sw128(q_addr + kk * 32, 0, 1024), idesc_s,
                       kk > 0 ? 1u : 0u);
         for (int kk = 0; kk < ksteps; ++kk)
-          umma_f16_ss(tmem_base + DP_COL, make_smem_desc_sw128(v_addr + kk * 32, 0, 1024), make_smem_desc_sw128(do_addr + kk * 32, 0, 1024), idesc_s,
+          umma_f16_ss(s_col(t + 1), make_smem_desc_sw128(v_addr + kk * 32, 0, 1024), make_smem_desc_sw128(do_addr + kk * 32, 0, 1024), idesc_s,
                       kk > 0 ? 1u : 0u);
         umma_commit(sdp_full);
-      }
-      __syncwarp();
-      ok = __all_sync(0xffffffffu, ok && tc_wait(pds_full, it & 1, stop));
-      ok = __all_sync(0xffffffffu, ok && tc_wait(dq_empty, (it & 1) ^ 1, stop));
-      tc_fence_after_sync();
-      if (ok && elect_one()) {
+      };
+      bool ok = true;
+      int t = 0, n = 0;
+      for (int item = blockIdx.x; item < items; item += gridDim.x, ++n) {
+        const int iters = item_of(item).iters;
+        ok = __all_sync(0xffffffffu, ok && tc_wait(kv_full, n & 1, stop) && tc_wait(&qdo_full[t & 1], (t >> 1) & 1, stop));
+        tc_fence_after_sync();
+        if (ok && elect_one()) scores(t);                // (K came after every product of the item before had completed)
+        __syncwarp();
+        for (int it = 0; it < iters; ++it, ++t) {
+          const int b = t & 1;
+          const uint32_t q_addr = smem_u32(sQ + b * SPL_TILE), do_addr = smem_u32(sDO + b * SPL_TILE);
+          ok = __all_sync(0xffffffffu, ok && tc_wait(p_full, t & 1, stop));
+          tc_fence_after_sync();
+          if (ok && elect_one()) {
 #pragma unroll
-        for (int part = 0; part < 3; ++part) {       // dQ first: its drain is the only consumer that is waited for
+            for (int kk = 0; kk < 8; ++kk) {             // 16 queries per step
+              const uint64_t bo = make_smem_desc_sw128(do_addr + kk * 2048, 128 * 128, 1024);
+              umma_f16_ts(tmem_base + DV_COL, tmem_base + P_COL + kk * 8, bo, idesc_t, (it > 0 || kk > 0) ? 1u : 0u);
+              umma_f16_ts(tmem_base + DV_COL, s_col(t) + kk * 16, bo, idesc_t, 1u);
+              umma_f16_ts(tmem_base + DV_COL, s_col(t) + kk * 16 + 8, bo, idesc_t, 1u);
+            }
+            umma_commit(dv_done);
+          }
+          __syncwarp();
+          ok = __all_sync(0xffffffffu, ok && tc_wait(ds_full, t & 1, stop));
+          tc_fence_after_sync();
+          if (it + 1 < iters) {
+            ok = __all_sync(0xffffffffu, ok && tc_wait(&qdo_full[b ^ 1], ((t + 1) >> 1) & 1, stop));
+            ok = __all_sync(0xffffffffu, ok && tc_wait(dv_done, t & 1, stop));
+            tc_fence_after_sync();
+            if (ok && elect_one()) scores(t + 1);
+            __syncwarp();
+          }
+          if (ok && elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < 8; ++kk)             // 16 keys per step
-            umma_f16_ss(tmem_base + DQ_COL, make_smem_desc_sw128(ds_addr + part * SPL_PS + kk * 2048, 128 * 128, 1024),
-                        make_smem_desc_sw128(k_addr + kk * 2048, 128 * 128, 1024), idesc_q, (part > 0 || kk > 0) ? 1u : 0u);
+            for (int kk = 0; kk < 8; ++kk) {
+              const uint64_t bq = make_smem_desc_sw128(q_addr + kk * 2048, 128 * 128, 1024);
+#pragma unroll
+              for (int part = 0; part < 3; ++part)
+                umma_f16_ss(tmem_base + DK_COL, make_smem_desc_sw128(ds_addr + part * SPL_PS + (kk / 4) * (128 * 128) + (kk % 4) * 32, 0, 1024), bq, idesc_t,
+                            (it > 0 || kk > 0 || part > 0) ? 1u : 0u);
+            }
+            umma_commit(&qdo_empty[b]);
+#pragma unroll
+            for (int part = 0; part < 3; ++part) {
+#pragma unroll
+              for (int kk = 0; kk < 8; ++kk)             // 16 keys per step
+                umma_f16_ss(tmem_base + DQ_COL, make_smem_desc_sw128(ds_addr + part * SPL_PS + kk * 2048, 128 * 128, 1024),
+                            make_smem_desc_sw128(k_addr + kk * 2048, 128 * 128, 1024), idesc_q, (part > 0 || kk > 0) ? 1u : 0u);
+            }
+            umma_commit(dq_done);
+            if (it + 1 == iters) umma_commit(kv_empty);
+          }
+          __syncwarp();
         }
-        umma_commit(dq_full);
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {             // 16 queries per step
-          const uint64_t bo = make_smem_desc_sw128(do_addr + kk * 2048, 128 * 128, 1024), bq = make_smem_desc_sw128(q_addr + kk * 2048, 128 * 128, 1024);
-          umma_f16_ts(tmem_base + DV_COL, tmem_base + P_COL + kk * 8, bo, idesc_t, (it > 0 || kk > 0) ? 1u : 0u);
-          umma_f16_ts(tmem_base + DV_COL, tmem_base + S_COL + kk * 16, bo, idesc_t, 1u);
-          umma_f16_ts(tmem_base + DV_COL, tmem_base + S_COL + kk * 16 + 8, bo, idesc_t, 1u);
-#pragma unroll
-          for (int part = 0; part < 3; ++part)
-            umma_f16_ss(tmem_base + DK_COL, make_smem_desc_sw128(ds_addr + part * SPL_PS + (kk / 4) * (128 * 128) + (kk % 4) * 32, 0, 1024), bq, idesc_t,
-                        (it > 0 || kk > 0 || part > 0) ? 1u : 0u);
-        }
-        umma_commit(qdo_empty);
       }
-      __syncwarp();
     }
   } else {
-    const int quad = warp_idx % 4, half = (warp_idx - 2) / 4;        // this warp's 32 of the 128 keys, its 64 of a tile's 128 queries
-    const int r = quad * 32 + lane, k_idx = k0 + r;
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 208;\n");
+    const int quad = warp_idx % 4, half = warp_idx / 4 - 1;          // this warp's 32 of the 128 keys, its 64 of a tile's 128 queries
+    const int r = quad * 32 + lane;
     const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
-    const size_t bh = static_cast<size_t>(batch) * p.A + head;
-    // what a tile's queries bring along: 128 threads fetch a query's numbers, the other 128 its mask words, one tile ahead
-    const int tid = static_cast<int>(threadIdx.x) - 64, fq = tid & 127;
+    // what a block's queries bring along, fetched one block ahead: 128 threads a query's numbers, every warp the mask words of its 64 queries, two per lane
+    const int tid = static_cast<int>(threadIdx.x) - 128, fq = tid & 127;
     float f_lse = 0.f, f_delta = 0.f;
     [[maybe_unused]] float f_fill = 0.f;
-    [[maybe_unused]] uint4 f_bits = make_uint4(0, 0, 0, 0);
-    auto fetch = [&](int it) {
-      const int q = min((i_begin + it) * 128 + fq, p.Sq - 1);        // (queries behind Sq are masked below)
-      [[maybe_unused]] const long row = MASKED ? batch * p.mask_b + head * p.mask_a + q : 0;
+    [[maybe_unused]] uint32_t f_bits[2] = {0u, 0u};
+    auto fetch = [&](const Item& w, int it) {
+      const int q_tile = (w.i_begin + it) * 128, q = min(q_tile + fq, p.Sq - 1);      // (queries behind Sq are masked below)
+      [[maybe_unused]] const long base = MASKED ? w.batch * p.mask_b + w.head * p.mask_a : 0;
+      const size_t bh = static_cast<size_t>(w.batch) * p.A + w.head;
       if (tid < 128) {
         f_lse = p.lse[bh * p.Sq + q];
         f_delta = p.delta[bh * p.Sq + q];
-        if constexpr (MASKED) f_fill = p.fill[row];
-      } else if constexpr (MASKED) {
-        f_bits = *reinterpret_cast<const uint4*>(p.mask + row * p.pitch + k0 / 32);
+        if constexpr (MASKED) f_fill = p.fill[base + q];
+      }
+      if constexpr (MASKED) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+          f_bits[i] = p.mask[(base + min(q_tile + half * 64 + i * 32 + lane, p.Sq - 1)) * p.pitch + w.k0 / 32 + quad];
       }
     };
-    fetch(0);
-    for (int it = 0; it < iters; ++it) {
-      const int q_blk = i_begin + it;
-      uint32_t* st = sStat + (it & 1) * SPL_STAT;                    // (whoever still reads the tile before last has not passed the barrier below)
-      if (tid < 128) {
-        const float lse2 = f_lse * SPL_LOG2E;
-        st[fq] = __float_as_uint(lse2);
-        st[128 + fq] = __float_as_uint(f_delta * p.scale);
-        if constexpr (MASKED) st[256 + fq] = __float_as_uint(fast_exp2(f_fill - lse2));
-      } else if constexpr (MASKED) {
-        st[384 + fq] = f_bits.x;
-        st[512 + fq] = f_bits.y;
-        st[640 + fq] = f_bits.z;
-        st[768 + fq] = f_bits.w;
-      }
-      __syncwarp();
-      asm volatile("bar.sync 1, 256;\n" ::: "memory");              // the eight warps of this branch
-      if (it + 1 < iters) fetch(it + 1);
-      // queries [q_lo, q_hi) of this half see key k_idx (the mask apart)
-      const int q_first = q_blk * 128 + half * 64;
-      const int q_lo = k_idx >= p.Sk ? 128 : (p.causal ? k_idx - p.off - q_first : 0), q_hi = p.Sq - q_first;
-      const bool edge = k0 + 128 > p.Sk || q_blk * 128 + 128 > p.Sq || (p.causal && k0 + 127 - p.off > q_blk * 128);
-      tc_wait(sdp_full, it & 1, stop);        // S(it) was issued after the products of block it-1 had read the parts of P and dS (one Q stage)
-      __syncwarp();
-      tc_fence_after_sync();
-      auto tile = [&](auto edge_tag) {
-        constexpr bool EDGE = decltype(edge_tag)::value;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {          // 16 queries at a time
-          const int kk = half * 4 + c;
-          uint32_t ts[16], td[16];
-          tmem_ld_32x32b_x16(tmem_base + lane_off + S_COL + kk * 16, ts);
-          tmem_ld_32x32b_x16(tmem_base + lane_off + DP_COL + kk * 16, td);
-          tmem_ld_wait();
-          uint32_t pp[3][8], dd[3][8];
-#pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            const int at = kk * 16 + v * 4;
-            const float4 l4 = *reinterpret_cast<const float4*>(st + at), d4 = *reinterpret_cast<const float4*>(st + 128 + at);
-            float4 m4 = make_float4(0.f, 0.f, 0.f, 0.f);
-            uint4 w4 = make_uint4(0, 0, 0, 0);
-            if constexpr (MASKED) {
-              m4 = *reinterpret_cast<const float4*>(st + 256 + at);
-              w4 = *reinterpret_cast<const uint4*>(st + 384 + quad * 128 + at);
-            }
-            const float ls[4] = {l4.x, l4.y, l4.z, l4.w}, de[4] = {d4.x, d4.y, d4.z, d4.w};
-            [[maybe_unused]] const float pm[4] = {m4.x, m4.y, m4.z, m4.w};
-            [[maybe_unused]] const uint32_t wd[4] = {w4.x, w4.y, w4.z, w4.w};
-            float pv[4], dv[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const int i = 4 * v + e;
-              pv[e] = fast_exp2(fmaf(__uint_as_float(ts[i]), p.scale_log2, -ls[e]));
-              dv[e] = pv[e] * fmaf(__uint_as_float(td[i]), p.scale, -de[e]);
-              if constexpr (MASKED) {
-                const bool on = (wd[e] >> lane) & 1u;
-                pv[e] = on ? pv[e] : pm[e];
-                dv[e] = on ? dv[e] : 0.f;                            // a masked score is a constant
-              }
-              if constexpr (EDGE) {
-                const bool in = c * 16 + i >= q_lo && c * 16 + i < q_hi;
-                pv[e] = in ? pv[e] : 0.f;
-                dv[e] = in ? dv[e] : 0.f;
-              }
-            }
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              split3(pv[2 * e], pv[2 * e + 1], pp[0][2 * v + e], pp[1][2 * v + e], pp[2][2 * v + e]);
-              split3(dv[2 * e], dv[2 * e + 1], dd[0][2 * v + e], dd[1][2 * v + e], dd[2][2 * v + e]);
-            }
-          }
-          tmem_st_32x32b_x8(tmem_base + lane_off + P_COL + kk * 8, pp[0]);
-          tmem_st_32x32b_x8(tmem_base + lane_off + S_COL + kk * 16, pp[1]);
-          tmem_st_32x32b_x8(tmem_base + lane_off + S_COL + kk * 16 + 8, pp[2]);
-          uint8_t* drow = sDS + half * (128 * 128) + r * 128;
-#pragma unroll
-          for (int v = 0; v < 2; ++v) {
-            const int phys = ((c * 2 + v) ^ (r & 7)) * 16;
-#pragma unroll
-            for (int part = 0; part < 3; ++part)
-              *reinterpret_cast<uint4*>(drow + part * SPL_PS + phys) = make_uint4(dd[part][4 * v], dd[part][4 * v + 1], dd[part][4 * v + 2], dd[part][4 * v + 3]);
-          }
-        }
-      };
-      if (edge) tile(std::true_type{}); else tile(std::false_type{});
-      tmem_st_wait();
-      tc_fence_before_sync();
-      fence_proxy_async();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(pds_full);
-      // ---- dQ of this block: TMEM -> swizzled [32 rows x 32 floats] box -> TMA reduction into the fp32 accumulator
-      const bool dq_ok = tc_wait(dq_full, it & 1, stop);
+    // dQ of block t, query block q_blk of the item: TMEM -> swizzled [32 rows x 32 floats] box -> TMA store into its layer of the fp32 accumulator
+    auto drain = [&](int t, int item, int q_blk) {
+      const bool dq_ok = tc_wait(dq_done, t & 1, stop);
       __syncwarp();
       tc_fence_after_sync();
       if (lane == 0) tma_store_wait_read<0>();                       // this warp's previous box has been read
       __syncwarp();
       uint8_t* box = sDQ + (quad * 2 + half) * SPL_DQ_BOX;
-      {
-        uint32_t t[32];
-        tmem_ld_32x32b_x32(tmem_base + lane_off + DQ_COL + half * 32, t);
-        tmem_ld_wait();
-        uint8_t* brow = box + lane * 128;
+      uint8_t* brow = box + lane * 128;
 #pragma unroll
-        for (int v = 0; v < 8; ++v)
-          *reinterpret_cast<uint4*>(brow + ((v ^ (lane & 7)) * 16)) = make_uint4(t[4 * v], t[4 * v + 1], t[4 * v + 2], t[4 * v + 3]);
+      for (int c = 0; c < 2; ++c) {
+        uint32_t t[16];
+        tmem_ld_32x32b_x16(tmem_base + lane_off + DQ_COL + half * 32 + c * 16, t);
+        tmem_ld_wait();
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+          *reinterpret_cast<uint4*>(brow + (((c * 4 + v) ^ (lane & 7)) * 16)) = make_uint4(t[4 * v], t[4 * v + 1], t[4 * v + 2], t[4 * v + 3]);
       }
-      tc_fence_before_sync();
       fence_proxy_async();
       __syncwarp();
       if (lane == 0) {
-        mbar_arrive(dq_empty);
-        if (dq_ok && half * 32 < p.d && q_blk * 128 + quad * 32 < p.Sq) {   // boxes start inside the layer; its edge clips them
+        const int q = q_blk * 128 + quad * 32;
+        if (dq_ok && half * 32 < p.d && q < p.Sq) {                  // boxes start inside the layer; its edge clips them
           asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3}], [%4];\n" ::"l"(reinterpret_cast<uint64_t>(&tmap_dq)),
-                       "r"(half * 32), "r"(q_blk * 128 + quad * 32), "r"(static_cast<int>(blockIdx.x * gridDim.z * gridDim.y + bh)), "r"(smem_u32(box))
+                       "r"(half * 32), "r"(q), "r"(item), "r"(smem_u32(box))
                        : "memory");
         }
         tma_store_commit();
       }
       __syncwarp();
-    }
-    if (lane == 0) tma_store_wait<0>();
-    __syncwarp();
-    // ---- dV / dK: thread r <-> key row r
-    tc_wait(qdo_empty, (iters - 1) & 1, stop);
-    __syncwarp();
-    tc_fence_after_sync();
-#pragma unroll
-    for (int which = 0; which < 2; ++which) {
-      uint32_t t[32];
-      tmem_ld_32x32b_x32(tmem_base + lane_off + (which == 0 ? DV_COL : DK_COL) + half * 32, t);
-      tmem_ld_wait();
-      if (k_idx < p.Sk) {
-        const long* st = which == 0 ? p.dv_strides : p.dk_strides;
-        __nv_bfloat16* row = (which == 0 ? p.dv : p.dk) + batch * st[0] + head * st[1] + k_idx * st[2] + half * 32;
-#pragma unroll
-        for (int i = 0; i < 32; i += 8) {
-          if (half * 32 + i >= p.d) break;
-          *reinterpret_cast<uint4*>(row + i) = make_uint4(
-              pack_bf16(__uint_as_float(t[i]), __uint_as_float(t[i + 1])), pack_bf16(__uint_as_float(t[i + 2]), __uint_as_float(t[i + 3])),
-              pack_bf16(__uint_as_float(t[i + 4]), __uint_as_float(t[i + 5])), pack_bf16(__uint_as_float(t[i + 6]), __uint_as_float(t[i + 7])));
+    };
+    int t = 0;
+    fetch(item_of(blockIdx.x), 0);
+    for (int item = blockIdx.x; item < items; item += gridDim.x) {
+      const Item w = item_of(item);
+      const int k0 = w.k0, k_idx = k0 + r, i_begin = w.i_begin, iters = w.iters;
+      for (int it = 0; it < iters; ++it, ++t) {
+        const int q_blk = i_begin + it;
+        uint32_t* st = sStat;
+        [[maybe_unused]] const uint32_t bits[2] = {f_bits[0], f_bits[1]};
+        if (t > 0) asm volatile("bar.sync 1, 256;\n" ::: "memory");   // the eight warps of this branch have read the block before's
+        if (tid < 128) {
+          const float lse2 = f_lse * SPL_LOG2E;
+          st[fq] = __float_as_uint(-lse2);                         // (negative: addends as they are)
+          st[128 + fq] = __float_as_uint(-(f_delta * p.scale));
+          if constexpr (MASKED) st[256 + fq] = __float_as_uint(fast_exp2(f_fill - lse2));
         }
+        __syncwarp();
+        asm volatile("bar.sync 1, 256;\n" ::: "memory");
+        if (it + 1 < iters) fetch(w, it + 1);
+        else if (item + static_cast<int>(gridDim.x) < items) fetch(item_of(item + gridDim.x), 0);
+        // queries [q_lo, q_hi) of this half see key k_idx (the mask apart)
+        const int q_first = q_blk * 128 + half * 64;
+        const int q_lo = k_idx >= p.Sk ? 128 : (p.causal ? k_idx - p.off - q_first : 0), q_hi = p.Sq - q_first;
+        const bool edge = k0 + 128 > p.Sk || q_blk * 128 + 128 > p.Sq || (p.causal && k0 + 127 - p.off > q_blk * 128);
+        tc_wait(sdp_full, t & 1, stop);         // S(t) and dP(t) were issued after dV of block t-1 had read the parts of P
+        __syncwarp();
+        tc_fence_after_sync();
+        const uint32_t s_addr = tmem_base + lane_off + (t & 1) * 128 + half * 64, dp_addr = tmem_base + lane_off + (~t & 1) * 128 + half * 64;
+        // MASK: the warp's 32 keys and 64 queries are looked at one by one (1), all masked (2) or all visible (0)
+        auto tile = [&](auto edge_tag, auto mask_tag) {
+          constexpr bool EDGE = decltype(edge_tag)::value;
+          constexpr int MASK = decltype(mask_tag)::value;
+          float pv[64];
+          // this key's 64 queries, a bit each: visible; in range
+          [[maybe_unused]] uint32_t seen[2] = {0xffffffffu, 0xffffffffu}, in[2] = {0xffffffffu, 0xffffffffu};
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            if constexpr (MASK == 1) seen[i] = transpose_bits(bits[i], lane);
+            if constexpr (EDGE) in[i] = bit_range(q_lo - 32 * i, q_hi - 32 * i);
+          }
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {          // P, 16 queries at a time
+            uint32_t ts[16], pp[3][8];
+            if constexpr (MASK != 2) {
+              tmem_ld_32x32b_x16(s_addr + c * 16, ts);
+              tmem_ld_wait();
+            }
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              const int at = half * 64 + c * 16 + v * 4;
+              const float4 l4 = *reinterpret_cast<const float4*>(st + (MASK == 2 ? 256 : 0) + at);
+              float4 m4 = l4;
+              if constexpr (MASK == 1) m4 = *reinterpret_cast<const float4*>(st + 256 + at);
+              const float ls[4] = {l4.x, l4.y, l4.z, l4.w};
+              [[maybe_unused]] const float pm[4] = {m4.x, m4.y, m4.z, m4.w};
+              float z[4] = {ls[0], ls[1], ls[2], ls[3]};
+              if constexpr (MASK != 2) {
+#pragma unroll
+                for (int e = 0; e < 4; e += 2) {
+                  const float2 y = fma2(__uint_as_float(ts[4 * v + e]), __uint_as_float(ts[4 * v + e + 1]), p.scale_log2, ls[e], ls[e + 1]);
+                  z[e] = fast_exp2(y.x);
+                  z[e + 1] = fast_exp2(y.y);
+                }
+              }
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const int i = 4 * v + e;
+                float x = z[e];
+                if constexpr (MASK == 1) x = seen[c / 2] & (1u << ((c & 1) * 16 + i)) ? x : pm[e];
+                if constexpr (EDGE) x = in[c / 2] & (1u << ((c & 1) * 16 + i)) ? x : 0.f;
+                pv[c * 16 + i] = x;
+              }
+#pragma unroll
+              for (int e = 0; e < 2; ++e) split3(pv[c * 16 + 4 * v + 2 * e], pv[c * 16 + 4 * v + 2 * e + 1], pp[0][2 * v + e], pp[1][2 * v + e], pp[2][2 * v + e]);
+            }
+            tmem_st_32x32b_x8(tmem_base + lane_off + P_COL + half * 32 + c * 8, pp[0]);
+            tmem_st_32x32b_x8(s_addr + c * 16, pp[1]);
+            tmem_st_32x32b_x8(s_addr + c * 16 + 8, pp[2]);
+          }
+          tmem_st_wait();
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(p_full);                      // dV runs while dS is made
+          seen[0] &= in[0];
+          seen[1] &= in[1];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            uint32_t td[16], dd[3][8];
+            if constexpr (MASK != 2) {
+              tmem_ld_32x32b_x16(dp_addr + c * 16, td);
+              tmem_ld_wait();
+            }
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              float4 d4 = make_float4(0.f, 0.f, 0.f, 0.f);
+              if constexpr (MASK != 2) d4 = *reinterpret_cast<const float4*>(st + 128 + half * 64 + c * 16 + v * 4);
+              const float de[4] = {d4.x, d4.y, d4.z, d4.w};
+              float dv[4];
+#pragma unroll
+              for (int e = 0; e < 4; e += 2) {
+                float2 y = make_float2(0.f, 0.f);
+                if constexpr (MASK != 2) {
+                  const int i = 4 * v + e;
+                  y = mul2(pv[c * 16 + i], pv[c * 16 + i + 1], fma2(__uint_as_float(td[i]), __uint_as_float(td[i + 1]), p.scale, de[e], de[e + 1]));
+                }
+                dv[e] = y.x;
+                dv[e + 1] = y.y;
+              }
+              if constexpr (MASK == 1 || EDGE) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) dv[e] = seen[c / 2] & (1u << ((c & 1) * 16 + 4 * v + e)) ? dv[e] : 0.f;      // a masked score is a constant
+              }
+#pragma unroll
+              for (int e = 0; e < 2; ++e) split3(dv[2 * e], dv[2 * e + 1], dd[0][2 * v + e], dd[1][2 * v + e], dd[2][2 * v + e]);
+            }
+            if (c == 0 && it > 0) drain(t - 1, item, q_blk - 1);   // dK and dQ of the block before have read its dS
+            uint8_t* drow = sDS + half * (128 * 128) + r * 128;
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+              const int phys = ((c * 2 + v) ^ (r & 7)) * 16;
+#pragma unroll
+              for (int part = 0; part < 3; ++part)
+                *reinterpret_cast<uint4*>(drow + part * SPL_PS + phys) = make_uint4(dd[part][4 * v], dd[part][4 * v + 1], dd[part][4 * v + 2], dd[part][4 * v + 3]);
+            }
+          }
+        };
+        using std::integral_constant;
+        if constexpr (MASKED) {
+          const bool on = __all_sync(0xffffffffu, (bits[0] & bits[1]) == 0xffffffffu), off = __all_sync(0xffffffffu, (bits[0] | bits[1]) == 0u);
+          if (edge) tile(std::true_type{}, integral_constant<int, 1>{});
+          else if (on) tile(std::false_type{}, integral_constant<int, 0>{});
+          else if (off) tile(std::false_type{}, integral_constant<int, 2>{});
+          else tile(std::false_type{}, integral_constant<int, 1>{});
+        } else {
+          if (edge) tile(std::true_type{}, integral_constant<int, 0>{}); else tile(std::false_type{}, integral_constant<int, 0>{});
+        }
+        tc_fence_before_sync();
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(ds_full);
       }
-      __syncwarp();                                                  // whole warps read tensor memory
+      drain(t - 1, item, i_begin + iters - 1);                         // (all products of the item have completed)
+      // ---- dV / dK: thread r <-> key row r
+#pragma unroll
+      for (int which = 0; which < 2; ++which) {
+        uint32_t t[32];
+        tmem_ld_32x32b_x32(tmem_base + lane_off + (which == 0 ? DV_COL : DK_COL) + half * 32, t);
+        tmem_ld_wait();
+        if (k_idx < p.Sk) {
+          const long* st = which == 0 ? p.dv_strides : p.dk_strides;
+          __nv_bfloat16* row = (which == 0 ? p.dv : p.dk) + w.batch * st[0] + w.head * st[1] + k_idx * st[2] + half * 32;
+#pragma unroll
+          for (int i = 0; i < 32; i += 8) {
+            if (half * 32 + i >= p.d) break;
+            *reinterpret_cast<uint4*>(row + i) = make_uint4(
+                pack_bf16(__uint_as_float(t[i]), __uint_as_float(t[i + 1])), pack_bf16(__uint_as_float(t[i + 2]), __uint_as_float(t[i + 3])),
+                pack_bf16(__uint_as_float(t[i + 4]), __uint_as_float(t[i + 5])), pack_bf16(__uint_as_float(t[i + 6]), __uint_as_float(t[i + 7])));
+          }
+        }
+        __syncwarp();                                                  // whole warps read tensor memory
+      }
     }
+    if (lane == 0) tma_store_wait_read<0>();
+    __syncwarp();
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -812,7 +996,10 @@ extern "C" int lb_attn_split_bwd(const void* dout, const void* q, const void* k,
   p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv;
   for (int i = 0; i < 3; ++i) { p.dk_strides[i] = dks[i]; p.dv_strides[i] = dvs[i]; }
   static std::atomic<unsigned long long> c0{0}, c1{0};
-  const dim3 grid(key_blocks, A, B);
+  const long items = (long)key_blocks * A * B;
+  int sms = 0, dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -2;
+  const dim3 grid((unsigned)(items < sms ? items : sms));
   cudaError_t e = mask ? split_configure(lb::attn_split_bwd_kernel<true>, lb::SPL_BWD_SMEM, c1) : split_configure(lb::attn_split_bwd_kernel<false>, lb::SPL_BWD_SMEM, c0);
   if (e != cudaSuccess) return (int)e;
   lb_host::launch_chained(mask ? lb::attn_split_bwd_kernel<true> : lb::attn_split_bwd_kernel<false>, grid, dim3(lb::SPL_THREADS), lb::SPL_BWD_SMEM, s, 0, tq, tk, tv, tdo,

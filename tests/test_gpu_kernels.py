@@ -1216,3 +1216,43 @@ def test_block_graph_refuses_what_changed_in_between():
     y.backward(_rand(y.shape, 5))
     with pytest.raises(RuntimeError, match="second time"):
         y.backward(_rand(y.shape, 5))
+
+
+@pytest.mark.parametrize("kind", ["causal", "none", "padded", "stripes"])
+@pytest.mark.parametrize("b,sq,sk,a,d", [(5, 300, 300, 16, 24), (30, 130, 260, 8, 48), (2, 128, 128, 150, 32), (37, 256, 256, 4, 64)])
+def test_split_attention_of_many_work_items(b, sq, sk, a, d, kind):
+    """Several work items per CTA, rows of the mask that are visible, masked or mixed for 32 or 64 keys at a time: as close to 64 bits as the unfused form, the same
+    bits again."""
+    if kind == "causal" and sk < sq:
+        pytest.skip("more queries than keys under a causal mask: unfused form")
+    m = None
+    if kind == "padded":
+        nq, nk = (torch.randint(1, n + 1, (b,), device="cuda", generator=torch.Generator(device="cuda").manual_seed(n)) for n in (sq, sk))
+        m = ((torch.arange(sq, device="cuda") < nq[:, None])[:, None, :, None] & (torch.arange(sk, device="cuda") < nk[:, None])[:, None, None, :])
+    if kind == "stripes":
+        m = ((torch.arange(sq, device="cuda") // 32)[:, None] + torch.arange(sk, device="cuda") // 64) % 3 != 0
+        m[sq // 3, sk // 2] ^= True
+    causal = kind == "causal" and d != 64         # (head dim 64 takes these kernels with a mask only)
+    if d == 64 and m is None:
+        m = torch.ones(sq, sk, dtype=torch.bool, device="cuda")
+        m = m.tril(sk - sq) if kind == "causal" else m
+    q, k, v, go = _rand((b, a, sq, d), 1), _rand((b, sk, a, d), 2).permute(0, 2, 1, 3), _rand((b, a, sk, d), 3), _rand((b, a, sq, d), 4)
+    keep = torch.ones(sq, sk, dtype=torch.bool, device="cuda").tril(sk - sq) if causal else m
+    x = [t.double().requires_grad_(True) for t in (q, k, v)]
+    s = x[0] @ x[1].transpose(-1, -2) * 0.3
+    if keep is not None:
+        s = s.masked_fill(~keep, float("-inf") if causal else -10000.0)
+    want = torch.softmax(s, -1) @ x[2]
+    want.backward(go.double())
+    far = []
+    for fn in (OF.attention, OF.attention_ref):
+        t = [y.detach().clone().requires_grad_(True) for y in (q, k, v)]
+        y = fn(*t, causal=causal, scale=0.3, mask=m)
+        y.backward(go)
+        far.append([float((u.double() - w).norm() / w.norm()) for u, w in zip((y, *(z.grad for z in t)), (want, *(z.grad for z in x)))])
+        if fn is OF.attention:
+            first = [z.grad for z in t]
+            again = torch.autograd.grad(OF.attention(*t, causal=causal, scale=0.3, mask=m), t, go)
+            assert all(torch.equal(u, w) for u, w in zip(first, again))
+    # the bf16 result's rounding is most of both; the sums of 32-bit products meet in another order
+    assert all(got < 1.05 * ref + 1e-5 for got, ref in zip(*far)), far
