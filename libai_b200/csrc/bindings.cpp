@@ -84,6 +84,8 @@ int lb_masked_attention_tc(const void* q, long ldq, const void* kmat, const void
                            const void* gate, long ldg, int gate_wide, const int* qt_seq, const int* qt_start, int ntiles,
                            const int* seq_off, const int* past, void* y, long ldy, long tokens, long rows, int H, int G, int D, int V,
                            int window, int chunk, float scale, float out_scale, float temp_coef, float temp_every, int* err, cudaStream_t s);
+int lb_gemm_small_norm(const void* x, const void* gamma, const void* beta, float eps, int rms, const void* w, void* out, int M, int N, int K, int ldx, int ldw,
+                       int ldo, const void* bias, int act, cudaStream_t s);
 int lb_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse, int B, int A, int S, int D,
                 const long* q_strides, const long* k_strides, const long* v_strides, int causal, float scale,
                 const int* kv_lens, const void* bias, const long* bias_strides, const float* alibi_slopes, float p_drop,
@@ -1066,6 +1068,23 @@ void block_linear(const void* x, const Tensor& w, const void* bias, int act, voi
         "linear_fwd");
 }
 
+// y [rows, n] = act(norm(x [rows, h]) wᵀ + bias): one kernel for a few rows (true), else the norm into `tmp` and the product (no beta: RMS norm; stats: 2 rows
+// of fp32)
+bool block_norm_linear(const void* x, const Tensor& gamma, const void* beta, double eps, const void* w, int64_t n, int64_t h, const void* bias, int act, void* y,
+                       int64_t rows, void* tmp, float* stats) {
+  const int rms = beta == nullptr ? 1 : 0;
+  if (rows <= 16) {
+    const int rc = lb_gemm_small_norm(x, gamma.data_ptr(), beta, (float)eps, rms, w, y, (int)rows, (int)n, (int)h, (int)h, (int)h, (int)n, bias, act, cur_stream());
+    if (rc != -1) {
+      check(rc, "norm_linear");
+      return true;
+    }
+  }
+  check(lb_norm_fwd(x, gamma.data_ptr(), beta, tmp, rms ? nullptr : stats, rms ? stats : stats + rows, (int)rows, (int)h, (float)eps, rms, 0, 0, cur_stream()), "norm_fwd");
+  check(lb_gemm_bf16(tmp, w, y, (int)rows, (int)n, (int)h, (int)h, (int)h, (int)n, 0, 0, bias, act, nullptr, 0, 0, cur_stream()), "linear_fwd");
+  return false;
+}
+
 // Pre-norm block: params = norm weight, bias; qkv weight, bias; projection weight, bias; norm weight, bias; h->4h weight, bias; 4h->h weight, bias.
 // x [B, S, h] -> {y} or, against caches, {y, keys, values}
 std::vector<Tensor> block_fwd(const Tensor& x, const std::vector<Tensor>& p, int64_t heads, double eps1, double eps2, double scale, bool causal,
@@ -1083,13 +1102,11 @@ std::vector<Tensor> block_fwd(const Tensor& x, const std::vector<Tensor>& p, int
   s.make(x);
   std::vector<Tensor> out{at::empty_like(x)};
   float* st = reinterpret_cast<float*>(s(stats));
-  check(lb_norm_fwd(x.data_ptr(), p[0].data_ptr(), p[1].data_ptr(), s(norm), st, st + T, (int)T, (int)h, (float)eps1, 0, 0, 0, cur_stream()), "norm_fwd");
-  block_linear(s(norm), p[2], p[3].data_ptr(), 0, s(wide), T);
+  block_norm_linear(x.data_ptr(), p[0], p[1].data_ptr(), eps1, p[2].data_ptr(), 3 * ad, h, p[3].data_ptr(), 0, s(wide), T, s(norm), st);
   block_attention(s(wide), s(norm), st, B, S, heads, d, causal, scale, past_k, past_v, out);
   check(lb_gemm_bf16_bias_residual(s(norm), p[4].data_ptr(), s(mid), (int)T, (int)h, (int)ad, (int)ad, (int)ad, p[5].data_ptr(), x.data_ptr(), cur_stream()),
         "linear_bias_residual");
-  check(lb_norm_fwd(s(mid), p[6].data_ptr(), p[7].data_ptr(), s(norm), st, st + T, (int)T, (int)h, (float)eps2, 0, 0, 0, cur_stream()), "norm_fwd");
-  block_linear(s(norm), p[8], p[9].data_ptr(), 1 /* GELU */, s(wide), T);
+  block_norm_linear(s(mid), p[6], p[7].data_ptr(), eps2, p[8].data_ptr(), f, h, p[9].data_ptr(), 1 /* GELU */, s(wide), T, s(norm), st);
   check(lb_gemm_bf16_bias_residual(s(wide), p[10].data_ptr(), out[0].data_ptr(), (int)T, (int)h, (int)f, (int)f, (int)f, p[11].data_ptr(), s(mid), cur_stream()),
         "linear_bias_residual");
   return out;
@@ -1120,21 +1137,19 @@ std::vector<Tensor> llama_block_fwd(const Tensor& x, const std::vector<Tensor>& 
   s.make(x);
   std::vector<Tensor> out{at::empty_like(x)};
   float* st = reinterpret_cast<float*>(s(stats));
-  check(lb_norm_fwd(x.data_ptr(), p[0].data_ptr(), nullptr, s(norm), nullptr, st, (int)T, (int)h, (float)eps1, 1, 0, 0, cur_stream()), "norm_fwd");
-  block_linear(s(norm), p[1], bias.has_value() ? bias->data_ptr() : nullptr, 0, s(wide), T);
+  block_norm_linear(x.data_ptr(), p[0], nullptr, eps1, p[1].data_ptr(), 3 * ad, h, bias.has_value() ? bias->data_ptr() : nullptr, 0, s(wide), T, s(norm), st);
   check(lb_rope_qkv(s(wide), cosv.data_ptr<float>(), sinv.data_ptr<float>(), s(rot), T * heads, (int)S, (int)heads, (int)d, (int)at0, 0, cur_stream()), "rope_qkv");
   block_attention(s(rot), s(norm), st, B, S, heads, d, true, scale, past_k, past_v, out);
   check(lb_gemm_bf16_bias_residual(s(norm), p[2].data_ptr(), s(mid), (int)T, (int)h, (int)ad, (int)ad, (int)ad, nullptr, x.data_ptr(), cur_stream()),
         "linear_bias_residual");
-  check(lb_norm_fwd(s(mid), p[3].data_ptr(), nullptr, s(norm), nullptr, st, (int)T, (int)h, (float)eps2, 1, 0, 0, cur_stream()), "norm_fwd");
+  auto project = [&](int i, int64_t n, void* y) { return block_norm_linear(s(mid), p[3], nullptr, eps2, p[i].data_ptr(), n, h, nullptr, 0, y, T, s(norm), st); };
   if (joint) {
-    check(lb_gemm_bf16(s(norm), p[4].data_ptr(), s(wide), (int)T, (int)(2 * f), (int)h, (int)h, (int)h, (int)(2 * f), 0, 0, nullptr, 0, nullptr, 0, 0, cur_stream()),
-          "gemm");
+    project(4, 2 * f, s(wide));
     check(lb_swiglu_packed_fwd(s(wide), s(rot), T, f, cur_stream()), "swiglu_packed_fwd");
   } else {
     char* up = s(wide) + T * f * 2;
-    block_linear(s(norm), p[4], nullptr, 0, s(wide), T);
-    block_linear(s(norm), p[5], nullptr, 0, up, T);
+    if (project(4, f, s(wide))) project(5, f, up);
+    else block_linear(s(norm), p[5], nullptr, 0, up, T);
     check(lb_swiglu_fwd(s(wide), up, s(rot), T * f, cur_stream()), "swiglu_fwd");
   }
   check(lb_gemm_bf16_bias_residual(s(rot), p[6].data_ptr(), out[0].data_ptr(), (int)T, (int)h, (int)f, (int)f, (int)f, nullptr, s(mid), cur_stream()),

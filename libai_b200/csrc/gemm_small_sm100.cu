@@ -26,7 +26,8 @@ struct GsCfg {
   static_assert(PART_BYTES <= 2 * STAGE, "partial sums fit the pipeline");
 };
 constexpr int GS_SMEM = 104000;                   // of pipeline: two CTAs per SM (one with twice the stages leaves no room for clusters of 8 in some GPCs)
-constexpr int GS_MAX_STAGES = GS_SMEM / GsCfg<16>::STAGE, GS_TAIL = 1024 + 256;   // alignment, barriers
+constexpr int GS_NORM_BLOCKS = 11;                // k-blocks per CTA with a norm in front: their rows of x beside five stages of w
+constexpr int GS_MAX_STAGES = GS_SMEM / GsCfg<16>::STAGE, GS_TAIL = 1024 + 512;   // alignment, barriers, statistics
 
 struct GemmSmallParams {
   int M, N, K, kb_total, kb_per_cta, stages;
@@ -35,7 +36,19 @@ struct GemmSmallParams {
   __nv_bfloat16 *out, *pre_out;   // [M, ldo]; pre_out (optional): before the activation
   int ldo, act;
   int* err;
+  // with a norm in front: rows of x as they are, its weight and bias (or nullptr)
+  const __nv_bfloat16 *x, *gamma, *beta;
+  int ldx, rms;
+  float eps;
 };
+
+// count, mean and sum of squared deviations of two sets of numbers together
+LB_DEVICE void merge_moments(float& n, float& mean, float& m2, float n2, float mean2, float m22) {
+  const float all = n + n2, d = mean2 - mean, f = all > 0.f ? n2 / all : 0.f;
+  mean = fmaf(d, f, mean);
+  m2 += m22 + d * d * n * f;
+  n = all;
+}
 
 // four partial sums of CTA `rank` of the cluster (its own through the same window)
 LB_DEVICE float4 gs_ld_remote(uint32_t addr, uint32_t rank) {
@@ -46,18 +59,23 @@ LB_DEVICE float4 gs_ld_remote(uint32_t addr, uint32_t rank) {
   return v;
 }
 
-// grid (cluster, tiles of 128 columns of y, tiles of NT rows of y)
-template <int NT, int RANKS>
+// grid (cluster, tiles of 128 columns of y, tiles of NT rows of y).  NORM: x are the rows before a layer or RMS norm; the epilogue's warps read them, take their
+// statistics (every CTA those of all its rows) and write the normalised bf16 rows of each k-block where TMA would have put them, while w is on its way.
+template <int NT, int RANKS, bool NORM>
 __global__ void __launch_bounds__(GS_THREADS, 2)
 gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, GemmSmallParams p) {
   using Cfg = GsCfg<NT>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + p.stages * Cfg::STAGE);
+  constexpr int STAGE = NORM ? GS_W_BYTES : Cfg::STAGE;             // NORM: all of the CTA's rows of x behind the stages of w
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + p.stages * STAGE + (NORM ? p.kb_per_cta * Cfg::X_BYTES : 0));
   uint64_t* empty_bar = full_bar + GS_MAX_STAGES;
   uint64_t* acc_full = empty_bar + GS_MAX_STAGES;
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(acc_full + 1);
   volatile int* stop = reinterpret_cast<volatile int*>(acc_full + 2);
+  [[maybe_unused]] uint64_t* x_full = acc_full + 3;
+  [[maybe_unused]] float* row_mean = reinterpret_cast<float*>(full_bar + 20);       // 16, then 16 reciprocal deviations (NORM: NT = 16)
+  static_assert(!NORM || (NT == 16 && 2 * GS_MAX_STAGES + 4 <= 20), "statistics lie behind the barriers");
   const int warp_idx = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int rank = blockIdx.x;
   const int n0 = blockIdx.y * 128, m0 = blockIdx.z * NT;
@@ -65,8 +83,9 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmap_w);
-    tma_prefetch_desc(&tmap_x);
+    if constexpr (!NORM) tma_prefetch_desc(&tmap_x);
     for (int i = 0; i < p.stages; ++i) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], 1); }
+    if constexpr (NORM) mbar_init(x_full, 4);
     mbar_init(acc_full, 1);
     *stop = 0;
     fence_barrier_init();
@@ -77,7 +96,8 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
-  chain_wait();
+  const __nv_bfloat16 *xg = p.x, *gamma = p.gamma, *beta = p.beta;
+  chain_wait(xg, gamma, beta);
   chain_next();
 
   if (warp_idx == 0) {
@@ -86,10 +106,10 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       uint32_t phase = 1;
       for (int kb = kb0; kb < kb1; ++kb) {
         if (!tc_wait(&empty_bar[s], phase, stop)) break;
-        uint8_t* sw = smem + s * Cfg::STAGE;
-        mbar_arrive_expect_tx(&full_bar[s], Cfg::STAGE);
+        uint8_t* sw = smem + s * STAGE;
+        mbar_arrive_expect_tx(&full_bar[s], STAGE);
         tma_load_2d(sw, &tmap_w, &full_bar[s], kb * 64, n0);
-        tma_load_2d(sw + GS_W_BYTES, &tmap_x, &full_bar[s], kb * 64, m0);
+        if constexpr (!NORM) tma_load_2d(sw + GS_W_BYTES, &tmap_x, &full_bar[s], kb * 64, m0);
         if (++s == p.stages) { s = 0; phase ^= 1; }
       }
     }
@@ -97,13 +117,14 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   } else if (warp_idx == 1) {
     constexpr uint32_t idesc = make_idesc_bf16(128, NT, false, false);
     bool ok = true;
+    if constexpr (NORM) ok = __all_sync(0xffffffffu, tc_wait(x_full, 0, stop));
     int s = 0;
     uint32_t phase = 0;
     for (int kb = kb0; kb < kb1; ++kb) {
       ok = __all_sync(0xffffffffu, ok && tc_wait(&full_bar[s], phase, stop));
       tc_fence_after_sync();
       if (ok && elect_one()) {
-        const uint32_t sw = smem_u32(smem + s * Cfg::STAGE), sx = sw + GS_W_BYTES;
+        const uint32_t sw = smem_u32(smem + s * STAGE), sx = NORM ? smem_u32(smem + p.stages * STAGE + (kb - kb0) * Cfg::X_BYTES) : sw + GS_W_BYTES;
 #pragma unroll
         for (int k = 0; k < 4; ++k)
           umma_f16_ss(tmem_base, make_smem_desc_sw128(sw + k * 32, 0, 1024), make_smem_desc_sw128(sx + k * 32, 0, 1024), idesc, (kb > kb0 || k > 0) ? 1u : 0u);
@@ -112,6 +133,124 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       }
       __syncwarp();
       if (++s == p.stages) { s = 0; phase ^= 1; }
+    }
+  }
+  if constexpr (NORM) {
+    if (warp_idx >= 2) {
+      const int tid = static_cast<int>(threadIdx.x) - 64, rows = min(16, p.M - m0);
+      auto unpack8 = [](const uint4& q, float (&v)[8]) {
+        const float2 a = unpack_bf16(q.x), b = unpack_bf16(q.y), c = unpack_bf16(q.z), d = unpack_bf16(q.w);
+        v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = c.x; v[5] = c.y; v[6] = d.x; v[7] = d.y;
+      };
+      // 16 bytes of a row of a k-block; those of the first two k-blocks are on their way while the statistics are taken
+      const int row = tid / 8, chunk = tid % 8;
+      const bool live = row < rows;
+      const __nv_bfloat16* xr = xg + static_cast<size_t>(m0 + (live ? row : 0)) * p.ldx;
+      uint4 first[2][3];
+      auto fetch = [&](int kb, uint4 (&q)[3]) {
+        const int k = kb * 64 + chunk * 8;
+        q[0] = q[1] = q[2] = make_uint4(0u, 0u, 0u, 0u);
+        if (live && kb < kb1 && k < p.K) {
+          q[0] = *reinterpret_cast<const uint4*>(xr + k);
+          q[1] = *reinterpret_cast<const uint4*>(gamma + k);
+          if (beta != nullptr) q[2] = *reinterpret_cast<const uint4*>(beta + k);
+        }
+      };
+      fetch(kb0, first[0]);
+      fetch(kb0 + 1, first[1]);
+      {                                             // statistics: a power of two of threads per row, as many as there are
+        int lanes = 8;
+        while (lanes < 128 && rows * lanes * 2 <= 128) lanes *= 2;
+        const int srow = tid / lanes, sub = tid % lanes;
+        float n = 0.f, mean = 0.f, m2 = 0.f;
+        if (srow < rows) {
+          const __nv_bfloat16* sr = xg + static_cast<size_t>(m0 + srow) * p.ldx;
+          for (int k = sub * 8; k < p.K; k += lanes * 32) {          // up to 32 numbers at a time: their mean, then their deviations from it
+            uint4 q[4];
+            float cnt = 0.f, sum = 0.f, sq = 0.f;
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+              const bool in = k + a * lanes * 8 < p.K;
+              q[a] = in ? *reinterpret_cast<const uint4*>(sr + k + a * lanes * 8) : make_uint4(0u, 0u, 0u, 0u);
+              cnt += in ? 8.f : 0.f;
+            }
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+              float v[8];
+              unpack8(q[a], v);
+#pragma unroll
+              for (int e = 0; e < 8; ++e) {
+                sum += v[e];
+                if (p.rms) sq = fmaf(v[e], v[e], sq);
+              }
+            }
+            if (p.rms) {
+              m2 += sq;
+              continue;
+            }
+            const float c = sum / cnt;
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+              float v[8];
+              unpack8(q[a], v);
+              float part = 0.f;
+#pragma unroll
+              for (int e = 0; e < 8; ++e) part = fmaf(v[e] - c, v[e] - c, part);
+              sq += 8.f * a < cnt ? part : 0.f;
+            }
+            merge_moments(n, mean, m2, cnt, c, sq);
+          }
+        }
+        for (int m = 1; m < min(lanes, 32); m <<= 1) {
+          const float n2 = __shfl_xor_sync(0xffffffffu, n, m), mean2 = __shfl_xor_sync(0xffffffffu, mean, m), m22 = __shfl_xor_sync(0xffffffffu, m2, m);
+          if (p.rms) m2 += m22;
+          else merge_moments(n, mean, m2, n2, mean2, m22);
+        }
+        float* over = row_mean + 32;                // sums of whole warps, where a row has several: [warp][3]
+        if (lanes > 32) {
+          if (lane == 0) {
+            over[(warp_idx - 2) * 3] = n;
+            over[(warp_idx - 2) * 3 + 1] = mean;
+            over[(warp_idx - 2) * 3 + 2] = m2;
+          }
+          asm volatile("bar.sync 1, 128;\n" ::: "memory");
+          const int per = lanes / 32, first = (warp_idx - 2) / per * per;
+          n = over[first * 3];
+          mean = over[first * 3 + 1];
+          m2 = over[first * 3 + 2];
+          for (int w = first + 1; w < first + per; ++w) {
+            if (p.rms) m2 += over[w * 3 + 2];
+            else merge_moments(n, mean, m2, over[w * 3], over[w * 3 + 1], over[w * 3 + 2]);
+          }
+        }
+        if (sub == 0 && srow < rows) {
+          row_mean[srow] = p.rms ? 0.f : mean;
+          row_mean[16 + srow] = rsqrtf(m2 / p.K + p.eps);
+        }
+        asm volatile("bar.sync 1, 128;\n" ::: "memory");
+      }
+      const float mean = live ? row_mean[row] : 0.f, rstd = live ? row_mean[16 + row] : 0.f;
+      uint8_t* xs = smem + p.stages * STAGE;        // the CTA's k-blocks one behind the other
+      auto put = [&](int kb, const uint4 (&q)[3]) {
+        float v[8], g[8], b[8];
+        unpack8(q[0], v);
+        unpack8(q[1], g);
+        unpack8(q[2], b);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = fmaf((v[e] - mean) * rstd, g[e], b[e]);          // (zeros behind the rows and columns there are)
+        *reinterpret_cast<uint4*>(xs + (kb - kb0) * Cfg::X_BYTES + row * 128 + ((chunk ^ (row & 7)) << 4)) =
+            make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+      };
+      if (kb0 < kb1) put(kb0, first[0]);
+      if (kb0 + 1 < kb1) put(kb0 + 1, first[1]);
+#pragma unroll 2
+      for (int kb = kb0 + 2; kb < kb1; ++kb) {
+        fetch(kb, first[0]);
+        put(kb, first[0]);
+      }
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(x_full);
     }
   }
   // the pipeline has run dry once acc_full has come (every full stage was consumed): its memory holds the partial sums [NT][128] now
@@ -191,13 +330,14 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   }
 }
 
-template <int NT, int RANKS>
+template <int NT, int RANKS, bool NORM = false>
 cudaError_t launch_gemm_small_r(const CUtensorMap& tw, const CUtensorMap& tx, GemmSmallParams p, cudaStream_t s) {
-  auto kern = gemm_small_kernel<NT, RANKS>;
-  const int fit = GS_SMEM / GsCfg<NT>::STAGE;
+  auto kern = gemm_small_kernel<NT, RANKS, NORM>;
+  const int stage = NORM ? GS_W_BYTES : GsCfg<NT>::STAGE, rows = NORM ? p.kb_per_cta * GsCfg<NT>::X_BYTES : 0;
+  const int fit = (GS_SMEM - rows) / stage;
   p.stages = p.kb_per_cta < 2 ? 2 : p.kb_per_cta;
   if (p.stages > fit) p.stages = fit;
-  const int smem = p.stages * GsCfg<NT>::STAGE + GS_TAIL;
+  const int smem = p.stages * stage + rows + GS_TAIL;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GS_SMEM + GS_TAIL);
@@ -319,4 +459,41 @@ extern "C" int lb_gemm_small(const void* x, const void* w, void* out, int M, int
   cudaError_t e = nt == 16 ? lb::launch_gemm_small<16>(tw, tx, p, ranks, s) : nt == 32 ? lb::launch_gemm_small<32>(tw, tx, p, ranks, s)
                   : nt == 64 ? lb::launch_gemm_small<64>(tw, tx, p, ranks, s) : lb::launch_gemm_small<128>(tw, tx, p, ranks, s);
   return (int)e;
+}
+
+// The same for up to 16 rows with a layer norm (without beta, `rms`: an RMS norm) of x in front: y = act(norm(x) · wᵀ + bias), two launches in one.  [8, 1024] x
+// [3072, 1024] and [4096, 1024] 6.8 us each, where norm and product took 2.4 + 4.9; what counts is the launch that the host does not make: a step of GPT-2 against a cache
+// (5 launches in place of 7) 44.5 -> 39.3 us.  Not where a CTA has more than 11 k-blocks ([4, 4096] x [12288, 4096], 32 of them): their rows do not fit beside the stages
+// of w, and normalised k-block by k-block behind w they hold it up (three products of Llama-2 7B 63 + 5 us for the norms, 83 so).
+extern "C" int lb_gemm_small_norm(const void* x, const void* gamma, const void* beta, float eps, int rms, const void* w, void* out, int M, int N, int K, int ldx,
+                                  int ldw, int ldo, const void* bias, int act, cudaStream_t s) {
+  const uintptr_t vec = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gamma) | reinterpret_cast<uintptr_t>(beta) | reinterpret_cast<uintptr_t>(w);
+  if (M <= 0 || M > 16 || N <= 0 || K <= 0 || N % 4 || K % 8 || ldo % 4 || ldx % 8 || ldw % 8 || (vec & 15) ||
+      ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(bias)) & 7) || (N + 127) / 128 > 65535)
+    return -1;
+  int nt = 0, ranks = 0;
+  if (!lb_gemm_small_rule(M, N, K, &nt, &ranks) || nt != 16) return -1;
+  if (((K + 63) / 64 + ranks - 1) / ranks > lb::GS_NORM_BLOCKS) return -1;
+  lb::GemmSmallParams p{};
+  p.err = small_wait_word();
+  if (p.err == nullptr) return -20;
+  p.M = M; p.N = N; p.K = K;
+  p.kb_total = (K + 63) / 64;
+  p.kb_per_cta = (p.kb_total + ranks - 1) / ranks;
+  p.bias = (const __nv_bfloat16*)bias;
+  p.out = (__nv_bfloat16*)out;
+  p.ldo = ldo;
+  p.act = act;
+  p.x = (const __nv_bfloat16*)x; p.gamma = (const __nv_bfloat16*)gamma; p.beta = (const __nv_bfloat16*)beta;
+  p.ldx = ldx; p.rms = rms; p.eps = eps;
+  CUtensorMap tw;
+  const uint64_t dims[2] = {(uint64_t)K, (uint64_t)N}, strides[2] = {2, (uint64_t)ldw * 2};
+  const uint32_t box[2] = {64u, 128u};
+  if (!lb_host::make_tmap_bf16(&tw, w, 2, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B)) return -2;
+  switch (ranks) {
+    case 1: return (int)lb::launch_gemm_small_r<16, 1, true>(tw, tw, p, s);
+    case 2: return (int)lb::launch_gemm_small_r<16, 2, true>(tw, tw, p, s);
+    case 4: return (int)lb::launch_gemm_small_r<16, 4, true>(tw, tw, p, s);
+    default: return (int)lb::launch_gemm_small_r<16, 8, true>(tw, tw, p, s);
+  }
 }

@@ -1256,3 +1256,22 @@ def test_split_attention_of_many_work_items(b, sq, sk, a, d, kind):
             assert all(torch.equal(u, w) for u, w in zip(first, again))
     # the bf16 result's rounding is most of both; the sums of 32-bit products meet in another order
     assert all(got < 1.05 * ref + 1e-5 for got, ref in zip(*far)), far
+
+
+@pytest.mark.parametrize("rms", [False, True])
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 5, 8, 9, 16])
+@pytest.mark.parametrize("n,k", [(40, 8), (136, 1032), (1152, 384), (3072, 1024), (6144, 2048), (520, 4096)])
+def test_linear_of_few_rows_behind_a_norm(n, k, m, rms):
+    """Statistics by 8 to 128 threads per row, rows and k-blocks that end early, clusters with empty CTAs; rows with a large common part, which a sum of squares would not survive."""
+    x, g, b = _rand((m, k), 1) * 2 + 50, 1 + 0.1 * _rand((k,), 2), None if rms else _rand((k,), 3)
+    w, bias = _rand((n, k), 4, k ** -0.5), _rand((n,), 5)
+    y = torch.full((m + 1, n), 7.0, device="cuda", dtype=BF16)
+    ptr = lambda t: ctypes.c_void_p(0 if t is None else t.data_ptr())
+    rc = ctypes.CDLL(so_path()).lb_gemm_small_norm(ptr(x), ptr(g), ptr(b), ctypes.c_float(1e-5), int(rms), ptr(w), ptr(y), m, n, k, k, k, n, ptr(bias), 0,
+                                                   ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    d = x.double()
+    d = d * torch.rsqrt(d.square().mean(-1, keepdim=True) + 1e-5) * g.double() if rms else torch.nn.functional.layer_norm(d, (k,), g.double(), b.double(), 1e-5)
+    want = d.to(BF16).double() @ w.double().t() + bias.double()
+    # the normalised rows are rounded to bf16 once (some a step off, where 32 and 64 bits round apart), the result once
+    assert float((y[:m].double() - want).norm()) < 2.0 ** -8 * float(want.norm()) and bool((y[m] == 7).all())
