@@ -1089,9 +1089,10 @@ static int split_choice(long tiles, int k_blocks, int sms) {
 }
 // Width of the pair tiles of an accumulation (weight gradients): fixed + rounds x (per round + k-blocks x per k-block) + bytes added.  Fitted over 48 products of up to
 // [3072, 1024], K = 512 .. 8192 (2.5 to 5 % rms; the narrow ones have to be 3 % ahead).  256 wide and the chosen width, us: [1152, 384] x K = 2048 9.9 -> 8.1, [1536, 384] x 2048 9.1 -> 7.4,
-// [2304, 768] x 5000 19.2 -> 16.7, [1280, 1280] x 5000 19.3 -> 16.2, [1024, 1024] x 512 8.4 -> 6.8; [3072, 1024] x 8192 and larger keep 256.
+// [2304, 768] x 5000 19.2 -> 16.7, [1280, 1280] x 5000 19.3 -> 16.2, [1024, 1024] x 512 8.4 -> 6.8; [3072, 1024] x 8192 and larger keep 256 (the fit's bytes are up to 13 MB, and a
+// MB costs all three the same: [21128, 768] x 1304 took 68 us 128 wide, 50 us 256 wide).
 static int wgrad_tile_choice(int M, int N, int K, int sms) {
-  static const struct { int bn; double fixed, round, block, mb; } kinds[3] = {{256, 6.56, 0.0, 0.322, 0.061}, {192, 5.25, 0.90, 0.273, 0.049}, {128, 6.10, 0.0, 0.207, 0.0129}};
+  static const struct { int bn; double fixed, round, block, mb; } kinds[3] = {{256, 6.56, 0.0, 0.322, 0.061}, {192, 5.25, 0.90, 0.273, 0.061}, {128, 6.10, 0.0, 0.207, 0.061}};
   const int kb = (K + lb::BLOCK_K - 1) / lb::BLOCK_K, m_blocks = (M + lb::BLOCK_M - 1) / lb::BLOCK_M;
   double best = 1e30;
   int bn = 256;
