@@ -514,6 +514,7 @@ struct Gradients {                        // of the parameters, by index
     }
   }
   void bias(size_t i, const Tensor& g, const Tensor& b) {
+    if (added[i]) return;
     count(1);
     if (fp32(main[i])) {
       lb_ops::colsum(g, main[i]);
@@ -534,6 +535,20 @@ struct Gradients {                        // of the parameters, by index
     out[i] = gw.to(w.scalar_type());
     if (has_bias) out[i + 1] = gb.to(w.scalar_type());
     return gx;
+  }
+  // the same of a layer norm, with the gradients of the biases around it: `before` that of the layer that made its input (column sums of the result), `behind` that of the
+  // layer whose output the skip connection joined (column sums of `skip`; -1: not asked for).  Those that it has not made are left to bias().
+  Tensor norm_and_biases(size_t i, const Tensor& g, const Tensor& x, const Tensor& w, const Tensor& mean, const Tensor& rstd, const Tensor& skip, int before, int behind) {
+    if (fp32(main[i]) && fp32(main[i + 1]) && fp32(main[before]) && (behind < 0 || fp32(main[behind]))) {
+      const Tensor gx = lb_ops::norm_bwd_sums(g, x, w, mean, rstd, main[i], main[i + 1], skip, behind < 0 ? Tensor() : main[behind], main[before]);
+      if (gx.defined()) {
+        count(1);
+        added[i] = added[i + 1] = added[before] = 1;
+        if (behind >= 0) added[behind] = 1;
+        return gx;
+      }
+    }
+    return norm(i, g, x, w, mean, rstd, false, true, skip);
   }
   void mark(at::TensorList p) const {
     pybind11::gil_scoped_acquire gil;
@@ -656,8 +671,8 @@ struct Block : Function<Block> {
       if (fused) g.added[m + 3] = 1;
       else g.bias(m + 3, dpre, p[m + 3]);
       Tensor dln = input_grad(dpre, p[m + 2]);
+      Tensor dy = g.norm_and_biases(m, dln, cross ? cr[10] : self[9], p[m], ff[1], ff[2], gy, cross ? 13 : 5, static_cast<int>(m) + 5);
       g.bias(m + 5, gy, p[m + 5]);
-      Tensor dy = g.norm(m, dln, cross ? cr[10] : self[9], p[m], ff[1], ff[2], false, true, gy);
       auto attend_back = [&](int64_t layout, const Tensor& t0, const Tensor& t1, const Tensor& dctx, const Tensor* kept, bool causal_, double scale, Tensor& g0,
                              Tensor& g1) {
         g0 = at::empty(t0.sizes(), t0.options());
@@ -683,7 +698,7 @@ struct Block : Function<Block> {
         dln = input_grad(gq, p[8]);
         g.weight(8, gq, cr[0], p[8]);
         g.bias(9, gq, p[9]);
-        dy = g.norm(6, dln, self[9], p[6], cr[1], cr[2], false, true, dy);
+        dy = g.norm_and_biases(6, dln, self[9], p[6], cr[1], cr[2], dy, 5, -1);
       }
       const Tensor qkv = self[3].view({B, S, heads, 3 * d});
       const Tensor dctx = input_grad(dy, p[4]);

@@ -84,6 +84,8 @@ int lb_masked_attention_tc(const void* q, long ldq, const void* kmat, const void
                            const void* gate, long ldg, int gate_wide, const int* qt_seq, const int* qt_start, int ntiles,
                            const int* seq_off, const int* past, void* y, long ldy, long tokens, long rows, int H, int G, int D, int V,
                            int window, int chunk, float scale, float out_scale, float temp_coef, float temp_every, int* err, cudaStream_t s);
+int lb_norm_bwd_sums(const void* gy, const void* x, const void* gamma, const float* mean, const float* rstd, void* gx, float* dgamma, float* dbeta, int rows, int H,
+                     const void* gadd, float* sum_add, float* sum_out, cudaStream_t s);
 int lb_gemm_small_norm(const void* x, const void* gamma, const void* beta, float eps, int rms, const void* w, void* out, int M, int N, int K, int ldx, int ldw,
                        int ldo, const void* bias, int act, cudaStream_t s);
 int lb_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse, int B, int A, int S, int D,
@@ -534,6 +536,26 @@ std::tuple<Tensor, Tensor, Tensor> norm_bwd(const Tensor& gy, const Tensor& x, c
   if (has_add && !fuse_add) gx.add_(gadd->to(gx.scalar_type()));
   if (acc) return std::make_tuple(gx, at::empty({0}, fopt), at::empty({0}, fopt));
   return std::make_tuple(gx, dgamma, dbeta);
+}
+
+// norm_bwd of a layer norm into fp32 gradients that also adds the column sums of gadd and of its result to `sum_add` and `sum_out` (fp32, either may be undefined);
+// undefined: not of that form
+Tensor norm_bwd_sums(const Tensor& gy, const Tensor& x, const Tensor& gamma, const Tensor& mean, const Tensor& rstd, const Tensor& dgamma, const Tensor& dbeta,
+                     const Tensor& gadd, const Tensor& sum_add, const Tensor& sum_out) {
+  const int rows = (int)x.size(0), H = (int)x.size(1);
+  for (const Tensor* t : {&gy, &x, &gadd})
+    if (!t->defined() || t->scalar_type() != at::kBFloat16 || !t->is_contiguous() || t->sizes() != x.sizes()) return {};
+  for (const Tensor* t : {&dgamma, &dbeta, &sum_add, &sum_out})
+    if (t->defined() && (t->scalar_type() != at::kFloat || !t->is_contiguous() || t->numel() != H || t->device() != x.device())) return {};
+  if (!dgamma.defined() || !dbeta.defined() || gamma.scalar_type() != at::kBFloat16) return {};
+  c10::cuda::CUDAGuard guard(x.device());
+  Tensor gx = at::empty_like(x);
+  auto ptr = [](const Tensor& t) { return t.defined() ? t.data_ptr<float>() : nullptr; };
+  const int rc = lb_norm_bwd_sums(gy.data_ptr(), x.data_ptr(), gamma.data_ptr(), mean.data_ptr<float>(), rstd.data_ptr<float>(), gx.data_ptr(), ptr(dgamma), ptr(dbeta),
+                                  rows, H, gadd.data_ptr(), ptr(sum_add), ptr(sum_out), cur_stream());
+  if (rc == -3) return {};
+  check(rc, "norm_bwd_sums");
+  return gx;
 }
 
 // ---- elementwise ------------------------------------------------------------------------------------

@@ -6,6 +6,7 @@
 //   bwd : dx = rstd * (g·γ - mean_h(g·γ) - x̂ · mean_h(g·γ·x̂))   (rms: no mean_h(g·γ) term)
 //         dγ = Σ_rows g·x̂ ,  dβ = Σ_rows g        (two-stage: per-CTA partials, then column reduce)
 #include "common.cuh"
+#include <atomic>
 #include <type_traits>
 
 namespace lb {
@@ -176,61 +177,85 @@ norm_bwd_kernel(const T* __restrict__ gy, const T* __restrict__ x, const W* __re
   }
 }
 
-// bf16 activations, bandwidth-oriented variant of the kernel above (same maths, same outputs).  The first version kept
-// x̂ and g·γ of a row as 2 x VPL x 8 floats across the two warp reductions and fetched the residual gradient afterwards:
-// 191 registers → one 8-warp block per SM, and three dependent memory phases per row — 19 µs for [8192, 1024] where
-// the 64 MB it moves take 9 µs.  Here a row's x, gy and residual gradient are
-// fetched together as raw 16-byte vectors (3 x VPL x 4 registers), unpacked twice (before and after the reductions:
-// ALU is free here), and blocks are 4 warps at <= 168 registers → 12 warps per SM with 12 loads each in flight.
-constexpr int NORM_BWD_WARPS = 4;
+// bf16 activations up to 1024 columns: a warp per row like the kernel above (same maths, same outputs), bounded by memory.  Rows go through a ring in shared memory, three
+// per warp, filled by cp.async (every lane copies what it reads itself: no barrier), so that loads are in flight while a row is worked on; x, gy and the residual's gradient in
+// registers, fetched row by row, took [8192, 1024] 16.0 -> 14.3 us (floor 10.2) and [12608, 1024] 23.0 -> 19.7 (15.8).  12 warps per SM.
+// SUMS: the column sums of the residual's gradient and of the result too, which are the gradients of the biases in front of and behind this norm in a block (they would read
+// both tensors again: with both 14.3 and 20.5 us, without column sums of 4 to 9 us each behind it).
+constexpr int NORM_BWD_WARPS = 4, NORM_BWD_STAGES = 3;
+LB_DEVICE void cp_async_16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
 
-template <typename W, int VPL, bool RMS, bool TAIL>
-__global__ void __launch_bounds__(NORM_BWD_WARPS * 32, 3)
+constexpr int norm_bwd_blocks(int vpl, bool sums) { return sums && vpl == 4 ? 2 : 3; }     // per SM: four column sums of 1024 columns need 190 registers
+template <typename W, int VPL, bool RMS, bool TAIL, bool SUMS>
+__global__ void __launch_bounds__(NORM_BWD_WARPS * 32, norm_bwd_blocks(VPL, SUMS))
 norm_bwd_bf16_kernel(const __nv_bfloat16* __restrict__ gy, const __nv_bfloat16* __restrict__ x, const W* __restrict__ gamma,
                      const float* __restrict__ mean_in, const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ gx,
                      float* __restrict__ part_dgamma, float* __restrict__ part_dbeta, int rows,
                      const __nv_bfloat16* __restrict__ gadd, float* __restrict__ acc_dgamma, float* __restrict__ acc_dbeta,
-                     int h_tail) {
+                     float* __restrict__ sum_add, float* __restrict__ sum_out, int h_tail) {
   chain_next();
   const int H = TAIL ? h_tail : VPL * 256;       // TAIL: lanes behind the row's end neither load nor store
   const float inv_h = 1.0f / static_cast<float>(H);
-  __shared__ float red[NORM_BWD_WARPS][32 * 8 + 8];
+  extern __shared__ uint4 norm_ring[];           // [warp][stage][x, gy, gadd][vector][lane]
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  uint4* ring = norm_ring + warp * (NORM_BWD_STAGES * 3 * VPL * 32) + lane;
+  const int step = gridDim.x * NORM_BWD_WARPS;
+  auto fetch = [&](int row, int stage) {
+    if (row < rows) {
+      const size_t base = static_cast<size_t>(row) * H;
+#pragma unroll
+      for (int i = 0; i < VPL; ++i) {
+        const int c = (i * 32 + lane) * 8;
+        if (TAIL && c >= H) continue;
+        uint4* at = ring + (stage * 3 * VPL + i) * 32;
+        cp_async_16(at, x + base + c);
+        cp_async_16(at + VPL * 32, gy + base + c);
+        if (gadd != nullptr) cp_async_16(at + 2 * VPL * 32, gadd + base + c);
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
   float dg[VPL][8], db[VPL][8];
+  [[maybe_unused]] float sa[SUMS ? VPL : 1][8], so[SUMS ? VPL : 1][8];
 #pragma unroll
   for (int i = 0; i < VPL; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) dg[i][j] = db[i][j] = 0.f;
-  // (γ is re-read from L1 in both passes instead of living in VPL x 8 registers)
+    for (int j = 0; j < 8; ++j) {
+      dg[i][j] = db[i][j] = 0.f;
+      if constexpr (SUMS) sa[i][j] = so[i][j] = 0.f;
+    }
   auto unpack8 = [](const uint4& q, float (&v)[8]) {
     const float2 a = unpack_bf16(q.x), b = unpack_bf16(q.y), c = unpack_bf16(q.z), d = unpack_bf16(q.w);
     v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = c.x; v[5] = c.y; v[6] = d.x; v[7] = d.y;
   };
 
-  for (int row = blockIdx.x * NORM_BWD_WARPS + warp; row < rows; row += gridDim.x * NORM_BWD_WARPS) {
-    const size_t base = static_cast<size_t>(row) * H;
-    uint4 xq[VPL], gq[VPL], aq[VPL];
+  int row = blockIdx.x * NORM_BWD_WARPS + warp, stage = 0;
 #pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-      const bool ok = !TAIL || (i * 32 + lane) * 8 < H;
-      xq[i] = ok ? *reinterpret_cast<const uint4*>(x + base + (i * 32 + lane) * 8) : make_uint4(0, 0, 0, 0);
-      gq[i] = ok ? *reinterpret_cast<const uint4*>(gy + base + (i * 32 + lane) * 8) : make_uint4(0, 0, 0, 0);
+  for (int k = 0; k < NORM_BWD_STAGES - 1; ++k) fetch(row + k * step, k);
+  float mean_next = 0.f, rstd_next = 0.f;
+  auto stats = [&](int r) {
+    if (r < rows) {
+      mean_next = RMS ? 0.f : mean_in[r];
+      rstd_next = rstd_in[r];
     }
-    if (gadd != nullptr) {
-#pragma unroll
-      for (int i = 0; i < VPL; ++i)
-        aq[i] = (!TAIL || (i * 32 + lane) * 8 < H) ? *reinterpret_cast<const uint4*>(gadd + base + (i * 32 + lane) * 8) : make_uint4(0, 0, 0, 0);
-    }
-    const float mean = RMS ? 0.f : mean_in[row];
-    const float rstd = rstd_in[row];
+  };
+  stats(row);
+  for (; row < rows; row += step) {
+    fetch(row + (NORM_BWD_STAGES - 1) * step, (stage + NORM_BWD_STAGES - 1) % NORM_BWD_STAGES);
+    const float mean = mean_next, rstd = rstd_next;
+    stats(row + step);
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(NORM_BWD_STAGES - 1) : "memory");
+    const uint4* at = ring + stage * 3 * VPL * 32;
     float s1 = 0.f, s2 = 0.f;
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
       if (TAIL && (i * 32 + lane) * 8 >= H) continue;
       float xv[8], gv[8], gm[8];
-      unpack8(xq[i], xv);
-      unpack8(gq[i], gv);
-      Vec8<W>::load(gamma + (i * 32 + lane) * 8, gm);
+      unpack8(at[i * 32], xv);
+      unpack8(at[(VPL + i) * 32], gv);
+      Vec8<W>::load(gamma + (i * 32 + lane) * 8, gm);      // (from L1 in both passes instead of VPL x 8 registers)
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const float xh = (xv[j] - mean) * rstd;
@@ -243,12 +268,13 @@ norm_bwd_bf16_kernel(const __nv_bfloat16* __restrict__ gy, const __nv_bfloat16* 
     }
     s1 = RMS ? 0.f : warp_sum(s1) * inv_h;
     s2 = warp_sum(s2) * inv_h;
+    const size_t base = static_cast<size_t>(row) * H;
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
       if (TAIL && (i * 32 + lane) * 8 >= H) continue;
       float xv[8], gv[8], gm[8], o[8];
-      unpack8(xq[i], xv);
-      unpack8(gq[i], gv);
+      unpack8(at[i * 32], xv);
+      unpack8(at[(VPL + i) * 32], gv);
       Vec8<W>::load(gamma + (i * 32 + lane) * 8, gm);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
@@ -257,33 +283,66 @@ norm_bwd_bf16_kernel(const __nv_bfloat16* __restrict__ gy, const __nv_bfloat16* 
       }
       if (gadd != nullptr) {  // the skip connection's gradient rides along: saves autograd's separate add kernel
         float a[8];
-        unpack8(aq[i], a);
+        unpack8(at[(2 * VPL + i) * 32], a);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] += a[j];
-      }
-      Vec8<__nv_bfloat16>::store(gx + base + (i * 32 + lane) * 8, o);
-    }
-  }
-  // block-level reduction of the per-warp column partials, one vector slot at a time
-  for (int i = 0; i < VPL; ++i) {
-    for (int which = 0; which < (part_dbeta != nullptr ? 2 : 1); ++which) {
-      __syncthreads();
-#pragma unroll
-      for (int j = 0; j < 8; ++j) red[warp][lane * 8 + j] = which == 0 ? dg[i][j] : db[i][j];
-      __syncthreads();
-      for (int c = threadIdx.x; c < 256; c += NORM_BWD_WARPS * 32) {
-        float acc = 0.f;
-        if (TAIL && i * 256 + c >= H) continue;
-#pragma unroll
-        for (int w = 0; w < NORM_BWD_WARPS; ++w) acc += red[w][c];
-        if (acc_dgamma != nullptr) {
-          // accumulate mode (training: dγ/dβ live in the fp32 main_grad buffer): one red.add per block and column
-          // straight into the gradient instead of a [blocks, H] partial matrix + a second reduction kernel
-          atomicAdd((which == 0 ? acc_dgamma : acc_dbeta) + i * 256 + c, acc);
-        } else {
-          float* dst = (which == 0 ? part_dgamma : part_dbeta) + static_cast<size_t>(blockIdx.x) * H + i * 256 + c;
-          *dst = acc;
+        for (int j = 0; j < 8; ++j) {
+          o[j] += a[j];
+          if constexpr (SUMS) sa[i][j] += a[j];
         }
+      }
+      const uint4 q = make_uint4(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]), pack_bf16(o[4], o[5]), pack_bf16(o[6], o[7]));
+      *reinterpret_cast<uint4*>(gx + base + (i * 32 + lane) * 8) = q;
+      if constexpr (SUMS) {                      // (of the bf16 numbers that the next layer gets)
+        unpack8(q, o);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) so[i][j] += o[j];
+      }
+    }
+    stage = stage + 1 == NORM_BWD_STAGES ? 0 : stage + 1;
+  }
+  // the block's column sums, over the ring
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+  __syncthreads();
+  float* sums = reinterpret_cast<float*>(norm_ring);       // [which][warp][column]
+  auto put = [&](int which, const float (*v)[8]) {
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) {
+      float* to = sums + ((which * NORM_BWD_WARPS + warp) * VPL + i) * 256 + lane * 8;
+      *reinterpret_cast<float4*>(to) = make_float4(v[i][0], v[i][1], v[i][2], v[i][3]);
+      *reinterpret_cast<float4*>(to + 4) = make_float4(v[i][4], v[i][5], v[i][6], v[i][7]);
+    }
+  };
+  put(0, dg);
+  put(1, db);
+  if constexpr (SUMS) {
+    put(2, sa);
+    put(3, so);
+  }
+  __syncthreads();
+  for (int which = 0; which < (SUMS ? 4 : 2); ++which) {
+    float* part = which == 0 ? part_dgamma : part_dbeta;
+    // accumulate mode (training: the parameters' fp32 main_grad buffers): straight into the gradients instead of a [blocks, H] matrix of partial
+    // sums and a second reduction kernel
+    float* acc = which == 0 ? acc_dgamma : which == 1 ? acc_dbeta : which == 2 ? sum_add : sum_out;
+    const bool add = which >= 2 || acc_dgamma != nullptr;
+    if (add ? acc == nullptr : part == nullptr) continue;
+    for (int c = threadIdx.x * 4; c < H; c += NORM_BWD_WARPS * 128) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int w = 0; w < NORM_BWD_WARPS; ++w) {
+        const float4 u = *reinterpret_cast<const float4*>(sums + (which * NORM_BWD_WARPS + w) * VPL * 256 + c);
+        v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+      }
+      float* dst = add ? acc + c : part + static_cast<size_t>(blockIdx.x) * H + c;
+      if (add && (reinterpret_cast<uintptr_t>(acc) & 15) == 0) {
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"l"(dst), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+      } else if (add) {
+        atomicAdd(dst, v.x);
+        atomicAdd(dst + 1, v.y);
+        atomicAdd(dst + 2, v.z);
+        atomicAdd(dst + 3, v.w);
+      } else {
+        *reinterpret_cast<float4*>(dst) = v;
       }
     }
   }
@@ -574,8 +633,12 @@ int norm_grid_of(int rows, int rows_per_block, int blocks_per_sm) {
 int norm_grid(int rows) { return norm_grid_of(rows, lb::NORM_WARPS, 2); }
 // forward: 64 registers → four 8-warp blocks per SM
 int norm_fwd_grid(int rows) { return norm_grid_of(rows, lb::NORM_WARPS, 4); }
-// bf16 backward: three 4-warp blocks per SM (one wave; every block leaves one row of column partials)
-int norm_bwd_bf16_grid(int rows) { return norm_grid_of(rows, lb::NORM_BWD_WARPS, 3); }
+// bf16 backward: up to three 4-warp blocks per SM (one wave), but no more than give every warp up to three rows once there is a block per SM: every block adds or leaves
+// a row of column sums, which took longer than the rows ([1812, 256] 453 blocks 5.3 us, 151 blocks 3.3; [2048, 384] 6.2 and 5.1; [200, 384] 50 blocks 2.8, 17 blocks 4.2).
+int norm_bwd_bf16_grid(int rows, int H, bool sums) {
+  const int per_sm = lb::NORM_BWD_WARPS * norm_sms(), want = (rows + per_sm - 1) / per_sm, each = want < lb::NORM_BWD_STAGES ? want : lb::NORM_BWD_STAGES;
+  return norm_grid_of(rows, lb::NORM_BWD_WARPS * each, lb::norm_bwd_blocks((H + 255) / 256, sums));
+}
 // wide rows: blocks loop over rows; the backward keeps to one wave, and to as few blocks as do it in the same number of rounds, because
 // every block leaves a row of column sums at the end
 int norm_fwd_wide_grid(int rows) { return norm_grid_of(rows, 1, 6); }
@@ -664,19 +727,32 @@ void fwd_dispatch_bf16(int H, const __nv_bfloat16* x, const W* g, const W* b, __
 #undef LB_CASE
 }
 
+template <typename W, int V, bool RMS, bool TAIL, bool SUMS, typename... A>
+void launch_norm_bwd(int grid, cudaStream_t s, const A&... args) {
+  auto kern = lb::norm_bwd_bf16_kernel<W, V, RMS, TAIL, SUMS>;
+  constexpr int smem = lb::NORM_BWD_WARPS * lb::NORM_BWD_STAGES * 3 * V * 512;
+  static_assert(smem >= 4 * lb::NORM_BWD_WARPS * V * 1024, "column sums fit the ring");
+  if (smem > 48 * 1024) {                        // the limit is per device
+    static std::atomic<unsigned long long> done{0};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+    if (!(done.load(std::memory_order_relaxed) & bit) && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess)
+      done.fetch_or(bit, std::memory_order_relaxed);
+  }
+  kern<<<grid, lb::NORM_BWD_WARPS * 32, smem, s>>>(args...);
+}
+
 template <typename W, bool RMS>
 void bwd_dispatch_bf16(int H, const __nv_bfloat16* gy, const __nv_bfloat16* x, const W* g, const float* mean, const float* rstd,
                        __nv_bfloat16* gx, float* pdg, float* pdb, int rows, int grid, cudaStream_t s, const __nv_bfloat16* gadd,
                        float* acc_dg, float* acc_db) {
   if (H <= NORM_WARP_MAX_H) {
-#define LB_CASE(V)                                                                                                                 \
-  case V:                                                                                                                          \
-    if (H % 256 == 0)                                                                                                             \
-      lb::norm_bwd_bf16_kernel<W, V, RMS, false><<<grid, lb::NORM_BWD_WARPS * 32, 0, s>>>(gy, x, g, mean, rstd, gx, pdg, pdb, rows, \
-                                                                                          gadd, acc_dg, acc_db, H);               \
-    else                                                                                                                          \
-      lb::norm_bwd_bf16_kernel<W, V, RMS, true><<<grid, lb::NORM_BWD_WARPS * 32, 0, s>>>(gy, x, g, mean, rstd, gx, pdg, pdb, rows,  \
-                                                                                         gadd, acc_dg, acc_db, H);                \
+    float* none = nullptr;
+#define LB_CASE(V)                                                                                                                                    \
+  case V:                                                                                                                                             \
+    if (H % 256 == 0) launch_norm_bwd<W, V, RMS, false, false>(grid, s, gy, x, g, mean, rstd, gx, pdg, pdb, rows, gadd, acc_dg, acc_db, none, none, H); \
+    else launch_norm_bwd<W, V, RMS, true, false>(grid, s, gy, x, g, mean, rstd, gx, pdg, pdb, rows, gadd, acc_dg, acc_db, none, none, H);              \
     break;
     switch ((H + 255) / 256) { LB_CASE(1) LB_CASE(2) LB_CASE(3) LB_CASE(4) }
 #undef LB_CASE
@@ -767,7 +843,7 @@ extern "C" int lb_norm_fwd(const void* x, const void* gamma, const void* beta, v
 
 // workspace: float[2 * grid_cap * H] where grid_cap = lb_norm_bwd_workspace_rows(); dgamma/dbeta fp32 [H]
 extern "C" int lb_norm_bwd_workspace_rows(int rows, int H) {
-  const int a = norm_grid(rows), b = norm_bwd_bf16_grid(rows), c = norm_bwd_wide_grid(rows, H);
+  const int a = norm_grid(rows), b = norm_bwd_bf16_grid(rows, H, false), c = norm_bwd_wide_grid(rows, H);
   return a > b ? (a > c ? a : c) : (b > c ? b : c);
 }
 // the fused "+ residual gradient" is implemented by the register-cached kernels only: bf16 rows of whole aligned vectors, fp32
@@ -791,7 +867,7 @@ extern "C" int lb_norm_bwd(const void* gy, const void* x, const void* gamma, con
       else norm_bwd_any<B, float>(gy, x, gamma, mean, rstd, gx, dgamma, dbeta, rows, H, rms, accumulate, s);
       return (int)cudaGetLastError();
     }
-    const int grid = H <= NORM_WARP_MAX_H ? norm_bwd_bf16_grid(rows) : norm_bwd_by_warp(rows, H) ? norm_grid(rows) : norm_bwd_wide_grid(rows, H);
+    const int grid = H <= NORM_WARP_MAX_H ? norm_bwd_bf16_grid(rows, H, false) : norm_bwd_by_warp(rows, H) ? norm_grid(rows) : norm_bwd_wide_grid(rows, H);
     float* pdg = workspace;
     float* pdb = dbeta != nullptr ? workspace + static_cast<size_t>(grid) * H : nullptr;
     // accumulate mode: the warp kernel's blocks add their column sums straight into dgamma / dbeta
@@ -819,5 +895,30 @@ extern "C" int lb_norm_bwd(const void* gy, const void* x, const void* gamma, con
   } else {
     return -1;
   }
+  return (int)cudaGetLastError();
+}
+
+// Layer norm backward on bf16 rows of up to 1024 columns that adds into fp32 gradients and, beside them, the column sums of gadd into sum_add and those of gx into sum_out
+// (either may be nullptr): the gradients of the biases around the norm.  -3: not of this form.
+extern "C" int lb_norm_bwd_sums(const void* gy, const void* x, const void* gamma, const float* mean, const float* rstd, void* gx, float* dgamma, float* dbeta, int rows,
+                                int H, const void* gadd, float* sum_add, float* sum_out, cudaStream_t s) {
+  using B = __nv_bfloat16;
+  if (H > NORM_WARP_MAX_H || !norm_vec_bf16(H, 0) || gadd == nullptr || dgamma == nullptr || dbeta == nullptr ||
+      !lb_norm_bwd_supports_gadd(H, 0, gy, x, gamma, gx, gadd))
+    return -3;
+  if (rows == 0) return 0;
+  const int grid = norm_bwd_bf16_grid(rows, H, true);
+  float* none = nullptr;
+#define LB_CASE(V)                                                                                                                                                     \
+  case V:                                                                                                                                                              \
+    if (H % 256 == 0)                                                                                                                                                  \
+      launch_norm_bwd<B, V, false, false, true>(grid, s, (const B*)gy, (const B*)x, (const B*)gamma, mean, rstd, (B*)gx, none, none, rows, (const B*)gadd, dgamma, dbeta, \
+                                                sum_add, sum_out, H);                                                                                                  \
+    else                                                                                                                                                               \
+      launch_norm_bwd<B, V, false, true, true>(grid, s, (const B*)gy, (const B*)x, (const B*)gamma, mean, rstd, (B*)gx, none, none, rows, (const B*)gadd, dgamma, dbeta, \
+                                               sum_add, sum_out, H);                                                                                                   \
+    break;
+  switch ((H + 255) / 256) { LB_CASE(1) LB_CASE(2) LB_CASE(3) LB_CASE(4) }
+#undef LB_CASE
   return (int)cudaGetLastError();
 }

@@ -20,6 +20,8 @@ std::tuple<Tensor, Tensor, Tensor> norm_fwd(const Tensor& x, const Tensor& gamma
 std::tuple<Tensor, Tensor, Tensor> norm_bwd(const Tensor& gy, const Tensor& x, const Tensor& gamma, const Tensor& mean, const Tensor& rstd, bool rms,
                                             bool has_bias, const c10::optional<Tensor>& dgamma_accum, const c10::optional<Tensor>& dbeta_accum,
                                             const c10::optional<Tensor>& gadd);
+Tensor norm_bwd_sums(const Tensor& gy, const Tensor& x, const Tensor& gamma, const Tensor& mean, const Tensor& rstd, const Tensor& dgamma, const Tensor& dbeta,
+                     const Tensor& gadd, const Tensor& sum_add, const Tensor& sum_out);
 Tensor swiglu_packed_fwd(const Tensor& gu);
 Tensor swiglu_packed_bwd(const Tensor& gy, const Tensor& gu);
 Tensor rope_qkv(const Tensor& qkv, const Tensor& cosv, const Tensor& sinv, int64_t pos_offset, bool backward, bool inplace);

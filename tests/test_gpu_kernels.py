@@ -1275,3 +1275,31 @@ def test_linear_of_few_rows_behind_a_norm(n, k, m, rms):
     want = d.to(BF16).double() @ w.double().t() + bias.double()
     # the normalised rows are rounded to bf16 once (some a step off, where 32 and 64 bits round apart), the result once
     assert float((y[:m].double() - want).norm()) < 2.0 ** -8 * float(want.norm()) and bool((y[m] == 7).all())
+
+
+@pytest.mark.parametrize("which", ["both", "before", "behind"])
+@pytest.mark.parametrize("rows", [1, 5, 131, 600, 1900])
+@pytest.mark.parametrize("h", [8, 264, 768, 1000, 1024])
+def test_norm_backward_with_the_biases_around_it(h, rows, which):
+    """Every width of vectors per lane, rows of a warp from none to several, results added to what the buffers hold; result and column sums against float64."""
+    gy, x, gadd, gamma = _rand((rows, h), 1), _rand((rows, h), 2) + 3, _rand((rows, h), 3), 1 + 0.1 * _rand((h,), 4)
+    ext = load_ext()
+    _, mean, rstd = ext.norm_fwd(x, gamma, torch.zeros_like(gamma), 1e-5, False)
+    sums = [_rand((h,), 5 + i, dtype=torch.float32) for i in range(4)]
+    old = [t.double() for t in sums]
+    gx = torch.full((rows + 1, h), 7.0, device="cuda", dtype=BF16)
+    ptr = lambda t: ctypes.c_void_p(0 if t is None else t.data_ptr())
+    rc = ctypes.CDLL(so_path()).lb_norm_bwd_sums(ptr(gy), ptr(x), ptr(gamma), ptr(mean), ptr(rstd), ptr(gx), ptr(sums[0]), ptr(sums[1]), rows, h, ptr(gadd),
+                                                 ptr(sums[2] if which != "before" else None), ptr(sums[3] if which != "behind" else None),
+                                                 ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    x64 = x.double().requires_grad_(True)
+    g64, b64 = gamma.double().requires_grad_(True), torch.zeros(h, device="cuda", dtype=torch.float64, requires_grad=True)
+    torch.nn.functional.layer_norm(x64, (h,), g64, b64, 1e-5).backward(gy.double())
+    want = x64.grad + gadd.double()
+    assert float((gx[:rows].double() - want).norm()) < 2.0 ** -8 * float(want.norm()) + 1e-6 and bool((gx[rows] == 7).all())
+    for got, was, d, n in ((sums[0], old[0], g64.grad, gy.double().abs().sum(0) * 4), (sums[1], old[1], b64.grad, gy.double().abs().sum(0)),
+                           (sums[2], old[2], gadd.double().sum(0) * (which != "before"), gadd.double().abs().sum(0)),
+                           (sums[3], old[3], gx[:rows].double().sum(0) * (which != "behind"), gx[:rows].double().abs().sum(0))):
+        # fp32 sums: a rounding of 2^-24 of the magnitudes per term of a chain of at most rows / 4, and of the normalised x (2^-20)
+        assert bool(((got.double() - was - d).abs() <= (2.0 ** -20 + rows * 2.0 ** -26) * (n + was.abs() + 1)).all())
