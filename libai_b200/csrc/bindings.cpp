@@ -84,6 +84,7 @@ int lb_masked_attention_tc(const void* q, long ldq, const void* kmat, const void
                            const void* gate, long ldg, int gate_wide, const int* qt_seq, const int* qt_start, int ntiles,
                            const int* seq_off, const int* past, void* y, long ldy, long tokens, long rows, int H, int G, int D, int V,
                            int window, int chunk, float scale, float out_scale, float temp_coef, float temp_every, int* err, cudaStream_t s);
+int lb_gemm_multi(const void* x, const void* const* w, const int* n, int count, void* out, int M, int K, int ldx, int ldo, cudaStream_t stream);
 int lb_norm_bwd_sums(const void* gy, const void* x, const void* gamma, const float* mean, const float* rstd, void* gx, float* dgamma, float* dbeta, int rows, int H,
                      const void* gadd, float* sum_add, float* sum_out, cudaStream_t s);
 int lb_gemm_small_norm(const void* x, const void* gamma, const void* beta, float eps, int rms, const void* w, void* out, int M, int N, int K, int ldx, int ldw,
@@ -319,6 +320,26 @@ Tensor dgrad_actgrad(const Tensor& gy, const Tensor& w, const Tensor& pre, int64
                              (int)w.stride(0), (int)N, 1, (int)act, pre.data_ptr(), colsum, cur_stream()),
         "dgrad_actgrad");
   return out;
+}
+
+// x [M, K] against several matrices [n_i, K] in one launch -> [M, Σ n_i]; undefined (an empty list): not of that form
+std::vector<Tensor> gemm_multi(const Tensor& x, const std::vector<Tensor>& w) {
+  if (!x.is_cuda() || x.dim() != 2 || x.scalar_type() != at::kBFloat16 || x.stride(1) != 1 || x.size(0) == 0 || w.empty() || w.size() > 8) return {};
+  const void* ptr[8];
+  int n[8], count = 0, total = 0;
+  for (const Tensor& t : w) {
+    if (t.dim() != 2 || t.scalar_type() != at::kBFloat16 || t.device() != x.device() || !t.is_contiguous() || t.size(1) != x.size(1)) return {};
+    ptr[count] = t.data_ptr();
+    n[count++] = (int)t.size(0);
+    total += (int)t.size(0);
+  }
+  c10::cuda::CUDAGuard guard(x.device());
+  if (total % 8) return {};
+  Tensor out = at::empty({x.size(0), total}, x.options());
+  const int rc = lb_gemm_multi(x.data_ptr(), ptr, n, count, out.data_ptr(), (int)x.size(0), (int)x.size(1), (int)x.stride(0), total, cur_stream());
+  if (rc < 0) return {};                                   // refused before anything ran
+  check(rc, "gemm_multi");
+  return {out};
 }
 
 // The GEMM's epilogue loads a residual in vectors of 16 bytes; a block's input may be a view that begins anywhere.
@@ -1303,6 +1324,7 @@ TORCH_LIBRARY(libai_b200, m) {
   m.def("gemm_grouped_blocks(Tensor a, Tensor w, Tensor tile_group, Tensor(a!) out) -> ()", &gemm_grouped_blocks);
   m.def("masked_attention_tc(Tensor q, Tensor kmat, Tensor vmat, Tensor ext_off, Tensor nsink, Tensor cstart, Tensor? gate, bool gate_wide, Tensor seq_off, Tensor past, Tensor qt_seq, Tensor qt_start, Tensor(a!) y, int H, int G, int D, int V, int window, int chunk, float scale, float out_scale, float temp_coef, float temp_every) -> ()", &masked_attention_tc);
   m.def("latent_prompt_tc(Tensor q, Tensor kv, Tensor rot, Tensor cs, Tensor? sink, Tensor ext_off, Tensor seq_off, Tensor past, Tensor qt_seq, Tensor qt_start, Tensor(a!) y, int H, int D, int R, int V, float scale) -> ()", &latent_prompt_tc);
+  m.def("gemm_multi(Tensor x, Tensor[] w) -> Tensor[]", &gemm_multi);
   m.def("linear_bias_residual(Tensor x, Tensor w, Tensor? bias, Tensor residual) -> Tensor", &linear_bias_residual);
   m.def("block_fwd(Tensor x, Tensor[] params, int heads, float eps1, float eps2, float scale, bool causal, Tensor? past_k, Tensor? past_v) -> Tensor[]", &block_fwd);
   m.def("llama_block_fwd(Tensor x, Tensor[] params, Tensor? bias, Tensor cos, Tensor sin, int heads, float eps1, float eps2, float scale, bool joint, Tensor? past_k, Tensor? past_v) -> Tensor[]", &llama_block_fwd);

@@ -191,12 +191,24 @@ LB_DEVICE void stg_store_chunk(uint8_t* stg, int lane, const float (&v)[32], __n
   }
 }
 
+// MULTI: B is several matrices [n[i], K] in memory of their own, one after the other along the columns of the output (NT, CTA pairs, bf16 results)
+constexpr int GEMM_MAX_B = 8;
+struct GemmMultiB {
+  CUtensorMap map[GEMM_MAX_B];
+  int count;
+  int n[GEMM_MAX_B], first[GEMM_MAX_B + 1], col[GEMM_MAX_B];   // columns; first tile along N; first column of the output
+};
+struct GemmOneB {};
+template <bool MULTI> struct GemmB { using type = GemmOneB; };
+template <> struct GemmB<true> { using type = GemmMultiB; };
+
 // CTAS == 2: `cta_group::2` — clusters of two CTAs (one TPC) compute 256 x BLOCK_N tiles; no fused collectives, bf16 only.
-template <int BLOCK_N, bool A_MN, bool B_MN, int EPI, bool FP8 = false, int CTAS = 1>
+template <int BLOCK_N, bool A_MN, bool B_MN, int EPI, bool FP8 = false, int CTAS = 1, bool MULTI = false>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
             const __grid_constant__ CUtensorMap tmap_g /* COMM_AG: the local shard of the gathered operand */,
-            const __grid_constant__ CUtensorMap tmap_o /* EPI_ATOMIC_F32: the output in boxes of 32 x 32 */, GemmParams p, CommParams cp) {
+            const __grid_constant__ CUtensorMap tmap_o /* EPI_ATOMIC_F32: the output in boxes of 32 x 32 */, GemmParams p, CommParams cp,
+            const __grid_constant__ typename GemmB<MULTI>::type mb) {
   using Cfg = StageCfg<BLOCK_N, CTAS, EPI == EPI_ATOMIC_F32, B_MN>;
   constexpr int NS = Cfg::NUM_STAGES;
   static_assert(CTAS == 1 || (CTAS == 2 && BLOCK_N >= 128 && !FP8), "CTA-pair mode: bf16 tiles of 128 columns and more");
@@ -215,7 +227,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 
   // (CTA pair: `m_blocks` counts 256-row blocks = one per pair; this CTA works on rows [256 m + 128 rank, +128))
   const int m_blocks = (p.M + BLOCK_M * CTAS - 1) / (BLOCK_M * CTAS);
-  const int n_blocks = (p.N + BLOCK_N - 1) / BLOCK_N;
+  static_assert(!MULTI || (CTAS == 2 && !A_MN && !B_MN && EPI == EPI_BF16), "several B: NT products on CTA pairs, bf16 results");
+  int n_blocks = (p.N + BLOCK_N - 1) / BLOCK_N;
+  if constexpr (MULTI) n_blocks = mb.first[mb.count];
+  [[maybe_unused]] auto segment = [&](int n_blk) {          // MULTI: which matrix a column tile belongs to
+    int i = 0;
+    if constexpr (MULTI)
+      while (n_blk >= mb.first[i + 1]) ++i;
+    return i;
+  };
   const int k_blocks_total = (p.K + BLOCK_K - 1) / BLOCK_K;
   const int num_tiles = m_blocks * n_blocks * p.k_splits;
   // CTAs [0, n_comm) are copy CTAs in COMM_AG mode; the rest run the GEMM roles
@@ -259,7 +279,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmap_a);
-    tma_prefetch_desc(&tmap_b);
+    if constexpr (MULTI) {
+      for (int i = 0; i < mb.count; ++i) tma_prefetch_desc(&mb.map[i]);
+    } else {
+      tma_prefetch_desc(&tmap_b);
+    }
     if (cp.mode == COMM_AG) tma_prefetch_desc(&tmap_g);
     if constexpr (EPI == EPI_ATOMIC_F32) tma_prefetch_desc(&tmap_o);
 #pragma unroll
@@ -423,7 +447,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         }
         const CUtensorMap* map_a = a_local ? &tmap_g : &tmap_a;
         const int m_row = a_local ? (m_blk - cp.rank * mbpr) * BLOCK_M : m_blk * BLOCK_M;
-        const int n_row = grp_row + n_blk * BLOCK_N + cta_rank * (BLOCK_N / CTAS);   // pair: this CTA's half of the B tile
+        int n_row = grp_row + n_blk * BLOCK_N + cta_rank * (BLOCK_N / CTAS);   // pair: this CTA's half of the B tile
+        const CUtensorMap* map_nt = &tmap_b;
+        if constexpr (MULTI) {
+          const int seg = segment(n_blk);
+          map_nt = &mb.map[seg];
+          n_row -= mb.first[seg] * BLOCK_N;
+        }
         const int kb0 = split * p.k_per_split;
         const int kb1 = min(kb0 + p.k_per_split, k_blocks_total);
         for (int kb = kb0; kb < kb1; ++kb) {
@@ -456,7 +486,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
                 tma_load_2d_2cta(sa + a * (BLOCK_K * 128), &tmap_a, &full_bar[stage], m_row + a * 64, kb * BLOCK_K);
             }
             if constexpr (!B_MN) {
-              tma_load_2d_2cta(sb, &tmap_b, &full_bar[stage], kb * BLOCK_K, n_row);
+              tma_load_2d_2cta(sb, map_nt, &full_bar[stage], kb * BLOCK_K, n_row);
             } else {
 #pragma unroll
               for (int a = 0; a < Cfg::B_COLS / 64; ++a)
@@ -573,10 +603,16 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       const int row = m_blk * BLOCK_M + quad * 32 + lane;
       const bool row_ok = row < p.M;
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BLOCK_N;
+      int tile_col = n_blk * BLOCK_N, tile_cols = p.N - tile_col;        // first column of the tile in the output, columns that there are from there
+      if constexpr (MULTI) {
+        const int seg = segment(n_blk), local = (n_blk - mb.first[seg]) * BLOCK_N;
+        tile_col = mb.col[seg] + local;
+        tile_cols = mb.n[seg] - local;
+      }
 #pragma unroll 1
       for (int c = half * CHUNKS_PER_HALF; c < (half + 1) * CHUNKS_PER_HALF; ++c) {
-        const int col0 = n_blk * BLOCK_N + c * 32;
-        if (col0 >= p.N) break;  // warp-uniform
+        const int col0 = tile_col + c * 32;
+        if (c * 32 >= tile_cols) break;  // warp-uniform
         uint32_t r[32];
         tmem_ld_32x32b_x32(t_row + c * 32, r);
         if constexpr (EPI == EPI_BF16) {
@@ -586,7 +622,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           uint8_t* stg = staging + (warp_idx - 2) * 2048;
           const int slab_row0 = m_blk * BLOCK_M + quad * 32;
           const int rows_valid = p.M - slab_row0;  // <= 0: nothing of this slab exists
-          const int cols_valid = p.N - col0;       // > 0, multiple of 8 (enforced on the host)
+          const int cols_valid = tile_cols - c * 32;   // > 0, multiple of 8 (enforced on the host)
           const int sub = lane & 3, rsel = lane >> 2;
           const bool use_bias = p.bias != nullptr && cp.mode != COMM_RS;  // RS: bias added once, in the reduce phase
           const bool use_pre = p.pre_in != nullptr;
@@ -955,7 +991,7 @@ cudaError_t launch_2cta(const CUtensorMap& ta, const CUtensorMap& tb, const CUte
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  if (chained(p, cp)) return lb_host::launch_chained(kern, dim3((unsigned)grid), dim3(lb::NUM_THREADS), Cfg::SMEM_BYTES, stream, 2, ta, tb, tg, to, p, cp);
+  if (chained(p, cp)) return lb_host::launch_chained(kern, dim3((unsigned)grid), dim3(lb::NUM_THREADS), Cfg::SMEM_BYTES, stream, 2, ta, tb, tg, to, p, cp, lb::GemmOneB{});
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3(lb::NUM_THREADS);
@@ -968,7 +1004,7 @@ cudaError_t launch_2cta(const CUtensorMap& ta, const CUtensorMap& tb, const CUte
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, ta, tb, tg, to, p, cp);
+  return cudaLaunchKernelEx(&cfg, kern, ta, tb, tg, to, p, cp, lb::GemmOneB{});
 }
 
 template <int BN, bool AMN, bool BMN, int EPI, bool FP8 = false>
@@ -982,8 +1018,8 @@ cudaError_t launch_cfg(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  if (chained(p, cp)) return lb_host::launch_chained(kern, dim3((unsigned)grid), dim3(lb::NUM_THREADS), Cfg::SMEM_BYTES, stream, 0, ta, tb, tg, to, p, cp);
-  kern<<<grid, lb::NUM_THREADS, Cfg::SMEM_BYTES, stream>>>(ta, tb, tg, to, p, cp);
+  if (chained(p, cp)) return lb_host::launch_chained(kern, dim3((unsigned)grid), dim3(lb::NUM_THREADS), Cfg::SMEM_BYTES, stream, 0, ta, tb, tg, to, p, cp, lb::GemmOneB{});
+  kern<<<grid, lb::NUM_THREADS, Cfg::SMEM_BYTES, stream>>>(ta, tb, tg, to, p, cp, lb::GemmOneB{});
   return cudaGetLastError();
 }
 
@@ -1328,6 +1364,75 @@ static int gemm_impl(const void* a, const void* b, void* out, int M, int N, int 
     else e = launch_bn<true, true, lb::EPI_ATOMIC_F32>(bn, ta, tb, tg, to, p, cp, grid, stream);
   }
   return (int)e;
+}
+
+template <int BN>
+static cudaError_t launch_multi(const CUtensorMap& ta, const lb::GemmParams& p, const lb::GemmMultiB& mb, int grid, cudaStream_t stream) {
+  using Cfg = lb::StageCfg<BN, 2, false, false>;
+  auto kern = lb::gemm_kernel<BN, false, false, lb::EPI_BF16, false, 2, true>;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
+    if (e != cudaSuccess) return e;
+    configured = true;
+  }
+  lb::CommParams cp;
+  memset(&cp, 0, sizeof(cp));
+  return lb_host::launch_chained(kern, dim3((unsigned)grid), dim3(lb::NUM_THREADS), Cfg::SMEM_BYTES, stream, 2, ta, ta, ta, ta, p, cp, mb);
+}
+// x [M, K] against `count` matrices w[i] [n[i], K] at once: out [M, ldo], the results one after the other.  One launch and one last wave in place of a launch each, and
+// the first of them put together by a copy: a mixer's projections (1024 + 1024 + 2048, 16, 16 and 2048 columns, K = 2048) of 1600 rows 68.4 -> 37.9 us, 300 rows 46.1 -> 15.2,
+// 16 rows 30.8 -> 16.3, 1 row 28.8 -> 21.0, 8192 rows 171.7 -> 144.9; K = 1024 with half the columns, 1 row 18.5 -> 9.9 and 8192 rows 72.1 -> 43.9.  Bounded by the tensor
+// cores from some 1000 rows (1600 rows: 1.07 PFLOP/s), below by the chain of k-blocks of one tile.  A matrix's last tile is not shared with the next one's first: a tile of its
+// own for 16 columns costs less than moving the matrix.  -1: not of a form that this takes.
+extern "C" int lb_gemm_multi(const void* x, const void* const* w, const int* n, int count, void* out, int M, int K, int ldx, int ldo, cudaStream_t stream) {
+  if (M <= 0 || K <= 0 || count < 1 || count > lb::GEMM_MAX_B || !gemm_allow_2cta() || K % 8 || ldx % 8 || ldo % 8 ||
+      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15))
+    return -1;
+  int total = 0;
+  for (int i = 0; i < count; ++i) {
+    if (n[i] <= 0 || n[i] % 8 || (reinterpret_cast<uintptr_t>(w[i]) & 15)) return -1;
+    total += n[i];
+  }
+  if (total > ldo) return -1;
+  const int pairs = num_sms() / 2, kb = (K + lb::BLOCK_K - 1) / lb::BLOCK_K, m_blocks = (M + 2 * lb::BLOCK_M - 1) / (2 * lb::BLOCK_M);
+  int bn = 256;
+  double best = 1e30;
+  for (int i = 0; i < 3; ++i) {                  // the pair tiles of tile_choice
+    const TileKind& t = kTileKinds[0][i];
+    long tiles = 0;
+    for (int j = 0; j < count; ++j) tiles += (n[j] + t.bn - 1) / t.bn;
+    const long waves = (tiles * m_blocks + pairs - 1) / pairs;
+    if (t.bn < 256 && waves > 4) continue;
+    const double us = t.fixed + (double)waves * (t.wave + kb * t.block);
+    if (us < best - 1e-9) {
+      best = us;
+      bn = t.bn;
+    }
+  }
+  lb::GemmParams p{};
+  p.M = M;
+  p.N = total;
+  p.K = K;
+  p.k_splits = 1;
+  p.k_per_split = kb;
+  p.group_m = (long)total * K * 2 >= (48L << 20) ? (int)(std::sqrt(pairs * (bn / (2.0 * lb::BLOCK_M))) + 0.5) : 1;   // as for one matrix
+  p.out = out;
+  p.ldo = ldo;
+  lb::GemmMultiB mb{};
+  mb.count = count;
+  CUtensorMap ta;
+  if (!operand_tmap(&ta, x, false, M, K, ldx, lb::BLOCK_M)) return -2;
+  for (int i = 0, col = 0; i < count; ++i) {
+    if (!operand_tmap(&mb.map[i], w[i], false, n[i], K, K, bn / 2)) return -2;
+    mb.n[i] = n[i];
+    mb.col[i] = col;
+    mb.first[i + 1] = mb.first[i] + (n[i] + bn - 1) / bn;
+    col += n[i];
+  }
+  const long tiles = (long)m_blocks * mb.first[count];
+  const int grid = 2 * (int)(tiles < pairs ? tiles : pairs);
+  return (int)(bn == 256 ? launch_multi<256>(ta, p, mb, grid, stream) : bn == 192 ? launch_multi<192>(ta, p, mb, grid, stream) : launch_multi<128>(ta, p, mb, grid, stream));
 }
 
 extern "C" int lb_gemm_bf16(const void* a, const void* b, void* out, int M, int N, int K, int lda, int ldb, int ldo,

@@ -86,8 +86,18 @@ class GatedDeltaMixer(nn.Module):
             SF.gated_rmsnorm(o, SF.linear(parts["g1"], self.g2), self.norm, self.eps, SF.GATE_SIGMOID, y, self.heads, self.vdim)
         return y
 
+    def _projections(self, h):
+        """The products of :meth:`input_weights`, from one launch on the matrices as they are where it takes them."""
+        names = ("b", "a" if self.decay == "head" else "a1", "g" if self.gate == "silu" else "g1")
+        rest = [getattr(self, n) for n in names]
+        joint = SF.linears(h, [self.q, self.k, self.v, *rest])
+        if joint is None:
+            return {name: SF.linear(h, w) for name, w in self.input_weights()}
+        qkv = 2 * self.kv_heads * self.dim + self.heads * self.vdim
+        return dict(zip(("qkv", *names), joint.split([qkv, *(w.shape[0] for w in rest)], 1)))
+
     def forward(self, h, rb, bufs):
         """Unfused form: ``h`` ``[tokens, width]`` packed rows → ``[tokens, width]``."""
-        parts = {name: SF.linear(h, w) for name, w in self.input_weights()}
+        parts = self._projections(h)
         y = torch.empty(h.shape[0], self.mix_features, dtype=h.dtype, device=h.device)
         return SF.linear(self.mix(parts, rb, bufs, y), self.o)

@@ -255,6 +255,19 @@ def linear(a, w, bias=None):
     return F.linear(a, w, bias)
 
 
+def linears(a, ws):
+    """``cat(ws)`` applied to ``a`` in one launch that reads the matrices where they are: ``[rows, Σ n_i]``, or ``None`` where that launch does not take them (the
+    products of up to 128 rows are ahead one by one, in the kernel for few rows)."""
+    from . import load_ext, use_native
+
+    if a.is_cuda and a.dtype == torch.bfloat16 and use_native(a) and a.dim() == 2:
+        out = load_ext().gemm_multi(a, ws)
+        if out:
+            count_launch()
+            return out[0]
+    return None
+
+
 _GEMM_REFUSED = set()
 
 

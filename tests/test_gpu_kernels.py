@@ -1118,6 +1118,26 @@ def test_gemm_tiles_of_every_width(bn, layout, m, n, k):
     assert torch.equal(out[:, :n].float(), want + (3.0 if layout == 2 else 0.0)) and bool((out[:, n:] == 3).all())
 
 
+@pytest.mark.parametrize("m,k,ns", [(1, 64, [8]), (129, 128, [16, 8]), (300, 72, [136, 16, 264]), (2500, 264, [384, 384, 192, 24]), (2500, 520, [512, 512, 256, 16, 8]),
+                                    (1000, 128, [8, 256, 264, 120, 192, 200, 16, 1032]), (600, 4104, [6144, 16])])
+def test_products_with_several_matrices_in_one_launch(m, k, ns):
+    """Every width of tile, up to eight matrices that end inside a tile, several waves, bands of rows; nothing written behind the last column.  Whole numbers, exact in
+    every format."""
+    g = torch.Generator(device="cuda").manual_seed(m + k)
+    ints = lambda *s: (torch.rand(*s, generator=g, device="cuda") < 0.2).to(BF16) * torch.randint(-1, 2, s, generator=g, device="cuda").to(BF16)
+    a, ws = ints(m, k + 8)[:, 8:], [ints(n, k) for n in ns]
+    total = sum(ns)
+    out = torch.full((m, total + 8), 3.0, device="cuda", dtype=BF16)
+    lib = ctypes.CDLL(so_path())
+    ptrs, cols = (ctypes.c_void_p * len(ns))(*[w.data_ptr() for w in ws]), (ctypes.c_int * len(ns))(*ns)
+    rc = lib.lb_gemm_multi(ctypes.c_void_p(a.data_ptr()), ptrs, cols, len(ns), ctypes.c_void_p(out.data_ptr()), m, k, k + 8, total + 8,
+                           ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    want = a.float() @ torch.cat(ws).float().t()
+    assert want.abs().max() < 256
+    assert torch.equal(out[:, :total].float(), want) and bool((out[:, total:] == 3).all())
+
+
 def _train_block(kind, dim, with_main_grad):
     """A block, its call and its inputs: causal, right-padded, without a mask, T5 decoder, Llama."""
     from libai_b200.layers import TransformerLayer
