@@ -171,20 +171,29 @@ __global__ void short_conv_vec8_kernel(const __nv_bfloat16* __restrict__ in, lon
 
 // The same for strips of STRIP tokens: the weights and the taps - 1 inputs before a token stay in registers, so an input is read 1 + 3 / STRIP
 // times instead of four and the weights (64 bytes per 16 of the result) once per strip.  [2560, 4096]: 31 -> 20 us; what is left are the
-// sigmoids in IEEE arithmetic (180 of 250 instructions per 8 channels).  Strips of 8 21, with their inputs loaded ahead 24.
+// sigmoids in IEEE arithmetic (22 of 33 instructions per element; 42 % of the issue slots at [3027, 4096]).  There the strip's inputs ahead of the weights
+// where it lies inside one sequence, quotients in 32 bits and six blocks per SM took 26.0 -> 24.5 us, the chained launch 2 us more.
 constexpr int CONV_STRIP = 4;
 template <int TAPS>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, 6)
 short_conv_strip_kernel(const __nv_bfloat16* __restrict__ in, long ldi, const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ tail,
                         const int* __restrict__ tok_seq, const int* __restrict__ seq_off, const int* __restrict__ slots, const int* __restrict__ past,
                         __nv_bfloat16* __restrict__ out, long ldo, long tokens, int C) {
-  lb::chain_next();
   const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
   const int C8 = C >> 3;
-  const long tok0 = idx / C8 * CONV_STRIP;
+  const long strip = idx <= 0xffffffffL ? (unsigned)idx / (unsigned)C8 : idx / C8, tok0 = strip * CONV_STRIP;
+  const int c = (int)(idx - strip * C8) * 8;
+  lb::chain_wait(in, w, tail, tok_seq, seq_off, slots, past);
+  lb::chain_next();
   if (tok0 >= tokens) return;
-  const int c = (int)(idx % C8) * 8;
   float wf[TAPS][8];                         // tap j of channel c + i
+  uint4 x[TAPS - 1 + CONV_STRIP];            // the input j - (TAPS - 1) tokens behind the first
+  const int last = (int)(tokens - tok0 < CONV_STRIP ? tokens - tok0 : CONV_STRIP), b0 = tok_seq[tok0], t0 = (int)(tok0 - seq_off[b0]);
+  const bool inside = last == CONV_STRIP && t0 >= TAPS - 1 && tok_seq[tok0 + CONV_STRIP - 1] == b0;
+  if (inside) {                              // one sequence, and nothing from before the call: all loads at once
+#pragma unroll
+    for (int j = 0; j < TAPS - 1 + CONV_STRIP; ++j) x[j] = *reinterpret_cast<const uint4*>(in + (tok0 + j - (TAPS - 1)) * ldi + c);
+  }
   {
     uint4 raw[TAPS];
 #pragma unroll
@@ -195,41 +204,43 @@ short_conv_strip_kernel(const __nv_bfloat16* __restrict__ in, long ldi, const __
 #pragma unroll
       for (int i = 0; i < 8; ++i) wf[j][i] = __bfloat162float(wv[i * TAPS + j]);
   }
-  uint4 x[TAPS];                             // x[j]: the input under tap j
-  const int last = (int)(tokens - tok0 < CONV_STRIP ? tokens - tok0 : CONV_STRIP);
-#pragma unroll
-  for (int j = 0; j < CONV_STRIP; ++j) {
-    if (j >= last) break;
-    const long tok = tok0 + j;
-    const int b = tok_seq[tok], t = (int)(tok - seq_off[b]);
-    if (j == 0 || t == 0) {                  // the inputs before this one
-      const bool has_past = past[b] > 0;
-      const __nv_bfloat16* tl = tail + (long)slots[b] * (TAPS - 1) * C;
-#pragma unroll
-      for (int k = 1; k < TAPS; ++k) {
-        uint4 raw = make_uint4(0u, 0u, 0u, 0u);
-        if (t - k >= 0) raw = *reinterpret_cast<const uint4*>(in + (tok - k) * ldi + c);
-        else if (has_past) raw = *reinterpret_cast<const uint4*>(tl + (long)(TAPS - 1 + t - k) * C + c);
-        x[TAPS - 1 - k] = raw;
-      }
-    }
-    x[TAPS - 1] = *reinterpret_cast<const uint4*>(in + tok * ldi + c);
+  auto token = [&](long tok, const uint4* at) {              // at[j]: the input under tap j
     float acc[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[i] = 0.f;
 #pragma unroll
     for (int k = 0; k < TAPS; ++k) {
-      const __nv_bfloat16* xv = reinterpret_cast<const __nv_bfloat16*>(&x[TAPS - 1 - k]);
+      const uint32_t xv[4] = {at[TAPS - 1 - k].x, at[TAPS - 1 - k].y, at[TAPS - 1 - k].z, at[TAPS - 1 - k].w};
 #pragma unroll
-      for (int i = 0; i < 8; ++i) acc[i] += wf[TAPS - 1 - k][i] * __bfloat162float(xv[i]);
+      for (int i = 0; i < 4; ++i) {
+        acc[2 * i] += wf[TAPS - 1 - k][2 * i] * __uint_as_float(xv[i] << 16);
+        acc[2 * i + 1] += wf[TAPS - 1 - k][2 * i + 1] * __uint_as_float(xv[i] & 0xffff0000u);
+      }
     }
     uint4 res;
     __nv_bfloat162* r2 = reinterpret_cast<__nv_bfloat162*>(&res);
 #pragma unroll
     for (int i = 0; i < 4; ++i) r2[i] = __floats2bfloat162_rn(acc[2 * i] * sigmoidf_(acc[2 * i]), acc[2 * i + 1] * sigmoidf_(acc[2 * i + 1]));
     *reinterpret_cast<uint4*>(out + tok * ldo + c) = res;
+  };
+  if (inside) {
 #pragma unroll
-    for (int k = 0; k < TAPS - 1; ++k) x[k] = x[k + 1];
+    for (int j = 0; j < CONV_STRIP; ++j) token(tok0 + j, x + j);
+    return;
+  }
+  for (int j = 0; j < last; ++j) {
+    const long tok = tok0 + j;
+    const int b = tok_seq[tok], t = (int)(tok - seq_off[b]);
+    const bool has_past = past[b] > 0;
+    const __nv_bfloat16* tl = tail + (long)slots[b] * (TAPS - 1) * C;
+#pragma unroll
+    for (int k = 0; k < TAPS; ++k) {
+      uint4 raw = make_uint4(0u, 0u, 0u, 0u);
+      if (t - k >= 0) raw = *reinterpret_cast<const uint4*>(in + (tok - k) * ldi + c);
+      else if (has_past) raw = *reinterpret_cast<const uint4*>(tl + (long)(TAPS - 1 + t - k) * C + c);
+      x[TAPS - 1 - k] = raw;
+    }
+    token(tok, x);
   }
 }
 
@@ -707,16 +718,18 @@ __device__ __forceinline__ void a_parts(const float (&l)[4], const float (&r)[4]
   }
 }
 
-// block = (chunk, key head); heads of a group by warps in turn
+// block = (chunk, key head); heads of a group by pairs of warps in turn: one has T, the other M and the factors (both run the decays of the chunk).
+// Bounded by the chain over the chunk's tokens.  Six blocks per SM (registers, 36 KB): 98 x 8 blocks are one wave instead of one and a twentieth, 29.7 -> 24 us.
 template <int DP>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, 6)
 delta_chunk_prep_kernel(const bf16* __restrict__ qkv, long ldq, int koff, const bf16* __restrict__ a, long lda, const bf16* __restrict__ bl, long ldb,
                         const bf16* __restrict__ A_log, const bf16* __restrict__ dt_bias, const int* __restrict__ seq_off, float* __restrict__ scratch,
                         int B, int H, int KH, int D) {
+  lb::chain_wait(qkv, a, bl, A_log, dt_bias, seq_off);
   lb::chain_next();
   constexpr int LD = DP + 8;
   __shared__ __align__(16) bf16 sK[CL * LD], sQ[CL * LD];
-  __shared__ float sKK[CL][CL + 1], sQK[CL][CL + 1], sA[4][CL][CL + 4];
+  __shared__ float sKK[CL][CL + 1], sQK[CL][CL + 1], sA[2][CL][CL + 4];
   __shared__ double ksc[CL], qsc[CL];
   __shared__ int where[2];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, kh = blockIdx.y;
@@ -814,7 +827,8 @@ delta_chunk_prep_kernel(const bf16* __restrict__ qkv, long ldq, int koff, const 
   }
   __syncthreads();
   const int group = H / KH;
-  for (int hh = warp; hh < group; hh += 4) {
+  const bool is_m = warp & 1;                // even warps: T of a head; odd ones: M and the factors
+  for (int hh = warp >> 1; hh < group; hh += 2) {
     const int h = kh * group + hh;
     float* mine = scratch + ((long)blockIdx.x * H + h) * CL_SCRATCH;
     bf16* Tp = reinterpret_cast<bf16*>(mine);
@@ -826,7 +840,7 @@ delta_chunk_prep_kernel(const bf16* __restrict__ qkv, long ldq, int koff, const 
       g = exp(-exp(static_cast<double>(ldf(A_log + h))) * (z > 40.0 ? z : log1p(exp(z))));
       beta = 1.0 / (1.0 + exp(-static_cast<double>(ldf(bl + (tok0 + lane) * ldb + h))));
     }
-    double x = 0.0, all = 1.0, G = 1.0;      // γ(t, lane); products of all decays up to t
+    double x = 0.0;                          // γ(t, lane)
     const double ks = ksc[lane];
     auto store3 = [&](bf16* p, double v) {
       float x = static_cast<float>(v);
@@ -839,31 +853,41 @@ delta_chunk_prep_kernel(const bf16* __restrict__ qkv, long ldq, int koff, const 
         if (e == 0) x += rest;
       }
     };
+    if (is_m) {
+      double all = 1.0, G = 1.0;             // products of all decays up to t
 #pragma unroll 4
-    for (int t = 0; t < CL; ++t) {
-      const double gt = __shfl_sync(0xffffffffu, g, t), bt = __shfl_sync(0xffffffffu, beta, t);
-      x = t == lane ? 1.0 : (t > lane ? x * gt : 0.0);
-      all *= gt;
-      if (t == lane) G = all;
-      sA[warp][t][lane] = lane < t ? static_cast<float>(bt * x * (ksc[t] * ks) * sKK[t][lane]) : 0.f;
-      store3(Mp + t * CL + lane, lane <= t ? x * qsc[t] * sQK[t][lane] : 0.0);
-    }
-    fac[lane] = static_cast<float>(G * ks);
-    fac[CL + lane] = static_cast<float>(G * qsc[lane]);
-    fac[2 * CL + lane] = static_cast<float>(x);        // (tokens behind the end decay by 1)
-    fac[3 * CL + lane] = static_cast<float>(beta * ks);
-    if (lane == 0) fac[4 * CL] = static_cast<float>(all);
-    __syncwarp();
-    float col[CL];                           // column `lane` of (I + A)^-1
+      for (int t = 0; t < CL; ++t) {
+        const double gt = __shfl_sync(0xffffffffu, g, t);
+        x = t == lane ? 1.0 : (t > lane ? x * gt : 0.0);
+        all *= gt;
+        if (t == lane) G = all;
+        store3(Mp + t * CL + lane, lane <= t ? x * qsc[t] * sQK[t][lane] : 0.0);
+      }
+      fac[lane] = static_cast<float>(G * ks);
+      fac[CL + lane] = static_cast<float>(G * qsc[lane]);
+      fac[2 * CL + lane] = static_cast<float>(x);        // (tokens behind the end decay by 1)
+      fac[3 * CL + lane] = static_cast<float>(beta * ks);
+      if (lane == 0) fac[4 * CL] = static_cast<float>(all);
+    } else {
+      float(*A)[CL + 4] = sA[warp >> 1];
+#pragma unroll 4
+      for (int t = 0; t < CL; ++t) {
+        const double gt = __shfl_sync(0xffffffffu, g, t), bt = __shfl_sync(0xffffffffu, beta, t);
+        x = t == lane ? 1.0 : (t > lane ? x * gt : 0.0);
+        A[t][lane] = lane < t ? static_cast<float>(bt * x * (ksc[t] * ks) * sKK[t][lane]) : 0.f;
+      }
+      __syncwarp();
+      float col[CL];                         // column `lane` of (I + A)^-1
 #pragma unroll
-    for (int t = 0; t < CL; ++t) {
-      float acc[4] = {0.f, 0.f, 0.f, 0.f};
+      for (int t = 0; t < CL; ++t) {
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int s = 0; s < t; ++s) acc[s & 3] += sA[warp][t][s] * col[s];
-      col[t] = t == lane ? 1.f : (t > lane ? -((acc[0] + acc[1]) + (acc[2] + acc[3])) : 0.f);
-      store3(Tp + t * CL + lane, t > lane ? ksc[t] * col[t] * beta : 0.0);
+        for (int s = 0; s < t; ++s) acc[s & 3] += A[t][s] * col[s];
+        col[t] = t == lane ? 1.f : (t > lane ? -((acc[0] + acc[1]) + (acc[2] + acc[3])) : 0.f);
+        store3(Tp + t * CL + lane, t > lane ? ksc[t] * col[t] * beta : 0.0);
+      }
+      __syncwarp();
     }
-    __syncwarp();
   }
 }
 
@@ -1128,8 +1152,9 @@ __global__ void gated_rmsnorm_kernel(const float* __restrict__ o, const T* __res
   }
 }
 
-// The same with 16-byte loads of o (8 bytes of gate, weight and y in bf16), the row kept in registers: V % 4 == 0, V <= 128 R, rows on their
-// vectors.  [2560, 16, 128]: 21.6 -> 12.5 us.
+// The same with 16-byte loads of o (8 bytes of gate, weight and y in bf16), the row kept in registers: V % 4 == 0, V <= 4 LANES R, rows on their
+// vectors.  [2560, 16, 128]: 21.6 -> 12.5 us.  Half of the instructions of a row of 128 are sums, root and addresses, so 16 lanes take it (8 up to 64):
+// [3027, 16, 128] 16.3 -> 15.3 us.
 __device__ __forceinline__ void ld4(const float* p, float (&v)[4]) { const float4 x = *reinterpret_cast<const float4*>(p); v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; }
 __device__ __forceinline__ void ld4(const bf16* p, float (&v)[4]) {
   const uint2 x = *reinterpret_cast<const uint2*>(p);
@@ -1140,34 +1165,36 @@ __device__ __forceinline__ void st4(bf16* p, const float (&v)[4]) {
   const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
   *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
 }
-template <typename T, int R>
+template <typename T, int LANES, int R>
 __global__ void __launch_bounds__(256)
 gated_rmsnorm_vec_kernel(const float* __restrict__ o, const T* __restrict__ gate, long ldg, const T* __restrict__ w, float eps, int act, T* __restrict__ y,
                          long ldy, long rows, int H, int V) {
+  const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x, wid = idx / LANES;
+  const int lane = threadIdx.x % LANES;
+  const long tok = wid <= 0xffffffffL ? (unsigned)wid / (unsigned)H : wid / H;
+  const int h = (int)(wid - tok * H);
   lb::chain_wait(o, gate, w);
   lb::chain_next();
-  const long wid = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (wid >= rows * H) return;
-  const long tok = wid / H; const int h = (int)(wid - tok * H);
+  const bool here = wid < rows * H;          // (the lanes of the others take part in the sums)
   const float* orow = o + wid * V;
   float x[R][4], g[R][4], ss = 0.f;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    const int i = r * 128 + lane * 4;
-    if (i < V) {
+    const int i = (r * LANES + lane) * 4;
+    if (here && i < V) {
       ld4(orow + i, x[r]);
       ld4(gate + tok * ldg + h * V + i, g[r]);
 #pragma unroll
       for (int e = 0; e < 4; ++e) ss += x[r][e] * x[r][e];
     }
   }
-  ss = warp_sum(ss);
+#pragma unroll
+  for (int m = LANES / 2; m > 0; m >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
   const float rr = 1.f / sqrtf(ss / (float)V + eps);
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    const int i = r * 128 + lane * 4;
-    if (i < V) {
+    const int i = (r * LANES + lane) * 4;
+    if (here && i < V) {
       float wv[4];
       ld4(w + i, wv);
 #pragma unroll
@@ -1613,8 +1640,8 @@ int lbs_short_conv(const void* in, long ldi, const void* w, void* tail, const in
     const bool strips = tokens * (C / 8) >= 148L * 8 * 128 * CONV_STRIP / 4;
     const int g = strips ? cdiv((tokens + CONV_STRIP - 1) / CONV_STRIP * (C / 8), 128) : cdiv(tokens * (C / 8), 256);
 #define SC(TP)                                                                                                                   \
-  if (strips) short_conv_strip_kernel<TP><<<g, 128, 0, s>>>((const bf16*)in, ldi, (const bf16*)w, (const bf16*)tail, tok_seq, seq_off, slots, past, \
-                                                            (bf16*)out, ldo, tokens, C);                                          \
+  if (strips) lb_host::launch_chained(short_conv_strip_kernel<TP>, dim3(g), dim3(128), 0, s, 0, (const bf16*)in, ldi, (const bf16*)w, (const bf16*)tail, tok_seq, seq_off, \
+                                      slots, past, (bf16*)out, ldo, tokens, C);                                                  \
   else short_conv_vec8_kernel<TP><<<g, 256, 0, s>>>((const bf16*)in, ldi, (const bf16*)w, (const bf16*)tail, tok_seq, seq_off, slots, past, \
                                                     (bf16*)out, ldo, tokens, C)
     if (taps == 2) { SC(2); } else if (taps == 3) { SC(3); } else { SC(4); }
@@ -1658,8 +1685,8 @@ int lbs_delta_scan(const void* qkv, long ldq, int koff, int voff, const void* a,
     const int smem = (int)sizeof(DeltaChunkSmem<DP>);                                                                                    \
     const cudaError_t e = cudaFuncSetAttribute(delta_chunk_scan_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);          \
     if (e != cudaSuccess) return (int)e;                                                                                                 \
-    delta_chunk_prep_kernel<DP><<<pg, 128, 0, s>>>((const bf16*)qkv, ldq, koff, (const bf16*)a, lda, (const bf16*)bl, ldb, (const bf16*)A_log, \
-                                                   (const bf16*)dt_bias, seq_off, scratch, B, H, KH, D);                                 \
+    lb_host::launch_chained(delta_chunk_prep_kernel<DP>, pg, dim3(128), 0, s, 0, (const bf16*)qkv, ldq, koff, (const bf16*)a, lda, (const bf16*)bl, ldb, \
+                            (const bf16*)A_log, (const bf16*)dt_bias, seq_off, scratch, B, H, KH, D);                                    \
     delta_chunk_scan_kernel<DP><<<sg, 32 * CL_WARPS, smem, s>>>((const bf16*)qkv, ldq, koff, voff, scratch, S, seq_off, slots, past, out, H, KH, D, V); \
   }
     if (D <= 64) DCH(64) else DCH(128)
@@ -1722,8 +1749,8 @@ int lbs_gated_rmsnorm(const float* o, const void* gate, long ldg, const void* w,
   const uintptr_t vec = dtype == 0 ? 16 : 8;                    // bytes of four elements
   if (V % 4 == 0 && V <= 512 && ldg % 4 == 0 && ldy % 4 == 0 && (reinterpret_cast<uintptr_t>(o) & 15) == 0 &&
       ((reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) & (vec - 1)) == 0) {
-#define GRV(R) DISPATCH(dtype, lb_host::launch_chained(gated_rmsnorm_vec_kernel<T, R>, dim3(cdiv(rows * H * 32, 256)), dim3(256), 0, s, 0, o, (const T*)gate, ldg, (const T*)w, eps, act, (T*)y, ldy, rows, H, V))
-    if (V <= 128) { GRV(1); } else if (V <= 256) { GRV(2); } else { GRV(4); }
+#define GRV(LN, R) DISPATCH(dtype, lb_host::launch_chained(gated_rmsnorm_vec_kernel<T, LN, R>, dim3(cdiv(rows * H * LN, 256)), dim3(256), 0, s, 0, o, (const T*)gate, ldg, (const T*)w, eps, act, (T*)y, ldy, rows, H, V))
+    if (V <= 64) { GRV(8, 2); } else if (V <= 128) { GRV(16, 2); } else if (V <= 256) { GRV(32, 2); } else { GRV(32, 4); }
 #undef GRV
     return ok();
   }

@@ -454,6 +454,22 @@ def test_gated_norm_of_read_outs(tokens, heads, v, pad, act, dtype):
     assert bool(((got - want).abs() <= (2.0 ** -20 + (2.0 ** -8 if dtype == BF16 else 0.0)) * want.abs() + 1e-30).all())
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, BF16])
+@pytest.mark.parametrize("rows,heads,v", [(13, 5, 60), (3, 1, 64), (7, 3, 68), (1, 1, 128), (3, 3, 256), (1, 3, 260)])
+def test_gated_norm_of_several_rows_per_warp(rows, heads, v, dtype):
+    """Widths around 8, 16 and 32 lanes per row, last warps with rows that are not there."""
+    from libai_b200.ops import seq_functional as SF
+
+    n = heads * v
+    o, gate, w, y = _rand((rows, n), 1, 2.0, torch.float32), _rand((rows, n), 2, 1.0, dtype), _rand((v,), 3, 1.0, dtype), torch.full((rows + 1, n), 3.0, device="cuda", dtype=dtype)
+    SF.gated_rmsnorm(o, gate, w, 1e-6, 0, y[:rows], heads, v)
+    x, g = o.double().view(rows, heads, v), gate.double().view(rows, heads, v)
+    want = (x * torch.rsqrt(x.square().mean(-1, keepdim=True) + 1e-6) * w.double() * torch.sigmoid(g) * g).view(rows, n)
+    # a dozen fp32 roundings and a sum of v squares, then one rounding to the type
+    assert bool(((y[:rows].double() - want).abs() <= (2.0 ** -20 + (2.0 ** -8 if dtype == BF16 else 0.0)) * want.abs() + 1e-30).all())
+    assert bool((y[rows] == 3).all())
+
+
 @pytest.mark.parametrize("value", [float("inf"), float("nan"), 3e38])
 def test_delta_scan_in_chunks_value_that_is_not_finite(value):
     """It reaches no earlier token, no other column and no other head."""
