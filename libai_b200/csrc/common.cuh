@@ -103,7 +103,7 @@ LB_DEVICE uint4 philox4x32_7(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3,
 
 // ---------------------------------------------------------------------------------------------
 // Launches that overlap the end of the kernel before them (lb_host::launch_chained below).  chain_wait() returns once that kernel has completed and
-// its writes can be seen: before it a kernel touches no global memory.  It takes the pointers that the kernel loads from through
+// its writes can be seen: before it a kernel touches no global memory (but may send for some: tma_prefetch_2d below).  It takes the pointers that the kernel loads from through
 // `const __restrict__` parameters: the compiler could otherwise move their loads in front of it or make them ld.global.nc, which wants memory that
 // nobody writes while the kernel runs, and a chained kernel runs while the one before still writes (so no __ldg in one either).  chain_next() lets the next
 // kernel's blocks start, as soon as every block of this one has got there: behind a block's allocation of TMEM, which the next kernel's blocks
@@ -159,6 +159,10 @@ LB_DEVICE void mbar_wait(uint64_t* bar, uint32_t parity) {
 // ---------------------------------------------------------------------------------------------
 LB_DEVICE void tma_prefetch_desc(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
+}
+// a tile into L2, where the chip's caches meet: may be sent before chain_wait() whoever writes the tile, since nothing is read by it
+LB_DEVICE void tma_prefetch_2d(const CUtensorMap* map, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];\n" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y) : "memory");
 }
 LB_DEVICE void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int32_t c0, int32_t c1) {
   asm volatile(

@@ -27,6 +27,10 @@ struct GsCfg {
 };
 constexpr int GS_SMEM = 104000;                   // of pipeline: two CTAs per SM (one with twice the stages leaves no room for clusters of 8 in some GPCs)
 constexpr int GS_NORM_BLOCKS = 11;                // k-blocks per CTA with a norm in front: their rows of x beside five stages of w
+// K-blocks of w that a CTA sends to L2 ahead of chain_wait(): memory stands still while the small kernel before (a norm, a rotation) ends.  128 KB per CTA are what
+// comes in 3 us.  Llama block, one token of 4 sequences on 2046: 151.5 -> 147.5 us (16 k-blocks 148.4); GPT-2 block of 8 sequences on 511: 38.1 -> 37.2.  The same for the first keys
+// and values of the decode attention gave nothing.
+constexpr int GS_AHEAD = 8;
 constexpr int GS_MAX_STAGES = GS_SMEM / GsCfg<16>::STAGE, GS_TAIL = 1024 + 512;   // alignment, barriers, statistics
 
 struct GemmSmallParams {
@@ -96,6 +100,8 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  if (threadIdx.x == 0)                      // on its way to L2 while the kernel before this one ends
+    for (int kb = kb0; kb < min(kb1, kb0 + GS_AHEAD); ++kb) tma_prefetch_2d(&tmap_w, kb * 64, n0);
   const __nv_bfloat16 *xg = p.x, *gamma = p.gamma, *beta = p.beta;
   chain_wait(xg, gamma, beta);
   chain_next();
