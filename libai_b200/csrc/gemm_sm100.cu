@@ -198,17 +198,19 @@ struct GemmMultiB {
   int count;
   int n[GEMM_MAX_B], first[GEMM_MAX_B + 1], col[GEMM_MAX_B];   // columns; first tile along N; first column of the output
 };
-struct GemmOneB {};
-template <bool MULTI> struct GemmB { using type = GemmOneB; };
-template <> struct GemmB<true> { using type = GemmMultiB; };
+// What only some kinds of the kernel take (a launch costs the host 0.3 us more with 128 bytes of parameters that nothing reads)
+struct GemmPlain {};
+struct GemmReduce { CUtensorMap map; };      // EPI_ATOMIC_F32: the output in boxes of 32 x 32
+template <int EPI, bool MULTI> struct GemmMore { using type = GemmPlain; };
+template <> struct GemmMore<EPI_ATOMIC_F32, false> { using type = GemmReduce; };
+template <> struct GemmMore<EPI_BF16, true> { using type = GemmMultiB; };
 
 // CTAS == 2: `cta_group::2` — clusters of two CTAs (one TPC) compute 256 x BLOCK_N tiles; no fused collectives, bf16 only.
 template <int BLOCK_N, bool A_MN, bool B_MN, int EPI, bool FP8 = false, int CTAS = 1, bool MULTI = false>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
             const __grid_constant__ CUtensorMap tmap_g /* COMM_AG: the local shard of the gathered operand */,
-            const __grid_constant__ CUtensorMap tmap_o /* EPI_ATOMIC_F32: the output in boxes of 32 x 32 */, GemmParams p, CommParams cp,
-            const __grid_constant__ typename GemmB<MULTI>::type mb) {
+            GemmParams p, CommParams cp, const __grid_constant__ typename GemmMore<EPI, MULTI>::type more) {
   using Cfg = StageCfg<BLOCK_N, CTAS, EPI == EPI_ATOMIC_F32, B_MN>;
   constexpr int NS = Cfg::NUM_STAGES;
   static_assert(CTAS == 1 || (CTAS == 2 && BLOCK_N >= 128 && !FP8), "CTA-pair mode: bf16 tiles of 128 columns and more");
@@ -229,11 +231,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   const int m_blocks = (p.M + BLOCK_M * CTAS - 1) / (BLOCK_M * CTAS);
   static_assert(!MULTI || (CTAS == 2 && !A_MN && !B_MN && EPI == EPI_BF16), "several B: NT products on CTA pairs, bf16 results");
   int n_blocks = (p.N + BLOCK_N - 1) / BLOCK_N;
-  if constexpr (MULTI) n_blocks = mb.first[mb.count];
+  if constexpr (MULTI) n_blocks = more.first[more.count];
   [[maybe_unused]] auto segment = [&](int n_blk) {          // MULTI: which matrix a column tile belongs to
     int i = 0;
     if constexpr (MULTI)
-      while (n_blk >= mb.first[i + 1]) ++i;
+      while (n_blk >= more.first[i + 1]) ++i;
     return i;
   };
   const int k_blocks_total = (p.K + BLOCK_K - 1) / BLOCK_K;
@@ -280,12 +282,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmap_a);
     if constexpr (MULTI) {
-      for (int i = 0; i < mb.count; ++i) tma_prefetch_desc(&mb.map[i]);
+      for (int i = 0; i < more.count; ++i) tma_prefetch_desc(&more.map[i]);
     } else {
       tma_prefetch_desc(&tmap_b);
     }
     if (cp.mode == COMM_AG) tma_prefetch_desc(&tmap_g);
-    if constexpr (EPI == EPI_ATOMIC_F32) tma_prefetch_desc(&tmap_o);
+    if constexpr (EPI == EPI_ATOMIC_F32) tma_prefetch_desc(&more.map);
 #pragma unroll
     for (int i = 0; i < NS; ++i) {
       mbar_init(&full_bar[i], CTAS);   // pair: the leader's barrier collects one arrival per CTA (+ both CTAs' bytes)
@@ -451,8 +453,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         const CUtensorMap* map_nt = &tmap_b;
         if constexpr (MULTI) {
           const int seg = segment(n_blk);
-          map_nt = &mb.map[seg];
-          n_row -= mb.first[seg] * BLOCK_N;
+          map_nt = &more.map[seg];
+          n_row -= more.first[seg] * BLOCK_N;
         }
         const int kb0 = split * p.k_per_split;
         const int kb1 = min(kb0 + p.k_per_split, k_blocks_total);
@@ -605,9 +607,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BLOCK_N;
       int tile_col = n_blk * BLOCK_N, tile_cols = p.N - tile_col;        // first column of the tile in the output, columns that there are from there
       if constexpr (MULTI) {
-        const int seg = segment(n_blk), local = (n_blk - mb.first[seg]) * BLOCK_N;
-        tile_col = mb.col[seg] + local;
-        tile_cols = mb.n[seg] - local;
+        const int seg = segment(n_blk), local = (n_blk - more.first[seg]) * BLOCK_N;
+        tile_col = more.col[seg] + local;
+        tile_cols = more.n[seg] - local;
       }
 #pragma unroll 1
       for (int c = half * CHUNKS_PER_HALF; c < (half + 1) * CHUNKS_PER_HALF; ++c) {
@@ -716,7 +718,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           __syncwarp();
           const int row0 = m_blk * BLOCK_M + quad * 32;
           if (lane == 0 && row0 < p.M) {                    // (rows and columns behind the end are left out by the map)
-            tma_reduce_add_2d(&tmap_o, stg, col0, row0);
+            tma_reduce_add_2d(&more.map, stg, col0, row0);
             tma_store_commit();
           }
         } else {
@@ -991,7 +993,9 @@ cudaError_t launch_2cta(const CUtensorMap& ta, const CUtensorMap& tb, const CUte
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  if (chained(p, cp)) return lb_host::launch_chained(kern, dim3((unsigned)grid), dim3(lb::NUM_THREADS), Cfg::SMEM_BYTES, stream, 2, ta, tb, tg, to, p, cp, lb::GemmOneB{});
+  typename lb::GemmMore<EPI, false>::type more;
+  if constexpr (EPI == lb::EPI_ATOMIC_F32) more.map = to;
+  if (chained(p, cp)) return lb_host::launch_chained(kern, dim3((unsigned)grid), dim3(lb::NUM_THREADS), Cfg::SMEM_BYTES, stream, 2, ta, tb, tg, p, cp, more);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3(lb::NUM_THREADS);
@@ -1004,7 +1008,7 @@ cudaError_t launch_2cta(const CUtensorMap& ta, const CUtensorMap& tb, const CUte
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, ta, tb, tg, to, p, cp, lb::GemmOneB{});
+  return cudaLaunchKernelEx(&cfg, kern, ta, tb, tg, p, cp, more);
 }
 
 template <int BN, bool AMN, bool BMN, int EPI, bool FP8 = false>
@@ -1018,8 +1022,10 @@ cudaError_t launch_cfg(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  if (chained(p, cp)) return lb_host::launch_chained(kern, dim3((unsigned)grid), dim3(lb::NUM_THREADS), Cfg::SMEM_BYTES, stream, 0, ta, tb, tg, to, p, cp, lb::GemmOneB{});
-  kern<<<grid, lb::NUM_THREADS, Cfg::SMEM_BYTES, stream>>>(ta, tb, tg, to, p, cp, lb::GemmOneB{});
+  typename lb::GemmMore<EPI, false>::type more;
+  if constexpr (EPI == lb::EPI_ATOMIC_F32) more.map = to;
+  if (chained(p, cp)) return lb_host::launch_chained(kern, dim3((unsigned)grid), dim3(lb::NUM_THREADS), Cfg::SMEM_BYTES, stream, 0, ta, tb, tg, p, cp, more);
+  kern<<<grid, lb::NUM_THREADS, Cfg::SMEM_BYTES, stream>>>(ta, tb, tg, p, cp, more);
   return cudaGetLastError();
 }
 
@@ -1378,7 +1384,7 @@ static cudaError_t launch_multi(const CUtensorMap& ta, const lb::GemmParams& p, 
   }
   lb::CommParams cp;
   memset(&cp, 0, sizeof(cp));
-  return lb_host::launch_chained(kern, dim3((unsigned)grid), dim3(lb::NUM_THREADS), Cfg::SMEM_BYTES, stream, 2, ta, ta, ta, ta, p, cp, mb);
+  return lb_host::launch_chained(kern, dim3((unsigned)grid), dim3(lb::NUM_THREADS), Cfg::SMEM_BYTES, stream, 2, ta, ta, ta, p, cp, mb);
 }
 // x [M, K] against `count` matrices w[i] [n[i], K] at once: out [M, ldo], the results one after the other.  One launch and one last wave in place of a launch each, and
 // the first of them put together by a copy: a mixer's projections (1024 + 1024 + 2048, 16, 16 and 2048 columns, K = 2048) of 1600 rows 68.4 -> 37.9 us, 300 rows 46.1 -> 15.2,

@@ -31,10 +31,11 @@ constexpr int GS_NORM_BLOCKS = 11;                // k-blocks per CTA with a nor
 // comes in 3 us.  Llama block, one token of 4 sequences on 2046: 151.5 -> 147.5 us (16 k-blocks 148.4); GPT-2 block of 8 sequences on 511: 38.1 -> 37.2.  The same for the first keys
 // and values of the decode attention gave nothing.
 constexpr int GS_AHEAD = 8;
+constexpr long GS_AHEAD_BYTES = 4 << 20;
 constexpr int GS_MAX_STAGES = GS_SMEM / GsCfg<16>::STAGE, GS_TAIL = 1024 + 512;   // alignment, barriers, statistics
 
 struct GemmSmallParams {
-  int M, N, K, kb_total, kb_per_cta, stages;
+  int M, N, K, kb_total, kb_per_cta, stages, ahead;
   const __nv_bfloat16* bias;      // [N] or nullptr
   const __nv_bfloat16* residual;  // [M, ldo] or nullptr
   __nv_bfloat16 *out, *pre_out;   // [M, ldo]; pre_out (optional): before the activation
@@ -100,8 +101,8 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
-  if (threadIdx.x == 0)                      // on its way to L2 while the kernel before this one ends
-    for (int kb = kb0; kb < min(kb1, kb0 + GS_AHEAD); ++kb) tma_prefetch_2d(&tmap_w, kb * 64, n0);
+  if (threadIdx.x == 32)                     // on its way to L2 while the kernel before this one ends; the warp whose own work begins last
+    for (int kb = kb0; kb < min(kb1, kb0 + p.ahead); ++kb) tma_prefetch_2d(&tmap_w, kb * 64, n0);
   const __nv_bfloat16 *xg = p.x, *gamma = p.gamma, *beta = p.beta;
   chain_wait(xg, gamma, beta);
   chain_next();
@@ -341,6 +342,7 @@ cudaError_t launch_gemm_small_r(const CUtensorMap& tw, const CUtensorMap& tx, Ge
   auto kern = gemm_small_kernel<NT, RANKS, NORM>;
   const int stage = NORM ? GS_W_BYTES : GsCfg<NT>::STAGE, rows = NORM ? p.kb_per_cta * GsCfg<NT>::X_BYTES : 0;
   const int fit = (GS_SMEM - rows) / stage;
+  p.ahead = (long)p.N * p.K * 2 >= GS_AHEAD_BYTES ? GS_AHEAD : 0;
   p.stages = p.kb_per_cta < 2 ? 2 : p.kb_per_cta;
   if (p.stages > fit) p.stages = fit;
   const int smem = p.stages * stage + rows + GS_TAIL;
