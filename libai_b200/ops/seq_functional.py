@@ -57,7 +57,7 @@ def slice_act(inp, out, act: int):
 
 def linear_accumulate(x32, a, w):
     """``x32 += a @ wᵀ`` with the fp32 residual stream as the accumulator: on the tcgen05 GEMM the product is added to
-    ``x32`` by the epilogue (fp32 ``red.add``), so the residual sum never passes through 16 bits."""
+    ``x32`` by the epilogue (fp32 TMA reductions), so the residual sum never passes through 16 bits."""
     from . import load_ext, use_native
 
     if (a.is_cuda and a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and use_native(a) and a.stride(-1) == 1
