@@ -198,7 +198,7 @@ struct GemmMultiB {
   int count;
   int n[GEMM_MAX_B], first[GEMM_MAX_B + 1], col[GEMM_MAX_B];   // columns; first tile along N; first column of the output
 };
-// What only some kinds of the kernel take (a launch costs the host 0.3 us more with 128 bytes of parameters that nothing reads)
+// What only some kinds of the kernel take
 struct GemmPlain {};
 struct GemmReduce { CUtensorMap map; };      // EPI_ATOMIC_F32: the output in boxes of 32 x 32
 template <int EPI, bool MULTI> struct GemmMore { using type = GemmPlain; };

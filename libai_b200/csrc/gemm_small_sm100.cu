@@ -29,7 +29,7 @@ constexpr int GS_SMEM = 104000;                   // of pipeline: two CTAs per S
 constexpr int GS_NORM_BLOCKS = 11;                // k-blocks per CTA with a norm in front: their rows of x beside five stages of w
 // K-blocks of w that a CTA sends to L2 ahead of chain_wait(): memory stands still while the small kernel before (a norm, a rotation) ends.  128 KB per CTA are what
 // comes in 3 us.  Llama block, one token of 4 sequences on 2046: 151.5 -> 147.5 us (16 k-blocks 148.4); GPT-2 block of 8 sequences on 511: 38.1 -> 37.2.  The same for the first keys
-// and values of the decode attention gave nothing.
+// and values of the decode attention gave nothing.  Not for small matrices, which are in L2 more often than not: [200, 384] x [384, 384] out of L2 4.56 us, 4.91 with it.
 constexpr int GS_AHEAD = 8;
 constexpr long GS_AHEAD_BYTES = 4 << 20;
 constexpr int GS_MAX_STAGES = GS_SMEM / GsCfg<16>::STAGE, GS_TAIL = 1024 + 512;   // alignment, barriers, statistics
