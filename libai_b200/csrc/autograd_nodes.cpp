@@ -455,7 +455,7 @@ struct BlockArgs {
   int64_t heads;
   std::vector<double> eps;
   double scale, cross_scale;
-  bool causal, fuse_bias;
+  bool causal, fuse_bias;               // causal: the triangle alone (a mask stands in its place, lengths stand beside it)
   Opt kv_lens, mask, cross_mask;
 };
 
@@ -474,7 +474,7 @@ Tensor block_of_nodes(const Tensor& x, at::TensorList p, const Opt& enc, const B
   auto [ln, skip] = norm_and_skip(x, p[0], p[1], a.eps[0], false);
   const Tensor qkv = Linear::apply(ln, p[2], Opt(p[3]), 0).view({B, -1, a.heads, 3 * d});
   const Tensor c = flash(a, d) ? FlashPacked::apply(qkv, a.causal, a.scale, a.kv_lens, 0.0, Opt(), 0)
-                               : SplitAttention::apply(qkv, Opt(), Opt(), 0, a.causal && !has(a.mask), a.scale, a.mask);
+                               : SplitAttention::apply(qkv, Opt(), Opt(), 0, a.causal, a.scale, a.mask);
   Tensor y = LinearResidual::apply(c.reshape({B, -1, ad}), p[4], Opt(p[5]), skip);
   if (has(enc)) {
     std::tie(ln, skip) = norm_and_skip(y, p[6], p[7], a.eps[1], false);
@@ -842,7 +842,7 @@ std::vector<Tensor> block(const Tensor& x, const std::vector<Tensor>& p, int64_t
   if (cross && (enc->dim() != 3 || !lb_ops::block_tensor(*enc, x) || enc->numel() == 0 || enc->size(0) != B || enc->size(2) != h || !norm_ok(6) ||
                 !linear_ok(8, ad, h) || !linear_ok(10, 2 * ad, h) || !linear_ok(12, h, ad)))
     return {};
-  const BlockArgs a{heads, eps.vec(), scale, cross_scale, causal, fuse_bias, kv_lens, mask, cross_mask};
+  const BlockArgs a{heads, eps.vec(), scale, cross_scale, causal && !has(mask), fuse_bias, kv_lens, mask, cross_mask};
   return {all_want_gradients(p) ? Block::apply(x, at::TensorList(p), enc, a) : block_of_nodes(x, p, enc, a)};
 }
 

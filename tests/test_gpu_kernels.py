@@ -1155,7 +1155,8 @@ def test_products_with_several_matrices_in_one_launch(m, k, ns):
 
 
 def _train_block(kind, dim, with_main_grad):
-    """A block, its call and its inputs: causal, right-padded, without a mask, T5 decoder, Llama."""
+    """A block, its call and its inputs: causal, right-padded, without a mask, T5 decoder, Llama; causal with a mask of its own, which stands in the triangle's place (dense,
+    padded on the left) or, in the flash kernels, beside it (right-padded)."""
     from libai_b200.layers import TransformerLayer
     from libai_b200.layers._param import param_defaults
     from libai_b200.layers.attention import AttnMaskType, KeyPaddingMask
@@ -1169,7 +1170,7 @@ def _train_block(kind, dim, with_main_grad):
             layer = LlamaDecoderLayer(hidden, 256, heads, rms_norm_eps=1e-6, max_position_embeddings=64)
         else:
             layer = TransformerLayer(hidden, 2 * hidden, heads, is_decoder=kind == "decoder",
-                                     attn_mask_type=AttnMaskType.causal if kind == "causal" else AttnMaskType.padding)
+                                     attn_mask_type=AttnMaskType.causal if kind.startswith("causal") else AttnMaskType.padding)
         for i, p in enumerate(layer.parameters()):
             p.data.copy_(_rand(p.shape, 10 + i, 0.05 if p.dim() > 1 else 0.1) + (p.dim() == 1))
     if with_main_grad or kind == "llama":       # (one buffer: gate and up weights side by side)
@@ -1184,12 +1185,18 @@ def _train_block(kind, dim, with_main_grad):
         m = torch.ones(3, 1, s, s, dtype=torch.bool, device="cuda").tril()
         cm = (torch.arange(24, device="cuda") < 20).expand(3, 1, s, 24)
         return layer, lambda: layer(x, m, enc, cm), [x, enc]
-    mask = KeyPaddingMask((torch.arange(s, device="cuda")[None] < torch.tensor([[s], [17], [1]], device="cuda")).long()) if kind == "padded" else None
+    mask = KeyPaddingMask((torch.arange(s, device="cuda")[None] < torch.tensor([[s], [17], [1]], device="cuda")).long()) if kind.endswith("padded") else None
+    if kind == "causal-left":
+        mask = KeyPaddingMask((torch.arange(s, device="cuda")[None] >= torch.tensor([[0], [17], [s - 1]], device="cuda")).long())
+    if kind == "causal-prefix":                 # the first 13 positions see one another
+        mask = torch.ones(s, s, dtype=torch.bool, device="cuda").tril()
+        mask[:13, :13] = True
     return layer, lambda: layer(x, mask), [x]
 
 
 @pytest.mark.parametrize("main_grad", [False, True])
-@pytest.mark.parametrize("kind,dim", [("causal", 64), ("causal", 24), ("padded", 128), ("padded", 48), ("none", 32), ("decoder", 32), ("decoder", 64), ("llama", 128)])
+@pytest.mark.parametrize("kind,dim", [("causal", 64), ("causal", 24), ("padded", 128), ("padded", 48), ("none", 32), ("decoder", 32), ("decoder", 64), ("llama", 128),
+                                      ("causal-prefix", 48), ("causal-prefix", 64), ("causal-padded", 24), ("causal-padded", 64), ("causal-left", 32), ("causal-left", 64)])
 def test_block_graph_in_one_call(kind, dim, main_grad):
     """One node per block, one per operator (a hook on a module) and the Python functions (a dispatch mode looks on) launch the same kernels: outputs to
     the bit, gradients up to the order of their sums; a second backward pass, checkpointing, frozen parameters and a graph of the gradients work as with the modules."""
@@ -1239,6 +1246,19 @@ def test_block_graph_in_one_call(kind, dim, main_grad):
     y = call()
     g = torch.autograd.grad(y, inputs, _rand(y.shape, 5), create_graph=True)
     assert float((g[0].double() - wg[0]).norm()) <= 2.0 ** -7 * float(wg[0].norm())
+
+
+@pytest.mark.parametrize("kind,dim", [("causal-prefix", 48), ("causal-prefix", 64), ("causal-padded", 24), ("causal-padded", 128), ("causal-left", 64), ("padded", 48)])
+def test_block_trains_the_function_that_it_evaluates(kind, dim):
+    """With a mask: as one node, with a node per operator (frozen parameters) and without a graph, to the bit."""
+    layer, call, _ = _train_block(kind, dim, False)
+    with torch.no_grad():
+        want = call()
+    y = call()
+    assert "Block" in y.grad_fn.name() and torch.equal(y, want)
+    layer.mlp.dense_4h_to_h.bias.requires_grad_(False)
+    y = call()
+    assert "Block" not in y.grad_fn.name() and torch.equal(y, want)
 
 
 def test_block_graph_refuses_what_changed_in_between():
