@@ -77,7 +77,8 @@ int64_t bits(std::initializer_list<bool> need) {
   for (bool b : need) m |= static_cast<int64_t>(b) << i++;
   return m;
 }
-// A block's parameters themselves, whose main_grad is asked for: what is unpacked may be a copy (checkpointing, saved-tensor hooks).
+// A block's parameters themselves, whose main_grad is asked for: what is unpacked may be a copy (checkpointing, saved-tensor hooks).  Like the Python functions, save_for_backward
+// gets the weights of norms and linear layers only; biases, and the weights of a gated MLP, which have to lie in one buffer, do not go through hooks.
 void hold_parameters(AutogradContext* ctx, at::TensorList p) { ctx->saved_data["params"] = c10::List<Tensor>(p); }
 std::vector<Tensor> held_parameters(AutogradContext* ctx) { return ctx->saved_data["params"].toTensorVector(); }
 bool wants(AutogradContext* ctx, int i) { return (ctx->saved_data["need"].toInt() >> i) & 1; }
@@ -566,6 +567,7 @@ struct Block : Function<Block> {
     const int64_t B = x.size(0), S = x.size(1), h = x.size(2), T = B * S, ad = p[2].size(0) / 3, d = ad / a.heads;
     const size_t m = has(enc) ? 14 : 6;
     variable_list keep(p.begin(), p.end());
+    for (size_t i = 1; i < p.size(); i += 2) keep[i] = Tensor();       // biases
     keep.push_back(x);
     keep.push_back(has(enc) ? *enc : Tensor());
     Tensor y;
@@ -638,24 +640,24 @@ struct Block : Function<Block> {
     const auto scales = ctx->saved_data["scales"].toDoubleVector();
     const Tensor &x = s[n], &enc = s[n + 1], mask = held(ctx, "mask");
     variable_list out(n + 3);              // x, parameters, enc, arguments
+    const std::vector<Tensor> own = held_parameters(ctx);
     if (at::GradMode::is_enabled()) {      // a graph of the gradients is wanted: that of the single nodes
       const Tensor cross_mask = held(ctx, "cross_mask");
       const BlockArgs a{heads, ctx->saved_data["eps"].toDoubleVector(), scales[0], scales[1], causal, fuse, flash_lens(s, n, mask), opt(mask), opt(cross_mask)};
-      const Tensor y = block_of_nodes(x, p, opt(enc), a);
+      const Tensor y = block_of_nodes(x, own, opt(enc), a);
       variable_list inputs;
       std::vector<size_t> at;
       auto add = [&](const Tensor& t, size_t i) {
         if (t.defined() && t.requires_grad()) { inputs.push_back(t); at.push_back(i); }
       };
       add(x, 0);
-      for (size_t i = 0; i < n; ++i) add(p[i], 1 + i);
+      for (size_t i = 0; i < n; ++i) add(own[i], 1 + i);
       add(enc, 1 + n);
       const auto got = torch::autograd::grad({y}, inputs, {grad[0]}, /*retain_graph=*/true, /*create_graph=*/true, /*allow_unused=*/true);
       for (size_t i = 0; i < got.size(); ++i) out[at[i]] = got[i];
       return out;
     }
     Tensor gx, genc;
-    const std::vector<Tensor> own = held_parameters(ctx);
     Gradients g(own);
     {
       at::AutoDispatchBelowADInplaceOrView guard;
@@ -669,10 +671,10 @@ struct Block : Function<Block> {
       g.weight(m + 4, gy, ff[4], p[m + 4]);
       g.weight(m + 2, dpre, ff[0], p[m + 2]);
       if (fused) g.added[m + 3] = 1;
-      else g.bias(m + 3, dpre, p[m + 3]);
+      else g.bias(m + 3, dpre, own[m + 3]);
       Tensor dln = input_grad(dpre, p[m + 2]);
       Tensor dy = g.norm_and_biases(m, dln, cross ? cr[10] : self[9], p[m], ff[1], ff[2], gy, cross ? 13 : 5, static_cast<int>(m) + 5);
-      g.bias(m + 5, gy, p[m + 5]);
+      g.bias(m + 5, gy, own[m + 5]);
       auto attend_back = [&](int64_t layout, const Tensor& t0, const Tensor& t1, const Tensor& dctx, const Tensor* kept, bool causal_, double scale, Tensor& g0,
                              Tensor& g1) {
         g0 = at::empty(t0.sizes(), t0.options());
@@ -687,23 +689,23 @@ struct Block : Function<Block> {
         const Tensor q = cr[3].view({B, S, heads, d}), kv = cr[4].view({B, -1, heads, 2 * d}), e2 = enc.view({-1, h});
         const Tensor dctx = input_grad(dy, p[12]);
         g.weight(12, dy, cr[9], p[12]);
-        g.bias(13, dy, p[13]);
+        g.bias(13, dy, own[13]);
         Tensor gq, gkv;
         attend_back(1, q, kv, dctx, cr + 5, false, scales[1], gq, gkv);
         gq = gq.view({T, ad});
         gkv = gkv.view({-1, 2 * ad});
         if (flags & 8) genc = input_grad(gkv, p[10]);
         g.weight(10, gkv, e2, p[10]);
-        g.bias(11, gkv, p[11]);
+        g.bias(11, gkv, own[11]);
         dln = input_grad(gq, p[8]);
         g.weight(8, gq, cr[0], p[8]);
-        g.bias(9, gq, p[9]);
+        g.bias(9, gq, own[9]);
         dy = g.norm_and_biases(6, dln, self[9], p[6], cr[1], cr[2], dy, 5, -1);
       }
       const Tensor qkv = self[3].view({B, S, heads, 3 * d});
       const Tensor dctx = input_grad(dy, p[4]);
       g.weight(4, dy, self[8], p[4]);
-      g.bias(5, dy, p[5]);
+      g.bias(5, dy, own[5]);
       Tensor dqkv, none;
       if (!mask.defined() && (d == 64 || d == 128)) {
         const auto [q, kk, v] = FlashPacked::parts(qkv);
@@ -716,7 +718,7 @@ struct Block : Function<Block> {
       dqkv = dqkv.view({T, 3 * ad});
       dln = input_grad(dqkv, p[2]);
       g.weight(2, dqkv, self[0], p[2]);
-      g.bias(3, dqkv, p[3]);
+      g.bias(3, dqkv, own[3]);
       gx = g.norm(0, dln, x2, p[0], self[1], self[2], false, true, dy);
     }
     g.mark(own);
@@ -737,6 +739,7 @@ struct LlamaBlock : Function<LlamaBlock> {
                         double scale) {
     const int64_t B = x.size(0), S = x.size(1), h = x.size(2), T = B * S, ad = p[1].size(0) / 3, d = ad / heads;
     variable_list keep(p.begin(), p.end());
+    for (size_t i = 4; i < p.size(); ++i) keep[i] = Tensor();          // gate, up, down, bias of qkv
     keep.insert(keep.end(), {x, cos, sin});
     Tensor y;
     {
@@ -769,9 +772,10 @@ struct LlamaBlock : Function<LlamaBlock> {
     const variable_list p(s.begin(), s.begin() + n);
     const Tensor &x = s[n], &cos = s[n + 1], &sin = s[n + 2], *k = &s[n + 3];
     variable_list out(n + 7);              // x, parameters, cos, sin, heads, eps, eps, scale
+    const std::vector<Tensor> own = held_parameters(ctx);
     if (at::GradMode::is_enabled()) {
-      const Tensor y = llama_of_nodes(x, at::TensorList(p.data(), 7), n > 7 ? Opt(p[7]) : Opt(), cos, sin, heads, eps[0], eps[1], eps[2]);
-      variable_list inputs(p);
+      const Tensor y = llama_of_nodes(x, at::TensorList(own.data(), 7), n > 7 ? Opt(own[7]) : Opt(), cos, sin, heads, eps[0], eps[1], eps[2]);
+      variable_list inputs(own);
       if (x.requires_grad()) inputs.push_back(x);
       const auto got = torch::autograd::grad({y}, inputs, {grad[0]}, /*retain_graph=*/true, /*create_graph=*/true, /*allow_unused=*/true);
       for (size_t i = 0; i < n; ++i) out[1 + i] = got[i];
@@ -779,16 +783,15 @@ struct LlamaBlock : Function<LlamaBlock> {
       return out;
     }
     Tensor gx;
-    const std::vector<Tensor> own = held_parameters(ctx);
     Gradients g(own);
     {
       at::AutoDispatchBelowADInplaceOrView guard;
-      const int64_t B = x.size(0), S = x.size(1), h = x.size(2), T = B * S, ad = p[1].size(0) / 3, d = ad / heads, f = p[4].size(0);
-      const Tensor x2 = x.view({T, h}), gy = rows(grad[0]), w = stacked(p[4], p[5]);
+      const int64_t B = x.size(0), S = x.size(1), h = x.size(2), T = B * S, ad = p[1].size(0) / 3, d = ad / heads, f = own[4].size(0);
+      const Tensor x2 = x.view({T, h}), gy = rows(grad[0]), w = stacked(own[4], own[5]);
       TORCH_CHECK(w.defined(), "llama block: gate and up weights of one buffer");
       const Tensor joint = fp32(g.main[4]) ? stacked(g.main[4], g.main[5]) : Tensor();
-      const Tensor dh = input_grad(gy, p[6]);
-      g.weight(6, gy, k[9], p[6]);
+      const Tensor dh = input_grad(gy, own[6]);
+      g.weight(6, gy, k[9], own[6]);
       const Tensor dgu = lb_ops::swiglu_packed_bwd(dh, k[8]);
       const Tensor dln2 = input_grad(dgu, w);
       if (joint.defined()) {
@@ -796,8 +799,8 @@ struct LlamaBlock : Function<LlamaBlock> {
         g.added[4] = g.added[5] = 1;
       } else {
         const Tensor both = lb_ops::gemm(dgu, k[6], 2, {}, {}, false, at::kFloat);
-        g.out[4] = both.narrow(0, 0, f).to(p[4].scalar_type());
-        g.out[5] = both.narrow(0, f, f).to(p[5].scalar_type());
+        g.out[4] = both.narrow(0, 0, f).to(own[4].scalar_type());
+        g.out[5] = both.narrow(0, f, f).to(own[5].scalar_type());
       }
       const Tensor dy = g.norm(3, dln2, k[5], p[3], k[10], k[7], true, false, gy);
       const Tensor dctx = input_grad(dy, p[2]);
@@ -808,7 +811,7 @@ struct LlamaBlock : Function<LlamaBlock> {
       dqkv = lb_ops::rope_qkv(dqkv.view({B, S, heads, 3 * d}), cos, sin, 0, true, true).view({T, 3 * ad});
       const Tensor dln1 = input_grad(dqkv, p[1]);
       g.weight(1, dqkv, k[0], p[1]);
-      if (n > 7) g.bias(7, dqkv, p[7]);
+      if (n > 7) g.bias(7, dqkv, own[7]);
       gx = g.norm(0, dln1, x2, p[0], k[10], k[1], true, false, dy);
       count(6);                            // attention, rotation, SwiGLU, gate and up weights
     }

@@ -1261,6 +1261,38 @@ def test_block_trains_the_function_that_it_evaluates(kind, dim):
     assert "Block" not in y.grad_fn.name() and torch.equal(y, want)
 
 
+@pytest.mark.parametrize("main_grad", [False, True])
+@pytest.mark.parametrize("kind,dim", [("causal", 64), ("padded", 48), ("decoder", 32), ("llama", 128)])
+def test_block_under_hooks_that_copy_what_is_saved(kind, dim, main_grad):
+    """Saved tensors that come back as copies (offloading): gradients as without the hooks."""
+    got = []
+    for hooks in (False, True):
+        layer, call, inputs = _train_block(kind, dim, main_grad)
+        if hooks:
+            with torch.autograd.graph.save_on_cpu():
+                y = call()
+        else:
+            y = call()
+        assert "Block" in y.grad_fn.name()
+        y.backward(_rand(y.shape, 5))
+        got.append([t.grad for t in inputs] + [p.main_grad if getattr(p, "main_grad", None) is not None else p.grad for p in layer.parameters()])
+    for a, b in zip(*got):
+        assert float((a.double() - b.double()).norm()) <= 2.0 ** -7 * float(a.double().norm())
+
+
+@pytest.mark.parametrize("kind,dim", [("causal", 64), ("llama", 128)])
+def test_block_graph_takes_biases_that_changed_in_between(kind, dim):
+    """They are no part of the backward pass."""
+    layer, call, inputs = _train_block(kind, dim, True)
+    y = call()
+    with torch.no_grad():
+        for m in layer.modules():
+            if getattr(m, "bias", None) is not None:
+                m.bias.add_(1)
+    y.backward(_rand(y.shape, 5))
+    assert inputs[0].grad is not None
+
+
 def test_block_graph_refuses_what_changed_in_between():
     layer, call, inputs = _train_block("causal", 64, True)
     y = call()
