@@ -3,7 +3,8 @@
 // An autograd function in Python costs 25 to 45 us forward and about as much backward (its own apply, views, checks, the dispatch of every kernel), more than
 // most kernels of a training block take up to some thousand tokens: a T5 decoder block of 16 x 128 tokens took 1200 us of which the GPU worked 420 (host time now 540).  Here
 // a node is a torch::autograd::Function that launches the same kernels in the same order and saves the same tensors through save_for_backward, so
-// saved-tensor hooks, checkpointing, retain_graph and the checks of versions see what they saw.  Whatever transforms a call (vmap, forward-mode, traces) takes the
+// saved-tensor hooks, checkpointing, retain_graph and the checks of versions see what they saw.  With create_graph the gradients are what they are without and have no graph, as
+// those of the Python functions have none (kernels record nothing); only SplitAttention alone differentiates the unfused form then, for q, k and v that come from elsewhere.  Whatever transforms a call (vmap, forward-mode, traces) takes the
 // Python functions as before; the caller decides (`_graph_node`).  Nothing is kept from one call for the next.
 //
 // Weight gradients go to `param.main_grad` where the parameter has one, which is a Python attribute that may come and go between forward and backward
@@ -623,40 +624,21 @@ struct Block : Function<Block> {
     ctx->save_for_backward(std::move(keep));
     hold_parameters(ctx, p);
     ctx->saved_data["heads"] = a.heads;
-    ctx->saved_data["eps"] = a.eps;
     ctx->saved_data["scales"] = std::vector<double>{a.scale, a.cross_scale};
-    ctx->saved_data["flags"] = bits({a.causal, a.fuse_bias, has(enc), requires_grad(enc)});
-    if (has(a.mask)) ctx->saved_data["mask"] = *a.mask;
-    if (has(a.cross_mask)) ctx->saved_data["cross_mask"] = *a.cross_mask;
+    ctx->saved_data["flags"] = bits({a.causal, a.fuse_bias, has(enc), requires_grad(enc), flash(a, d)});
     return y.view(x.sizes());
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grad) {
     auto s = ctx->get_saved_variables();
     const int64_t flags = ctx->saved_data["flags"].toInt(), heads = ctx->saved_data["heads"].toInt();
-    const bool causal = flags & 1, fuse = flags & 2, cross = flags & 4;
+    const bool causal = flags & 1, fuse = flags & 2, cross = flags & 4, by_flash = flags & 16;
     const size_t m = cross ? 14 : 6, n = m + 6;
     const variable_list p(s.begin(), s.begin() + n);
     const auto scales = ctx->saved_data["scales"].toDoubleVector();
-    const Tensor &x = s[n], &enc = s[n + 1], mask = held(ctx, "mask");
+    const Tensor &x = s[n], &enc = s[n + 1];
     variable_list out(n + 3);              // x, parameters, enc, arguments
     const std::vector<Tensor> own = held_parameters(ctx);
-    if (at::GradMode::is_enabled()) {      // a graph of the gradients is wanted: that of the single nodes
-      const Tensor cross_mask = held(ctx, "cross_mask");
-      const BlockArgs a{heads, ctx->saved_data["eps"].toDoubleVector(), scales[0], scales[1], causal, fuse, flash_lens(s, n, mask), opt(mask), opt(cross_mask)};
-      const Tensor y = block_of_nodes(x, own, opt(enc), a);
-      variable_list inputs;
-      std::vector<size_t> at;
-      auto add = [&](const Tensor& t, size_t i) {
-        if (t.defined() && t.requires_grad()) { inputs.push_back(t); at.push_back(i); }
-      };
-      add(x, 0);
-      for (size_t i = 0; i < n; ++i) add(own[i], 1 + i);
-      add(enc, 1 + n);
-      const auto got = torch::autograd::grad({y}, inputs, {grad[0]}, /*retain_graph=*/true, /*create_graph=*/true, /*allow_unused=*/true);
-      for (size_t i = 0; i < got.size(); ++i) out[at[i]] = got[i];
-      return out;
-    }
     Tensor gx, genc;
     Gradients g(own);
     {
@@ -707,7 +689,7 @@ struct Block : Function<Block> {
       g.weight(4, dy, self[8], p[4]);
       g.bias(5, dy, own[5]);
       Tensor dqkv, none;
-      if (!mask.defined() && (d == 64 || d == 128)) {
+      if (by_flash) {
         const auto [q, kk, v] = FlashPacked::parts(qkv);
         dqkv = std::get<3>(lb_ops::attn_bwd(dctx.view({B, S, heads, d}).permute({0, 2, 1, 3}), q, kk, v, self[8].view({B, S, heads, d}).permute({0, 2, 1, 3}), self[4],
                                             causal, scales[0], opt(self[5]), {}, {}, {}, 0.0, {}));
@@ -726,10 +708,6 @@ struct Block : Function<Block> {
     for (size_t i = 0; i < n; ++i) out[1 + i] = g.out[i];
     if (genc.defined()) out[1 + n] = genc.view(enc.sizes());
     return out;
-  }
-  static Opt flash_lens(const variable_list& s, size_t n, const Tensor& mask) {
-    // (the flash kernels' saved tensors: log-sum-exp, lengths; the others': fp32 result, log-sum-exp)
-    return s[n + 2 + 5].defined() && s[n + 2 + 5].scalar_type() == at::kInt && !mask.defined() ? Opt(s[n + 2 + 5]) : Opt();
   }
 };
 
@@ -761,27 +739,18 @@ struct LlamaBlock : Function<LlamaBlock> {
     hold_parameters(ctx, p);
     ctx->saved_data["n"] = static_cast<int64_t>(p.size());
     ctx->saved_data["heads"] = heads;
-    ctx->saved_data["eps"] = std::vector<double>{eps1, eps2, scale};
+    ctx->saved_data["scale"] = scale;
     return y.view(x.sizes());
   }
   static variable_list backward(AutogradContext* ctx, variable_list grad) {
     auto s = ctx->get_saved_variables();
     const size_t n = ctx->saved_data["n"].toInt();
     const int64_t heads = ctx->saved_data["heads"].toInt();
-    const auto eps = ctx->saved_data["eps"].toDoubleVector();
+    const double scale = ctx->saved_data["scale"].toDouble();
     const variable_list p(s.begin(), s.begin() + n);
     const Tensor &x = s[n], &cos = s[n + 1], &sin = s[n + 2], *k = &s[n + 3];
     variable_list out(n + 7);              // x, parameters, cos, sin, heads, eps, eps, scale
     const std::vector<Tensor> own = held_parameters(ctx);
-    if (at::GradMode::is_enabled()) {
-      const Tensor y = llama_of_nodes(x, at::TensorList(own.data(), 7), n > 7 ? Opt(own[7]) : Opt(), cos, sin, heads, eps[0], eps[1], eps[2]);
-      variable_list inputs(own);
-      if (x.requires_grad()) inputs.push_back(x);
-      const auto got = torch::autograd::grad({y}, inputs, {grad[0]}, /*retain_graph=*/true, /*create_graph=*/true, /*allow_unused=*/true);
-      for (size_t i = 0; i < n; ++i) out[1 + i] = got[i];
-      if (x.requires_grad()) out[0] = got[n];
-      return out;
-    }
     Tensor gx;
     Gradients g(own);
     {
@@ -807,7 +776,7 @@ struct LlamaBlock : Function<LlamaBlock> {
       g.weight(2, dy, k[4], p[2]);
       const auto [q, kk, v] = FlashPacked::parts(k[2]);
       Tensor dqkv = std::get<3>(lb_ops::attn_bwd(dctx.view({B, S, heads, d}).permute({0, 2, 1, 3}), q, kk, v, k[4].view({B, S, heads, d}).permute({0, 2, 1, 3}), k[3],
-                                                 true, eps[2], {}, {}, {}, {}, 0.0, {}));
+                                                 true, scale, {}, {}, {}, {}, 0.0, {}));
       dqkv = lb_ops::rope_qkv(dqkv.view({B, S, heads, 3 * d}), cos, sin, 0, true, true).view({T, 3 * ad});
       const Tensor dln1 = input_grad(dqkv, p[1]);
       g.weight(1, dqkv, k[0], p[1]);

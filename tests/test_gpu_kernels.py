@@ -1293,6 +1293,32 @@ def test_block_graph_takes_biases_that_changed_in_between(kind, dim):
     assert inputs[0].grad is not None
 
 
+@pytest.mark.parametrize("kind,dim", [("causal", 64), ("causal-prefix", 48), ("decoder", 32), ("llama", 128)])
+def test_block_gradients_with_create_graph_are_constants(kind, dim):
+    """As one node, with a node per operator and from the Python functions: the gradients of an ordinary pass, without a graph of their own."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Look(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    for how in ("block", "nodes", "python"):
+        layer, call, inputs = _train_block(kind, dim, False)
+        if how == "nodes":
+            layer.input_layernorm.register_forward_hook(lambda *a: None)
+        if how == "python":
+            with Look():
+                y = call()
+        else:
+            y = call()
+        params = [p for p in layer.parameters() if getattr(p, "main_grad", None) is None]
+        gy = _rand(y.shape, 5)
+        got = torch.autograd.grad(y, inputs + params, gy, create_graph=True)
+        want = torch.autograd.grad(y, inputs + params, gy)
+        for a, b in zip(got, want):
+            assert not a.requires_grad and float((a.double() - b.double()).norm()) <= 2.0 ** -7 * float(b.double().norm()), how
+
+
 def test_block_graph_refuses_what_changed_in_between():
     layer, call, inputs = _train_block("causal", 64, True)
     y = call()
