@@ -78,8 +78,8 @@ int64_t bits(std::initializer_list<bool> need) {
   for (bool b : need) m |= static_cast<int64_t>(b) << i++;
   return m;
 }
-// A block's parameters themselves, whose main_grad is asked for: what is unpacked may be a copy (checkpointing, saved-tensor hooks).  Like the Python functions, save_for_backward
-// gets the weights of norms and linear layers only; biases, and the weights of a gated MLP, which have to lie in one buffer, do not go through hooks.
+// A block's parameters themselves, whose main_grad is asked for: what is unpacked may be a copy (checkpointing, saved-tensor hooks).  As with the Python functions only the weights of
+// norms and linear layers are saved tensors too; biases, and the weights of a gated MLP, which have to lie in one buffer, do not go through hooks.
 void hold_parameters(AutogradContext* ctx, at::TensorList p) { ctx->saved_data["params"] = c10::List<Tensor>(p); }
 std::vector<Tensor> held_parameters(AutogradContext* ctx) { return ctx->saved_data["params"].toTensorVector(); }
 bool wants(AutogradContext* ctx, int i) { return (ctx->saved_data["need"].toInt() >> i) & 1; }
@@ -502,27 +502,28 @@ Tensor llama_of_nodes(const Tensor& x, at::TensorList p, const Opt& bias, const 
 struct Gradients {                        // of the parameters, by index
   std::vector<Tensor> main, out;          // main_grad, or undefined; what goes back to the engine
   std::vector<char> added;
-  explicit Gradients(at::TensorList p) : main(p.size()), out(p.size()), added(p.size(), 0) {
+  const std::vector<Tensor>& params;
+  explicit Gradients(const std::vector<Tensor>& p) : main(p.size()), out(p.size()), added(p.size(), 0), params(p) {
     pybind11::gil_scoped_acquire gil;
     for (size_t i = 0; i < p.size(); ++i) main[i] = main_grad(p[i]);
   }
-  void weight(size_t i, const Tensor& g, const Tensor& x, const Tensor& w) {
+  void weight(size_t i, const Tensor& g, const Tensor& x) {
     count(1);
     if (main[i].defined()) {
       lb_ops::gemm(g, x, 2, {}, main[i], true, at::kFloat);
       added[i] = 1;
     } else {
-      out[i] = lb_ops::gemm(g, x, 2, {}, {}, false, at::kFloat).to(w.scalar_type());
+      out[i] = lb_ops::gemm(g, x, 2, {}, {}, false, at::kFloat).to(params[i].scalar_type());
     }
   }
-  void bias(size_t i, const Tensor& g, const Tensor& b) {
+  void bias(size_t i, const Tensor& g) {
     if (added[i]) return;
     count(1);
     if (fp32(main[i])) {
       lb_ops::colsum(g, main[i]);
       added[i] = 1;
     } else {
-      out[i] = lb_ops::colsum(g, {}).to(b.scalar_type());
+      out[i] = lb_ops::colsum(g, {}).to(params[i].scalar_type());
     }
   }
   // gradient of the norm's input, `skip` added; the norm's parameters are i and, with has_bias, i + 1
@@ -552,10 +553,10 @@ struct Gradients {                        // of the parameters, by index
     }
     return norm(i, g, x, w, mean, rstd, false, true, skip);
   }
-  void mark(at::TensorList p) const {
+  void mark() const {
     pybind11::gil_scoped_acquire gil;
-    for (size_t i = 0; i < p.size(); ++i)
-      if (added[i]) mark_added(p[i]);
+    for (size_t i = 0; i < params.size(); ++i)
+      if (added[i]) mark_added(params[i]);
   }
 };
 Tensor input_grad(const Tensor& g, const Tensor& w) {
@@ -563,26 +564,73 @@ Tensor input_grad(const Tensor& g, const Tensor& w) {
   return lb_ops::gemm(g, w, 1, {}, {}, false, at::kBFloat16);
 }
 
+// What a block's backward pass needs of its forward pass.  A tensor goes through saved-tensor hooks and the check of its version as save_for_backward sends it, but alone and as
+// soon as it is there: hooks that take it elsewhere free it then, and the backward pass unpacks it where it is used and, unless the graph is kept, lets go of it behind that, as the
+// engine does between the nodes of single operators.  Peak of a step of 4 x 1024 tokens, MiB, all saved at once and unpacked at once -> so (a node per operator): GPT-2 block of width
+// 1024 233 -> 168 (176), 16 heads of 48 271 -> 174 (174), T5 decoder 313 -> 179 (185), Llama block 272 -> 182 (212); forward under checkpointing hooks 128 -> 80 (88).
+struct Kept : torch::CustomClassHolder {
+  std::vector<torch::autograd::SavedVariable> at;
+};
+class Keep {
+ public:
+  Keep(AutogradContext* ctx, size_t n) : kept_(c10::make_intrusive<Kept>()), outside_(c10::impl::tls_local_dispatch_key_set()) {
+    kept_->at.resize(n);
+    ctx->saved_data["kept"] = c10::IValue::make_capsule(kept_);
+  }
+  const Tensor& operator()(size_t i, const Tensor& t) {
+    c10::impl::ForceDispatchKeyGuard as_outside(outside_);              // (hooks run whatever they like)
+    kept_->at[i] = torch::autograd::SavedVariable(t, /*is_output=*/false);
+    return t;
+  }
+
+ private:
+  c10::intrusive_ptr<Kept> kept_;
+  const c10::impl::LocalDispatchKeySet outside_;
+};
+class Take {
+ public:
+  explicit Take(AutogradContext* ctx)
+      : kept_(c10::static_intrusive_pointer_cast<Kept>(ctx->saved_data["kept"].toCapsule())), outside_(c10::impl::tls_local_dispatch_key_set()),
+        keep_graph_(torch::autograd::get_current_graph_task_keep_graph()) {
+    ctx->get_saved_variables();                                         // (none; raises where an earlier pass has let go of what was kept)
+  }
+  Tensor operator()(size_t i) {                                         // once per pass: checkpointing hooks allow no more
+    c10::impl::ForceDispatchKeyGuard as_outside(outside_);
+    Tensor t = kept_->at[i].unpack();
+    if (!keep_graph_) kept_->at[i].reset_data();
+    return t;
+  }
+
+ private:
+  const c10::intrusive_ptr<Kept> kept_;
+  const c10::impl::LocalDispatchKeySet outside_;
+  const bool keep_graph_;
+};
+
 struct Block : Function<Block> {
+  // a norm's weight, result, mean and reciprocal deviation; the weights of products with what they read; attention: o32, log-sum-exp, mask words and fill, or of the flash
+  // kernels log-sum-exp and lengths
+  enum : size_t {
+    X, ENC, NORM1, QKV_W = NORM1 + 4, QKV, ATT, CTX = ATT + 4, O_W, Y1, NORMC, Q_W = NORMC + 4, Q, KV_W, KV, CATT, CCTX = CATT + 4, CO_W, Y2, NORM2, FF1_W = NORM2 + 4, PRE, FF2_W, ACT, KEPT
+  };
   static Tensor forward(AutogradContext* ctx, const Tensor& x, at::TensorList p, const Opt& enc, const BlockArgs& a) {
     const int64_t B = x.size(0), S = x.size(1), h = x.size(2), T = B * S, ad = p[2].size(0) / 3, d = ad / a.heads;
     const size_t m = has(enc) ? 14 : 6;
-    variable_list keep(p.begin(), p.end());
-    for (size_t i = 1; i < p.size(); i += 2) keep[i] = Tensor();       // biases
-    keep.push_back(x);
-    keep.push_back(has(enc) ? *enc : Tensor());
+    Keep keep(ctx, KEPT);
+    keep(X, x);
     Tensor y;
     {
       at::AutoDispatchBelowADInplaceOrView guard;
-      auto save = [&](const Tensor& t) { keep.push_back(t); return t; };
-      auto norm = [&](const Tensor& t, size_t i, double eps) {
+      auto norm = [&](const Tensor& t, size_t i, double eps, size_t to) {
         auto [ln, mean, rstd] = lb_ops::norm_fwd(t, p[i], p[i + 1], eps, false);
-        keep.insert(keep.end(), {ln, mean, rstd});
+        keep(to, p[i]);
+        keep(to + 1, ln);
+        keep(to + 2, mean);
+        keep(to + 3, rstd);
         return ln;
       };
-      const Tensor x2 = x.view({T, h});
-      const Tensor qkv = save(std::get<0>(lb_ops::linear_fwd(norm(x2, 0, a.eps[0]), p[2], p[3], 0, false))).view({B, S, a.heads, 3 * d});
-      auto attend = [&](const Tensor& q, const Tensor& k, const Tensor& v, bool causal, double scale, const Opt& mask) {       // saves o32, lse, words, fill
+      auto linear = [&](const Tensor& t, size_t i, size_t to) { return keep(to + 1, std::get<0>(lb_ops::linear_fwd(t, keep(to, p[i]), p[i + 1], 0, false))); };
+      auto attend = [&](const Tensor& q, const Tensor& k, const Tensor& v, bool causal, double scale, const Opt& mask, size_t to) {
         Tensor words, fill;
         if (has(mask)) {
           Tensor w = *mask;
@@ -591,37 +639,47 @@ struct Block : Function<Block> {
           count(1);
         }
         auto [o, o32, lse] = lb_ops::attn_split_fwd(q, k, v, causal && !has(mask), scale, opt(words), opt(fill), true);
-        keep.insert(keep.end(), {o32, lse, words, fill});
+        keep(to, o32);
+        keep(to + 1, lse);
+        keep(to + 2, words);
+        keep(to + 3, fill);
         return o;
       };
-      Tensor o;
-      if (flash(a, d)) {
-        const auto [q, k, v] = FlashPacked::parts(qkv);
-        auto [f, lse, rng] = lb_ops::attn_fwd(q, k, v, a.causal, a.scale, a.kv_lens, {}, {}, 0.0, 0);
-        keep.insert(keep.end(), {lse, a.kv_lens.value_or(Tensor()), Tensor(), Tensor()});
-        o = f;
-      } else {
-        const auto [q, k, v] = SplitAttention::parts(0, qkv, {}, {});
-        o = attend(q, k, v, a.causal, a.scale, a.mask);
+      const Tensor x2 = x.view({T, h});
+      {
+        const Tensor qkv = linear(norm(x2, 0, a.eps[0], NORM1), 2, QKV_W).view({B, S, a.heads, 3 * d});
+        Tensor o;
+        if (flash(a, d)) {
+          const auto [q, k, v] = FlashPacked::parts(qkv);
+          auto [f, lse, rng] = lb_ops::attn_fwd(q, k, v, a.causal, a.scale, a.kv_lens, {}, {}, 0.0, 0);
+          keep(ATT, lse);
+          if (has(a.kv_lens)) keep(ATT + 1, *a.kv_lens);
+          o = f;
+        } else {
+          const auto [q, k, v] = SplitAttention::parts(0, qkv, {}, {});
+          o = attend(q, k, v, a.causal, a.scale, a.mask, ATT);
+        }
+        const Tensor c = keep(CTX, o.permute({0, 2, 1, 3}).view({T, ad}));
+        y = keep(Y1, lb_ops::linear_bias_residual(c, keep(O_W, p[4]), p[5], x2));
       }
-      const Tensor c = save(o.permute({0, 2, 1, 3}).view({T, ad}));
-      y = save(lb_ops::linear_bias_residual(c, p[4], p[5], x2));
       if (has(enc)) {
-        const Tensor e2 = enc->view({-1, h});
-        const Tensor q = save(std::get<0>(lb_ops::linear_fwd(norm(y, 6, a.eps[1]), p[8], p[9], 0, false))).view({B, S, a.heads, d});
-        const Tensor kv = save(std::get<0>(lb_ops::linear_fwd(e2, p[10], p[11], 0, false))).view({B, -1, a.heads, 2 * d});
-        const auto [q4, k4, v4] = SplitAttention::parts(1, q, kv, {});
-        const Tensor cc = save(attend(q4, k4, v4, false, a.cross_scale, a.cross_mask).permute({0, 2, 1, 3}).view({T, ad}));
-        y = save(lb_ops::linear_bias_residual(cc, p[12], p[13], y));
+        Tensor cc;
+        {
+          const Tensor q = linear(norm(y, 6, a.eps[1], NORMC), 8, Q_W).view({B, S, a.heads, d});
+          const Tensor kv = linear(keep(ENC, *enc).view({-1, h}), 10, KV_W).view({B, -1, a.heads, 2 * d});
+          const auto [q4, k4, v4] = SplitAttention::parts(1, q, kv, {});
+          cc = keep(CCTX, attend(q4, k4, v4, false, a.cross_scale, a.cross_mask, CATT).permute({0, 2, 1, 3}).view({T, ad}));
+        }
+        y = keep(Y2, lb_ops::linear_bias_residual(cc, keep(CO_W, p[12]), p[13], y));
         count(5);
       }
-      auto [act, pre] = lb_ops::linear_fwd(norm(y, m, a.eps.back()), p[m + 2], p[m + 3], 1 /* GELU */, true);
-      save(pre);
-      save(act);
-      y = lb_ops::linear_bias_residual(act, p[m + 4], p[m + 5], y);
+      auto [act, pre] = lb_ops::linear_fwd(norm(y, m, a.eps.back(), NORM2), keep(FF1_W, p[m + 2]), p[m + 3], 1 /* GELU */, true);
+      keep(PRE, pre);
+      keep(ACT, act);
+      pre = Tensor();
+      y = lb_ops::linear_bias_residual(act, keep(FF2_W, p[m + 4]), p[m + 5], y);
       count(7);
     }
-    ctx->save_for_backward(std::move(keep));
     hold_parameters(ctx, p);
     ctx->saved_data["heads"] = a.heads;
     ctx->saved_data["scales"] = std::vector<double>{a.scale, a.cross_scale};
@@ -630,162 +688,197 @@ struct Block : Function<Block> {
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grad) {
-    auto s = ctx->get_saved_variables();
+    Take take(ctx);
     const int64_t flags = ctx->saved_data["flags"].toInt(), heads = ctx->saved_data["heads"].toInt();
     const bool causal = flags & 1, fuse = flags & 2, cross = flags & 4, by_flash = flags & 16;
-    const size_t m = cross ? 14 : 6, n = m + 6;
-    const variable_list p(s.begin(), s.begin() + n);
+    const size_t m = cross ? 14 : 6;
     const auto scales = ctx->saved_data["scales"].toDoubleVector();
-    const Tensor &x = s[n], &enc = s[n + 1];
-    variable_list out(n + 3);              // x, parameters, enc, arguments
-    const std::vector<Tensor> own = held_parameters(ctx);
+    const std::vector<Tensor> p = held_parameters(ctx);
+    const std::vector<int64_t> sizes = grad[0].sizes().vec();
+    Gradients g(p);
     Tensor gx, genc;
-    Gradients g(own);
     {
       at::AutoDispatchBelowADInplaceOrView guard;
-      const int64_t B = x.size(0), S = x.size(1), h = x.size(2), T = B * S, ad = p[2].size(0) / 3, d = ad / heads;
-      const Tensor* k = &s[n + 2];         // ln, mean, rstd; qkv; o32, lse, words, fill or lse, lengths, -, -; context; y [ln, mean, rstd; q, kv; ..]; ln, mean, rstd; pre; h
-      const Tensor *self = k, *cr = cross ? k + 10 : nullptr, *ff = cross ? k + 21 : k + 10;
-      const Tensor x2 = x.view({T, h}), gy = rows(grad[0]);
-      const bool fused = fuse && fp32(g.main[m + 3]) && g.main[m + 3].is_contiguous();
-      const Tensor dpre = lb_ops::dgrad_actgrad(gy, p[m + 4], ff[3], 1, fused ? Opt(g.main[m + 3]) : Opt());
-      count(1);
-      g.weight(m + 4, gy, ff[4], p[m + 4]);
-      g.weight(m + 2, dpre, ff[0], p[m + 2]);
-      if (fused) g.added[m + 3] = 1;
-      else g.bias(m + 3, dpre, own[m + 3]);
-      Tensor dln = input_grad(dpre, p[m + 2]);
-      Tensor dy = g.norm_and_biases(m, dln, cross ? cr[10] : self[9], p[m], ff[1], ff[2], gy, cross ? 13 : 5, static_cast<int>(m) + 5);
-      g.bias(m + 5, gy, own[m + 5]);
-      auto attend_back = [&](int64_t layout, const Tensor& t0, const Tensor& t1, const Tensor& dctx, const Tensor* kept, bool causal_, double scale, Tensor& g0,
-                             Tensor& g1) {
+      const int64_t B = sizes[0], S = sizes[1], h = sizes[2], T = B * S, ad = p[2].size(0) / 3, d = ad / heads;
+      Tensor gy = rows(grad[0]), dln;
+      grad.clear();
+      {
+        const bool fused = fuse && fp32(g.main[m + 3]) && g.main[m + 3].is_contiguous();
+        const Tensor dpre = lb_ops::dgrad_actgrad(gy, take(FF2_W), take(PRE), 1, fused ? Opt(g.main[m + 3]) : Opt());
+        count(1);
+        g.weight(m + 4, gy, take(ACT));
+        g.weight(m + 2, dpre, take(NORM2 + 1));
+        if (fused) g.added[m + 3] = 1;
+        else g.bias(m + 3, dpre);
+        dln = input_grad(dpre, take(FF1_W));
+      }
+      Tensor dy = g.norm_and_biases(m, dln, take(cross ? Y2 : Y1), take(NORM2), take(NORM2 + 2), take(NORM2 + 3), gy, cross ? 13 : 5, static_cast<int>(m) + 5);
+      g.bias(m + 5, gy);
+      gy = dln = Tensor();
+      auto attend_back = [&](int64_t layout, const Tensor& t0, const Tensor& t1, const Tensor& dctx, size_t kept, bool causal_, double scale, Tensor& g0, Tensor& g1) {
         g0 = at::empty(t0.sizes(), t0.options());
         if (layout == 1) g1 = at::empty(t1.sizes(), t1.options());
         const auto [q, kk, v] = SplitAttention::parts(layout, t0, t1, {});
         const auto [gq, gk, gv] = SplitAttention::parts(layout, g0, g1, {});
-        lb_ops::attn_split_bwd(dctx.view({B, S, heads, d}).permute({0, 2, 1, 3}), q, kk, v, kept[0], kept[1], gq, gk, gv, causal_ && !kept[2].defined(), scale,
-                               opt(kept[2]), opt(kept[3]));
+        const Tensor words = take(kept + 2);
+        lb_ops::attn_split_bwd(dctx.view({B, S, heads, d}).permute({0, 2, 1, 3}), q, kk, v, take(kept), take(kept + 1), gq, gk, gv, causal_ && !words.defined(), scale,
+                               opt(words), opt(take(kept + 3)));
         count(3);
       };
       if (cross) {
-        const Tensor q = cr[3].view({B, S, heads, d}), kv = cr[4].view({B, -1, heads, 2 * d}), e2 = enc.view({-1, h});
-        const Tensor dctx = input_grad(dy, p[12]);
-        g.weight(12, dy, cr[9], p[12]);
-        g.bias(13, dy, own[13]);
         Tensor gq, gkv;
-        attend_back(1, q, kv, dctx, cr + 5, false, scales[1], gq, gkv);
+        {
+          const Tensor dctx = input_grad(dy, take(CO_W));
+          g.weight(12, dy, take(CCTX));
+          g.bias(13, dy);
+          attend_back(1, take(Q).view({B, S, heads, d}), take(KV).view({B, -1, heads, 2 * d}), dctx, CATT, false, scales[1], gq, gkv);
+        }
         gq = gq.view({T, ad});
         gkv = gkv.view({-1, 2 * ad});
-        if (flags & 8) genc = input_grad(gkv, p[10]);
-        g.weight(10, gkv, e2, p[10]);
-        g.bias(11, gkv, own[11]);
-        dln = input_grad(gq, p[8]);
-        g.weight(8, gq, cr[0], p[8]);
-        g.bias(9, gq, own[9]);
-        dy = g.norm_and_biases(6, dln, self[9], p[6], cr[1], cr[2], dy, 5, -1);
+        const Tensor kv_w = take(KV_W);
+        if (flags & 8) genc = input_grad(gkv, kv_w).view({B, -1, h});
+        g.weight(10, gkv, take(ENC).view({-1, h}));
+        g.bias(11, gkv);
+        gkv = Tensor();
+        dln = input_grad(gq, take(Q_W));
+        g.weight(8, gq, take(NORMC + 1));
+        g.bias(9, gq);
+        gq = Tensor();
+        dy = g.norm_and_biases(6, dln, take(Y1), take(NORMC), take(NORMC + 2), take(NORMC + 3), dy, 5, -1);
+        dln = Tensor();
       }
-      const Tensor qkv = self[3].view({B, S, heads, 3 * d});
-      const Tensor dctx = input_grad(dy, p[4]);
-      g.weight(4, dy, self[8], p[4]);
-      g.bias(5, dy, own[5]);
       Tensor dqkv, none;
-      if (by_flash) {
-        const auto [q, kk, v] = FlashPacked::parts(qkv);
-        dqkv = std::get<3>(lb_ops::attn_bwd(dctx.view({B, S, heads, d}).permute({0, 2, 1, 3}), q, kk, v, self[8].view({B, S, heads, d}).permute({0, 2, 1, 3}), self[4],
-                                            causal, scales[0], opt(self[5]), {}, {}, {}, 0.0, {}));
-        count(3);
-      } else {
-        attend_back(0, qkv, {}, dctx, self + 4, causal, scales[0], dqkv, none);
+      {
+        const Tensor dctx = input_grad(dy, take(O_W));
+        Tensor c = take(CTX);
+        g.weight(4, dy, c);
+        g.bias(5, dy);
+        if (!by_flash) c = Tensor();
+        const Tensor qkv = take(QKV).view({B, S, heads, 3 * d});
+        if (by_flash) {
+          const auto [q, kk, v] = FlashPacked::parts(qkv);
+          dqkv = std::get<3>(lb_ops::attn_bwd(dctx.view({B, S, heads, d}).permute({0, 2, 1, 3}), q, kk, v, c.view({B, S, heads, d}).permute({0, 2, 1, 3}), take(ATT), causal,
+                                              scales[0], opt(take(ATT + 1)), {}, {}, {}, 0.0, {}));
+          count(3);
+        } else {
+          attend_back(0, qkv, {}, dctx, ATT, causal, scales[0], dqkv, none);
+        }
       }
       dqkv = dqkv.view({T, 3 * ad});
-      dln = input_grad(dqkv, p[2]);
-      g.weight(2, dqkv, self[0], p[2]);
-      g.bias(3, dqkv, own[3]);
-      gx = g.norm(0, dln, x2, p[0], self[1], self[2], false, true, dy);
+      dln = input_grad(dqkv, take(QKV_W));
+      g.weight(2, dqkv, take(NORM1 + 1));
+      g.bias(3, dqkv);
+      dqkv = Tensor();
+      gx = g.norm(0, dln, take(X).view({T, h}), take(NORM1), take(NORM1 + 2), take(NORM1 + 3), false, true, dy);
     }
-    g.mark(own);
-    out[0] = gx.view(x.sizes());
+    g.mark();
+    const size_t n = p.size();
+    variable_list out(n + 3);              // x, parameters, enc, arguments
+    out[0] = gx.view(sizes);
     for (size_t i = 0; i < n; ++i) out[1 + i] = g.out[i];
-    if (genc.defined()) out[1 + n] = genc.view(enc.sizes());
+    out[1 + n] = genc;
     return out;
   }
 };
 
 // Llama block, head dim 64 or 128: parameters norm; qkv; projection; norm; gate, up (one behind the other in memory), down[; bias of qkv]
 struct LlamaBlock : Function<LlamaBlock> {
+  enum : size_t { X, COS, SIN, NORM1, QKV_W = NORM1 + 4, QKV, LSE, CTX, O_W, Y1, NORM2, GU = NORM2 + 4, ACT, KEPT };       // (norms as in Block)
   static Tensor forward(AutogradContext* ctx, const Tensor& x, at::TensorList p, const Tensor& cos, const Tensor& sin, int64_t heads, double eps1, double eps2,
                         double scale) {
     const int64_t B = x.size(0), S = x.size(1), h = x.size(2), T = B * S, ad = p[1].size(0) / 3, d = ad / heads;
-    variable_list keep(p.begin(), p.end());
-    for (size_t i = 4; i < p.size(); ++i) keep[i] = Tensor();          // gate, up, down, bias of qkv
-    keep.insert(keep.end(), {x, cos, sin});
+    Keep keep(ctx, KEPT);
+    keep(X, x);
+    keep(COS, cos);
+    keep(SIN, sin);
     Tensor y;
     {
       at::AutoDispatchBelowADInplaceOrView guard;
+      auto norm = [&](const Tensor& t, size_t i, double eps, size_t to) {
+        auto [ln, mean, rstd] = lb_ops::norm_fwd(t, p[i], {}, eps, true);
+        keep(to, p[i]);
+        keep(to + 1, ln);
+        keep(to + 2, mean);
+        keep(to + 3, rstd);
+        return ln;
+      };
       const Tensor x2 = x.view({T, h});
-      auto [ln1, none1, rstd1] = lb_ops::norm_fwd(x2, p[0], {}, eps1, true);
-      const Tensor raw = std::get<0>(lb_ops::linear_fwd(ln1, p[1], p.size() > 7 ? Opt(p[7]) : Opt(), 0, false)).view({B, S, heads, 3 * d});
-      const Tensor qkv = lb_ops::rope_qkv(raw, cos, sin, 0, false, false);
-      const auto [q, k, v] = FlashPacked::parts(qkv);
-      auto [o, lse, rng] = lb_ops::attn_fwd(q, k, v, true, scale, {}, {}, {}, 0.0, 0);
-      const Tensor c = o.permute({0, 2, 1, 3}).view({T, ad}), y1 = lb_ops::linear_bias_residual(c, p[2], {}, x2);
-      auto [ln2, none2, rstd2] = lb_ops::norm_fwd(y1, p[3], {}, eps2, true);
-      const Tensor gu = lb_ops::gemm(ln2, stacked(p[4], p[5]), 0, {}, {}, false, at::kBFloat16), act = lb_ops::swiglu_packed_fwd(gu);
+      Tensor y1, act;
+      {
+        Tensor qkv = std::get<0>(lb_ops::linear_fwd(norm(x2, 0, eps1, NORM1), keep(QKV_W, p[1]), p.size() > 7 ? Opt(p[7]) : Opt(), 0, false)).view({B, S, heads, 3 * d});
+        qkv = keep(QKV, lb_ops::rope_qkv(qkv, cos, sin, 0, false, false));
+        const auto [q, k, v] = FlashPacked::parts(qkv);
+        auto [o, lse, rng] = lb_ops::attn_fwd(q, k, v, true, scale, {}, {}, {}, 0.0, 0);
+        keep(LSE, lse);
+        y1 = keep(Y1, lb_ops::linear_bias_residual(keep(CTX, o.permute({0, 2, 1, 3}).view({T, ad})), keep(O_W, p[2]), {}, x2));
+      }
+      {
+        const Tensor gu = keep(GU, lb_ops::gemm(norm(y1, 3, eps2, NORM2), stacked(p[4], p[5]), 0, {}, {}, false, at::kBFloat16));
+        act = keep(ACT, lb_ops::swiglu_packed_fwd(gu));
+      }
       y = lb_ops::linear_bias_residual(act, p[6], {}, y1);
-      keep.insert(keep.end(), {ln1, rstd1, qkv, lse, c, y1, ln2, rstd2, gu, act, none1});
       count(9);
     }
-    ctx->save_for_backward(std::move(keep));
     hold_parameters(ctx, p);
-    ctx->saved_data["n"] = static_cast<int64_t>(p.size());
     ctx->saved_data["heads"] = heads;
     ctx->saved_data["scale"] = scale;
     return y.view(x.sizes());
   }
   static variable_list backward(AutogradContext* ctx, variable_list grad) {
-    auto s = ctx->get_saved_variables();
-    const size_t n = ctx->saved_data["n"].toInt();
+    Take take(ctx);
     const int64_t heads = ctx->saved_data["heads"].toInt();
     const double scale = ctx->saved_data["scale"].toDouble();
-    const variable_list p(s.begin(), s.begin() + n);
-    const Tensor &x = s[n], &cos = s[n + 1], &sin = s[n + 2], *k = &s[n + 3];
-    variable_list out(n + 7);              // x, parameters, cos, sin, heads, eps, eps, scale
-    const std::vector<Tensor> own = held_parameters(ctx);
+    const std::vector<Tensor> p = held_parameters(ctx);
+    const std::vector<int64_t> sizes = grad[0].sizes().vec();
+    const size_t n = p.size();
+    Gradients g(p);
     Tensor gx;
-    Gradients g(own);
     {
       at::AutoDispatchBelowADInplaceOrView guard;
-      const int64_t B = x.size(0), S = x.size(1), h = x.size(2), T = B * S, ad = p[1].size(0) / 3, d = ad / heads, f = own[4].size(0);
-      const Tensor x2 = x.view({T, h}), gy = rows(grad[0]), w = stacked(own[4], own[5]);
+      const int64_t B = sizes[0], S = sizes[1], h = sizes[2], T = B * S, ad = p[1].size(0) / 3, d = ad / heads, f = p[4].size(0);
+      const Tensor w = stacked(p[4], p[5]);
       TORCH_CHECK(w.defined(), "llama block: gate and up weights of one buffer");
-      const Tensor joint = fp32(g.main[4]) ? stacked(g.main[4], g.main[5]) : Tensor();
-      const Tensor dh = input_grad(gy, own[6]);
-      g.weight(6, gy, k[9], own[6]);
-      const Tensor dgu = lb_ops::swiglu_packed_bwd(dh, k[8]);
-      const Tensor dln2 = input_grad(dgu, w);
-      if (joint.defined()) {
-        lb_ops::gemm(dgu, k[6], 2, {}, joint, true, at::kFloat);
-        g.added[4] = g.added[5] = 1;
-      } else {
-        const Tensor both = lb_ops::gemm(dgu, k[6], 2, {}, {}, false, at::kFloat);
-        g.out[4] = both.narrow(0, 0, f).to(own[4].scalar_type());
-        g.out[5] = both.narrow(0, f, f).to(own[5].scalar_type());
+      Tensor gy = rows(grad[0]), dln;
+      grad.clear();
+      {
+        const Tensor joint = fp32(g.main[4]) ? stacked(g.main[4], g.main[5]) : Tensor();
+        Tensor dh = input_grad(gy, p[6]);
+        g.weight(6, gy, take(ACT));
+        const Tensor dgu = lb_ops::swiglu_packed_bwd(dh, take(GU));
+        dh = Tensor();
+        dln = input_grad(dgu, w);
+        const Tensor ln = take(NORM2 + 1);
+        if (joint.defined()) {
+          lb_ops::gemm(dgu, ln, 2, {}, joint, true, at::kFloat);
+          g.added[4] = g.added[5] = 1;
+        } else {
+          const Tensor both = lb_ops::gemm(dgu, ln, 2, {}, {}, false, at::kFloat);
+          g.out[4] = both.narrow(0, 0, f).to(p[4].scalar_type());
+          g.out[5] = both.narrow(0, f, f).to(p[5].scalar_type());
+        }
       }
-      const Tensor dy = g.norm(3, dln2, k[5], p[3], k[10], k[7], true, false, gy);
-      const Tensor dctx = input_grad(dy, p[2]);
-      g.weight(2, dy, k[4], p[2]);
-      const auto [q, kk, v] = FlashPacked::parts(k[2]);
-      Tensor dqkv = std::get<3>(lb_ops::attn_bwd(dctx.view({B, S, heads, d}).permute({0, 2, 1, 3}), q, kk, v, k[4].view({B, S, heads, d}).permute({0, 2, 1, 3}), k[3],
-                                                 true, scale, {}, {}, {}, {}, 0.0, {}));
+      const Tensor dy = g.norm(3, dln, take(Y1), take(NORM2), take(NORM2 + 2), take(NORM2 + 3), true, false, gy);
+      gy = dln = Tensor();
+      const Tensor cos = take(COS), sin = take(SIN);
+      Tensor dqkv;
+      {
+        const Tensor dctx = input_grad(dy, take(O_W)), c = take(CTX);
+        g.weight(2, dy, c);
+        const auto [q, kk, v] = FlashPacked::parts(take(QKV));
+        dqkv = std::get<3>(lb_ops::attn_bwd(dctx.view({B, S, heads, d}).permute({0, 2, 1, 3}), q, kk, v, c.view({B, S, heads, d}).permute({0, 2, 1, 3}), take(LSE), true, scale,
+                                            {}, {}, {}, {}, 0.0, {}));
+      }
       dqkv = lb_ops::rope_qkv(dqkv.view({B, S, heads, 3 * d}), cos, sin, 0, true, true).view({T, 3 * ad});
-      const Tensor dln1 = input_grad(dqkv, p[1]);
-      g.weight(1, dqkv, k[0], p[1]);
-      if (n > 7) g.bias(7, dqkv, own[7]);
-      gx = g.norm(0, dln1, x2, p[0], k[10], k[1], true, false, dy);
+      dln = input_grad(dqkv, take(QKV_W));
+      g.weight(1, dqkv, take(NORM1 + 1));
+      if (n > 7) g.bias(7, dqkv);
+      dqkv = Tensor();
+      gx = g.norm(0, dln, take(X).view({T, h}), take(NORM1), take(NORM1 + 2), take(NORM1 + 3), true, false, dy);
       count(6);                            // attention, rotation, SwiGLU, gate and up weights
     }
-    g.mark(own);
-    out[0] = gx.view(x.sizes());
+    g.mark();
+    variable_list out(n + 7);              // x, parameters, cos, sin, heads, eps, eps, scale
+    out[0] = gx.view(sizes);
     for (size_t i = 0; i < n; ++i) out[1 + i] = g.out[i];
     return out;
   }

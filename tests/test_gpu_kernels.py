@@ -1154,7 +1154,7 @@ def test_products_with_several_matrices_in_one_launch(m, k, ns):
     assert torch.equal(out[:, :total].float(), want) and bool((out[:, total:] == 3).all())
 
 
-def _train_block(kind, dim, with_main_grad):
+def _train_block(kind, dim, with_main_grad, s=40):
     """A block, its call and its inputs: causal, right-padded, without a mask, T5 decoder, Llama; causal with a mask of its own, which stands in the triangle's place (dense,
     padded on the left) or, in the flash kernels, beside it (right-padded)."""
     from libai_b200.layers import TransformerLayer
@@ -1163,11 +1163,11 @@ def _train_block(kind, dim, with_main_grad):
     from libai_b200.models.llama_model import LlamaDecoderLayer, rotary_tables
     from libai_b200.optim import AdamW, get_default_optimizer_params
 
-    heads, s = 4, 40
+    heads = 4
     hidden = heads * dim
     with param_defaults(dtype=BF16, device="cuda", seed=1):
         if kind == "llama":
-            layer = LlamaDecoderLayer(hidden, 256, heads, rms_norm_eps=1e-6, max_position_embeddings=64)
+            layer = LlamaDecoderLayer(hidden, 256, heads, rms_norm_eps=1e-6, max_position_embeddings=max(64, s))
         else:
             layer = TransformerLayer(hidden, 2 * hidden, heads, is_decoder=kind == "decoder",
                                      attn_mask_type=AttnMaskType.causal if kind.startswith("causal") else AttnMaskType.padding)
@@ -1178,7 +1178,7 @@ def _train_block(kind, dim, with_main_grad):
         opt.setup()
     x = _rand((3, s, hidden), 2).requires_grad_(True)
     if kind == "llama":
-        cos, sin = rotary_tables(dim, 64, device="cuda")
+        cos, sin = rotary_tables(dim, max(64, s), device="cuda")
         return layer, lambda: layer(x, cos_cached=cos, sin_cached=sin), [x]
     if kind == "decoder":
         enc = _rand((3, 24, hidden), 3).requires_grad_(True)
@@ -1317,6 +1317,37 @@ def test_block_gradients_with_create_graph_are_constants(kind, dim):
         want = torch.autograd.grad(y, inputs + params, gy)
         for a, b in zip(got, want):
             assert not a.requires_grad and float((a.double() - b.double()).norm()) <= 2.0 ** -7 * float(b.double().norm()), how
+
+
+@pytest.mark.parametrize("recompute", [False, True])
+@pytest.mark.parametrize("kind,dim", [("causal", 64), ("causal-prefix", 48), ("decoder", 48), ("llama", 128)])
+def test_block_graph_holds_no_more_than_its_operators(kind, dim, recompute):
+    """Peak of memory of a pass forward and one back, as one node and with a node per operator: what is saved goes when its operator is done (and with checkpointing hooks when it is made)."""
+    from torch.utils.checkpoint import checkpoint
+
+    peak = []
+    for how in ("nodes", "block"):
+        layer, call, inputs = _train_block(kind, dim, True, 512)
+        if how == "nodes":
+            layer.input_layernorm.register_forward_hook(lambda *a: None)
+        step = (lambda: checkpoint(lambda *_: call(), *inputs, use_reentrant=False)) if recompute else call
+        step().sum().backward()
+        for t in inputs:
+            t.grad = None
+        torch.cuda.synchronize()
+        base, peak_of = torch.cuda.memory_allocated(), []
+        torch.cuda.reset_peak_memory_stats()
+        y = step()
+        peak_of.append(torch.cuda.max_memory_allocated() - base)
+        gy = _rand(y.shape, 5)
+        torch.cuda.reset_peak_memory_stats()
+        y.backward(gy)
+        peak_of.append(torch.cuda.max_memory_allocated() - base)
+        peak.append(peak_of)
+        assert ("Block" in y.grad_fn.name()) == (how == "block")
+        del y, gy
+    unit = inputs[0].numel() * 2                  # a [tokens, width] tensor in bf16; statistics and the like apart
+    assert all(b <= n + unit / 4 for n, b in zip(*peak)), [[round(v / unit, 2) for v in p] for p in peak]
 
 
 def test_block_graph_refuses_what_changed_in_between():
