@@ -1181,14 +1181,17 @@ static int gemm_impl(const void* a, const void* b, void* out, int M, int N, int 
   const bool plain = cp.mode == lb::COMM_NONE && deq_a == nullptr && !tile_group;
   int bn = force_bn;
   bool pair = force_bn == 256;
+  const int forced = force_bn < 0 ? -force_bn : force_bn;
+  if (force_bn != 0 && forced != 256 && forced != 192 && forced != 128 && force_bn != 64) return -1;
   if (force_bn < 0) {                       // (timing: a pair's tile of that width)
-    bn = -force_bn;
+    bn = forced;
     pair = true;
   } else if (force_bn == 0 && epi == 2) {
     // split-K fills the machine for the accumulate (wgrad) epilogue: the widest tile that fits N, on pairs the width that is estimated best
     bn = N >= 192 ? 256 : (N >= 96 ? 128 : 64);
-    if (plain && pairs_ok && layout == 2 && N >= 96) bn = wgrad_tile_choice(M, N, K, sms);
-    pair = bn == 256 || (plain && pairs_ok && layout == 2 && N >= 96);
+    const bool narrow_pairs = plain && pairs_ok && layout == 2 && N >= 96 && !wgrad_rmw();       // (read-modify-write: 256 wide only)
+    if (narrow_pairs) bn = wgrad_tile_choice(M, N, K, sms);
+    pair = bn == 256 || narrow_pairs;
   } else if (force_bn == 0 && plain && epi == 0 && layout != 2) {
     tile_choice(M, N, K, layout == 1, &bn, &pair);
   } else if (force_bn == 0) {
@@ -1280,6 +1283,8 @@ static int gemm_impl(const void* a, const void* b, void* out, int M, int N, int 
   const bool comm_ok = cp.mode == lb::COMM_NONE ||
                        (cp.rows_per_rank % (2 * lb::BLOCK_M) == 0 && cp.n_comm % 2 == 0 && gemm_allow_2cta() >= 2);
   const bool two_cta = pair && pairs_ok && comm_ok;
+  // (there is no kernel of narrower pairs for the others, and the boxes of another width would bring fewer bytes than it waits for)
+  if (two_cta && bn != 256 && !(layout == 2 ? epi == 2 : epi == 0)) return -1;
   // Order of the tiles.  Row by row, the CTAs in flight hold one or two row blocks of A and up to 74 column blocks of B: a B that does
   // not stay in L2 beside the output is read from HBM again for (nearly) every row block (LM head [8192, 1024] x [50304, 1024]: 32 x
   // 103 MB).  In bands of G row blocks they hold G of A and C / G of B, the least bytes at equal sides: G = sqrt(C * columns / rows of a

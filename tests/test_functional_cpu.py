@@ -72,6 +72,16 @@ def test_norm_backward_never_drops_the_residual_gradient():
     assert lib.lb_norm_bwd_supports_gadd(512, 0, *aligned) == 1
 
 
+@pytest.mark.skipif(torch.cuda.is_available() or not os.path.exists(so_path()), reason="host side of the C entry only: no launch may follow")
+@pytest.mark.parametrize("width,layout,epi", [(-64, 0, 0), (-96, 2, 2), (100, 0, 0), (320, 1, 0), (-128, 0, 1), (-192, 0, 2), (-128, 1, 1), (-192, 1, 2), (-128, 2, 0), (-192, 2, 1)])
+def test_gemm_refuses_forced_widths_without_a_kernel(width, layout, epi):
+    """-1 before a tensor map is made (-2 where that has no driver): a 256-wide kernel on boxes of another width would wait for bytes that nobody sends."""
+    lib, p = ctypes.CDLL(so_path()), ctypes.c_void_p
+    call = lambda w, lay, e: lib.lb_gemm_bf16(p(0x10000), p(0x20000), p(0x30000), 512, 512, 512, 512, 512, 512, lay, e, p(0), 0, p(0), w, 1, p(0))
+    assert call(width, layout, epi) == -1
+    assert call(-256, layout, epi) == call(256, layout, epi) == call(64, layout, epi) == -2
+
+
 def test_implementation_switch_follows_the_environment(monkeypatch):
     monkeypatch.delenv("LIBAI_B200_IMPL", raising=False)
     assert ops.impl() == "native"
