@@ -954,11 +954,11 @@ bool make_tmap_bf16(CUtensorMap* out, const void* base, int rank, const uint64_t
 namespace {
 
 int g_num_sms = 0;
-int num_sms() {
+int num_sms() {                                   // (without a device the rules below answer for the chip they are fitted on)
   if (g_num_sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
+    g_num_sms = n;
   }
   return g_num_sms;
 }

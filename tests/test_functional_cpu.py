@@ -82,6 +82,13 @@ def test_gemm_refuses_forced_widths_without_a_kernel(width, layout, epi):
     assert call(-256, layout, epi) == call(256, layout, epi) == call(64, layout, epi) == -2
 
 
+@pytest.mark.skipif(torch.cuda.is_available() or not os.path.exists(so_path()), reason="host side of the C entry only")
+@pytest.mark.parametrize("m,n,k,few", [(8, 1024, 4096, 1), (200, 1024, 4096, 1), (128, 4096, 1024, 1), (2048, 4096, 1024, 0), (8192, 1024, 1024, 0)])
+def test_rule_of_few_rows_answers_without_a_device(m, n, k, few):
+    nt, ranks = ctypes.c_int(0), ctypes.c_int(0)
+    assert ctypes.CDLL(so_path()).lb_gemm_small_rule(m, n, k, ctypes.byref(nt), ctypes.byref(ranks)) == few
+
+
 def test_implementation_switch_follows_the_environment(monkeypatch):
     monkeypatch.delenv("LIBAI_B200_IMPL", raising=False)
     assert ops.impl() == "native"
