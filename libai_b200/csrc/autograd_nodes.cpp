@@ -28,7 +28,7 @@ using torch::autograd::Function;
 using torch::autograd::variable_list;
 using Opt = std::optional<Tensor>;
 
-std::atomic<int64_t> launches{0};       // kernels launched from here (ops.launch_count())
+std::atomic<int64_t> launches{0};       // kernels launched from here and by the blocks without a graph (ops.launch_count())
 void count(int64_t n) { launches.fetch_add(n, std::memory_order_relaxed); }
 
 // ---- attributes of parameters -----------------------------------------------------------------------------------

@@ -1120,11 +1120,13 @@ bool block_norm_linear(const void* x, const Tensor& gamma, const void* beta, dou
     const int rc = lb_gemm_small_norm(x, gamma.data_ptr(), beta, (float)eps, rms, w, y, (int)rows, (int)n, (int)h, (int)h, (int)h, (int)n, bias, act, cur_stream());
     if (rc != -1) {
       check(rc, "norm_linear");
+      lb_nodes::count(1);
       return true;
     }
   }
   check(lb_norm_fwd(x, gamma.data_ptr(), beta, tmp, rms ? nullptr : stats, rms ? stats : stats + rows, (int)rows, (int)h, (float)eps, rms, 0, 0, cur_stream()), "norm_fwd");
   check(lb_gemm_bf16(tmp, w, y, (int)rows, (int)n, (int)h, (int)h, (int)h, (int)n, 0, 0, bias, act, nullptr, 0, 0, cur_stream()), "linear_fwd");
+  lb_nodes::count(2);
   return false;
 }
 
@@ -1152,6 +1154,7 @@ std::vector<Tensor> block_fwd(const Tensor& x, const std::vector<Tensor>& p, int
   block_norm_linear(s(mid), p[6], p[7].data_ptr(), eps2, p[8].data_ptr(), f, h, p[9].data_ptr(), 1 /* GELU */, s(wide), T, s(norm), st);
   check(lb_gemm_bf16_bias_residual(s(wide), p[10].data_ptr(), out[0].data_ptr(), (int)T, (int)h, (int)f, (int)f, (int)f, p[11].data_ptr(), s(mid), cur_stream()),
         "linear_bias_residual");
+  lb_nodes::count(3);                    // beside the norms and the products behind them
   return out;
 }
 
@@ -1191,12 +1194,17 @@ std::vector<Tensor> llama_block_fwd(const Tensor& x, const std::vector<Tensor>& 
     check(lb_swiglu_packed_fwd(s(wide), s(rot), T, f, cur_stream()), "swiglu_packed_fwd");
   } else {
     char* up = s(wide) + T * f * 2;
-    if (project(4, f, s(wide))) project(5, f, up);
-    else block_linear(s(norm), p[5], nullptr, 0, up, T);
+    if (project(4, f, s(wide))) {
+      project(5, f, up);
+    } else {
+      block_linear(s(norm), p[5], nullptr, 0, up, T);
+      lb_nodes::count(1);
+    }
     check(lb_swiglu_fwd(s(wide), up, s(rot), T * f, cur_stream()), "swiglu_fwd");
   }
   check(lb_gemm_bf16_bias_residual(s(rot), p[6].data_ptr(), out[0].data_ptr(), (int)T, (int)h, (int)f, (int)f, (int)f, nullptr, s(mid), cur_stream()),
         "linear_bias_residual");
+  lb_nodes::count(5);                    // rotation, attention, two products, SwiGLU
   return out;
 }
 

@@ -5,6 +5,9 @@
 #include <tuple>
 #include <vector>
 
+namespace lb_nodes {
+void count(int64_t n);      // kernels launched from C++ (ops.launch_count())
+}
 namespace lb_ops {
 
 using at::Tensor;

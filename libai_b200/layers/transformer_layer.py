@@ -8,7 +8,7 @@ The pipeline hand-off the reference performs inside ``forward`` (``to_global(pla
 """
 from torch import nn
 
-from libai_b200.ops import count_launch, functional as OF, fused_bias_grad, load_ext
+from libai_b200.ops import functional as OF, fused_bias_grad, load_ext
 
 from . import _native_block as native
 from ._param import xavier_normal_
@@ -172,7 +172,6 @@ class TransformerLayer(nn.Module):
         out = load_ext().block_fwd(x, params, attn.local_heads, ln1.eps, ln2.eps, attn.softmax_scale, attn.attn_mask_type == AttnMaskType.causal, *pair)
         if not out:
             return None
-        count_launch(7)
         return (out[0], tuple(out[1:])) if use_cache else out[0]
 
     def _graph_forward(self, x, mask, enc, cross_mask):

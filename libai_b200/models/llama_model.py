@@ -25,7 +25,7 @@ from libai_b200.layers import _native_block as native
 from libai_b200.layers._param import xavier_normal_
 from libai_b200.layers.attention import AttnMaskType
 from libai_b200.layers.embedding import get_sp_shape, set_sp_shape
-from libai_b200.ops import count_launch, load_ext
+from libai_b200.ops import load_ext
 from libai_b200.ops import functional as OF
 from libai_b200.parallel import mappings
 from libai_b200.utils import distributed as dutil
@@ -288,7 +288,6 @@ class LlamaDecoderLayer(nn.Module):
         out = load_ext().llama_block_fwd(x, params, bias, cos, sin, attn.local_heads, ln1.eps, ln2.eps, attn.norm_factor, gated_mlp.enabled(), *pair)
         if not out:
             return None
-        count_launch(9)                 # one more where gate and up projection are two products
         return (out[0], tuple(out[1:])) if use_cache else out[0]
 
 

@@ -1448,3 +1448,32 @@ def test_norm_backward_with_the_biases_around_it(h, rows, which):
                            (sums[3], old[3], gx[:rows].double().sum(0) * (which != "behind"), gx[:rows].double().abs().sum(0))):
         # fp32 sums: a rounding of 2^-24 of the magnitudes per term of a chain of at most rows / 4, and of the normalised x (2^-20)
         assert bool(((got.double() - was - d).abs() <= (2.0 ** -20 + rows * 2.0 ** -26) * (n + was.abs() + 1)).all())
+
+
+@pytest.mark.parametrize("batch", [4, 40])
+@pytest.mark.parametrize("kind", ["gpt", "llama"])
+def test_launches_of_a_generation_step_are_counted(kind, batch):
+    """One kernel or two for a norm and the product behind it: the count is what the device ran."""
+    from libai_b200 import ops
+    from libai_b200.layers import TransformerLayer
+    from libai_b200.layers._param import param_defaults
+    from libai_b200.layers.attention import AttnMaskType
+    from libai_b200.models.llama_model import LlamaDecoderLayer, rotary_tables
+
+    with param_defaults(dtype=BF16, device="cuda", seed=1):
+        layer = (TransformerLayer(512, 2048, 8, attn_mask_type=AttnMaskType.causal) if kind == "gpt"
+                 else LlamaDecoderLayer(512, 1024, 8, rms_norm_eps=1e-6, max_position_embeddings=64)).eval()
+    x, past = _rand((batch, 1, 512), 1), (_rand((batch, 8, 20, 64), 2), _rand((batch, 8, 20, 64), 3))
+    kw = {}
+    if kind == "llama":
+        kw["cos_cached"], kw["sin_cached"] = rotary_tables(64, 64, device="cuda")
+    with torch.no_grad():
+        step = lambda: layer(x, past_key_value=past, use_cache=True, **kw)
+        step()
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+            before = ops.launch_count()
+            step()
+            counted = ops.launch_count() - before
+            torch.cuda.synchronize()
+    ran = sum(e.count for e in prof.key_averages() if "lb::" in e.key)
+    assert counted == ran > 0
