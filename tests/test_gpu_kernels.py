@@ -1,5 +1,6 @@
 """GPU tier: single kernels of the training path at the sizes where a tile, a remainder or a wait can go wrong, against plain PyTorch."""
 import ctypes
+import gc
 import math
 
 import pytest
@@ -1334,15 +1335,17 @@ def test_block_graph_holds_no_more_than_its_operators(kind, dim, recompute):
         step().sum().backward()
         for t in inputs:
             t.grad = None
+        gc.collect()                             # (what earlier tests left must not go in between)
         torch.cuda.synchronize()
-        base, peak_of = torch.cuda.memory_allocated(), []
+        stat = lambda which: torch.cuda.memory_stats()["requested_bytes.all." + which]       # (allocated ones count the whole of a cached block)
+        base, peak_of = stat("current"), []
         torch.cuda.reset_peak_memory_stats()
         y = step()
-        peak_of.append(torch.cuda.max_memory_allocated() - base)
+        peak_of.append(stat("peak") - base)
         gy = _rand(y.shape, 5)
         torch.cuda.reset_peak_memory_stats()
         y.backward(gy)
-        peak_of.append(torch.cuda.max_memory_allocated() - base)
+        peak_of.append(stat("peak") - base)
         peak.append(peak_of)
         assert ("Block" in y.grad_fn.name()) == (how == "block")
         del y, gy
