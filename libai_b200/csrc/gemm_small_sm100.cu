@@ -35,17 +35,22 @@ constexpr long GS_AHEAD_BYTES = 4 << 20;
 constexpr int GS_MAX_STAGES = GS_SMEM / GsCfg<16>::STAGE, GS_TAIL = 1024 + 512;   // alignment, barriers, statistics
 
 struct GemmSmallParams {
-  int M, N, K, kb_total, kb_per_cta, stages, ahead;
+  int M, N, K, kb_per_cta, stages, ahead;
   const __nv_bfloat16* bias;      // [N] or nullptr
   const __nv_bfloat16* residual;  // [M, ldo] or nullptr
   __nv_bfloat16 *out, *pre_out;   // [M, ldo]; pre_out (optional): before the activation
   int ldo, act;
   int* err;
-  // with a norm in front: rows of x as they are, its weight and bias (or nullptr)
+};
+// with a norm in front: rows of x as they are, its weight and bias (or nullptr)
+struct alignas(64) GemmSmallNormParams : GemmSmallParams {
   const __nv_bfloat16 *x, *gamma, *beta;
   int ldx, rms;
   float eps;
 };
+template <bool NORM> using GemmSmallArgs = std::conditional_t<NORM, GemmSmallNormParams, GemmSmallParams>;
+// (two tensor maps and these: what a launch costs the host depends on the bytes, see GemmReduce; 376 for both kinds took 3.7 us, 328 and 384 take 3.5)
+static_assert((sizeof(GemmSmallParams) + 7) % 64 < 16 && (sizeof(GemmSmallNormParams) + 7) % 64 < 16, "bytes of the arguments");
 
 // count, mean and sum of squared deviations of two sets of numbers together
 LB_DEVICE void merge_moments(float& n, float& mean, float& m2, float n2, float mean2, float m22) {
@@ -68,7 +73,7 @@ LB_DEVICE float4 gs_ld_remote(uint32_t addr, uint32_t rank) {
 // statistics (every CTA those of all its rows) and write the normalised bf16 rows of each k-block where TMA would have put them, while w is on its way.
 template <int NT, int RANKS, bool NORM>
 __global__ void __launch_bounds__(GS_THREADS, 2)
-gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, GemmSmallParams p) {
+gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, GemmSmallArgs<NORM> p) {
   using Cfg = GsCfg<NT>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -84,7 +89,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   const int warp_idx = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int rank = blockIdx.x;
   const int n0 = blockIdx.y * 128, m0 = blockIdx.z * NT;
-  const int kb0 = min(p.kb_total, rank * p.kb_per_cta), kb1 = min(p.kb_total, kb0 + p.kb_per_cta);
+  const int kb_total = (p.K + 63) / 64, kb0 = min(kb_total, rank * p.kb_per_cta), kb1 = min(kb_total, kb0 + p.kb_per_cta);
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmap_w);
@@ -103,7 +108,8 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   const uint32_t tmem_base = *tmem_ptr_smem;
   if (threadIdx.x == 32)                     // on its way to L2 while the kernel before this one ends; the warp whose own work begins last
     for (int kb = kb0; kb < min(kb1, kb0 + p.ahead); ++kb) tma_prefetch_2d(&tmap_w, kb * 64, n0);
-  const __nv_bfloat16 *xg = p.x, *gamma = p.gamma, *beta = p.beta;
+  [[maybe_unused]] const __nv_bfloat16 *xg = nullptr, *gamma = nullptr, *beta = nullptr;
+  if constexpr (NORM) { xg = p.x; gamma = p.gamma; beta = p.beta; }
   chain_wait(xg, gamma, beta);
   chain_next();
 
@@ -338,7 +344,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 }
 
 template <int NT, int RANKS, bool NORM = false>
-cudaError_t launch_gemm_small_r(const CUtensorMap& tw, const CUtensorMap& tx, GemmSmallParams p, cudaStream_t s) {
+cudaError_t launch_gemm_small_r(const CUtensorMap& tw, const CUtensorMap& tx, GemmSmallArgs<NORM> p, cudaStream_t s) {
   auto kern = gemm_small_kernel<NT, RANKS, NORM>;
   const int stage = NORM ? GS_W_BYTES : GsCfg<NT>::STAGE, rows = NORM ? p.kb_per_cta * GsCfg<NT>::X_BYTES : 0;
   const int fit = (GS_SMEM - rows) / stage;
@@ -448,8 +454,7 @@ extern "C" int lb_gemm_small(const void* x, const void* w, void* out, int M, int
   p.err = small_wait_word();
   if (p.err == nullptr) return -20;
   p.M = M; p.N = N; p.K = K;
-  p.kb_total = (K + 63) / 64;
-  p.kb_per_cta = (p.kb_total + ranks - 1) / ranks;
+  p.kb_per_cta = ((K + 63) / 64 + ranks - 1) / ranks;
   p.bias = (const __nv_bfloat16*)bias;
   p.residual = (const __nv_bfloat16*)residual;
   p.out = (__nv_bfloat16*)out;
@@ -482,12 +487,11 @@ extern "C" int lb_gemm_small_norm(const void* x, const void* gamma, const void* 
   int nt = 0, ranks = 0;
   if (!lb_gemm_small_rule(M, N, K, &nt, &ranks) || nt != 16) return -1;
   if (((K + 63) / 64 + ranks - 1) / ranks > lb::GS_NORM_BLOCKS) return -1;
-  lb::GemmSmallParams p{};
+  lb::GemmSmallNormParams p{};
   p.err = small_wait_word();
   if (p.err == nullptr) return -20;
   p.M = M; p.N = N; p.K = K;
-  p.kb_total = (K + 63) / 64;
-  p.kb_per_cta = (p.kb_total + ranks - 1) / ranks;
+  p.kb_per_cta = ((K + 63) / 64 + ranks - 1) / ranks;
   p.bias = (const __nv_bfloat16*)bias;
   p.out = (__nv_bfloat16*)out;
   p.ldo = ldo;
