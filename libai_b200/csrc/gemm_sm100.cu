@@ -1073,13 +1073,16 @@ static int gemm_allow_2cta() {
   return v;
 }
 
-// Time of a product with bf16 results by its tiles, in us: fixed + waves x (per wave + k-blocks x per k-block), but not below w at 6 TB/s.  Fitted over 290
-// products, layouts NT and NN, M = 256 .. 12608, N and K = 384 .. 5120 (3 to 5 % rms per kind).  A pair's tile takes half of B from L2 per SM: 256 x 192 a k-block in
-// 0.235 us on two SMs where two single 128 x 192 tiles take 0.29.  B along rows comes in boxes of 64 columns, of which the 96 of a pair's half take two: 192 wide tiles are dearer
-// there.  Single and pair, us: [8192, 768] x K = 3072 34.8 -> 30.4, [2560, 2048] x 2048 24.9 -> 20.9 (NN 21.8), [2048, 1024] x 4096 21.8 -> 18.1, [12608, 512] x 2048 31.3 -> 25.8.
-// A pair's narrower tile has to be 4 % ahead: it leaves more SMs without work where tiles are few ([180, 1912] x [1912, 1712] 12.0 us in 54 single tiles, 13.3 in 14 of pairs),
-// and against one tile of columns single CTAs are kept ([5997, 2040] x [104, 2040] 13.4 against 14.7).  Beyond four waves the last one matters less than the traffic and power
-// per product ([2048, 4096] x [12288, 4096] 135.8 us 256 wide in six waves, 139.7 192 wide in seven).  256 wide single tiles are for up to 128 rows against much of w.
+// Time of a product with bf16 results by its tiles, in us: fixed + waves x (per wave + k-blocks x per k-block), but not below w at 6 TB/s.  Measured: 150 products each NT and NN
+// (and 48 TN, below), M = 256 .. 12608, N and K = 384 .. 5120; fitted over both together without NT of 256 rows, which the few-row kernel takes, 290 in all (3 to 5 % rms per kind),
+// the 192 wide pair's by layout.  A pair's tile takes half of B from L2 per SM: 256 x 192 a k-block in 0.235 us on two SMs where two single 128 x 192 tiles take 0.29.  B along rows
+// comes in boxes of 64 columns, of which the 96 of a pair's half take two: 192 wide tiles are dearer there.  Single and pair, us: [8192, 768] x K = 3072 34.8 -> 30.4,
+// [2560, 2048] x 2048 24.9 -> 20.9 (NN 21.8), [2048, 1024] x 4096 21.8 -> 18.1, [12608, 512] x 2048 31.3 -> 25.8.
+// The numbers of the 192 and 128 wide pairs are the fit's times 1.04, so that they have to be 4 % ahead: they leave more SMs without work where tiles are few ([180, 1912] x [1912, 1712]
+// 12.0 us in 54 single tiles, 13.3 in 14 of pairs).  Against one tile of columns single CTAs are kept ([5997, 2040] x [104, 2040] 13.4 against 14.7).  Beyond four waves the last one
+// matters less than the traffic and power per product ([2048, 4096] x [12288, 4096] 135.8 us 256 wide in six waves, 139.7 192 wide in seven).  256 wide single tiles are for up to 128 rows
+// against much of w.  Of kinds that are even the one with less to do per SM is taken (`order`: it decides 8 of 2128 sizes tried, 0.2 % apart by the estimate; [6300, 4096] x
+// [4096, 1024] 45.5 us 128 wide, 44.7 256 wide).
 struct TileKind {
   int bn;
   bool pair;
@@ -1135,7 +1138,7 @@ static int split_choice(long tiles, int k_blocks, int sms) {
   return splits;
 }
 // Width of the pair tiles of an accumulation (weight gradients): fixed + rounds x (per round + k-blocks x per k-block) + bytes added.  Fitted over 48 products of up to
-// [3072, 1024], K = 512 .. 8192 (2.5 to 5 % rms; the narrow ones have to be 3 % ahead).  256 wide and the chosen width, us: [1152, 384] x K = 2048 9.9 -> 8.1, [1536, 384] x 2048 9.1 -> 7.4,
+// [3072, 1024], K = 512 .. 8192 (2.5 to 5 % rms; the numbers of the narrow ones are the fit's times 1.03: they have to be 3 % ahead).  256 wide and the chosen width, us: [1152, 384] x K = 2048 9.9 -> 8.1, [1536, 384] x 2048 9.1 -> 7.4,
 // [2304, 768] x 5000 19.2 -> 16.7, [1280, 1280] x 5000 19.3 -> 16.2, [1024, 1024] x 512 8.4 -> 6.8; [3072, 1024] x 8192 and larger keep 256 (the fit's bytes are up to 13 MB, and a
 // MB costs all three the same: [21128, 768] x 1304 took 68 us 128 wide, 50 us 256 wide).
 static int wgrad_tile_choice(int M, int N, int K, int sms) {

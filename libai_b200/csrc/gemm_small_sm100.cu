@@ -26,7 +26,7 @@ struct GsCfg {
   static_assert(PART_BYTES <= 2 * STAGE, "partial sums fit the pipeline");
 };
 constexpr int GS_SMEM = 104000;                   // of pipeline: two CTAs per SM (one with twice the stages leaves no room for clusters of 8 in some GPCs)
-constexpr int GS_NORM_BLOCKS = 11;                // k-blocks per CTA with a norm in front: their rows of x beside five stages of w
+constexpr int GS_NORM_BLOCKS = 11;                // k-blocks per CTA with a norm in front: their rows of x beside four stages of w (five up to ten k-blocks)
 // K-blocks of w that a CTA sends to L2 ahead of chain_wait(): memory stands still while the small kernel before (a norm, a rotation) ends.  128 KB per CTA are what
 // comes in 3 us.  Llama block, one token of 4 sequences on 2046: 151.5 -> 147.5 us (16 k-blocks 148.4); GPT-2 block of 8 sequences on 511: 38.1 -> 37.2.  The same for the first keys
 // and values of the decode attention gave nothing.  Not for small matrices, which are in L2 more often than not: [200, 384] x [384, 384] out of L2 4.56 us, 4.91 with it.
@@ -86,6 +86,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   [[maybe_unused]] uint64_t* x_full = acc_full + 3;
   [[maybe_unused]] float* row_mean = reinterpret_cast<float*>(full_bar + 20);       // 16, then 16 reciprocal deviations (NORM: NT = 16)
   static_assert(!NORM || (NT == 16 && 2 * GS_MAX_STAGES + 4 <= 20), "statistics lie behind the barriers");
+  static_assert(!NORM || (GS_SMEM - GS_NORM_BLOCKS * Cfg::X_BYTES) / GS_W_BYTES == 4, "stages of w beside the most rows of x");
   const int warp_idx = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int rank = blockIdx.x;
   const int n0 = blockIdx.y * 128, m0 = blockIdx.z * NT;
@@ -404,7 +405,8 @@ int* small_wait_word() {
 // kernel was the better one everywhere (nearest: [32, 1024] x [50304, 1024] 24.8 against 25.3 us); above that it is taken where the estimate
 // is 4 % and 0.5 us ahead: few tiles and a long K ([128, 4096] x [1024, 4096] 9.3 against 19.9 us, [200, 11008] x [4096, 11008] 28.6 against
 // 46.6), not many tiles ([64, 1024] x [50304, 1024] 27.3 against 23.4 us, [2048, 5120] x [1280, 5120] 39.6 against 29.3) and not a short K
-// ([256, 384] x [1536, 384] 6.2 against 5.8).  Clusters of 4 and 8 are kept to 264 CTAs: the SMs of a GPC do not divide by them, and 72
+// ([256, 384] x [1536, 384] 6.2 against 5.8).  Near the line, 414 products with 33 to 2048 rows, it is 0.2 % from the better kernel on average; 0.45 us instead of 0.5 would win
+// [136 .. 152, 384] x [1152, 384] (4.9 against 5.2) and lose [512, 768] x [768, 768] and [128, 768] x [3072, 768] (6.8 against 6.6).  Clusters of 4 and 8 are kept to 264 CTAs: the SMs of a GPC do not divide by them, and 72
 // clusters of 4 with two CTAs per SM ran in two waves ([96, 1024] x [3072, 1024] 10.2 against 8.2 us).
 // More than 2048 rows only against one tile of 16 to 128 columns (the gates of a mixer), where the other kernel walks all of K in one CTA:
 // [2560, 2048] x [16, 2048] 9.6 against 11.1 us, x [128, 2048] 9.2 against 11.4, [4096, 4096] x [32, 4096] 9.8 against 18.6, [8192, 4096] x [64, 4096]

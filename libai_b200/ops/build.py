@@ -6,7 +6,8 @@ hyper-connection streams, decayed linear-attention recurrences, matrix memory wi
     python -m libai_b200.ops.build [--force] [--verbose] [--only _C|_C_seq|_C_kv|_C_lin]
 
 CUDA sources are compiled for sm_100a only (``-gencode arch=compute_100a,code=sm_100a -lineinfo``);
-nvcc cross-compiles without a GPU.  Objects are cached under ``libai_b200/csrc/build`` keyed by
+nvcc cross-compiles without a GPU.  ``_C`` also wants Python's headers and links ``libtorch_python``: its graph nodes read
+and set attributes of parameters (``main_grad``).  Objects are cached under ``libai_b200/csrc/build`` keyed by
 source mtime.
 """
 from __future__ import annotations
@@ -91,7 +92,7 @@ def _build_lib(SO_PATH, CU_SOURCES, CPP_SOURCES, NVCC_FLAGS, ext_name, force, ve
         objs.append(obj)
         if force or _stale(src, obj, headers):
             jobs.append((s, [NVCC, *NVCC_FLAGS, "-I", CSRC, "-c", src, "-o", obj]))
-    inc = ["-isystem", sysconfig.get_paths()["include"]]
+    inc = ["-isystem", sysconfig.get_paths()["include"]] if "autograd_nodes.cpp" in cpp else []
     for p in cpp_extension.include_paths(device_type="cuda"):
         inc += ["-isystem", p]
     abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)

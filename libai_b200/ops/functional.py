@@ -726,7 +726,7 @@ _SPLIT_LAYOUTS = {"qkv": 0, "q_kv": 1, "q_k_v": 2}
 
 
 class _SplitAttnFn(torch.autograd.Function):
-    """Attention whose probabilities reach the tensor core as two bf16 parts (``layout``: see :func:`_split_views`)."""
+    """Attention whose probabilities reach the tensor core as three bf16 parts (``layout``: see :func:`_split_views`)."""
 
     @staticmethod
     def forward(ctx, layout, causal, scale, mask, *ts):

@@ -256,8 +256,8 @@ def linear(a, w, bias=None):
 
 
 def linears(a, ws):
-    """``cat(ws)`` applied to ``a`` in one launch that reads the matrices where they are: ``[rows, Σ n_i]``, or ``None`` where that launch does not take them (the
-    products of up to 128 rows are ahead one by one, in the kernel for few rows)."""
+    """``cat(ws)`` applied to ``a`` in one launch that reads the matrices where they are: ``[rows, Σ n_i]``, or ``None`` where that launch does not take them (more than
+    eight matrices, rows or widths that are no multiples of 8, memory off its 16 bytes, other types)."""
     from . import load_ext, use_native
 
     if a.is_cuda and a.dtype == torch.bfloat16 and use_native(a) and a.dim() == 2:
