@@ -541,8 +541,9 @@ std::tuple<Tensor, Tensor, Tensor> norm_bwd(const Tensor& gy, const Tensor& x, c
                               dbeta_accum->is_contiguous()),
                 "norm_bwd: dbeta_accum must be contiguous fp32 [H]");
   }
-  Tensor dgamma = acc ? dgamma_accum.value() : at::empty({H}, fopt);
-  Tensor dbeta = !has_bias ? at::empty({0}, fopt) : (acc ? dbeta_accum.value() : at::empty({H}, fopt));
+  auto column = [&] { return rows == 0 ? at::zeros({H}, fopt) : at::empty({H}, fopt); };      // (no rows: nothing is launched)
+  Tensor dgamma = acc ? dgamma_accum.value() : column();
+  Tensor dbeta = !has_bias ? at::empty({0}, fopt) : (acc ? dbeta_accum.value() : column());
   const int wrows = lb_norm_bwd_workspace_rows(rows, H);
   Tensor ws = at::empty({2 * (int64_t)wrows * H}, fopt);
   // optional gradient of the skip connection around this norm: added to gx inside the kernel when supported

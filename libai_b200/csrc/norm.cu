@@ -616,12 +616,12 @@ __global__ void norm_bwd_generic(const T* __restrict__ gy, const T* __restrict__
 }  // namespace lb
 
 namespace {
-int norm_sms() {
+int norm_sms() {                                  // (without a device: of the chip that the grids are made for)
   static int sms = 0;
   if (sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
+    sms = n;
   }
   return sms;
 }
@@ -636,6 +636,7 @@ int norm_fwd_grid(int rows) { return norm_grid_of(rows, lb::NORM_WARPS, 4); }
 // bf16 backward: up to three 4-warp blocks per SM (one wave), but no more than give every warp up to three rows once there is a block per SM: every block adds or leaves
 // a row of column sums, which took longer than the rows ([1812, 256] 453 blocks 5.3 us, 151 blocks 3.3; [2048, 384] 6.2 and 5.1; [200, 384] 50 blocks 2.8, 17 blocks 4.2).
 int norm_bwd_bf16_grid(int rows, int H, bool sums) {
+  if (rows <= 0) return 0;
   const int per_sm = lb::NORM_BWD_WARPS * norm_sms(), want = (rows + per_sm - 1) / per_sm, each = want < lb::NORM_BWD_STAGES ? want : lb::NORM_BWD_STAGES;
   return norm_grid_of(rows, lb::NORM_BWD_WARPS * each, lb::norm_bwd_blocks((H + 255) / 256, sums));
 }

@@ -89,6 +89,15 @@ def test_rule_of_few_rows_answers_without_a_device(m, n, k, few):
     assert ctypes.CDLL(so_path()).lb_gemm_small_rule(m, n, k, ctypes.byref(nt), ctypes.byref(ranks)) == few
 
 
+@pytest.mark.skipif(torch.cuda.is_available() or not os.path.exists(so_path()), reason="host side of the C entry only")
+@pytest.mark.parametrize("h", [8, 512, 1024, 1280, 4096, 8192])
+def test_workspace_of_norm_backward(h):
+    """One row per block, none for no rows."""
+    rows = ctypes.CDLL(so_path()).lb_norm_bwd_workspace_rows
+    assert rows(0, h) == 0 and rows(1, h) == 1
+    assert all(0 < rows(n, h) <= min(n, 3 * 148) for n in (2, 5, 148, 593, 1777, 8192, 100000))
+
+
 def test_implementation_switch_follows_the_environment(monkeypatch):
     monkeypatch.delenv("LIBAI_B200_IMPL", raising=False)
     assert ops.impl() == "native"

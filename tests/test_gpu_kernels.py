@@ -1480,3 +1480,20 @@ def test_launches_of_a_generation_step_are_counted(kind, batch):
             torch.cuda.synchronize()
     ran = sum(e.count for e in prof.key_averages() if "lb::" in e.key)
     assert counted == ran > 0
+
+
+@pytest.mark.parametrize("main_grad", [False, True])
+@pytest.mark.parametrize("rms", [False, True])
+@pytest.mark.parametrize("h", [64, 1000, 1280, 12288])
+def test_norm_of_no_rows(h, rms, main_grad):
+    """An empty batch forward and back: empty results, zeros for the parameters."""
+    x = torch.empty(0, h, device="cuda", dtype=BF16, requires_grad=True)
+    w, b = (torch.nn.Parameter(_rand((h,), i)) for i in (1, 2))
+    for p in (w, b):
+        if main_grad:
+            p.main_grad = torch.full((h,), 3.0, device="cuda")
+    y = OF.rms_norm(x, w) if rms else OF.layer_norm(x, w, b)
+    y.backward(torch.empty_like(y))
+    assert y.shape == x.grad.shape == (0, h)
+    for p in (w,) if rms else (w, b):
+        assert bool((p.main_grad == 3).all()) if main_grad else bool((p.grad == 0).all())
