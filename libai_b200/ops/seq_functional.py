@@ -62,7 +62,7 @@ def linear_accumulate(x32, a, w):
 
     if (a.is_cuda and a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and use_native(a) and a.stride(-1) == 1
             and a.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 and w.shape[0] % 8 == 0 and x32.stride(0) % 4 == 0
-            and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and a.shape[0] > 0):
+            and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and x32.data_ptr() % 16 == 0 and a.shape[0] > 0):
         if _tcgen05_gemm(a, w, x32, True, torch.float32) is not None:
             return x32
     if a.dtype == torch.float32:

@@ -1497,3 +1497,18 @@ def test_norm_of_no_rows(h, rms, main_grad):
     assert y.shape == x.grad.shape == (0, h)
     for p in (w,) if rms else (w, b):
         assert bool((p.main_grad == 3).all()) if main_grad else bool((p.grad == 0).all())
+
+
+def test_residual_stream_off_its_alignment_refuses_nothing_for_later():
+    """A stream that TMA cannot write takes the other product; the next one of those sizes, on its 16 bytes, does not."""
+    from libai_b200.ops import seq_functional as SF
+
+    a, w, buf = _rand((40, 64), 1), _rand((24, 64), 2), _rand((40 * 24 + 1,), 3, dtype=torch.float32)
+    before = set(SF._GEMM_REFUSED)
+    for off in (1, 0):
+        x = buf[off:off + 40 * 24].view(40, 24)
+        want = x.double() + a.double() @ w.double().t()
+        SF.linear_accumulate(x, a, w)
+        # (the product passes through bf16 where the stream is off its alignment)
+        assert float((x.double() - want).norm()) < (2.0 ** -8 if off else 2.0 ** -20) * float(want.norm())
+    assert SF._GEMM_REFUSED == before
