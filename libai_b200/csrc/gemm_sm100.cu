@@ -192,7 +192,8 @@ LB_DEVICE void stg_store_chunk(uint8_t* stg, int lane, const float (&v)[32], __n
 }
 
 // What only some kinds of the kernel take lies behind the collectives' parameters in one argument, so that the others pass nothing for it.  What a launch costs the host depends on the
-// bytes of its arguments: with 57 to 72 beyond a multiple of 64 it is 0.3 us less (3.5 against 3.8 us; an empty struct as an argument of its own made 776 bytes 777).
+// bytes of its arguments: with 57 to 72 beyond a multiple of 64 it is 0.25 us less (776 bytes and 56 more 3.5 us, 8 to 48 more 3.7 to 3.8; an empty struct as an argument of its own had made
+// 776 bytes 777).
 struct GemmReduce : CommParams { CUtensorMap map; };      // EPI_ATOMIC_F32: the output in boxes of 32 x 32
 // MULTI: B is several matrices [n[i], K] in memory of their own, one after the other along the columns of the output (NT, CTA pairs, bf16 results)
 constexpr int GEMM_MAX_B = 8;
