@@ -1200,7 +1200,8 @@ def _train_block(kind, dim, with_main_grad, s=40):
                                       ("causal-prefix", 48), ("causal-prefix", 64), ("causal-padded", 24), ("causal-padded", 64), ("causal-left", 32), ("causal-left", 64)])
 def test_block_graph_in_one_call(kind, dim, main_grad):
     """One node per block, one per operator (a hook on a module) and the Python functions (a dispatch mode looks on) launch the same kernels: outputs to
-    the bit, gradients up to the order of their sums; a second backward pass, checkpointing, frozen parameters and a graph of the gradients work as with the modules."""
+    the bit, gradients up to the order of their sums; a second backward pass, checkpointing and frozen parameters work as with the modules, and create_graph gives the same gradients
+    (constants: the test below)."""
     from torch.utils._python_dispatch import TorchDispatchMode
     from torch.utils.checkpoint import checkpoint
 
